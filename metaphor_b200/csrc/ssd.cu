@@ -29,6 +29,8 @@
 #include <cuda.h>
 #include <mutex>
 
+bool mp_ssd_walk_supported(int L, int H, int P, int N, int G);   // ssd_walk.cu
+
 namespace {
 
 #ifndef SSD_XF
@@ -598,7 +600,8 @@ __global__ void __launch_bounds__(256) ssd_boundary_dot_kernel(const __half* __r
 }
 
 // One CTA per (b, h); one thread per step of a chunk (Q <= 256), chunks walked from the last to the first.
-// `halves` = 2: u and v are the sums of two arrays, the second `B*H*L` elements after the first.
+// u, v, dtt: [B, H, LP], LP = L padded to whole chunks (dt = 0 there).  `halves` = 2: u and v are the sums of two arrays, the
+// second `B*H*LP` elements after the first.
 // With `raw` (the projection's raw step sizes, r16, pitched) the reverse of dt = softplus(raw + bias[h]) is applied on the
 // way out: graw = gdt * sigmoid(raw + bias) (r16, pitched), gbias[h] += its sum (the arithmetic of launch_softplus_bias_reverse).
 __device__ __forceinline__ float ssd_sigmoid(float x) {
@@ -610,7 +613,7 @@ __device__ __forceinline__ float ssd_sigmoid(float x) {
 __global__ void __launch_bounds__(256) ssd_scalar_grads_kernel(const float* __restrict__ u, const float* __restrict__ v,
                                                                const float* __restrict__ dtt, const float* __restrict__ A,
                                                                const float* __restrict__ pin, float* __restrict__ gdt,
-                                                               float* __restrict__ gA_part, int B, int L, int H, int Q, int halves,
+                                                               float* __restrict__ gA_part, int B, int L, int LP, int H, int Q, int halves,
                                                                const __half* __restrict__ raw = nullptr, size_t raw_pitch = 0,
                                                                const float* __restrict__ bias = nullptr, __half* __restrict__ graw = nullptr,
                                                                size_t graw_pitch = 0, float* __restrict__ gbias = nullptr) {
@@ -620,15 +623,15 @@ __global__ void __launch_bounds__(256) ssd_scalar_grads_kernel(const float* __re
   __shared__ float gb_red[8];
   float gb_acc = 0.f;
   const int h = blockIdx.x % H, b = blockIdx.x / H;
-  const size_t base = (static_cast<size_t>(b) * H + h) * L;
-  const int nc = L / Q;
+  const size_t base = (static_cast<size_t>(b) * H + h) * LP;
+  const int nc = LP / Q;
   const float Ah = A[h];
   float ga_acc = 0.f;
   for (int c = nc - 1; c >= 0; --c) {
     const int j = static_cast<int>(threadIdx.x);           // thread 0 holds the latest step of the chunk
     const int t = c * Q + (Q - 1 - j);
     const bool in = j < Q;
-    const size_t hs = static_cast<size_t>(B) * H * L;
+    const size_t hs = static_cast<size_t>(B) * H * LP;
     float ut = 0.f, vt = 0.f;
     if (in) {
       ut = u[base + t]; vt = v[base + t];
@@ -651,7 +654,7 @@ __global__ void __launch_bounds__(256) ssd_scalar_grads_kernel(const float* __re
     const float right = pin[(static_cast<size_t>(b) * H + h) * nc + c];          // g_a just after the chunk
     float resid = 0.f;
     if (c > 0) resid = pin[(static_cast<size_t>(b) * H + h) * nc + c - 1] - (right + total_s);   // what the first step should reach
-    if (in) {
+    if (in && t < L) {
       const float ga = right + within + resid * (static_cast<float>(j + 1) / static_cast<float>(Q));
       const float dtv = dtt[base + t];
       const float gd = vt / dtv + Ah * ga;
@@ -905,11 +908,17 @@ void ssd_operator(const SsdDims& d, const Roles& r, const SsdScratch& sc, uint32
   }
 }
 
-// Shapes the tensor-core path covers; everything else takes the sequential-recurrence kernels of ssd_generic.cu.
+// The shapes whose `chunk` argument the three-phase path can evaluate.
+bool ssd_whole_chunks(const SsdDims& d) {
+  return d.N == 128 && (d.P == 64 || d.P == 128) && (d.Q == 128 || d.Q == 256) && d.L % d.Q == 0;
+}
+
+// Shapes the tensor-core paths cover; everything else takes the sequential-recurrence kernels of ssd_generic.cu.  The
+// chunk walk takes any sequence length, whatever the `chunk` argument (its chunks are 128 steps, the last one padded): on
+// [2, 1000, 24, 64] forward + reverse the recurrence needs 43.7 ms, one step after the other on 48 SMs.
 bool ssd_tensor_path(const SsdDims& d) {
   if (d.G <= 0 || d.H % d.G != 0) MP_FATAL("ssd_scan: heads %d not divisible by groups %d", d.H, d.G);
-  return d.N == 128 && (d.P == 64 || d.P == 128) && (d.Q == 128 || d.Q == 256) && d.L % d.Q == 0 &&
-         getenv("MP_SSD_FORCE_GENERIC") == nullptr;
+  return (mp_ssd_walk_supported(d.L, d.H, d.P, d.N, d.G) || ssd_whole_chunks(d)) && getenv("MP_SSD_FORCE_GENERIC") == nullptr;
 }
 
 SsdDims ssd_dims(len_t batch, len_t seqlen, len_t heads, len_t headdim, len_t dstate, len_t ngroups, len_t chunk) {
@@ -931,7 +940,6 @@ void mp_ssd_generic_reverse_r16(const void* x, const void* dt, const void* A, co
                                 len_t dstate, len_t ngroups, StreamContext ctx);
 
 // chunk-walk kernels (ssd_walk.cu)
-bool mp_ssd_walk_supported(int L, int H, int P, int N, int G);
 void mp_ssd_walk_cumsum(const float* dt, const float* A, float* cum, float* dtt, float* colf_c, float* colf_a, int B, int L, int H,
                         int* carry_flags, int n_flags, cudaStream_t st);
 void mp_ssd_walk_cumsum_raw(const __half* raw, size_t raw_pitch, const float* bias, const float* A_log, float* dt_out, float* A_out, float* cum,
@@ -948,19 +956,24 @@ namespace {
 // Scratch of the walk path: prefix sums and dt in [B,H,L] order; for the reverse also the states every 128-step
 // chunk receives from its predecessors and from its successors (r16 [B,H,L/128][128][64]).
 struct WalkScratch { float* cum; float* dtt; float* colf_c; float* colf_a; __half* hs_causal; __half* hs_anti; float* pin; float* u; float* v; float* ga_part; float* carry_c; float* carry_a; int* flags; size_t total; };
+// The forward takes the chunk walk where it applies; MP_SSD_LEGACY_FORWARD selects the three-phase path on the shapes that it has too.
+bool ssd_forward_walks(const SsdDims& d) {
+  return mp_ssd_walk_supported(d.L, d.H, d.P, d.N, d.G) && (getenv("MP_SSD_LEGACY_FORWARD") == nullptr || !ssd_whole_chunks(d));
+}
 WalkScratch walk_carve(void* base, const SsdDims& d, bool reverse, size_t off0) {
   WalkScratch w;
   size_t off = off0;
   auto take = [&](size_t bytes) { void* p = base ? static_cast<unsigned char*>(base) + off : nullptr; off += (bytes + 255) & ~size_t(255); return p; };
-  const size_t bhl = static_cast<size_t>(d.B) * d.H * d.L;
+  const size_t nc = (static_cast<size_t>(d.L) + 127) / 128;
+  const size_t bhl = static_cast<size_t>(d.B) * d.H * nc * 128;
   w.cum = static_cast<float*>(take(bhl * 4));
   w.dtt = static_cast<float*>(take(bhl * 4));
   w.colf_c = static_cast<float*>(take(bhl * 4));
   w.colf_a = static_cast<float*>(take(reverse ? bhl * 4 : 0));
-  const size_t st = static_cast<size_t>(d.B) * d.H * (d.L / 128) * 128 * 64 * 2;
+  const size_t st = static_cast<size_t>(d.B) * d.H * nc * 128 * 64 * 2;
   w.hs_causal = static_cast<__half*>(take(reverse ? st : 0));
   w.hs_anti = static_cast<__half*>(take(reverse ? st : 0));
-  w.pin = static_cast<float*>(take(reverse ? static_cast<size_t>(d.B) * d.H * (d.L / 128) * 4 : 0));
+  w.pin = static_cast<float*>(take(reverse ? static_cast<size_t>(d.B) * d.H * nc * 4 : 0));
   w.u = static_cast<float*>(take(reverse ? 2 * bhl * 4 : 0));     // one array per half of the columns
   w.v = static_cast<float*>(take(reverse ? 2 * bhl * 4 : 0));
   w.ga_part = static_cast<float*>(take(reverse ? static_cast<size_t>(d.B) * d.H * 4 : 0));
@@ -983,7 +996,7 @@ extern "C" len_t mpSsdScanScratchBytes(len_t batch, len_t seqlen, len_t heads, l
   if (mp_ssd_walk_supported(d.L, d.H, d.P, d.N, d.G)) {
     if (reverse != 0) return walk_carve(nullptr, d, true, 0).total;
     // (the three-phase forward, an A/B switch, needs its own larger scratch: ask with the switch set)
-    return getenv("MP_SSD_LEGACY_FORWARD") == nullptr ? walk_carve(nullptr, d, false, 0).total : ssd_carve(nullptr, d, false).total;
+    return ssd_forward_walks(d) ? walk_carve(nullptr, d, false, 0).total : ssd_carve(nullptr, d, false).total;
   }
   return ssd_carve(nullptr, d, reverse != 0).total;
 }
@@ -995,7 +1008,7 @@ extern "C" void launch_ssd_scan_r16(const void* x, const void* dt, const void* A
                                     len_t ngroups, len_t chunk, StreamContext ctx) {
   if (batch == 0 || seqlen == 0 || heads == 0) return;
   const SsdDims d = ssd_dims(batch, seqlen, heads, headdim, dstate, ngroups, chunk);
-  if (!ssd_tensor_path(d)) {
+  if (!ssd_tensor_path(d) || (scratch == nullptr && !ssd_whole_chunks(d))) {   // the recurrence's forward needs no scratch
     mp_ssd_generic_forward_r16(x, dt, A, Bm, Cm, y, batch, seqlen, heads, headdim, dstate, ngroups, ctx);
     return;
   }
@@ -1004,7 +1017,7 @@ extern "C" void launch_ssd_scan_r16(const void* x, const void* dt, const void* A
   cudaStream_t st = mp_stream(ctx);
   // The chunk walk (no chunk state in global memory) where it applies; MP_SSD_LEGACY_FORWARD selects the three-phase
   // path (scores, chunk states, scan, output as separate kernels), which also serves head size 128.
-  if (mp_ssd_walk_supported(d.L, d.H, d.P, d.N, d.G) && getenv("MP_SSD_LEGACY_FORWARD") == nullptr) {
+  if (ssd_forward_walks(d)) {
     const WalkScratch w = walk_carve(scratch, d, false, 0);
     mp_ssd_walk_cumsum(static_cast<const float*>(dt), static_cast<const float*>(A), w.cum, w.dtt, w.colf_c, nullptr, d.B, d.L, d.H, w.flags,
                        2 * d.B * d.H, st);
@@ -1049,7 +1062,7 @@ extern "C" void launch_ssd_scan_raw_r16(const void* x, const void* dt_raw, len_t
                                         len_t headdim, len_t dstate, len_t ngroups, len_t chunk, StreamContext ctx) {
   if (batch == 0 || seqlen == 0 || heads == 0) return;
   const SsdDims d = ssd_dims(batch, seqlen, heads, headdim, dstate, ngroups, chunk);
-  if (ssd_tensor_path(d) && mp_ssd_walk_supported(d.L, d.H, d.P, d.N, d.G) && getenv("MP_SSD_LEGACY_FORWARD") == nullptr) {
+  if (ssd_tensor_path(d) && ssd_forward_walks(d) && (scratch != nullptr || ssd_whole_chunks(d))) {
     if (scratch == nullptr) MP_FATAL("ssd_scan_raw: scratch must not be NULL");
     MpStreamState* state = mp_state(ctx);
     cudaStream_t st = mp_stream(ctx);
@@ -1145,16 +1158,16 @@ static bool ssd_scan_reverse_r16_impl(const void* x, const void* dt, const void*
     }
     mp_ssd_group_grads(gyh, xh, bh, ch, w.hs_causal, w.hs_anti, w.cum, w.dtt, w.colf_c, static_cast<__half*>(gB), static_cast<__half*>(gC),
                        d.B, d.L, d.H, d.G, state->status_dev, st);
-    const int wnc = d.L / 128;
+    const int wnc = (d.L + 127) / 128;
     ssd_boundary_dot_kernel<<<d.B * d.H * wnc, 256, 0, lane1>>>(w.hs_anti, w.hs_causal, w.pin, wnc, d.N * d.P);
     MP_LAUNCH_CHECK();
     if (rs != nullptr)
       ssd_scalar_grads_kernel<<<d.B * d.H, 256, 0, lane1>>>(w.u, w.v, w.dtt, static_cast<const float*>(A), w.pin, static_cast<float*>(gdt), w.ga_part,
-                                                           d.B, d.L, d.H, 128, 2, rs->raw, rs->raw_pitch, rs->bias, rs->graw, rs->graw_pitch,
+                                                           d.B, d.L, wnc * 128, d.H, 128, 2, rs->raw, rs->raw_pitch, rs->bias, rs->graw, rs->graw_pitch,
                                                            rs->gbias);
     else
       ssd_scalar_grads_kernel<<<d.B * d.H, 256, 0, lane1>>>(w.u, w.v, w.dtt, static_cast<const float*>(A), w.pin, static_cast<float*>(gdt), w.ga_part,
-                                                           d.B, d.L, d.H, 128, 2);
+                                                           d.B, d.L, wnc * 128, d.H, 128, 2);
     MP_LAUNCH_CHECK();
     ssd_sum_batches_kernel<<<(d.H + 127) / 128, 128, 0, lane1>>>(w.ga_part, static_cast<float*>(gA), d.B, d.H, static_cast<const float*>(A),
                                                                  rs != nullptr ? rs->gA_log : nullptr);
@@ -1224,7 +1237,7 @@ static bool ssd_scan_reverse_r16_impl(const void* x, const void* dt, const void*
     ssd_boundary_dot_kernel<<<d.B * d.H * d.nc, 256, 0, st>>>(sc.hs_op[0], sc.hs_op[1], sc.pin, d.nc, d.N * d.P);
     MP_LAUNCH_CHECK();
     ssd_scalar_grads_kernel<<<d.B * d.H, 256, 0, st>>>(sc.u, sc.v, sc.dtt, static_cast<const float*>(A), sc.pin, static_cast<float*>(gdt),
-                                                      sc.ga_part, d.B, d.L, d.H, d.Q, 1);
+                                                      sc.ga_part, d.B, d.L, d.L, d.H, d.Q, 1);
     MP_LAUNCH_CHECK();
   ssd_sum_batches_kernel<<<(d.H + 127) / 128, 128, 0, st>>>(sc.ga_part, static_cast<float*>(gA), d.B, d.H);
   MP_LAUNCH_CHECK();

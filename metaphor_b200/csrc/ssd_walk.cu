@@ -48,14 +48,17 @@ constexpr uint32_t TC_G = 0, TC_S = 128, TC_Y = 192, TC_COLS = 512;   // Yd / Yo
 
 enum { B_FULL0 = 0, B_FULL1, B_EMPTY0, B_EMPTY1, B_GFULL, B_PREADY, B_VSREADY, B_HREADY, B_YFULL, B_SFULL, B_SCAL, B_COUNT };
 
+// Sequence lengths need not be a multiple of the chunk: the tensor maps are [batch, step, column], so the rows of the last
+// chunk beyond the sequence are read as zeros (and not written), and their dt is zero, which makes them steps that neither
+// decay nor feed the state.  Arrays per step of the scratch are padded to LP = nc * 128 steps.
 struct WalkArgs {
   int B, L, H, G, nc;
-  const float* cum;        // [B, H, L] inclusive prefix sums of dt*A inside each 128-step chunk
-  const float* dtt;        // [B, H, L] dt
-  const float* colf;       // [B, H, L] column factor of every step relative to the far end of its 8-step piece
+  const float* cum;        // [B, H, LP] inclusive prefix sums of dt*A inside each 128-step chunk
+  const float* dtt;        // [B, H, LP] dt
+  const float* colf;       // [B, H, LP] column factor of every step relative to the far end of its 8-step piece
   __half* out;             // [B*L, H*64] or null
   const __half* z;         // dot partner, same indexing as out, or null
-  float* dot_out;          // [2][B, H, L] row dots <z, out> from the fp32 accumulators, one array per half of the columns, or null
+  float* dot_out;          // [2][B, H, LP] row dots <z, out> from the fp32 accumulators, one array per half of the columns, or null
   __half* hs_out;          // [B, H, nc][128][64]: state every chunk receives, or null
   float* carry;            // [B * H][128][64] fp32: state handed from the CTA that walked the first part of a sequence to the next
   int* carry_flag;         // [B * H]: number of worker warps (of 8) that have written their part of `carry`; zero before the launch
@@ -112,9 +115,9 @@ __device__ __forceinline__ bool walk_wait(uint64_t* bar, uint32_t parity, uint32
   return mbar_wait_abortable(bar, parity, status, abort);
 }
 
-// DOT: the row dots <z, out> are wanted (the reverse pass); a template parameter, so that the forward pass does not
+// RAGGED: L is no multiple of the chunk (rows of z and out beyond it must not be touched).  DOT: the row dots <z, out> are wanted (the reverse pass); a template parameter, so that the forward pass does not
 // carry the registers of the dot partner's rows.
-template <int ANTI, bool DOT>
+template <int ANTI, bool DOT, bool RAGGED>
 __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_constant__ CUtensorMap map_q,
                                                                const __grid_constant__ CUtensorMap map_k,
                                                                const __grid_constant__ CUtensorMap map_v,
@@ -165,13 +168,13 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_con
           const int s = q & 1;
           if (!walk_wait(bars + B_EMPTY0 + s, ((q >> 1) & 1) ^ 1u, g.status, abort)) { ok = false; break; }
           unsigned char* st = smem + s * W_STAGE;
-          const int row0 = b * g.L + c * WQ;
+          const int row0 = c * WQ;
           mbar_arrive_expect_tx(bars + B_FULL0 + s, W_STAGE);
-          tma_load_2d(st, &map_q, grp * WN, row0, bars + B_FULL0 + s);
-          tma_load_2d(st + WQ * 128, &map_q, grp * WN + 64, row0, bars + B_FULL0 + s);
-          tma_load_2d(st + W_TILE_QK, &map_k, grp * WN, row0, bars + B_FULL0 + s);
-          tma_load_2d(st + W_TILE_QK + WQ * 128, &map_k, grp * WN + 64, row0, bars + B_FULL0 + s);
-          tma_load_2d(st + 2 * W_TILE_QK, &map_v, h * WP, row0, bars + B_FULL0 + s);
+          tma_load_3d(st, &map_q, grp * WN, row0, b, bars + B_FULL0 + s);
+          tma_load_3d(st + WQ * 128, &map_q, grp * WN + 64, row0, b, bars + B_FULL0 + s);
+          tma_load_3d(st + W_TILE_QK, &map_k, grp * WN, row0, b, bars + B_FULL0 + s);
+          tma_load_3d(st + W_TILE_QK + WQ * 128, &map_k, grp * WN + 64, row0, b, bars + B_FULL0 + s);
+          tma_load_3d(st + 2 * W_TILE_QK, &map_v, h * WP, row0, b, bars + B_FULL0 + s);
         }
         qb += sg.n;
       }
@@ -271,9 +274,9 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_con
     const int n = sg.n;
     const int h = sg.seq % g.H, b = sg.seq / g.H;
     const size_t bh = static_cast<size_t>(sg.seq);
-    const float* cum_g = g.cum + bh * g.L;
-    const float* dt_g = g.dtt + bh * g.L;
-    const float* colf_g = g.colf + bh * g.L;
+    // this thread's step in the first chunk of the sequence, in the arrays per step (one offset, not one pointer per array:
+    // the loop below is short of registers)
+    const size_t step0 = bh * (static_cast<size_t>(g.nc) * WQ) + r;
     float state[32];
     const int c_first = ANTI ? nc - 1 - sg.p0 : sg.p0;
     if (sg.cin) {
@@ -328,12 +331,12 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_con
     // scalars of the walk: chunk in hand (cur), the one after it (nxt), and one more in flight (pre), so that
     // their loads are never waited for
     float cum_cur = 0.f, dt_cur = 0.f, last_cur = 0.f;
-    float cum_nxt = cum_g[c_first * WQ + r], dt_nxt = dt_g[c_first * WQ + r], colf_nxt = colf_g[c_first * WQ + r];
+    float cum_nxt = g.cum[step0 + c_first * WQ], dt_nxt = g.dtt[step0 + c_first * WQ], colf_nxt = g.colf[step0 + c_first * WQ];
     float last_nxt = 0.f;
     float cum_pre = 0.f, dt_pre = 0.f, colf_pre = 0.f;
     if (n > 1) {
       const int c1 = ANTI ? c_first - 1 : c_first + 1;
-      cum_pre = cum_g[c1 * WQ + r]; dt_pre = dt_g[c1 * WQ + r]; colf_pre = colf_g[c1 * WQ + r];
+      cum_pre = g.cum[step0 + c1 * WQ]; dt_pre = g.dtt[step0 + c1 * WQ]; colf_pre = g.colf[step0 + c1 * WQ];
     }
 
     // Iteration k finishes chunk k of the segment and prepares chunk k+1; k = -1 is the lead-in that only prepares chunk 0.
@@ -353,7 +356,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_con
           cum_nxt = cum_pre; dt_nxt = dt_pre; colf_nxt = colf_pre;
           if (k + 2 < n) {
             const int c2 = ANTI ? c_first - k - 2 : c_first + k + 2;
-            cum_pre = cum_g[c2 * WQ + r]; dt_pre = dt_g[c2 * WQ + r]; colf_pre = colf_g[c2 * WQ + r];
+            cum_pre = g.cum[step0 + c2 * WQ]; dt_pre = g.dtt[step0 + c2 * WQ]; colf_pre = g.colf[step0 + c2 * WQ];
           }
         }
         // Yd(k) has consumed the P tile, and every warp is past the shared scalars of chunk k
@@ -427,7 +430,9 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_con
         if (DOT) {    // the dot partner's rows of chunk k, whole 64-byte row pieces per load
 #pragma unroll
           for (int it = 0; it < 4; ++it) {
-            const size_t zrow = static_cast<size_t>(b) * g.L + c * WQ + quarter * 32 + it * 8 + (lane >> 2);
+            int zt = c * WQ + quarter * 32 + it * 8 + (lane >> 2);
+            if (RAGGED) zt = min(zt, g.L - 1);   // the output rows beyond the sequence are zero: any row serves as their partner
+            const size_t zrow = static_cast<size_t>(b) * g.L + zt;
             zc[it] = *reinterpret_cast<const uint4*>(g.z + zrow * pitch + h * WP + ch * 32 + (lane & 3) * 8);
           }
         }
@@ -503,7 +508,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_con
               dot += zf.x * o[q4 * 8 + 2 * e] + zf.y * o[q4 * 8 + 2 * e + 1];
             }
           }
-          g.dot_out[static_cast<size_t>(ch) * g.B * g.H * g.L + bh * g.L + c * WQ + r] = dot;
+          g.dot_out[static_cast<size_t>(ch) * g.B * g.H * (static_cast<size_t>(g.nc) * WQ) + step0 + c * WQ] = dot;
           __syncwarp();
         }
         if (g.out != nullptr) {
@@ -525,7 +530,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_con
             const int lr = quarter * 32 + it * 8 + (lane >> 2), cc = ch * 4 + (lane & 3);
             const uint4 val = *reinterpret_cast<const uint4*>(stg + lr * 128 + ((cc ^ (lr & 7)) << 4));
             const size_t orow = static_cast<size_t>(b) * g.L + c * WQ + lr;
-            *reinterpret_cast<uint4*>(g.out + orow * pitch + h * WP + cc * 8) = val;
+            if (!RAGGED || c * WQ + lr < g.L) *reinterpret_cast<uint4*>(g.out + orow * pitch + h * WP + cc * 8) = val;
           }
           __syncwarp();
         }
@@ -580,7 +585,7 @@ enum { GB_FULL0 = 0, GB_FULL1, GB_EMPTY0, GB_EMPTY1, GB_SC0, GB_SC1, GB_SCALED, 
 
 struct GroupArgs {
   int B, L, H, G, nc;
-  const float* cum; const float* dtt; const float* colf;   // [B, H, L], causal column factors
+  const float* cum; const float* dtt; const float* colf;   // [B, H, nc * 128], causal column factors
   uint32_t* status;
 };
 
@@ -606,7 +611,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_group_grads_kernel(const __g
   const int grp = blockIdx.x % g.G;
   const int c = (blockIdx.x / g.G) % g.nc;
   const int b = blockIdx.x / (g.G * g.nc);
-  const int row0 = b * g.L + c * WQ;
+  const int row0 = c * WQ;
   const int nh = hpg;
 
   if (threadIdx.x == 0) {
@@ -634,8 +639,8 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_group_grads_kernel(const __g
         unsigned char* st = smem + s * GG_STAGE;
         const int srow = ((b * g.H + h) * g.nc + c) * WN;
         mbar_arrive_expect_tx(bars + GB_FULL0 + s, GG_STAGE);
-        tma_load_2d(st, &map_gy, h * WP, row0, bars + GB_FULL0 + s);
-        tma_load_2d(st + GG_TILE, &map_x, h * WP, row0, bars + GB_FULL0 + s);
+        tma_load_3d(st, &map_gy, h * WP, row0, b, bars + GB_FULL0 + s);
+        tma_load_3d(st + GG_TILE, &map_x, h * WP, row0, b, bars + GB_FULL0 + s);
         tma_load_2d(st + 2 * GG_TILE, &map_hc, 0, srow, bars + GB_FULL0 + s);
         tma_load_2d(st + 3 * GG_TILE, &map_ha, 0, srow, bars + GB_FULL0 + s);
       }
@@ -646,16 +651,16 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_group_grads_kernel(const __g
       }
       if (ok) {
         mbar_arrive_expect_tx(bars + GB_BCFULL, 4 * GG_TILE);
-        tma_load_2d(smem, &map_b, grp * WN, row0, bars + GB_BCFULL);
-        tma_load_2d(smem + GG_TILE, &map_b, grp * WN + 64, row0, bars + GB_BCFULL);
-        tma_load_2d(smem + GG_STAGE, &map_c, grp * WN, row0, bars + GB_BCFULL);
-        tma_load_2d(smem + GG_STAGE + GG_TILE, &map_c, grp * WN + 64, row0, bars + GB_BCFULL);
+        tma_load_3d(smem, &map_b, grp * WN, row0, b, bars + GB_BCFULL);
+        tma_load_3d(smem + GG_TILE, &map_b, grp * WN + 64, row0, b, bars + GB_BCFULL);
+        tma_load_3d(smem + GG_STAGE, &map_c, grp * WN, row0, b, bars + GB_BCFULL);
+        tma_load_3d(smem + GG_STAGE + GG_TILE, &map_c, grp * WN + 64, row0, b, bars + GB_BCFULL);
         if (walk_wait(bars + GB_OUT, 0, g.status, abort)) {
           // staged outputs: gC behind the B tiles of stage 0, gB behind the C tiles of stage 1
-          tma_store_2d(&map_gc, smem + 2 * GG_TILE, grp * WN, row0);
-          tma_store_2d(&map_gc, smem + 3 * GG_TILE, grp * WN + 64, row0);
-          tma_store_2d(&map_gb, smem + GG_STAGE + 2 * GG_TILE, grp * WN, row0);
-          tma_store_2d(&map_gb, smem + GG_STAGE + 3 * GG_TILE, grp * WN + 64, row0);
+          tma_store_3d(&map_gc, smem + 2 * GG_TILE, grp * WN, row0, b);
+          tma_store_3d(&map_gc, smem + 3 * GG_TILE, grp * WN + 64, row0, b);
+          tma_store_3d(&map_gb, smem + GG_STAGE + 2 * GG_TILE, grp * WN, row0, b);
+          tma_store_3d(&map_gb, smem + GG_STAGE + 3 * GG_TILE, grp * WN + 64, row0, b);
           bulk_commit();
           bulk_wait_all<0>();
         }
@@ -721,7 +726,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_group_grads_kernel(const __g
     float acc[64];
 #pragma unroll
     for (int e = 0; e < 64; ++e) acc[e] = 0.f;
-    auto scal_ptr = [&](const float* base, int hi) { return base + (static_cast<size_t>(b) * g.H + grp * hpg + hi) * g.L + c * WQ + r; };
+    auto scal_ptr = [&](const float* base, int hi) { return base + (static_cast<size_t>(b) * g.H + grp * hpg + hi) * (static_cast<size_t>(g.nc) * WQ) + c * WQ + r; };
     float cum_n = *scal_ptr(g.cum, 0), dt_n = *scal_ptr(g.dtt, 0), colf_n = *scal_ptr(g.colf, 0);
     float cum_p = 0.f, dt_p = 0.f, colf_p = 0.f;
     if (nh > 1) { cum_p = *scal_ptr(g.cum, 1); dt_p = *scal_ptr(g.dtt, 1); colf_p = *scal_ptr(g.colf, 1); }
@@ -840,7 +845,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_group_grads_kernel(const __g
 }
 
 // dt*A prefix sums inside every 128-step chunk, dt, and the column factors of both walk directions, all in
-// [B, H, L] order.  One CTA per (b, h, chunk).  Column factor of step t relative to the far end of its 8-step
+// [B, H, nc * 128] order (steps beyond the sequence: dt = 0).  One CTA per (b, h, chunk).  Column factor of step t relative to the far end of its 8-step
 // piece: causal exp(cum[t | 7] - cum[t]) dt[t], anti-causal exp(cum[t] - cum[t & ~7]); both are at most one (dt).
 // RAW: the step sizes arrive as the projection's raw r16 output (row pitch `raw_pitch`) and the decay rates as A_log:
 //   dt = softplus(raw + bias[h]), A = -exp(A_log[h])  (the arithmetic of launch_softplus_bias / launch_neg_exp),
@@ -854,19 +859,22 @@ __global__ void __launch_bounds__(WQ) ssd_walk_cumsum_kernel(const float* __rest
   __shared__ float warp_tot[4];
   if (blockIdx.x == 0)   // the walks that follow in stream order hand states from CTA to CTA through these counters
     for (int i = threadIdx.x; i < n_flags; i += WQ) carry_flags[i] = 0;
-  const int nc = L / WQ;
+  const int nc = (L + WQ - 1) / WQ;
   const int c = blockIdx.x % nc, h = (blockIdx.x / nc) % H, b = blockIdx.x / (nc * H);
   const int t = threadIdx.x;
-  float d, a;
+  const bool inside = c * WQ + t < L;
+  const size_t row = static_cast<size_t>(b) * L + c * WQ + t;
+  float d = 0.f, a;
   if (RAW) {
-    const size_t row = static_cast<size_t>(b) * L + c * WQ + t;
-    const float pre = __half2float(raw[row * raw_pitch + h]) + bias[h];
-    d = pre > 20.f ? pre : log1pf(__expf(pre));
     a = -__expf(A[h]);
-    dt_out[row * H + h] = d;
+    if (inside) {
+      const float pre = __half2float(raw[row * raw_pitch + h]) + bias[h];
+      d = pre > 20.f ? pre : log1pf(__expf(pre));
+      dt_out[row * H + h] = d;
+    }
     if (b == 0 && c == 0 && t == 0) A_out[h] = a;
   } else {
-    d = dt[(static_cast<size_t>(b) * L + c * WQ + t) * H + h];
+    if (inside) d = dt[row * H + h];
     a = A[h];
   }
   float v = d * a;
@@ -881,7 +889,7 @@ __global__ void __launch_bounds__(WQ) ssd_walk_cumsum_kernel(const float* __rest
   for (int w = 0; w < (t >> 5); ++w) base += warp_tot[w];
   const float cv = v + base;
   const float c_hi = __shfl_sync(0xffffffffu, cv, (t & 31) | 7), c_lo = __shfl_sync(0xffffffffu, cv, (t & 31) & ~7);
-  const size_t o = (static_cast<size_t>(b) * H + h) * L + c * WQ + t;
+  const size_t o = (static_cast<size_t>(b) * H + h) * (static_cast<size_t>(nc) * WQ) + c * WQ + t;
   cum[o] = cv;
   dtt[o] = d;
   colf_c[o] = w_exp(c_hi - cv) * d;
@@ -916,6 +924,20 @@ CUtensorMap walk_map(const void* base, size_t rows, size_t cols) {
   return m;
 }
 
+// r16 tensor [batch, rows, cols] (row-major), box {64 columns, 128 rows, 1}, 128-byte swizzle: rows past the end of a batch
+// entry read as zeros and are not written.
+CUtensorMap walk_map3(const void* base, size_t batch, size_t rows, size_t cols) {
+  CUtensorMap m;
+  const cuuint64_t dims[3] = {cols, rows, batch};
+  const cuuint64_t strides[2] = {cols * sizeof(__half), rows * cols * sizeof(__half)};
+  const cuuint32_t box[3] = {64, 128, 1};
+  const cuuint32_t es[3] = {1, 1, 1};
+  MP_CU_CHECK(walk_encode_tiled()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box, es,
+                                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE));
+  return m;
+}
+
 }  // namespace
 
 // Host-side view of the chunk walk's work partition (the function the kernels use, compiled for the host): segment
@@ -932,13 +954,15 @@ extern "C" int mpSsdWalkPartition(int cta, int ncta, int nseq, int nc, int idx, 
 // ---------------------------------------------------------------------------
 // Interface to the launchers in ssd.cu.
 // ---------------------------------------------------------------------------
+// Sequences of less than 32 steps stay with the recurrence: A's gradient there is a difference of nearly equal row dots, of
+// which the walk's r16 score tile leaves too little.
 bool mp_ssd_walk_supported(int L, int H, int P, int N, int G) {
-  return P == WP && N == WN && L % WQ == 0 && L > 0 && G > 0 && H % G == 0 && getenv("MP_SSD_NO_WALK") == nullptr;
+  return P == WP && N == WN && L >= 32 && G > 0 && H % G == 0 && getenv("MP_SSD_NO_WALK") == nullptr;
 }
 
 void mp_ssd_walk_cumsum(const float* dt, const float* A, float* cum, float* dtt, float* colf_c, float* colf_a, int B, int L, int H,
                         int* carry_flags, int n_flags, cudaStream_t st) {
-  ssd_walk_cumsum_kernel<false><<<B * H * (L / WQ), WQ, 0, st>>>(dt, A, cum, dtt, colf_c, colf_a, L, H, carry_flags, n_flags, nullptr, 0, nullptr,
+  ssd_walk_cumsum_kernel<false><<<B * H * ((L + WQ - 1) / WQ), WQ, 0, st>>>(dt, A, cum, dtt, colf_c, colf_a, L, H, carry_flags, n_flags, nullptr, 0, nullptr,
                                                                  nullptr, nullptr);
   MP_LAUNCH_CHECK();
 }
@@ -946,27 +970,26 @@ void mp_ssd_walk_cumsum(const float* dt, const float* A, float* cum, float* dtt,
 // The same from the raw projection output and A_log (see the kernel); dt_out and A_out are what the reverse pass takes.
 void mp_ssd_walk_cumsum_raw(const __half* raw, size_t raw_pitch, const float* bias, const float* A_log, float* dt_out, float* A_out, float* cum,
                             float* dtt, float* colf_c, int B, int L, int H, int* carry_flags, int n_flags, cudaStream_t st) {
-  ssd_walk_cumsum_kernel<true><<<B * H * (L / WQ), WQ, 0, st>>>(nullptr, A_log, cum, dtt, colf_c, nullptr, L, H, carry_flags, n_flags, raw, raw_pitch,
+  ssd_walk_cumsum_kernel<true><<<B * H * ((L + WQ - 1) / WQ), WQ, 0, st>>>(nullptr, A_log, cum, dtt, colf_c, nullptr, L, H, carry_flags, n_flags, raw, raw_pitch,
                                                                 bias, dt_out, A_out);
   MP_LAUNCH_CHECK();
 }
 
-// One walk.  q, k: [B*L, G*128]; v, z, out: [B*L, H*64]; cum, dtt, colf (of the walk's direction): [B, H, L] from mp_ssd_walk_cumsum.
+// One walk.  q, k: [B*L, G*128]; v, z, out: [B*L, H*64]; cum, dtt, colf (of the walk's direction): [B, H, nc * 128] from mp_ssd_walk_cumsum.
 void mp_ssd_walk(int anti, const __half* q, const __half* k, const __half* v, const float* cum, const float* dtt, const float* colf, __half* out,
                  const __half* z,
                  float* dot_out, __half* hs_out, float* carry, int* carry_flag, int max_ctas, int B, int L, int H, int G, uint32_t* status,
                  cudaStream_t st) {
   WalkArgs g;
-  g.B = B; g.L = L; g.H = H; g.G = G; g.nc = L / WQ;
+  g.B = B; g.L = L; g.H = H; g.G = G; g.nc = (L + WQ - 1) / WQ;
   g.cum = cum; g.dtt = dtt; g.colf = colf; g.out = out; g.z = z; g.dot_out = dot_out; g.hs_out = hs_out; g.status = status;
   g.carry = carry; g.carry_flag = carry_flag;
   // One CTA per SM slot it may use, every CTA the same number of chunks; never more CTAs than sequences, so that a CTA's
   // range is at least one sequence long (see walk_segment).  MP_SSD_WALK_PER_SEQUENCE: one CTA per sequence, no hand-off.
   int grid = B * H;
   if (max_ctas > 0 && max_ctas < grid && getenv("MP_SSD_WALK_PER_SEQUENCE") == nullptr) grid = max_ctas;
-  const size_t rows = static_cast<size_t>(B) * L;
-  const CUtensorMap mq = walk_map(q, rows, static_cast<size_t>(G) * WN), mk = walk_map(k, rows, static_cast<size_t>(G) * WN);
-  const CUtensorMap mv = walk_map(v, rows, static_cast<size_t>(H) * WP);
+  const CUtensorMap mq = walk_map3(q, B, L, static_cast<size_t>(G) * WN), mk = walk_map3(k, B, L, static_cast<size_t>(G) * WN);
+  const CUtensorMap mv = walk_map3(v, B, L, static_cast<size_t>(H) * WP);
   const CUtensorMap mh = hs_out != nullptr ? walk_map(hs_out, static_cast<size_t>(B) * H * g.nc * WN, WP) : mv;
   auto launch = [&](auto kernel) {
     MP_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, W_SMEM_BYTES));
@@ -974,28 +997,31 @@ void mp_ssd_walk(int anti, const __half* q, const __half* k, const __half* v, co
   };
   const bool dot = z != nullptr && dot_out != nullptr;
   if (!dot) { g.z = nullptr; g.dot_out = nullptr; }
+  if (anti && !dot) MP_FATAL("ssd walk: the anti-causal form comes with its row dots");
+  const bool ragged = L % WQ != 0;
   if (anti) {
-    if (dot) launch(ssd_walk_kernel<1, true>); else launch(ssd_walk_kernel<1, false>);
+    if (ragged) launch(ssd_walk_kernel<1, true, true>); else launch(ssd_walk_kernel<1, true, false>);
+  } else if (dot) {
+    if (ragged) launch(ssd_walk_kernel<0, true, true>); else launch(ssd_walk_kernel<0, true, false>);
   } else {
-    if (dot) launch(ssd_walk_kernel<0, true>); else launch(ssd_walk_kernel<0, false>);
+    if (ragged) launch(ssd_walk_kernel<0, false, true>); else launch(ssd_walk_kernel<0, false, false>);
   }
   MP_LAUNCH_CHECK();
 }
 
 // gB, gC [B*L, G*128] from gy, x [B*L, H*64], Bm, Cm [B*L, G*128] and the states left by the two walks
-// (hs_causal, hs_anti: [B, H, L/128][128][64]).
+// (hs_causal, hs_anti: [B, H, nc][128][64]).
 void mp_ssd_group_grads(const __half* gy, const __half* x, const __half* Bm, const __half* Cm, const __half* hs_causal, const __half* hs_anti,
                         const float* cum, const float* dtt, const float* colf_c, __half* gB, __half* gC, int B, int L, int H, int G,
                         uint32_t* status, cudaStream_t st) {
   GroupArgs g;
-  g.B = B; g.L = L; g.H = H; g.G = G; g.nc = L / WQ;
+  g.B = B; g.L = L; g.H = H; g.G = G; g.nc = (L + WQ - 1) / WQ;
   g.cum = cum; g.dtt = dtt; g.colf = colf_c; g.status = status;
-  const size_t rows = static_cast<size_t>(B) * L;
   const size_t srows = static_cast<size_t>(B) * H * g.nc * WN;
-  const CUtensorMap mgy = walk_map(gy, rows, static_cast<size_t>(H) * WP), mx = walk_map(x, rows, static_cast<size_t>(H) * WP);
+  const CUtensorMap mgy = walk_map3(gy, B, L, static_cast<size_t>(H) * WP), mx = walk_map3(x, B, L, static_cast<size_t>(H) * WP);
   const CUtensorMap mhc = walk_map(hs_causal, srows, WP), mha = walk_map(hs_anti, srows, WP);
-  const CUtensorMap mb = walk_map(Bm, rows, static_cast<size_t>(G) * WN), mc = walk_map(Cm, rows, static_cast<size_t>(G) * WN);
-  const CUtensorMap mgb = walk_map(gB, rows, static_cast<size_t>(G) * WN), mgc = walk_map(gC, rows, static_cast<size_t>(G) * WN);
+  const CUtensorMap mb = walk_map3(Bm, B, L, static_cast<size_t>(G) * WN), mc = walk_map3(Cm, B, L, static_cast<size_t>(G) * WN);
+  const CUtensorMap mgb = walk_map3(gB, B, L, static_cast<size_t>(G) * WN), mgc = walk_map3(gC, B, L, static_cast<size_t>(G) * WN);
   MP_CUDA_CHECK(cudaFuncSetAttribute(ssd_group_grads_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GG_SMEM_BYTES));
   ssd_group_grads_kernel<<<B * g.nc * G, W_THREADS, GG_SMEM_BYTES, st>>>(mgy, mx, mhc, mha, mb, mc, mgb, mgc, g);
   MP_LAUNCH_CHECK();

@@ -183,3 +183,32 @@ def test_reverse_with_the_raw_side_gradients_is_the_three_launches_in_one(mp, st
     assert np.all(outs[1][5][:, H:] == 2)
     for a, b, name in zip(outs[0][6:], outs[1][6:], ("gdt_bias", "gA_log")):
         assert_close(b, a.astype(np.float64), 1e-5, name)
+
+
+@pytest.mark.parametrize("dims", [
+    # (batch, seqlen, heads, headdim, dstate, groups, chunk): the chunk walk on lengths that are no multiple of its 128-step
+    # chunk - the shortest, less than one chunk, one step past a chunk, one step short of one, and sequences cut between CTAs
+    (2, 32, 2, 64, 128, 1, 128), (1, 50, 4, 64, 128, 2, 64), (2, 129, 2, 64, 128, 1, 128), (1, 383, 4, 64, 128, 1, 256),
+    (10, 333, 16, 64, 128, 1, 128)])
+def test_ssd_on_ragged_lengths(mp, stream, orc, dims):
+    import torch
+    nb, L, H, P, N, G, Q = dims
+    x, dt, A, Bm, Cm, gy = make_inputs(9, nb, L, H, P, N, G)
+    f64 = lambda a: np.ascontiguousarray(a.astype(np.float64))
+    args = [dev(a) for a in (x, dt, A, Bm, Cm)]
+    # outputs carry guard rows: nothing may be written behind the last step of the last batch entry
+    guarded = lambda a: dev(np.full((a.size + 4096,), np.nan, a.dtype))
+    y, gx, gdt, gB, gC = (guarded(a) for a in (x, x, dt, Bm, Cm))
+    gA = dev(np.full(A.shape, np.nan, np.float32))
+    n = max(mp.lib().mpSsdScanScratchBytes(*dims, 0), mp.lib().mpSsdScanScratchBytes(*dims, 1))
+    scratch = torch.full((n,), 255, dtype=torch.uint8, device="cuda")
+    torch.cuda.current_stream().synchronize()
+    mp.launch("ssd_scan", torch.float16, *args, y, scratch, *dims, stream)
+    mp.launch("ssd_scan_reverse", torch.float16, *args, dev(gy), gx, gdt, gA, gB, gC, scratch, *dims, stream)
+    stream.sync()
+    assert stream.status() == 0
+    ref = (orc.ssd_forward(f64(x), f64(dt), f64(A), f64(Bm), f64(Cm)),) + tuple(orc.ssd_reverse(f64(x), f64(dt), f64(A), f64(Bm), f64(Cm), f64(gy)))
+    for got, want, name in zip((y, gx, gdt, gA, gB, gC), ref, ("y", "gx", "gdt", "gA", "gB", "gC")):
+        got = host(got)
+        assert np.isnan(got[want.size:]).all(), f"{name} written past its end {dims}"
+        assert_close(got[:want.size].reshape(want.shape), want.astype(got.dtype), TOL, f"{name} {dims}")
