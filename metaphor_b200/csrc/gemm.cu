@@ -15,13 +15,11 @@
 // SM walking the output tiles) with two TMEM accumulators, so one tile's
 // epilogue overlaps the next tile's main loop.  Transposed operands need no scratch
 // copy: the shared-memory descriptor and the instruction descriptor carry the
-// operand's major-ness.  r32 uses kind::tf32 on an error-compensated split
-// (hi + lo, three MMAs) unless MP_GEMM_TF32X1 is set; r64 and shapes TMA cannot
-// address (row pitch not a multiple of 16 bytes) use an FP-pipe tile kernel.
-#include "mp_tcgen05.cuh"
-
-#include <cuda.h>
-#include <mutex>
+// operand's major-ness.  r32 has a kernel of its own (gemm_r32.cu: three tf32 MMAs per
+// product on an error-compensated split).  Operands TMA cannot address
+// (row pitch not a multiple of 16 bytes) are copied into aligned rows first; r64 and
+// the smallest of those problems use an FP-pipe tile kernel.
+#include "mp_gemm.cuh"
 
 namespace {
 
@@ -94,52 +92,20 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const T* __restrict__ a,
 // ---------------------------------------------------------------------------
 // tcgen05 kernel.
 // ---------------------------------------------------------------------------
-constexpr int BM = 128;               // UMMA M (one TMEM lane per output row)
-constexpr int SWIZZLE_BYTES = 128;    // one operand row / k-row in shared memory
 constexpr int GEMM_THREADS = 320;     // warp 0: TMA, warp 1: MMA + TMEM, warps 2-9: epilogue
-constexpr int GEMM_MAX_THREADS = 448; // + warps 10-13: operand split (r32)
 constexpr int EPI_THREADS = 256;      // two epilogue warps per TMEM lane quarter, each takes half of the columns
 constexpr int MAX_STAGES = 8;
 
-// Staging blocks per epilogue warp.  r16: one per 32-column block of the warp's half tile (4 at BN = 256), so
-// a tile's TMA stores are issued back to back and the staging is only waited for at the next tile.
-template <typename T> struct EpiBufs { static constexpr int value = sizeof(T) == 2 ? 4 : 1; };
+// 32-column staging blocks per epilogue warp: one per block of the warp's half tile (4 at BN = 256), so a tile's TMA stores are
+// issued back to back and the staging is only waited for at the next tile.
+constexpr int EPI_BUFS = 4;
 
-template <typename T> struct GemmT;
-template <> struct GemmT<__half> {
+struct GemmT {
   static constexpr int BK = 64;       // elements per 128-byte row
   static constexpr int UMMA_K = 16;
-  static constexpr bool TF32 = false;
-  static constexpr uint32_t FMT = UMMA_FMT_F16;
-};
-template <> struct GemmT<float> {
-  static constexpr int BK = 32;
-  static constexpr int UMMA_K = 8;
-  static constexpr bool TF32 = true;
-  static constexpr uint32_t FMT = UMMA_FMT_TF32;
 };
 
-struct GemmArgs {
-  const void* bias;   // N values of T (bias_pitch = 0), a full [M, N] matrix (bias_pitch = N), or nullptr
-  size_t bias_pitch = 0;
-  void* c;            // [M, N] row-major
-  float alpha, beta;
-  int M, N, K;
-  int a_mn, b_mn;     // operand major-ness: 0 = K contiguous, 1 = M resp. N contiguous
-  int stages;
-  int epi_boxes = 2;  // pair kernel: 64-column staging boxes per epilogue warp
-  int split;          // r32 only: 1 = error-compensated hi/lo split (3 MMAs per k-slice)
-  int ksplit;         // > 1: the K range of every tile is cut into ksplit work units whose raw fp32
-  float* partial;     //      accumulators go to partial[unit_split][M][N]; a fold kernel finishes C
-  int batch;          // > 1: densely packed [batch, M, K] x [batch, K, N] -> [batch, M, N] over 3-D tensor maps (ksplit = 1)
-  uint32_t* status;
-};
-
-// Shared memory of one stage: A tile (BM x 128 B), B tile (BN x 128 B), and for
-// the split mode the "lo" copies of both.
-template <int BN> constexpr int stage_bytes(bool split) {
-  return (BM * SWIZZLE_BYTES + BN * SWIZZLE_BYTES) * (split ? 2 : 1);
-}
+template <int BN> constexpr int stage_bytes() { return BM * SWIZZLE_BYTES + BN * SWIZZLE_BYTES; }
 
 // Persistent kernel: grid = min(tiles, SMs); every CTA walks output tiles
 // t = blockIdx.x, blockIdx.x + gridDim.x, ... (consecutive tiles share the B
@@ -150,30 +116,32 @@ template <int BN> constexpr int stage_bytes(bool split) {
 //   warp 1      MMA issuer (one elected thread), owns the TMEM allocation
 //   warps 2-9   epilogue: warp w reads TMEM lane quarter w % 4 and one half of the tile's columns;
 //               32x32 blocks go registers -> shared staging -> TMA store (coalesced, edge-clipped)
-//   warps 10-13 r32 split mode only: write the hi / lo operand tiles
-template <typename T, int BN>
-__global__ void __launch_bounds__(GEMM_MAX_THREADS, 1) gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
-                                                                          const __grid_constant__ CUtensorMap tmap_b,
-                                                                          const __grid_constant__ CUtensorMap tmap_c,
-                                                                          const GemmArgs g) {
-  using G = GemmT<T>;
+//
+// EXACT: the tensor core's fp32 accumulation truncates, which drifts by up to 2^-24 of the sum per MMA.  Problems that were
+// summed on the FP pipe before (padded operands) keep its exactness where they are small enough for the single-CTA kernel: the
+// accumulator is handed over every CHUNK_KB k-blocks (8 MMAs) and added up in the epilogue warps' registers with rounding.
+constexpr int CHUNK_KB = 2;
+template <int BN, bool EXACT>
+__global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
+                                                                      const __grid_constant__ CUtensorMap tmap_b,
+                                                                      const __grid_constant__ CUtensorMap tmap_c, const GemmArgs g) {
+  using T = __half;
+  using G = GemmT;
   constexpr int BK = G::BK;
   constexpr int A_BYTES = BM * SWIZZLE_BYTES, B_BYTES = BN * SWIZZLE_BYTES;
   constexpr int KSLICES = BK / G::UMMA_K;  // 4
   constexpr int ACC_BUFS = 2;
   constexpr int EPI_TILE_BYTES = 32 * 32 * sizeof(T);   // one 32 x 32 staging block for the TMA store
-  constexpr int EPI_BUFS = EpiBufs<T>::value;           // staging blocks per warp: no wait between the blocks of a tile
-  // r16, BN >= 128: two 32-column blocks share one [32 rows][64 columns] staging box in the 128-byte swizzle,
+  // BN >= 128: two 32-column blocks share one [32 rows][64 columns] staging box in the 128-byte swizzle,
   // written out by one TMA store with full 128-byte rows (64-byte rows halve the store engine's throughput)
-  constexpr bool WIDE_STORE = sizeof(T) == 2 && BN >= 128;
+  constexpr bool WIDE_STORE = BN >= 128;
   extern __shared__ unsigned char gemm_smem_raw[];
   // 1024-byte alignment: swizzle atoms are 8 rows x 128 bytes
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(gemm_smem_raw) + 1023) & ~uintptr_t(1023));
   const int stages = g.stages;
-  const int stage_sz = (A_BYTES + B_BYTES) * (g.split ? 2 : 1);
+  constexpr int stage_sz = A_BYTES + B_BYTES;
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + static_cast<size_t>(stages) * stage_sz);
-  uint64_t* ready = full + MAX_STAGES;      // split mode: hi / lo tiles written
-  uint64_t* empty = ready + MAX_STAGES;
+  uint64_t* empty = full + MAX_STAGES;
   uint64_t* acc_full = empty + MAX_STAGES;  // [2] accumulator complete
   uint64_t* acc_empty = acc_full + ACC_BUFS;  // [2] accumulator drained by the epilogue
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + ACC_BUFS);
@@ -193,7 +161,6 @@ __global__ void __launch_bounds__(GEMM_MAX_THREADS, 1) gemm_tcgen05_kernel(const
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
       mbar_init(full + s, 1);
-      mbar_init(ready + s, 128);
       mbar_init(empty + s, 1);
     }
     for (int a = 0; a < ACC_BUFS; ++a) { mbar_init(acc_full + a, 1); mbar_init(acc_empty + a, EPI_THREADS); }
@@ -260,85 +227,44 @@ __global__ void __launch_bounds__(GEMM_MAX_THREADS, 1) gemm_tcgen05_kernel(const
       }
     }
   } else if (warp == 1) {
-    // ------------------------------ MMA issuer --------------------------------
-    if (lane == 0) {
-      const uint32_t idesc = umma_instr_desc(G::FMT, g.a_mn, g.b_mn, BM, BN);
-      // K-major: rows of 128 B, 8-row groups 1024 B apart, k-slice = +32 B.
-      // MN-major: k-rows of 128 B, 64/32-column blocks BK*128 B apart, k-slice = +UMMA_K*128 B.
-      const uint32_t a_lbo = g.a_mn ? BK * SWIZZLE_BYTES : 16, b_lbo = g.b_mn ? BK * SWIZZLE_BYTES : 16;
-      const uint32_t a_kstep = g.a_mn ? G::UMMA_K * SWIZZLE_BYTES : 32, b_kstep = g.b_mn ? G::UMMA_K * SWIZZLE_BYTES : 32;
-      // 32-bit MN-major tiles use the 32-byte-atom swizzle (groups of 4 k-rows, 512 B)
-      const uint32_t a_lay = (G::TF32 && g.a_mn) ? UMMA_LAYOUT_SW128_BASE32B : UMMA_LAYOUT_SW128;
-      const uint32_t b_lay = (G::TF32 && g.b_mn) ? UMMA_LAYOUT_SW128_BASE32B : UMMA_LAYOUT_SW128;
-      const uint32_t a_sbo = (G::TF32 && g.a_mn) ? 512 : 1024, b_sbo = (G::TF32 && g.b_mn) ? 512 : 1024;
-      int s = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      int local = 0;
-      for (int unit = blockIdx.x; unit < num_units && ok; unit += gridDim.x, ++local) {
-        const int buf = local & 1;
-        const uint32_t use = static_cast<uint32_t>(local >> 1);
-        // the epilogue must have drained this accumulator (passes at once on its first use)
-        if (!mbar_wait_abortable(acc_empty + buf, (use & 1u) ^ 1u, g.status, abort)) { ok = false; break; }
-        tcgen05_fence_after_sync();
-        const uint32_t tmem_acc = tmem_base + buf * BN;
-        const int sp = batched ? 0 : unit / num_tiles;
-        const int kb0 = sp * kb_per, kb1 = min(num_kb, kb0 + kb_per);
-        for (int kb = kb0; kb < kb1; ++kb) {
-          uint64_t* wait_on = g.split ? (ready + s) : (full + s);
-          if (!mbar_wait_abortable(wait_on, phase, g.status, abort)) { ok = false; break; }
-          tcgen05_fence_after_sync();
-          const uint32_t sa = mp_smem_u32(smem + static_cast<size_t>(s) * stage_sz);
-          const uint32_t sb = sa + A_BYTES;
-          const uint32_t sa_lo = sb + B_BYTES, sb_lo = sa_lo + A_BYTES;
-#pragma unroll
-          for (int ks = 0; ks < KSLICES; ++ks) {
-            const uint64_t ad = umma_smem_desc(sa + ks * a_kstep, a_lbo, a_sbo, a_lay);
-            const uint64_t bd = umma_smem_desc(sb + ks * b_kstep, b_lbo, b_sbo, b_lay);
-            umma<G::TF32>(tmem_acc, ad, bd, idesc, (kb != kb0 || ks != 0) ? 1u : 0u);
-            if (g.split) {
-              const uint64_t adl = umma_smem_desc(sa_lo + ks * a_kstep, a_lbo, a_sbo, a_lay);
-              const uint64_t bdl = umma_smem_desc(sb_lo + ks * b_kstep, b_lbo, b_sbo, b_lay);
-              umma<G::TF32>(tmem_acc, ad, bdl, idesc, 1u);   // hi * lo
-              umma<G::TF32>(tmem_acc, adl, bd, idesc, 1u);   // lo * hi
-            }
-          }
-          umma_commit(empty + s);  // the stage may be refilled once these MMAs have read it
-          if (++s == stages) { s = 0; phase ^= 1u; }
-        }
-        if (ok) umma_commit(acc_full + buf);
-      }
-    }
-  } else if (warp >= 10) {
-    // ---------------- r32 split mode: hi / lo operand tiles --------------------
-    // hi = x with the 13 low mantissa bits cleared (exactly representable in
-    // tf32, so the tensor core's own fp32 -> tf32 conversion cannot change it),
-    // lo = x - hi (exact in fp32; its tf32 conversion error is ~2^-21 |x|).
-    const int et = threadIdx.x - 320;  // 0..127
+    // ------------------------------ MMA issuer (the warp as a whole, see elect_one) ----
+    const uint32_t idesc = umma_instr_desc(UMMA_FMT_F16, g.a_mn, g.b_mn, BM, BN);
+    // K-major: rows of 128 B, 8-row groups 1024 B apart, k-slice = +32 B.
+    // MN-major: k-rows of 128 B, 64-column blocks BK*128 B apart, k-slice = +UMMA_K*128 B.
+    const uint32_t a_lbo = g.a_mn ? BK * SWIZZLE_BYTES : 16, b_lbo = g.b_mn ? BK * SWIZZLE_BYTES : 16;
+    const uint32_t a_kunits = (g.a_mn ? G::UMMA_K * SWIZZLE_BYTES : 32) >> 4, b_kunits = (g.b_mn ? G::UMMA_K * SWIZZLE_BYTES : 32) >> 4;
+    // descriptors of stage 0, k-slice 0; the others differ in the address field (16-byte units)
+    const uint64_t ad0 = umma_smem_desc(mp_smem_u32(smem), a_lbo, 1024), bd0 = umma_smem_desc(mp_smem_u32(smem) + A_BYTES, b_lbo, 1024);
     int s = 0;
-    uint32_t phase = 0;
+    uint32_t phase = 0, chunk = 0;
     bool ok = true;
     for (int unit = blockIdx.x; unit < num_units && ok; unit += gridDim.x) {
       const int sp = batched ? 0 : unit / num_tiles;
       const int kb0 = sp * kb_per, kb1 = min(num_kb, kb0 + kb_per);
-      for (int kb = kb0; kb < kb1; ++kb) {
-        if (!mbar_wait_abortable(full + s, phase, g.status, abort)) { ok = false; break; }
-        unsigned char* hi = smem + static_cast<size_t>(s) * stage_sz;
-        unsigned char* lo = hi + A_BYTES + B_BYTES;
-        for (int off = et * 16; off < A_BYTES + B_BYTES; off += 128 * 16) {
-          const uint4 v = *reinterpret_cast<const uint4*>(hi + off);
-          uint4 h, r;
-          h.x = v.x & 0xFFFFE000u; h.y = v.y & 0xFFFFE000u; h.z = v.z & 0xFFFFE000u; h.w = v.w & 0xFFFFE000u;
-          r.x = __float_as_uint(__uint_as_float(v.x) - __uint_as_float(h.x));
-          r.y = __float_as_uint(__uint_as_float(v.y) - __uint_as_float(h.y));
-          r.z = __float_as_uint(__uint_as_float(v.z) - __uint_as_float(h.z));
-          r.w = __float_as_uint(__uint_as_float(v.w) - __uint_as_float(h.w));
-          *reinterpret_cast<uint4*>(hi + off) = h;
-          *reinterpret_cast<uint4*>(lo + off) = r;
+      for (int kc = kb0; kc < kb1 && ok; ++chunk) {
+        const int kend = EXACT ? min(kb1, kc + CHUNK_KB) : kb1;
+        const uint32_t buf = chunk & 1u;
+        // the epilogue must have drained this accumulator (passes at once on its first use)
+        ok = mbar_wait_abortable(acc_empty + buf, ((chunk >> 1) & 1u) ^ 1u, g.status, abort);
+        ok = __all_sync(0xffffffffu, ok);
+        const uint32_t tmem_acc = tmem_base + buf * BN;
+        for (int kb = kc; ok && kb < kend; ++kb) {
+          ok = mbar_wait_abortable(full + s, phase, g.status, abort);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          tcgen05_fence_after_sync();
+          const uint64_t ad = ad0 + static_cast<uint32_t>(s * (stage_sz >> 4)), bd = bd0 + static_cast<uint32_t>(s * (stage_sz >> 4));
+          const uint32_t first = kb != kc ? 1u : 0u;
+          if (elect_one()) {
+#pragma unroll
+            for (int ks = 0; ks < KSLICES; ++ks) umma<false>(tmem_acc, ad + ks * a_kunits, bd + ks * b_kunits, idesc, ks != 0 ? 1u : first);
+            umma_commit(empty + s);  // the stage may be refilled once these MMAs have read it
+            if (kb + 1 == kend) umma_commit(acc_full + buf);
+          }
+          __syncwarp();
+          if (++s == stages) { s = 0; phase ^= 1u; }
         }
-        fence_proxy_async_smem();  // generic-proxy writes -> visible to the tensor core's reads
-        mbar_arrive(ready + s);
-        if (++s == stages) { s = 0; phase ^= 1u; }
+        kc = kend;
       }
     }
   } else {
@@ -346,36 +272,71 @@ __global__ void __launch_bounds__(GEMM_MAX_THREADS, 1) gemm_tcgen05_kernel(const
     const int quarter = warp & 3;                 // TMEM lanes this warp may read
     const int half = (warp - 2) >> 2;             // which half of the tile's columns
     const T* bias = static_cast<const T*>(g.bias);
-    const bool vec_ok = (static_cast<size_t>(g.N) * sizeof(T)) % 16 == 0 && mp_aligned16(g.c);
+    const bool vec_ok = (g.ldc * sizeof(T)) % 16 == 0 && mp_aligned16(g.c);
     const bool use_tma = vec_ok && g.beta == 0.0f && g.ksplit == 1;   // overwrite: stage 32x32 blocks and let TMA write them
     unsigned char* stage_base = epi_stage + (warp - 2) * (EPI_BUFS * EPI_TILE_BYTES);
-    int local = 0;
-    for (int unit = blockIdx.x; unit < num_units; unit += gridDim.x, ++local) {
+    constexpr int BLOCKS = BN / 64;   // 32-column blocks of a warp's half tile
+    const uint32_t tmem_lane = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * (BN / 2);
+    uint32_t chunk = 0;
+    bool ok = true;
+    // hands an accumulator back to the MMA warp
+    auto release = [&]() {
+      tcgen05_fence_before_sync();
+      mbar_arrive(acc_empty + (chunk & 1u));
+      ++chunk;
+    };
+    auto acquire = [&]() {   // tcgen05.ld is warp-collective
+      const bool ready = mbar_wait_abortable(acc_full + (chunk & 1u), (chunk >> 1) & 1u, g.status, abort);
+      ok = __all_sync(0xffffffffu, ready) != 0;
+      tcgen05_fence_after_sync();
+      return ok;
+    };
+    for (int unit = blockIdx.x; unit < num_units; unit += gridDim.x) {
       const int bz = batched ? unit / num_tiles : 0;
       const int tile = batched ? unit - bz * num_tiles : unit % num_tiles, sp = batched ? 0 : unit / num_tiles;
-      const int buf = local & 1;
-      const uint32_t use = static_cast<uint32_t>(local >> 1);
       const int m0 = (tile % tiles_m) * BM, n0 = (tile / tiles_m) * BN;
-      const bool acc_ready = mbar_wait_abortable(acc_full + buf, use & 1u, g.status, abort);
-      __syncwarp();  // tcgen05.ld is warp-collective
-      if (!acc_ready) break;
-      tcgen05_fence_after_sync();
-      const uint32_t tmem_acc = tmem_base + buf * BN;
+      float sum[EXACT ? BLOCKS : 1][32];
+      if constexpr (EXACT) {
+#pragma unroll
+        for (int q = 0; q < BLOCKS; ++q)
+#pragma unroll
+          for (int j = 0; j < 32; ++j) sum[q][j] = 0.f;
+        const int kb0 = sp * kb_per, kb1 = min(num_kb, kb0 + kb_per);
+        for (int kc = kb0; kc < kb1 && acquire(); kc += CHUNK_KB) {
+#pragma unroll
+          for (int q = 0; q < BLOCKS; ++q) {
+            uint32_t v[32];
+            tmem_ld_32x32(tmem_lane + (chunk & 1u) * BN + q * 32, v);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 32; ++j) sum[q][j] += __uint_as_float(v[j]);
+          }
+          release();
+        }
+      } else {
+        acquire();
+      }
+      if (!ok) break;
+      const uint32_t tmem_acc = tmem_lane + (chunk & 1u) * BN;
       const int row = m0 + quarter * 32 + lane;
-      T* crow = static_cast<T*>(g.c) + (static_cast<size_t>(bz) * g.M + row) * g.N;
-      int blk = 0;
-#pragma unroll 1
-      for (int c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += 32, ++blk) {
-        const int col0 = n0 + c0;
+      T* crow = static_cast<T*>(g.c) + (static_cast<size_t>(bz) * g.M + row) * g.ldc;
+#pragma unroll(EXACT ? BLOCKS : 1)
+      for (int blk = 0; blk < BLOCKS; ++blk) {
+        const int col0 = n0 + half * (BN / 2) + blk * 32;
         if (col0 >= g.N) break;   // uniform across the warp
         unsigned char* stage = stage_base + (blk % EPI_BUFS) * EPI_TILE_BYTES;
         uint32_t v[32];
-        tmem_ld_32x32(tmem_acc + (static_cast<uint32_t>(quarter * 32) << 16) + c0, v);
-        tmem_ld_wait();
+        if constexpr (EXACT) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(sum[blk][j]);
+        } else {
+          tmem_ld_32x32(tmem_acc + blk * 32, v);
+          tmem_ld_wait();
+        }
         if (g.ksplit > 1) {   // raw partial sums; alpha, bias and beta are applied by the fold
           if (row < g.M) {
-            float* prow = g.partial + (static_cast<size_t>(sp) * g.M + row) * g.N + col0;
-            if ((g.N & 3) == 0 && col0 + 32 <= g.N) {
+            float* prow = g.partial + (static_cast<size_t>(sp) * g.M + row) * g.partial_ld + col0;
+            if (col0 + 32 <= g.N) {
 #pragma unroll
               for (int p = 0; p < 8; ++p) *reinterpret_cast<uint4*>(prow + p * 4) = make_uint4(v[p * 4], v[p * 4 + 1], v[p * 4 + 2], v[p * 4 + 3]);
             } else {
@@ -389,7 +350,8 @@ __global__ void __launch_bounds__(GEMM_MAX_THREADS, 1) gemm_tcgen05_kernel(const
         float r[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) r[j] = g.alpha * __uint_as_float(v[j]);
-        if (bias != nullptr && (g.bias_pitch == 0 || row < g.M)) {
+        const bool by_rows = !use_tma && !(vec_ok && col0 + 32 <= g.N);   // store_block_rows; it adds a matrix term itself
+        if (bias != nullptr && (g.bias_pitch == 0 || (row < g.M && !by_rows))) {
           const T* brow = bias + static_cast<size_t>(row) * g.bias_pitch;
 #pragma unroll
           for (int j = 0; j < 32; ++j)
@@ -419,16 +381,12 @@ __global__ void __launch_bounds__(GEMM_MAX_THREADS, 1) gemm_tcgen05_kernel(const
             continue;
           }
           // the store that last used this staging block has finished reading it
-          if (lane == 0) { if (EPI_BUFS == 1 || blk < EPI_BUFS) { if (EPI_BUFS == 1 || blk == 0) bulk_wait_read<0>(); } else bulk_wait_read<EPI_BUFS - 1>(); }
+          if (lane == 0) { if (blk < EPI_BUFS) { if (blk == 0) bulk_wait_read<0>(); } else bulk_wait_read<EPI_BUFS - 1>(); }
           __syncwarp();
-          // r32: 128-byte rows in the 128-byte swizzle (conflict-free); r16 at BN = 64: linear 64-byte rows.
-          // Register indices stay compile-time constants (a lane-dependent slot order would push r[] to local memory).
+          // BN = 64: linear 64-byte rows
           unsigned char* srow = stage + lane * (32 * sizeof(T));
 #pragma unroll
-          for (int p = 0; p < 32 / PN; ++p) {
-            const int slot = sizeof(T) == 4 ? (p ^ (lane & 7)) : p;
-            *reinterpret_cast<Pack<T>*>(srow + slot * 16) = pack<T>(r + p * PN);
-          }
+          for (int p = 0; p < 32 / PN; ++p) *reinterpret_cast<Pack<T>*>(srow + p * 16) = pack<T>(r + p * PN);
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
@@ -436,35 +394,28 @@ __global__ void __launch_bounds__(GEMM_MAX_THREADS, 1) gemm_tcgen05_kernel(const
             else tma_store_2d(&tmap_c, stage, col0, m0 + quarter * 32);
             bulk_commit();
           }
+        } else if (by_rows) {
+          const int row0 = m0 + quarter * 32;
+          store_block_rows<T>(reinterpret_cast<float*>(stage_base), r, lane, crow - static_cast<size_t>(lane) * g.ldc + col0, g.ldc,
+                              min(32, g.M - row0), col0 + lane < g.N,
+                              bias != nullptr && g.bias_pitch != 0 ? bias + static_cast<size_t>(row0) * g.bias_pitch + col0 : nullptr, g.bias_pitch,
+                              g.beta);
         } else if (row < g.M) {
-          if (vec_ok && col0 + 32 <= g.N) {
-            constexpr int PN = Pack<T>::N;
-            if (g.beta != 0.0f) {
+          constexpr int PN = Pack<T>::N;
+          if (g.beta != 0.0f) {
 #pragma unroll
-              for (int p = 0; p < 32 / PN; ++p) {
-                float old[PN];
-                unpack<T>(ld_pack(crow + col0, p), old);
+            for (int p = 0; p < 32 / PN; ++p) {
+              float old[PN];
+              unpack<T>(ld_pack(crow + col0, p), old);
 #pragma unroll
-                for (int e = 0; e < PN; ++e) r[p * PN + e] += g.beta * old[e];
-              }
-            }
-#pragma unroll
-            for (int p = 0; p < 32 / PN; ++p) st_pack(crow + col0, p, pack<T>(r + p * PN));
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              if (col0 + j < g.N) {
-                float o = r[j];
-                if (g.beta != 0.0f) o += g.beta * mp_up(crow[col0 + j]);
-                crow[col0 + j] = mp_down<T>(o);
-              }
+              for (int e = 0; e < PN; ++e) r[p * PN + e] += g.beta * old[e];
             }
           }
+#pragma unroll
+          for (int p = 0; p < 32 / PN; ++p) st_pack(crow + col0, p, pack<T>(r + p * PN));
         }
       }
-      // hand the accumulator back to the MMA warp
-      tcgen05_fence_before_sync();
-      mbar_arrive(acc_empty + buf);
+      if constexpr (!EXACT) release();
     }
     if (use_tma && lane == 0) bulk_wait_all<0>();   // all of this warp's stores have completed
   }
@@ -493,7 +444,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
     gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                              const __grid_constant__ CUtensorMap tmap_c, const GemmArgs g) {
   using T = __half;
-  using G = GemmT<T>;
+  using G = GemmT;
   constexpr int BK = G::BK, BN = PAIR_BN;
   constexpr int A_BYTES = BM * SWIZZLE_BYTES, B_BYTES = (BN / 2) * SWIZZLE_BYTES;
   constexpr int KSLICES = BK / G::UMMA_K;
@@ -572,10 +523,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (rank 0) -------------------------
-    if (lane == 0 && rank == 0) {
-      const uint32_t idesc = umma_instr_desc(G::FMT, g.a_mn, g.b_mn, 2 * BM, BN);
+    if (rank == 0) {   // the warp as a whole, see elect_one
+      const uint32_t idesc = umma_instr_desc(UMMA_FMT_F16, g.a_mn, g.b_mn, 2 * BM, BN);
       const uint32_t a_lbo = g.a_mn ? BK * SWIZZLE_BYTES : 16, b_lbo = g.b_mn ? BK * SWIZZLE_BYTES : 16;
-      const uint32_t a_kstep = g.a_mn ? G::UMMA_K * SWIZZLE_BYTES : 32, b_kstep = g.b_mn ? G::UMMA_K * SWIZZLE_BYTES : 32;
+      const uint32_t a_kunits = (g.a_mn ? G::UMMA_K * SWIZZLE_BYTES : 32) >> 4, b_kunits = (g.b_mn ? G::UMMA_K * SWIZZLE_BYTES : 32) >> 4;
+      const uint64_t ad0 = umma_smem_desc(mp_smem_u32(smem), a_lbo, 1024), bd0 = umma_smem_desc(mp_smem_u32(smem) + A_BYTES, b_lbo, 1024);
       int s = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -583,26 +535,27 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
       for (int unit = pair; unit < num_units && ok; unit += num_pairs, ++local) {
         const int buf = local & 1;
         const uint32_t use = static_cast<uint32_t>(local >> 1);
-        if (!mbar_wait_abortable(acc_empty + buf, (use & 1u) ^ 1u, g.status, abort)) { ok = false; break; }
-        tcgen05_fence_after_sync();
+        ok = mbar_wait_abortable(acc_empty + buf, (use & 1u) ^ 1u, g.status, abort);
+        ok = __all_sync(0xffffffffu, ok);
         const uint32_t tmem_acc = tmem_base + buf * BN;
         const int sp = unit / num_tiles;
         const int kb0 = sp * kb_per, kb1 = min(num_kb, kb0 + kb_per);
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait_abortable(full + s, phase, g.status, abort)) { ok = false; break; }
+        for (int kb = kb0; ok && kb < kb1; ++kb) {
+          ok = mbar_wait_abortable(full + s, phase, g.status, abort);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
           tcgen05_fence_after_sync();
-          const uint32_t sa = mp_smem_u32(smem + static_cast<size_t>(s) * PAIR_STAGE_BYTES);
-          const uint32_t sb = sa + A_BYTES;
+          const uint64_t ad = ad0 + static_cast<uint32_t>(s * (PAIR_STAGE_BYTES >> 4)), bd = bd0 + static_cast<uint32_t>(s * (PAIR_STAGE_BYTES >> 4));
+          const uint32_t first = kb != kb0 ? 1u : 0u;
+          if (elect_one()) {
 #pragma unroll
-          for (int ks = 0; ks < KSLICES; ++ks) {
-            const uint64_t ad = umma_smem_desc(sa + ks * a_kstep, a_lbo, 1024);
-            const uint64_t bd = umma_smem_desc(sb + ks * b_kstep, b_lbo, 1024);
-            umma_pair_f16(tmem_acc, ad, bd, idesc, (kb != kb0 || ks != 0) ? 1u : 0u);
+            for (int ks = 0; ks < KSLICES; ++ks) umma_pair_f16(tmem_acc, ad + ks * a_kunits, bd + ks * b_kunits, idesc, ks != 0 ? 1u : first);
+            umma_commit_pair_to(empty + s, 3);   // the stage is free in both CTAs
+            if (kb + 1 == kb1) umma_commit_pair_to(acc_full + buf, 3);
           }
-          umma_commit_pair_to(empty + s, 3);   // the stage is free in both CTAs
+          __syncwarp();
           if (++s == stages) { s = 0; phase ^= 1u; }
         }
-        if (ok) umma_commit_pair_to(acc_full + buf, 3);
       }
     }
   } else {
@@ -610,7 +563,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
     const int quarter = warp & 3;
     const int half = (warp - 2) >> 2;
     const T* bias = static_cast<const T*>(g.bias);
-    const bool vec_ok = (static_cast<size_t>(g.N) * sizeof(T)) % 16 == 0 && mp_aligned16(g.c);
+    const bool vec_ok = (g.ldc * sizeof(T)) % 16 == 0 && mp_aligned16(g.c);
     const bool use_tma = vec_ok && g.beta == 0.0f && g.ksplit == 1;
     unsigned char* stage_base = epi_stage + (warp - 2) * (epi_boxes * BOX_BYTES);
     int local = 0;
@@ -625,7 +578,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
       tcgen05_fence_after_sync();
       const uint32_t tmem_acc = tmem_base + buf * BN;
       const int row = m0 + quarter * 32 + lane;
-      T* crow = static_cast<T*>(g.c) + static_cast<size_t>(row) * g.N;
+      T* crow = static_cast<T*>(g.c) + static_cast<size_t>(row) * g.ldc;
       // one staging box (64 columns) per iteration: both TMEM loads are in flight before the wait
       int boxi = 0;
 #pragma unroll 1
@@ -641,8 +594,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 #pragma unroll
             for (int hb = 0; hb < 2; ++hb) {
               const int colb = col0 + 32 * hb;
-              float* prow = g.partial + (static_cast<size_t>(sp) * g.M + row) * g.N + colb;
-              if ((g.N & 3) == 0 && colb + 32 <= g.N) {
+              float* prow = g.partial + (static_cast<size_t>(sp) * g.M + row) * g.partial_ld + colb;
+              if (colb + 32 <= g.N) {
 #pragma unroll
                 for (int p = 0; p < 8; ++p)
                   *reinterpret_cast<uint4*>(prow + p * 4) = make_uint4(v[hb][p * 4], v[hb][p * 4 + 1], v[hb][p * 4 + 2], v[hb][p * 4 + 3]);
@@ -668,7 +621,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
           float r[32];
 #pragma unroll
           for (int j = 0; j < 32; ++j) r[j] = g.alpha * __uint_as_float(v[hb][j]);
-          if (bias != nullptr && (g.bias_pitch == 0 || row < g.M)) {
+          const bool by_rows = !use_tma && !(vec_ok && colb + 32 <= g.N);
+          if (bias != nullptr && (g.bias_pitch == 0 || (row < g.M && !by_rows))) {
             const T* brow = bias + static_cast<size_t>(row) * g.bias_pitch;
             if (g.bias_pitch != 0 && colb + 32 <= g.N && (g.bias_pitch * sizeof(T)) % 16 == 0 && mp_aligned16(bias)) {
               // a full-matrix term (a residual): the lane's 32 values are one contiguous 64-byte piece of its row
@@ -689,29 +643,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 #pragma unroll
             for (int p = 0; p < 4; ++p)
               *reinterpret_cast<Pack<T>*>(box + lane * 128 + (((4 * hb + p) ^ (lane & 7)) << 4)) = pack<T>(r + p * PN);
+          } else if (by_rows) {
+            const int row0 = m0 + quarter * 32;
+            store_block_rows<T>(reinterpret_cast<float*>(stage_base), r, lane, crow - static_cast<size_t>(lane) * g.ldc + colb, g.ldc,
+                                min(32, g.M - row0), colb + lane < g.N,
+                                bias != nullptr && g.bias_pitch != 0 ? bias + static_cast<size_t>(row0) * g.bias_pitch + colb : nullptr,
+                                g.bias_pitch, g.beta);
           } else if (row < g.M) {
-            if (vec_ok && colb + 32 <= g.N) {
-              if (g.beta != 0.0f) {
+            if (g.beta != 0.0f) {
 #pragma unroll
-                for (int p = 0; p < 32 / PN; ++p) {
-                  float old[PN];
-                  unpack<T>(ld_pack(crow + colb, p), old);
+              for (int p = 0; p < 32 / PN; ++p) {
+                float old[PN];
+                unpack<T>(ld_pack(crow + colb, p), old);
 #pragma unroll
-                  for (int e = 0; e < PN; ++e) r[p * PN + e] += g.beta * old[e];
-                }
-              }
-#pragma unroll
-              for (int p = 0; p < 32 / PN; ++p) st_pack(crow + colb, p, pack<T>(r + p * PN));
-            } else {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                if (colb + j < g.N) {
-                  float o = r[j];
-                  if (g.beta != 0.0f) o += g.beta * mp_up(crow[colb + j]);
-                  crow[colb + j] = mp_down<T>(o);
-                }
+                for (int e = 0; e < PN; ++e) r[p * PN + e] += g.beta * old[e];
               }
             }
+#pragma unroll
+            for (int p = 0; p < 32 / PN; ++p) st_pack(crow + colb, p, pack<T>(r + p * PN));
           }
           }
         }
@@ -740,125 +689,87 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
   if (warp == 1) tmem_dealloc_pair(tmem_base, ACC_BUFS * BN);
 }
 
-// C = alpha * sum_s partial[s] + bias + beta * C  (finishes a split-K contraction)
-template <typename T>
-__global__ void __launch_bounds__(256) gemm_fold_kernel(const float* __restrict__ partial, int ksplit, size_t mn, int N, float alpha,
-                                                        const T* __restrict__ bias, float beta, T* __restrict__ c, size_t bias_pitch = 0) {
-  const size_t i0 = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) * 4;
-  if (i0 >= mn) return;
-  const bool vec = (mn & 3) == 0;
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  const int cnt = vec ? 4 : static_cast<int>(mn - i0 < 4 ? mn - i0 : 4);
-  for (int sidx = 0; sidx < ksplit; ++sidx) {
-    const float* p = partial + sidx * mn + i0;
-    if (vec) {
-      const float4 v = *reinterpret_cast<const float4*>(p);
-      acc[0] += v.x; acc[1] += v.y; acc[2] += v.z; acc[3] += v.w;
-    } else {
-      for (int e = 0; e < cnt; ++e) acc[e] += p[e];
+// ---------------------------------------------------------------------------
+// Operands that TMA cannot address (a row pitch or a base that is no multiple of 16 bytes: odd widths) are copied into rows of
+// a 16-byte pitch in the stream's workspace and multiplied from there.  The copy moves each element twice against the tensor
+// pipe's M or N uses of it; the FP-pipe kernel that served these shapes before reached 16 TFLOP/s ([2000, 999] x [999, 1501] and
+// the two contractions of its reverse in r32: 1150 us there, 190 us from copies, 15 us of them the copies).  One thread makes one
+// 16-byte chunk of a destination row from 2- or 4-byte loads (neighbouring threads share the sectors); the bytes of the last
+// chunk past the row's end are zeros that the tensor map does not read.
+// ---------------------------------------------------------------------------
+struct PadJob {
+  const unsigned char* src;
+  unsigned char* dst;
+  size_t src_pitch;        // bytes
+  uint32_t row_bytes;      // bytes of a row that are copied
+  uint32_t chunks;         // 16-byte chunks of a destination row
+  uint32_t total;          // chunks of all rows
+};
+__global__ void __launch_bounds__(256) pad_rows_kernel(const PadJob ja, const PadJob jb, uint32_t blocks_a) {
+  const bool second = blockIdx.x >= blocks_a;
+  const PadJob j = second ? jb : ja;
+  const uint32_t id = (second ? blockIdx.x - blocks_a : blockIdx.x) * 256u + threadIdx.x;
+  if (id >= j.total) return;
+  const uint32_t row = id / j.chunks, off = (id - row * j.chunks) * 16u;
+  const unsigned char* s = j.src + row * j.src_pitch + off;
+  uint32_t w[4];
+  if (off + 16u <= j.row_bytes) {
+    if ((reinterpret_cast<uintptr_t>(s) & 3u) == 0) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) w[e] = *reinterpret_cast<const uint32_t*>(s + 4 * e);
+    } else {   // r16 at an odd element: half words at both ends, words between
+      const uint32_t h0 = *reinterpret_cast<const uint16_t*>(s), h7 = *reinterpret_cast<const uint16_t*>(s + 14);
+      const uint32_t a = *reinterpret_cast<const uint32_t*>(s + 2), b = *reinterpret_cast<const uint32_t*>(s + 6), c = *reinterpret_cast<const uint32_t*>(s + 10);
+      w[0] = h0 | (a << 16);
+      w[1] = (a >> 16) | (b << 16);
+      w[2] = (b >> 16) | (c << 16);
+      w[3] = (c >> 16) | (h7 << 16);
+    }
+  } else {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      w[e] = 0u;
+      if (off + 4 * e + 2 <= j.row_bytes) w[e] = *reinterpret_cast<const uint16_t*>(s + 4 * e);
+      if (off + 4 * e + 4 <= j.row_bytes) w[e] |= static_cast<uint32_t>(*reinterpret_cast<const uint16_t*>(s + 4 * e + 2)) << 16;
     }
   }
-  for (int e = 0; e < cnt; ++e) {
-    float o = alpha * acc[e];
-    if (bias != nullptr) o += mp_up(bias_pitch != 0 ? bias[(i0 + e) / N * bias_pitch + (i0 + e) % N] : bias[(i0 + e) % N]);
-    if (beta != 0.0f) o += beta * mp_up(c[i0 + e]);
-    c[i0 + e] = mp_down<T>(o);
-  }
+  *reinterpret_cast<uint4*>(j.dst + static_cast<size_t>(id) * 16u) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
 // ---------------------------------------------------------------------------
 // Host side: tensor maps and dispatch.
 // ---------------------------------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_tiled() {
-  static EncodeTiledFn fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, []() {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    MP_CUDA_CHECK(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qres));
-    if (p == nullptr || qres != cudaDriverEntryPointSuccess) MP_FATAL("cuTensorMapEncodeTiled is not available");
-    fn = reinterpret_cast<EncodeTiledFn>(p);
-  });
-  return fn;
-}
-
-// 2-D row-major matrix [rows, cols] of T, box = {box_cols (128 bytes), box_rows}, 128-byte swizzle
-// (16-byte atoms, or 32-byte atoms when `atom32`), out-of-range elements read as zero.
-// batch > 1: [batch, rows, cols] densely packed as a 3-D tensor, boxes one batch entry deep.
-template <typename T>
-CUtensorMap make_map(const void* base, size_t rows, size_t cols, uint32_t box_cols, uint32_t box_rows, bool atom32 = false,
-                     size_t batch = 1) {
-  CUtensorMap map;
-  const cuuint64_t dims[3] = {cols, rows, batch};
-  const cuuint64_t strides[2] = {cols * sizeof(T), rows * cols * sizeof(T)};
-  const cuuint32_t box[3] = {box_cols, box_rows, 1};
-  const cuuint32_t estr[3] = {1, 1, 1};
-  const CUtensorMapDataType dt = sizeof(T) == 2 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-  MP_CU_CHECK(encode_tiled()(&map, dt, batch > 1 ? 3 : 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                             atom32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
-                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE));
-  return map;
-}
-
-// Row-major [rows, cols] output, box {32 cols, 32 rows} unswizzled, or (wide) {64 cols, 32 rows} of r16 in the
-// 128-byte swizzle.
-template <typename T>
-CUtensorMap make_store_map(void* base, size_t rows, size_t cols, bool wide = false, size_t batch = 1) {
-  CUtensorMap map;
-  const cuuint64_t dims[3] = {cols, rows, batch};
-  const cuuint64_t strides[2] = {cols * sizeof(T), rows * cols * sizeof(T)};
-  const cuuint32_t box[3] = {wide ? 64u : 32u, 32, 1};
-  const bool swizzle = wide || sizeof(T) == 4;   // 128-byte rows: r16 wide boxes and every r32 box
-  const cuuint32_t estr[3] = {1, 1, 1};
-  const CUtensorMapDataType dt = sizeof(T) == 2 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-  MP_CU_CHECK(encode_tiled()(&map, dt, batch > 1 ? 3 : 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                             swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE));
-  return map;
-}
-
-template <typename T, int BN>
-void launch_tc(const T* a, const T* b, const GemmArgs& args, int sm_count, cudaStream_t st) {
-  using G = GemmT<T>;
+template <int BN, bool EXACT>
+void launch_tc(Operand<__half> a, Operand<__half> b, const GemmArgs& args, int sm_count, cudaStream_t st) {
+  using T = __half;
+  using G = GemmT;
   const int M = args.M, N = args.N, K = args.K;
   // A: K-major [M,K] box {BK, BM};  MN-major [K,M] box {BK (along M), BK (k-rows)}
-  // (32-bit MN-major tiles: 128-byte swizzle with 32-byte atoms, the only MN-major layout tf32 accepts)
   const size_t nb = static_cast<size_t>(args.batch);
-  const CUtensorMap ta = args.a_mn ? make_map<T>(a, K, M, G::BK, G::BK, G::TF32, nb) : make_map<T>(a, M, K, G::BK, BM, false, nb);
-  const CUtensorMap tb = args.b_mn ? make_map<T>(b, K, N, G::BK, G::BK, G::TF32, nb) : make_map<T>(b, N, K, G::BK, BN, false, nb);
+  const CUtensorMap ta = args.a_mn ? make_map<T>(a.p, K, M, a.ld, G::BK, G::BK, CU_TENSOR_MAP_SWIZZLE_128B, nb) : make_map<T>(a.p, M, K, a.ld, G::BK, BM, CU_TENSOR_MAP_SWIZZLE_128B, nb);
+  const CUtensorMap tb = args.b_mn ? make_map<T>(b.p, K, N, b.ld, G::BK, G::BK, CU_TENSOR_MAP_SWIZZLE_128B, nb) : make_map<T>(b.p, N, K, b.ld, G::BK, BN, CU_TENSOR_MAP_SWIZZLE_128B, nb);
   // C as a TMA store target: 32 x 32 blocks, no swizzle (only used when the row pitch is a multiple of 16 bytes)
   CUtensorMap tc = ta;
-  if ((static_cast<size_t>(N) * sizeof(T)) % 16 == 0 && mp_aligned16(args.c)) tc = make_store_map<T>(args.c, M, N, sizeof(T) == 2 && BN >= 128, nb);
-  const size_t smem = static_cast<size_t>(args.stages) * stage_bytes<BN>(args.split != 0) + 1024 /*align*/ + 1024 /*barriers*/ +
-                      8 * EpiBufs<T>::value * 32 * 32 * sizeof(T) /*epilogue staging*/;
-  MP_CUDA_CHECK(cudaFuncSetAttribute(gemm_tcgen05_kernel<T, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  if ((args.ldc * sizeof(T)) % 16 == 0 && mp_aligned16(args.c)) tc = make_store_map<T>(args.c, M, N, args.ldc, BN >= 128, nb);
+  const size_t smem = static_cast<size_t>(args.stages) * stage_bytes<BN>() + 1024 /*align*/ + 1024 /*barriers*/ +
+                      8 * EPI_BUFS * 32 * 32 * sizeof(T) /*epilogue staging*/;
+  MP_CUDA_CHECK(cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      static_cast<int>(smem)));
   const long tiles = static_cast<long>((N + BN - 1) / BN) * ((M + BM - 1) / BM) * args.ksplit * args.batch;
   const int grid = tiles < sm_count ? static_cast<int>(tiles) : sm_count;   // persistent: one CTA per SM
-  gemm_tcgen05_kernel<T, BN><<<grid, args.split ? GEMM_MAX_THREADS : GEMM_THREADS, smem, st>>>(ta, tb, tc, args);
+  gemm_tcgen05_kernel<BN, EXACT><<<grid, GEMM_THREADS, smem, st>>>(ta, tb, tc, args);
   MP_LAUNCH_CHECK();
-  if (args.ksplit > 1) {
-    const size_t mn = static_cast<size_t>(M) * N;
-    gemm_fold_kernel<T><<<static_cast<unsigned>((mn / 4 + 256) / 256), 256, 0, st>>>(args.partial, args.ksplit, mn, N, args.alpha,
-                                                                                  static_cast<const T*>(args.bias), args.beta,
-                                                                                  static_cast<T*>(args.c), args.bias_pitch);
-    MP_LAUNCH_CHECK();
-  }
+  if (args.ksplit > 1) launch_fold<T>(args, st);
 }
 
-void launch_pair(const __half* a, const __half* b, GemmArgs args, int sm_count, cudaStream_t st) {
+void launch_pair(Operand<__half> a, Operand<__half> b, GemmArgs args, int sm_count, cudaStream_t st) {
   using T = __half;
-  using G = GemmT<T>;
+  using G = GemmT;
   const int M = args.M, N = args.N, K = args.K;
-  const CUtensorMap ta = args.a_mn ? make_map<T>(a, K, M, G::BK, G::BK) : make_map<T>(a, M, K, G::BK, BM);
-  const CUtensorMap tb = args.b_mn ? make_map<T>(b, K, N, G::BK, G::BK) : make_map<T>(b, N, K, G::BK, PAIR_BN / 2);
+  const CUtensorMap ta = args.a_mn ? make_map<T>(a.p, K, M, a.ld, G::BK, G::BK) : make_map<T>(a.p, M, K, a.ld, G::BK, BM);
+  const CUtensorMap tb = args.b_mn ? make_map<T>(b.p, K, N, b.ld, G::BK, G::BK) : make_map<T>(b.p, N, K, b.ld, G::BK, PAIR_BN / 2);
   CUtensorMap tc = ta;
-  if ((static_cast<size_t>(N) * sizeof(T)) % 16 == 0 && mp_aligned16(args.c)) tc = make_store_map<T>(args.c, M, N, true);
+  if ((args.ldc * sizeof(T)) % 16 == 0 && mp_aligned16(args.c)) tc = make_store_map<T>(args.c, M, N, args.ldc, true);
   // 227 KB: six 32 KB stages + one 4 KB staging box per epilogue warp, or five stages + two boxes.  The ring depth is what
   // feeds the tensor pipe: a stage is refilled only after its MMAs have completed, so (stages - 1) x 32 KB are in flight
   // per SM against an L2 latency of 2 - 3 k cycles under load (measured: the MMA thread waited for operands 35 - 40 % of
@@ -873,18 +784,7 @@ void launch_pair(const __half* a, const __half* b, GemmArgs args, int sm_count, 
   const int pairs = tiles < sm_count / 2 ? tiles : sm_count / 2;
   gemm_tcgen05_pair_kernel<<<2 * pairs, GEMM_THREADS, smem, st>>>(ta, tb, tc, args);
   MP_LAUNCH_CHECK();
-  if (args.ksplit > 1) {
-    const size_t mn = static_cast<size_t>(M) * N;
-    gemm_fold_kernel<T><<<static_cast<unsigned>((mn / 4 + 256) / 256), 256, 0, st>>>(args.partial, args.ksplit, mn, N, args.alpha,
-                                                                                  static_cast<const T*>(args.bias), args.beta,
-                                                                                  static_cast<T*>(args.c), args.bias_pitch);
-    MP_LAUNCH_CHECK();
-  }
-}
-
-bool env_flag(const char* name) {
-  const char* e = getenv(name);
-  return e != nullptr && e[0] != '\0' && e[0] != '0';
+  if (args.ksplit > 1) launch_fold<T>(args, st);
 }
 
 // Output-tile width: wide tiles for wide problems, narrower ones when they are
@@ -900,16 +800,16 @@ int pick_bn(int M, int N, int sms, int batch = 1) {
 // idle or run a mostly empty last wave.  Cost model in k-block steps of one CTA:
 //   waves(tiles * ks / SMs) * (k-blocks per unit + fixed cost per unit) * step time(BN)  [+ fold traffic]
 // The unsplit choice of pick_bn stays unless a split is predicted to be at least 15 % faster.
-void pick_split_k(GemmArgs& args, size_t elem, int sms, size_t workspace_bytes, int* bn_io) {
-  const int bk = static_cast<int>(128 / elem);
+void pick_split_k(GemmArgs& args, int sms, size_t workspace_bytes, int* bn_io) {
+  constexpr int bk = GemmT::BK;
   const long num_kb = (args.K + bk - 1) / bk;
   if (num_kb < 32) return;
-  const double mn_bytes = static_cast<double>(args.M) * args.N * 4.0;
+  const double mn_bytes = static_cast<double>(args.M) * args.partial_ld * 4.0;
   auto cost = [&](int bn, int ks) {
     const long tiles = static_cast<long>((args.M + BM - 1) / BM) * ((args.N + bn - 1) / bn);
     const long waves = (tiles * ks + sms - 1) / sms;
-    // one k-block step of a CTA at ~1000 TFLOP/s over all SMs (r32: half the rate, three MMAs per slice), in microseconds
-    const double step_us = 2.0 * BM * bn * bk / (1000.0e6 / sms) * (args.split ? 3.0 : 1.0) * (elem == 4 ? 2.0 : 1.0);
+    // one k-block step of a CTA at ~1000 TFLOP/s over all SMs, in microseconds
+    const double step_us = 2.0 * BM * bn * bk / (1000.0e6 / sms);
     double t = waves * ((num_kb + ks - 1) / ks + 8.0) * step_us;
     if (ks > 1) t += 2.0 * ks * mn_bytes / 6.0e6 + 3.0;   // partial write + read at ~6 TB/s, one more launch
     return t;
@@ -932,97 +832,194 @@ void pick_split_k(GemmArgs& args, size_t elem, int sms, size_t workspace_bytes, 
   if (best_ks > 1 && best < 0.85 * base) { args.ksplit = best_ks; *bn_io = best_bn; }
 }
 
+// One r16 contraction whose operands TMA can address.  `args` carries the problem; the tile width, the K split and the ring depth
+// are chosen here.  workspace: room for split-K partials.
+void gemm_run_r16(Operand<__half> a, Operand<__half> b, GemmArgs args, int sms, void* workspace, size_t workspace_bytes, cudaStream_t st) {
+  args.partial_ld = (args.N + 3) & ~3;
+  int bn = pick_bn(args.M, args.N, sms, args.batch);
+  args.ksplit = 1;
+  args.partial = static_cast<float*>(workspace);
+  if (args.batch == 1 && !env_flag("MP_GEMM_NO_SPLITK")) pick_split_k(args, sms, workspace_bytes, &bn);
+  // shared memory of the ring: 227 KB per CTA minus alignment slack, barriers and the epilogue staging (64 KB)
+  const int budget = 159 * 1024;
+  auto stages_for = [&](int per_stage) {   // the ring runs across tiles, so depth is bounded by memory only
+    int s = budget / per_stage;
+    if (s > MAX_STAGES) s = MAX_STAGES;
+    return s < 2 ? 2 : s;
+  };
+  // CTA pairs for wide problems with enough 256 x 256 tiles to fill the pairs
+  const long pair_tiles = static_cast<long>((args.M + 255) / 256) * ((args.N + 255) / 256);
+  if (args.batch == 1 && !env_flag("MP_GEMM_NO_PAIRS") && args.M >= 256 && args.N >= 256) {
+    if (args.ksplit == 1 && bn == 256 && pair_tiles >= sms / 2) {
+      launch_pair(a, b, args, sms, st);
+      return;
+    }
+    if (args.ksplit > 1) {
+      // long K, few tiles: 256 x 256 pair tiles with the K range cut so that the units fill the pairs about evenly
+      const long num_kb = (args.K + 63) / 64;
+      const int pairs = sms / 2;
+      int best = 0; double best_cost = 1e30;
+      for (int ks = 1; ks <= 16; ++ks) {
+        if (num_kb / ks < 8 || (ks - 1) * ((num_kb + ks - 1) / ks) >= num_kb) continue;
+        if (static_cast<double>(ks) * args.M * args.partial_ld * 4.0 > static_cast<double>(workspace_bytes)) break;
+        const long waves = (pair_tiles * ks + pairs - 1) / pairs;
+        const double cost = waves * ((num_kb + ks - 1) / ks + 10.0) + (ks > 1 ? 2.0 * ks * args.M * args.N * 4.0 / 6.0e6 / 0.5 : 0.0);
+        if (cost < best_cost) { best_cost = cost; best = ks; }
+      }
+      if (best >= 1) {
+        args.ksplit = best;
+        launch_pair(a, b, args, sms, st);
+        return;
+      }
+    }
+  }
+  if (bn == 256 && args.exact) bn = 128;
+  if (bn == 256) {
+    args.stages = stages_for(stage_bytes<256>());
+    launch_tc<256, false>(a, b, args, sms, st);
+  } else if (bn == 128) {
+    args.stages = stages_for(stage_bytes<128>());
+    if (args.exact) launch_tc<128, true>(a, b, args, sms, st); else launch_tc<128, false>(a, b, args, sms, st);
+  } else {
+    args.stages = stages_for(stage_bytes<64>());
+    if (args.exact) launch_tc<64, true>(a, b, args, sms, st); else launch_tc<64, false>(a, b, args, sms, st);
+  }
+}
+
+inline void gemm_run(Operand<__half> a, Operand<__half> b, const GemmArgs& args, int sms, void* ws, size_t ws_bytes, cudaStream_t st) {
+  gemm_run_r16(a, b, args, sms, ws, ws_bytes, st);
+}
+inline void gemm_run(Operand<float> a, Operand<float> b, const GemmArgs& args, int sms, void* ws, size_t ws_bytes, cudaStream_t st) {
+  gemm_run_r32(a, b, args, sms, ws, ws_bytes, st);
+}
+
+// The FP-pipe kernel: r64, and what does not pay on the tensor cores.
+template <typename T>
+void gemm_simt(const T* a, const T* b, const T* bias, double alpha, T* c, double beta, len_t M, len_t N, len_t K, int a_mn, int b_mn, len_t batch,
+               len_t bias_pitch, cudaStream_t st) {
+  using A = typename Acc<T>::type;
+  if ((M + 63) / 64 > 65535) MP_FATAL("inner_product: M too large for the FP-pipe kernel");
+  for (len_t b0 = 0; b0 < batch; b0 += 65535) {   // grid.z carries the batch index
+    const len_t nb = batch - b0 < 65535 ? batch - b0 : 65535;
+    const dim3 grid(static_cast<unsigned>((N + 63) / 64), static_cast<unsigned>((M + 63) / 64), static_cast<unsigned>(nb));
+    gemm_simt_kernel<T><<<grid, 256, 0, st>>>(a + b0 * M * K, b + b0 * K * N, bias, static_cast<A>(alpha), c + b0 * M * N, static_cast<A>(beta), M,
+                                              N, K, a_mn, b_mn, bias_pitch);
+    MP_LAUNCH_CHECK();
+  }
+}
+
+// A contraction with operands that need a copy into aligned rows (see pad_rows_kernel).  Where the copies of whole operands do
+// not fit three quarters of the workspace (the rest is left to split-K partials), the batch, then the rows of C, then its
+// columns are worked off in slabs.  Returns false where even the smallest slab does not fit (a K of tens of thousands with a
+// small MP_WORKSPACE_MB).
+template <typename T>
+bool gemm_padded(const T* a, const T* b, bool pad_a, bool pad_b, GemmArgs args, MpStreamState* state, cudaStream_t st) {
+  const size_t M = args.M, N = args.N, K = args.K, batch = args.batch;
+  const size_t limit = state->workspace_bytes / 4 * 3;
+  constexpr size_t LINE = 16 / sizeof(T);
+  auto up = [](size_t v, size_t to) { return (v + to - 1) / to * to; };
+  auto bytes_a = [&](size_t m) { return pad_a ? up((args.a_mn ? K * up(m, LINE) : m * up(K, LINE)) * sizeof(T), 256) : 0; };
+  auto bytes_b = [&](size_t n) { return pad_b ? up((args.b_mn ? K * up(n, LINE) : n * up(K, LINE)) * sizeof(T), 256) : 0; };
+  size_t ms = M, ns = N, bs = batch;
+  if (bytes_a(M) + bytes_b(N) > limit) {
+    bs = 1;
+    while (bytes_a(ms) + bytes_b(ns) > limit) {
+      size_t* cut = (bytes_a(ms) >= bytes_b(ns) && ms > 256) || ns <= 256 ? &ms : &ns;
+      if (*cut <= 256) return false;
+      *cut = up((*cut + 1) / 2, 256);
+    }
+  } else if (batch > 1) {
+    const size_t per = bytes_a(M) + bytes_b(N);
+    if (per * batch > limit) bs = limit / per;
+  }
+  unsigned char* ws = static_cast<unsigned char*>(state->workspace);
+  const T* bias = static_cast<const T*>(args.bias);
+  T* c = static_cast<T*>(args.c);
+  for (size_t b0 = 0; b0 < batch; b0 += bs) {
+    const size_t nb = batch - b0 < bs ? batch - b0 : bs;
+    for (size_t n0 = 0; n0 < N; n0 += ns) {
+      for (size_t m0 = 0; m0 < M; m0 += ms) {
+        const size_t m = M - m0 < ms ? M - m0 : ms, n = N - n0 < ns ? N - n0 : ns;
+        size_t used = 0;
+        PadJob jobs[2] = {};
+        uint32_t blocks[2] = {0, 0};
+        auto place = [&](int which, const T* src, bool pad, bool mn, size_t ext, size_t full) {   // ext of `full` rows resp. columns
+          const size_t rows = (mn ? K : ext) * nb, cols = mn ? ext : K, src_ld = mn ? full : K;
+          if (!pad) return Operand<T>{src, src_ld};
+          const size_t ld = up(cols, LINE);
+          PadJob& j = jobs[which];
+          j.src = reinterpret_cast<const unsigned char*>(src);
+          j.dst = ws + used;
+          j.src_pitch = src_ld * sizeof(T);
+          j.row_bytes = static_cast<uint32_t>(cols * sizeof(T));
+          j.chunks = static_cast<uint32_t>(ld / LINE);
+          j.total = static_cast<uint32_t>(rows * (ld / LINE));
+          blocks[which] = (j.total + 255) / 256;
+          used += up(rows * ld * sizeof(T), 256);
+          return Operand<T>{reinterpret_cast<const T*>(j.dst), ld};
+        };
+        // (slabs inside an entry only with bs = 1, so a copy of several entries is always of whole, densely packed ones)
+        const Operand<T> oa = place(0, a + b0 * M * K + (args.a_mn ? m0 : m0 * K), pad_a, args.a_mn != 0, m, M);
+        const Operand<T> ob = place(1, b + b0 * N * K + (args.b_mn ? n0 : n0 * K), pad_b, args.b_mn != 0, n, N);
+        pad_rows_kernel<<<blocks[0] + blocks[1], 256, 0, st>>>(jobs[0], jobs[1], blocks[0]);
+        MP_LAUNCH_CHECK();
+        GemmArgs s = args;
+        s.exact = 1;
+        s.M = static_cast<int>(m);
+        s.N = static_cast<int>(n);
+        s.batch = static_cast<int>(nb);
+        s.c = c + b0 * M * N + m0 * args.ldc + n0;
+        if (bias != nullptr) s.bias = bias + m0 * args.bias_pitch + n0;
+        gemm_run(oa, ob, s, state->sm_count, ws + used, state->workspace_bytes - used, st);
+      }
+    }
+  }
+  return true;
+}
+
 template <typename T>
 void gemm_dispatch(const void* a_, const void* b_, const void* bias, double alpha, void* c_, double beta, len_t M, len_t N,
                    len_t K, int a_mn, int b_mn, StreamContext ctx, len_t batch = 1, len_t bias_pitch = 0) {
-  using A = typename Acc<T>::type;
   if (M == 0 || N == 0 || batch == 0) return;
   cudaStream_t st = mp_stream(ctx);
   const T* a = static_cast<const T*>(a_);
   const T* b = static_cast<const T*>(b_);
   T* c = static_cast<T*>(c_);
-  bool tensor_path = !std::is_same<T, double>::value && K > 0 && !env_flag("MP_GEMM_FORCE_SIMT");
-  if (tensor_path) {
-    // TMA needs 16-byte aligned bases and row pitches, and 32-bit coordinates
-    const size_t a_pitch = (a_mn ? M : K) * sizeof(T), b_pitch = (b_mn ? N : K) * sizeof(T);
-    tensor_path = mp_aligned16(a) && mp_aligned16(b) && a_pitch % 16 == 0 && b_pitch % 16 == 0 &&
-                  M < (1ull << 31) && N < (1ull << 31) && K < (1ull << 31) && mp_state_or_null(ctx) != nullptr;
-    if (batch > 1) {
-      // 3-D maps: the batch pitch must keep 16-byte alignment, and the work-unit count stays in 32 bits
-      const double units = static_cast<double>((M + BM - 1) / BM) * static_cast<double>((N + 63) / 64) * static_cast<double>(batch);
-      tensor_path = tensor_path && (M * K * sizeof(T)) % 16 == 0 && (K * N * sizeof(T)) % 16 == 0 && units < 2.0e9;
-    }
-  }
-  if (!tensor_path) {
-    if ((M + 63) / 64 > 65535) MP_FATAL("inner_product: M too large for the FP-pipe kernel");
-    for (len_t b0 = 0; b0 < batch; b0 += 65535) {   // grid.z carries the batch index
-      const len_t nb = batch - b0 < 65535 ? batch - b0 : 65535;
-      const dim3 grid(static_cast<unsigned>((N + 63) / 64), static_cast<unsigned>((M + 63) / 64), static_cast<unsigned>(nb));
-      gemm_simt_kernel<T><<<grid, 256, 0, st>>>(a + b0 * M * K, b + b0 * K * N, static_cast<const T*>(bias), static_cast<A>(alpha),
-                                                c + b0 * M * N, static_cast<A>(beta), M, N, K, a_mn, b_mn, bias_pitch);
-      MP_LAUNCH_CHECK();
-    }
-    return;
-  }
   if constexpr (!std::is_same<T, double>::value) {
-    MpStreamState* state = mp_state(ctx);
-    GemmArgs args;
-    args.bias = bias;
-    args.bias_pitch = bias_pitch;
-    args.c = c;
-    args.alpha = static_cast<float>(alpha);
-    args.beta = static_cast<float>(beta);
-    args.M = static_cast<int>(M);
-    args.N = static_cast<int>(N);
-    args.K = static_cast<int>(K);
-    args.a_mn = a_mn;
-    args.b_mn = b_mn;
-    args.split = (std::is_same<T, float>::value && !env_flag("MP_GEMM_TF32X1")) ? 1 : 0;
-    args.status = state->status_dev;
-    args.batch = static_cast<int>(batch);
-    int bn = pick_bn(args.M, args.N, state->sm_count, args.batch);
-    args.ksplit = 1;
-    args.partial = static_cast<float*>(state->workspace);
-    if (batch == 1 && !env_flag("MP_GEMM_NO_SPLITK")) pick_split_k(args, sizeof(T), state->sm_count, state->workspace_bytes, &bn);
-    // shared memory of the ring: 227 KB per CTA minus alignment slack, barriers and the epilogue staging (r16: 64 KB, r32: 32 KB)
-    const int budget = (sizeof(T) == 2 ? 159 : 168) * 1024;
-    auto stages_for = [&](int per_stage) {   // the ring runs across tiles, so depth is bounded by memory only
-      int s = budget / per_stage;
-      if (s > MAX_STAGES) s = MAX_STAGES;
-      return s < 2 ? 2 : s;
-    };
-    if constexpr (std::is_same<T, __half>::value) {
-      // CTA pairs for wide problems with enough 256 x 256 tiles to fill the pairs
-      const long pair_tiles = static_cast<long>((args.M + 255) / 256) * ((args.N + 255) / 256);
-      if (batch == 1 && !env_flag("MP_GEMM_NO_PAIRS") && args.M >= 256 && args.N >= 256) {
-        if (args.ksplit == 1 && bn == 256 && pair_tiles >= state->sm_count / 2) {
-          launch_pair(a, b, args, state->sm_count, st);
-          return;
-        }
-        if (args.ksplit > 1) {
-          // long K, few tiles: 256 x 256 pair tiles with the K range cut so that the units fill the pairs about evenly
-          const long num_kb = (args.K + 63) / 64;
-          const int pairs = state->sm_count / 2;
-          int best = 0; double best_cost = 1e30;
-          for (int ks = 1; ks <= 16; ++ks) {
-            if (num_kb / ks < 8 || (ks - 1) * ((num_kb + ks - 1) / ks) >= num_kb) continue;
-            if (static_cast<double>(ks) * args.M * args.N * 4.0 > static_cast<double>(state->workspace_bytes)) break;
-            const long waves = (pair_tiles * ks + pairs - 1) / pairs;
-            const double cost = waves * ((num_kb + ks - 1) / ks + 10.0) + (ks > 1 ? 2.0 * ks * args.M * args.N * 4.0 / 6.0e6 / 0.5 : 0.0);
-            if (cost < best_cost) { best_cost = cost; best = ks; }
-          }
-          if (best >= 1) {
-            args.ksplit = best;
-            launch_pair(a, b, args, state->sm_count, st);
-            return;
-          }
-        }
+    // tiles are counted, and TMA addressed, in 32 bits
+    const double units = static_cast<double>((M + BM - 1) / BM) * static_cast<double>((N + 63) / 64) * static_cast<double>(batch);
+    MpStreamState* state = mp_state_or_null(ctx);
+    bool tensor_path = state != nullptr && K > 0 && M < (1ull << 31) && N < (1ull << 31) && K < (1ull << 31) && units < 2.0e9 &&
+                       !env_flag("MP_GEMM_FORCE_SIMT");
+    // TMA needs 16-byte aligned bases, row pitches and batch pitches
+    const size_t a_pitch = (a_mn ? M : K) * sizeof(T), b_pitch = (b_mn ? N : K) * sizeof(T);
+    const bool pad_a = !mp_aligned16(a) || a_pitch % 16 != 0, pad_b = !mp_aligned16(b) || b_pitch % 16 != 0;
+    // a problem of one or two tiles is over on the FP pipe before the copy's launch has paid
+    if (pad_a || pad_b) tensor_path = tensor_path && static_cast<double>(M) * N * K * batch > 1.0e6;
+    if (tensor_path) {
+      GemmArgs args;
+      args.bias = bias;
+      args.bias_pitch = bias_pitch;
+      args.c = c;
+      args.ldc = N;
+      args.alpha = static_cast<float>(alpha);
+      args.beta = static_cast<float>(beta);
+      args.M = static_cast<int>(M);
+      args.N = static_cast<int>(N);
+      args.K = static_cast<int>(K);
+      args.a_mn = a_mn;
+      args.b_mn = b_mn;
+      args.split = (std::is_same<T, float>::value && !env_flag("MP_GEMM_TF32X1")) ? 1 : 0;
+      args.status = state->status_dev;
+      args.batch = static_cast<int>(batch);
+      if (!pad_a && !pad_b) {
+        gemm_run(Operand<T>{a, a_mn ? M : K}, Operand<T>{b, b_mn ? N : K}, args, state->sm_count, state->workspace, state->workspace_bytes, st);
+        return;
       }
+      if (gemm_padded<T>(a, b, pad_a, pad_b, args, state, st)) return;
     }
-    if (bn == 256) { args.stages = stages_for(stage_bytes<256>(args.split != 0)); launch_tc<T, 256>(a, b, args, state->sm_count, st); }
-    else if (bn == 128) { args.stages = stages_for(stage_bytes<128>(args.split != 0)); launch_tc<T, 128>(a, b, args, state->sm_count, st); }
-    else { args.stages = stages_for(stage_bytes<64>(args.split != 0)); launch_tc<T, 64>(a, b, args, state->sm_count, st); }
   }
+  gemm_simt<T>(a, b, static_cast<const T*>(bias), alpha, c, beta, M, N, K, a_mn, b_mn, batch, bias_pitch, st);
 }
 
 }  // namespace

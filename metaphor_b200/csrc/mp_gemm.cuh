@@ -1,0 +1,173 @@
+// What the contraction kernels of gemm.cu (r16) and gemm_r32.cu share: the problem description, the store of blocks that
+// TMA cannot write, the split-K fold and the tensor maps.
+#pragma once
+
+#include "mp_tcgen05.cuh"
+
+#include <cuda.h>
+#include <mutex>
+
+struct GemmArgs {
+  const void* bias;   // N values of T (bias_pitch = 0), a full [M, N] matrix (bias_pitch = N), or nullptr
+  size_t bias_pitch = 0;
+  void* c;            // [M, N] row-major, row pitch ldc
+  size_t ldc;
+  float alpha, beta;
+  int M, N, K;
+  int a_mn, b_mn;     // operand major-ness: 0 = K contiguous, 1 = M resp. N contiguous
+  int stages;
+  int exact = 0;      // r16: sum with rounding between chunks of K where the single-CTA kernel runs
+  int epi_boxes = 2;  // pair kernel: 64-column staging boxes per epilogue warp
+  int split;          // r32 only: 1 = error-compensated hi/lo split (3 MMAs per k-slice), 0 = one tf32 MMA (for timing)
+  int ksplit;         // > 1: the K range of every tile is cut into ksplit work units whose raw fp32
+  float* partial;     //      accumulators go to partial[unit_split][M][partial_ld]; a fold kernel finishes C
+  int partial_ld;     // N rounded up to four columns
+  int batch;          // > 1: densely packed [batch, M, K] x [batch, K, N] -> [batch, M, N] over 3-D tensor maps (ksplit = 1)
+  uint32_t* status;
+};
+
+// An operand as the tensor maps see it: rows of `ld` elements, 16-byte aligned.
+template <typename T> struct Operand { const T* p; size_t ld; };
+
+namespace {
+
+constexpr int BM = 128;               // UMMA M (one TMEM lane per output row)
+constexpr int SWIZZLE_BYTES = 128;    // one operand row / k-row in shared memory
+
+// One 32 x 32 block of a tile (lane = row, r = its 32 columns) into a C that TMA and 16-byte stores cannot write: odd row
+// pitch or base, or the last columns under beta.  A lane's own row is 32 separate sectors per store instruction, so the block is
+// turned around through 4 KB of the warp's staging (column XOR row: no bank conflicts either way) and leaves one row per
+// instruction; the matrix term and the old C come in the same way.
+template <typename T>
+__device__ __forceinline__ void store_block_rows(float* stage, const float* r, int lane, T* c, size_t ldc, int rows, bool col_in, const T* mat,
+                                                 size_t mat_ld, float beta) {
+#pragma unroll
+  for (int j = 0; j < 32; ++j) stage[lane * 32 + (j ^ lane)] = r[j];
+  __syncwarp();
+#pragma unroll 4
+  for (int i = 0; i < rows; ++i) {
+    float v = stage[i * 32 + (lane ^ i)];
+    if (col_in) {
+      if (mat != nullptr) v += mp_up(mat[i * mat_ld + lane]);
+      if (beta != 0.0f) v += beta * mp_up(c[i * ldc + lane]);
+      c[i * ldc + lane] = mp_down<T>(v);
+    }
+  }
+  __syncwarp();
+}
+
+// C = alpha * sum_s partial[s] + bias + beta * C  (finishes a split-K contraction).  A thread folds four neighbouring columns
+// of a row; partial rows have a pitch of whole fours whatever N is.
+template <typename T>
+__global__ void __launch_bounds__(256) gemm_fold_kernel(const float* __restrict__ partial, int ksplit, int M, int N, int ld, float alpha,
+                                                        const T* __restrict__ bias, float beta, T* c, size_t ldc, size_t bias_pitch) {
+  const size_t mn = static_cast<size_t>(M) * ld;
+  const size_t i0 = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) * 4;
+  if (i0 >= mn) return;
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+  for (int sidx = 0; sidx < ksplit; ++sidx) {
+    const float4 v = *reinterpret_cast<const float4*>(partial + sidx * mn + i0);
+    acc[0] += v.x; acc[1] += v.y; acc[2] += v.z; acc[3] += v.w;
+  }
+  const int per_row = ld / 4;
+  const size_t unit = i0 / 4;
+  const size_t row = unit < (size_t(1) << 32) ? static_cast<uint32_t>(unit) / static_cast<uint32_t>(per_row) : unit / per_row;
+  const int col = static_cast<int>(unit - row * per_row) * 4;
+  T* cr = c + row * ldc + col;
+  const T* br = bias != nullptr ? bias + row * bias_pitch + col : nullptr;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    if (col + e < N) {
+      float o = alpha * acc[e];
+      if (br != nullptr) o += mp_up(br[e]);
+      if (beta != 0.0f) o += beta * mp_up(cr[e]);
+      acc[e] = o;
+    }
+  }
+  if (col + 4 <= N && (ldc * sizeof(T)) % 16 == 0 && mp_aligned16(c)) {
+    struct alignas(4 * sizeof(T)) Four { T v[4]; } f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) f.v[e] = mp_down<T>(acc[e]);
+    *reinterpret_cast<Four*>(cr) = f;
+  } else {
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (col + e < N) cr[e] = mp_down<T>(acc[e]);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Host side.
+// ---------------------------------------------------------------------------
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+EncodeTiledFn encode_tiled() {
+  static EncodeTiledFn fn = nullptr;
+  static std::once_flag once;
+  std::call_once(once, []() {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult qres;
+    MP_CUDA_CHECK(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qres));
+    if (p == nullptr || qres != cudaDriverEntryPointSuccess) MP_FATAL("cuTensorMapEncodeTiled is not available");
+    fn = reinterpret_cast<EncodeTiledFn>(p);
+  });
+  return fn;
+}
+
+// 2-D row-major matrix [rows, cols] of T, box = {box_cols (128 bytes), box_rows}, out-of-range
+// elements read as zero.
+// ld: row pitch in elements.  batch > 1: [batch, rows, ld] as a 3-D tensor, boxes one batch entry deep.
+template <typename T>
+CUtensorMap make_map(const void* base, size_t rows, size_t cols, size_t ld, uint32_t box_cols, uint32_t box_rows,
+                     CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B, size_t batch = 1) {
+  CUtensorMap map;
+  const cuuint64_t dims[3] = {cols, rows, batch};
+  const cuuint64_t strides[2] = {ld * sizeof(T), rows * ld * sizeof(T)};
+  const cuuint32_t box[3] = {box_cols, box_rows, 1};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  const CUtensorMapDataType dt = sizeof(T) == 2 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+  MP_CU_CHECK(encode_tiled()(&map, dt, batch > 1 ? 3 : 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                             swizzle,
+                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE));
+  return map;
+}
+
+// Row-major [rows, cols] output, box {32 cols, 32 rows} unswizzled, or (wide) {64 cols, 32 rows} of r16 in the
+// 128-byte swizzle.
+template <typename T>
+CUtensorMap make_store_map(void* base, size_t rows, size_t cols, size_t ld, bool wide = false, size_t batch = 1) {
+  CUtensorMap map;
+  const cuuint64_t dims[3] = {cols, rows, batch};
+  const cuuint64_t strides[2] = {ld * sizeof(T), rows * ld * sizeof(T)};
+  const cuuint32_t box[3] = {wide ? 64u : 32u, 32, 1};
+  const bool swizzle = wide || sizeof(T) == 4;   // 128-byte rows: r16 wide boxes and every r32 box
+  const cuuint32_t estr[3] = {1, 1, 1};
+  const CUtensorMapDataType dt = sizeof(T) == 2 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+  MP_CU_CHECK(encode_tiled()(&map, dt, batch > 1 ? 3 : 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                             swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE));
+  return map;
+}
+
+template <typename T>
+void launch_fold(const GemmArgs& args, cudaStream_t st) {
+  const size_t units = static_cast<size_t>(args.M) * args.partial_ld / 4;
+  gemm_fold_kernel<T><<<static_cast<unsigned>((units + 255) / 256), 256, 0, st>>>(args.partial, args.ksplit, args.M, args.N, args.partial_ld,
+                                                                                args.alpha, static_cast<const T*>(args.bias), args.beta,
+                                                                                static_cast<T*>(args.c), args.ldc, args.bias_pitch);
+  MP_LAUNCH_CHECK();
+}
+
+bool env_flag(const char* name) {
+  const char* e = getenv(name);
+  return e != nullptr && e[0] != '\0' && e[0] != '0';
+}
+
+}  // namespace
+
+// gemm_r32.cu: one r32 contraction whose operands TMA can address; picks the tile and the K split itself.
+void gemm_run_r32(Operand<float> a, Operand<float> b, GemmArgs args, int sms, void* workspace, size_t workspace_bytes, cudaStream_t st);

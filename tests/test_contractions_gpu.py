@@ -148,3 +148,49 @@ def test_large_shape_against_float64_matmul(mp, stream, sfx):
     err = float((c.double() - ref).abs().max() / ref.abs().max())
     assert err <= TOL_RED[sfx], err
     assert stream.status() == 0
+
+
+# Operands whose rows are not 16-byte aligned are copied into aligned rows and multiplied on the tensor cores.  (batch, m, n, k):
+# one ragged tile, ragged tiles of the single-CTA kernel, enough 256 x 256 tiles for the CTA-pair kernel, a split of a long odd n
+# (partial rows padded to four columns), odd batch entries, and copies beyond the workspace (worked off in slabs of rows, of
+# columns, of batch entries).
+ODD_SHAPES = [(1, 101, 103, 107), (1, 257, 65, 515), (1, 2571, 77, 1993), (1, 255, 4099, 130), (1, 130, 4098, 131), (7, 101, 99, 63),
+              (1, 16411, 1101, 67), (1, 67, 1101, 16411), (90, 513, 301, 515)]
+
+
+@pytest.mark.parametrize("sfx", ["r16", "r32"])
+@pytest.mark.parametrize("shape", ODD_SHAPES)
+@pytest.mark.parametrize("variant", ["ij_jk_ik", "ij_kj_ik", "ji_jk_ik"])
+def test_unaligned_operands(mp, stream, sfx, shape, variant):
+    import torch
+    from util import torch_dtype
+    nb, m, n, k = shape
+    dt = torch_dtype(sfx)
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    ta, tb = variant[0] == "j", variant[3:5] == "kj"
+    # bases one element off a 16-byte boundary in two of three variants
+    def operand(rows, cols, scale, off):
+        flat = (torch.randn(nb * rows * cols + off, generator=g, device="cuda") * scale).to(dt)
+        return flat[off:].view(nb, rows, cols)
+    a = operand(*((n, m) if ta else (m, n)), 1.0, int(ta))
+    b = operand(*((k, n) if tb else (n, k)), n ** -0.5, int(tb))
+    c0 = operand(m, k, 1.0, 1)
+    c = torch.full_like(c0, float("nan"))
+    name = "inner_product_" + ("_".join("b" + p for p in variant.split("_")) if nb > 1 else variant)
+    dims = (nb, m, n, k) if nb > 1 else (m, n, k)
+    ref = (a.double().transpose(1, 2) if ta else a.double()) @ (b.double().transpose(1, 2) if tb else b.double())
+    run(mp, stream, name, sfx, a, b, 1.0, c, 0.0, *dims)
+    assert float((c.double() - ref).abs().max() / ref.abs().max()) <= TOL_RED[sfx]
+    c1 = operand(m, k, 0.0, 1)
+    c1.copy_(c0)
+    run(mp, stream, name, sfx, a, b, 0.5, c1, 1.0, *dims)
+    ref = 0.5 * ref + c0.double()
+    assert float((c1.double() - ref).abs().max() / ref.abs().max()) <= TOL_RED[sfx]
+    if nb == 1 and variant == "ij_jk_ik":      # the bias and the matrix term through the same stores
+        bias = operand(1, k, 1.0, 1)
+        run(mp, stream, "linear_ij_jk_ik", sfx, a, b, bias, 1.0, c, 0.0, *dims)
+        ref = a.double()[0] @ b.double()[0]
+        assert float((c.double()[0] - ref - bias.double()[0]).abs().max() / ref.abs().max()) <= TOL_RED[sfx]
+        run(mp, stream, "linear_ij_jk_ik_ik", sfx, a, b, c0, 1.0, c, 0.0, *dims)
+        assert float((c.double()[0] - ref - c0.double()[0]).abs().max() / ref.abs().max()) <= TOL_RED[sfx]
+    assert stream.status() == 0
