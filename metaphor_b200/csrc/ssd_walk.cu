@@ -182,70 +182,85 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_con
   } else if (warp == 1) {
     // ------------------------------ MMA issuer --------------------------------
     // Order per chunk k: Yd(k) as soon as its P tile is written, Yo(k) as soon as the state the chunk
-    // receives is in shared memory, S(k), then the scores of chunk k+1.
-    if (lane == 0) {
-      const uint32_t id_g = umma_instr_desc(UMMA_FMT_F16, 0u, 0u, 128, 128);   // q (K-major) x k (K-major)
-      const uint32_t id_y = umma_instr_desc(UMMA_FMT_F16, 0u, 1u, 128, 64);    // K-major A x MN-major B
-      const uint32_t id_s = umma_instr_desc(UMMA_FMT_F16, 1u, 1u, 128, 64);    // k^T (MN-major A) x MN-major B
-      const uint32_t sp = mp_smem_u32(sP), sh = mp_smem_u32(sH), svs = mp_smem_u32(sVs);
-      auto issue_g = [&](int s) {
-        const uint32_t sq = mp_smem_u32(smem + s * W_STAGE), sk = sq + W_TILE_QK;
+    // receives is in shared memory, S(k), then the scores of chunk k+1.  The warp walks the loop as a whole, one elected lane
+    // issues (see elect_one): a chunk's 32 MMAs are on the critical path of the hand-offs, and under `lane == 0` each of them
+    // cost about 65 cycles of moving its descriptors into uniform registers.
+    const uint32_t id_g = umma_instr_desc(UMMA_FMT_F16, 0u, 0u, 128, 128);   // q (K-major) x k (K-major)
+    const uint32_t id_y = umma_instr_desc(UMMA_FMT_F16, 0u, 1u, 128, 64);    // K-major A x MN-major B
+    const uint32_t id_s = umma_instr_desc(UMMA_FMT_F16, 1u, 1u, 128, 64);    // k^T (MN-major A) x MN-major B
+    // descriptors of ring stage 0; stage 1 and the k-slices differ in the address field (16-byte units)
+    const uint32_t s0 = mp_smem_u32(smem);
+    const uint64_t d_q = umma_smem_desc(s0, 16, 1024), d_k = umma_smem_desc(s0 + W_TILE_QK, 16, 1024);
+    const uint64_t d_kt = umma_smem_desc(s0 + W_TILE_QK, WQ * 128, 1024), d_v = umma_smem_desc(s0 + 2 * W_TILE_QK, W_TILE_V, 1024);
+    const uint64_t d_p = umma_smem_desc(mp_smem_u32(sP), 16, 1024), d_h = umma_smem_desc(mp_smem_u32(sH), W_TILE_V, 1024);
+    const uint64_t d_vs = umma_smem_desc(mp_smem_u32(sVs), W_TILE_V, 1024);
+    constexpr uint32_t STAGE_U = W_STAGE >> 4, ROWS_U = 2048 >> 4;           // MN-major k-slice: 16 rows of 128 bytes
+    auto kslice = [](int ks) { return static_cast<uint32_t>(((ks >> 2) * (WQ * 128) + (ks & 3) * 32) >> 4); };   // K-major: two 64-column blocks
+    auto issue_g = [&](int s) {
+      tcgen05_fence_after_sync();
+      if (elect_one()) {
+        const uint64_t dq = d_q + s * STAGE_U, dk = d_k + s * STAGE_U;
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) {
-          const uint32_t o = (ks >> 2) * (WQ * 128) + (ks & 3) * 32;
-          umma<false>(tmem + TC_G, umma_smem_desc(sq + o, 16, 1024), umma_smem_desc(sk + o, 16, 1024), id_g, ks != 0 ? 1u : 0u);
-        }
+        for (int ks = 0; ks < 8; ++ks) umma<false>(tmem + TC_G, dq + kslice(ks), dk + kslice(ks), id_g, ks != 0 ? 1u : 0u);
         umma_commit(bars + B_GFULL);
-      };
-      WalkSeg sg;
-      int qb = 0;          // chunks walked before this segment
-      uint32_t hq = 0;     // completions of B_HREADY consumed so far (one per received state, incl. a carried-in one)
-      bool ok = true;
-      for (int si = 0; ok && walk_segment(cta, ncta, nseq, nc, si, sg); ++si) {
-        ok = walk_wait(bars + B_FULL0 + (qb & 1), (qb >> 1) & 1, g.status, abort);
-        if (ok) { tcgen05_fence_after_sync(); issue_g(qb & 1); }
-        for (int k = 0; ok && k < sg.n; ++k) {
-          const int q = qb + k;
-          const int s = q & 1;
-          const uint32_t sq = mp_smem_u32(smem + s * W_STAGE), sk = sq + W_TILE_QK, sv = sk + W_TILE_QK;
-          const uint32_t ty = tmem + TC_Y + (q & 1) * 128;
-          if (!walk_wait(bars + B_PREADY, q & 1, g.status, abort)) { ok = false; break; }
-          tcgen05_fence_after_sync();
+      }
+      __syncwarp();
+    };
+    WalkSeg sg;
+    int qb = 0;          // chunks walked before this segment
+    uint32_t hq = 0;     // completions of B_HREADY consumed so far (one per received state, incl. a carried-in one)
+    bool ok = true;
+    auto await = [&](int bar, uint32_t parity) {
+      ok = walk_wait(bars + bar, parity, g.status, abort);
+      ok = __all_sync(0xffffffffu, ok) != 0;
+      return ok;
+    };
+    for (int si = 0; ok && walk_segment(cta, ncta, nseq, nc, si, sg); ++si) {
+      if (await(B_FULL0 + (qb & 1), (qb >> 1) & 1)) issue_g(qb & 1);
+      for (int k = 0; ok && k < sg.n; ++k) {
+        const int q = qb + k;
+        const int s = q & 1;
+        const uint32_t ty = tmem + TC_Y + (q & 1) * 128;
+        if (!await(B_PREADY, q & 1)) break;
+        tcgen05_fence_after_sync();
+        const uint64_t dv = d_v + s * STAGE_U;
+        if (elect_one()) {
 #pragma unroll
-          for (int ks = 0; ks < 8; ++ks) {
-            const uint32_t o = (ks >> 2) * (WQ * 128) + (ks & 3) * 32;
-            umma<false>(ty, umma_smem_desc(sp + o, 16, 1024), umma_smem_desc(sv + ks * 2048, W_TILE_V, 1024), id_y, ks != 0 ? 1u : 0u);
-          }
-          const bool has_state = k > 0 || sg.cin != 0;
+          for (int ks = 0; ks < 8; ++ks) umma<false>(ty, d_p + kslice(ks), dv + ks * ROWS_U, id_y, ks != 0 ? 1u : 0u);
+        }
+        __syncwarp();
+        const bool has_state = k > 0 || sg.cin != 0;
+        if (has_state) {
+          if (!await(B_HREADY, hq & 1u)) break;
+          ++hq;
+          tcgen05_fence_after_sync();
+        }
+        if (elect_one()) {
           if (has_state) {
-            if (!walk_wait(bars + B_HREADY, hq & 1u, g.status, abort)) { ok = false; break; }
-            ++hq;
-            tcgen05_fence_after_sync();
             if (g.hs_out != nullptr) {   // the state this chunk receives, straight from its operand tile
               const int c = ANTI ? nc - 1 - (sg.p0 + k) : sg.p0 + k;
               tma_store_2d(&map_hs, sH, 0, static_cast<int>((static_cast<size_t>(sg.seq) * nc + c) * WN));
               bulk_commit();
             }
+            const uint64_t dq = d_q + s * STAGE_U;
 #pragma unroll
-            for (int ks = 0; ks < 8; ++ks) {
-              const uint32_t o = (ks >> 2) * (WQ * 128) + (ks & 3) * 32;
-              umma<false>(ty + 64, umma_smem_desc(sq + o, 16, 1024), umma_smem_desc(sh + ks * 2048, W_TILE_V, 1024), id_y, ks != 0 ? 1u : 0u);
-            }
+            for (int ks = 0; ks < 8; ++ks) umma<false>(ty + 64, dq + kslice(ks), d_h + ks * ROWS_U, id_y, ks != 0 ? 1u : 0u);
           }
           umma_commit(bars + B_YFULL);
-          // scores of the next chunk (its stage was released by S(k-1); the workers are past G(k))
-          if (k + 1 < sg.n) {
-            const int s1 = (q + 1) & 1;
-            if (!walk_wait(bars + B_FULL0 + s1, ((q + 1) >> 1) & 1, g.status, abort)) { ok = false; break; }
-            tcgen05_fence_after_sync();
-            issue_g(s1);
-          }
-          if (!walk_wait(bars + B_VSREADY, q & 1, g.status, abort)) { ok = false; break; }
-          tcgen05_fence_after_sync();
+        }
+        __syncwarp();
+        // scores of the next chunk (its stage was released by S(k-1); the workers are past G(k))
+        if (k + 1 < sg.n) {
+          const int s1 = (q + 1) & 1;
+          if (!await(B_FULL0 + s1, ((q + 1) >> 1) & 1)) break;
+          issue_g(s1);
+        }
+        if (!await(B_VSREADY, q & 1)) break;
+        tcgen05_fence_after_sync();
+        const uint64_t dkt = d_kt + s * STAGE_U;
+        if (elect_one()) {
 #pragma unroll
-          for (int ks = 0; ks < 8; ++ks)
-            umma<false>(tmem + TC_S, umma_smem_desc(sk + ks * 2048, WQ * 128, 1024), umma_smem_desc(svs + ks * 2048, W_TILE_V, 1024), id_s,
-                        ks != 0 ? 1u : 0u);
+          for (int ks = 0; ks < 8; ++ks) umma<false>(tmem + TC_S, dkt + ks * ROWS_U, d_vs + ks * ROWS_U, id_s, ks != 0 ? 1u : 0u);
           // The workers rewrite the state tile once S(k) is complete: the store issued above must have read it by then.
           // (Waiting here, behind the next chunk's score MMAs, costs nothing; waiting right after the store held back
           // the commit of the output accumulators by the store's whole latency in every chunk.)
@@ -253,10 +268,11 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_con
           umma_commit(bars + B_SFULL);
           umma_commit(bars + B_EMPTY0 + s);
         }
-        qb += sg.n;
+        __syncwarp();
       }
-      if (g.hs_out != nullptr) bulk_wait_all<0>();
+      qb += sg.n;
     }
+    if (g.hs_out != nullptr) bulk_wait_all<0>();
   } else {
     // ------------------------------ workers -----------------------------------
     // Software pipeline: in iteration k the warps write the P tile of chunk k+1, fold S(k) into the carried
@@ -667,55 +683,64 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_group_grads_kernel(const __g
       }
     }
   } else if (warp == 1) {
-    // ------------------------------ MMA issuer --------------------------------
-    if (lane == 0) {
-      const uint32_t id_kk = umma_instr_desc(UMMA_FMT_F16, 0u, 0u, 128, 128);   // K-major x K-major
-      const uint32_t id_kn = umma_instr_desc(UMMA_FMT_F16, 0u, 1u, 128, 128);   // K-major A x MN-major B
-      const uint32_t id_nn = umma_instr_desc(UMMA_FMT_F16, 1u, 1u, 128, 128);   // MN-major A x MN-major B
-      auto issue_score = [&](int hi) {
-        const uint32_t st = mp_smem_u32(smem + (hi & 1) * GG_STAGE);
+    // ------------------------------ MMA issuer (the warp as a whole, see elect_one) ----
+    const uint32_t id_kk = umma_instr_desc(UMMA_FMT_F16, 0u, 0u, 128, 128);   // K-major x K-major
+    const uint32_t id_kn = umma_instr_desc(UMMA_FMT_F16, 0u, 1u, 128, 128);   // K-major A x MN-major B
+    const uint32_t id_nn = umma_instr_desc(UMMA_FMT_F16, 1u, 1u, 128, 128);   // MN-major A x MN-major B
+    // K-major descriptors of the tiles of stage 0 (gy, x, Hc, Ha); stage 1 and the k-slices differ in the address field
+    const uint32_t s0 = mp_smem_u32(smem);
+    const uint64_t d_t = umma_smem_desc(s0, 16, 1024);
+    constexpr uint32_t STAGE_U = GG_STAGE >> 4, TILE_U = GG_TILE >> 4, ROWS_U = 2048 >> 4;
+    bool ok = true;
+    auto await = [&](int bar, uint32_t parity) {
+      ok = walk_wait(bars + bar, parity, g.status, abort);
+      ok = __all_sync(0xffffffffu, ok) != 0;
+      return ok;
+    };
+    auto issue_score = [&](int hi) {
+      tcgen05_fence_after_sync();
+      const uint64_t dt = d_t + (hi & 1) * STAGE_U;
+      if (elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          umma<false>(tmem + GT_SC + (hi & 1) * 128, umma_smem_desc(st + ks * 32, 16, 1024), umma_smem_desc(st + GG_TILE + ks * 32, 16, 1024),
-                      id_kk, ks != 0 ? 1u : 0u);
+        for (int ks = 0; ks < 4; ++ks) umma<false>(tmem + GT_SC + (hi & 1) * 128, dt + 2 * ks, dt + TILE_U + 2 * ks, id_kk, ks != 0 ? 1u : 0u);
         umma_commit(bars + GB_SC0 + (hi & 1));
-      };
-      bool ok = walk_wait(bars + GB_FULL0, 0, g.status, abort);
-      if (ok) { tcgen05_fence_after_sync(); issue_score(0); }
-      for (int hi = 0; ok && hi < nh; ++hi) {
-        const int s = hi & 1;
-        if (hi + 1 < nh) {   // the next head's scores run while the workers transform this head's
-          if (!walk_wait(bars + GB_FULL0 + ((hi + 1) & 1), ((hi + 1) >> 1) & 1, g.status, abort)) { ok = false; break; }
-          tcgen05_fence_after_sync();
-          issue_score(hi + 1);
-        }
-        if (!walk_wait(bars + GB_SCALED, hi & 1, g.status, abort)) { ok = false; break; }
-        tcgen05_fence_after_sync();
-        const uint32_t st = mp_smem_u32(smem + s * GG_STAGE);
+      }
+      __syncwarp();
+    };
+    if (await(GB_FULL0, 0)) issue_score(0);
+    for (int hi = 0; ok && hi < nh; ++hi) {
+      const int s = hi & 1;
+      if (hi + 1 < nh) {   // the next head's scores run while the workers transform this head's
+        if (!await(GB_FULL0 + ((hi + 1) & 1), ((hi + 1) >> 1) & 1)) break;
+        issue_score(hi + 1);
+      }
+      if (!await(GB_SCALED, hi & 1)) break;
+      tcgen05_fence_after_sync();
+      const uint64_t dt = d_t + s * STAGE_U;
+      if (elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          umma<false>(tmem + GT_C, umma_smem_desc(st + ks * 32, 16, 1024), umma_smem_desc(st + 2 * GG_TILE + ks * 32, 16, 1024), id_kk,
-                      (hi | ks) != 0 ? 1u : 0u);
+        for (int ks = 0; ks < 4; ++ks) umma<false>(tmem + GT_C, dt + 2 * ks, dt + 2 * TILE_U + 2 * ks, id_kk, (hi | ks) != 0 ? 1u : 0u);
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          umma<false>(tmem + GT_B, umma_smem_desc(st + GG_TILE + ks * 32, 16, 1024), umma_smem_desc(st + 3 * GG_TILE + ks * 32, 16, 1024), id_kk,
-                      (hi | ks) != 0 ? 1u : 0u);
+        for (int ks = 0; ks < 4; ++ks) umma<false>(tmem + GT_B, dt + TILE_U + 2 * ks, dt + 3 * TILE_U + 2 * ks, id_kk, (hi | ks) != 0 ? 1u : 0u);
         umma_commit(bars + GB_EMPTY0 + s);
       }
-      // summed scores x B and (summed scores)^T x C
-      if (ok) ok = walk_wait(bars + GB_GG, 0, g.status, abort) && walk_wait(bars + GB_BCFULL, 0, g.status, abort);
-      if (ok) {
-        tcgen05_fence_after_sync();
-        const uint32_t sg = mp_smem_u32(sGG), sb = mp_smem_u32(smem), sc = mp_smem_u32(smem + GG_STAGE);
+      __syncwarp();
+    }
+    // summed scores x B and (summed scores)^T x C
+    if (ok && await(GB_GG, 0) && await(GB_BCFULL, 0)) {
+      tcgen05_fence_after_sync();
+      const uint64_t d_sg = umma_smem_desc(mp_smem_u32(sGG), 16, 1024), d_sgt = umma_smem_desc(mp_smem_u32(sGG), GG_TILE, 1024);
+      const uint64_t d_b = umma_smem_desc(s0, GG_TILE, 1024), d_c = umma_smem_desc(s0 + GG_STAGE, GG_TILE, 1024);
+      if (elect_one()) {
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks)     // K = step j: A K-major over the two 64-column blocks, B rows j (MN-major, two 64-column blocks)
-          umma<false>(tmem + GT_C, umma_smem_desc(sg + (ks >> 2) * GG_TILE + (ks & 3) * 32, 16, 1024), umma_smem_desc(sb + ks * 2048, GG_TILE, 1024),
-                      id_kn, 1u);
+          umma<false>(tmem + GT_C, d_sg + (ks >> 2) * TILE_U + (ks & 3) * 2, d_b + ks * ROWS_U, id_kn, 1u);
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks)     // K = step i: A = transposed view of the same tile (MN-major), C rows i
-          umma<false>(tmem + GT_B, umma_smem_desc(sg + ks * 2048, GG_TILE, 1024), umma_smem_desc(sc + ks * 2048, GG_TILE, 1024), id_nn, 1u);
+          umma<false>(tmem + GT_B, d_sgt + ks * ROWS_U, d_c + ks * ROWS_U, id_nn, 1u);
         umma_commit(bars + GB_ACC);
       }
+      __syncwarp();
     }
   } else {
     // ------------------------------ workers -----------------------------------
