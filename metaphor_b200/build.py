@@ -4,6 +4,8 @@ Outputs (all under ``metaphor_b200/lib/``, git-ignored, shipped as built files):
 
 * ``libmp_kernels.so`` - every launcher plus the ``mp*`` utilities; this is
   what the Python binding and the tests load.
+* ``mp_launch.so`` - the CPython module through which ``launch`` and the fused
+  chains call that library;
 * ``mp_kernels.a`` and ``libdev_utils.so`` - the same objects under the
   artefact names the reference's build.zig links (build.zig:125-146), so a Zig
   build can link this library in place of its own.
@@ -74,6 +76,7 @@ def build(force: bool = False, verbose: bool = True) -> Path:
         if verbose:
             print(f"built {so}")
     build_host()
+    build_launch()
     return so
 
 
@@ -87,6 +90,19 @@ def build_host() -> Path:
     if not out.exists() or out.stat().st_mtime < newest:
         subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall", "-o", str(out), str(src),
                         "-L" + str(LIB), "-lmp_kernels", "-Wl,-rpath,$ORIGIN"], check=True)
+    return out
+
+
+def build_launch() -> Path:
+    """CPython module of the launch path (host/py_launch.cpp) -> lib/mp_launch.so, linked against libmp_kernels.so in
+    the same directory."""
+    import sysconfig
+    src = ROOT / "host" / "py_launch.cpp"
+    out = LIB / "mp_launch.so"
+    newest = max([src.stat().st_mtime, (LIB / "libmp_kernels.so").stat().st_mtime] + [h.stat().st_mtime for h in INCLUDE.glob("*.h")])
+    if not out.exists() or out.stat().st_mtime < newest:
+        subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall", "-I" + sysconfig.get_paths()["include"], "-o", str(out),
+                        str(src), "-L" + str(LIB), "-lmp_kernels", "-Wl,-rpath,$ORIGIN"], check=True)
     return out
 
 

@@ -14,10 +14,15 @@ def lib() -> C.CDLL:
     return abi.load()
 
 
+@functools.lru_cache(maxsize=None)
+def _suffixes():
+    import torch
+    return {torch.float16: "r16", torch.float32: "r32", torch.float64: "r64"}
+
+
 def suffix_of(dtype) -> str:
     """Dtype-key suffix in the order of the reference's scalar.zig Tag enum."""
-    import torch
-    return {torch.float16: "r16", torch.float32: "r32", torch.float64: "r64"}[dtype]
+    return _suffixes()[dtype]
 
 
 def _arg(a):
@@ -67,13 +72,35 @@ class Stream:
         self.close()
 
 
-def launch(name: str, dtype, *args):
-    """Call ``launch_<name>_<suffix>(*args)``; tensors become device pointers.
-    The last argument must be a Stream or a StreamContext."""
+def _launch_ctypes(name: str, dtype, *args):
+    """``launch`` for arguments that the native path does not convert itself."""
     fn = getattr(lib(), f"launch_{name}_{suffix_of(dtype)}")
     conv = [_arg(a) for a in args[:-1]]
     ctx = args[-1].ctx if isinstance(args[-1], Stream) else args[-1]
     fn(*conv, ctx)
+
+
+def _load_native():
+    """The native call path (host/py_launch.cpp), None while the library is not built."""
+    import importlib.machinery
+    import importlib.util
+    path = abi.LIB_PATH.parent / "mp_launch.so"
+    if not path.exists():
+        return None
+    import torch
+    loader = importlib.machinery.ExtensionFileLoader("mp_launch", str(path))
+    mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("mp_launch", loader))
+    loader.exec_module(mod)
+    mod.setup((torch.float16, torch.float32, torch.float64), torch.Tensor, C.Array, C.c_void_p, abi.StreamContext, Stream, _launch_ctypes)
+    return mod
+
+
+_native = _load_native()
+if _native is not None:
+    launch = _native.launch
+else:
+    def launch(name: str, dtype, *args):
+        raise ImportError(f"{abi.LIB_PATH.parent / 'mp_launch.so'} is missing: run `python -m metaphor_b200.build` (needs nvcc)")
 
 
 class FusedChain:
@@ -89,18 +116,13 @@ class FusedChain:
         n = self._lib.mpJitNumLeaves(self.handle)
         self.leaves = [self._lib.mpJitLeafName(self.handle, i).decode() for i in range(n)]
 
-    def _ptrs(self, tensors):
-        arr = (C.c_void_p * len(tensors))(*[(t.data_ptr() if t is not None else 0) for t in tensors])
-        return arr
-
     def forward(self, leaves, out, n, stream):
         assert len(leaves) == len(self.leaves)
-        self._lib.mpJitForward(self.handle, self._ptrs(leaves), C.c_void_p(out.data_ptr()), n, stream.ctx)
+        _native.chain_forward(self.handle, leaves, out, n, stream)
 
     def reverse(self, leaves, g_out, g_leaves, alpha, n, stream):
         assert len(leaves) == len(self.leaves) == len(g_leaves)
-        self._lib.mpJitReverse(self.handle, self._ptrs(leaves), C.c_void_p(g_out.data_ptr() if g_out is not None else 0),
-                               self._ptrs(g_leaves), float(alpha), n, stream.ctx)
+        _native.chain_reverse(self.handle, leaves, g_out, g_leaves, float(alpha), n, stream)
 
     def close(self):
         if self.handle:
