@@ -174,6 +174,7 @@ namespace {
 // One CTA waits for a phase of a shared-memory barrier that nothing completes: the bounded wait runs out, records
 // MP_STATUS_WAIT_TIMEOUT in the stream's status word and the kernel returns normally.
 __global__ void wait_timeout_selftest_kernel(uint32_t* status) {
+  mp_grid_dependency();
   __shared__ uint64_t bar;
   if (threadIdx.x == 0) {
     mbar_init(&bar, 1);
@@ -186,7 +187,7 @@ __global__ void wait_timeout_selftest_kernel(uint32_t* status) {
 // Exercises the time-out path of the bounded waits without any fault: returns after the wait limit of the stream.
 extern "C" void mpSelfTestWaitTimeout(StreamContext ctx) {
   MpStreamState* st = mp_state(ctx);
-  wait_timeout_selftest_kernel<<<1, 32, 0, st->stream>>>(st->status_dev);
+  MpLaunch(1, 32, 0, st->stream)(wait_timeout_selftest_kernel, st->status_dev);
   MP_LAUNCH_CHECK();
 }
 

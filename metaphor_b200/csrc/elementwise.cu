@@ -24,6 +24,7 @@ template <typename T> struct OpCopyTag;  // defined below as the copy functor
 // value, A = arithmetic type, operator()(x0, x1, old, index).
 template <typename T, typename Op, bool VEC>
 __global__ void __launch_bounds__(EW_THREADS) ew_kernel(Op op, const T* in0, const T* in1, T* out, size_t n) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   const size_t tid = threadIdx.x;
   if constexpr (VEC) {
@@ -98,11 +99,11 @@ void ew_launch(Op op, const void* in0, const void* in1, void* out, len_t n, Stre
     const size_t per_cta = static_cast<size_t>(EW_THREADS) * EW_UNROLL * Pack<T>::N;
     size_t grid = (n + per_cta - 1) / per_cta;
     if (grid > cap) grid = cap;
-    ew_kernel<T, Op, true><<<static_cast<unsigned>(grid), EW_THREADS, 0, mp_stream(ctx)>>>(op, p0, p1, po, n);
+    MpLaunch(static_cast<unsigned>(grid), EW_THREADS, 0, mp_stream(ctx))(ew_kernel<T, Op, true>, op, p0, p1, po, n);
   } else {
     size_t grid = (n + EW_THREADS - 1) / EW_THREADS;
     if (grid > cap) grid = cap;
-    ew_kernel<T, Op, false><<<static_cast<unsigned>(grid), EW_THREADS, 0, mp_stream(ctx)>>>(op, p0, p1, po, n);
+    MpLaunch(static_cast<unsigned>(grid), EW_THREADS, 0, mp_stream(ctx))(ew_kernel<T, Op, false>, op, p0, p1, po, n);
   }
   MP_LAUNCH_CHECK();
 }
@@ -240,6 +241,7 @@ __device__ __forceinline__ void adam_one(const AdamParams<T>& p, T& w, T g, T& m
 // Single pass over (w, g, m, v): 4 reads + 3 writes per element.
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(EW_THREADS) adam_kernel(AdamParams<T> p, T* w, const T* g, T* m, T* v, size_t n) {
+  mp_grid_dependency();
   const size_t tid = threadIdx.x;
   if constexpr (VEC) {
     constexpr int PN = Pack<T>::N;
@@ -318,11 +320,11 @@ static void adam_impl(void* w, const void* g, void* m, void* v, double lr, doubl
   if (vec) {
     const size_t per_cta = static_cast<size_t>(EW_THREADS) * 2 * Pack<T>::N;
     size_t grid = (n + per_cta - 1) / per_cta; if (grid > cap) grid = cap;
-    adam_kernel<T, true><<<static_cast<unsigned>(grid), EW_THREADS, 0, mp_stream(s)>>>(
+    MpLaunch(static_cast<unsigned>(grid), EW_THREADS, 0, mp_stream(s))(adam_kernel<T, true>, 
         p, static_cast<T*>(w), static_cast<const T*>(g), static_cast<T*>(m), static_cast<T*>(v), n);
   } else {
     size_t grid = (n + EW_THREADS - 1) / EW_THREADS; if (grid > cap) grid = cap;
-    adam_kernel<T, false><<<static_cast<unsigned>(grid), EW_THREADS, 0, mp_stream(s)>>>(
+    MpLaunch(static_cast<unsigned>(grid), EW_THREADS, 0, mp_stream(s))(adam_kernel<T, false>, 
         p, static_cast<T*>(w), static_cast<const T*>(g), static_cast<T*>(m), static_cast<T*>(v), n);
   }
   MP_LAUNCH_CHECK();

@@ -31,7 +31,8 @@ template <typename T>
 __global__ void __launch_bounds__(256) gemm_simt_kernel(const T* __restrict__ a, const T* __restrict__ b,
                                                         const T* __restrict__ bias, typename Acc<T>::type alpha, T* c,
                                                         typename Acc<T>::type beta, size_t M, size_t N, size_t K, int a_mn,
-                                                        int b_mn, size_t bias_pitch = 0) {
+                                                        int b_mn, size_t bias_pitch) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   constexpr int TS = 64, KS = 16;
   a += static_cast<size_t>(blockIdx.z) * M * K;   // batch entries are densely packed
@@ -175,6 +176,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
   __syncthreads();
   tcgen05_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  mp_grid_dependency();
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -486,6 +488,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
   cluster_sync_all();   // both CTAs' barriers and TMEM exist before anything crosses the pair
   tcgen05_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  mp_grid_dependency();
 
   if (warp == 0) {
     // ------------------------------ TMA producer (both ranks) ------------------
@@ -706,6 +709,7 @@ struct PadJob {
   uint32_t total;          // chunks of all rows
 };
 __global__ void __launch_bounds__(256) pad_rows_kernel(const PadJob ja, const PadJob jb, uint32_t blocks_a) {
+  mp_grid_dependency();
   const bool second = blockIdx.x >= blocks_a;
   const PadJob j = second ? jb : ja;
   const uint32_t id = (second ? blockIdx.x - blocks_a : blockIdx.x) * 256u + threadIdx.x;
@@ -757,7 +761,7 @@ void launch_tc(Operand<__half> a, Operand<__half> b, const GemmArgs& args, int s
                                      static_cast<int>(smem)));
   const long tiles = static_cast<long>((N + BN - 1) / BN) * ((M + BM - 1) / BM) * args.ksplit * args.batch;
   const int grid = tiles < sm_count ? static_cast<int>(tiles) : sm_count;   // persistent: one CTA per SM
-  gemm_tcgen05_kernel<BN, EXACT><<<grid, GEMM_THREADS, smem, st>>>(ta, tb, tc, args);
+  MpLaunch(grid, GEMM_THREADS, smem, st)(gemm_tcgen05_kernel<BN, EXACT>, ta, tb, tc, args);
   MP_LAUNCH_CHECK();
   if (args.ksplit > 1) launch_fold<T>(args, st);
 }
@@ -782,7 +786,7 @@ void launch_pair(Operand<__half> a, Operand<__half> b, GemmArgs args, int sm_cou
   MP_CUDA_CHECK(cudaFuncSetAttribute(gemm_tcgen05_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
   const int tiles = ((N + PAIR_BN - 1) / PAIR_BN) * ((M + 2 * BM - 1) / (2 * BM)) * args.ksplit;
   const int pairs = tiles < sm_count / 2 ? tiles : sm_count / 2;
-  gemm_tcgen05_pair_kernel<<<2 * pairs, GEMM_THREADS, smem, st>>>(ta, tb, tc, args);
+  MpLaunch(2 * pairs, GEMM_THREADS, smem, st)(gemm_tcgen05_pair_kernel, ta, tb, tc, args);
   MP_LAUNCH_CHECK();
   if (args.ksplit > 1) launch_fold<T>(args, st);
 }
@@ -902,7 +906,7 @@ void gemm_simt(const T* a, const T* b, const T* bias, double alpha, T* c, double
   for (len_t b0 = 0; b0 < batch; b0 += 65535) {   // grid.z carries the batch index
     const len_t nb = batch - b0 < 65535 ? batch - b0 : 65535;
     const dim3 grid(static_cast<unsigned>((N + 63) / 64), static_cast<unsigned>((M + 63) / 64), static_cast<unsigned>(nb));
-    gemm_simt_kernel<T><<<grid, 256, 0, st>>>(a + b0 * M * K, b + b0 * K * N, bias, static_cast<A>(alpha), c + b0 * M * N, static_cast<A>(beta), M,
+    MpLaunch(grid, 256, 0, st)(gemm_simt_kernel<T>, a + b0 * M * K, b + b0 * K * N, bias, static_cast<A>(alpha), c + b0 * M * N, static_cast<A>(beta), M,
                                               N, K, a_mn, b_mn, bias_pitch);
     MP_LAUNCH_CHECK();
   }
@@ -961,7 +965,7 @@ bool gemm_padded(const T* a, const T* b, bool pad_a, bool pad_b, GemmArgs args, 
         // (slabs inside an entry only with bs = 1, so a copy of several entries is always of whole, densely packed ones)
         const Operand<T> oa = place(0, a + b0 * M * K + (args.a_mn ? m0 : m0 * K), pad_a, args.a_mn != 0, m, M);
         const Operand<T> ob = place(1, b + b0 * N * K + (args.b_mn ? n0 : n0 * K), pad_b, args.b_mn != 0, n, N);
-        pad_rows_kernel<<<blocks[0] + blocks[1], 256, 0, st>>>(jobs[0], jobs[1], blocks[0]);
+        MpLaunch(blocks[0] + blocks[1], 256, 0, st)(pad_rows_kernel, jobs[0], jobs[1], blocks[0]);
         MP_LAUNCH_CHECK();
         GemmArgs s = args;
         s.exact = 1;

@@ -96,6 +96,7 @@ __global__ void __launch_bounds__(R_THREADS, 1) gemm_r32_kernel(const __grid_con
   __syncthreads();
   tcgen05_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  mp_grid_dependency();
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -372,7 +373,7 @@ void launch_r32(Operand<float> a, Operand<float> b, const GemmArgs& g, int sms, 
   if ((g.ldc * sizeof(float)) % 16 == 0 && mp_aligned16(g.c)) tc = make_store_map<float>(g.c, g.M, g.N, g.ldc, false, nb);
   MP_CUDA_CHECK(cudaFuncSetAttribute(gemm_r32_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM));
   const long units = static_cast<long>((g.N + BN - 1) / BN) * ((g.M + BM - 1) / BM) * g.ksplit * g.batch;
-  gemm_r32_kernel<BN><<<static_cast<unsigned>(units < sms ? units : sms), R_THREADS, Cfg::SMEM, st>>>(ta, tb, tc, g);
+  MpLaunch(static_cast<unsigned>(units < sms ? units : sms), R_THREADS, Cfg::SMEM, st)(gemm_r32_kernel<BN>, ta, tb, tc, g);
   MP_LAUNCH_CHECK();
   if (g.ksplit > 1) launch_fold<float>(g, st);
 }

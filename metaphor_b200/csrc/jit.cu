@@ -152,6 +152,11 @@ class Parser {
 struct TypeInfo { const char* storage; const char* acc; int pack; int bytes; };
 const TypeInfo kTypes[3] = {{"unsigned short", "float", 8, 2}, {"float", "float", 4, 4}, {"double", "double", 2, 8}};
 
+// mp_grid_dependency() of mp_common.cuh: the kernels are launched like the library's own.
+const std::string kGridDependency = "  if (gridDim.x <= " + std::to_string(MP_OVERLAP_CTAS) +
+                                    "u) {\n    asm volatile(\"griddepcontrol.launch_dependents;\" ::: \"memory\");\n"
+                                    "    asm volatile(\"griddepcontrol.wait;\" ::: \"memory\");\n  }\n";
+
 std::string lit(double v, const char* acc) {
   std::ostringstream o;
   o.precision(17);
@@ -253,7 +258,7 @@ __device__ __forceinline__ T down(A f) { T h; asm("cvt.rn.f16.f32 %0, %1;" : "=h
   };
   for (int vec = 1; vec >= 0; --vec) {
     o << "extern \"C\" __global__ void __launch_bounds__(THREADS) mp_jit_fwd_" << (vec ? "vec" : "scalar") << "("
-      << leaf_params("l", true) << "T* out, u64 n) {\n";
+      << leaf_params("l", true) << "T* out, u64 n) {\n" << kGridDependency;
     if (vec) {
       o << "  const u64 nvec = n / PN, trip = (u64)THREADS * UNROLL;\n"
         << "  for (u64 base = blockIdx.x * trip; base < nvec; base += (u64)gridDim.x * trip) {\n";
@@ -288,7 +293,7 @@ __device__ __forceinline__ T down(A f) { T h; asm("cvt.rn.f16.f32 %0, %1;" : "=h
   };
   for (int vec = 1; vec >= 0; --vec) {
     o << "extern \"C\" __global__ void __launch_bounds__(THREADS) mp_jit_rev_" << (vec ? "vec" : "scalar") << "("
-      << leaf_params("l", true) << "const T* go, " << leaf_params("g_", false) << "A alpha, u64 n) {\n";
+      << leaf_params("l", true) << "const T* go, " << leaf_params("g_", false) << "A alpha, u64 n) {\n" << kGridDependency;
     if (vec) {
       o << "  const u64 nvec = n / PN, trip = (u64)THREADS * UNROLL;\n"
         << "  for (u64 base = blockIdx.x * trip; base < nvec; base += (u64)gridDim.x * trip) {\n";
@@ -357,7 +362,7 @@ struct Driver {
   CUresult (*moduleLoadData)(CUmodule*, const void*) = nullptr;
   CUresult (*moduleGetFunction)(CUfunction*, CUmodule, const char*) = nullptr;
   CUresult (*moduleUnload)(CUmodule) = nullptr;
-  CUresult (*launchKernel)(CUfunction, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, CUstream, void**, void**) = nullptr;
+  CUresult (*launchKernelEx)(const CUlaunchConfig*, CUfunction, void**, void**) = nullptr;
 };
 
 Driver* driver() {
@@ -374,7 +379,7 @@ Driver* driver() {
     d.moduleLoadData = reinterpret_cast<decltype(d.moduleLoadData)>(get("cuModuleLoadData"));
     d.moduleGetFunction = reinterpret_cast<decltype(d.moduleGetFunction)>(get("cuModuleGetFunction"));
     d.moduleUnload = reinterpret_cast<decltype(d.moduleUnload)>(get("cuModuleUnload"));
-    d.launchKernel = reinterpret_cast<decltype(d.launchKernel)>(get("cuLaunchKernel"));
+    d.launchKernelEx = reinterpret_cast<decltype(d.launchKernelEx)>(get("cuLaunchKernelEx"));
   });
   return &d;
 }
@@ -492,6 +497,19 @@ extern "C" void mpJitRelease(void* handle) {
   delete p;
 }
 
+static void jit_launch(CUfunction f, unsigned grid, void** args, StreamContext ctx) {
+  CUlaunchAttribute attr;
+  attr.id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
+  attr.value.programmaticStreamSerializationAllowed = 1;
+  CUlaunchConfig cfg = {};
+  cfg.gridDimX = grid; cfg.gridDimY = 1; cfg.gridDimZ = 1;
+  cfg.blockDimX = JIT_THREADS; cfg.blockDimY = 1; cfg.blockDimZ = 1;
+  cfg.hStream = reinterpret_cast<CUstream>(mp_stream(ctx));
+  cfg.attrs = &attr;
+  cfg.numAttrs = mp_overlaps(grid) ? 1 : 0;
+  MP_CU_CHECK(driver()->launchKernelEx(&cfg, f, args, nullptr));
+}
+
 static unsigned jit_grid(bool vec, len_t n, int pack, int unroll) {
   const size_t per_cta = vec ? static_cast<size_t>(JIT_THREADS) * unroll * pack : JIT_THREADS;
   size_t grid = (n + per_cta - 1) / per_cta;
@@ -513,8 +531,7 @@ extern "C" void mpJitForward(void* handle, const void* const* leaves, void* out,
   args.push_back(&out);
   args.push_back(&nn);
   const unsigned grid = jit_grid(vec, n, kTypes[p->dtype].pack, p->unroll);
-  MP_CU_CHECK(driver()->launchKernel(vec ? p->fwd_vec : p->fwd_scalar, grid, 1, 1, JIT_THREADS, 1, 1, 0,
-                                     reinterpret_cast<CUstream>(mp_stream(ctx)), args.data(), nullptr));
+  jit_launch(vec ? p->fwd_vec : p->fwd_scalar, grid, args.data(), ctx);
 }
 
 // g_leaves[l] = d out / d leaf_l * g_out + alpha * g_leaves[l]; g_out NULL means
@@ -538,6 +555,5 @@ extern "C" void mpJitReverse(void* handle, const void* const* leaves, const void
   args.push_back(p->dtype == 2 ? static_cast<void*>(&alpha_d) : static_cast<void*>(&alpha_f));
   args.push_back(&nn);
   const unsigned grid = jit_grid(vec, n, kTypes[p->dtype].pack, p->unroll);
-  MP_CU_CHECK(driver()->launchKernel(vec ? p->rev_vec : p->rev_scalar, grid, 1, 1, JIT_THREADS, 1, 1, 0,
-                                     reinterpret_cast<CUstream>(mp_stream(ctx)), args.data(), nullptr));
+  jit_launch(vec ? p->rev_vec : p->rev_scalar, grid, args.data(), ctx);
 }

@@ -62,6 +62,7 @@ bool vec_ok(const void* p, size_t pitch, size_t width) {
 template <typename T, int V>
 __global__ void __launch_bounds__(256) embedding_kernel(const T* __restrict__ table, const int* __restrict__ ids,
                                                         T* __restrict__ out, size_t n, size_t dim, size_t vocab) {
+  mp_grid_dependency();
   const size_t per_row = dim / V;
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n * per_row;
        i += static_cast<size_t>(gridDim.x) * blockDim.x) {
@@ -83,6 +84,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) embedding_reverse_kernel(const int* __restrict__ ids, const T* __restrict__ gy,
                                                                 typename Acc<T>::type* __restrict__ gtable, size_t n,
                                                                 size_t dim, size_t vocab) {
+  mp_grid_dependency();
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n * dim;
        i += static_cast<size_t>(gridDim.x) * blockDim.x) {
     const size_t t = i / dim, j = i % dim;
@@ -123,6 +125,7 @@ template <typename T, int V, int W>
 __global__ void __launch_bounds__(32 * CONV_TY) conv1d_silu_kernel(const T* __restrict__ x, size_t xp, const T* __restrict__ w,
                                                                   const T* __restrict__ bias, T* __restrict__ y, size_t yp,
                                                                   int L, int C) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   const int c0 = (blockIdx.x * 32 + threadIdx.x) * V;
   const int l0 = (blockIdx.y * CONV_TY + threadIdx.y) * CONV_LT;
@@ -177,6 +180,7 @@ __global__ void __launch_bounds__(32 * CONV_TY) conv1d_silu_reverse_kernel(const
                                                                           typename Acc<T>::type* __restrict__ gw,
                                                                           typename Acc<T>::type* __restrict__ gbias, int L,
                                                                           int C) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   constexpr int H = W - 1;                   // look-ahead steps
   constexpr int ND = CONV_LT + H;            // dpre values a thread needs
@@ -358,6 +362,7 @@ template <int W>
 __global__ void __launch_bounds__(CT_THREADS) conv1d_silu_tiled_kernel(const __half* __restrict__ x, size_t xp, const __half* __restrict__ w,
                                                                        const __half* __restrict__ bias, const ConvSegs sg, int L,
                                                                        int tiles_per_cta) {
+  mp_grid_dependency();
   constexpr int H = W - 1;
   __shared__ __align__(16) __half xs[2][CT_L + H][CT_C];    // two tiles in turn; row r = step l0 - H + r
   __shared__ __align__(16) __half ys[CT_L][CT_C];
@@ -434,6 +439,7 @@ __global__ void __launch_bounds__(CT_THREADS) conv1d_silu_reverse_tiled_kernel(c
                                                                                const ConvSegs sg, __half* __restrict__ gx, size_t gxp,
                                                                                float* __restrict__ gw, float* __restrict__ gbias, int L,
                                                                                int tiles_per_cta) {
+  mp_grid_dependency();
   constexpr int H = W - 1;
   constexpr int NBUF = SKIP ? 1 : 2;
   extern __shared__ __align__(16) unsigned char conv_rev_smem[];
@@ -585,6 +591,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) softplus_bias_kernel(const T* __restrict__ raw, size_t rp,
                                                             const typename Acc<T>::type* __restrict__ bias,
                                                             typename Acc<T>::type* __restrict__ out, size_t rows, int H) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < rows * H;
        i += static_cast<size_t>(gridDim.x) * blockDim.x) {
@@ -603,6 +610,7 @@ __global__ void __launch_bounds__(256) softplus_bias_reverse_kernel(const T* __r
                                                                     T* __restrict__ graw, size_t gp,
                                                                     typename Acc<T>::type* __restrict__ gbias, size_t rows,
                                                                     int H) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   extern __shared__ unsigned char sp_smem[];
   A* bins = reinterpret_cast<A*>(sp_smem);
@@ -632,6 +640,7 @@ __global__ void __launch_bounds__(256) softplus_bias_reverse_heads_kernel(const 
                                                                           T* __restrict__ graw, size_t gp,
                                                                           typename Acc<T>::type* __restrict__ gbias, size_t rows,
                                                                           int H, int RR) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   __shared__ A part[256];
   const int tid = threadIdx.x;
@@ -662,6 +671,7 @@ template <typename T, int V>
 __global__ void __launch_bounds__(256) ssd_gate_kernel(const T* __restrict__ y, const T* __restrict__ x,
                                                        const typename Acc<T>::type* __restrict__ D, const T* __restrict__ z,
                                                        size_t zp, T* __restrict__ u, size_t rows, int H, int P) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   const size_t width = static_cast<size_t>(H) * P, per_row = width / V;
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < rows * per_row;
@@ -686,6 +696,7 @@ __global__ void __launch_bounds__(256) ssd_gate_reverse_kernel(const T* __restri
                                                                T* __restrict__ gy, T* __restrict__ gz, size_t gzp,
                                                                typename Acc<T>::type* __restrict__ gD, size_t rows, int H,
                                                                int P) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   extern __shared__ unsigned char gate_smem[];
   A* bins = reinterpret_cast<A*>(gate_smem);
@@ -751,6 +762,7 @@ __global__ void __launch_bounds__(GN_THREADS) gate_rmsnorm_kernel(const T* __res
                                                                   size_t zp, const T* __restrict__ gain, typename Acc<T>::type eps,
                                                                   T* __restrict__ out, typename Acc<T>::type* __restrict__ rstd,
                                                                   size_t rows, int H, int P) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   const int lane = threadIdx.x & 31;
   const size_t width = static_cast<size_t>(H) * P;
@@ -810,6 +822,7 @@ __global__ void __launch_bounds__(GN_THREADS) gate_rmsnorm_reverse_kernel(
     const T* __restrict__ gain, const typename Acc<T>::type* __restrict__ rstd, const T* __restrict__ gout, T* __restrict__ gy,
     T* __restrict__ gz, size_t gzp, typename Acc<T>::type* __restrict__ gD, typename Acc<T>::type* __restrict__ partial, size_t rows,
     int H, int P) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   extern __shared__ unsigned char gn_smem[];
   A* cols = reinterpret_cast<A*>(gn_smem);
@@ -933,6 +946,7 @@ __global__ void __launch_bounds__(GN_THREADS) gate_rmsnorm_h2_kernel(const __hal
                                                                      const float* __restrict__ D, const __half* __restrict__ z, size_t zp,
                                                                      const __half* __restrict__ gain, float eps, __half* __restrict__ out,
                                                                      float* __restrict__ rstd, size_t rows, int P) {
+  mp_grid_dependency();
   __shared__ float slot[2][GN_THREADS / 64][2];
   constexpr size_t width = static_cast<size_t>(NP) * 512;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, pair = warp >> 1, wsub = warp & 1;
@@ -997,6 +1011,7 @@ __global__ void __launch_bounds__(GN_THREADS) gate_rmsnorm_reverse_h2_kernel(
     const __half* __restrict__ y, const __half* __restrict__ x, const float* __restrict__ D, const __half* __restrict__ z, size_t zp,
     const __half* __restrict__ gain, const float* __restrict__ rstd, const __half* __restrict__ gout, __half* __restrict__ gy,
     __half* __restrict__ gz, size_t gzp, float* __restrict__ gD, float* __restrict__ partial, size_t rows, int H, int P) {
+  mp_grid_dependency();
   extern __shared__ unsigned char gn_smem[];
   float* cols = reinterpret_cast<float*>(gn_smem);
   constexpr size_t width = static_cast<size_t>(NP) * 512;
@@ -1105,6 +1120,7 @@ __global__ void __launch_bounds__(GN_THREADS) gate_rmsnorm_reverse_h2_kernel(
 template <typename T>
 __global__ void __launch_bounds__(1024) gate_rmsnorm_fold_kernel(const typename Acc<T>::type* __restrict__ partial, int nrows, size_t width,
                                                                  typename Acc<T>::type alpha, T* __restrict__ ggain) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   __shared__ A part[32][33];
   const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5;   // 32 columns x 32 row slices: ~10 dependent additions per thread
@@ -1128,6 +1144,7 @@ template <typename T, int V>
 __global__ void __launch_bounds__(256) head_scale_accumulate_kernel(const typename Acc<T>::type* __restrict__ D,
                                                                     const T* __restrict__ gy, T* __restrict__ gx, size_t rows,
                                                                     int H, int P) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   const size_t width = static_cast<size_t>(H) * P, per_row = width / V;
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < rows * per_row;
@@ -1156,6 +1173,7 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(const T* logi
                                                                   typename Acc<T>::type scale,
                                                                   typename Acc<T>::type* __restrict__ loss, T* glogits,
                                                                   size_t n) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   extern __shared__ __align__(128) unsigned char ce_smem[];
   __shared__ A red[CE_THREADS / 32];
@@ -1245,6 +1263,7 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_bulk_kernel(const T*
                                                                        typename Acc<T>::type scale,
                                                                        typename Acc<T>::type* __restrict__ loss, T* glogits,
                                                                        size_t n, uint32_t* status) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   extern __shared__ __align__(128) unsigned char ce_smem[];
   __shared__ uint64_t bar;
@@ -1339,6 +1358,7 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_bulk_kernel(const T*
 // ---------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(256) neg_exp_kernel(const T* __restrict__ src, T* __restrict__ dst, size_t n) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<size_t>(gridDim.x) * blockDim.x)
@@ -1349,6 +1369,7 @@ __global__ void __launch_bounds__(256) neg_exp_kernel(const T* __restrict__ src,
 template <int V>
 __global__ void __launch_bounds__(512) convert_r16_r32_kernel(const __half* __restrict__ src, float* __restrict__ dst, float beta,
                                                               size_t n) {
+  mp_grid_dependency();
   const size_t nv = n / V;
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < nv;
        i += static_cast<size_t>(gridDim.x) * blockDim.x) {
@@ -1364,6 +1385,7 @@ __global__ void __launch_bounds__(512) convert_r16_r32_kernel(const __half* __re
 }
 template <int V>
 __global__ void __launch_bounds__(512) convert_r32_r16_kernel(const float* __restrict__ src, __half* __restrict__ dst, size_t n) {
+  mp_grid_dependency();
   const size_t nv = n / V;
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < nv;
        i += static_cast<size_t>(gridDim.x) * blockDim.x) {
@@ -1377,6 +1399,7 @@ __global__ void __launch_bounds__(512) convert_r32_r16_kernel(const float* __res
 // from device memory, so a captured graph can replay the call for every step.
 struct AdamTick { float inv_bc1, inv_bc2; uint32_t step, nonfinite; };
 __global__ void adam_tick_kernel(AdamTick* t, float beta1, float beta2) {
+  mp_grid_dependency();
   const uint32_t step = t->step + 1;
   t->step = step;
   t->inv_bc1 = 1.f / (1.f - powf(beta1, static_cast<float>(step)));
@@ -1386,6 +1409,7 @@ template <int V>
 __global__ void __launch_bounds__(512) adam_mixed_kernel(float* __restrict__ w32, __half* __restrict__ w16, const float* __restrict__ g32,
                                                          const __half* __restrict__ g16, float* __restrict__ m, float* __restrict__ v,
                                                          float lr, float b1, float b2, float eps, float gscale, AdamTick* tick, size_t n) {
+  mp_grid_dependency();
   const float ib1 = tick->inv_bc1, ib2 = tick->inv_bc2;
   const size_t nv = n / V;
   bool bad = false;
@@ -1428,10 +1452,10 @@ void embedding_impl(const void* table, const void* ids, void* out, len_t n, len_
   constexpr int PN = Pack<T>::N;
   cudaStream_t st = mp_stream(ctx);
   if (dim % PN == 0 && mp_aligned16(table) && mp_aligned16(out))
-    embedding_kernel<T, PN><<<grid_for(n * (dim / PN), 256), 256, 0, st>>>(static_cast<const T*>(table), static_cast<const int*>(ids),
+    MpLaunch(grid_for(n * (dim / PN), 256), 256, 0, st)(embedding_kernel<T, PN>, static_cast<const T*>(table), static_cast<const int*>(ids),
                                                                          static_cast<T*>(out), n, dim, vocab);
   else
-    embedding_kernel<T, 1><<<grid_for(n * dim, 256), 256, 0, st>>>(static_cast<const T*>(table), static_cast<const int*>(ids),
+    MpLaunch(grid_for(n * dim, 256), 256, 0, st)(embedding_kernel<T, 1>, static_cast<const T*>(table), static_cast<const int*>(ids),
                                                                  static_cast<T*>(out), n, dim, vocab);
   MP_LAUNCH_CHECK();
 }
@@ -1440,7 +1464,7 @@ template <typename T>
 void embedding_reverse_impl(const void* ids, const void* gy, void* gtable, len_t n, len_t dim, len_t vocab, StreamContext ctx) {
   if (n == 0 || dim == 0) return;
   using A = typename Acc<T>::type;
-  embedding_reverse_kernel<T><<<grid_for(n * dim, 256), 256, 0, mp_stream(ctx)>>>(static_cast<const int*>(ids), static_cast<const T*>(gy),
+  MpLaunch(grid_for(n * dim, 256), 256, 0, mp_stream(ctx))(embedding_reverse_kernel<T>, static_cast<const int*>(ids), static_cast<const T*>(gy),
                                                                               static_cast<A*>(gtable), n, dim, vocab);
   MP_LAUNCH_CHECK();
 }
@@ -1454,9 +1478,9 @@ void conv_forward_dispatch(const T* x, size_t xp, const T* w, const T* bias, T* 
                   static_cast<unsigned>(batch));
   const int L = static_cast<int>(len), C = static_cast<int>(channels);
   switch (width) {
-    case 2: conv1d_silu_kernel<T, V, 2><<<grid, block, 0, st>>>(x, xp, w, bias, y, yp, L, C); break;
-    case 3: conv1d_silu_kernel<T, V, 3><<<grid, block, 0, st>>>(x, xp, w, bias, y, yp, L, C); break;
-    case 4: conv1d_silu_kernel<T, V, 4><<<grid, block, 0, st>>>(x, xp, w, bias, y, yp, L, C); break;
+    case 2: MpLaunch(grid, block, 0, st)(conv1d_silu_kernel<T, V, 2>, x, xp, w, bias, y, yp, L, C); break;
+    case 3: MpLaunch(grid, block, 0, st)(conv1d_silu_kernel<T, V, 3>, x, xp, w, bias, y, yp, L, C); break;
+    case 4: MpLaunch(grid, block, 0, st)(conv1d_silu_kernel<T, V, 4>, x, xp, w, bias, y, yp, L, C); break;
     default: MP_FATAL("causal_conv1d_silu: kernel width %llu is not supported (2, 3 or 4)", static_cast<unsigned long long>(width));
   }
   MP_LAUNCH_CHECK();
@@ -1472,9 +1496,9 @@ void conv_reverse_dispatch(const T* x, size_t xp, const T* w, const T* bias, con
                   static_cast<unsigned>(batch));
   const int L = static_cast<int>(len), C = static_cast<int>(channels);
   switch (width) {
-    case 2: conv1d_silu_reverse_kernel<T, V, 2><<<grid, block, 0, st>>>(x, xp, w, bias, gy, gyp, gx, gxp, gw, gbias, L, C); break;
-    case 3: conv1d_silu_reverse_kernel<T, V, 3><<<grid, block, 0, st>>>(x, xp, w, bias, gy, gyp, gx, gxp, gw, gbias, L, C); break;
-    case 4: conv1d_silu_reverse_kernel<T, V, 4><<<grid, block, 0, st>>>(x, xp, w, bias, gy, gyp, gx, gxp, gw, gbias, L, C); break;
+    case 2: MpLaunch(grid, block, 0, st)(conv1d_silu_reverse_kernel<T, V, 2>, x, xp, w, bias, gy, gyp, gx, gxp, gw, gbias, L, C); break;
+    case 3: MpLaunch(grid, block, 0, st)(conv1d_silu_reverse_kernel<T, V, 3>, x, xp, w, bias, gy, gyp, gx, gxp, gw, gbias, L, C); break;
+    case 4: MpLaunch(grid, block, 0, st)(conv1d_silu_reverse_kernel<T, V, 4>, x, xp, w, bias, gy, gyp, gx, gxp, gw, gbias, L, C); break;
     default: MP_FATAL("causal_conv1d_silu_reverse: kernel width %llu is not supported (2, 3 or 4)", static_cast<unsigned long long>(width));
   }
   MP_LAUNCH_CHECK();
@@ -1517,9 +1541,9 @@ static void conv_tiled_forward(const void* x, len_t x_pitch, const void* w, cons
   cudaStream_t st = mp_stream(ctx);
   const __half* xh = static_cast<const __half*>(x); const __half* wh = static_cast<const __half*>(w);
   const __half* bh = static_cast<const __half*>(bias);
-  if (width == 4) conv1d_silu_tiled_kernel<4><<<grid, CT_THREADS, 0, st>>>(xh, x_pitch, wh, bh, sg, L, tp);
-  else if (width == 3) conv1d_silu_tiled_kernel<3><<<grid, CT_THREADS, 0, st>>>(xh, x_pitch, wh, bh, sg, L, tp);
-  else conv1d_silu_tiled_kernel<2><<<grid, CT_THREADS, 0, st>>>(xh, x_pitch, wh, bh, sg, L, tp);
+  if (width == 4) MpLaunch(grid, CT_THREADS, 0, st)(conv1d_silu_tiled_kernel<4>, xh, x_pitch, wh, bh, sg, L, tp);
+  else if (width == 3) MpLaunch(grid, CT_THREADS, 0, st)(conv1d_silu_tiled_kernel<3>, xh, x_pitch, wh, bh, sg, L, tp);
+  else MpLaunch(grid, CT_THREADS, 0, st)(conv1d_silu_tiled_kernel<2>, xh, x_pitch, wh, bh, sg, L, tp);
   MP_LAUNCH_CHECK();
 }
 static void conv_tiled_reverse(const void* x, len_t x_pitch, const void* w, const void* bias, const ConvSegs& sg, void* gx, len_t gx_pitch,
@@ -1543,7 +1567,7 @@ static void conv_tiled_reverse(const void* x, len_t x_pitch, const void* w, cons
     if (smem > 48 * 1024)                                                                                                           \
       MP_CUDA_CHECK(cudaFuncSetAttribute(conv1d_silu_reverse_tiled_kernel<WV, SK>, cudaFuncAttributeMaxDynamicSharedMemorySize,     \
                                          static_cast<int>(smem)));                                                                  \
-    conv1d_silu_reverse_tiled_kernel<WV, SK><<<grid, CT_THREADS, smem, st>>>(xh, x_pitch, wh, bh, sg, gxh, gx_pitch, gwf, gbf, L, tp); \
+    MpLaunch(grid, CT_THREADS, smem, st)(conv1d_silu_reverse_tiled_kernel<WV, SK>, xh, x_pitch, wh, bh, sg, gxh, gx_pitch, gwf, gbf, L, tp); \
   } while (0)
   if (skip) { if (width == 4) CONV_REV(4, true); else if (width == 3) CONV_REV(3, true); else CONV_REV(2, true); }
   else { if (width == 4) CONV_REV(4, false); else if (width == 3) CONV_REV(3, false); else CONV_REV(2, false); }
@@ -1697,7 +1721,7 @@ template <typename T>
 void softplus_bias_impl(const void* raw, len_t raw_pitch, const void* bias, void* out, len_t rows, len_t heads, StreamContext ctx) {
   if (rows == 0 || heads == 0) return;
   using A = typename Acc<T>::type;
-  softplus_bias_kernel<T><<<grid_for(rows * heads, 256), 256, 0, mp_stream(ctx)>>>(static_cast<const T*>(raw), raw_pitch, static_cast<const A*>(bias),
+  MpLaunch(grid_for(rows * heads, 256), 256, 0, mp_stream(ctx))(softplus_bias_kernel<T>, static_cast<const T*>(raw), raw_pitch, static_cast<const A*>(bias),
                                                                                static_cast<A*>(out), rows, static_cast<int>(heads));
   MP_LAUNCH_CHECK();
 }
@@ -1712,7 +1736,7 @@ void softplus_bias_reverse_impl(const void* raw, len_t raw_pitch, const void* bi
     size_t ctas = (rows + static_cast<size_t>(RR) * 4 - 1) / (static_cast<size_t>(RR) * 4);   // about four rows per thread
     const size_t cap = static_cast<size_t>(mp_sm_count(ctx)) * 8;
     if (ctas > cap) ctas = cap;
-    softplus_bias_reverse_heads_kernel<T><<<static_cast<unsigned>(ctas < 1 ? 1 : ctas), 256, 0, mp_stream(ctx)>>>(
+    MpLaunch(static_cast<unsigned>(ctas < 1 ? 1 : ctas), 256, 0, mp_stream(ctx))(softplus_bias_reverse_heads_kernel<T>, 
         static_cast<const T*>(raw), raw_pitch, static_cast<const A*>(bias), static_cast<const A*>(gdt), static_cast<T*>(graw), graw_pitch,
         static_cast<A*>(gbias), rows, static_cast<int>(heads), RR);
     MP_LAUNCH_CHECK();
@@ -1720,7 +1744,7 @@ void softplus_bias_reverse_impl(const void* raw, len_t raw_pitch, const void* bi
   }
   // few, fat CTAs: each one ends with `heads` global atomics
   const unsigned grid = grid_for((rows * heads + 15) / 16, 256);
-  softplus_bias_reverse_kernel<T><<<grid, 256, heads * sizeof(A), mp_stream(ctx)>>>(
+  MpLaunch(grid, 256, heads * sizeof(A), mp_stream(ctx))(softplus_bias_reverse_kernel<T>, 
       static_cast<const T*>(raw), raw_pitch, static_cast<const A*>(bias), static_cast<const A*>(gdt), static_cast<T*>(graw), graw_pitch,
       static_cast<A*>(gbias), rows, static_cast<int>(heads));
   MP_LAUNCH_CHECK();
@@ -1735,10 +1759,10 @@ void ssd_gate_impl(const void* y, const void* x, const void* D, const void* z, l
   const size_t width = heads * headdim;
   const bool v = headdim % PN == 0 && vec_ok<T>(z, z_pitch, width) && mp_aligned16(y) && mp_aligned16(x) && mp_aligned16(u);
   cudaStream_t st = mp_stream(ctx);
-  if (v) ssd_gate_kernel<T, PN><<<grid_for(rows * (width / PN), 256), 256, 0, st>>>(static_cast<const T*>(y), static_cast<const T*>(x), static_cast<const A*>(D),
+  if (v) MpLaunch(grid_for(rows * (width / PN), 256), 256, 0, st)(ssd_gate_kernel<T, PN>, static_cast<const T*>(y), static_cast<const T*>(x), static_cast<const A*>(D),
                                                                                  static_cast<const T*>(z), z_pitch, static_cast<T*>(u), rows,
                                                                                  static_cast<int>(heads), static_cast<int>(headdim));
-  else ssd_gate_kernel<T, 1><<<grid_for(rows * width, 256), 256, 0, st>>>(static_cast<const T*>(y), static_cast<const T*>(x), static_cast<const A*>(D),
+  else MpLaunch(grid_for(rows * width, 256), 256, 0, st)(ssd_gate_kernel<T, 1>, static_cast<const T*>(y), static_cast<const T*>(x), static_cast<const A*>(D),
                                                                         static_cast<const T*>(z), z_pitch, static_cast<T*>(u), rows,
                                                                         static_cast<int>(heads), static_cast<int>(headdim));
   MP_LAUNCH_CHECK();
@@ -1755,10 +1779,10 @@ void ssd_gate_reverse_impl(const void* y, const void* x, const void* D, const vo
                  mp_aligned16(x) && mp_aligned16(gu) && mp_aligned16(gy);
   cudaStream_t st = mp_stream(ctx);
   const size_t smem = heads * sizeof(A);
-  if (v) ssd_gate_reverse_kernel<T, PN><<<grid_for((rows * (width / PN) + 7) / 8, 256), 256, smem, st>>>(
+  if (v) MpLaunch(grid_for((rows * (width / PN) + 7) / 8, 256), 256, smem, st)(ssd_gate_reverse_kernel<T, PN>, 
         static_cast<const T*>(y), static_cast<const T*>(x), static_cast<const A*>(D), static_cast<const T*>(z), z_pitch, static_cast<const T*>(gu),
         static_cast<T*>(gy), static_cast<T*>(gz), gz_pitch, static_cast<A*>(gD), rows, static_cast<int>(heads), static_cast<int>(headdim));
-  else ssd_gate_reverse_kernel<T, 1><<<grid_for((rows * width + 7) / 8, 256), 256, smem, st>>>(
+  else MpLaunch(grid_for((rows * width + 7) / 8, 256), 256, smem, st)(ssd_gate_reverse_kernel<T, 1>, 
         static_cast<const T*>(y), static_cast<const T*>(x), static_cast<const A*>(D), static_cast<const T*>(z), z_pitch, static_cast<const T*>(gu),
         static_cast<T*>(gy), static_cast<T*>(gz), gz_pitch, static_cast<A*>(gD), rows, static_cast<int>(heads), static_cast<int>(headdim));
   MP_LAUNCH_CHECK();
@@ -1792,7 +1816,7 @@ void ssd_gate_rmsnorm_impl(const void* y, const void* x, const void* D, const vo
     if (v && width % 512 == 0 && width / 512 <= 4 && headdim % 8 == 0 && getenv("MP_GATED_NORM_ONE_WARP") == nullptr) {
       const unsigned g2 = grid_for(rows * 64, GN_THREADS);
 #define GN_FWD2(NPV)                                                                                                                 \
-  gate_rmsnorm_h2_kernel<NPV><<<g2, GN_THREADS, 0, st>>>(static_cast<const __half*>(y), static_cast<const __half*>(x),               \
+  MpLaunch(g2, GN_THREADS, 0, st)(gate_rmsnorm_h2_kernel<NPV>, static_cast<const __half*>(y), static_cast<const __half*>(x),               \
                                                          static_cast<const float*>(D), static_cast<const __half*>(z), z_pitch,      \
                                                          static_cast<const __half*>(gain), static_cast<float>(eps),                 \
                                                          static_cast<__half*>(out), static_cast<float*>(rstd), rows, static_cast<int>(headdim))
@@ -1809,7 +1833,7 @@ void ssd_gate_rmsnorm_impl(const void* y, const void* x, const void* D, const vo
   }
   const unsigned grid = grid_for(rows * 32, GN_THREADS);
 #define GN_FWD(VV, NPV)                                                                                                              \
-  gate_rmsnorm_kernel<T, VV, NPV><<<grid, GN_THREADS, 0, st>>>(static_cast<const T*>(y), static_cast<const T*>(x), static_cast<const A*>(D), \
+  MpLaunch(grid, GN_THREADS, 0, st)(gate_rmsnorm_kernel<T, VV, NPV>, static_cast<const T*>(y), static_cast<const T*>(x), static_cast<const A*>(D), \
                                                                static_cast<const T*>(z), z_pitch, static_cast<const T*>(gain), static_cast<A>(eps), \
                                                                static_cast<T*>(out), static_cast<A*>(rstd), rows, static_cast<int>(heads),   \
                                                                static_cast<int>(headdim))
@@ -1848,7 +1872,7 @@ void ssd_gate_rmsnorm_reverse_impl(const void* y, const void* x, const void* D, 
   if constexpr (std::is_same<T, __half>::value) {
     if (v && width % 512 == 0 && width / 512 <= 4 && headdim % 8 == 0 && getenv("MP_GATED_NORM_ONE_WARP") == nullptr) {
 #define GN_REV2(NPV)                                                                                                                 \
-  gate_rmsnorm_reverse_h2_kernel<NPV><<<grid, GN_THREADS, smem, st>>>(                                                               \
+  MpLaunch(grid, GN_THREADS, smem, st)(gate_rmsnorm_reverse_h2_kernel<NPV>, \
       static_cast<const __half*>(y), static_cast<const __half*>(x), static_cast<const float*>(D), static_cast<const __half*>(z), z_pitch, \
       static_cast<const __half*>(gain), static_cast<const float*>(rstd), static_cast<const __half*>(gout), static_cast<__half*>(gy),   \
       static_cast<__half*>(gz), gz_pitch, static_cast<float*>(gD), static_cast<float*>(scratch), rows, static_cast<int>(heads),        \
@@ -1868,7 +1892,7 @@ void ssd_gate_rmsnorm_reverse_impl(const void* y, const void* x, const void* D, 
     if (smem > 48 * 1024)                                                                                                            \
       MP_CUDA_CHECK(cudaFuncSetAttribute(gate_rmsnorm_reverse_kernel<T, VV, NPV>, cudaFuncAttributeMaxDynamicSharedMemorySize,       \
                                          static_cast<int>(smem)));                                                                   \
-    gate_rmsnorm_reverse_kernel<T, VV, NPV><<<grid, GN_THREADS, smem, st>>>(                                                         \
+    MpLaunch(grid, GN_THREADS, smem, st)(gate_rmsnorm_reverse_kernel<T, VV, NPV>, \
         static_cast<const T*>(y), static_cast<const T*>(x), static_cast<const A*>(D), static_cast<const T*>(z), z_pitch,             \
         static_cast<const T*>(gain), static_cast<const A*>(rstd), static_cast<const T*>(gout), static_cast<T*>(gy), static_cast<T*>(gz), \
         gz_pitch, static_cast<A*>(gD), static_cast<A*>(scratch), rows, static_cast<int>(heads), static_cast<int>(headdim));          \
@@ -1889,7 +1913,7 @@ void ssd_gate_rmsnorm_reverse_impl(const void* y, const void* x, const void* D, 
 #undef GN_REV
   MP_LAUNCH_CHECK();
   if (ggain != nullptr) {
-    gate_rmsnorm_fold_kernel<T><<<static_cast<unsigned>((width + 31) / 32), 1024, 0, st>>>(static_cast<const A*>(scratch), static_cast<int>(grid), width,
+    MpLaunch(static_cast<unsigned>((width + 31) / 32), 1024, 0, st)(gate_rmsnorm_fold_kernel<T>, static_cast<const A*>(scratch), static_cast<int>(grid), width,
                                                                                           static_cast<A>(alpha), static_cast<T*>(ggain));
     MP_LAUNCH_CHECK();
   }
@@ -1903,11 +1927,11 @@ void head_scale_accumulate_impl(const void* D, const void* gy, void* gx, len_t r
   const size_t width = heads * headdim;
   cudaStream_t st = mp_stream(ctx);
   if (headdim % PN == 0 && mp_aligned16(gy) && mp_aligned16(gx))
-    head_scale_accumulate_kernel<T, PN><<<grid_for(rows * (width / PN), 256), 256, 0, st>>>(static_cast<const A*>(D), static_cast<const T*>(gy),
+    MpLaunch(grid_for(rows * (width / PN), 256), 256, 0, st)(head_scale_accumulate_kernel<T, PN>, static_cast<const A*>(D), static_cast<const T*>(gy),
                                                                                         static_cast<T*>(gx), rows, static_cast<int>(heads),
                                                                                         static_cast<int>(headdim));
   else
-    head_scale_accumulate_kernel<T, 1><<<grid_for(rows * width, 256), 256, 0, st>>>(static_cast<const A*>(D), static_cast<const T*>(gy), static_cast<T*>(gx),
+    MpLaunch(grid_for(rows * width, 256), 256, 0, st)(head_scale_accumulate_kernel<T, 1>, static_cast<const A*>(D), static_cast<const T*>(gy), static_cast<T*>(gx),
                                                                                 rows, static_cast<int>(heads), static_cast<int>(headdim));
   MP_LAUNCH_CHECK();
 }
@@ -1921,14 +1945,14 @@ void ce_launch(const T* logits, const int* targets, double scale, typename Acc<T
       (glogits == nullptr || mp_aligned16(glogits)) && getenv("MP_CE_NO_BULK") == nullptr) {
     // (two CTAs per SM need the row below ~110 KB)
     MP_CUDA_CHECK(cudaFuncSetAttribute(cross_entropy_bulk_kernel<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024));
-    cross_entropy_bulk_kernel<T, V><<<static_cast<unsigned>(m), CE_THREADS, (row_bytes + 127) & ~size_t(127), st>>>(
+    MpLaunch(static_cast<unsigned>(m), CE_THREADS, (row_bytes + 127) & ~size_t(127), st)(cross_entropy_bulk_kernel<T, V>, 
         logits, targets, static_cast<A>(scale), loss, glogits, n, status);
   } else if (row_bytes <= 200 * 1024) {
     MP_CUDA_CHECK(cudaFuncSetAttribute(cross_entropy_kernel<T, V, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    cross_entropy_kernel<T, V, true><<<static_cast<unsigned>(m), CE_THREADS, (row_bytes + 15) & ~size_t(15), st>>>(logits, targets, static_cast<A>(scale), loss,
+    MpLaunch(static_cast<unsigned>(m), CE_THREADS, (row_bytes + 15) & ~size_t(15), st)(cross_entropy_kernel<T, V, true>, logits, targets, static_cast<A>(scale), loss,
                                                                                                                  glogits, n);
   } else {
-    cross_entropy_kernel<T, V, false><<<static_cast<unsigned>(m), CE_THREADS, 0, st>>>(logits, targets, static_cast<A>(scale), loss, glogits, n);
+    MpLaunch(static_cast<unsigned>(m), CE_THREADS, 0, st)(cross_entropy_kernel<T, V, false>, logits, targets, static_cast<A>(scale), loss, glogits, n);
   }
   MP_LAUNCH_CHECK();
 }
@@ -1948,7 +1972,7 @@ void cross_entropy_impl(const void* logits, const void* targets, double scale, v
 template <typename T>
 void neg_exp_impl(const void* src, void* dst, len_t n, StreamContext ctx) {
   if (n == 0) return;
-  neg_exp_kernel<T><<<grid_for(n, 256), 256, 0, mp_stream(ctx)>>>(static_cast<const T*>(src), static_cast<T*>(dst), n);
+  MpLaunch(grid_for(n, 256), 256, 0, mp_stream(ctx))(neg_exp_kernel<T>, static_cast<const T*>(src), static_cast<T*>(dst), n);
   MP_LAUNCH_CHECK();
 }
 
@@ -2018,9 +2042,9 @@ extern "C" void launch_convert_r16_r32(const void* src, void* dst, double beta, 
   if (n == 0) return;
   cudaStream_t st = mp_stream(ctx);
   if (n % 8 == 0 && mp_aligned16(src) && (reinterpret_cast<uintptr_t>(dst) & 31u) == 0)
-    convert_r16_r32_kernel<8><<<grid_for(n / 8, 512), 512, 0, st>>>(static_cast<const __half*>(src), static_cast<float*>(dst), static_cast<float>(beta), n);
+    MpLaunch(grid_for(n / 8, 512), 512, 0, st)(convert_r16_r32_kernel<8>, static_cast<const __half*>(src), static_cast<float*>(dst), static_cast<float>(beta), n);
   else
-    convert_r16_r32_kernel<1><<<grid_for(n, 512), 512, 0, st>>>(static_cast<const __half*>(src), static_cast<float*>(dst), static_cast<float>(beta), n);
+    MpLaunch(grid_for(n, 512), 512, 0, st)(convert_r16_r32_kernel<1>, static_cast<const __half*>(src), static_cast<float*>(dst), static_cast<float>(beta), n);
   MP_LAUNCH_CHECK();
 }
 
@@ -2028,9 +2052,9 @@ extern "C" void launch_convert_r32_r16(const void* src, void* dst, len_t n, Stre
   if (n == 0) return;
   cudaStream_t st = mp_stream(ctx);
   if (n % 8 == 0 && mp_aligned16(dst) && (reinterpret_cast<uintptr_t>(src) & 31u) == 0)
-    convert_r32_r16_kernel<8><<<grid_for(n / 8, 512), 512, 0, st>>>(static_cast<const float*>(src), static_cast<__half*>(dst), n);
+    MpLaunch(grid_for(n / 8, 512), 512, 0, st)(convert_r32_r16_kernel<8>, static_cast<const float*>(src), static_cast<__half*>(dst), n);
   else
-    convert_r32_r16_kernel<1><<<grid_for(n, 512), 512, 0, st>>>(static_cast<const float*>(src), static_cast<__half*>(dst), n);
+    MpLaunch(grid_for(n, 512), 512, 0, st)(convert_r32_r16_kernel<1>, static_cast<const float*>(src), static_cast<__half*>(dst), n);
   MP_LAUNCH_CHECK();
 }
 
@@ -2039,7 +2063,7 @@ extern "C" void launch_convert_r32_r16(const void* src, void* dst, len_t n, Stre
 // launch_adam_tick advances t and refreshes the two corrections; it runs on the stream like any launcher (one
 // thread), so a step that is replayed from a captured graph still sees its own step number.
 extern "C" void launch_adam_tick(void* tick, double beta1, double beta2, StreamContext ctx) {
-  adam_tick_kernel<<<1, 1, 0, mp_stream(ctx)>>>(static_cast<AdamTick*>(tick), static_cast<float>(beta1), static_cast<float>(beta2));
+  MpLaunch(1, 1, 0, mp_stream(ctx))(adam_tick_kernel, static_cast<AdamTick*>(tick), static_cast<float>(beta1), static_cast<float>(beta2));
   MP_LAUNCH_CHECK();
 }
 
@@ -2054,12 +2078,12 @@ extern "C" void launch_adam_mixed_r32(void* w32, void* w16, const void* g32, con
                    ((reinterpret_cast<uintptr_t>(w32) | reinterpret_cast<uintptr_t>(g32) | reinterpret_cast<uintptr_t>(m) |
                      reinterpret_cast<uintptr_t>(v)) & 31u) == 0;
   if (vec)
-    adam_mixed_kernel<8><<<grid_for(n / 8, 512), 512, 0, st>>>(static_cast<float*>(w32), static_cast<__half*>(w16), static_cast<const float*>(g32),
+    MpLaunch(grid_for(n / 8, 512), 512, 0, st)(adam_mixed_kernel<8>, static_cast<float*>(w32), static_cast<__half*>(w16), static_cast<const float*>(g32),
                                                              static_cast<const __half*>(g16), static_cast<float*>(m), static_cast<float*>(v),
                                                              static_cast<float>(lr), static_cast<float>(beta1), static_cast<float>(beta2),
                                                              static_cast<float>(eps), static_cast<float>(grad_scale), static_cast<AdamTick*>(tick), n);
   else
-    adam_mixed_kernel<1><<<grid_for(n, 512), 512, 0, st>>>(static_cast<float*>(w32), static_cast<__half*>(w16), static_cast<const float*>(g32),
+    MpLaunch(grid_for(n, 512), 512, 0, st)(adam_mixed_kernel<1>, static_cast<float*>(w32), static_cast<__half*>(w16), static_cast<const float*>(g32),
                                                          static_cast<const __half*>(g16), static_cast<float*>(m), static_cast<float*>(v),
                                                          static_cast<float>(lr), static_cast<float>(beta1), static_cast<float>(beta2),
                                                          static_cast<float>(eps), static_cast<float>(grad_scale), static_cast<AdamTick*>(tick), n);

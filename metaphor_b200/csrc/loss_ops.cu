@@ -22,6 +22,7 @@ template <typename T, bool BCE>
 __global__ void __launch_bounds__(LOSS_THREADS) loss_partial_kernel(const T* __restrict__ x, T* __restrict__ grad,
                                                                     const T* __restrict__ trg,
                                                                     typename Acc<T>::type* __restrict__ scratch, size_t n) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   __shared__ A red[LOSS_THREADS / 32];
   const A inv_n = A(1) / static_cast<A>(n);
@@ -58,6 +59,7 @@ __global__ void __launch_bounds__(LOSS_THREADS) loss_partial_kernel(const T* __r
 template <typename A>
 __global__ void __launch_bounds__(LOSS_THREADS) loss_fold_kernel(const A* __restrict__ scratch, A* __restrict__ redux, size_t parts,
                                                                  A inv_n) {
+  mp_grid_dependency();
   __shared__ A red[LOSS_THREADS];
   A s = A(0);
   for (size_t i = threadIdx.x; i < parts; i += LOSS_THREADS) s += scratch[i];   // fixed order per thread
@@ -77,11 +79,11 @@ void loss_launch(const void* x, void* grad, const void* trg, void* scratch, void
   if (scratch == nullptr) MP_FATAL("loss: scratch must not be NULL (n / 4096 + 2 accumulator-typed slots)");
   const size_t parts = (n + LOSS_PER_CTA - 1) / LOSS_PER_CTA;
   cudaStream_t st = mp_stream(ctx);
-  loss_partial_kernel<T, BCE><<<static_cast<unsigned>(parts), LOSS_THREADS, 0, st>>>(static_cast<const T*>(x), static_cast<T*>(grad),
+  MpLaunch(static_cast<unsigned>(parts), LOSS_THREADS, 0, st)(loss_partial_kernel<T, BCE>, static_cast<const T*>(x), static_cast<T*>(grad),
                                                                                     static_cast<const T*>(trg), static_cast<A*>(scratch), n);
   MP_LAUNCH_CHECK();
   if (redux != nullptr) {
-    loss_fold_kernel<A><<<1, LOSS_THREADS, 0, st>>>(static_cast<const A*>(scratch), static_cast<A*>(redux), parts, A(1) / static_cast<A>(n));
+    MpLaunch(1, LOSS_THREADS, 0, st)(loss_fold_kernel<A>, static_cast<const A*>(scratch), static_cast<A*>(redux), parts, A(1) / static_cast<A>(n));
     MP_LAUNCH_CHECK();
   }
 }
@@ -99,6 +101,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) momentum_kernel(T* __restrict__ w, const T* __restrict__ g, T* __restrict__ m,
                                                        typename Acc<T>::type rate, typename Acc<T>::type alpha,
                                                        typename Acc<T>::type lo, typename Acc<T>::type hi, size_t n) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   constexpr int PN = Pack<T>::N;
   const size_t nvec = n / PN;
@@ -141,7 +144,7 @@ void momentum_impl(void* w, const void* g, void* m, double rate, double alpha, d
   const size_t work = (n + Pack<T>::N - 1) / Pack<T>::N;
   size_t grid = (work + 255) / 256;
   if (grid > (1u << 30)) grid = 1u << 30;
-  momentum_kernel<T><<<static_cast<unsigned>(grid), 256, 0, mp_stream(ctx)>>>(static_cast<T*>(w), static_cast<const T*>(g), static_cast<T*>(m),
+  MpLaunch(static_cast<unsigned>(grid), 256, 0, mp_stream(ctx))(momentum_kernel<T>, static_cast<T*>(w), static_cast<const T*>(g), static_cast<T*>(m),
                                                                           static_cast<A>(rate), static_cast<A>(alpha), static_cast<A>(lo),
                                                                           static_cast<A>(hi), n);
   MP_LAUNCH_CHECK();

@@ -22,6 +22,7 @@ template <typename T> struct TpTile { static constexpr int value = sizeof(T) == 
 template <typename T, bool VL, bool VS, bool BLEND>
 __global__ void __launch_bounds__(TP_THREADS) transpose_kernel(const T* __restrict__ src, T* dst,
                                                                typename Acc<T>::type alpha, size_t row, size_t col) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   constexpr int PN = Pack<T>::N;
   constexpr int TP_TILE = TpTile<T>::value;
@@ -94,8 +95,8 @@ __global__ void __launch_bounds__(TP_THREADS) transpose_kernel(const T* __restri
 template <typename T, bool VL, bool VS>
 void transpose_dispatch(const T* src, T* dst, double alpha, size_t row, size_t col, dim3 grid, cudaStream_t st) {
   using A = typename Acc<T>::type;
-  if (alpha == 0.0) transpose_kernel<T, VL, VS, false><<<grid, TP_THREADS, 0, st>>>(src, dst, A(0), row, col);
-  else transpose_kernel<T, VL, VS, true><<<grid, TP_THREADS, 0, st>>>(src, dst, static_cast<A>(alpha), row, col);
+  if (alpha == 0.0) MpLaunch(grid, TP_THREADS, 0, st)(transpose_kernel<T, VL, VS, false>, src, dst, A(0), row, col);
+  else MpLaunch(grid, TP_THREADS, 0, st)(transpose_kernel<T, VL, VS, true>, src, dst, static_cast<A>(alpha), row, col);
 }
 
 // ------------------------------- row sums ---------------------------------
@@ -105,6 +106,7 @@ void transpose_dispatch(const T* src, T* dst, double alpha, size_t row, size_t c
 template <typename T, int GROUP, bool VEC>
 __global__ void __launch_bounds__(256) row_sum_kernel(const T* __restrict__ src, T* dst, typename Acc<T>::type alpha,
                                                       bool blend, size_t m, size_t n) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   constexpr int PN = Pack<T>::N;
   static_assert(GROUP == 32, "one warp per row");
@@ -144,6 +146,7 @@ __global__ void __launch_bounds__(256) row_sum_kernel(const T* __restrict__ src,
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256) row_sum_cta_kernel(const T* __restrict__ src, T* dst, typename Acc<T>::type alpha,
                                                           bool blend, size_t m, size_t n) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   constexpr int PN = Pack<T>::N;
   __shared__ A red[32];
@@ -188,6 +191,7 @@ template <typename T, bool VEC>
 __global__ void __launch_bounds__(256) col_sum_kernel(const T* __restrict__ src, T* dst, typename Acc<T>::type* partial,
                                                       typename Acc<T>::type alpha, bool blend, size_t m, size_t n,
                                                       size_t rows_per_split) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   constexpr int W = VEC ? Pack<T>::N : 1;
   __shared__ A sm[8][32 * W + 1];
@@ -237,6 +241,7 @@ __global__ void __launch_bounds__(256) col_sum_kernel(const T* __restrict__ src,
 template <typename T>
 __global__ void __launch_bounds__(256) col_sum_fold_kernel(const typename Acc<T>::type* __restrict__ partial, T* dst,
                                                            typename Acc<T>::type alpha, bool blend, size_t n, int splits) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   const size_t col = static_cast<size_t>(blockIdx.x) * 256 + threadIdx.x;
   if (col >= n) return;
@@ -250,6 +255,7 @@ __global__ void __launch_bounds__(256) col_sum_fold_kernel(const typename Acc<T>
 template <typename T, bool BY_ROW, bool VEC, bool BLEND>
 __global__ void __launch_bounds__(256) broadcast_kernel(const T* __restrict__ src, T* dst, typename Acc<T>::type alpha,
                                                         size_t m, size_t n) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   constexpr int PN = Pack<T>::N;
   const size_t total = m * n;
@@ -312,11 +318,11 @@ void broadcast_launch(const void* src_, void* dst_, double alpha, len_t m, len_t
   const A a = static_cast<A>(alpha);
   const unsigned g = static_cast<unsigned>(grid);
   if (vec) {
-    if (alpha == 0.0) broadcast_kernel<T, BY_ROW, true, false><<<g, 256, 0, st>>>(src, dst, a, m, n);
-    else broadcast_kernel<T, BY_ROW, true, true><<<g, 256, 0, st>>>(src, dst, a, m, n);
+    if (alpha == 0.0) MpLaunch(g, 256, 0, st)(broadcast_kernel<T, BY_ROW, true, false>, src, dst, a, m, n);
+    else MpLaunch(g, 256, 0, st)(broadcast_kernel<T, BY_ROW, true, true>, src, dst, a, m, n);
   } else {
-    if (alpha == 0.0) broadcast_kernel<T, BY_ROW, false, false><<<g, 256, 0, st>>>(src, dst, a, m, n);
-    else broadcast_kernel<T, BY_ROW, false, true><<<g, 256, 0, st>>>(src, dst, a, m, n);
+    if (alpha == 0.0) MpLaunch(g, 256, 0, st)(broadcast_kernel<T, BY_ROW, false, false>, src, dst, a, m, n);
+    else MpLaunch(g, 256, 0, st)(broadcast_kernel<T, BY_ROW, false, true>, src, dst, a, m, n);
   }
   MP_LAUNCH_CHECK();
 }
@@ -364,12 +370,12 @@ static void reduce_ij_i_impl(const void* src_, void* dst_, double alpha, len_t m
   cudaStream_t st = mp_stream(ctx);
   if (n * sizeof(T) <= 4096) {  // short rows: one warp each, 8 rows per CTA
     size_t grid = (m + 7) / 8; if (grid > cap) grid = cap;
-    if (vec) row_sum_kernel<T, 32, true><<<static_cast<unsigned>(grid), 256, 0, st>>>(src, dst, a, blend, m, n);
-    else row_sum_kernel<T, 32, false><<<static_cast<unsigned>(grid), 256, 0, st>>>(src, dst, a, blend, m, n);
+    if (vec) MpLaunch(static_cast<unsigned>(grid), 256, 0, st)(row_sum_kernel<T, 32, true>, src, dst, a, blend, m, n);
+    else MpLaunch(static_cast<unsigned>(grid), 256, 0, st)(row_sum_kernel<T, 32, false>, src, dst, a, blend, m, n);
   } else {
     size_t grid = m; if (grid > cap) grid = cap;
-    if (vec) row_sum_cta_kernel<T, true><<<static_cast<unsigned>(grid), 256, 0, st>>>(src, dst, a, blend, m, n);
-    else row_sum_cta_kernel<T, false><<<static_cast<unsigned>(grid), 256, 0, st>>>(src, dst, a, blend, m, n);
+    if (vec) MpLaunch(static_cast<unsigned>(grid), 256, 0, st)(row_sum_cta_kernel<T, true>, src, dst, a, blend, m, n);
+    else MpLaunch(static_cast<unsigned>(grid), 256, 0, st)(row_sum_cta_kernel<T, false>, src, dst, a, blend, m, n);
   }
   MP_LAUNCH_CHECK();
 }
@@ -404,11 +410,11 @@ static void reduce_ij_j_impl(const void* src_, void* dst_, double alpha, len_t m
   splits = m == 0 ? 1 : (m + rows_per_split - 1) / rows_per_split;
   A* partial = splits > 1 ? static_cast<A*>(state->workspace) : nullptr;
   const dim3 grid(static_cast<unsigned>(strips), static_cast<unsigned>(splits));
-  if (vec) col_sum_kernel<T, true><<<grid, 256, 0, st>>>(src, dst, partial, a, blend, m, n, rows_per_split);
-  else col_sum_kernel<T, false><<<grid, 256, 0, st>>>(src, dst, partial, a, blend, m, n, rows_per_split);
+  if (vec) MpLaunch(grid, 256, 0, st)(col_sum_kernel<T, true>, src, dst, partial, a, blend, m, n, rows_per_split);
+  else MpLaunch(grid, 256, 0, st)(col_sum_kernel<T, false>, src, dst, partial, a, blend, m, n, rows_per_split);
   MP_LAUNCH_CHECK();
   if (splits > 1) {
-    col_sum_fold_kernel<T><<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(partial, dst, a, blend, n,
+    MpLaunch(static_cast<unsigned>((n + 255) / 256), 256, 0, st)(col_sum_fold_kernel<T>, partial, dst, a, blend, n,
                                                                                    static_cast<int>(splits));
     MP_LAUNCH_CHECK();
   }

@@ -61,6 +61,7 @@ __device__ __forceinline__ void store_block_rows(float* stage, const float* r, i
 template <typename T>
 __global__ void __launch_bounds__(256) gemm_fold_kernel(const float* __restrict__ partial, int ksplit, int M, int N, int ld, float alpha,
                                                         const T* __restrict__ bias, float beta, T* c, size_t ldc, size_t bias_pitch) {
+  mp_grid_dependency();
   const size_t mn = static_cast<size_t>(M) * ld;
   const size_t i0 = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) * 4;
   if (i0 >= mn) return;
@@ -156,7 +157,7 @@ CUtensorMap make_store_map(void* base, size_t rows, size_t cols, size_t ld, bool
 template <typename T>
 void launch_fold(const GemmArgs& args, cudaStream_t st) {
   const size_t units = static_cast<size_t>(args.M) * args.partial_ld / 4;
-  gemm_fold_kernel<T><<<static_cast<unsigned>((units + 255) / 256), 256, 0, st>>>(args.partial, args.ksplit, args.M, args.N, args.partial_ld,
+  MpLaunch(static_cast<unsigned>((units + 255) / 256), 256, 0, st)(gemm_fold_kernel<T>, args.partial, args.ksplit, args.M, args.N, args.partial_ld,
                                                                                 args.alpha, static_cast<const T*>(args.bias), args.beta,
                                                                                 static_cast<T*>(args.c), args.ldc, args.bias_pitch);
   MP_LAUNCH_CHECK();

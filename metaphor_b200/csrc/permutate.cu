@@ -36,6 +36,7 @@ template <typename T, typename I, bool VEC, bool BLEND>
 __global__ void __launch_bounds__(PERM_THREADS) permute_rows_kernel(const T* __restrict__ src, T* dst, typename Acc<T>::type alpha,
                                                                     const PermDims o, I pieces, I segs, size_t inner_units,
                                                                     unsigned seg_units, int group_log2) {
+  mp_grid_dependency();
   // A row of `inner_units` units (16-byte packs when VEC, else elements) is cut into `segs` pieces of `seg_units`.
   // A warp takes 32 consecutive pieces: every lane decodes ONE piece (the index arithmetic costs more than the
   // copy of a short row), then the warp walks the 32 pieces with 2^group_log2 lanes per piece, the offsets
@@ -165,6 +166,7 @@ __global__ void __launch_bounds__(PERM_THREADS) permute_tiles_kernel(const T* __
                                                                      const PermDims batch, size_t n_s, size_t n_d, size_t s_pitch,
                                                                      size_t d_pitch, unsigned tiles_s, unsigned tiles_d,
                                                                      const PermSplit sp) {
+  mp_grid_dependency();
   constexpr int PN = Pack<T>::N;
   constexpr int TILE = PermTile<T>::value;
   constexpr int VPR = TILE / PN;
@@ -251,6 +253,7 @@ __global__ void __launch_bounds__(PERM_THREADS, 5) permute_tiles_h2_kernel(const
                                                                         const PermDims batch, size_t n_s, size_t n_d, size_t s_pitch,
                                                                         size_t d_pitch, unsigned tiles_s, unsigned tiles_d,
                                                                         const PermSplit sp) {
+  mp_grid_dependency();
   constexpr int TILE = 128, PN = 8, VPR = TILE / PN;
   __shared__ __align__(16) uint32_t tile[TILE][TILE / 2];   // tile[s][(d / 2) ^ swz(s)] = (value at d, value at d + 1)
   size_t s0, d0, sbase, dbase;
@@ -322,9 +325,9 @@ void rows_launch(const T* src, T* dst, double alpha, const PermDims& o, size_t p
                  int glog, unsigned grid, cudaStream_t st) {
   using A = typename Acc<T>::type;
   if (alpha == 0.0)
-    permute_rows_kernel<T, I, VEC, false><<<grid, PERM_THREADS, 0, st>>>(src, dst, A(0), o, static_cast<I>(pieces), static_cast<I>(segs), units, seg_units, glog);
+    MpLaunch(grid, PERM_THREADS, 0, st)(permute_rows_kernel<T, I, VEC, false>, src, dst, A(0), o, static_cast<I>(pieces), static_cast<I>(segs), units, seg_units, glog);
   else
-    permute_rows_kernel<T, I, VEC, true><<<grid, PERM_THREADS, 0, st>>>(src, dst, static_cast<A>(alpha), o, static_cast<I>(pieces), static_cast<I>(segs), units, seg_units, glog);
+    MpLaunch(grid, PERM_THREADS, 0, st)(permute_rows_kernel<T, I, VEC, true>, src, dst, static_cast<A>(alpha), o, static_cast<I>(pieces), static_cast<I>(segs), units, seg_units, glog);
 }
 
 template <typename T, bool VL, bool VS>
@@ -332,9 +335,9 @@ void tiles_launch(const T* src, T* dst, double alpha, const PermDims& b, size_t 
                   unsigned tiles_s, unsigned tiles_d, const PermSplit& sp, unsigned grid, cudaStream_t st) {
   using A = typename Acc<T>::type;
   if (alpha == 0.0)
-    permute_tiles_kernel<T, VL, VS, false><<<grid, PERM_THREADS, 0, st>>>(src, dst, A(0), b, n_s, n_d, s_pitch, d_pitch, tiles_s, tiles_d, sp);
+    MpLaunch(grid, PERM_THREADS, 0, st)(permute_tiles_kernel<T, VL, VS, false>, src, dst, A(0), b, n_s, n_d, s_pitch, d_pitch, tiles_s, tiles_d, sp);
   else
-    permute_tiles_kernel<T, VL, VS, true><<<grid, PERM_THREADS, 0, st>>>(src, dst, static_cast<A>(alpha), b, n_s, n_d, s_pitch, d_pitch, tiles_s, tiles_d, sp);
+    MpLaunch(grid, PERM_THREADS, 0, st)(permute_tiles_kernel<T, VL, VS, true>, src, dst, static_cast<A>(alpha), b, n_s, n_d, s_pitch, d_pitch, tiles_s, tiles_d, sp);
 }
 
 }  // namespace
@@ -428,8 +431,8 @@ static void permutate_run(const T* src, T* dst, double alpha, const size_t* n, c
   const unsigned ts = static_cast<unsigned>(tiles_s), td = static_cast<unsigned>(tiles_d);
   if constexpr (std::is_same<T, __half>::value) {
     if (vl && vs) {
-      if (alpha == 0.0) permute_tiles_h2_kernel<false><<<grid, PERM_THREADS, 0, st>>>(src, dst, 0.f, b, n_s, n_d, s_pitch, d_pitch, ts, td, sp);
-      else permute_tiles_h2_kernel<true><<<grid, PERM_THREADS, 0, st>>>(src, dst, static_cast<float>(alpha), b, n_s, n_d, s_pitch, d_pitch, ts, td, sp);
+      if (alpha == 0.0) MpLaunch(grid, PERM_THREADS, 0, st)(permute_tiles_h2_kernel<false>, src, dst, 0.f, b, n_s, n_d, s_pitch, d_pitch, ts, td, sp);
+      else MpLaunch(grid, PERM_THREADS, 0, st)(permute_tiles_h2_kernel<true>, src, dst, static_cast<float>(alpha), b, n_s, n_d, s_pitch, d_pitch, ts, td, sp);
       MP_LAUNCH_CHECK();
       return;
     }

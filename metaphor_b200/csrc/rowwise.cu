@@ -69,6 +69,7 @@ __device__ __forceinline__ void group_sum2(A& a, A& b, A* smem) {
 // ------------------------------- softmax ----------------------------------
 template <typename T, int GROUP, int PPT, bool FULL>
 __global__ void __launch_bounds__(RowCfg<GROUP>::THREADS) softmax_fwd_kernel(const T* x, T* y, size_t m, size_t n) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   constexpr int PN = Pack<T>::N;
   constexpr int ROWS = RowCfg<GROUP>::ROWS;
@@ -122,6 +123,7 @@ __global__ void __launch_bounds__(RowCfg<GROUP>::THREADS) softmax_fwd_kernel(con
 template <typename T, int GROUP, int PPT, bool FULL, bool BLEND>
 __global__ void __launch_bounds__(RowCfg<GROUP>::THREADS) softmax_rev_kernel(const T* y, const T* gy, T* gx,
                                                                             typename Acc<T>::type alpha, size_t m, size_t n) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   constexpr int PN = Pack<T>::N;
   constexpr int ROWS = RowCfg<GROUP>::ROWS;
@@ -176,6 +178,7 @@ __global__ void __launch_bounds__(RowCfg<GROUP>::THREADS) rmsnorm_fwd_kernel(con
                                                                             typename Acc<T>::type eps, T* y,
                                                                             typename Acc<T>::type* __restrict__ rstd_out,
                                                                             size_t m, size_t n) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   constexpr int PN = Pack<T>::N;
   constexpr int ROWS = RowCfg<GROUP>::ROWS;
@@ -345,6 +348,7 @@ __global__ void __launch_bounds__(RowCfg<GROUP>::THREADS) rmsnorm_rev_kernel(
     const T* x, const T* __restrict__ gain, const typename Acc<T>::type* __restrict__ rstd_in, const T* gy,
     typename Acc<T>::type eps, T* gx, typename Acc<T>::type alpha, typename Acc<T>::type* __restrict__ partial, size_t m,
     size_t n, size_t rows_per_cta) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   constexpr int PN = Pack<T>::N;
   constexpr int ROWS = RowCfg<GROUP>::ROWS;
@@ -418,6 +422,7 @@ template <typename T, int NP, bool BLEND>
 __global__ void __launch_bounds__(WROW_THREADS, 3) rmsnorm_rev_warp_kernel(
     const T* x, const T* __restrict__ gain, const typename Acc<T>::type* __restrict__ rstd_in, const T* gy,
     typename Acc<T>::type eps, T* gx, typename Acc<T>::type alpha, typename Acc<T>::type* __restrict__ partial, size_t m) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   constexpr int PN = Pack<T>::N;
   constexpr size_t n = static_cast<size_t>(NP) * 32 * PN;
@@ -518,6 +523,7 @@ template <int NP, bool BLEND>
 __global__ void __launch_bounds__(WROWH_THREADS, 2) rmsnorm_rev_warp_h_kernel(const __half* x, const __half* __restrict__ gain,
                                                                          const float* __restrict__ rstd_in, const __half* gy, __half* gx,
                                                                          float alpha, float* __restrict__ partial, size_t m) {
+  mp_grid_dependency();
   constexpr size_t n = static_cast<size_t>(NP) * 256;
   __shared__ float cols[NP * 256];
   for (int i = threadIdx.x; i < NP * 256; i += WROWH_THREADS) cols[i] = 0.f;
@@ -604,6 +610,7 @@ __global__ void __launch_bounds__(STG_THREADS, StgOcc<T, PPT>::value) rmsnorm_re
     const T* x, const T* __restrict__ gain, const typename Acc<T>::type* __restrict__ rstd_in, const T* gy,
     typename Acc<T>::type eps, T* gx, typename Acc<T>::type alpha, typename Acc<T>::type* __restrict__ partial,
     size_t m, size_t n, size_t rows_per_cta, int stages, uint32_t* status) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   constexpr int PN = Pack<T>::N;
   constexpr int GROUP = STG_THREADS;
@@ -679,6 +686,7 @@ __global__ void __launch_bounds__(STG_THREADS, StgOcc<T, PPT>::value) rmsnorm_re
 template <typename T>
 __global__ void __launch_bounds__(1024) rmsnorm_fold_kernel(const typename Acc<T>::type* __restrict__ partial, T* ggain,
                                                             typename Acc<T>::type alpha, bool blend, size_t n, size_t slots) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   __shared__ A sm[32][33];
   const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5, slices = blockDim.x >> 5;
@@ -707,6 +715,7 @@ constexpr int FOLD_SPLITS = 16;
 template <typename A>
 __global__ void __launch_bounds__(256) rmsnorm_fold_stage1_kernel(const A* __restrict__ partial, A* __restrict__ partial2,
                                                                   size_t n, size_t slots) {
+  mp_grid_dependency();
   constexpr int W = 16 / sizeof(A);
   __shared__ A sm[8][32 * W + 1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -756,6 +765,7 @@ constexpr int GEN_THREADS = 256;
 
 template <typename T>
 __global__ void __launch_bounds__(GEN_THREADS) softmax_fwd_generic(const T* x, T* y, size_t m, size_t n) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   __shared__ A red[64];
   for (size_t row = blockIdx.x; row < m; row += gridDim.x) {
@@ -775,6 +785,7 @@ __global__ void __launch_bounds__(GEN_THREADS) softmax_fwd_generic(const T* x, T
 template <typename T>
 __global__ void __launch_bounds__(GEN_THREADS) softmax_rev_generic(const T* y, const T* gy, T* gx, typename Acc<T>::type alpha,
                                                                    bool blend, size_t m, size_t n) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   __shared__ A red[64];
   for (size_t row = blockIdx.x; row < m; row += gridDim.x) {
@@ -793,6 +804,7 @@ __global__ void __launch_bounds__(GEN_THREADS) softmax_rev_generic(const T* y, c
 template <typename T>
 __global__ void __launch_bounds__(GEN_THREADS) rmsnorm_fwd_generic(const T* x, const T* gain, typename Acc<T>::type eps, T* y,
                                                                    typename Acc<T>::type* rstd_out, size_t m, size_t n) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   __shared__ A red[64];
   const A inv_n = A(1) / static_cast<A>(n);
@@ -815,6 +827,7 @@ __global__ void __launch_bounds__(GEN_THREADS) rmsnorm_rev_generic(const T* x, c
                                                                    typename Acc<T>::type alpha, bool blend,
                                                                    typename Acc<T>::type* partial, size_t m, size_t n,
                                                                    size_t rows_per_cta) {
+  mp_grid_dependency();
   using A = typename Acc<T>::type;
   __shared__ A red[64];
   const A inv_n = A(1) / static_cast<A>(n);
@@ -1008,9 +1021,9 @@ static void softmax_ij_j_impl(const void* src_, void* dst_, len_t m, len_t n, St
   cudaStream_t st = mp_stream(ctx);
   const unsigned grid = static_cast<unsigned>(row_grid(p, m, mp_sm_count(ctx), 0));
   if (p.generic) {
-    softmax_fwd_generic<T><<<grid, GEN_THREADS, 0, st>>>(src, dst, m, n);
+    MpLaunch(grid, GEN_THREADS, 0, st)(softmax_fwd_generic<T>, src, dst, m, n);
   } else {
-#define CALL(G, P, F) softmax_fwd_kernel<T, G, P, F><<<grid, RowCfg<G>::THREADS, 0, st>>>(src, dst, m, n)
+#define CALL(G, P, F) MpLaunch(grid, RowCfg<G>::THREADS, 0, st)(softmax_fwd_kernel<T, G, P, F>, src, dst, m, n)
     MP_ROW_DISPATCH(p, CALL);
 #undef CALL
   }
@@ -1031,13 +1044,13 @@ static void softmax_ij_j_reverse_impl(const void* y_, const void* gy_, void* gx_
   const bool blend = alpha != 0.0;
   const unsigned grid = static_cast<unsigned>(row_grid(p, m, mp_sm_count(ctx), 0));
   if (p.generic) {
-    softmax_rev_generic<T><<<grid, GEN_THREADS, 0, st>>>(y, gy, gx, a, blend, m, n);
+    MpLaunch(grid, GEN_THREADS, 0, st)(softmax_rev_generic<T>, y, gy, gx, a, blend, m, n);
   } else if (blend) {
-#define CALL(G, P, F) softmax_rev_kernel<T, G, P, F, true><<<grid, RowCfg<G>::THREADS, 0, st>>>(y, gy, gx, a, m, n)
+#define CALL(G, P, F) MpLaunch(grid, RowCfg<G>::THREADS, 0, st)(softmax_rev_kernel<T, G, P, F, true>, y, gy, gx, a, m, n)
     MP_ROW_DISPATCH(p, CALL);
 #undef CALL
   } else {
-#define CALL(G, P, F) softmax_rev_kernel<T, G, P, F, false><<<grid, RowCfg<G>::THREADS, 0, st>>>(y, gy, gx, a, m, n)
+#define CALL(G, P, F) MpLaunch(grid, RowCfg<G>::THREADS, 0, st)(softmax_rev_kernel<T, G, P, F, false>, y, gy, gx, a, m, n)
     MP_ROW_DISPATCH(p, CALL);
 #undef CALL
   }
@@ -1058,9 +1071,9 @@ static void rmsnorm_ij_j_impl(const void* x_, const void* gain_, double eps, voi
   const A e = static_cast<A>(eps);
   const unsigned grid = static_cast<unsigned>(row_grid(p, m, mp_sm_count(ctx), 0));
   if (p.generic) {
-    rmsnorm_fwd_generic<T><<<grid, GEN_THREADS, 0, st>>>(x, gain, e, y, rstd, m, n);
+    MpLaunch(grid, GEN_THREADS, 0, st)(rmsnorm_fwd_generic<T>, x, gain, e, y, rstd, m, n);
   } else {
-#define CALL(G, P, F) rmsnorm_fwd_kernel<T, G, P, F><<<grid, RowCfg<G>::THREADS, 0, st>>>(x, gain, e, y, rstd, m, n)
+#define CALL(G, P, F) MpLaunch(grid, RowCfg<G>::THREADS, 0, st)(rmsnorm_fwd_kernel<T, G, P, F>, x, gain, e, y, rstd, m, n)
     MP_ROW_DISPATCH(p, CALL);
 #undef CALL
   }
@@ -1120,8 +1133,8 @@ static void rmsnorm_ij_j_reverse_impl(const void* x_, const void* gain_, const v
         slots = grid;
 #define WROWH(NPV)                                                                                                     \
   do {                                                                                                                 \
-    if (blend) rmsnorm_rev_warp_h_kernel<NPV, true><<<grid, WROWH_THREADS, 0, st>>>(x, gain, rstd, gy, gx, a, partial, m);   \
-    else rmsnorm_rev_warp_h_kernel<NPV, false><<<grid, WROWH_THREADS, 0, st>>>(x, gain, rstd, gy, gx, a, partial, m);        \
+    if (blend) MpLaunch(grid, WROWH_THREADS, 0, st)(rmsnorm_rev_warp_h_kernel<NPV, true>, x, gain, rstd, gy, gx, a, partial, m);   \
+    else MpLaunch(grid, WROWH_THREADS, 0, st)(rmsnorm_rev_warp_h_kernel<NPV, false>, x, gain, rstd, gy, gx, a, partial, m);        \
   } while (0)
         switch (n / 256) {
           case 1: WROWH(1); break;
@@ -1138,8 +1151,8 @@ static void rmsnorm_ij_j_reverse_impl(const void* x_, const void* gain_, const v
       slots = grid;
 #define WROW(NPV)                                                                                                          \
   do {                                                                                                                     \
-    if (blend) rmsnorm_rev_warp_kernel<T, NPV, true><<<grid, WROW_THREADS, 0, st>>>(x, gain, rstd, gy, e, gx, a, partial, m);   \
-    else rmsnorm_rev_warp_kernel<T, NPV, false><<<grid, WROW_THREADS, 0, st>>>(x, gain, rstd, gy, e, gx, a, partial, m);        \
+    if (blend) MpLaunch(grid, WROW_THREADS, 0, st)(rmsnorm_rev_warp_kernel<T, NPV, true>, x, gain, rstd, gy, e, gx, a, partial, m);   \
+    else MpLaunch(grid, WROW_THREADS, 0, st)(rmsnorm_rev_warp_kernel<T, NPV, false>, x, gain, rstd, gy, e, gx, a, partial, m);        \
   } while (0)
       switch (wnp) {
         case 1: WROW(1); break;
@@ -1160,7 +1173,7 @@ static void rmsnorm_ij_j_reverse_impl(const void* x_, const void* gain_, const v
   do {                                                                                                     \
     MP_CUDA_CHECK(cudaFuncSetAttribute(rmsnorm_rev_staged_kernel<T, P, F, B>,                              \
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));          \
-    rmsnorm_rev_staged_kernel<T, P, F, B><<<grid, STG_THREADS, sp.smem_bytes, st>>>(                       \
+    MpLaunch(grid, STG_THREADS, sp.smem_bytes, st)(rmsnorm_rev_staged_kernel<T, P, F, B>, \
         x, gain, rstd, gy, e, gx, a, partial, m, n, rpc, sp.stages, status);                               \
   } while (0)
 #define STG_P(F, B)                                                                 \
@@ -1170,13 +1183,13 @@ static void rmsnorm_ij_j_reverse_impl(const void* x_, const void* gain_, const v
 #undef STG_P
 #undef STG
     } else if (p.generic) {
-      rmsnorm_rev_generic<T><<<grid, GEN_THREADS, 0, st>>>(x, gain, rstd, gy, e, gx, a, blend, partial, m, n, rpc);
+      MpLaunch(grid, GEN_THREADS, 0, st)(rmsnorm_rev_generic<T>, x, gain, rstd, gy, e, gx, a, blend, partial, m, n, rpc);
     } else if (blend) {
-#define CALL(G, P, F) rmsnorm_rev_kernel<T, G, P, F, true><<<grid, RowCfg<G>::THREADS, 0, st>>>(x, gain, rstd, gy, e, gx, a, partial, m, n, rpc)
+#define CALL(G, P, F) MpLaunch(grid, RowCfg<G>::THREADS, 0, st)(rmsnorm_rev_kernel<T, G, P, F, true>, x, gain, rstd, gy, e, gx, a, partial, m, n, rpc)
       MP_ROW_DISPATCH(p, CALL);
 #undef CALL
     } else {
-#define CALL(G, P, F) rmsnorm_rev_kernel<T, G, P, F, false><<<grid, RowCfg<G>::THREADS, 0, st>>>(x, gain, rstd, gy, e, gx, a, partial, m, n, rpc)
+#define CALL(G, P, F) MpLaunch(grid, RowCfg<G>::THREADS, 0, st)(rmsnorm_rev_kernel<T, G, P, F, false>, x, gain, rstd, gy, e, gx, a, partial, m, n, rpc)
       MP_ROW_DISPATCH(p, CALL);
 #undef CALL
     }
@@ -1186,11 +1199,11 @@ static void rmsnorm_ij_j_reverse_impl(const void* x_, const void* gain_, const v
   if (slots >= 512 && n % W == 0 && mp_aligned16(partial)) {   // (a few hundred rows: one launch is cheaper than two)
     A* partial2 = partial + slots * n;  // FOLD_SPLITS rows after the per-CTA partials
     const dim3 g1(static_cast<unsigned>((n + 32 * W - 1) / (32 * W)), FOLD_SPLITS);
-    rmsnorm_fold_stage1_kernel<A><<<g1, 256, 0, st>>>(partial, partial2, n, slots);
+    MpLaunch(g1, 256, 0, st)(rmsnorm_fold_stage1_kernel<A>, partial, partial2, n, slots);
     MP_LAUNCH_CHECK();
-    rmsnorm_fold_kernel<T><<<static_cast<unsigned>((n + 31) / 32), rmsnorm_fold_threads(FOLD_SPLITS), 0, st>>>(partial2, ggain, a, blend, n, FOLD_SPLITS);
+    MpLaunch(static_cast<unsigned>((n + 31) / 32), rmsnorm_fold_threads(FOLD_SPLITS), 0, st)(rmsnorm_fold_kernel<T>, partial2, ggain, a, blend, n, FOLD_SPLITS);
   } else {
-    rmsnorm_fold_kernel<T><<<static_cast<unsigned>((n + 31) / 32), rmsnorm_fold_threads(slots), 0, st>>>(partial, ggain, a, blend, n, slots);
+    MpLaunch(static_cast<unsigned>((n + 31) / 32), rmsnorm_fold_threads(slots), 0, st)(rmsnorm_fold_kernel<T>, partial, ggain, a, blend, n, slots);
   }
   MP_LAUNCH_CHECK();
 }
@@ -1310,13 +1323,13 @@ extern "C" int launch_rmsnorm_ij_j_reverse_static_r32(const void* x_, const void
     const unsigned grid = static_cast<unsigned>((groups + rpc - 1) / rpc);
     slots = static_cast<size_t>(grid) * p.rows;
     if (p.generic) {
-      rmsnorm_rev_generic<T><<<grid, GEN_THREADS, 0, st>>>(x, gain, rstd, gy, e, gx, a, blend, partial, m, n, rpc);
+      MpLaunch(grid, GEN_THREADS, 0, st)(rmsnorm_rev_generic<T>, x, gain, rstd, gy, e, gx, a, blend, partial, m, n, rpc);
     } else if (blend) {
-#define CALL(G, P, F) rmsnorm_rev_kernel<T, G, P, F, true><<<grid, RowCfg<G>::THREADS, 0, st>>>(x, gain, rstd, gy, e, gx, a, partial, m, n, rpc)
+#define CALL(G, P, F) MpLaunch(grid, RowCfg<G>::THREADS, 0, st)(rmsnorm_rev_kernel<T, G, P, F, true>, x, gain, rstd, gy, e, gx, a, partial, m, n, rpc)
       MP_ROW_DISPATCH(p, CALL);
 #undef CALL
     } else {
-#define CALL(G, P, F) rmsnorm_rev_kernel<T, G, P, F, false><<<grid, RowCfg<G>::THREADS, 0, st>>>(x, gain, rstd, gy, e, gx, a, partial, m, n, rpc)
+#define CALL(G, P, F) MpLaunch(grid, RowCfg<G>::THREADS, 0, st)(rmsnorm_rev_kernel<T, G, P, F, false>, x, gain, rstd, gy, e, gx, a, partial, m, n, rpc)
       MP_ROW_DISPATCH(p, CALL);
 #undef CALL
     }
@@ -1326,11 +1339,11 @@ extern "C" int launch_rmsnorm_ij_j_reverse_static_r32(const void* x_, const void
   if (slots >= 128 && n % W == 0) {
     A* partial2 = partial + slots * n;
     const dim3 g1(static_cast<unsigned>((n + 32 * W - 1) / (32 * W)), FOLD_SPLITS);
-    rmsnorm_fold_stage1_kernel<A><<<g1, 256, 0, st>>>(partial, partial2, n, slots);
+    MpLaunch(g1, 256, 0, st)(rmsnorm_fold_stage1_kernel<A>, partial, partial2, n, slots);
     MP_LAUNCH_CHECK();
-    rmsnorm_fold_kernel<T><<<static_cast<unsigned>((n + 31) / 32), rmsnorm_fold_threads(FOLD_SPLITS), 0, st>>>(partial2, ggain, a, blend, n, FOLD_SPLITS);
+    MpLaunch(static_cast<unsigned>((n + 31) / 32), rmsnorm_fold_threads(FOLD_SPLITS), 0, st)(rmsnorm_fold_kernel<T>, partial2, ggain, a, blend, n, FOLD_SPLITS);
   } else {
-    rmsnorm_fold_kernel<T><<<static_cast<unsigned>((n + 31) / 32), rmsnorm_fold_threads(slots), 0, st>>>(partial, ggain, a, blend, n, slots);
+    MpLaunch(static_cast<unsigned>((n + 31) / 32), rmsnorm_fold_threads(slots), 0, st)(rmsnorm_fold_kernel<T>, partial, ggain, a, blend, n, slots);
   }
   MP_LAUNCH_CHECK();
   return 0;

@@ -75,6 +75,7 @@ __device__ __forceinline__ float ssd_exp(float x) { return __expf(x); }
 __global__ void __launch_bounds__(256) ssd_cumsum_kernel(const float* __restrict__ dt, const float* __restrict__ A,
                                                          float* __restrict__ cum, float* __restrict__ dtt, int B, int L,
                                                          int H, int Q) {
+  mp_grid_dependency();
   __shared__ float warp_tot[8];
   const int nc = L / Q;
   const int c = blockIdx.x % nc, h = (blockIdx.x / nc) % H, b = blockIdx.x / (nc * H);
@@ -109,6 +110,7 @@ __global__ void __launch_bounds__(256) ssd_cumsum_kernel(const float* __restrict
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) ssd_scan_kernel(const float* __restrict__ S, __half* __restrict__ Hs,
                                                        const float* __restrict__ cum, int nc, int Q, int E, int anti) {
+  mp_grid_dependency();
   const int bh = blockIdx.y;
   const int e = blockIdx.x * 256 + threadIdx.x;
   if (e >= E) return;
@@ -183,6 +185,7 @@ __global__ void __launch_bounds__(SSD_THREADS, 4) ssd_mma_kernel(const __grid_co
                                                                 const __grid_constant__ CUtensorMap map_a1,
                                                                 const __grid_constant__ CUtensorMap map_b1,
                                                                 const SsdArgs g) {
+  mp_grid_dependency();
   extern __shared__ unsigned char ssd_smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(ssd_smem_raw) + 1023) & ~uintptr_t(1023));
   const int STAGES = g.stages, STAGE_BYTES = g.stage_bytes;
@@ -577,6 +580,7 @@ __global__ void __launch_bounds__(SSD_THREADS, 4) ssd_mma_kernel(const __grid_co
 // pin[b,h,c] = < Hs_anti[b,h,c], Hs_causal[b,h,c+1] >  (0 for the last chunk); one CTA per (b, h, c)
 __global__ void __launch_bounds__(256) ssd_boundary_dot_kernel(const __half* __restrict__ hs_anti, const __half* __restrict__ hs_causal,
                                                                float* __restrict__ pin, int nc, int E) {
+  mp_grid_dependency();
   __shared__ float red[8];
   const int c = blockIdx.x % nc;
   const size_t bh = blockIdx.x / nc;
@@ -614,9 +618,10 @@ __global__ void __launch_bounds__(256) ssd_scalar_grads_kernel(const float* __re
                                                                const float* __restrict__ dtt, const float* __restrict__ A,
                                                                const float* __restrict__ pin, float* __restrict__ gdt,
                                                                float* __restrict__ gA_part, int B, int L, int LP, int H, int Q, int halves,
-                                                               const __half* __restrict__ raw = nullptr, size_t raw_pitch = 0,
-                                                               const float* __restrict__ bias = nullptr, __half* __restrict__ graw = nullptr,
-                                                               size_t graw_pitch = 0, float* __restrict__ gbias = nullptr) {
+                                                               const __half* __restrict__ raw, size_t raw_pitch,
+                                                               const float* __restrict__ bias, __half* __restrict__ graw,
+                                                               size_t graw_pitch, float* __restrict__ gbias) {
+  mp_grid_dependency();
   __shared__ float warp_tot[8];
   __shared__ float total_s;
   __shared__ float ga_red[8];
@@ -684,6 +689,7 @@ __global__ void __launch_bounds__(256) ssd_scalar_grads_kernel(const float* __re
 // out[i] = sum_s part[s][i] rounded to r16 (fold of the per-group partial outputs), 8 elements per thread
 __global__ void __launch_bounds__(256) ssd_fold_parts_kernel(const float* __restrict__ part, __half* __restrict__ out, size_t n,
                                                              int splits) {
+  mp_grid_dependency();
   const size_t i = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) * 8;
   if (i >= n) return;
   float acc[8];
@@ -700,7 +706,8 @@ __global__ void __launch_bounds__(256) ssd_fold_parts_kernel(const float* __rest
 
 // gA[h] = sum over the batch; with A_log's gradient wanted (A = -exp(A_log), so dA / dA_log = A): gA_log[h] += gA[h] * A[h]
 __global__ void ssd_sum_batches_kernel(const float* __restrict__ part, float* __restrict__ gA, int B, int H,
-                                       const float* __restrict__ A = nullptr, float* __restrict__ gA_log = nullptr) {
+                                       const float* __restrict__ A, float* __restrict__ gA_log) {
+  mp_grid_dependency();
   const int h = blockIdx.x * blockDim.x + threadIdx.x;
   if (h >= H) return;
   float s = 0.f;
@@ -820,7 +827,7 @@ template <int MODE>
 void ssd_launch(const CUtensorMap& a0, const CUtensorMap& b0, const CUtensorMap& a1, const CUtensorMap& b1, const SsdArgs& g,
                 dim3 grid, size_t smem, cudaStream_t st) {
   MP_CUDA_CHECK(cudaFuncSetAttribute(ssd_mma_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  ssd_mma_kernel<MODE><<<grid, SSD_THREADS, smem, st>>>(a0, b0, a1, b1, g);
+  MpLaunch(grid, SSD_THREADS, smem, st)(ssd_mma_kernel<MODE>, a0, b0, a1, b1, g);
   MP_LAUNCH_CHECK();
 }
 
@@ -881,7 +888,7 @@ void ssd_operator(const SsdDims& d, const Roles& r, const SsdScratch& sc, uint32
   {
     const int E = 128 * d2;
     const dim3 grid((E + 255) / 256, d.B * d.H);
-    ssd_scan_kernel<<<grid, 256, 0, st>>>(sc.states, sc.hs, sc.cum, d.nc, d.Q, E, r.anti);
+    MpLaunch(grid, 256, 0, st)(ssd_scan_kernel, sc.states, sc.hs, sc.cum, d.nc, d.Q, E, r.anti);
     MP_LAUNCH_CHECK();
   }
   // output
@@ -901,7 +908,7 @@ void ssd_operator(const SsdDims& d, const Roles& r, const SsdScratch& sc, uint32
     ssd_launch<MODE_OUTPUT>(ms, mv, mq, mh, g, grid, smem, st);
     if (splits > 1) {
       const size_t n = static_cast<size_t>(d.B) * d.L * d.G * r.dv;
-      ssd_fold_parts_kernel<<<static_cast<unsigned>((n / 8 + 255) / 256), 256, 0, st>>>(sc.parts, r.out, n, splits);
+      MpLaunch(static_cast<unsigned>((n / 8 + 255) / 256), 256, 0, st)(ssd_fold_parts_kernel, sc.parts, r.out, n, splits);
       MP_LAUNCH_CHECK();
     }
     g.head_splits = 1; g.part_out = nullptr;
@@ -1027,7 +1034,7 @@ extern "C" void launch_ssd_scan_r16(const void* x, const void* dt, const void* A
     return;
   }
   const SsdScratch sc = ssd_carve(scratch, d, false);
-  ssd_cumsum_kernel<<<d.B * d.H * d.nc, 256, 0, st>>>(static_cast<const float*>(dt), static_cast<const float*>(A), sc.cum, sc.dtt,
+  MpLaunch(d.B * d.H * d.nc, 256, 0, st)(ssd_cumsum_kernel, static_cast<const float*>(dt), static_cast<const float*>(A), sc.cum, sc.dtt,
                                                      d.B, d.L, d.H, d.Q);
   MP_LAUNCH_CHECK();
   Roles r;
@@ -1159,17 +1166,15 @@ static bool ssd_scan_reverse_r16_impl(const void* x, const void* dt, const void*
     mp_ssd_group_grads(gyh, xh, bh, ch, w.hs_causal, w.hs_anti, w.cum, w.dtt, w.colf_c, static_cast<__half*>(gB), static_cast<__half*>(gC),
                        d.B, d.L, d.H, d.G, state->status_dev, st);
     const int wnc = (d.L + 127) / 128;
-    ssd_boundary_dot_kernel<<<d.B * d.H * wnc, 256, 0, lane1>>>(w.hs_anti, w.hs_causal, w.pin, wnc, d.N * d.P);
+    MpLaunch(d.B * d.H * wnc, 256, 0, lane1)(ssd_boundary_dot_kernel, w.hs_anti, w.hs_causal, w.pin, wnc, d.N * d.P);
     MP_LAUNCH_CHECK();
-    if (rs != nullptr)
-      ssd_scalar_grads_kernel<<<d.B * d.H, 256, 0, lane1>>>(w.u, w.v, w.dtt, static_cast<const float*>(A), w.pin, static_cast<float*>(gdt), w.ga_part,
-                                                           d.B, d.L, wnc * 128, d.H, 128, 2, rs->raw, rs->raw_pitch, rs->bias, rs->graw, rs->graw_pitch,
-                                                           rs->gbias);
-    else
-      ssd_scalar_grads_kernel<<<d.B * d.H, 256, 0, lane1>>>(w.u, w.v, w.dtt, static_cast<const float*>(A), w.pin, static_cast<float*>(gdt), w.ga_part,
-                                                           d.B, d.L, wnc * 128, d.H, 128, 2);
+    const RawSide none{nullptr, 0, nullptr, nullptr, 0, nullptr, nullptr};
+    const RawSide& side_out = rs != nullptr ? *rs : none;
+    MpLaunch(d.B * d.H, 256, 0, lane1)(ssd_scalar_grads_kernel, w.u, w.v, w.dtt, static_cast<const float*>(A), w.pin, static_cast<float*>(gdt), w.ga_part,
+                                       d.B, d.L, wnc * 128, d.H, 128, 2, side_out.raw, side_out.raw_pitch, side_out.bias, side_out.graw,
+                                       side_out.graw_pitch, side_out.gbias);
     MP_LAUNCH_CHECK();
-    ssd_sum_batches_kernel<<<(d.H + 127) / 128, 128, 0, lane1>>>(w.ga_part, static_cast<float*>(gA), d.B, d.H, static_cast<const float*>(A),
+    MpLaunch((d.H + 127) / 128, 128, 0, lane1)(ssd_sum_batches_kernel, w.ga_part, static_cast<float*>(gA), d.B, d.H, static_cast<const float*>(A),
                                                                  rs != nullptr ? rs->gA_log : nullptr);
     MP_LAUNCH_CHECK();
     if (side) {
@@ -1179,7 +1184,7 @@ static bool ssd_scan_reverse_r16_impl(const void* x, const void* dt, const void*
     return true;
   }
   const SsdScratch sc = ssd_carve(scratch, d, true);
-  ssd_cumsum_kernel<<<d.B * d.H * d.nc, 256, 0, st>>>(static_cast<const float*>(dt), static_cast<const float*>(A), sc.cum, sc.dtt,
+  MpLaunch(d.B * d.H * d.nc, 256, 0, st)(ssd_cumsum_kernel, static_cast<const float*>(dt), static_cast<const float*>(A), sc.cum, sc.dtt,
                                                      d.B, d.L, d.H, d.Q);
   MP_LAUNCH_CHECK();
   // The four operator instances are independent of one another: each runs on its own stream (forked from and
@@ -1234,12 +1239,12 @@ static bool ssd_scan_reverse_r16_impl(const void* x, const void* dt, const void*
   }
   // gdt, gA
   // (operator 0 = gx: anti-causal states of C gy^T; operator 1 = u: causal states of B x^T; both [B,H,nc][N][P])
-    ssd_boundary_dot_kernel<<<d.B * d.H * d.nc, 256, 0, st>>>(sc.hs_op[0], sc.hs_op[1], sc.pin, d.nc, d.N * d.P);
+    MpLaunch(d.B * d.H * d.nc, 256, 0, st)(ssd_boundary_dot_kernel, sc.hs_op[0], sc.hs_op[1], sc.pin, d.nc, d.N * d.P);
     MP_LAUNCH_CHECK();
-    ssd_scalar_grads_kernel<<<d.B * d.H, 256, 0, st>>>(sc.u, sc.v, sc.dtt, static_cast<const float*>(A), sc.pin, static_cast<float*>(gdt),
-                                                      sc.ga_part, d.B, d.L, d.L, d.H, d.Q, 1);
+    MpLaunch(d.B * d.H, 256, 0, st)(ssd_scalar_grads_kernel, sc.u, sc.v, sc.dtt, static_cast<const float*>(A), sc.pin, static_cast<float*>(gdt),
+                                                      sc.ga_part, d.B, d.L, d.L, d.H, d.Q, 1, nullptr, 0, nullptr, nullptr, 0, nullptr);
     MP_LAUNCH_CHECK();
-  ssd_sum_batches_kernel<<<(d.H + 127) / 128, 128, 0, st>>>(sc.ga_part, static_cast<float*>(gA), d.B, d.H);
+  MpLaunch((d.H + 127) / 128, 128, 0, st)(ssd_sum_batches_kernel, sc.ga_part, static_cast<float*>(gA), d.B, d.H, nullptr, nullptr);
   MP_LAUNCH_CHECK();
   return false;
 }

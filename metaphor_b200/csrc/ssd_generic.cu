@@ -60,6 +60,7 @@ __global__ void __launch_bounds__(GEN_THREADS) ssd_generic_kernel(const T* __res
                                                                   A* __restrict__ gdt, A* __restrict__ gA, A* __restrict__ gB,
                                                                   A* __restrict__ gC, A* __restrict__ ckpt, A* __restrict__ cs,
                                                                   GenDims d) {
+  mp_grid_dependency();
   extern __shared__ __align__(16) unsigned char gen_smem[];
   A* sB = reinterpret_cast<A*>(gen_smem);
   A* sC = sB + d.N;
@@ -220,6 +221,7 @@ __global__ void __launch_bounds__(GEN_THREADS) ssd_generic_kernel(const T* __res
 
 template <typename A>
 __global__ void gen_round_kernel(const A* __restrict__ src, void* __restrict__ dst, size_t n, int to_half) {
+  mp_grid_dependency();
   const size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
   if (i >= n) return;
   if (to_half) static_cast<__half*>(dst)[i] = __float2half_rn(static_cast<float>(src[i]));
@@ -251,7 +253,7 @@ static void ssd_generic_forward(const void* x, const void* dt, const void* Av, c
   if (ngroups == 0 || heads % ngroups != 0) MP_FATAL("ssd_scan: heads %d not divisible by groups %d", d.H, d.G);
   if (!gen_plan(d)) MP_FATAL("ssd_scan: headdim %d x d_state %d is beyond the generic path (headdim <= 256, d_state * headdim <= 16384)", d.P, d.N);
   const size_t smem = gen_smem_bytes(d, sizeof(A));
-  ssd_generic_kernel<T, A, false><<<d.B * d.H, GEN_THREADS, smem, mp_stream(ctx)>>>(
+  MpLaunch(d.B * d.H, GEN_THREADS, smem, mp_stream(ctx))(ssd_generic_kernel<T, A, false>, 
       static_cast<const T*>(x), static_cast<const A*>(dt), static_cast<const A*>(Av), static_cast<const T*>(Bm), static_cast<const T*>(Cm),
       static_cast<T*>(y), nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, d);
   MP_LAUNCH_CHECK();
@@ -281,13 +283,13 @@ static void ssd_generic_reverse(const void* x, const void* dt, const void* Av, c
   MP_CUDA_CHECK(cudaMemsetAsync(gC_acc, 0, bc * sizeof(A), st));
   MP_CUDA_CHECK(cudaMemsetAsync(gA, 0, static_cast<size_t>(d.H) * sizeof(A), st));
   const size_t smem = gen_smem_bytes(d, sizeof(A));
-  ssd_generic_kernel<T, A, true><<<d.B * d.H, GEN_THREADS, smem, st>>>(
+  MpLaunch(d.B * d.H, GEN_THREADS, smem, st)(ssd_generic_kernel<T, A, true>, 
       static_cast<const T*>(x), static_cast<const A*>(dt), static_cast<const A*>(Av), static_cast<const T*>(Bm), static_cast<const T*>(Cm),
       nullptr, static_cast<const T*>(gy), static_cast<T*>(gx), static_cast<A*>(gdt), static_cast<A*>(gA), gB_acc, gC_acc, ckpt, cs, d);
   MP_LAUNCH_CHECK();
   if (narrow) {
-    gen_round_kernel<A><<<static_cast<unsigned>((bc + 255) / 256), 256, 0, st>>>(gB_acc, gB, bc, 1);
-    gen_round_kernel<A><<<static_cast<unsigned>((bc + 255) / 256), 256, 0, st>>>(gC_acc, gC, bc, 1);
+    MpLaunch(static_cast<unsigned>((bc + 255) / 256), 256, 0, st)(gen_round_kernel<A>, gB_acc, gB, bc, 1);
+    MpLaunch(static_cast<unsigned>((bc + 255) / 256), 256, 0, st)(gen_round_kernel<A>, gC_acc, gC, bc, 1);
     MP_LAUNCH_CHECK();
   }
 }

@@ -151,6 +151,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_con
   __syncthreads();
   tcgen05_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
+  mp_grid_dependency();
 
 
   if (warp == 0) {
@@ -644,6 +645,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_group_grads_kernel(const __g
   __syncthreads();
   tcgen05_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
+  mp_grid_dependency();
 
   if (warp == 0) {
     // ------------------------------ TMA: loads, then the output stores -------------
@@ -881,6 +883,7 @@ __global__ void __launch_bounds__(WQ) ssd_walk_cumsum_kernel(const float* __rest
                                                              int L, int H, int* __restrict__ carry_flags, int n_flags,
                                                              const __half* __restrict__ raw, size_t raw_pitch, const float* __restrict__ bias,
                                                              float* __restrict__ dt_out, float* __restrict__ A_out) {
+  mp_grid_dependency();
   __shared__ float warp_tot[4];
   if (blockIdx.x == 0)   // the walks that follow in stream order hand states from CTA to CTA through these counters
     for (int i = threadIdx.x; i < n_flags; i += WQ) carry_flags[i] = 0;
@@ -987,7 +990,7 @@ bool mp_ssd_walk_supported(int L, int H, int P, int N, int G) {
 
 void mp_ssd_walk_cumsum(const float* dt, const float* A, float* cum, float* dtt, float* colf_c, float* colf_a, int B, int L, int H,
                         int* carry_flags, int n_flags, cudaStream_t st) {
-  ssd_walk_cumsum_kernel<false><<<B * H * ((L + WQ - 1) / WQ), WQ, 0, st>>>(dt, A, cum, dtt, colf_c, colf_a, L, H, carry_flags, n_flags, nullptr, 0, nullptr,
+  MpLaunch(B * H * ((L + WQ - 1) / WQ), WQ, 0, st)(ssd_walk_cumsum_kernel<false>, dt, A, cum, dtt, colf_c, colf_a, L, H, carry_flags, n_flags, nullptr, 0, nullptr,
                                                                  nullptr, nullptr);
   MP_LAUNCH_CHECK();
 }
@@ -995,7 +998,7 @@ void mp_ssd_walk_cumsum(const float* dt, const float* A, float* cum, float* dtt,
 // The same from the raw projection output and A_log (see the kernel); dt_out and A_out are what the reverse pass takes.
 void mp_ssd_walk_cumsum_raw(const __half* raw, size_t raw_pitch, const float* bias, const float* A_log, float* dt_out, float* A_out, float* cum,
                             float* dtt, float* colf_c, int B, int L, int H, int* carry_flags, int n_flags, cudaStream_t st) {
-  ssd_walk_cumsum_kernel<true><<<B * H * ((L + WQ - 1) / WQ), WQ, 0, st>>>(nullptr, A_log, cum, dtt, colf_c, nullptr, L, H, carry_flags, n_flags, raw, raw_pitch,
+  MpLaunch(B * H * ((L + WQ - 1) / WQ), WQ, 0, st)(ssd_walk_cumsum_kernel<true>, nullptr, A_log, cum, dtt, colf_c, nullptr, L, H, carry_flags, n_flags, raw, raw_pitch,
                                                                 bias, dt_out, A_out);
   MP_LAUNCH_CHECK();
 }
@@ -1018,7 +1021,7 @@ void mp_ssd_walk(int anti, const __half* q, const __half* k, const __half* v, co
   const CUtensorMap mh = hs_out != nullptr ? walk_map(hs_out, static_cast<size_t>(B) * H * g.nc * WN, WP) : mv;
   auto launch = [&](auto kernel) {
     MP_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, W_SMEM_BYTES));
-    kernel<<<grid, W_THREADS, W_SMEM_BYTES, st>>>(mq, mk, mv, mh, g);
+    MpLaunch(grid, W_THREADS, W_SMEM_BYTES, st)(kernel, mq, mk, mv, mh, g);
   };
   const bool dot = z != nullptr && dot_out != nullptr;
   if (!dot) { g.z = nullptr; g.dot_out = nullptr; }
@@ -1048,6 +1051,6 @@ void mp_ssd_group_grads(const __half* gy, const __half* x, const __half* Bm, con
   const CUtensorMap mb = walk_map3(Bm, B, L, static_cast<size_t>(G) * WN), mc = walk_map3(Cm, B, L, static_cast<size_t>(G) * WN);
   const CUtensorMap mgb = walk_map3(gB, B, L, static_cast<size_t>(G) * WN), mgc = walk_map3(gC, B, L, static_cast<size_t>(G) * WN);
   MP_CUDA_CHECK(cudaFuncSetAttribute(ssd_group_grads_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GG_SMEM_BYTES));
-  ssd_group_grads_kernel<<<B * g.nc * G, W_THREADS, GG_SMEM_BYTES, st>>>(mgy, mx, mhc, mha, mb, mc, mgb, mgc, g);
+  MpLaunch(B * g.nc * G, W_THREADS, GG_SMEM_BYTES, st)(ssd_group_grads_kernel, mgy, mx, mhc, mha, mb, mc, mgb, mgc, g);
   MP_LAUNCH_CHECK();
 }
