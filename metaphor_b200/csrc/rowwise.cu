@@ -12,6 +12,7 @@
 #include "mp_async.cuh"
 
 #include <cfloat>
+#include <initializer_list>
 #include <mutex>
 
 namespace {
@@ -693,7 +694,15 @@ __global__ void __launch_bounds__(1024) rmsnorm_fold_kernel(const typename Acc<T
   const size_t col = static_cast<size_t>(blockIdx.x) * 32 + lane;
   A s = A(0);
   if (col < n) {
-    for (size_t p = slice; p < slots; p += slices) s += partial[p * n + col];
+    size_t p = slice;
+    for (; p + 7 * static_cast<size_t>(slices) < slots; p += 8 * static_cast<size_t>(slices)) {   // eight loads in flight
+      A v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = partial[(p + u * static_cast<size_t>(slices)) * n + col];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) s += v[u];
+    }
+    for (; p < slots; p += slices) s += partial[p * n + col];
   }
   sm[slice][lane] = s;
   __syncthreads();
@@ -757,7 +766,337 @@ __global__ void __launch_bounds__(256) rmsnorm_fold_stage1_kernel(const A* __res
   }
 }
 
-// --------------------- generic fallback (any n, any alignment) ------------
+// --------------------- rows that are not 16-byte aligned -------------------
+// An odd number of columns puts every row at another offset from a 16-byte boundary.  The tensors of a call share it (their bases
+// are aligned alike), so a row is still read and written in whole packs of 16 bytes, counted from the boundary below its first
+// element; only the packs at its two ends are taken apart.  Elements of a pack outside the row hold a neutral value, so that the
+// arithmetic needs no guards.  Rows lie in registers as in the kernels above.  A CTA that walks several rows steps by a multiple
+// of the pack length: the offset, and with it the columns that a thread holds of gain and gain gradient, stay the same.
+// (Plain accesses, not streaming ones: the sectors at a row's two ends are shared with its neighbours.)
+// Softmax forward / reverse, RMSNorm forward / reverse in us, before (one element per thread and step, three passes over a row) and
+// now: [3000, 1001] r32 12.5 / 9.5 / 10.5 / 33 -> 7.4 / 6.3 / 6.2 / 14; [50000, 77] r32 78 / 48 / 54 / 93 -> 12 / 12 / 14 / 34;
+// [65536, 4097] r16 307 / 386 / 281 / 1031 -> 245 / 293 / 223 / 583, r32 373 / 578 / 396 / 1377 -> 338 / 486 / 360 / 681.
+template <typename T, int GROUP, int PPT> struct ShiftRow {
+  static constexpr int PN = Pack<T>::N;
+  int n, off, t;
+  __device__ __forceinline__ int first(int u) const { return (t + u * GROUP) * PN - off; }   // column of a pack's first element
+  // A row group has the fewest packs per thread that hold the row, so only the last two can lie beyond it (live: at least one element
+  // of the row) and only they and the first can be cut.
+  __device__ __forceinline__ bool live(int u) const { return u < PPT - 2 || first(u) < n; }
+  __device__ __forceinline__ bool edge(int u) const { return (u == 0 && first(u) < 0) || (u >= PPT - 2 && first(u) + PN > n); }
+  // The live packs, as whole aligned packs (16 bytes around a valid element are readable whatever lies beside it).  The elements
+  // outside are replaced by `cut` later, when all loads of a row have been issued: doing it here would wait for them.
+  __device__ __forceinline__ void load(const T* row, Pack<T>* p) const {
+#pragma unroll
+    for (int u = 0; u < PPT; ++u)
+      if (live(u)) p[u] = ld_pack(row + first(u), 0);
+  }
+  __device__ __forceinline__ void cut(Pack<T>* p, T fill) const {
+#pragma unroll
+    for (int u = 0; u < PPT; ++u) {
+      if ((u == 0 || u >= PPT - 2) && live(u) && edge(u)) {
+        const int c = first(u);
+#pragma unroll
+        for (int k = 0; k < PN; ++k)
+          if (c + k < 0 || c + k >= n) p[u].v[k] = fill;
+      }
+    }
+  }
+  // A 16-byte aligned vector of n columns (the gain): its packs lie `off` elements further than this row's, so a pack is put
+  // together from two of them by a three-step barrel shift over their words and a funnel shift inside.
+  __device__ __forceinline__ void load_columns(const T* v, Pack<T>* p) const {
+    const uint32_t start = 16u - off * static_cast<uint32_t>(sizeof(T)), q = start >> 2, r = (start & 3u) * 8u;
+#pragma unroll
+    for (int u = 0; u < PPT; ++u) {
+      if (!live(u)) continue;
+      const int c = (t + u * GROUP) * PN;   // the aligned pack at or behind the wanted one
+      union { uint4 q4[2]; uint32_t w[8]; } b;
+      b.q4[0] = c > 0 && c - PN < n ? *reinterpret_cast<const uint4*>(v + c - PN) : make_uint4(0u, 0u, 0u, 0u);
+      b.q4[1] = c < n ? *reinterpret_cast<const uint4*>(v + c) : make_uint4(0u, 0u, 0u, 0u);
+      uint32_t w[9];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) w[k] = b.w[k];
+      w[8] = 0u;
+#pragma unroll
+      for (int k = 0; k < 5; ++k) w[k] = (q & 4u) != 0 ? w[k + 4] : w[k];
+#pragma unroll
+      for (int k = 0; k < 6; ++k) w[k] = (q & 2u) != 0 ? w[k + 2] : w[k];
+#pragma unroll
+      for (int k = 0; k < 5; ++k) w[k] = (q & 1u) != 0 ? w[k + 1] : w[k];
+      union { uint4 q4; Pack<T> p; } o;
+      o.q4 = make_uint4(__funnelshift_r(w[0], w[1], r), __funnelshift_r(w[1], w[2], r), __funnelshift_r(w[2], w[3], r), __funnelshift_r(w[3], w[4], r));
+      p[u] = o.p;
+    }
+    cut(p, mp_down<T>(0));
+  }
+  __device__ __forceinline__ void store(T* row, int u, const typename Acc<T>::type* e) const {
+    const int c = first(u);
+    const Pack<T> q = pack<T>(e);
+    if (!edge(u)) {
+      st_pack(row + c, 0, q);
+    } else {
+#pragma unroll
+      for (int k = 0; k < PN; ++k)
+        if (c + k >= 0 && c + k < n) row[c + k] = q.v[k];
+    }
+  }
+};
+// off0: elements between a 16-byte boundary and the tensors' bases
+#define MP_SHIFT_ROW()                                                                                                   \
+  using A = typename Acc<T>::type;                                                                                       \
+  constexpr int PN = Pack<T>::N, ROWS = RowCfg<GROUP>::ROWS;                                                             \
+  const int g = threadIdx.x / GROUP;                                                                                     \
+  const size_t step = static_cast<size_t>(gridDim.x) * ROWS;                                                             \
+  size_t row = static_cast<size_t>(blockIdx.x) * ROWS + g;                                                               \
+  const ShiftRow<T, GROUP, PPT> sr{static_cast<int>(n), static_cast<int>((row * n + off0) % PN), static_cast<int>(threadIdx.x % GROUP)}
+
+template <typename T, int GROUP, int PPT>
+__global__ void __launch_bounds__(RowCfg<GROUP>::THREADS) softmax_fwd_shift(const T* x, T* y, size_t m, size_t n, int off0) {
+  mp_grid_dependency();
+  MP_SHIFT_ROW();
+  __shared__ A red[64];
+  for (; row < m; row += step) {
+    Pack<T> p[PPT];
+    sr.load(x + row * n, p);
+    sr.cut(p, mp_down<T>(mp_neg_inf(A(0))));
+    A e[PPT][PN];
+    A mx = mp_neg_inf(A(0));
+#pragma unroll
+    for (int u = 0; u < PPT; ++u) {
+      if (sr.live(u)) {
+        unpack<T>(p[u], e[u]);
+#pragma unroll
+        for (int k = 0; k < PN; ++k) mx = MaxOp::apply(mx, e[u][k]);
+      }
+    }
+    mx = group_reduce<MaxOp, GROUP>(mx, red, mp_neg_inf(A(0)));
+    const A mxs = mp_exp_prescale(mx);
+    A sum = A(0);
+#pragma unroll
+    for (int u = 0; u < PPT; ++u) {
+      if (sr.live(u)) {
+#pragma unroll
+        for (int k = 0; k < PN; ++k) {
+          e[u][k] = mp_exp_diff(e[u][k], mxs);
+          sum += e[u][k];
+        }
+      }
+    }
+    sum = group_reduce<SumOp, GROUP>(sum, red, A(0));
+    const A inv = A(1) / sum;
+#pragma unroll
+    for (int u = 0; u < PPT; ++u) {
+      if (sr.live(u)) {
+#pragma unroll
+        for (int k = 0; k < PN; ++k) e[u][k] *= inv;
+        sr.store(y + row * n, u, e[u]);
+      }
+    }
+  }
+}
+
+template <typename T, int GROUP, int PPT>
+__global__ void __launch_bounds__(RowCfg<GROUP>::THREADS) softmax_rev_shift(const T* y, const T* gy, T* gx, typename Acc<T>::type alpha, bool blend,
+                                                                           size_t m, size_t n, int off0) {
+  mp_grid_dependency();
+  MP_SHIFT_ROW();
+  __shared__ A red[64];
+  for (; row < m; row += step) {
+    Pack<T> py[PPT], pg[PPT];
+    sr.load(y + row * n, py);
+    sr.load(gy + row * n, pg);
+    sr.cut(py, mp_down<T>(0));
+    sr.cut(pg, mp_down<T>(0));
+    A dot = A(0);
+#pragma unroll
+    for (int u = 0; u < PPT; ++u) {
+      if (sr.live(u)) {
+        A fy[PN], fg[PN];
+        unpack<T>(py[u], fy);
+        unpack<T>(pg[u], fg);
+#pragma unroll
+        for (int k = 0; k < PN; ++k) dot += fy[k] * fg[k];
+      }
+    }
+    dot = group_reduce<SumOp, GROUP>(dot, red, A(0));
+#pragma unroll
+    for (int u = 0; u < PPT; ++u) {
+      if (sr.live(u)) {
+        A fy[PN], fg[PN];   // (unpacked a second time: kept, the r16 values would take four registers more per pair)
+        unpack<T>(py[u], fy);
+        unpack<T>(pg[u], fg);
+#pragma unroll
+        for (int k = 0; k < PN; ++k) fy[k] = fy[k] * (fg[k] - dot);
+        if (blend) {
+          const Pack<T> po = ld_pack(gx + row * n + sr.first(u), 0);
+          unpack<T>(po, fg);
+#pragma unroll
+          for (int k = 0; k < PN; ++k) fy[k] += alpha * fg[k];
+        }
+        sr.store(gx + row * n, u, fy);
+      }
+    }
+  }
+}
+
+template <typename T, int GROUP, int PPT>
+__global__ void __launch_bounds__(RowCfg<GROUP>::THREADS) rmsnorm_fwd_shift(const T* x, const T* gain, typename Acc<T>::type eps, T* y,
+                                                                           typename Acc<T>::type* rstd_out, size_t m, size_t n, int off0) {
+  mp_grid_dependency();
+  MP_SHIFT_ROW();
+  __shared__ A red[64];
+  Pack<T> pn[PPT];
+  sr.load_columns(gain, pn);
+  const A inv_n = A(1) / static_cast<A>(n);
+  // A CTA walks several rows (it has the gain put together once), so the next one is requested before this one is reduced.
+  constexpr bool AHEAD = GROUP <= 512;
+  Pack<T> p[PPT], next[AHEAD ? PPT : 1];
+  if (AHEAD && row < m) sr.load(x + row * n, p);
+  for (; row < m; row += step) {
+    if constexpr (AHEAD) {
+      if (row + step < m) sr.load(x + (row + step) * n, next);
+    } else {
+      sr.load(x + row * n, p);
+    }
+    sr.cut(p, mp_down<T>(0));
+    A e[PPT][PN];
+    A ss = A(0);
+#pragma unroll
+    for (int u = 0; u < PPT; ++u) {
+      if (sr.live(u)) {
+        unpack<T>(p[u], e[u]);
+#pragma unroll
+        for (int k = 0; k < PN; ++k) ss += e[u][k] * e[u][k];
+      }
+    }
+    ss = group_reduce<SumOp, GROUP>(ss, red, A(0));
+    const A rstd = mp_rsqrt(ss * inv_n + eps);
+    if (rstd_out != nullptr && sr.t == 0) rstd_out[row] = rstd;
+#pragma unroll
+    for (int u = 0; u < PPT; ++u) {
+      if (sr.live(u)) {
+        A fn[PN];
+        unpack<T>(pn[u], fn);
+#pragma unroll
+        for (int k = 0; k < PN; ++k) e[u][k] = e[u][k] * rstd * fn[k];
+        sr.store(y + row * n, u, e[u]);
+        if constexpr (AHEAD) p[u] = next[u];
+      }
+    }
+  }
+}
+
+// A CTA walks its share of the rows (grid-stride over row groups), the next row requested before the current one is reduced; its
+// gain-gradient sums leave as one partial row.
+template <typename T, int GROUP, int PPT>
+__global__ void __launch_bounds__(RowCfg<GROUP>::THREADS) rmsnorm_rev_shift(const T* x, const T* gain, const typename Acc<T>::type* rstd_in,
+                                                                           const T* gy, typename Acc<T>::type eps, T* gx,
+                                                                           typename Acc<T>::type alpha, bool blend, typename Acc<T>::type* partial,
+                                                                           size_t m, size_t n, int off0) {
+  mp_grid_dependency();
+  MP_SHIFT_ROW();
+  __shared__ A red[64];
+  __shared__ A sums[ROWS > 1 ? ROWS - 1 : 1][ROWS > 1 ? GROUP * PPT * PN : 1];
+  constexpr bool AHEAD = GROUP <= 256 || (GROUP == 512 && PPT <= 3);   // (the others have no registers left for the next row)
+  Pack<T> pn[PPT], px[PPT], pg[PPT], nx[AHEAD ? PPT : 1], ng[AHEAD ? PPT : 1];
+  sr.load_columns(gain, pn);
+  A acc[PPT][PN];
+#pragma unroll
+  for (int u = 0; u < PPT; ++u)
+#pragma unroll
+    for (int k = 0; k < PN; ++k) acc[u][k] = A(0);
+  const A inv_n = A(1) / static_cast<A>(n);
+  if (AHEAD && row < m) {
+    sr.load(x + row * n, px);
+    sr.load(gy + row * n, pg);
+  }
+  for (; row < m; row += step) {
+    if constexpr (AHEAD) {
+      if (row + step < m) {
+        sr.load(x + (row + step) * n, nx);
+        sr.load(gy + (row + step) * n, ng);
+      }
+    } else {
+      sr.load(x + row * n, px);
+      sr.load(gy + row * n, pg);
+    }
+    sr.cut(px, mp_down<T>(0));
+    sr.cut(pg, mp_down<T>(0));
+    A ss = A(0), dot = A(0);
+#pragma unroll
+    for (int u = 0; u < PPT; ++u) {
+      if (sr.live(u)) {
+        A fx[PN], fg[PN], fn[PN];
+        unpack<T>(px[u], fx);
+        unpack<T>(pg[u], fg);
+        unpack<T>(pn[u], fn);
+#pragma unroll
+        for (int k = 0; k < PN; ++k) {
+          ss += fx[k] * fx[k];
+          dot += fg[k] * fn[k] * fx[k];
+        }
+      }
+    }
+    group_sum2<GROUP>(ss, dot, red);
+    const A rstd = rstd_in != nullptr ? rstd_in[row] : mp_rsqrt(ss * inv_n + eps);
+    const A coef = rstd * rstd * rstd * dot * inv_n;
+#pragma unroll
+    for (int u = 0; u < PPT; ++u) {
+      if (sr.live(u)) {
+        A fx[PN], fg[PN], fn[PN];
+        unpack<T>(px[u], fx);
+        unpack<T>(pg[u], fg);
+        unpack<T>(pn[u], fn);
+#pragma unroll
+        for (int k = 0; k < PN; ++k) {
+          acc[u][k] += fg[k] * fx[k] * rstd;
+          fg[k] = rstd * fg[k] * fn[k] - fx[k] * coef;
+        }
+        if (blend) {
+          const Pack<T> po = ld_pack(gx + row * n + sr.first(u), 0);
+          unpack<T>(po, fx);
+#pragma unroll
+          for (int k = 0; k < PN; ++k) fg[k] += alpha * fx[k];
+        }
+        sr.store(gx + row * n, u, fg);
+        if constexpr (AHEAD) {
+          px[u] = nx[u];
+          pg[u] = ng[u];
+        }
+      }
+    }
+  }
+  if constexpr (ROWS > 1) {   // the row groups of the CTA meet in the first one, column by column (their offsets differ)
+    if (g > 0) {
+#pragma unroll
+      for (int u = 0; u < PPT; ++u)
+#pragma unroll
+        for (int k = 0; k < PN; ++k) {
+          const int c = sr.first(u) + k;
+          if (c >= 0 && c < sr.n) sums[g - 1][c] = acc[u][k];
+        }
+    }
+    __syncthreads();
+    if (g > 0) return;
+  }
+  A* pr = partial + static_cast<size_t>(blockIdx.x) * n;
+#pragma unroll
+  for (int u = 0; u < PPT; ++u)
+#pragma unroll
+    for (int k = 0; k < PN; ++k) {
+      const int c = sr.first(u) + k;
+      if (c >= 0 && c < sr.n) {
+        A v = acc[u][k];
+        if constexpr (ROWS > 1) {
+#pragma unroll
+          for (int q = 0; q < ROWS - 1; ++q) v += sums[q][c];
+        }
+        pr[c] = v;
+      }
+    }
+}
+
+// --------------------- fallback (any n, any alignment) ---------------------
 // One CTA per row, scalar coalesced accesses, the row is re-read from L2 for
 // each pass.  Used when n is not a multiple of the pack width, a pointer is
 // not 16-byte aligned, or the row does not fit the register-resident kernels.
@@ -999,6 +1338,71 @@ int rms_rev_warp_packs(size_t n, bool aligned) {
   const size_t np = n / (32 * PN);
   return np <= (sizeof(T) == 4 ? 5 : 4) ? static_cast<int>(np) : 0;   // wider rows spill the register plan
 }
+// Plan of the *_shift kernels: the smallest row group whose threads hold all the packs that a row can touch, up to five each (four
+// would put the rows just past a power of two on twice the threads); off0 < 0: the row does not fit, or the tensors lie at
+// different offsets from a 16-byte boundary.
+template <typename T>
+RowPlan shift_plan(size_t n, std::initializer_list<const void*> ptrs, int* off0) {
+  constexpr size_t PN = Pack<T>::N;
+  RowPlan p{true, 1024, 5, 1024, 1, false};
+  *off0 = -1;
+  const size_t nv = (n + 2 * PN - 2) / PN;
+  for (int group : {32, 128, 256, 512, 1024}) {
+    if (nv > static_cast<size_t>(group) * 5) continue;
+    p.generic = false;
+    p.group = group;
+    p.ppt = static_cast<int>((nv + group - 1) / group);
+    p.threads = group < 128 ? 128 : group;
+    p.rows = p.threads / group;
+    break;
+  }
+  if (p.generic) return p;
+  int off = -1;
+  for (const void* q : ptrs) {
+    const int o = static_cast<int>(reinterpret_cast<uintptr_t>(q) % 16);
+    if (o % sizeof(T) != 0 || (off >= 0 && o != off)) return p;
+    off = o;
+  }
+  *off0 = off < 0 ? 0 : off / static_cast<int>(sizeof(T));
+  return p;
+}
+
+#define MP_SHIFT_DISPATCH_G(PLAN, CALL, G)                                    \
+  do {                                                                        \
+    if ((PLAN).ppt == 1) { CALL(G, 1); }                                      \
+    else if ((PLAN).ppt == 2) { CALL(G, 2); }                                 \
+    else if ((PLAN).ppt == 3) { CALL(G, 3); }                                 \
+    else if ((PLAN).ppt == 4) { CALL(G, 4); }                                 \
+    else { CALL(G, 5); }                                                      \
+  } while (0)
+#define MP_SHIFT_DISPATCH(PLAN, CALL)                                         \
+  do {                                                                        \
+    if ((PLAN).group == 32) MP_SHIFT_DISPATCH_G(PLAN, CALL, 32);              \
+    else if ((PLAN).group == 128) MP_SHIFT_DISPATCH_G(PLAN, CALL, 128);       \
+    else if ((PLAN).group == 256) MP_SHIFT_DISPATCH_G(PLAN, CALL, 256);       \
+    else if ((PLAN).group == 512) MP_SHIFT_DISPATCH_G(PLAN, CALL, 512);       \
+    else MP_SHIFT_DISPATCH_G(PLAN, CALL, 1024);                               \
+  } while (0)
+// Softmax: one CTA per row group, or one wave of eight per SM (a multiple of every pack length) where that is at most four rows
+// each (the launches then overlap, see MP_OVERLAP_CTAS).
+inline unsigned shift_grid(const RowPlan& p, size_t m) {
+  const size_t groups = (m + p.rows - 1) / p.rows;
+  if (groups > MP_OVERLAP_CTAS && groups / MP_OVERLAP_CTAS < 4) return MP_OVERLAP_CTAS;
+  return static_cast<unsigned>(groups < (1u << 30) ? groups : 1u << 30);
+}
+// RMSNorm forward: a CTA puts the gain together once, so at most one wave of eight per SM (16 % faster at [65536, 4097] r16 than one
+// CTA per row, and than six per SM).
+inline unsigned shift_grid_walk(const RowPlan& p, size_t m) {
+  const size_t groups = (m + p.rows - 1) / p.rows;
+  return static_cast<unsigned>(groups < MP_OVERLAP_CTAS ? groups : MP_OVERLAP_CTAS);
+}
+// RMSNorm reverse: a CTA also leaves a partial row, so as many as are resident (a multiple of every pack length).
+inline unsigned rms_rev_shift_grid(const RowPlan& p, size_t m, int sm_count) {
+  const size_t groups = (m + p.rows - 1) / p.rows;
+  const size_t per_sm = p.threads <= 128 ? 4 : (p.threads <= 256 ? 2 : 1);
+  const size_t cap = (static_cast<size_t>(sm_count > 0 ? sm_count : 148) * per_sm + 7) / 8 * 8;
+  return static_cast<unsigned>(groups < cap ? groups : cap);
+}
 inline size_t rms_rev_warp_grid(size_t m, int sm_count, int per_sm = 3) {
   const size_t want = (m + WROW_THREADS / 32 - 1) / (WROW_THREADS / 32), cap = per_sm * static_cast<size_t>(sm_count > 0 ? sm_count : 148);
   return want < 1 ? 1 : (want < cap ? want : cap);
@@ -1020,7 +1424,13 @@ static void softmax_ij_j_impl(const void* src_, void* dst_, len_t m, len_t n, St
   const RowPlan p = plan_rows<T>(n, mp_aligned16(src) && mp_aligned16(dst));
   cudaStream_t st = mp_stream(ctx);
   const unsigned grid = static_cast<unsigned>(row_grid(p, m, mp_sm_count(ctx), 0));
-  if (p.generic) {
+  int off0 = -1;
+  const RowPlan sp = shift_plan<T>(n, {src, dst}, &off0);
+  if (p.generic && off0 >= 0) {
+#define CALL(G, P) MpLaunch(shift_grid(sp, m), RowCfg<G>::THREADS, 0, st)(softmax_fwd_shift<T, G, P>, src, dst, m, n, off0)
+    MP_SHIFT_DISPATCH(sp, CALL);
+#undef CALL
+  } else if (p.generic) {
     MpLaunch(grid, GEN_THREADS, 0, st)(softmax_fwd_generic<T>, src, dst, m, n);
   } else {
 #define CALL(G, P, F) MpLaunch(grid, RowCfg<G>::THREADS, 0, st)(softmax_fwd_kernel<T, G, P, F>, src, dst, m, n)
@@ -1043,7 +1453,13 @@ static void softmax_ij_j_reverse_impl(const void* y_, const void* gy_, void* gx_
   const A a = static_cast<A>(alpha);
   const bool blend = alpha != 0.0;
   const unsigned grid = static_cast<unsigned>(row_grid(p, m, mp_sm_count(ctx), 0));
-  if (p.generic) {
+  int off0 = -1;
+  const RowPlan sp = shift_plan<T>(n, {y, gy, gx}, &off0);
+  if (p.generic && off0 >= 0) {
+#define CALL(G, P) MpLaunch(shift_grid(sp, m), RowCfg<G>::THREADS, 0, st)(softmax_rev_shift<T, G, P>, y, gy, gx, a, blend, m, n, off0)
+    MP_SHIFT_DISPATCH(sp, CALL);
+#undef CALL
+  } else if (p.generic) {
     MpLaunch(grid, GEN_THREADS, 0, st)(softmax_rev_generic<T>, y, gy, gx, a, blend, m, n);
   } else if (blend) {
 #define CALL(G, P, F) MpLaunch(grid, RowCfg<G>::THREADS, 0, st)(softmax_rev_kernel<T, G, P, F, true>, y, gy, gx, a, m, n)
@@ -1070,7 +1486,13 @@ static void rmsnorm_ij_j_impl(const void* x_, const void* gain_, double eps, voi
   cudaStream_t st = mp_stream(ctx);
   const A e = static_cast<A>(eps);
   const unsigned grid = static_cast<unsigned>(row_grid(p, m, mp_sm_count(ctx), 0));
-  if (p.generic) {
+  int off0 = -1;
+  const RowPlan sp = shift_plan<T>(n, {x, y}, &off0);
+  if (p.generic && off0 >= 0 && mp_aligned16(gain)) {
+#define CALL(G, P) MpLaunch(shift_grid_walk(sp, m), RowCfg<G>::THREADS, 0, st)(rmsnorm_fwd_shift<T, G, P>, x, gain, e, y, rstd, m, n, off0)
+    MP_SHIFT_DISPATCH(sp, CALL);
+#undef CALL
+  } else if (p.generic) {
     MpLaunch(grid, GEN_THREADS, 0, st)(rmsnorm_fwd_generic<T>, x, gain, e, y, rstd, m, n);
   } else {
 #define CALL(G, P, F) MpLaunch(grid, RowCfg<G>::THREADS, 0, st)(rmsnorm_fwd_kernel<T, G, P, F>, x, gain, e, y, rstd, m, n)
@@ -1090,7 +1512,10 @@ static size_t rmsnorm_rev_slots(size_t m, size_t n, int sm_count, bool aligned) 
   const size_t staged = (m + rms_rev_rows_per_cta(m, sm_count) - 1) / rms_rev_rows_per_cta(m, sm_count);  // one slot per CTA
   if (staged > slots) slots = staged;
   const size_t warp_rows = rms_rev_warp_grid(m, sm_count, 3);
-  return slots > warp_rows ? slots : warp_rows;
+  if (warp_rows > slots) slots = warp_rows;
+  int off0 = -1;
+  const size_t shifted = rms_rev_shift_grid(shift_plan<T>(n, {}, &off0), m, sm_count);
+  return slots > shifted ? slots : shifted;
 }
 
 template <typename T>
@@ -1116,6 +1541,8 @@ static void rmsnorm_ij_j_reverse_impl(const void* x_, const void* gain_, const v
     const bool aligned = mp_aligned16(x) && mp_aligned16(gain) && mp_aligned16(gy) && mp_aligned16(gx);
     const RowPlan p = plan_rows_rev<T>(n, aligned);
     const StagedPlan sp = plan_staged<T>(n, aligned);
+    int off0 = -1;
+    const RowPlan shp = shift_plan<T>(n, {x, gy, gx}, &off0);
     const int sms = mp_sm_count(ctx);
     unsigned grid = static_cast<unsigned>(rms_rev_grid(p, m, sms));
     size_t rpc = rms_rev_rows_per_cta((m + p.rows - 1) / p.rows, sms);
@@ -1182,6 +1609,12 @@ static void rmsnorm_ij_j_reverse_impl(const void* x_, const void* gain_, const v
       else { if (sp.full) STG_P(true, false); else STG_P(false, false); }
 #undef STG_P
 #undef STG
+    } else if (p.generic && off0 >= 0 && mp_aligned16(gain)) {
+      grid = rms_rev_shift_grid(shp, m, sms);
+      slots = grid;
+#define CALL(G, P) MpLaunch(grid, RowCfg<G>::THREADS, 0, st)(rmsnorm_rev_shift<T, G, P>, x, gain, rstd, gy, e, gx, a, blend, partial, m, n, off0)
+      MP_SHIFT_DISPATCH(shp, CALL);
+#undef CALL
     } else if (p.generic) {
       MpLaunch(grid, GEN_THREADS, 0, st)(rmsnorm_rev_generic<T>, x, gain, rstd, gy, e, gx, a, blend, partial, m, n, rpc);
     } else if (blend) {

@@ -119,3 +119,58 @@ def test_full_size_properties(mp, stream, sfx):
     ref = (gy.double() * x.double() * rstd).sum(0)
     err = float((gg.double() - ref).abs().max() / ref.abs().max())
     assert err < (1e-2 if sfx == "r16" else 1e-4)
+
+
+# Rows that are not 16-byte aligned.  (m, n): one pack and less, the edges of every row group's packs, several rows per CTA
+# (1184 CTAs), the widest rows of the packed plan and the first beyond it.  offs: elements between a 16-byte boundary and the bases
+# of x and the outputs, of gy, and of gain (a gain off the boundary and tensors at different offsets take the other kernels).
+@pytest.mark.parametrize("sfx", DTYPES)
+@pytest.mark.parametrize("shape,offs", [((9, 5), (0, 0, 0)), ((40, 129), (0, 0, 0)), ((5003, 41), (1, 1, 0)), ((1301, 1283), (0, 0, 0)), ((33, 2561), (1, 1, 0)),
+                                        ((1190, 514), (1, 1, 0)), ((30, 321), (0, 0, 1)), ((30, 322), (1, 0, 0)), ((7, 20477), (0, 0, 0)), ((6, 40959), (0, 0, 0))])
+def test_rows_off_the_16_byte_boundary(mp, stream, sfx, shape, offs):
+    import torch
+    m, n = shape
+    dt = torch_dtype(sfx)
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+
+    def tensor(*size, off=0, fill=None):
+        count = int(np.prod(size))
+        flat = torch.full((count + off + 16,), fill or 0.0, device="cuda", dtype=dt)
+        if fill is None:
+            flat.copy_(torch.randn(count + off + 16, generator=g, device="cuda"))
+        return flat, flat[off:off + count].view(*size)
+
+    (_, x), (_, gy), (_, gain) = tensor(m, n, off=offs[0]), tensor(m, n, off=offs[1]), tensor(n, off=offs[2])
+    gain.mul_(0.02).add_(1)
+
+    def check(flat, out, ref, what):      # guard elements around the output stay as they are
+        assert torch.all(flat[:offs[0]] == 7) and torch.all(flat[offs[0] + m * n:] == 7), what
+        assert float((out.double() - ref).abs().max() / ref.abs().max()) <= TOL_RED[sfx], what
+
+    fresh = lambda: tensor(m, n, off=offs[0], fill=7.0)
+    xd, gd, nd = x.double(), gy.double(), gain.double()
+    f, y = fresh()
+    run(mp, stream, "softmax_ij_j", sfx, x, y, m, n)
+    check(f, y, torch.softmax(xd, 1), "softmax")
+    yd = y.double()
+    sref = yd * (gd - (gd * yd).sum(1, keepdim=True))
+    for alpha in (0.0, 1.0):
+        f, gx = fresh()
+        run(mp, stream, "softmax_ij_j_reverse", sfx, y, gy, gx, alpha, m, n)
+        check(f, gx, sref + 7 * alpha, f"softmax reverse {alpha}")
+    rstd = torch.empty(m, device="cuda", dtype=torch.float64 if sfx == "r64" else torch.float32)
+    f, y = fresh()
+    run(mp, stream, "rmsnorm_ij_j", sfx, x, gain, 1e-6, y, rstd, m, n)
+    rref = 1 / torch.sqrt((xd * xd).mean(1, keepdim=True) + 1e-6)
+    check(f, y, xd * rref * nd, "rmsnorm")
+    assert float((rstd.double() - rref[:, 0]).abs().max() / rref.max()) <= 1e-5
+    scratch = torch.empty(mp.lib().mpRmsnormReverseScratchBytes(m, n, stream.ctx), dtype=torch.uint8, device="cuda")
+    gref = rref * (gd * nd) - xd * rref ** 3 * (gd * nd * xd).mean(1, keepdim=True)
+    for alpha, given in ((0.0, rstd), (1.0, None)):
+        f, gx = fresh()
+        gg = torch.full((n,), 3.0, device="cuda", dtype=dt)
+        run(mp, stream, "rmsnorm_ij_j_reverse", sfx, x, gain, given, gy, 1e-6, gx, gg, alpha, scratch, m, n)
+        check(f, gx, gref + 7 * alpha, f"rmsnorm reverse {alpha}")
+        ggref = (gd * xd * rref).sum(0) + 3 * alpha
+        assert float((gg.double() - ggref).abs().max() / ggref.abs().max()) <= TOL_RED[sfx]
+    assert stream.status() == 0
