@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
   __syncthreads();
   tcgen05_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  mp_grid_dependency();
+  mp_grid_wait();
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -269,6 +269,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
         kc = kend;
       }
     }
+    mp_launch_dependents();
   } else {
     // ------------------------------ epilogue -----------------------------------
     const int quarter = warp & 3;                 // TMEM lanes this warp may read
@@ -488,7 +489,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
   cluster_sync_all();   // both CTAs' barriers and TMEM exist before anything crosses the pair
   tcgen05_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  mp_grid_dependency();
+  mp_grid_wait();
 
   if (warp == 0) {
     // ------------------------------ TMA producer (both ranks) ------------------
@@ -561,6 +562,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
         }
       }
     }
+    mp_launch_dependents();
   } else {
     // ------------------------------ epilogue (both ranks) -----------------------
     const int quarter = warp & 3;

@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(R_THREADS, 1) gemm_r32_kernel(const __grid_con
   __syncthreads();
   tcgen05_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  mp_grid_dependency();
+  mp_grid_wait();
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -175,6 +175,7 @@ __global__ void __launch_bounds__(R_THREADS, 1) gemm_r32_kernel(const __grid_con
         }
       }
     }
+    mp_launch_dependents();
   } else if (warp < R_EPI_FIRST) {
     // ------------------------------ split ---------------------------------------
     const bool does_b = warp >= R_SPLIT_B_FIRST;

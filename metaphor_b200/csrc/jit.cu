@@ -154,8 +154,8 @@ const TypeInfo kTypes[3] = {{"unsigned short", "float", 8, 2}, {"float", "float"
 
 // mp_grid_dependency() of mp_common.cuh: the kernels are launched like the library's own.
 const std::string kGridDependency = "  if (gridDim.x <= " + std::to_string(MP_OVERLAP_CTAS) +
-                                    "u) {\n    asm volatile(\"griddepcontrol.launch_dependents;\" ::: \"memory\");\n"
-                                    "    asm volatile(\"griddepcontrol.wait;\" ::: \"memory\");\n  }\n";
+                                    "u) {\n    asm volatile(\"griddepcontrol.wait;\" ::: \"memory\");\n"
+                                    "    asm volatile(\"griddepcontrol.launch_dependents;\" ::: \"memory\");\n  }\n";
 
 std::string lit(double v, const char* acc) {
   std::ostringstream o;

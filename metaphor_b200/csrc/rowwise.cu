@@ -1396,11 +1396,12 @@ inline unsigned shift_grid_walk(const RowPlan& p, size_t m) {
   const size_t groups = (m + p.rows - 1) / p.rows;
   return static_cast<unsigned>(groups < MP_OVERLAP_CTAS ? groups : MP_OVERLAP_CTAS);
 }
-// RMSNorm reverse: a CTA also leaves a partial row, so as many as are resident (a multiple of every pack length).
+// RMSNorm reverse: a CTA also leaves a partial row, so no more than are resident (a multiple of every
+// pack length, rounded down: four CTAs in a second wave doubled the time of wide rows).
 inline unsigned rms_rev_shift_grid(const RowPlan& p, size_t m, int sm_count) {
   const size_t groups = (m + p.rows - 1) / p.rows;
   const size_t per_sm = p.threads <= 128 ? 4 : (p.threads <= 256 ? 2 : 1);
-  const size_t cap = (static_cast<size_t>(sm_count > 0 ? sm_count : 148) * per_sm + 7) / 8 * 8;
+  const size_t sms = sm_count > 7 ? sm_count : 148, cap = sms * per_sm / 8 * 8;
   return static_cast<unsigned>(groups < cap ? groups : cap);
 }
 inline size_t rms_rev_warp_grid(size_t m, int sm_count, int per_sm = 3) {

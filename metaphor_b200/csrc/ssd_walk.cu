@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_con
   __syncthreads();
   tcgen05_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  mp_grid_dependency();
+  mp_grid_wait();
 
 
   if (warp == 0) {
@@ -273,6 +273,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_con
       }
       qb += sg.n;
     }
+    mp_launch_dependents();
     if (g.hs_out != nullptr) bulk_wait_all<0>();
   } else {
     // ------------------------------ workers -----------------------------------
@@ -645,7 +646,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_group_grads_kernel(const __g
   __syncthreads();
   tcgen05_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
-  mp_grid_dependency();
+  mp_grid_wait();
 
   if (warp == 0) {
     // ------------------------------ TMA: loads, then the output stores -------------
@@ -744,6 +745,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_group_grads_kernel(const __g
       }
       __syncwarp();
     }
+    mp_launch_dependents();
   } else {
     // ------------------------------ workers -----------------------------------
     const int quarter = warp & 3;
