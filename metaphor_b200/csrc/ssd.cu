@@ -604,44 +604,25 @@ __global__ void __launch_bounds__(256) ssd_boundary_dot_kernel(const __half* __r
 }
 
 // One CTA per (b, h); one thread per step of a chunk (Q <= 256), chunks walked from the last to the first.
-// u, v, dtt: [B, H, LP], LP = L padded to whole chunks (dt = 0 there).  `halves` = 2: u and v are the sums of two arrays, the
-// second `B*H*LP` elements after the first.
-// With `raw` (the projection's raw step sizes, r16, pitched) the reverse of dt = softplus(raw + bias[h]) is applied on the
-// way out: graw = gdt * sigmoid(raw + bias) (r16, pitched), gbias[h] += its sum (the arithmetic of launch_softplus_bias_reverse).
-__device__ __forceinline__ float ssd_sigmoid(float x) {
-  float e, r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * -1.4426950408889634f));
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
-  return r;
-}
 __global__ void __launch_bounds__(256) ssd_scalar_grads_kernel(const float* __restrict__ u, const float* __restrict__ v,
                                                                const float* __restrict__ dtt, const float* __restrict__ A,
                                                                const float* __restrict__ pin, float* __restrict__ gdt,
-                                                               float* __restrict__ gA_part, int B, int L, int LP, int H, int Q, int halves,
-                                                               const __half* __restrict__ raw, size_t raw_pitch,
-                                                               const float* __restrict__ bias, __half* __restrict__ graw,
-                                                               size_t graw_pitch, float* __restrict__ gbias) {
+                                                               float* __restrict__ gA_part, int B, int L, int H, int Q) {
   mp_grid_dependency();
   __shared__ float warp_tot[8];
   __shared__ float total_s;
   __shared__ float ga_red[8];
-  __shared__ float gb_red[8];
-  float gb_acc = 0.f;
   const int h = blockIdx.x % H, b = blockIdx.x / H;
-  const size_t base = (static_cast<size_t>(b) * H + h) * LP;
-  const int nc = LP / Q;
+  const size_t base = (static_cast<size_t>(b) * H + h) * L;
+  const int nc = L / Q;
   const float Ah = A[h];
   float ga_acc = 0.f;
   for (int c = nc - 1; c >= 0; --c) {
     const int j = static_cast<int>(threadIdx.x);           // thread 0 holds the latest step of the chunk
     const int t = c * Q + (Q - 1 - j);
     const bool in = j < Q;
-    const size_t hs = static_cast<size_t>(B) * H * LP;
     float ut = 0.f, vt = 0.f;
-    if (in) {
-      ut = u[base + t]; vt = v[base + t];
-      if (halves == 2) { ut += u[hs + base + t]; vt += v[hs + base + t]; }
-    }
+    if (in) { ut = u[base + t]; vt = v[base + t]; }
     const float d = ut - vt;
     float s = d;
 #pragma unroll
@@ -659,30 +640,23 @@ __global__ void __launch_bounds__(256) ssd_scalar_grads_kernel(const float* __re
     const float right = pin[(static_cast<size_t>(b) * H + h) * nc + c];          // g_a just after the chunk
     float resid = 0.f;
     if (c > 0) resid = pin[(static_cast<size_t>(b) * H + h) * nc + c - 1] - (right + total_s);   // what the first step should reach
-    if (in && t < L) {
+    if (in) {
       const float ga = right + within + resid * (static_cast<float>(j + 1) / static_cast<float>(Q));
       const float dtv = dtt[base + t];
       const float gd = vt / dtv + Ah * ga;
       const size_t row = static_cast<size_t>(b) * L + t;
       gdt[row * H + h] = gd;
       ga_acc += dtv * ga;
-      if (raw != nullptr) {
-        const float gr = gd * ssd_sigmoid(__half2float(raw[row * raw_pitch + h]) + bias[h]);
-        graw[row * graw_pitch + h] = __float2half_rn(gr);
-        gb_acc += gr;
-      }
     }
     __syncthreads();
   }
   ga_acc = warp_reduce<SumOp>(ga_acc);
-  gb_acc = warp_reduce<SumOp>(gb_acc);
-  if ((threadIdx.x & 31) == 0) { ga_red[threadIdx.x >> 5] = ga_acc; gb_red[threadIdx.x >> 5] = gb_acc; }
+  if ((threadIdx.x & 31) == 0) ga_red[threadIdx.x >> 5] = ga_acc;
   __syncthreads();
   if (threadIdx.x == 0) {
-    float t = 0.f, tb = 0.f;
-    for (int w = 0; w < 8; ++w) { t += ga_red[w]; tb += gb_red[w]; }
+    float t = 0.f;
+    for (int w = 0; w < 8; ++w) t += ga_red[w];
     gA_part[blockIdx.x] = t;
-    if (raw != nullptr && gbias != nullptr) atomicAdd(gbias + h, tb);
   }
 }
 
@@ -704,16 +678,14 @@ __global__ void __launch_bounds__(256) ssd_fold_parts_kernel(const float* __rest
   st_pack(out + i, 0, pack<__half>(acc));
 }
 
-// gA[h] = sum over the batch; with A_log's gradient wanted (A = -exp(A_log), so dA / dA_log = A): gA_log[h] += gA[h] * A[h]
-__global__ void ssd_sum_batches_kernel(const float* __restrict__ part, float* __restrict__ gA, int B, int H,
-                                       const float* __restrict__ A, float* __restrict__ gA_log) {
+// gA[h] = sum over the batch
+__global__ void ssd_sum_batches_kernel(const float* __restrict__ part, float* __restrict__ gA, int B, int H) {
   mp_grid_dependency();
   const int h = blockIdx.x * blockDim.x + threadIdx.x;
   if (h >= H) return;
   float s = 0.f;
   for (int b = 0; b < B; ++b) s += part[b * H + h];
   gA[h] = s;
-  if (gA_log != nullptr) gA_log[h] += s * A[h];
 }
 
 // ---------------------------------------------------------------------------
@@ -952,17 +924,20 @@ void mp_ssd_walk_cumsum(const float* dt, const float* A, float* cum, float* dtt,
 void mp_ssd_walk_cumsum_raw(const __half* raw, size_t raw_pitch, const float* bias, const float* A_log, float* dt_out, float* A_out, float* cum,
                             float* dtt, float* colf_c, int B, int L, int H, int* carry_flags, int n_flags, cudaStream_t st);
 void mp_ssd_walk(int anti, const __half* q, const __half* k, const __half* v, const float* cum, const float* dtt, const float* colf, __half* out,
-                 const __half* z, float* dot_out, __half* hs_out, float* carry, int* carry_flag, int max_ctas, int B, int L, int H, int G,
+                 const __half* z, float* dot_out, float* state_dot, __half* hs_out, float* carry, int* carry_flag, int max_ctas, int B, int L, int H, int G,
                  uint32_t* status, cudaStream_t st);
 
 void mp_ssd_group_grads(const __half* gy, const __half* x, const __half* Bm, const __half* Cm, const __half* hs_causal, const __half* hs_anti,
-                        const float* cum, const float* dtt, const float* colf_c, __half* gB, __half* gC, int B, int L, int H, int G,
-                        uint32_t* status, cudaStream_t st);
+                        const float* cum, const float* dtt, const float* colf_c, float* state_dot, __half* gB, __half* gC, int B, int L,
+                        int H, int G, uint32_t* status, cudaStream_t st);
+void mp_ssd_walk_scalars(const float* u, const float* v, const float* dtt, const float* A, const float* pin, float* gdt, float* gA, float* ga_part,
+                         float* gb_part, const __half* raw, size_t raw_pitch, const float* bias, __half* graw, size_t graw_pitch, float* gbias,
+                         float* gA_log, int B, int L, int H, cudaStream_t st);
 
 namespace {
 // Scratch of the walk path: prefix sums and dt in [B,H,L] order; for the reverse also the states every 128-step
 // chunk receives from its predecessors and from its successors (r16 [B,H,L/128][128][64]).
-struct WalkScratch { float* cum; float* dtt; float* colf_c; float* colf_a; __half* hs_causal; __half* hs_anti; float* pin; float* u; float* v; float* ga_part; float* carry_c; float* carry_a; int* flags; size_t total; };
+struct WalkScratch { float* cum; float* dtt; float* colf_c; float* colf_a; __half* hs_causal; __half* hs_anti; float* pin; float* u; float* v; float* ga_part; float* gb_part; float* carry_c; float* carry_a; int* flags; size_t total; };
 // The forward takes the chunk walk where it applies; MP_SSD_LEGACY_FORWARD selects the three-phase path on the shapes that it has too.
 bool ssd_forward_walks(const SsdDims& d) {
   return mp_ssd_walk_supported(d.L, d.H, d.P, d.N, d.G) && (getenv("MP_SSD_LEGACY_FORWARD") == nullptr || !ssd_whole_chunks(d));
@@ -980,10 +955,11 @@ WalkScratch walk_carve(void* base, const SsdDims& d, bool reverse, size_t off0) 
   const size_t st = static_cast<size_t>(d.B) * d.H * nc * 128 * 64 * 2;
   w.hs_causal = static_cast<__half*>(take(reverse ? st : 0));
   w.hs_anti = static_cast<__half*>(take(reverse ? st : 0));
-  w.pin = static_cast<float*>(take(reverse ? static_cast<size_t>(d.B) * d.H * nc * 4 : 0));
+  w.pin = static_cast<float*>(take(reverse ? static_cast<size_t>(d.B) * d.H * nc * 16 * 4 : 0));   // sixteen parts each
   w.u = static_cast<float*>(take(reverse ? 2 * bhl * 4 : 0));     // one array per half of the columns
   w.v = static_cast<float*>(take(reverse ? 2 * bhl * 4 : 0));
-  w.ga_part = static_cast<float*>(take(reverse ? static_cast<size_t>(d.B) * d.H * 4 : 0));
+  w.ga_part = static_cast<float*>(take(reverse ? static_cast<size_t>(d.B) * d.H * nc * 4 : 0));
+  w.gb_part = static_cast<float*>(take(reverse ? static_cast<size_t>(d.B) * d.H * nc * 4 : 0));
   // states handed from CTA to CTA inside a walk (fp32 [128][64] per sequence and walk) and their arrival counters
   const size_t carry = static_cast<size_t>(d.B) * d.H * 128 * 64 * 4;
   w.carry_c = static_cast<float*>(take(carry));
@@ -1029,7 +1005,7 @@ extern "C" void launch_ssd_scan_r16(const void* x, const void* dt, const void* A
     mp_ssd_walk_cumsum(static_cast<const float*>(dt), static_cast<const float*>(A), w.cum, w.dtt, w.colf_c, nullptr, d.B, d.L, d.H, w.flags,
                        2 * d.B * d.H, st);
     mp_ssd_walk(0, static_cast<const __half*>(Cm), static_cast<const __half*>(Bm), static_cast<const __half*>(x), w.cum, w.dtt, w.colf_c,
-                static_cast<__half*>(y), nullptr, nullptr, nullptr, w.carry_c, w.flags, state->sm_count, d.B, d.L, d.H, d.G, state->status_dev,
+                static_cast<__half*>(y), nullptr, nullptr, nullptr, nullptr, w.carry_c, w.flags, state->sm_count, d.B, d.L, d.H, d.G, state->status_dev,
                 st);
     return;
   }
@@ -1077,7 +1053,7 @@ extern "C" void launch_ssd_scan_raw_r16(const void* x, const void* dt_raw, len_t
     mp_ssd_walk_cumsum_raw(static_cast<const __half*>(dt_raw), dt_pitch, static_cast<const float*>(dt_bias), static_cast<const float*>(A_log),
                            static_cast<float*>(dt_out), static_cast<float*>(A_out), w.cum, w.dtt, w.colf_c, d.B, d.L, d.H, w.flags, 2 * d.B * d.H, st);
     mp_ssd_walk(0, static_cast<const __half*>(Cm), static_cast<const __half*>(Bm), static_cast<const __half*>(x), w.cum, w.dtt, w.colf_c,
-                static_cast<__half*>(y), nullptr, nullptr, nullptr, w.carry_c, w.flags, state->sm_count, d.B, d.L, d.H, d.G, state->status_dev,
+                static_cast<__half*>(y), nullptr, nullptr, nullptr, nullptr, w.carry_c, w.flags, state->sm_count, d.B, d.L, d.H, d.G, state->status_dev,
                 st);
     return;
   }
@@ -1152,35 +1128,21 @@ static bool ssd_scan_reverse_r16_impl(const void* x, const void* dt, const void*
       MP_CUDA_CHECK(cudaEventRecord(state->aux_fork, st));
       MP_CUDA_CHECK(cudaStreamWaitEvent(lane1, state->aux_fork, 0));
     }
-    mp_ssd_walk(1, bh, ch, gyh, w.cum, w.dtt, w.colf_a, static_cast<__half*>(gx), xh, w.v, w.hs_anti, w.carry_a, w.flags + d.B * d.H, walk_ctas,
+    mp_ssd_walk(1, bh, ch, gyh, w.cum, w.dtt, w.colf_a, static_cast<__half*>(gx), xh, w.v, nullptr, w.hs_anti, w.carry_a, w.flags + d.B * d.H, walk_ctas,
                 d.B, d.L, d.H, d.G, state->status_dev, st);
-    mp_ssd_walk(0, ch, bh, xh, w.cum, w.dtt, w.colf_c, nullptr, gyh, w.u, w.hs_causal, w.carry_c, w.flags, walk_ctas, d.B, d.L, d.H, d.G,
+    mp_ssd_walk(0, ch, bh, xh, w.cum, w.dtt, w.colf_c, nullptr, gyh, w.u, w.pin, w.hs_causal, w.carry_c, w.flags, walk_ctas, d.B, d.L, d.H, d.G,
                 state->status_dev, lane1);
     if (side) {
       MP_CUDA_CHECK(cudaEventRecord(state->aux_join[0], lane1));
       MP_CUDA_CHECK(cudaStreamWaitEvent(st, state->aux_join[0], 0));
-      // gdt / gA need both walks (u, v, states) but not gB / gC: they run beside the group-gradient kernel
-      MP_CUDA_CHECK(cudaEventRecord(state->aux_sub_fork[0], st));
-      MP_CUDA_CHECK(cudaStreamWaitEvent(lane1, state->aux_sub_fork[0], 0));
     }
-    mp_ssd_group_grads(gyh, xh, bh, ch, w.hs_causal, w.hs_anti, w.cum, w.dtt, w.colf_c, static_cast<__half*>(gB), static_cast<__half*>(gC),
+    mp_ssd_group_grads(gyh, xh, bh, ch, w.hs_causal, w.hs_anti, w.cum, w.dtt, w.colf_c, w.pin, static_cast<__half*>(gB), static_cast<__half*>(gC),
                        d.B, d.L, d.H, d.G, state->status_dev, st);
-    const int wnc = (d.L + 127) / 128;
-    MpLaunch(d.B * d.H * wnc, 256, 0, lane1)(ssd_boundary_dot_kernel, w.hs_anti, w.hs_causal, w.pin, wnc, d.N * d.P);
-    MP_LAUNCH_CHECK();
     const RawSide none{nullptr, 0, nullptr, nullptr, 0, nullptr, nullptr};
     const RawSide& side_out = rs != nullptr ? *rs : none;
-    MpLaunch(d.B * d.H, 256, 0, lane1)(ssd_scalar_grads_kernel, w.u, w.v, w.dtt, static_cast<const float*>(A), w.pin, static_cast<float*>(gdt), w.ga_part,
-                                       d.B, d.L, wnc * 128, d.H, 128, 2, side_out.raw, side_out.raw_pitch, side_out.bias, side_out.graw,
-                                       side_out.graw_pitch, side_out.gbias);
-    MP_LAUNCH_CHECK();
-    MpLaunch((d.H + 127) / 128, 128, 0, lane1)(ssd_sum_batches_kernel, w.ga_part, static_cast<float*>(gA), d.B, d.H, static_cast<const float*>(A),
-                                                                 rs != nullptr ? rs->gA_log : nullptr);
-    MP_LAUNCH_CHECK();
-    if (side) {
-      MP_CUDA_CHECK(cudaEventRecord(state->aux_join[1], lane1));
-      MP_CUDA_CHECK(cudaStreamWaitEvent(st, state->aux_join[1], 0));
-    }
+    mp_ssd_walk_scalars(w.u, w.v, w.dtt, static_cast<const float*>(A), w.pin, static_cast<float*>(gdt), static_cast<float*>(gA), w.ga_part, w.gb_part,
+                        side_out.raw, side_out.raw_pitch, side_out.bias, side_out.graw, side_out.graw_pitch, side_out.gbias, side_out.gA_log, d.B, d.L,
+                        d.H, st);
     return true;
   }
   const SsdScratch sc = ssd_carve(scratch, d, true);
@@ -1242,9 +1204,9 @@ static bool ssd_scan_reverse_r16_impl(const void* x, const void* dt, const void*
     MpLaunch(d.B * d.H * d.nc, 256, 0, st)(ssd_boundary_dot_kernel, sc.hs_op[0], sc.hs_op[1], sc.pin, d.nc, d.N * d.P);
     MP_LAUNCH_CHECK();
     MpLaunch(d.B * d.H, 256, 0, st)(ssd_scalar_grads_kernel, sc.u, sc.v, sc.dtt, static_cast<const float*>(A), sc.pin, static_cast<float*>(gdt),
-                                                      sc.ga_part, d.B, d.L, d.L, d.H, d.Q, 1, nullptr, 0, nullptr, nullptr, 0, nullptr);
+                                                      sc.ga_part, d.B, d.L, d.H, d.Q);
     MP_LAUNCH_CHECK();
-  MpLaunch((d.H + 127) / 128, 128, 0, st)(ssd_sum_batches_kernel, sc.ga_part, static_cast<float*>(gA), d.B, d.H, nullptr, nullptr);
+  MpLaunch((d.H + 127) / 128, 128, 0, st)(ssd_sum_batches_kernel, sc.ga_part, static_cast<float*>(gA), d.B, d.H);
   MP_LAUNCH_CHECK();
   return false;
 }

@@ -59,6 +59,7 @@ struct WalkArgs {
   __half* out;             // [B*L, H*64] or null
   const __half* z;         // dot partner, same indexing as out, or null
   float* dot_out;          // [2][B, H, LP] row dots <z, out> from the fp32 accumulators, one array per half of the columns, or null
+  float* state_dot;        // [B, H, nc][16], first eight: sums over a chunk's rows of <z, the received state's share of out>, one per worker warp, or null
   __half* hs_out;          // [B, H, nc][128][64]: state every chunk receives, or null
   float* carry;            // [B * H][128][64] fp32: state handed from the CTA that walked the first part of a sequence to the next
   int* carry_flag;         // [B * H]: number of worker warps (of 8) that have written their part of `carry`; zero before the launch
@@ -510,12 +511,9 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_con
 #pragma unroll
           for (int e = 0; e < 32; ++e) yo[e] = 0u;
         }
-        float o[32];
-#pragma unroll
-        for (int e = 0; e < 32; ++e) o[e] = ro * (__uint_as_float(yd[e]) + fo * __uint_as_float(yo[e]));
         tcgen05_fence_before_sync();
         if (DOT) {   // this thread's row of z comes back from the staging positions before the output overwrites them
-          float dot = 0.f;
+          float dot = 0.f, dot_state = 0.f;
 #pragma unroll
           for (int q4 = 0; q4 < 4; ++q4) {
             const uint4 zq = *reinterpret_cast<const uint4*>(stg + r * 128 + (((ch * 4 + q4) ^ (r & 7)) << 4));
@@ -523,12 +521,22 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_con
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               const float2 zf = __half22float2(z2[e]);
-              dot += zf.x * o[q4 * 8 + 2 * e] + zf.y * o[q4 * 8 + 2 * e + 1];
+              const int k0 = q4 * 8 + 2 * e;
+              dot += zf.x * __uint_as_float(yd[k0]) + zf.y * __uint_as_float(yd[k0 + 1]);
+              dot_state += zf.x * __uint_as_float(yo[k0]) + zf.y * __uint_as_float(yo[k0 + 1]);
             }
           }
-          g.dot_out[static_cast<size_t>(ch) * g.B * g.H * (static_cast<size_t>(g.nc) * WQ) + step0 + c * WQ] = dot;
+          dot_state *= ro * fo;
+          g.dot_out[static_cast<size_t>(ch) * g.B * g.H * (static_cast<size_t>(g.nc) * WQ) + step0 + c * WQ] = ro * dot + dot_state;
+          if (g.state_dot != nullptr) {
+            dot_state = warp_reduce<SumOp>(dot_state);
+            if (lane == 0) g.state_dot[(bh * g.nc + c) * 16 + (warp - 2)] = dot_state;
+          }
           __syncwarp();
         }
+        float o[32];
+#pragma unroll
+        for (int e = 0; e < 32; ++e) o[e] = ro * (__uint_as_float(yd[e]) + fo * __uint_as_float(yo[e]));
         if (g.out != nullptr) {
 #pragma unroll
           for (int q4 = 0; q4 < 4; ++q4) {
@@ -604,6 +612,7 @@ enum { GB_FULL0 = 0, GB_FULL1, GB_EMPTY0, GB_EMPTY1, GB_SC0, GB_SC1, GB_SCALED, 
 struct GroupArgs {
   int B, L, H, G, nc;
   const float* cum; const float* dtt; const float* colf;   // [B, H, nc * 128], causal column factors
+  float* state_dot;                                        // [B, H, nc][16], last eight: exp(cum_last) <Hc, Ha>, one part per worker warp
   uint32_t* status;
 };
 
@@ -810,9 +819,20 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_group_grads_kernel(const __g
         const __half2 w2 = __float2half2_rn(w_exp(cum_last - cum_r) * dt_r);
         unsigned char* gyrow = smem + s * GG_STAGE + r * 128;
         unsigned char* xrow = gyrow + GG_TILE;
+        float hdot = 0.f;
 #pragma unroll
         for (int q4 = 0; q4 < 4; ++q4) {
           const int off = ((ch * 4 + q4) ^ (r & 7)) << 4;
+          {   // <Hc, Ha> of the chunk: see ssd_walk_scalars_kernel
+            const uint4 c4 = *reinterpret_cast<const uint4*>(gyrow + 2 * GG_TILE + off), a4 = *reinterpret_cast<const uint4*>(gyrow + 3 * GG_TILE + off);
+            const __half2* hc = reinterpret_cast<const __half2*>(&c4);
+            const __half2* ha2 = reinterpret_cast<const __half2*>(&a4);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float2 p = __half22float2(hc[e]), q = __half22float2(ha2[e]);
+              hdot += p.x * q.x + p.y * q.y;
+            }
+          }
           uint4 a = *reinterpret_cast<const uint4*>(gyrow + off);
           uint4 x4 = *reinterpret_cast<const uint4*>(xrow + off);
           __half2* ha = reinterpret_cast<__half2*>(&a);
@@ -822,6 +842,8 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_group_grads_kernel(const __g
           *reinterpret_cast<uint4*>(gyrow + off) = a;
           *reinterpret_cast<uint4*>(xrow + off) = x4;
         }
+        hdot = warp_reduce<SumOp>(hdot * w_exp(cum_last));
+        if (lane == 0) g.state_dot[((static_cast<size_t>(b) * g.H + grp * hpg + hi) * g.nc + c) * 16 + 8 + (warp - 2)] = hdot;
       }
       warp_arrive(bars + GB_SCALED, lane);
     }
@@ -874,56 +896,199 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_group_grads_kernel(const __g
 }
 
 // dt*A prefix sums inside every 128-step chunk, dt, and the column factors of both walk directions, all in
-// [B, H, nc * 128] order (steps beyond the sequence: dt = 0).  One CTA per (b, h, chunk).  Column factor of step t relative to the far end of its 8-step
-// piece: causal exp(cum[t | 7] - cum[t]) dt[t], anti-causal exp(cum[t] - cum[t & ~7]); both are at most one (dt).
+// [B, H, nc * 128] order (steps beyond the sequence: dt = 0).  One CTA per (b, chunk, eight heads), one warp per head, four
+// neighbouring steps per lane; dt comes in as rows of eight heads (one sector each) through shared memory, where one head per CTA
+// read a sector for every value.
+// Column factor of step t relative to the far end of its 8-step piece: causal exp(cum[t | 7] - cum[t]) dt[t], anti-causal
+// exp(cum[t] - cum[t & ~7]); both are at most one (dt).
 // RAW: the step sizes arrive as the projection's raw r16 output (row pitch `raw_pitch`) and the decay rates as A_log:
 //   dt = softplus(raw + bias[h]), A = -exp(A_log[h])  (the arithmetic of launch_softplus_bias / launch_neg_exp),
 // both also written out (dt_out [B, L, H], A_out [H]) for the reverse pass.
+constexpr int WS_HEADS = 8;                    // heads per CTA of the two scalar kernels
+constexpr int WS_THREADS = 32 * WS_HEADS;
 template <bool RAW>
-__global__ void __launch_bounds__(WQ) ssd_walk_cumsum_kernel(const float* __restrict__ dt, const float* __restrict__ A, float* __restrict__ cum,
-                                                             float* __restrict__ dtt, float* __restrict__ colf_c, float* __restrict__ colf_a,
-                                                             int L, int H, int* __restrict__ carry_flags, int n_flags,
-                                                             const __half* __restrict__ raw, size_t raw_pitch, const float* __restrict__ bias,
-                                                             float* __restrict__ dt_out, float* __restrict__ A_out) {
+__global__ void __launch_bounds__(WS_THREADS) ssd_walk_cumsum_kernel(const float* __restrict__ dt, const float* __restrict__ A,
+                                                                     float* __restrict__ cum, float* __restrict__ dtt,
+                                                                     float* __restrict__ colf_c, float* __restrict__ colf_a, int L, int H, int hblocks,
+                                                                     int* __restrict__ carry_flags, int n_flags, const __half* __restrict__ raw,
+                                                                     size_t raw_pitch, const float* __restrict__ bias, float* __restrict__ dt_out,
+                                                                     float* __restrict__ A_out) {
   mp_grid_dependency();
-  __shared__ float warp_tot[4];
+  __shared__ float s_dt[WQ][WS_HEADS + 1];
   if (blockIdx.x == 0)   // the walks that follow in stream order hand states from CTA to CTA through these counters
-    for (int i = threadIdx.x; i < n_flags; i += WQ) carry_flags[i] = 0;
+    for (int i = threadIdx.x; i < n_flags; i += WS_THREADS) carry_flags[i] = 0;
   const int nc = (L + WQ - 1) / WQ;
-  const int c = blockIdx.x % nc, h = (blockIdx.x / nc) % H, b = blockIdx.x / (nc * H);
-  const int t = threadIdx.x;
-  const bool inside = c * WQ + t < L;
-  const size_t row = static_cast<size_t>(b) * L + c * WQ + t;
-  float d = 0.f, a;
-  if (RAW) {
-    a = -__expf(A[h]);
-    if (inside) {
-      const float pre = __half2float(raw[row * raw_pitch + h]) + bias[h];
-      d = pre > 20.f ? pre : log1pf(__expf(pre));
-      dt_out[row * H + h] = d;
+  const int h0 = static_cast<int>(blockIdx.x % hblocks) * WS_HEADS, bc = blockIdx.x / hblocks, c = bc % nc, b = bc / nc;
+#pragma unroll
+  for (int k = 0; k < WQ * WS_HEADS / WS_THREADS; ++k) {
+    const int idx = k * WS_THREADS + threadIdx.x, t = idx / WS_HEADS, h = h0 + idx % WS_HEADS;
+    float d = 0.f;
+    if (c * WQ + t < L && h < H) {
+      const size_t row = static_cast<size_t>(b) * L + c * WQ + t;
+      if (RAW) {
+        const float pre = __half2float(raw[row * raw_pitch + h]) + bias[h];
+        d = pre > 20.f ? pre : log1pf(__expf(pre));
+        dt_out[row * H + h] = d;
+      } else {
+        d = dt[row * H + h];
+      }
     }
-    if (b == 0 && c == 0 && t == 0) A_out[h] = a;
-  } else {
-    if (inside) d = dt[row * H + h];
-    a = A[h];
+    s_dt[t][idx % WS_HEADS] = d;
   }
-  float v = d * a;
+  __syncthreads();
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, h = h0 + w;
+  if (h >= H) return;
+  const float a = RAW ? -__expf(A[h]) : A[h];
+  if (RAW && bc == 0 && lane == 0) A_out[h] = a;
+  float d[4], v[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    d[e] = s_dt[lane * 4 + e][w];
+    v[e] = d[e] * a + (e > 0 ? v[e - 1] : 0.f);
+  }
+  float incl = v[3];
 #pragma unroll
   for (int off = 1; off < 32; off <<= 1) {
-    const float n = __shfl_up_sync(0xffffffffu, v, off);
-    if ((t & 31) >= off) v += n;
+    const float up = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += up;
   }
-  if ((t & 31) == 31) warp_tot[t >> 5] = v;
+  const float base = incl - v[3];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) v[e] += base;
+  const float c_hi = __shfl_sync(0xffffffffu, v[3], lane | 1), c_lo = __shfl_sync(0xffffffffu, v[0], lane & ~1);
+  const size_t o = (static_cast<size_t>(b) * H + h) * (static_cast<size_t>(nc) * WQ) + c * WQ + lane * 4;
+  *reinterpret_cast<float4*>(cum + o) = make_float4(v[0], v[1], v[2], v[3]);
+  *reinterpret_cast<float4*>(dtt + o) = make_float4(d[0], d[1], d[2], d[3]);
+  *reinterpret_cast<float4*>(colf_c + o) = make_float4(w_exp(c_hi - v[0]) * d[0], w_exp(c_hi - v[1]) * d[1], w_exp(c_hi - v[2]) * d[2], w_exp(c_hi - v[3]) * d[3]);
+  if (colf_a != nullptr) *reinterpret_cast<float4*>(colf_a + o) = make_float4(w_exp(v[0] - c_lo), w_exp(v[1] - c_lo), w_exp(v[2] - c_lo), w_exp(v[3] - c_lo));
+}
+
+// ---------------------------------------------------------------------------
+// gdt, gA from the walks' row dots u = <gy, y>, v = <gx, x>.  With g_a_t the gradient of the loss with respect to dt_t A_h:
+//   g_a_t = g_a_{t+1} + u_t - v_t,  gdt_t = v_t / dt_t + A_h g_a_t,  gA_h = sum_t dt_t g_a_t.
+// u_t - v_t cancels and carries the rounding noise of two different operator instances, so a suffix sum over the whole
+// sequence random-walks (measured: gA off by 5 % at 8192 steps).  The sum is therefore pinned at every chunk boundary to a value
+// without such noise, summed only inside a chunk, and the residual between a chunk's two pins is spread linearly over its steps.
+//   pin(c) = g_a at the first step of chunk c = < what chunk c-1 receives from its successors, Hc = what chunk c receives from its
+//            predecessors >  and, the first factor being exp(cum_last) Ha + sum_i e_i C_i gy_i^T over the steps i of chunk c,
+//          = exp(cum_last) <Hc, Ha>  [the group-gradient kernel, which has both tiles in shared memory]
+//            + sum_i (the received state's share of u_i)  [the causal walk]
+// (state_dot, eight parts of each), so the states are not read again for it: a kernel of its own spent 89 us on that for
+// [8, 8192, 32, 64] and 70 us for [8, 2048, 24, 64].
+// Every chunk is then on its own: one CTA per (b, chunk, eight heads), one warp per head, four neighbouring steps per lane, and
+// gdt (and graw) leave as rows of eight heads.
+// With `raw` (the projection's raw step sizes, r16, pitched) the reverse of dt = softplus(raw + bias[h]) is applied on the
+// way out: graw = gdt * sigmoid(raw + bias) (r16, pitched); its sums go to gb_part (the arithmetic of launch_softplus_bias_reverse).
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ float walk_sigmoid(float x) {
+  float e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * -1.4426950408889634f));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
+  return r;
+}
+struct ScalarArgs {
+  const float* u; const float* v;   // [2][B, H, nc * 128]: one array per half of the columns
+  const float* dtt;                 // [B, H, nc * 128]
+  const float* A;
+  const float* pin;                 // [B, H, nc][16]
+  float* gdt;                       // [B, L, H]
+  float* ga_part; float* gb_part;   // [B * nc][H]
+  const __half* raw; size_t raw_pitch; const float* bias; __half* graw; size_t graw_pitch;
+  int B, L, H, nc, hblocks;
+};
+template <bool RAW>
+__global__ void __launch_bounds__(WS_THREADS) ssd_walk_scalars_kernel(const ScalarArgs g) {
+  mp_grid_dependency();
+  __shared__ float s_gd[WQ][WS_HEADS + 1];
+  const int h0 = static_cast<int>(blockIdx.x % g.hblocks) * WS_HEADS, bc = blockIdx.x / g.hblocks, c = bc % g.nc, b = bc / g.nc;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, h = h0 + w;
+  if (h < g.H) {
+    const size_t bh = static_cast<size_t>(b) * g.H + h, LP = static_cast<size_t>(g.nc) * WQ, half = static_cast<size_t>(g.B) * g.H * LP;
+    const size_t o = bh * LP + c * WQ + lane * 4;
+    const float4 u0 = *reinterpret_cast<const float4*>(g.u + o), u1 = *reinterpret_cast<const float4*>(g.u + half + o);
+    const float4 v0 = *reinterpret_cast<const float4*>(g.v + o), v1 = *reinterpret_cast<const float4*>(g.v + half + o);
+    const float4 d4 = *reinterpret_cast<const float4*>(g.dtt + o);
+    // lanes 0-15: the parts of this chunk's pin, lanes 16-31: those of the next chunk's (zero behind the last chunk)
+    float part = 0.f;
+    if (lane < 16 || c + 1 < g.nc) part = g.pin[(bh * g.nc + c) * 16 + lane];
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1) part += __shfl_xor_sync(0xffffffffu, part, off);
+    const float left = __shfl_sync(0xffffffffu, part, 0), right = __shfl_sync(0xffffffffu, part, 16);
+    const float vt[4] = {v0.x + v1.x, v0.y + v1.y, v0.z + v1.z, v0.w + v1.w}, dt[4] = {d4.x, d4.y, d4.z, d4.w};
+    float within[4] = {u0.x + u1.x - vt[0], u0.y + u1.y - vt[1], u0.z + u1.z - vt[2], u0.w + u1.w - vt[3]};   // suffix sums of u - v
+#pragma unroll
+    for (int e = 2; e >= 0; --e) within[e] += within[e + 1];
+    float incl = within[0];
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const float dn = __shfl_down_sync(0xffffffffu, incl, off);
+      if (lane + off < 32) incl += dn;
+    }
+    const float total = __shfl_sync(0xffffffffu, incl, 0), behind = incl - within[0];
+    const float resid = c > 0 ? left - (right + total) : 0.f;   // what the sum misses of the pin at the chunk's first step
+    const float a_h = g.A[h];
+    float ga_acc = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int t = lane * 4 + e;
+      const float ga = right + within[e] + behind + resid * (static_cast<float>(WQ - t) / static_cast<float>(WQ));
+      if (c * WQ + t < g.L) ga_acc += dt[e] * ga;
+      s_gd[t][w] = vt[e] / dt[e] + a_h * ga;
+    }
+    ga_acc = warp_reduce<SumOp>(ga_acc);
+    if (lane == 0) g.ga_part[static_cast<size_t>(bc) * g.H + h] = ga_acc;
+  }
   __syncthreads();
-  float base = 0.f;
-  for (int w = 0; w < (t >> 5); ++w) base += warp_tot[w];
-  const float cv = v + base;
-  const float c_hi = __shfl_sync(0xffffffffu, cv, (t & 31) | 7), c_lo = __shfl_sync(0xffffffffu, cv, (t & 31) & ~7);
-  const size_t o = (static_cast<size_t>(b) * H + h) * (static_cast<size_t>(nc) * WQ) + c * WQ + t;
-  cum[o] = cv;
-  dtt[o] = d;
-  colf_c[o] = w_exp(c_hi - cv) * d;
-  if (colf_a != nullptr) colf_a[o] = w_exp(cv - c_lo);
+  float gb = 0.f;
+#pragma unroll
+  for (int k = 0; k < WQ * WS_HEADS / WS_THREADS; ++k) {
+    const int idx = k * WS_THREADS + threadIdx.x, t = idx / WS_HEADS, hh = h0 + idx % WS_HEADS;
+    if (c * WQ + t < g.L && hh < g.H) {
+      const size_t row = static_cast<size_t>(b) * g.L + c * WQ + t;
+      const float gd = s_gd[t][idx % WS_HEADS];
+      g.gdt[row * g.H + hh] = gd;
+      if (RAW) {
+        const float gr = gd * walk_sigmoid(__half2float(g.raw[row * g.raw_pitch + hh]) + g.bias[hh]);
+        g.graw[row * g.graw_pitch + hh] = __float2half_rn(gr);
+        gb += gr;
+      }
+    }
+  }
+  if (RAW) {   // a thread has one head in all its steps: threads of equal idx % 8 meet
+    __shared__ float s_gb[WS_HEADS][WS_HEADS];
+#pragma unroll
+    for (int off = 16; off >= WS_HEADS; off >>= 1) gb += __shfl_xor_sync(0xffffffffu, gb, off);
+    if (lane < WS_HEADS) s_gb[w][lane] = gb;
+    __syncthreads();
+    if (threadIdx.x < WS_HEADS && h0 + static_cast<int>(threadIdx.x) < g.H) {
+      float t = 0.f;
+#pragma unroll
+      for (int q = 0; q < WS_HEADS; ++q) t += s_gb[q][threadIdx.x];
+      g.gb_part[static_cast<size_t>(bc) * g.H + h0 + threadIdx.x] = t;
+    }
+  }
+}
+
+// One CTA per head: gA[h] = the sum of its parts; with A_log's gradient wanted (A = -exp(A_log), so dA / dA_log = A)
+// gA_log[h] += gA[h] * A[h]; with the step bias's gradient wanted gbias[h] += the sum of its parts.
+__global__ void __launch_bounds__(128) ssd_walk_sum_parts_kernel(const float* __restrict__ ga_part, const float* __restrict__ gb_part, int parts, int H,
+                                                                 const float* __restrict__ A, float* __restrict__ gA, float* __restrict__ gA_log,
+                                                                 float* __restrict__ gbias) {
+  mp_grid_dependency();
+  __shared__ float red[64];
+  const int h = blockIdx.x;
+  float sa = 0.f, sb = 0.f;
+  for (int i = threadIdx.x; i < parts; i += 128) {
+    sa += ga_part[static_cast<size_t>(i) * H + h];
+    if (gbias != nullptr) sb += gb_part[static_cast<size_t>(i) * H + h];
+  }
+  sa = cta_reduce<SumOp, 128>(sa, red, 0.f);
+  sb = cta_reduce<SumOp, 128>(sb, red, 0.f);
+  if (threadIdx.x == 0) {
+    gA[h] = sa;
+    if (gA_log != nullptr) gA_log[h] += sa * A[h];
+    if (gbias != nullptr) gbias[h] += sb;
+  }
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
@@ -990,29 +1155,49 @@ bool mp_ssd_walk_supported(int L, int H, int P, int N, int G) {
   return P == WP && N == WN && L >= 32 && G > 0 && H % G == 0 && getenv("MP_SSD_NO_WALK") == nullptr;
 }
 
+static int walk_head_blocks(int H) { return (H + WS_HEADS - 1) / WS_HEADS; }
+
 void mp_ssd_walk_cumsum(const float* dt, const float* A, float* cum, float* dtt, float* colf_c, float* colf_a, int B, int L, int H,
                         int* carry_flags, int n_flags, cudaStream_t st) {
-  MpLaunch(B * H * ((L + WQ - 1) / WQ), WQ, 0, st)(ssd_walk_cumsum_kernel<false>, dt, A, cum, dtt, colf_c, colf_a, L, H, carry_flags, n_flags, nullptr, 0, nullptr,
-                                                                 nullptr, nullptr);
+  const int hb = walk_head_blocks(H);
+  MpLaunch(B * ((L + WQ - 1) / WQ) * hb, WS_THREADS, 0, st)(ssd_walk_cumsum_kernel<false>, dt, A, cum, dtt, colf_c, colf_a, L, H, hb, carry_flags, n_flags,
+                                                            nullptr, 0, nullptr, nullptr, nullptr);
   MP_LAUNCH_CHECK();
 }
 
 // The same from the raw projection output and A_log (see the kernel); dt_out and A_out are what the reverse pass takes.
 void mp_ssd_walk_cumsum_raw(const __half* raw, size_t raw_pitch, const float* bias, const float* A_log, float* dt_out, float* A_out, float* cum,
                             float* dtt, float* colf_c, int B, int L, int H, int* carry_flags, int n_flags, cudaStream_t st) {
-  MpLaunch(B * H * ((L + WQ - 1) / WQ), WQ, 0, st)(ssd_walk_cumsum_kernel<true>, nullptr, A_log, cum, dtt, colf_c, nullptr, L, H, carry_flags, n_flags, raw, raw_pitch,
-                                                                bias, dt_out, A_out);
+  const int hb = walk_head_blocks(H);
+  MpLaunch(B * ((L + WQ - 1) / WQ) * hb, WS_THREADS, 0, st)(ssd_walk_cumsum_kernel<true>, nullptr, A_log, cum, dtt, colf_c, nullptr, L, H, hb, carry_flags,
+                                                            n_flags, raw, raw_pitch, bias, dt_out, A_out);
+  MP_LAUNCH_CHECK();
+}
+
+// gdt, gA (and graw, gbias, gA_log, with raw) from the row dots and the pins' parts; ga_part, gb_part: [B * nc][H].
+void mp_ssd_walk_scalars(const float* u, const float* v, const float* dtt, const float* A, const float* pin, float* gdt, float* gA, float* ga_part,
+                         float* gb_part, const __half* raw, size_t raw_pitch, const float* bias, __half* graw, size_t graw_pitch, float* gbias,
+                         float* gA_log, int B, int L, int H, cudaStream_t st) {
+  ScalarArgs g;
+  g.u = u; g.v = v; g.dtt = dtt; g.A = A; g.pin = pin; g.gdt = gdt; g.ga_part = ga_part; g.gb_part = gb_part;
+  g.raw = raw; g.raw_pitch = raw_pitch; g.bias = bias; g.graw = graw; g.graw_pitch = graw_pitch;
+  g.B = B; g.L = L; g.H = H; g.nc = (L + WQ - 1) / WQ; g.hblocks = walk_head_blocks(H);
+  const int grid = B * g.nc * g.hblocks;
+  if (raw != nullptr) MpLaunch(grid, WS_THREADS, 0, st)(ssd_walk_scalars_kernel<true>, g);
+  else MpLaunch(grid, WS_THREADS, 0, st)(ssd_walk_scalars_kernel<false>, g);
+  MP_LAUNCH_CHECK();
+  MpLaunch(H, 128, 0, st)(ssd_walk_sum_parts_kernel, ga_part, gb_part, B * g.nc, H, A, gA, gA_log, raw != nullptr ? gbias : nullptr);
   MP_LAUNCH_CHECK();
 }
 
 // One walk.  q, k: [B*L, G*128]; v, z, out: [B*L, H*64]; cum, dtt, colf (of the walk's direction): [B, H, nc * 128] from mp_ssd_walk_cumsum.
 void mp_ssd_walk(int anti, const __half* q, const __half* k, const __half* v, const float* cum, const float* dtt, const float* colf, __half* out,
                  const __half* z,
-                 float* dot_out, __half* hs_out, float* carry, int* carry_flag, int max_ctas, int B, int L, int H, int G, uint32_t* status,
+                 float* dot_out, float* state_dot, __half* hs_out, float* carry, int* carry_flag, int max_ctas, int B, int L, int H, int G, uint32_t* status,
                  cudaStream_t st) {
   WalkArgs g;
   g.B = B; g.L = L; g.H = H; g.G = G; g.nc = (L + WQ - 1) / WQ;
-  g.cum = cum; g.dtt = dtt; g.colf = colf; g.out = out; g.z = z; g.dot_out = dot_out; g.hs_out = hs_out; g.status = status;
+  g.cum = cum; g.dtt = dtt; g.colf = colf; g.out = out; g.z = z; g.dot_out = dot_out; g.state_dot = state_dot; g.hs_out = hs_out; g.status = status;
   g.carry = carry; g.carry_flag = carry_flag;
   // One CTA per SM slot it may use, every CTA the same number of chunks; never more CTAs than sequences, so that a CTA's
   // range is at least one sequence long (see walk_segment).  MP_SSD_WALK_PER_SEQUENCE: one CTA per sequence, no hand-off.
@@ -1042,11 +1227,11 @@ void mp_ssd_walk(int anti, const __half* q, const __half* k, const __half* v, co
 // gB, gC [B*L, G*128] from gy, x [B*L, H*64], Bm, Cm [B*L, G*128] and the states left by the two walks
 // (hs_causal, hs_anti: [B, H, nc][128][64]).
 void mp_ssd_group_grads(const __half* gy, const __half* x, const __half* Bm, const __half* Cm, const __half* hs_causal, const __half* hs_anti,
-                        const float* cum, const float* dtt, const float* colf_c, __half* gB, __half* gC, int B, int L, int H, int G,
-                        uint32_t* status, cudaStream_t st) {
+                        const float* cum, const float* dtt, const float* colf_c, float* state_dot, __half* gB, __half* gC, int B, int L,
+                        int H, int G, uint32_t* status, cudaStream_t st) {
   GroupArgs g;
   g.B = B; g.L = L; g.H = H; g.G = G; g.nc = (L + WQ - 1) / WQ;
-  g.cum = cum; g.dtt = dtt; g.colf = colf_c; g.status = status;
+  g.cum = cum; g.dtt = dtt; g.colf = colf_c; g.state_dot = state_dot; g.status = status;
   const size_t srows = static_cast<size_t>(B) * H * g.nc * WN;
   const CUtensorMap mgy = walk_map3(gy, B, L, static_cast<size_t>(H) * WP), mx = walk_map3(x, B, L, static_cast<size_t>(H) * WP);
   const CUtensorMap mhc = walk_map(hs_causal, srows, WP), mha = walk_map(hs_anti, srows, WP);
