@@ -59,7 +59,7 @@ struct WalkArgs {
   __half* out;             // [B*L, H*64] or null
   const __half* z;         // dot partner, same indexing as out, or null
   float* dot_out;          // [2][B, H, LP] row dots <z, out> from the fp32 accumulators, one array per half of the columns, or null
-  float* state_dot;        // [B, H, nc][16], first eight: sums over a chunk's rows of <z, the received state's share of out>, one per worker warp, or null
+  float* state_dot;        // [B, H, nc][16], first eight: sums over a chunk's rows of <z, the received state's share of out>, one per worker warp (causal form with dot_out)
   __half* hs_out;          // [B, H, nc][128][64]: state every chunk receives, or null
   float* carry;            // [B * H][128][64] fp32: state handed from the CTA that walked the first part of a sequence to the next
   int* carry_flag;         // [B * H]: number of worker warps (of 8) that have written their part of `carry`; zero before the launch
@@ -512,6 +512,9 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_con
           for (int e = 0; e < 32; ++e) yo[e] = 0u;
         }
         tcgen05_fence_before_sync();
+        float o[32];
+#pragma unroll
+        for (int e = 0; e < 32; ++e) o[e] = ro * (__uint_as_float(yd[e]) + fo * __uint_as_float(yo[e]));
         if (DOT) {   // this thread's row of z comes back from the staging positions before the output overwrites them
           float dot = 0.f, dot_state = 0.f;
 #pragma unroll
@@ -522,21 +525,17 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_con
             for (int e = 0; e < 4; ++e) {
               const float2 zf = __half22float2(z2[e]);
               const int k0 = q4 * 8 + 2 * e;
-              dot += zf.x * __uint_as_float(yd[k0]) + zf.y * __uint_as_float(yd[k0 + 1]);
-              dot_state += zf.x * __uint_as_float(yo[k0]) + zf.y * __uint_as_float(yo[k0 + 1]);
+              dot += zf.x * o[k0] + zf.y * o[k0 + 1];
+              if (!ANTI) dot_state += zf.x * __uint_as_float(yo[k0]) + zf.y * __uint_as_float(yo[k0 + 1]);
             }
           }
-          dot_state *= ro * fo;
-          g.dot_out[static_cast<size_t>(ch) * g.B * g.H * (static_cast<size_t>(g.nc) * WQ) + step0 + c * WQ] = ro * dot + dot_state;
-          if (g.state_dot != nullptr) {
-            dot_state = warp_reduce<SumOp>(dot_state);
+          g.dot_out[static_cast<size_t>(ch) * g.B * g.H * (static_cast<size_t>(g.nc) * WQ) + step0 + c * WQ] = dot;
+          if (!ANTI) {   // the received state's share of the row dots, summed over the rows
+            dot_state = warp_reduce<SumOp>(dot_state * fo);
             if (lane == 0) g.state_dot[(bh * g.nc + c) * 16 + (warp - 2)] = dot_state;
           }
           __syncwarp();
         }
-        float o[32];
-#pragma unroll
-        for (int e = 0; e < 32; ++e) o[e] = ro * (__uint_as_float(yd[e]) + fo * __uint_as_float(yo[e]));
         if (g.out != nullptr) {
 #pragma unroll
           for (int q4 = 0; q4 < 4; ++q4) {
