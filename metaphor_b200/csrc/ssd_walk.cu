@@ -89,6 +89,18 @@ __host__ __device__ __forceinline__ bool walk_segment(int cta, int ncta, int nse
   return false;
 }
 
+// Eight floats -> eight r16.
+__device__ __forceinline__ uint4 walk_pack8(const float* f) {
+  uint4 pk;
+  uint32_t* w = reinterpret_cast<uint32_t*>(&pk);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const __half2 hv = __floats2half2_rn(f[2 * e], f[2 * e + 1]);
+    w[e] = *reinterpret_cast<const uint32_t*>(&hv);
+  }
+  return pk;
+}
+
 __device__ __forceinline__ float w_exp(float x) { return __expf(x); }
 
 // One arrival per warp: every lane has made its shared-memory writes visible to the asynchronous proxy (and
@@ -581,6 +593,458 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_con
       }
     }
     qb += n;
+    }
+  }
+  tcgen05_fence_before_sync();
+  __syncthreads();
+  if (warp == 1) tmem_dealloc(tmem, TC_COLS);
+}
+
+// ---------------------------------------------------------------------------
+// The walk for two neighbouring heads of a group at once.  They share q and k (B and C belong to the group), so a chunk of both loads
+// them once and its scores are computed once; Yo and S of both are single MMAs with 128 columns.  What this buys is the chain: with
+// one head a chunk is a sequence of hand-offs between the tensor core and the worker warps that leaves both idle most of the time,
+// with two the workers have twice the work per hand-off.
+// Order of a chunk k for the workers: fold S(k) into the states, epilogue of Y(k), scale the values of chunk k+1, write P(k+1);
+// for the MMA warp: [P(k) written] Yd(k), G(k+1), [values and states of k+1 written] Yo(k+1), S(k+1).  Every MMA then runs while
+// the workers are in the step before the one that needs it.
+// Shared memory has room for one v tile of each head only: v(k+1) is requested when Yd(k) has read v(k).  P lies in TMEM, in the columns
+// of the scores it is made from (32 score columns become 16 + 16 columns of packed r16 pairs, one block per head): Yd reads its
+// A operand there.
+// ---------------------------------------------------------------------------
+constexpr int WP2_QK = 2 * W_TILE_QK;              // q and k of a chunk, 64 KB; two stages
+constexpr int WP2_OFF_V = 2 * WP2_QK;              // v of both heads
+constexpr int WP2_OFF_H = WP2_OFF_V + 2 * W_TILE_V;
+constexpr int WP2_OFF_VS = WP2_OFF_H + 2 * W_TILE_V;
+constexpr int WP2_OFF_TAIL = WP2_OFF_VS + 2 * W_TILE_V;   // 229376
+constexpr int WP2_SMEM_BYTES = WP2_OFF_TAIL + 2048 + 1024;
+constexpr uint32_t TP_G = 0, TP_S = 128, TP_YD = 256, TP_YO = 384;   // TMEM columns; head h of a pair at + 64 h
+enum { PB_FULL0 = 0, PB_FULL1, PB_EMPTY0, PB_EMPTY1, PB_VFULL, PB_GFULL, PB_PREADY, PB_VSREADY, PB_YFULL, PB_SFULL, PB_SCAL, PB_COUNT };
+
+template <int ANTI, bool DOT, bool RAGGED>
+__global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_pair_kernel(const __grid_constant__ CUtensorMap map_q,
+                                                                    const __grid_constant__ CUtensorMap map_k,
+                                                                    const __grid_constant__ CUtensorMap map_v,
+                                                                    const __grid_constant__ CUtensorMap map_hs, const WalkArgs g) {
+  constexpr bool OUT = ANTI != 0 || !DOT;   // the causal form with row dots has no other output
+  extern __shared__ unsigned char walk_smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(walk_smem_raw) + 1023) & ~uintptr_t(1023));
+  unsigned char* sV = smem + WP2_OFF_V;
+  unsigned char* sH = smem + WP2_OFF_H;
+  unsigned char* sVs = smem + WP2_OFF_VS;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + WP2_OFF_TAIL);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + WP2_OFF_TAIL + 112);
+  volatile int* abort = reinterpret_cast<volatile int*>(smem + WP2_OFF_TAIL + 116);
+  float* s_colf = reinterpret_cast<float*>(smem + WP2_OFF_TAIL + 128);   // [2][128]
+  float* s_ref = s_colf + 2 * WQ;                                        // [2][16]: cum at the far end of every 8-step piece
+  float* s_last = s_ref + 32;                                            // [2]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nc = g.nc, hp = g.H / 2;
+  const int nseq = g.B * hp, cta = blockIdx.x, ncta = gridDim.x;
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < PB_COUNT; ++i) mbar_init(bars + i, i == PB_PREADY || i == PB_VSREADY || i == PB_SCAL ? 8 : 1);
+    *abort = 0;
+    mbar_fence_init();
+  }
+  if (warp == 1) tmem_alloc(tmem_slot, TC_COLS);
+  tcgen05_fence_before_sync();
+  __syncthreads();
+  tcgen05_fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
+  mp_grid_wait();
+
+  if (warp == 0) {
+    // ------------------------------ TMA producer ------------------------------
+    if (lane == 0) {
+      WalkSeg sg;
+      int qb = 0;   // chunks walked by this CTA before the segment in hand: the barriers' phases run on across segments
+      bool ok = true;
+      for (int si = 0; ok && walk_segment(cta, ncta, nseq, nc, si, sg); ++si) {
+        const int h = 2 * (sg.seq % hp), b = sg.seq / hp;
+        const int grp = h / (g.H / g.G);
+        auto load_qk = [&](int k) {
+          const int q = qb + k, s = q & 1, row0 = (ANTI ? nc - 1 - (sg.p0 + k) : sg.p0 + k) * WQ;
+          if (!walk_wait(bars + PB_EMPTY0 + s, ((q >> 1) & 1) ^ 1u, g.status, abort)) return false;
+          unsigned char* st = smem + s * WP2_QK;
+          uint64_t* full = bars + PB_FULL0 + s;
+          mbar_arrive_expect_tx(full, WP2_QK);
+          tma_load_3d(st, &map_q, grp * WN, row0, b, full);
+          tma_load_3d(st + WQ * 128, &map_q, grp * WN + 64, row0, b, full);
+          tma_load_3d(st + W_TILE_QK, &map_k, grp * WN, row0, b, full);
+          tma_load_3d(st + W_TILE_QK + WQ * 128, &map_k, grp * WN + 64, row0, b, full);
+          return true;
+        };
+        ok = load_qk(0);
+        for (int k = 0; ok && k < sg.n; ++k) {
+          const int q = qb + k, row0 = (ANTI ? nc - 1 - (sg.p0 + k) : sg.p0 + k) * WQ;
+          // Yd of the previous chunk has read the v tiles (the workers scaled them before they wrote its P)
+          if (q > 0 && !walk_wait(bars + PB_YFULL, (q - 1) & 1, g.status, abort)) { ok = false; break; }
+          mbar_arrive_expect_tx(bars + PB_VFULL, 2 * W_TILE_V);
+          tma_load_3d(sV, &map_v, h * WP, row0, b, bars + PB_VFULL);
+          tma_load_3d(sV + W_TILE_V, &map_v, (h + 1) * WP, row0, b, bars + PB_VFULL);
+          if (k + 1 < sg.n) ok = load_qk(k + 1);
+        }
+        qb += sg.n;
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------ MMA issuer (the warp as a whole, see elect_one) ----
+    const uint32_t id_g = umma_instr_desc(UMMA_FMT_F16, 0u, 0u, 128, 128);    // q (K-major) x k (K-major)
+    const uint32_t id_yd = umma_instr_desc(UMMA_FMT_F16, 0u, 1u, 128, 64);    // P (TMEM) x MN-major v
+    const uint32_t id_yo = umma_instr_desc(UMMA_FMT_F16, 0u, 1u, 128, 128);   // q (K-major) x MN-major states of both heads
+    const uint32_t id_s = umma_instr_desc(UMMA_FMT_F16, 1u, 1u, 128, 128);    // k^T (MN-major A) x MN-major scaled values of both
+    const uint32_t s0 = mp_smem_u32(smem);
+    const uint64_t d_q = umma_smem_desc(s0, 16, 1024), d_k = umma_smem_desc(s0 + W_TILE_QK, 16, 1024);
+    const uint64_t d_kt = umma_smem_desc(s0 + W_TILE_QK, WQ * 128, 1024), d_v = umma_smem_desc(mp_smem_u32(sV), W_TILE_V, 1024);
+    const uint64_t d_h = umma_smem_desc(mp_smem_u32(sH), W_TILE_V, 1024), d_vs = umma_smem_desc(mp_smem_u32(sVs), W_TILE_V, 1024);
+    constexpr uint32_t STAGE_U = WP2_QK >> 4, ROWS_U = 2048 >> 4, HEAD_U = W_TILE_V >> 4;
+    auto kslice = [](int ks) { return static_cast<uint32_t>(((ks >> 2) * (WQ * 128) + (ks & 3) * 32) >> 4); };   // K-major: two 64-column blocks
+    bool ok = true;
+    auto await = [&](int bar, uint32_t parity) {
+      ok = walk_wait(bars + bar, parity, g.status, abort);
+      ok = __all_sync(0xffffffffu, ok) != 0;
+      tcgen05_fence_after_sync();
+      return ok;
+    };
+    auto issue_g = [&](int q) {
+      if (!await(PB_FULL0 + (q & 1), (q >> 1) & 1)) return;
+      const uint64_t dq = d_q + (q & 1) * STAGE_U, dk = d_k + (q & 1) * STAGE_U;
+      if (elect_one()) {
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks) umma<false>(tmem + TP_G, dq + kslice(ks), dk + kslice(ks), id_g, ks != 0 ? 1u : 0u);
+        umma_commit(bars + PB_GFULL);
+      }
+      __syncwarp();
+    };
+    WalkSeg sg{};
+    int qb = 0;
+    // Yo and S of chunk k: the workers have written its scaled values and the states it receives
+    auto issue_state = [&](int k) {
+      const int q = qb + k;
+      if (!await(PB_VSREADY, q & 1)) return;
+      const bool has_state = k > 0 || sg.cin != 0;
+      const uint64_t dq = d_q + (q & 1) * STAGE_U, dkt = d_kt + (q & 1) * STAGE_U;
+      if (elect_one()) {
+        if (has_state) {
+          if (g.hs_out != nullptr) {   // the states this chunk receives, straight from their operand tiles
+            const int c = ANTI ? nc - 1 - (sg.p0 + k) : sg.p0 + k;
+            const size_t bh = static_cast<size_t>(sg.seq) * 2;
+            tma_store_2d(&map_hs, sH, 0, static_cast<int>((bh * nc + c) * WN));
+            tma_store_2d(&map_hs, sH + W_TILE_V, 0, static_cast<int>(((bh + 1) * nc + c) * WN));
+            bulk_commit();
+          }
+#pragma unroll
+          for (int ks = 0; ks < 8; ++ks) umma<false>(tmem + TP_YO, dq + kslice(ks), d_h + ks * ROWS_U, id_yo, ks != 0 ? 1u : 0u);
+        }
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks) umma<false>(tmem + TP_S, dkt + ks * ROWS_U, d_vs + ks * ROWS_U, id_s, ks != 0 ? 1u : 0u);
+        // the workers rewrite the state tiles once S(k) is complete: the stores must have read them by then
+        if (g.hs_out != nullptr && has_state) bulk_wait_read<0>();
+        umma_commit(bars + PB_SFULL);
+        umma_commit(bars + PB_EMPTY0 + (q & 1));
+      }
+      __syncwarp();
+    };
+    for (int si = 0; ok && walk_segment(cta, ncta, nseq, nc, si, sg); ++si) {
+      issue_g(qb);
+      if (ok) issue_state(0);
+      for (int k = 0; ok && k < sg.n; ++k) {
+        const int q = qb + k;
+        if (!await(PB_PREADY, q & 1) || !await(PB_VFULL, q & 1)) break;
+        if (elect_one()) {
+#pragma unroll
+          for (int hh = 0; hh < 2; ++hh)
+#pragma unroll
+            for (int ks = 0; ks < 8; ++ks)   // 16 steps are 8 columns of P; 32 score columns hold 16 of head 0 and 16 of head 1
+              umma_f16_ta(tmem + TP_YD + hh * 64, tmem + TP_G + (ks >> 1) * 32 + hh * 16 + (ks & 1) * 8, d_v + hh * HEAD_U + ks * ROWS_U, id_yd, ks != 0 ? 1u : 0u);
+          umma_commit(bars + PB_YFULL);
+        }
+        __syncwarp();
+        if (k + 1 < sg.n) {
+          issue_g(q + 1);
+          if (ok) issue_state(k + 1);
+        }
+      }
+      qb += sg.n;
+    }
+    mp_launch_dependents();
+    if (g.hs_out != nullptr) bulk_wait_all<0>();
+  } else {
+    // ------------------------------ workers -----------------------------------
+    const int quarter = warp & 3;              // TMEM lane quarter this warp may read
+    const int ch = (warp - 2) >> 2;            // score columns: half `ch` for both heads; everything else: head `ch` of the pair
+    const int r = quarter * 32 + lane;         // row of every 128-row tile
+    const uint32_t tl = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
+    const int pitch = g.H * WP;
+    unsigned char* hrow = sH + ch * W_TILE_V + r * 128;
+    unsigned char* stg = sVs + ch * W_TILE_V;  // this warp's rows: scaled values of chunk k+1, before that the staging of chunk k's output
+    WalkSeg sg;
+    int qb = 0;
+    bool alive = true;
+    for (int si = 0; alive && walk_segment(cta, ncta, nseq, nc, si, sg); ++si) {
+      const int n = sg.n;
+      const int h = 2 * (sg.seq % hp) + ch, b = sg.seq / hp;
+      const size_t bh = static_cast<size_t>(b) * g.H + h;
+      const size_t LP = static_cast<size_t>(nc) * WQ;
+      const size_t step0 = bh * LP + r, other0 = (ch == 0 ? bh + 1 : bh - 1) * LP + r;
+      float state[64];
+      const int c_first = ANTI ? nc - 1 - sg.p0 : sg.p0;
+      if (sg.cin) {
+        // the states the first part of these sequences ended with: written by all eight worker warps of the CTA that walked it
+        if (lane == 0) {
+          const uint64_t t0 = mp_globaltimer_ns();
+          const uint64_t limit = mp_wait_limit_ns(g.status);
+          while (true) {
+            int seen;
+            asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(g.carry_flag + sg.seq) : "memory");
+            if (seen >= 8) break;
+            if (*abort != 0) break;
+            if (mp_globaltimer_ns() - t0 > limit) {
+              *abort = 1;
+              if (g.status != nullptr) atomicExch(g.status, MP_STATUS_WAIT_TIMEOUT);
+              break;
+            }
+            __nanosleep(200);
+          }
+        }
+        __syncwarp();
+        if (*abort != 0) { alive = false; break; }
+        const float4* src = reinterpret_cast<const float4*>(g.carry + (bh * WN + r) * WP);
+#pragma unroll
+        for (int q4 = 0; q4 < 16; ++q4) {
+          const float4 v4 = __ldcg(src + q4);
+          state[q4 * 4] = v4.x; state[q4 * 4 + 1] = v4.y; state[q4 * 4 + 2] = v4.z; state[q4 * 4 + 3] = v4.w;
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < 64; ++e) state[e] = 0.f;
+        if (g.hs_out != nullptr) {   // the first chunk of a sequence's walk receives nothing
+          uint4* dst = reinterpret_cast<uint4*>(g.hs_out + ((bh * nc + c_first) * WN + r) * WP);
+#pragma unroll
+          for (int q4 = 0; q4 < 8; ++q4) dst[q4] = make_uint4(0u, 0u, 0u, 0u);
+        }
+      }
+      // r16 copy of the state: operand of the next chunk's q H
+      auto write_state = [&]() {
+#pragma unroll
+        for (int q4 = 0; q4 < 8; ++q4) *reinterpret_cast<uint4*>(hrow + ((q4 ^ (r & 7)) << 4)) = walk_pack8(state + q4 * 8);
+      };
+      if (sg.cin) write_state();   // (the tile is free: its last readers were complete before the previous segment's last S was)
+      // scalars: chunk in hand (cur), the one after it (nxt), one more in flight (pre)
+      float cum_cur = 0.f, dt_cur = 0.f, last_cur = 0.f, last_nxt = 0.f;
+      const size_t i0 = static_cast<size_t>(c_first) * WQ;
+      float cum_nxt = g.cum[step0 + i0], dt_nxt = g.dtt[step0 + i0], colf_nxt = g.colf[step0 + i0], oth_nxt = g.cum[other0 + i0];
+      float cum_pre = 0.f, dt_pre = 0.f, colf_pre = 0.f, oth_pre = 0.f;
+      auto prefetch = [&](int k) {
+        const size_t i = static_cast<size_t>(ANTI ? c_first - k : c_first + k) * WQ;
+        cum_pre = g.cum[step0 + i]; dt_pre = g.dtt[step0 + i]; colf_pre = g.colf[step0 + i]; oth_pre = g.cum[other0 + i];
+      };
+      if (n > 1) prefetch(1);
+
+#pragma unroll 1
+      for (int k = -1; k < n; ++k) {   // finishes chunk k, prepares chunk k+1; k = -1 only prepares
+        const bool more = k + 1 < n;
+        const int c = ANTI ? c_first - k : c_first + k;
+        const int q = qb + k;
+        const uint32_t par = static_cast<uint32_t>(q) & 1u, parn = static_cast<uint32_t>(q + 1) & 1u;
+        if (k >= 0) {
+          const bool has_state = k > 0 || sg.cin != 0;
+          cum_cur = cum_nxt; dt_cur = dt_nxt; last_cur = last_nxt;
+          if (more) {
+            cum_nxt = cum_pre; dt_nxt = dt_pre; colf_nxt = colf_pre; oth_nxt = oth_pre;
+            if (k + 2 < n) prefetch(k + 2);
+          }
+          uint4 zc[8];
+          if (DOT) {   // the dot partner's rows of chunk k, whole 128-byte row pieces per load
+#pragma unroll
+            for (int it = 0; it < 8; ++it) {
+              int zt = c * WQ + quarter * 32 + it * 4 + (lane >> 3);
+              if (RAGGED) zt = min(zt, g.L - 1);   // the output rows beyond the sequence are zero: any row serves as their partner
+              zc[it] = *reinterpret_cast<const uint4*>(g.z + (static_cast<size_t>(b) * g.L + zt) * pitch + h * WP + (lane & 7) * 8);
+            }
+          }
+          // ---- H' = D H + S ---------------------------------------------------------------
+          if (!walk_wait(bars + PB_SFULL, par, g.status, abort)) { alive = false; break; }
+          tcgen05_fence_after_sync();
+          if (more || sg.cout) {
+            const float D = w_exp(last_cur);
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+              uint32_t sv[32];
+              tmem_ld_32x32(tl + TP_S + ch * 64 + p * 32, sv);
+              tmem_ld_wait();
+#pragma unroll
+              for (int e = 0; e < 32; ++e) state[p * 32 + e] = D * state[p * 32 + e] + __uint_as_float(sv[e]);
+            }
+            if (more) {
+              write_state();
+            } else {
+              // the first part of the sequences ends here: their states go to the CTA that walks the rest
+              float4* dst = reinterpret_cast<float4*>(g.carry + (bh * WN + r) * WP);
+#pragma unroll
+              for (int q4 = 0; q4 < 16; ++q4) __stcg(dst + q4, make_float4(state[q4 * 4], state[q4 * 4 + 1], state[q4 * 4 + 2], state[q4 * 4 + 3]));
+              __threadfence();
+              __syncwarp();
+              if (lane == 0) atomicAdd(g.carry_flag + sg.seq, 1);
+            }
+          }
+          // ---- out = r o (Yd + f o Yo) of chunk k -------------------------------------------
+          if (DOT) {
+#pragma unroll
+            for (int it = 0; it < 8; ++it) {
+              const int lr = quarter * 32 + it * 4 + (lane >> 3);
+              *reinterpret_cast<uint4*>(stg + lr * 128 + (((lane & 7) ^ (lr & 7)) << 4)) = zc[it];
+            }
+            __syncwarp();
+          }
+          if (!walk_wait(bars + PB_YFULL, par, g.status, abort)) { alive = false; break; }
+          tcgen05_fence_after_sync();
+          const float fo = has_state ? (ANTI ? w_exp(last_cur - cum_cur) : w_exp(cum_cur)) : 0.f;
+          const float ro = ANTI ? dt_cur : 1.f;
+          float dot = 0.f, dot_state = 0.f;
+#pragma unroll
+          for (int p = 0; p < 4; ++p) {
+            uint32_t yd[16], yo[16];
+            tmem_ld_32x16(tl + TP_YD + ch * 64 + p * 16, yd);
+            if (has_state) tmem_ld_32x16(tl + TP_YO + ch * 64 + p * 16, yo);
+            tmem_ld_wait();
+            if (!has_state) {
+#pragma unroll
+              for (int e = 0; e < 16; ++e) yo[e] = 0u;
+            }
+            float o[16];
+            if (OUT) {
+#pragma unroll
+              for (int e = 0; e < 16; ++e) o[e] = ro * (__uint_as_float(yd[e]) + fo * __uint_as_float(yo[e]));
+            }
+#pragma unroll
+            for (int q4 = 0; q4 < 2; ++q4) {
+              uint4* slot = reinterpret_cast<uint4*>(stg + r * 128 + (((p * 2 + q4) ^ (r & 7)) << 4));
+              if (DOT) {   // this thread's row of z, before the output overwrites it
+                const uint4 zq = *slot;
+                const __half2* z2 = reinterpret_cast<const __half2*>(&zq);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  const float2 zf = __half22float2(z2[e]);
+                  const int k0 = q4 * 8 + 2 * e;
+                  if (OUT) {
+                    dot += zf.x * o[k0] + zf.y * o[k0 + 1];
+                  } else {
+                    dot += zf.x * __uint_as_float(yd[k0]) + zf.y * __uint_as_float(yd[k0 + 1]);
+                    dot_state += zf.x * __uint_as_float(yo[k0]) + zf.y * __uint_as_float(yo[k0 + 1]);
+                  }
+                }
+              }
+              if (OUT) *slot = walk_pack8(o + q4 * 8);
+            }
+          }
+          if (DOT) {
+            if (!OUT) {   // the received state's share of the row dots, summed over the rows
+              dot_state *= fo;
+              dot += dot_state;
+              dot_state = warp_reduce<SumOp>(dot_state);
+              if (lane < 2) g.state_dot[(bh * nc + c) * 16 + quarter * 2 + lane] = lane == 0 ? dot_state : 0.f;
+            }
+            g.dot_out[step0 + static_cast<size_t>(c) * WQ] = dot;
+            g.dot_out[static_cast<size_t>(g.B) * g.H * LP + step0 + static_cast<size_t>(c) * WQ] = 0.f;
+          }
+          __syncwarp();
+          if (OUT) {   // whole 128-byte row pieces per store
+#pragma unroll
+            for (int it = 0; it < 8; ++it) {
+              const int lr = quarter * 32 + it * 4 + (lane >> 3);
+              const uint4 val = *reinterpret_cast<const uint4*>(stg + lr * 128 + (((lane & 7) ^ (lr & 7)) << 4));
+              if (!RAGGED || c * WQ + lr < g.L)
+                *reinterpret_cast<uint4*>(g.out + (static_cast<size_t>(b) * g.L + c * WQ + lr) * pitch + h * WP + (lane & 7) * 8) = val;
+            }
+            __syncwarp();
+          }
+        }
+        if (more) {
+          // ---- scalars of chunk k+1 into shared memory (every warp is past its P(k): Yd(k) was complete) -------------
+          s_colf[ch * WQ + r] = colf_nxt;
+          if ((r & 7) == (ANTI ? 0 : 7)) s_ref[ch * 16 + (r >> 3)] = cum_nxt;
+          if (r == WQ - 1) s_last[ch] = cum_nxt;
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bars + PB_SCAL);
+          if (!walk_wait(bars + PB_SCAL, parn, g.status, abort)) { alive = false; break; }
+          last_nxt = s_last[ch];
+          // ---- w o v of chunk k+1: operand of its state update ------------------------------------------------------
+          if (!walk_wait(bars + PB_VFULL, parn, g.status, abort)) { alive = false; break; }
+          {
+            const __half2 wt2 = __float2half2_rn(ANTI ? w_exp(cum_nxt) : w_exp(last_nxt - cum_nxt) * dt_nxt);
+            const unsigned char* src = sV + ch * W_TILE_V + r * 128;
+#pragma unroll
+            for (int q4 = 0; q4 < 8; ++q4) {
+              const int off = (q4 ^ (r & 7)) << 4;
+              uint4 v = *reinterpret_cast<const uint4*>(src + off);
+              __half2* h2 = reinterpret_cast<__half2*>(&v);
+#pragma unroll
+              for (int e = 0; e < 4; ++e) h2[e] = __hmul2(h2[e], wt2);
+              *reinterpret_cast<uint4*>(stg + r * 128 + off) = v;
+            }
+          }
+          warp_arrive(bars + PB_VSREADY, lane);
+          // ---- P = G o F of chunk k+1, both heads, in place of the scores -------------------------------------------
+          if (!walk_wait(bars + PB_GFULL, parn, g.status, abort)) { alive = false; break; }
+          tcgen05_fence_after_sync();
+#pragma unroll 1
+          for (int pp = 0; pp < 2; ++pp) {
+            const int pc = ch * 2 + pp;              // 32-column piece of the chunk
+            const int j0 = pc * 32;
+            if (ANTI ? (pc < quarter) : (pc > quarter)) {   // warp-uniform: the whole piece is masked
+              uint32_t zero[16];
+#pragma unroll
+              for (int e = 0; e < 16; ++e) zero[e] = 0u;
+              tmem_st_32x16(tl + TP_G + j0, zero);
+              tmem_st_32x16(tl + TP_G + j0 + 16, zero);
+            } else {
+              uint32_t v[32];
+              tmem_ld_32x32(tl + TP_G + j0, v);
+              // F: see ssd_walk_kernel
+              const bool diag = pc == quarter;
+              tmem_ld_wait();
+#pragma unroll 1
+              for (int hh = 0; hh < 2; ++hh) {
+                const float cum_r = hh == ch ? cum_nxt : oth_nxt;
+                uint32_t po[16];   // this head's 16 columns
+#pragma unroll
+                for (int sp = 0; sp < 4; ++sp) {
+                  const int jb = j0 + sp * 8;
+                  const float cref = s_ref[hh * 16 + (jb >> 3)];
+                  const float rarg = ANTI ? cref - cum_r : cum_r - cref;   // <= 0 off the diagonal
+                  const bool direct = rarg > 80.f;
+                  const float rowf = w_exp(direct ? 0.f : rarg);
+                  const float4 c0 = *reinterpret_cast<const float4*>(s_colf + hh * WQ + jb);
+                  const float4 c1 = *reinterpret_cast<const float4*>(s_colf + hh * WQ + jb + 4);
+                  float f[8] = {c0.x * rowf, c0.y * rowf, c0.z * rowf, c0.w * rowf, c1.x * rowf, c1.y * rowf, c1.z * rowf, c1.w * rowf};
+                  if (direct) {   // rare: the step factors from global memory
+                    const size_t o0 = (hh == ch ? step0 : other0) - r + static_cast<size_t>(ANTI ? c_first - k - 1 : c_first + k + 1) * WQ + jb;
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                      f[e] = ANTI ? w_exp(fminf(g.cum[o0 + e] - cum_r, 0.f)) : w_exp(fminf(cum_r - g.cum[o0 + e], 0.f)) * g.dtt[o0 + e];
+                  }
+                  if (diag) {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                      if (ANTI ? (sp * 8 + e < lane) : (sp * 8 + e > lane)) f[e] = 0.f;
+                  }
+#pragma unroll
+                  for (int e = 0; e < 4; ++e) {
+                    const __half2 hv = __floats2half2_rn(__uint_as_float(v[sp * 8 + 2 * e]) * f[2 * e], __uint_as_float(v[sp * 8 + 2 * e + 1]) * f[2 * e + 1]);
+                    po[sp * 4 + e] = *reinterpret_cast<const uint32_t*>(&hv);
+                  }
+                }
+                tmem_st_32x16(tl + TP_G + j0 + hh * 16, po);
+              }
+            }
+          }
+          tmem_st_wait();
+          warp_arrive(bars + PB_PREADY, lane);
+        }
+      }
+      qb += n;
     }
   }
   tcgen05_fence_before_sync();
@@ -1200,26 +1664,32 @@ void mp_ssd_walk(int anti, const __half* q, const __half* k, const __half* v, co
   g.carry = carry; g.carry_flag = carry_flag;
   // One CTA per SM slot it may use, every CTA the same number of chunks; never more CTAs than sequences, so that a CTA's
   // range is at least one sequence long (see walk_segment).  MP_SSD_WALK_PER_SEQUENCE: one CTA per sequence, no hand-off.
-  int grid = B * H;
-  if (max_ctas > 0 && max_ctas < grid && getenv("MP_SSD_WALK_PER_SEQUENCE") == nullptr) grid = max_ctas;
+  // Two heads at a time where their group has an even number of heads and there are enough sequences: a chunk of a pair takes about
+  // 1.4 times as long as a chunk of one head, which pays unless CTAs are left without a sequence.
+  const bool bounded = max_ctas > 0 && getenv("MP_SSD_WALK_PER_SEQUENCE") == nullptr;
+  auto load = [&](int seqs) { return bounded && seqs > max_ctas ? static_cast<double>(seqs) / max_ctas : 1.0; };   // sequences per CTA
+  const bool pairs = (H / G) % 2 == 0 && 1.4 * load(B * H / 2) < load(B * H) && getenv("MP_SSD_WALK_NO_PAIRS") == nullptr;
+  int grid = pairs ? B * H / 2 : B * H;
+  if (bounded && max_ctas < grid) grid = max_ctas;
   const CUtensorMap mq = walk_map3(q, B, L, static_cast<size_t>(G) * WN), mk = walk_map3(k, B, L, static_cast<size_t>(G) * WN);
   const CUtensorMap mv = walk_map3(v, B, L, static_cast<size_t>(H) * WP);
   const CUtensorMap mh = hs_out != nullptr ? walk_map(hs_out, static_cast<size_t>(B) * H * g.nc * WN, WP) : mv;
-  auto launch = [&](auto kernel) {
-    MP_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, W_SMEM_BYTES));
-    MpLaunch(grid, W_THREADS, W_SMEM_BYTES, st)(kernel, mq, mk, mv, mh, g);
+  auto launch = [&](auto kernel, int smem) {
+    MP_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    MpLaunch(grid, W_THREADS, smem, st)(kernel, mq, mk, mv, mh, g);
   };
   const bool dot = z != nullptr && dot_out != nullptr;
   if (!dot) { g.z = nullptr; g.dot_out = nullptr; }
   if (anti && !dot) MP_FATAL("ssd walk: the anti-causal form comes with its row dots");
-  const bool ragged = L % WQ != 0;
-  if (anti) {
-    if (ragged) launch(ssd_walk_kernel<1, true, true>); else launch(ssd_walk_kernel<1, true, false>);
-  } else if (dot) {
-    if (ragged) launch(ssd_walk_kernel<0, true, true>); else launch(ssd_walk_kernel<0, true, false>);
-  } else {
-    if (ragged) launch(ssd_walk_kernel<0, false, true>); else launch(ssd_walk_kernel<0, false, false>);
-  }
+#define MP_WALK_FORM(A, D)                                                                                                          \
+  do {                                                                                                                              \
+    if (pairs) { if (L % WQ != 0) launch(ssd_walk_pair_kernel<A, D, true>, WP2_SMEM_BYTES); else launch(ssd_walk_pair_kernel<A, D, false>, WP2_SMEM_BYTES); } \
+    else { if (L % WQ != 0) launch(ssd_walk_kernel<A, D, true>, W_SMEM_BYTES); else launch(ssd_walk_kernel<A, D, false>, W_SMEM_BYTES); }                   \
+  } while (0)
+  if (anti) MP_WALK_FORM(1, true);
+  else if (dot) MP_WALK_FORM(0, true);
+  else MP_WALK_FORM(0, false);
+#undef MP_WALK_FORM
   MP_LAUNCH_CHECK();
 }
 
