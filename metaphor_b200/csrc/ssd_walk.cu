@@ -609,7 +609,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_con
 // for the MMA warp: [P(k) written] Yd(k), G(k+1), [values and states of k+1 written] Yo(k+1), S(k+1).  Every MMA then runs while
 // the workers are in the step before the one that needs it.
 // Shared memory has room for one v tile of each head only: v(k+1) is requested when Yd(k) has read v(k).  P lies in TMEM, in the columns
-// of the scores it is made from (32 score columns become 16 + 16 columns of packed r16 pairs, one block per head): Yd reads its
+// of the scores it is made from (16 score columns become 8 + 8 columns of packed r16 pairs, one block per head): Yd reads its
 // A operand there.
 // ---------------------------------------------------------------------------
 constexpr int WP2_QK = 2 * W_TILE_QK;              // q and k of a chunk, 64 KB; two stages
@@ -619,10 +619,11 @@ constexpr int WP2_OFF_VS = WP2_OFF_H + 2 * W_TILE_V;
 constexpr int WP2_OFF_TAIL = WP2_OFF_VS + 2 * W_TILE_V;   // 229376
 constexpr int WP2_SMEM_BYTES = WP2_OFF_TAIL + 2048 + 1024;
 constexpr uint32_t TP_G = 0, TP_S = 128, TP_YD = 256, TP_YO = 384;   // TMEM columns; head h of a pair at + 64 h
+constexpr int WP2_THREADS = 32 * 18;   // warps 0-1 control, warps 2-17 workers
 enum { PB_FULL0 = 0, PB_FULL1, PB_EMPTY0, PB_EMPTY1, PB_VFULL, PB_GFULL, PB_PREADY, PB_VSREADY, PB_YFULL, PB_SFULL, PB_SCAL, PB_COUNT };
 
 template <int ANTI, bool DOT, bool RAGGED>
-__global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_pair_kernel(const __grid_constant__ CUtensorMap map_q,
+__global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __grid_constant__ CUtensorMap map_q,
                                                                     const __grid_constant__ CUtensorMap map_k,
                                                                     const __grid_constant__ CUtensorMap map_v,
                                                                     const __grid_constant__ CUtensorMap map_hs, const WalkArgs g) {
@@ -643,7 +644,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_pair_kernel(const __gri
   const int nseq = g.B * hp, cta = blockIdx.x, ncta = gridDim.x;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < PB_COUNT; ++i) mbar_init(bars + i, i == PB_PREADY || i == PB_VSREADY || i == PB_SCAL ? 8 : 1);
+    for (int i = 0; i < PB_COUNT; ++i) mbar_init(bars + i, i == PB_PREADY || i == PB_VSREADY || i == PB_SCAL ? 16 : 1);
     *abort = 0;
     mbar_fence_init();
   }
@@ -756,8 +757,8 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_pair_kernel(const __gri
 #pragma unroll
           for (int hh = 0; hh < 2; ++hh)
 #pragma unroll
-            for (int ks = 0; ks < 8; ++ks)   // 16 steps are 8 columns of P; 32 score columns hold 16 of head 0 and 16 of head 1
-              umma_f16_ta(tmem + TP_YD + hh * 64, tmem + TP_G + (ks >> 1) * 32 + hh * 16 + (ks & 1) * 8, d_v + hh * HEAD_U + ks * ROWS_U, id_yd, ks != 0 ? 1u : 0u);
+            for (int ks = 0; ks < 8; ++ks)   // 16 steps: 16 score columns, then 8 columns of head 0's P and 8 of head 1's
+              umma_f16_ta(tmem + TP_YD + hh * 64, tmem + TP_G + ks * 16 + hh * 8, d_v + hh * HEAD_U + ks * ROWS_U, id_yd, ks != 0 ? 1u : 0u);
           umma_commit(bars + PB_YFULL);
         }
         __syncwarp();
@@ -773,12 +774,13 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_pair_kernel(const __gri
   } else {
     // ------------------------------ workers -----------------------------------
     const int quarter = warp & 3;              // TMEM lane quarter this warp may read
-    const int ch = (warp - 2) >> 2;            // score columns: half `ch` for both heads; everything else: head `ch` of the pair
+    const int wg = (warp - 2) >> 2;            // score columns: 32-column piece `wg` for both heads
+    const int ch = wg >> 1, half = wg & 1;     // everything else: 32 columns (`half`) of head `ch` of the pair
     const int r = quarter * 32 + lane;         // row of every 128-row tile
     const uint32_t tl = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
     const int pitch = g.H * WP;
     unsigned char* hrow = sH + ch * W_TILE_V + r * 128;
-    unsigned char* stg = sVs + ch * W_TILE_V;  // this warp's rows: scaled values of chunk k+1, before that the staging of chunk k's output
+    unsigned char* stg = sVs + ch * W_TILE_V;  // this warp's rows and columns: scaled values of chunk k+1, before that the staging of chunk k's output
     WalkSeg sg;
     int qb = 0;
     bool alive = true;
@@ -788,17 +790,17 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_pair_kernel(const __gri
       const size_t bh = static_cast<size_t>(b) * g.H + h;
       const size_t LP = static_cast<size_t>(nc) * WQ;
       const size_t step0 = bh * LP + r, other0 = (ch == 0 ? bh + 1 : bh - 1) * LP + r;
-      float state[64];
+      float state[32];
       const int c_first = ANTI ? nc - 1 - sg.p0 : sg.p0;
       if (sg.cin) {
-        // the states the first part of these sequences ended with: written by all eight worker warps of the CTA that walked it
+        // the states the first part of these sequences ended with: written by all worker warps of the CTA that walked it
         if (lane == 0) {
           const uint64_t t0 = mp_globaltimer_ns();
           const uint64_t limit = mp_wait_limit_ns(g.status);
           while (true) {
             int seen;
             asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(g.carry_flag + sg.seq) : "memory");
-            if (seen >= 8) break;
+            if (seen >= 16) break;
             if (*abort != 0) break;
             if (mp_globaltimer_ns() - t0 > limit) {
               *abort = 1;
@@ -810,25 +812,25 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_pair_kernel(const __gri
         }
         __syncwarp();
         if (*abort != 0) { alive = false; break; }
-        const float4* src = reinterpret_cast<const float4*>(g.carry + (bh * WN + r) * WP);
+        const float4* src = reinterpret_cast<const float4*>(g.carry + (bh * WN + r) * WP + half * 32);
 #pragma unroll
-        for (int q4 = 0; q4 < 16; ++q4) {
+        for (int q4 = 0; q4 < 8; ++q4) {
           const float4 v4 = __ldcg(src + q4);
           state[q4 * 4] = v4.x; state[q4 * 4 + 1] = v4.y; state[q4 * 4 + 2] = v4.z; state[q4 * 4 + 3] = v4.w;
         }
       } else {
 #pragma unroll
-        for (int e = 0; e < 64; ++e) state[e] = 0.f;
+        for (int e = 0; e < 32; ++e) state[e] = 0.f;
         if (g.hs_out != nullptr) {   // the first chunk of a sequence's walk receives nothing
-          uint4* dst = reinterpret_cast<uint4*>(g.hs_out + ((bh * nc + c_first) * WN + r) * WP);
+          uint4* dst = reinterpret_cast<uint4*>(g.hs_out + ((bh * nc + c_first) * WN + r) * WP + half * 32);
 #pragma unroll
-          for (int q4 = 0; q4 < 8; ++q4) dst[q4] = make_uint4(0u, 0u, 0u, 0u);
+          for (int q4 = 0; q4 < 4; ++q4) dst[q4] = make_uint4(0u, 0u, 0u, 0u);
         }
       }
       // r16 copy of the state: operand of the next chunk's q H
       auto write_state = [&]() {
 #pragma unroll
-        for (int q4 = 0; q4 < 8; ++q4) *reinterpret_cast<uint4*>(hrow + ((q4 ^ (r & 7)) << 4)) = walk_pack8(state + q4 * 8);
+        for (int q4 = 0; q4 < 4; ++q4) *reinterpret_cast<uint4*>(hrow + (((half * 4 + q4) ^ (r & 7)) << 4)) = walk_pack8(state + q4 * 8);
       };
       if (sg.cin) write_state();   // (the tile is free: its last readers were complete before the previous segment's last S was)
       // scalars: chunk in hand (cur), the one after it (nxt), one more in flight (pre)
@@ -855,13 +857,13 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_pair_kernel(const __gri
             cum_nxt = cum_pre; dt_nxt = dt_pre; colf_nxt = colf_pre; oth_nxt = oth_pre;
             if (k + 2 < n) prefetch(k + 2);
           }
-          uint4 zc[8];
-          if (DOT) {   // the dot partner's rows of chunk k, whole 128-byte row pieces per load
+          uint4 zc[4];
+          if (DOT) {   // the dot partner's rows of chunk k, whole 64-byte row pieces per load
 #pragma unroll
-            for (int it = 0; it < 8; ++it) {
-              int zt = c * WQ + quarter * 32 + it * 4 + (lane >> 3);
+            for (int it = 0; it < 4; ++it) {
+              int zt = c * WQ + quarter * 32 + it * 8 + (lane >> 2);
               if (RAGGED) zt = min(zt, g.L - 1);   // the output rows beyond the sequence are zero: any row serves as their partner
-              zc[it] = *reinterpret_cast<const uint4*>(g.z + (static_cast<size_t>(b) * g.L + zt) * pitch + h * WP + (lane & 7) * 8);
+              zc[it] = *reinterpret_cast<const uint4*>(g.z + (static_cast<size_t>(b) * g.L + zt) * pitch + h * WP + half * 32 + (lane & 3) * 8);
             }
           }
           // ---- H' = D H + S ---------------------------------------------------------------
@@ -871,19 +873,19 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_pair_kernel(const __gri
             const float D = w_exp(last_cur);
 #pragma unroll
             for (int p = 0; p < 2; ++p) {
-              uint32_t sv[32];
-              tmem_ld_32x32(tl + TP_S + ch * 64 + p * 32, sv);
+              uint32_t sv[16];
+              tmem_ld_32x16(tl + TP_S + ch * 64 + half * 32 + p * 16, sv);
               tmem_ld_wait();
 #pragma unroll
-              for (int e = 0; e < 32; ++e) state[p * 32 + e] = D * state[p * 32 + e] + __uint_as_float(sv[e]);
+              for (int e = 0; e < 16; ++e) state[p * 16 + e] = D * state[p * 16 + e] + __uint_as_float(sv[e]);
             }
             if (more) {
               write_state();
             } else {
               // the first part of the sequences ends here: their states go to the CTA that walks the rest
-              float4* dst = reinterpret_cast<float4*>(g.carry + (bh * WN + r) * WP);
+              float4* dst = reinterpret_cast<float4*>(g.carry + (bh * WN + r) * WP + half * 32);
 #pragma unroll
-              for (int q4 = 0; q4 < 16; ++q4) __stcg(dst + q4, make_float4(state[q4 * 4], state[q4 * 4 + 1], state[q4 * 4 + 2], state[q4 * 4 + 3]));
+              for (int q4 = 0; q4 < 8; ++q4) __stcg(dst + q4, make_float4(state[q4 * 4], state[q4 * 4 + 1], state[q4 * 4 + 2], state[q4 * 4 + 3]));
               __threadfence();
               __syncwarp();
               if (lane == 0) atomicAdd(g.carry_flag + sg.seq, 1);
@@ -892,9 +894,9 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_pair_kernel(const __gri
           // ---- out = r o (Yd + f o Yo) of chunk k -------------------------------------------
           if (DOT) {
 #pragma unroll
-            for (int it = 0; it < 8; ++it) {
-              const int lr = quarter * 32 + it * 4 + (lane >> 3);
-              *reinterpret_cast<uint4*>(stg + lr * 128 + (((lane & 7) ^ (lr & 7)) << 4)) = zc[it];
+            for (int it = 0; it < 4; ++it) {
+              const int lr = quarter * 32 + it * 8 + (lane >> 2), cc = half * 4 + (lane & 3);
+              *reinterpret_cast<uint4*>(stg + lr * 128 + ((cc ^ (lr & 7)) << 4)) = zc[it];
             }
             __syncwarp();
           }
@@ -904,10 +906,10 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_pair_kernel(const __gri
           const float ro = ANTI ? dt_cur : 1.f;
           float dot = 0.f, dot_state = 0.f;
 #pragma unroll
-          for (int p = 0; p < 4; ++p) {
+          for (int p = 0; p < 2; ++p) {
             uint32_t yd[16], yo[16];
-            tmem_ld_32x16(tl + TP_YD + ch * 64 + p * 16, yd);
-            if (has_state) tmem_ld_32x16(tl + TP_YO + ch * 64 + p * 16, yo);
+            tmem_ld_32x16(tl + TP_YD + ch * 64 + half * 32 + p * 16, yd);
+            if (has_state) tmem_ld_32x16(tl + TP_YO + ch * 64 + half * 32 + p * 16, yo);
             tmem_ld_wait();
             if (!has_state) {
 #pragma unroll
@@ -920,7 +922,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_pair_kernel(const __gri
             }
 #pragma unroll
             for (int q4 = 0; q4 < 2; ++q4) {
-              uint4* slot = reinterpret_cast<uint4*>(stg + r * 128 + (((p * 2 + q4) ^ (r & 7)) << 4));
+              uint4* slot = reinterpret_cast<uint4*>(stg + r * 128 + (((half * 4 + p * 2 + q4) ^ (r & 7)) << 4));
               if (DOT) {   // this thread's row of z, before the output overwrites it
                 const uint4 zq = *slot;
                 const __half2* z2 = reinterpret_cast<const __half2*>(&zq);
@@ -944,28 +946,29 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_pair_kernel(const __gri
               dot_state *= fo;
               dot += dot_state;
               dot_state = warp_reduce<SumOp>(dot_state);
-              if (lane < 2) g.state_dot[(bh * nc + c) * 16 + quarter * 2 + lane] = lane == 0 ? dot_state : 0.f;
+              if (lane == 0) g.state_dot[(bh * nc + c) * 16 + quarter * 2 + half] = dot_state;
             }
-            g.dot_out[step0 + static_cast<size_t>(c) * WQ] = dot;
-            g.dot_out[static_cast<size_t>(g.B) * g.H * LP + step0 + static_cast<size_t>(c) * WQ] = 0.f;
+            g.dot_out[half * (static_cast<size_t>(g.B) * g.H * LP) + step0 + static_cast<size_t>(c) * WQ] = dot;
           }
           __syncwarp();
-          if (OUT) {   // whole 128-byte row pieces per store
+          if (OUT) {   // whole 64-byte row pieces per store
 #pragma unroll
-            for (int it = 0; it < 8; ++it) {
-              const int lr = quarter * 32 + it * 4 + (lane >> 3);
-              const uint4 val = *reinterpret_cast<const uint4*>(stg + lr * 128 + (((lane & 7) ^ (lr & 7)) << 4));
+            for (int it = 0; it < 4; ++it) {
+              const int lr = quarter * 32 + it * 8 + (lane >> 2), cc = half * 4 + (lane & 3);
+              const uint4 val = *reinterpret_cast<const uint4*>(stg + lr * 128 + ((cc ^ (lr & 7)) << 4));
               if (!RAGGED || c * WQ + lr < g.L)
-                *reinterpret_cast<uint4*>(g.out + (static_cast<size_t>(b) * g.L + c * WQ + lr) * pitch + h * WP + (lane & 7) * 8) = val;
+                *reinterpret_cast<uint4*>(g.out + (static_cast<size_t>(b) * g.L + c * WQ + lr) * pitch + h * WP + cc * 8) = val;
             }
             __syncwarp();
           }
         }
         if (more) {
           // ---- scalars of chunk k+1 into shared memory (every warp is past its P(k): Yd(k) was complete) -------------
-          s_colf[ch * WQ + r] = colf_nxt;
-          if ((r & 7) == (ANTI ? 0 : 7)) s_ref[ch * 16 + (r >> 3)] = cum_nxt;
-          if (r == WQ - 1) s_last[ch] = cum_nxt;
+          if (half == 0) {
+            s_colf[ch * WQ + r] = colf_nxt;
+            if ((r & 7) == (ANTI ? 0 : 7)) s_ref[ch * 16 + (r >> 3)] = cum_nxt;
+            if (r == WQ - 1) s_last[ch] = cum_nxt;
+          }
           __syncwarp();
           if (lane == 0) mbar_arrive(bars + PB_SCAL);
           if (!walk_wait(bars + PB_SCAL, parn, g.status, abort)) { alive = false; break; }
@@ -976,8 +979,8 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_pair_kernel(const __gri
             const __half2 wt2 = __float2half2_rn(ANTI ? w_exp(cum_nxt) : w_exp(last_nxt - cum_nxt) * dt_nxt);
             const unsigned char* src = sV + ch * W_TILE_V + r * 128;
 #pragma unroll
-            for (int q4 = 0; q4 < 8; ++q4) {
-              const int off = (q4 ^ (r & 7)) << 4;
+            for (int q4 = 0; q4 < 4; ++q4) {
+              const int off = ((half * 4 + q4) ^ (r & 7)) << 4;
               uint4 v = *reinterpret_cast<const uint4*>(src + off);
               __half2* h2 = reinterpret_cast<__half2*>(&v);
 #pragma unroll
@@ -989,56 +992,54 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_pair_kernel(const __gri
           // ---- P = G o F of chunk k+1, both heads, in place of the scores -------------------------------------------
           if (!walk_wait(bars + PB_GFULL, parn, g.status, abort)) { alive = false; break; }
           tcgen05_fence_after_sync();
+          // One block of 16 steps after the other, this warp's two; F: see ssd_walk_kernel.
 #pragma unroll 1
-          for (int pp = 0; pp < 2; ++pp) {
-            const int pc = ch * 2 + pp;              // 32-column piece of the chunk
-            const int j0 = pc * 32;
-            if (ANTI ? (pc < quarter) : (pc > quarter)) {   // warp-uniform: the whole piece is masked
+          for (int blk = 2 * wg; blk < 2 * wg + 2; ++blk) {
+            const uint32_t gcol = tl + TP_G + blk * 16;
+            if (ANTI ? (wg < quarter) : (wg > quarter)) {   // warp-uniform: the whole piece is masked
               uint32_t zero[16];
 #pragma unroll
               for (int e = 0; e < 16; ++e) zero[e] = 0u;
-              tmem_st_32x16(tl + TP_G + j0, zero);
-              tmem_st_32x16(tl + TP_G + j0 + 16, zero);
-            } else {
-              uint32_t v[32];
-              tmem_ld_32x32(tl + TP_G + j0, v);
-              // F: see ssd_walk_kernel
-              const bool diag = pc == quarter;
-              tmem_ld_wait();
-#pragma unroll 1
-              for (int hh = 0; hh < 2; ++hh) {
-                const float cum_r = hh == ch ? cum_nxt : oth_nxt;
-                uint32_t po[16];   // this head's 16 columns
+              tmem_st_32x16(gcol, zero);
+              continue;
+            }
+            const bool diag = wg == quarter;
+            const int l0 = (blk & 1) * 16;   // first step of the block relative to the piece, as `lane` counts rows on the diagonal
+            uint32_t v[16], po[16];
+            tmem_ld_32x16(gcol, v);
+            tmem_ld_wait();
 #pragma unroll
-                for (int sp = 0; sp < 4; ++sp) {
-                  const int jb = j0 + sp * 8;
-                  const float cref = s_ref[hh * 16 + (jb >> 3)];
-                  const float rarg = ANTI ? cref - cum_r : cum_r - cref;   // <= 0 off the diagonal
-                  const bool direct = rarg > 80.f;
-                  const float rowf = w_exp(direct ? 0.f : rarg);
-                  const float4 c0 = *reinterpret_cast<const float4*>(s_colf + hh * WQ + jb);
-                  const float4 c1 = *reinterpret_cast<const float4*>(s_colf + hh * WQ + jb + 4);
-                  float f[8] = {c0.x * rowf, c0.y * rowf, c0.z * rowf, c0.w * rowf, c1.x * rowf, c1.y * rowf, c1.z * rowf, c1.w * rowf};
-                  if (direct) {   // rare: the step factors from global memory
-                    const size_t o0 = (hh == ch ? step0 : other0) - r + static_cast<size_t>(ANTI ? c_first - k - 1 : c_first + k + 1) * WQ + jb;
+            for (int hh = 0; hh < 2; ++hh) {
+              const float cum_r = hh == ch ? cum_nxt : oth_nxt;
 #pragma unroll
-                    for (int e = 0; e < 8; ++e)
-                      f[e] = ANTI ? w_exp(fminf(g.cum[o0 + e] - cum_r, 0.f)) : w_exp(fminf(cum_r - g.cum[o0 + e], 0.f)) * g.dtt[o0 + e];
-                  }
-                  if (diag) {
+              for (int sp = 0; sp < 2; ++sp) {
+                const int jb = blk * 16 + sp * 8;
+                const float cref = s_ref[hh * 16 + (jb >> 3)];
+                const float rarg = ANTI ? cref - cum_r : cum_r - cref;   // <= 0 off the diagonal
+                const bool direct = rarg > 80.f;
+                const float rowf = w_exp(direct ? 0.f : rarg);
+                const float4 c0 = *reinterpret_cast<const float4*>(s_colf + hh * WQ + jb);
+                const float4 c1 = *reinterpret_cast<const float4*>(s_colf + hh * WQ + jb + 4);
+                float f[8] = {c0.x * rowf, c0.y * rowf, c0.z * rowf, c0.w * rowf, c1.x * rowf, c1.y * rowf, c1.z * rowf, c1.w * rowf};
+                if (direct) {   // rare: the step factors from global memory
+                  const size_t o0 = (hh == ch ? step0 : other0) - r + static_cast<size_t>(ANTI ? c_first - k - 1 : c_first + k + 1) * WQ + jb;
 #pragma unroll
-                    for (int e = 0; e < 8; ++e)
-                      if (ANTI ? (sp * 8 + e < lane) : (sp * 8 + e > lane)) f[e] = 0.f;
-                  }
-#pragma unroll
-                  for (int e = 0; e < 4; ++e) {
-                    const __half2 hv = __floats2half2_rn(__uint_as_float(v[sp * 8 + 2 * e]) * f[2 * e], __uint_as_float(v[sp * 8 + 2 * e + 1]) * f[2 * e + 1]);
-                    po[sp * 4 + e] = *reinterpret_cast<const uint32_t*>(&hv);
-                  }
+                  for (int e = 0; e < 8; ++e)
+                    f[e] = ANTI ? w_exp(fminf(g.cum[o0 + e] - cum_r, 0.f)) : w_exp(fminf(cum_r - g.cum[o0 + e], 0.f)) * g.dtt[o0 + e];
                 }
-                tmem_st_32x16(tl + TP_G + j0 + hh * 16, po);
+                if (diag) {
+#pragma unroll
+                  for (int e = 0; e < 8; ++e)
+                    if (ANTI ? (l0 + sp * 8 + e < lane) : (l0 + sp * 8 + e > lane)) f[e] = 0.f;
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  const __half2 hv = __floats2half2_rn(__uint_as_float(v[sp * 8 + 2 * e]) * f[2 * e], __uint_as_float(v[sp * 8 + 2 * e + 1]) * f[2 * e + 1]);
+                  po[hh * 8 + sp * 4 + e] = *reinterpret_cast<const uint32_t*>(&hv);
+                }
               }
             }
+            tmem_st_32x16(gcol, po);
           }
           tmem_st_wait();
           warp_arrive(bars + PB_PREADY, lane);
@@ -1676,7 +1677,7 @@ void mp_ssd_walk(int anti, const __half* q, const __half* k, const __half* v, co
   const CUtensorMap mh = hs_out != nullptr ? walk_map(hs_out, static_cast<size_t>(B) * H * g.nc * WN, WP) : mv;
   auto launch = [&](auto kernel, int smem) {
     MP_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    MpLaunch(grid, W_THREADS, smem, st)(kernel, mq, mk, mv, mh, g);
+    MpLaunch(grid, pairs ? WP2_THREADS : W_THREADS, smem, st)(kernel, mq, mk, mv, mh, g);
   };
   const bool dot = z != nullptr && dot_out != nullptr;
   if (!dot) { g.z = nullptr; g.dot_out = nullptr; }
