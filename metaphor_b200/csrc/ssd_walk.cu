@@ -610,7 +610,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_con
 // the workers are in the step before the one that needs it.
 // Shared memory has room for one v tile of each head only: v(k+1) is requested when Yd(k) has read v(k).  P lies in TMEM, in the columns
 // of the scores it is made from (16 score columns become 8 + 8 columns of packed r16 pairs, one block per head): Yd reads its
-// A operand there.
+// A operand there.  The states lie in TMEM as well: the workers leave D H (fp32) in S's accumulator, S adds to it.
 // ---------------------------------------------------------------------------
 constexpr int WP2_QK = 2 * W_TILE_QK;              // q and k of a chunk, 64 KB; two stages
 constexpr int WP2_OFF_V = 2 * WP2_QK;              // v of both heads
@@ -638,7 +638,6 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
   volatile int* abort = reinterpret_cast<volatile int*>(smem + WP2_OFF_TAIL + 116);
   float* s_colf = reinterpret_cast<float*>(smem + WP2_OFF_TAIL + 128);   // [2][128]
   float* s_ref = s_colf + 2 * WQ;                                        // [2][16]: cum at the far end of every 8-step piece
-  float* s_last = s_ref + 32;                                            // [2]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nc = g.nc, hp = g.H / 2;
   const int nseq = g.B * hp, cta = blockIdx.x, ncta = gridDim.x;
@@ -739,7 +738,7 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
           for (int ks = 0; ks < 8; ++ks) umma<false>(tmem + TP_YO, dq + kslice(ks), d_h + ks * ROWS_U, id_yo, ks != 0 ? 1u : 0u);
         }
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) umma<false>(tmem + TP_S, dkt + ks * ROWS_U, d_vs + ks * ROWS_U, id_s, ks != 0 ? 1u : 0u);
+        for (int ks = 0; ks < 8; ++ks) umma<false>(tmem + TP_S, dkt + ks * ROWS_U, d_vs + ks * ROWS_U, id_s, (has_state || ks != 0) ? 1u : 0u);
         // the workers rewrite the state tiles once S(k) is complete: the stores must have read them by then
         if (g.hs_out != nullptr && has_state) bulk_wait_read<0>();
         umma_commit(bars + PB_SFULL);
@@ -748,12 +747,11 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
       __syncwarp();
     };
     for (int si = 0; ok && walk_segment(cta, ncta, nseq, nc, si, sg); ++si) {
-      issue_g(qb);
-      if (ok) issue_state(0);
-      for (int k = 0; ok && k < sg.n; ++k) {
+#pragma unroll 1
+      for (int k = -1; ok && k < sg.n; ++k) {   // k = -1 only starts chunk 0
         const int q = qb + k;
-        if (!await(PB_PREADY, q & 1) || !await(PB_VFULL, q & 1)) break;
-        if (elect_one()) {
+        if (k >= 0 && (!await(PB_PREADY, q & 1) || !await(PB_VFULL, q & 1))) break;
+        if (k >= 0 && elect_one()) {
 #pragma unroll
           for (int hh = 0; hh < 2; ++hh)
 #pragma unroll
@@ -789,9 +787,19 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
       const int h = 2 * (sg.seq % hp) + ch, b = sg.seq / hp;
       const size_t bh = static_cast<size_t>(b) * g.H + h;
       const size_t LP = static_cast<size_t>(nc) * WQ;
+      // this thread's step in the first chunk of the walk, in the arrays per step of its head and of the other one
       const size_t step0 = bh * LP + r, other0 = (ch == 0 ? bh + 1 : bh - 1) * LP + r;
-      float state[32];
+      const uint32_t tstate = tl + TP_S + ch * 64 + half * 32;
       const int c_first = ANTI ? nc - 1 - sg.p0 : sg.p0;
+      // 16 columns of the state a chunk receives: an r16 copy for its q H, and D times it (D: the chunk's decay) for its S to add to
+      auto store_state = [&](const float* hv, int p, float D) {
+#pragma unroll
+        for (int q4 = 0; q4 < 2; ++q4) *reinterpret_cast<uint4*>(hrow + (((half * 4 + p * 2 + q4) ^ (r & 7)) << 4)) = walk_pack8(hv + q4 * 8);
+        uint32_t sv[16];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) sv[e] = __float_as_uint(D * hv[e]);
+        tmem_st_32x16(tstate + p * 16, sv);
+      };
       if (sg.cin) {
         // the states the first part of these sequences ended with: written by all worker warps of the CTA that walked it
         if (lane == 0) {
@@ -813,36 +821,34 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
         __syncwarp();
         if (*abort != 0) { alive = false; break; }
         const float4* src = reinterpret_cast<const float4*>(g.carry + (bh * WN + r) * WP + half * 32);
+        const float D = w_exp(g.cum[step0 - r + static_cast<size_t>(c_first) * WQ + WQ - 1]);
 #pragma unroll
-        for (int q4 = 0; q4 < 8; ++q4) {
-          const float4 v4 = __ldcg(src + q4);
-          state[q4 * 4] = v4.x; state[q4 * 4 + 1] = v4.y; state[q4 * 4 + 2] = v4.z; state[q4 * 4 + 3] = v4.w;
+        for (int p = 0; p < 2; ++p) {
+          float hv[16];
+#pragma unroll
+          for (int q4 = 0; q4 < 4; ++q4) {
+            const float4 v4 = __ldcg(src + p * 4 + q4);
+            hv[q4 * 4] = v4.x; hv[q4 * 4 + 1] = v4.y; hv[q4 * 4 + 2] = v4.z; hv[q4 * 4 + 3] = v4.w;
+          }
+          store_state(hv, p, D);   // (the tiles are free: their last readers were complete before the previous segment's last S was)
         }
+        tmem_st_wait();
       } else {
-#pragma unroll
-        for (int e = 0; e < 32; ++e) state[e] = 0.f;
         if (g.hs_out != nullptr) {   // the first chunk of a sequence's walk receives nothing
           uint4* dst = reinterpret_cast<uint4*>(g.hs_out + ((bh * nc + c_first) * WN + r) * WP + half * 32);
 #pragma unroll
           for (int q4 = 0; q4 < 4; ++q4) dst[q4] = make_uint4(0u, 0u, 0u, 0u);
         }
       }
-      // r16 copy of the state: operand of the next chunk's q H
-      auto write_state = [&]() {
-#pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4) *reinterpret_cast<uint4*>(hrow + (((half * 4 + q4) ^ (r & 7)) << 4)) = walk_pack8(state + q4 * 8);
-      };
-      if (sg.cin) write_state();   // (the tile is free: its last readers were complete before the previous segment's last S was)
-      // scalars: chunk in hand (cur), the one after it (nxt), one more in flight (pre)
-      float cum_cur = 0.f, dt_cur = 0.f, last_cur = 0.f, last_nxt = 0.f;
-      const size_t i0 = static_cast<size_t>(c_first) * WQ;
-      float cum_nxt = g.cum[step0 + i0], dt_nxt = g.dtt[step0 + i0], colf_nxt = g.colf[step0 + i0], oth_nxt = g.cum[other0 + i0];
-      float cum_pre = 0.f, dt_pre = 0.f, colf_pre = 0.f, oth_pre = 0.f;
-      auto prefetch = [&](int k) {
+      // scalars of the chunk in hand (cur) and of the one after it (nxt), which are requested a whole chunk before they are used
+      float cum_cur = 0.f, dt_cur = 0.f, last_cur = 0.f;
+      float cum_nxt, dt_nxt, colf_nxt, oth_nxt, last_nxt;
+      auto fetch = [&](int k) {
         const size_t i = static_cast<size_t>(ANTI ? c_first - k : c_first + k) * WQ;
-        cum_pre = g.cum[step0 + i]; dt_pre = g.dtt[step0 + i]; colf_pre = g.colf[step0 + i]; oth_pre = g.cum[other0 + i];
+        cum_nxt = g.cum[step0 + i]; dt_nxt = g.dtt[step0 + i]; colf_nxt = g.colf[step0 + i]; oth_nxt = g.cum[other0 + i];
+        last_nxt = g.cum[step0 - r + i + WQ - 1];
       };
-      if (n > 1) prefetch(1);
+      fetch(0);
 
 #pragma unroll 1
       for (int k = -1; k < n; ++k) {   // finishes chunk k, prepares chunk k+1; k = -1 only prepares
@@ -853,10 +859,7 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
         if (k >= 0) {
           const bool has_state = k > 0 || sg.cin != 0;
           cum_cur = cum_nxt; dt_cur = dt_nxt; last_cur = last_nxt;
-          if (more) {
-            cum_nxt = cum_pre; dt_nxt = dt_pre; colf_nxt = colf_pre; oth_nxt = oth_pre;
-            if (k + 2 < n) prefetch(k + 2);
-          }
+          if (more) fetch(k + 1);
           uint4 zc[4];
           if (DOT) {   // the dot partner's rows of chunk k, whole 64-byte row pieces per load
 #pragma unroll
@@ -866,26 +869,29 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
               zc[it] = *reinterpret_cast<const uint4*>(g.z + (static_cast<size_t>(b) * g.L + zt) * pitch + h * WP + half * 32 + (lane & 3) * 8);
             }
           }
-          // ---- H' = D H + S ---------------------------------------------------------------
+          // ---- the state chunk k+1 receives: D H + S of chunk k, complete in S's accumulator -------------------------
           if (!walk_wait(bars + PB_SFULL, par, g.status, abort)) { alive = false; break; }
           tcgen05_fence_after_sync();
           if (more || sg.cout) {
-            const float D = w_exp(last_cur);
+            const float D = w_exp(last_nxt);
 #pragma unroll
             for (int p = 0; p < 2; ++p) {
               uint32_t sv[16];
-              tmem_ld_32x16(tl + TP_S + ch * 64 + half * 32 + p * 16, sv);
+              tmem_ld_32x16(tstate + p * 16, sv);
               tmem_ld_wait();
+              if (more) {
+                store_state(reinterpret_cast<const float*>(sv), p, D);
+              } else {   // the first part of the sequences ends here: their states go to the CTA that walks the rest
+                float4* dst = reinterpret_cast<float4*>(g.carry + (bh * WN + r) * WP + half * 32 + p * 16);
 #pragma unroll
-              for (int e = 0; e < 16; ++e) state[p * 16 + e] = D * state[p * 16 + e] + __uint_as_float(sv[e]);
+                for (int q4 = 0; q4 < 4; ++q4)
+                  __stcg(dst + q4, make_float4(__uint_as_float(sv[q4 * 4]), __uint_as_float(sv[q4 * 4 + 1]), __uint_as_float(sv[q4 * 4 + 2]),
+                                               __uint_as_float(sv[q4 * 4 + 3])));
+              }
             }
             if (more) {
-              write_state();
+              tmem_st_wait();
             } else {
-              // the first part of the sequences ends here: their states go to the CTA that walks the rest
-              float4* dst = reinterpret_cast<float4*>(g.carry + (bh * WN + r) * WP + half * 32);
-#pragma unroll
-              for (int q4 = 0; q4 < 8; ++q4) __stcg(dst + q4, make_float4(state[q4 * 4], state[q4 * 4 + 1], state[q4 * 4 + 2], state[q4 * 4 + 3]));
               __threadfence();
               __syncwarp();
               if (lane == 0) atomicAdd(g.carry_flag + sg.seq, 1);
@@ -967,12 +973,10 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
           if (half == 0) {
             s_colf[ch * WQ + r] = colf_nxt;
             if ((r & 7) == (ANTI ? 0 : 7)) s_ref[ch * 16 + (r >> 3)] = cum_nxt;
-            if (r == WQ - 1) s_last[ch] = cum_nxt;
           }
           __syncwarp();
           if (lane == 0) mbar_arrive(bars + PB_SCAL);
           if (!walk_wait(bars + PB_SCAL, parn, g.status, abort)) { alive = false; break; }
-          last_nxt = s_last[ch];
           // ---- w o v of chunk k+1: operand of its state update ------------------------------------------------------
           if (!walk_wait(bars + PB_VFULL, parn, g.status, abort)) { alive = false; break; }
           {
@@ -1005,12 +1009,13 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
             }
             const bool diag = wg == quarter;
             const int l0 = (blk & 1) * 16;   // first step of the block relative to the piece, as `lane` counts rows on the diagonal
-            uint32_t v[16], po[16];
+            uint32_t v[16];
             tmem_ld_32x16(gcol, v);
             tmem_ld_wait();
-#pragma unroll
+#pragma unroll 1
             for (int hh = 0; hh < 2; ++hh) {
               const float cum_r = hh == ch ? cum_nxt : oth_nxt;
+              uint32_t po[8];
 #pragma unroll
               for (int sp = 0; sp < 2; ++sp) {
                 const int jb = blk * 16 + sp * 8;
@@ -1035,11 +1040,11 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                   const __half2 hv = __floats2half2_rn(__uint_as_float(v[sp * 8 + 2 * e]) * f[2 * e], __uint_as_float(v[sp * 8 + 2 * e + 1]) * f[2 * e + 1]);
-                  po[hh * 8 + sp * 4 + e] = *reinterpret_cast<const uint32_t*>(&hv);
+                  po[sp * 4 + e] = *reinterpret_cast<const uint32_t*>(&hv);
                 }
               }
+              tmem_st_32x8(gcol + hh * 8, po);
             }
-            tmem_st_32x16(gcol, po);
           }
           tmem_st_wait();
           warp_arrive(bars + PB_PREADY, lane);
