@@ -112,6 +112,12 @@ __device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
   if (lane == 0) mbar_arrive(bar);
 }
 
+// 16 bytes global -> shared by this thread, without a register in between.
+__device__ __forceinline__ void cp_async_16(void* smem_dst, const void* gmem_src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(mp_smem_u32(smem_dst)), "l"(gmem_src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // The hand-offs of the walk sit on its critical path: poll without a suspend hint first (a suspended warp
 // wakes up hundreds of cycles after the phase completes), then fall back to the bounded, abortable wait.
 __device__ __forceinline__ bool walk_wait(uint64_t* bar, uint32_t parity, uint32_t* status, volatile int* abort) {
@@ -619,7 +625,8 @@ constexpr int WP2_OFF_VS = WP2_OFF_H + 2 * W_TILE_V;
 constexpr int WP2_OFF_TAIL = WP2_OFF_VS + 2 * W_TILE_V;   // 229376
 constexpr int WP2_SMEM_BYTES = WP2_OFF_TAIL + 2048 + 1024;
 constexpr uint32_t TP_G = 0, TP_S = 128, TP_YD = 256, TP_YO = 384;   // TMEM columns; head h of a pair at + 64 h
-constexpr int WP2_THREADS = 32 * 18;   // warps 0-1 control, warps 2-17 workers
+constexpr int WP2_THREADS = 32 * 20;   // warps 0-1 control (2-3 idle), warps 4-19 workers: 640 threads are launched with 96 registers each,
+                                       // of which the control warpgroup keeps 64 and the workers take 104 (128 * 64 + 512 * 104 = 640 * 96)
 enum { PB_FULL0 = 0, PB_FULL1, PB_EMPTY0, PB_EMPTY1, PB_VFULL, PB_GFULL, PB_PREADY, PB_VSREADY, PB_YFULL, PB_SFULL, PB_SCAL, PB_COUNT };
 
 template <int ANTI, bool DOT, bool RAGGED>
@@ -654,6 +661,8 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
   const uint32_t tmem = *tmem_slot;
   mp_grid_wait();
 
+  if (warp < 4) {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
     if (lane == 0) {
@@ -695,11 +704,16 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
     const uint32_t id_yo = umma_instr_desc(UMMA_FMT_F16, 0u, 1u, 128, 128);   // q (K-major) x MN-major states of both heads
     const uint32_t id_s = umma_instr_desc(UMMA_FMT_F16, 1u, 1u, 128, 128);    // k^T (MN-major A) x MN-major scaled values of both
     const uint32_t s0 = mp_smem_u32(smem);
-    const uint64_t d_q = umma_smem_desc(s0, 16, 1024), d_k = umma_smem_desc(s0 + W_TILE_QK, 16, 1024);
+    const uint64_t d_q = umma_smem_desc(s0, 16, 1024);
     const uint64_t d_kt = umma_smem_desc(s0 + W_TILE_QK, WQ * 128, 1024), d_v = umma_smem_desc(mp_smem_u32(sV), W_TILE_V, 1024);
-    const uint64_t d_h = umma_smem_desc(mp_smem_u32(sH), W_TILE_V, 1024), d_vs = umma_smem_desc(mp_smem_u32(sVs), W_TILE_V, 1024);
-    constexpr uint32_t STAGE_U = WP2_QK >> 4, ROWS_U = 2048 >> 4, HEAD_U = W_TILE_V >> 4;
+    const uint64_t d_h = umma_smem_desc(mp_smem_u32(sH), W_TILE_V, 1024);   // the scaled values follow the states
+    constexpr uint32_t STAGE_U = WP2_QK >> 4, QK_U = W_TILE_QK >> 4, ROWS_U = 2048 >> 4, HEAD_U = W_TILE_V >> 4;
     auto kslice = [](int ks) { return static_cast<uint32_t>(((ks >> 2) * (WQ * 128) + (ks & 3) * 32) >> 4); };   // K-major: two 64-column blocks
+    // The operands' steps are added up where they are used: hoisted out of the walk's loop they take more registers than this role has.
+    auto fresh = [](uint64_t d) {
+      asm volatile("" : "+l"(d));
+      return d;
+    };
     bool ok = true;
     auto await = [&](int bar, uint32_t parity) {
       ok = walk_wait(bars + bar, parity, g.status, abort);
@@ -709,7 +723,7 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
     };
     auto issue_g = [&](int q) {
       if (!await(PB_FULL0 + (q & 1), (q >> 1) & 1)) return;
-      const uint64_t dq = d_q + (q & 1) * STAGE_U, dk = d_k + (q & 1) * STAGE_U;
+      const uint64_t dq = fresh(d_q) + (q & 1) * STAGE_U, dk = dq + QK_U;
       if (elect_one()) {
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) umma<false>(tmem + TP_G, dq + kslice(ks), dk + kslice(ks), id_g, ks != 0 ? 1u : 0u);
@@ -724,7 +738,7 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
       const int q = qb + k;
       if (!await(PB_VSREADY, q & 1)) return;
       const bool has_state = k > 0 || sg.cin != 0;
-      const uint64_t dq = d_q + (q & 1) * STAGE_U, dkt = d_kt + (q & 1) * STAGE_U;
+      const uint64_t dq = fresh(d_q) + (q & 1) * STAGE_U, dkt = fresh(d_kt) + (q & 1) * STAGE_U, dh = fresh(d_h), dvs = dh + 2 * HEAD_U;
       if (elect_one()) {
         if (has_state) {
           if (g.hs_out != nullptr) {   // the states this chunk receives, straight from their operand tiles
@@ -735,10 +749,10 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
             bulk_commit();
           }
 #pragma unroll
-          for (int ks = 0; ks < 8; ++ks) umma<false>(tmem + TP_YO, dq + kslice(ks), d_h + ks * ROWS_U, id_yo, ks != 0 ? 1u : 0u);
+          for (int ks = 0; ks < 8; ++ks) umma<false>(tmem + TP_YO, dq + kslice(ks), dh + ks * ROWS_U, id_yo, ks != 0 ? 1u : 0u);
         }
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) umma<false>(tmem + TP_S, dkt + ks * ROWS_U, d_vs + ks * ROWS_U, id_s, (has_state || ks != 0) ? 1u : 0u);
+        for (int ks = 0; ks < 8; ++ks) umma<false>(tmem + TP_S, dkt + ks * ROWS_U, dvs + ks * ROWS_U, id_s, (has_state || ks != 0) ? 1u : 0u);
         // the workers rewrite the state tiles once S(k) is complete: the stores must have read them by then
         if (g.hs_out != nullptr && has_state) bulk_wait_read<0>();
         umma_commit(bars + PB_SFULL);
@@ -752,11 +766,12 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
         const int q = qb + k;
         if (k >= 0 && (!await(PB_PREADY, q & 1) || !await(PB_VFULL, q & 1))) break;
         if (k >= 0 && elect_one()) {
+          const uint64_t dv = fresh(d_v);
 #pragma unroll
           for (int hh = 0; hh < 2; ++hh)
 #pragma unroll
             for (int ks = 0; ks < 8; ++ks)   // 16 steps: 16 score columns, then 8 columns of head 0's P and 8 of head 1's
-              umma_f16_ta(tmem + TP_YD + hh * 64, tmem + TP_G + ks * 16 + hh * 8, d_v + hh * HEAD_U + ks * ROWS_U, id_yd, ks != 0 ? 1u : 0u);
+              umma_f16_ta(tmem + TP_YD + hh * 64, tmem + TP_G + ks * 16 + hh * 8, dv + hh * HEAD_U + ks * ROWS_U, id_yd, ks != 0 ? 1u : 0u);
           umma_commit(bars + PB_YFULL);
         }
         __syncwarp();
@@ -769,10 +784,12 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
     }
     mp_launch_dependents();
     if (g.hs_out != nullptr) bulk_wait_all<0>();
+  }
   } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
     // ------------------------------ workers -----------------------------------
     const int quarter = warp & 3;              // TMEM lane quarter this warp may read
-    const int wg = (warp - 2) >> 2;            // score columns: 32-column piece `wg` for both heads
+    const int wg = (warp - 4) >> 2;            // score columns: 32-column piece `wg` for both heads
     const int ch = wg >> 1, half = wg & 1;     // everything else: 32 columns (`half`) of head `ch` of the pair
     const int r = quarter * 32 + lane;         // row of every 128-row tile
     const uint32_t tl = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
@@ -860,18 +877,18 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
           const bool has_state = k > 0 || sg.cin != 0;
           cum_cur = cum_nxt; dt_cur = dt_nxt; last_cur = last_nxt;
           if (more) fetch(k + 1);
-          uint4 zc[4];
-          if (DOT) {   // the dot partner's rows of chunk k, whole 64-byte row pieces per load
-#pragma unroll
-            for (int it = 0; it < 4; ++it) {
-              int zt = c * WQ + quarter * 32 + it * 8 + (lane >> 2);
-              if (RAGGED) zt = min(zt, g.L - 1);   // the output rows beyond the sequence are zero: any row serves as their partner
-              zc[it] = *reinterpret_cast<const uint4*>(g.z + (static_cast<size_t>(b) * g.L + zt) * pitch + h * WP + half * 32 + (lane & 3) * 8);
-            }
-          }
           // ---- the state chunk k+1 receives: D H + S of chunk k, complete in S's accumulator -------------------------
           if (!walk_wait(bars + PB_SFULL, par, g.status, abort)) { alive = false; break; }
           tcgen05_fence_after_sync();
+          if (DOT) {   // the dot partner's rows of chunk k into this warp's part of the tile that S(k) has read, whole 64-byte row pieces
+#pragma unroll
+            for (int it = 0; it < 4; ++it) {
+              const int lr = quarter * 32 + it * 8 + (lane >> 2), cc = half * 4 + (lane & 3);
+              int zt = c * WQ + lr;
+              if (RAGGED) zt = min(zt, g.L - 1);   // the output rows beyond the sequence are zero: any row serves as their partner
+              cp_async_16(stg + lr * 128 + ((cc ^ (lr & 7)) << 4), g.z + (static_cast<size_t>(b) * g.L + zt) * pitch + h * WP + cc * 8);
+            }
+          }
           if (more || sg.cout) {
             const float D = w_exp(last_nxt);
 #pragma unroll
@@ -898,18 +915,14 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
             }
           }
           // ---- out = r o (Yd + f o Yo) of chunk k -------------------------------------------
-          if (DOT) {
-#pragma unroll
-            for (int it = 0; it < 4; ++it) {
-              const int lr = quarter * 32 + it * 8 + (lane >> 2), cc = half * 4 + (lane & 3);
-              *reinterpret_cast<uint4*>(stg + lr * 128 + ((cc ^ (lr & 7)) << 4)) = zc[it];
-            }
-            __syncwarp();
-          }
           if (!walk_wait(bars + PB_YFULL, par, g.status, abort)) { alive = false; break; }
           tcgen05_fence_after_sync();
           const float fo = has_state ? (ANTI ? w_exp(last_cur - cum_cur) : w_exp(cum_cur)) : 0.f;
           const float ro = ANTI ? dt_cur : 1.f;
+          if (DOT) {
+            cp_async_wait_all();
+            __syncwarp();
+          }
           float dot = 0.f, dot_state = 0.f;
 #pragma unroll
           for (int p = 0; p < 2; ++p) {
