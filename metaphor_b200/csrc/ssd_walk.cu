@@ -808,14 +808,14 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
       const size_t step0 = bh * LP + r, other0 = (ch == 0 ? bh + 1 : bh - 1) * LP + r;
       const uint32_t tstate = tl + TP_S + ch * 64 + half * 32;
       const int c_first = ANTI ? nc - 1 - sg.p0 : sg.p0;
-      // 16 columns of the state a chunk receives: an r16 copy for its q H, and D times it (D: the chunk's decay) for its S to add to
-      auto store_state = [&](const float* hv, int p, float D) {
+      // the 32 columns of the state a chunk receives: an r16 copy for its q H, and D times it (D: the chunk's decay) for its S to add to
+      auto store_state = [&](float* hv, float D) {
 #pragma unroll
-        for (int q4 = 0; q4 < 2; ++q4) *reinterpret_cast<uint4*>(hrow + (((half * 4 + p * 2 + q4) ^ (r & 7)) << 4)) = walk_pack8(hv + q4 * 8);
-        uint32_t sv[16];
+        for (int q4 = 0; q4 < 4; ++q4) *reinterpret_cast<uint4*>(hrow + (((half * 4 + q4) ^ (r & 7)) << 4)) = walk_pack8(hv + q4 * 8);
 #pragma unroll
-        for (int e = 0; e < 16; ++e) sv[e] = __float_as_uint(D * hv[e]);
-        tmem_st_32x16(tstate + p * 16, sv);
+        for (int e = 0; e < 32; ++e) hv[e] *= D;
+        tmem_st_32x32(tstate, reinterpret_cast<const uint32_t*>(hv));
+        tmem_st_wait();
       };
       if (sg.cin) {
         // the states the first part of these sequences ended with: written by all worker warps of the CTA that walked it
@@ -839,17 +839,13 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
         if (*abort != 0) { alive = false; break; }
         const float4* src = reinterpret_cast<const float4*>(g.carry + (bh * WN + r) * WP + half * 32);
         const float D = w_exp(g.cum[step0 - r + static_cast<size_t>(c_first) * WQ + WQ - 1]);
+        float hv[32];
 #pragma unroll
-        for (int p = 0; p < 2; ++p) {
-          float hv[16];
-#pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4) {
-            const float4 v4 = __ldcg(src + p * 4 + q4);
-            hv[q4 * 4] = v4.x; hv[q4 * 4 + 1] = v4.y; hv[q4 * 4 + 2] = v4.z; hv[q4 * 4 + 3] = v4.w;
-          }
-          store_state(hv, p, D);   // (the tiles are free: their last readers were complete before the previous segment's last S was)
+        for (int q4 = 0; q4 < 8; ++q4) {
+          const float4 v4 = __ldcg(src + q4);
+          hv[q4 * 4] = v4.x; hv[q4 * 4 + 1] = v4.y; hv[q4 * 4 + 2] = v4.z; hv[q4 * 4 + 3] = v4.w;
         }
-        tmem_st_wait();
+        store_state(hv, D);   // (the tiles are free: their last readers were complete before the previous segment's last S was)
       } else {
         if (g.hs_out != nullptr) {   // the first chunk of a sequence's walk receives nothing
           uint4* dst = reinterpret_cast<uint4*>(g.hs_out + ((bh * nc + c_first) * WN + r) * WP + half * 32);
@@ -890,25 +886,15 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
             }
           }
           if (more || sg.cout) {
-            const float D = w_exp(last_nxt);
-#pragma unroll
-            for (int p = 0; p < 2; ++p) {
-              uint32_t sv[16];
-              tmem_ld_32x16(tstate + p * 16, sv);
-              tmem_ld_wait();
-              if (more) {
-                store_state(reinterpret_cast<const float*>(sv), p, D);
-              } else {   // the first part of the sequences ends here: their states go to the CTA that walks the rest
-                float4* dst = reinterpret_cast<float4*>(g.carry + (bh * WN + r) * WP + half * 32 + p * 16);
-#pragma unroll
-                for (int q4 = 0; q4 < 4; ++q4)
-                  __stcg(dst + q4, make_float4(__uint_as_float(sv[q4 * 4]), __uint_as_float(sv[q4 * 4 + 1]), __uint_as_float(sv[q4 * 4 + 2]),
-                                               __uint_as_float(sv[q4 * 4 + 3])));
-              }
-            }
+            float hv[32];
+            tmem_ld_32x32(tstate, reinterpret_cast<uint32_t*>(hv));
+            tmem_ld_wait();
             if (more) {
-              tmem_st_wait();
-            } else {
+              store_state(hv, w_exp(last_nxt));
+            } else {   // the first part of the sequences ends here: their states go to the CTA that walks the rest
+              float4* dst = reinterpret_cast<float4*>(g.carry + (bh * WN + r) * WP + half * 32);
+#pragma unroll
+              for (int q4 = 0; q4 < 8; ++q4) __stcg(dst + q4, make_float4(hv[q4 * 4], hv[q4 * 4 + 1], hv[q4 * 4 + 2], hv[q4 * 4 + 3]));
               __threadfence();
               __syncwarp();
               if (lane == 0) atomicAdd(g.carry_flag + sg.seq, 1);
@@ -934,13 +920,13 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
 #pragma unroll
               for (int e = 0; e < 16; ++e) yo[e] = 0u;
             }
-            float o[16];
-            if (OUT) {
-#pragma unroll
-              for (int e = 0; e < 16; ++e) o[e] = ro * (__uint_as_float(yd[e]) + fo * __uint_as_float(yo[e]));
-            }
 #pragma unroll
             for (int q4 = 0; q4 < 2; ++q4) {
+              float o[8];
+              if (OUT) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) o[e] = ro * (__uint_as_float(yd[q4 * 8 + e]) + fo * __uint_as_float(yo[q4 * 8 + e]));
+              }
               uint4* slot = reinterpret_cast<uint4*>(stg + r * 128 + (((half * 4 + p * 2 + q4) ^ (r & 7)) << 4));
               if (DOT) {   // this thread's row of z, before the output overwrites it
                 const uint4 zq = *slot;
@@ -950,14 +936,14 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
                   const float2 zf = __half22float2(z2[e]);
                   const int k0 = q4 * 8 + 2 * e;
                   if (OUT) {
-                    dot += zf.x * o[k0] + zf.y * o[k0 + 1];
+                    dot += zf.x * o[2 * e] + zf.y * o[2 * e + 1];
                   } else {
                     dot += zf.x * __uint_as_float(yd[k0]) + zf.y * __uint_as_float(yd[k0 + 1]);
                     dot_state += zf.x * __uint_as_float(yo[k0]) + zf.y * __uint_as_float(yo[k0 + 1]);
                   }
                 }
               }
-              if (OUT) *slot = walk_pack8(o + q4 * 8);
+              if (OUT) *slot = walk_pack8(o);
             }
           }
           if (DOT) {
@@ -989,7 +975,6 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
           }
           __syncwarp();
           if (lane == 0) mbar_arrive(bars + PB_SCAL);
-          if (!walk_wait(bars + PB_SCAL, parn, g.status, abort)) { alive = false; break; }
           // ---- w o v of chunk k+1: operand of its state update ------------------------------------------------------
           if (!walk_wait(bars + PB_VFULL, parn, g.status, abort)) { alive = false; break; }
           {
@@ -1007,33 +992,31 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
           }
           warp_arrive(bars + PB_VSREADY, lane);
           // ---- P = G o F of chunk k+1, both heads, in place of the scores -------------------------------------------
+          if (!walk_wait(bars + PB_SCAL, parn, g.status, abort)) { alive = false; break; }
           if (!walk_wait(bars + PB_GFULL, parn, g.status, abort)) { alive = false; break; }
           tcgen05_fence_after_sync();
-          // One block of 16 steps after the other, this warp's two; F: see ssd_walk_kernel.
-#pragma unroll 1
-          for (int blk = 2 * wg; blk < 2 * wg + 2; ++blk) {
-            const uint32_t gcol = tl + TP_G + blk * 16;
-            if (ANTI ? (wg < quarter) : (wg > quarter)) {   // warp-uniform: the whole piece is masked
-              uint32_t zero[16];
+          // This warp's 32 steps, one head after the other; F: see ssd_walk_kernel.
+          const uint32_t gcol = tl + TP_G + wg * 32;
+          if (ANTI ? (wg < quarter) : (wg > quarter)) {   // warp-uniform: the whole piece is masked
+            uint32_t zero[32];
 #pragma unroll
-              for (int e = 0; e < 16; ++e) zero[e] = 0u;
-              tmem_st_32x16(gcol, zero);
-              continue;
-            }
+            for (int e = 0; e < 32; ++e) zero[e] = 0u;
+            tmem_st_32x32(gcol, zero);
+          } else {
             const bool diag = wg == quarter;
-            const int l0 = (blk & 1) * 16;   // first step of the block relative to the piece, as `lane` counts rows on the diagonal
-            uint32_t v[16];
-            tmem_ld_32x16(gcol, v);
-            tmem_ld_wait();
 #pragma unroll 1
-            for (int hh = 0; hh < 2; ++hh) {
-              const float cum_r = hh == ch ? cum_nxt : oth_nxt;
-              uint32_t po[8];
+            for (int blk = 0; blk < 2; ++blk) {
+              uint32_t v[16], po[16];
+              tmem_ld_32x16(gcol + blk * 16, v);
+              const int jb0 = wg * 32 + blk * 16;
+              const float2 ref0 = *reinterpret_cast<const float2*>(s_ref + (jb0 >> 3)), ref1 = *reinterpret_cast<const float2*>(s_ref + 16 + (jb0 >> 3));
+              tmem_ld_wait();
 #pragma unroll
-              for (int sp = 0; sp < 2; ++sp) {
-                const int jb = blk * 16 + sp * 8;
-                const float cref = s_ref[hh * 16 + (jb >> 3)];
-                const float rarg = ANTI ? cref - cum_r : cum_r - cref;   // <= 0 off the diagonal
+              for (int hs = 0; hs < 4; ++hs) {   // head of the pair, 8 steps
+                const int hh = hs >> 1, sp = hs & 1, jb = jb0 + sp * 8;
+                const float cum_r = hh == ch ? cum_nxt : oth_nxt;
+                const float cr = hh == 0 ? (sp == 0 ? ref0.x : ref0.y) : (sp == 0 ? ref1.x : ref1.y);
+                const float rarg = ANTI ? cr - cum_r : cum_r - cr;   // <= 0 off the diagonal
                 const bool direct = rarg > 80.f;
                 const float rowf = w_exp(direct ? 0.f : rarg);
                 const float4 c0 = *reinterpret_cast<const float4*>(s_colf + hh * WQ + jb);
@@ -1046,17 +1029,18 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
                     f[e] = ANTI ? w_exp(fminf(g.cum[o0 + e] - cum_r, 0.f)) : w_exp(fminf(cum_r - g.cum[o0 + e], 0.f)) * g.dtt[o0 + e];
                 }
                 if (diag) {
+                  const int l0 = blk * 16 + sp * 8;
 #pragma unroll
                   for (int e = 0; e < 8; ++e)
-                    if (ANTI ? (l0 + sp * 8 + e < lane) : (l0 + sp * 8 + e > lane)) f[e] = 0.f;
+                    if (ANTI ? (l0 + e < lane) : (l0 + e > lane)) f[e] = 0.f;
                 }
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                   const __half2 hv = __floats2half2_rn(__uint_as_float(v[sp * 8 + 2 * e]) * f[2 * e], __uint_as_float(v[sp * 8 + 2 * e + 1]) * f[2 * e + 1]);
-                  po[sp * 4 + e] = *reinterpret_cast<const uint32_t*>(&hv);
+                  po[hs * 4 + e] = *reinterpret_cast<const uint32_t*>(&hv);
                 }
               }
-              tmem_st_32x8(gcol + hh * 8, po);
+              tmem_st_32x16(gcol + blk * 16, po);
             }
           }
           tmem_st_wait();
