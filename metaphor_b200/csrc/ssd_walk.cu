@@ -27,6 +27,7 @@
 
 #include <cuda.h>
 #include <mutex>
+#include <type_traits>
 
 namespace {
 
@@ -111,12 +112,6 @@ __device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
   __syncwarp();
   if (lane == 0) mbar_arrive(bar);
 }
-
-// 16 bytes global -> shared by this thread, without a register in between.
-__device__ __forceinline__ void cp_async_16(void* smem_dst, const void* gmem_src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(mp_smem_u32(smem_dst)), "l"(gmem_src) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // The hand-offs of the walk sit on its critical path: poll without a suspend hint first (a suspended warp
 // wakes up hundreds of cycles after the phase completes), then fall back to the bounded, abortable wait.
@@ -619,6 +614,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_con
 // A operand there.  The states lie in TMEM as well: the workers leave D H (fp32) in S's accumulator, S adds to it.
 // ---------------------------------------------------------------------------
 constexpr int WP2_QK = 2 * W_TILE_QK;              // q and k of a chunk, 64 KB; two stages
+constexpr int WP2_HALF = W_TILE_V / 2;             // 32 columns of one head
 constexpr int WP2_OFF_V = 2 * WP2_QK;              // v of both heads
 constexpr int WP2_OFF_H = WP2_OFF_V + 2 * W_TILE_V;
 constexpr int WP2_OFF_VS = WP2_OFF_H + 2 * W_TILE_V;
@@ -627,13 +623,14 @@ constexpr int WP2_SMEM_BYTES = WP2_OFF_TAIL + 2048 + 1024;
 constexpr uint32_t TP_G = 0, TP_S = 128, TP_YD = 256, TP_YO = 384;   // TMEM columns; head h of a pair at + 64 h
 constexpr int WP2_THREADS = 32 * 20;   // warps 0-1 control (2-3 idle), warps 4-19 workers: 640 threads are launched with 96 registers each,
                                        // of which the control warpgroup keeps 64 and the workers take 104 (128 * 64 + 512 * 104 = 640 * 96)
-enum { PB_FULL0 = 0, PB_FULL1, PB_EMPTY0, PB_EMPTY1, PB_VFULL, PB_GFULL, PB_PREADY, PB_VSREADY, PB_YFULL, PB_SFULL, PB_SCAL, PB_COUNT };
+enum { PB_FULL0 = 0, PB_FULL1, PB_EMPTY0, PB_EMPTY1, PB_VFULL, PB_GFULL, PB_PREADY, PB_VSREADY, PB_YFULL, PB_SFULL, PB_SCAL, PB_ZFULL, PB_COUNT };
 
 template <int ANTI, bool DOT, bool RAGGED>
 __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __grid_constant__ CUtensorMap map_q,
                                                                     const __grid_constant__ CUtensorMap map_k,
                                                                     const __grid_constant__ CUtensorMap map_v,
-                                                                    const __grid_constant__ CUtensorMap map_hs, const WalkArgs g) {
+                                                                    const __grid_constant__ CUtensorMap map_hs, const __grid_constant__ CUtensorMap map_z,
+                                                                    const __grid_constant__ CUtensorMap map_out, const WalkArgs g) {
   constexpr bool OUT = ANTI != 0 || !DOT;   // the causal form with row dots has no other output
   extern __shared__ unsigned char walk_smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(walk_smem_raw) + 1023) & ~uintptr_t(1023));
@@ -650,7 +647,7 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
   const int nseq = g.B * hp, cta = blockIdx.x, ncta = gridDim.x;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < PB_COUNT; ++i) mbar_init(bars + i, i == PB_PREADY || i == PB_VSREADY || i == PB_SCAL ? 16 : 1);
+    for (int i = 0; i < PB_COUNT; ++i) mbar_init(bars + i, i == PB_PREADY || i == PB_VSREADY || i == PB_SCAL || i == PB_EMPTY0 || i == PB_EMPTY1 ? 16 : 1);
     *abort = 0;
     mbar_fence_init();
   }
@@ -684,15 +681,26 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
           tma_load_3d(st + W_TILE_QK + WQ * 128, &map_k, grp * WN + 64, row0, b, full);
           return true;
         };
-        ok = load_qk(0);
-        for (int k = 0; ok && k < sg.n; ++k) {
+        auto load_v = [&](int k) {   // Yd of the previous chunk has read the v tiles (the workers scaled them before they wrote its P)
           const int q = qb + k, row0 = (ANTI ? nc - 1 - (sg.p0 + k) : sg.p0 + k) * WQ;
-          // Yd of the previous chunk has read the v tiles (the workers scaled them before they wrote its P)
-          if (q > 0 && !walk_wait(bars + PB_YFULL, (q - 1) & 1, g.status, abort)) { ok = false; break; }
+          if (q > 0 && !walk_wait(bars + PB_YFULL, (q - 1) & 1, g.status, abort)) return false;
           mbar_arrive_expect_tx(bars + PB_VFULL, 2 * W_TILE_V);
           tma_load_3d(sV, &map_v, h * WP, row0, b, bars + PB_VFULL);
           tma_load_3d(sV + W_TILE_V, &map_v, (h + 1) * WP, row0, b, bars + PB_VFULL);
+          return true;
+        };
+        ok = load_qk(0) && load_v(0);
+        for (int k = 0; ok && k < sg.n; ++k) {
+          const int q = qb + k, row0 = (ANTI ? nc - 1 - (sg.p0 + k) : sg.p0 + k) * WQ;
           if (k + 1 < sg.n) ok = load_qk(k + 1);
+          if (DOT && ok) {   // the dot partner's rows into the k tile that S(k) has read
+            ok = walk_wait(bars + PB_SFULL, q & 1, g.status, abort);
+            if (!ok) break;
+            mbar_arrive_expect_tx(bars + PB_ZFULL, 2 * W_TILE_V);
+            for (int t = 0; t < 4; ++t)
+              tma_load_3d(smem + (q & 1) * WP2_QK + W_TILE_QK + t * WP2_HALF, &map_z, h * WP + t * 32, row0, b, bars + PB_ZFULL);
+          }
+          if (ok && k + 1 < sg.n) ok = load_v(k + 1);
         }
         qb += sg.n;
       }
@@ -756,7 +764,6 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
         // the workers rewrite the state tiles once S(k) is complete: the stores must have read them by then
         if (g.hs_out != nullptr && has_state) bulk_wait_read<0>();
         umma_commit(bars + PB_SFULL);
-        umma_commit(bars + PB_EMPTY0 + (q & 1));
       }
       __syncwarp();
     };
@@ -793,9 +800,9 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
     const int ch = wg >> 1, half = wg & 1;     // everything else: 32 columns (`half`) of head `ch` of the pair
     const int r = quarter * 32 + lane;         // row of every 128-row tile
     const uint32_t tl = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
-    const int pitch = g.H * WP;
     unsigned char* hrow = sH + ch * W_TILE_V + r * 128;
-    unsigned char* stg = sVs + ch * W_TILE_V;  // this warp's rows and columns: scaled values of chunk k+1, before that the staging of chunk k's output
+    // this thread's 64 bytes of a [128][32] tile of z or of the output, 64-byte swizzle (two 16-byte pieces a row apart share a bank line)
+    const uint32_t half_row = (ch * 2 + half) * WP2_HALF + r * 64, half_sw = (r >> 1) & 3;
     WalkSeg sg;
     int qb = 0;
     bool alive = true;
@@ -876,15 +883,6 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
           // ---- the state chunk k+1 receives: D H + S of chunk k, complete in S's accumulator -------------------------
           if (!walk_wait(bars + PB_SFULL, par, g.status, abort)) { alive = false; break; }
           tcgen05_fence_after_sync();
-          if (DOT) {   // the dot partner's rows of chunk k into this warp's part of the tile that S(k) has read, whole 64-byte row pieces
-#pragma unroll
-            for (int it = 0; it < 4; ++it) {
-              const int lr = quarter * 32 + it * 8 + (lane >> 2), cc = half * 4 + (lane & 3);
-              int zt = c * WQ + lr;
-              if (RAGGED) zt = min(zt, g.L - 1);   // the output rows beyond the sequence are zero: any row serves as their partner
-              cp_async_16(stg + lr * 128 + ((cc ^ (lr & 7)) << 4), g.z + (static_cast<size_t>(b) * g.L + zt) * pitch + h * WP + cc * 8);
-            }
-          }
           if (more || sg.cout) {
             float hv[32];
             tmem_ld_32x32(tstate, reinterpret_cast<uint32_t*>(hv));
@@ -905,10 +903,8 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
           tcgen05_fence_after_sync();
           const float fo = has_state ? (ANTI ? w_exp(last_cur - cum_cur) : w_exp(cum_cur)) : 0.f;
           const float ro = ANTI ? dt_cur : 1.f;
-          if (DOT) {
-            cp_async_wait_all();
-            __syncwarp();
-          }
+          unsigned char* stage = smem + (q & 1) * WP2_QK;   // q and k of chunk k, read by now: the output goes where q was, z is where k was
+          if (DOT && !walk_wait(bars + PB_ZFULL, par, g.status, abort)) { alive = false; break; }
           float dot = 0.f, dot_state = 0.f;
 #pragma unroll
           for (int p = 0; p < 2; ++p) {
@@ -927,9 +923,9 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
 #pragma unroll
                 for (int e = 0; e < 8; ++e) o[e] = ro * (__uint_as_float(yd[q4 * 8 + e]) + fo * __uint_as_float(yo[q4 * 8 + e]));
               }
-              uint4* slot = reinterpret_cast<uint4*>(stg + r * 128 + (((half * 4 + p * 2 + q4) ^ (r & 7)) << 4));
-              if (DOT) {   // this thread's row of z, before the output overwrites it
-                const uint4 zq = *slot;
+              const uint32_t slot = half_row + ((((p * 2 + q4) ^ half_sw)) << 4);
+              if (DOT) {
+                const uint4 zq = *reinterpret_cast<const uint4*>(stage + W_TILE_QK + slot);
                 const __half2* z2 = reinterpret_cast<const __half2*>(&zq);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
@@ -943,7 +939,7 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
                   }
                 }
               }
-              if (OUT) *slot = walk_pack8(o);
+              if (OUT) *reinterpret_cast<uint4*>(stage + slot) = walk_pack8(o);
             }
           }
           if (DOT) {
@@ -955,18 +951,25 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
             }
             g.dot_out[half * (static_cast<size_t>(g.B) * g.H * LP) + step0 + static_cast<size_t>(c) * WQ] = dot;
           }
-          __syncwarp();
-          if (OUT) {   // whole 64-byte row pieces per store
-#pragma unroll
-            for (int it = 0; it < 4; ++it) {
-              const int lr = quarter * 32 + it * 8 + (lane >> 2), cc = half * 4 + (lane & 3);
-              const uint4 val = *reinterpret_cast<const uint4*>(stg + lr * 128 + ((cc ^ (lr & 7)) << 4));
-              if (!RAGGED || c * WQ + lr < g.L)
-                *reinterpret_cast<uint4*>(g.out + (static_cast<size_t>(b) * g.L + c * WQ + lr) * pitch + h * WP + cc * 8) = val;
-            }
+          if (OUT) {
+            fence_proxy_async_smem();
             __syncwarp();
+            const int row0 = c * WQ + quarter * 32;
+            if (lane == 0 && (!RAGGED || row0 < g.L)) {   // rows beyond the sequence are not written
+              tma_store_3d(&map_out, stage + (ch * 2 + half) * WP2_HALF + quarter * 32 * 64, h * WP + half * 32, row0, b);
+              bulk_commit();
+            }
           }
         }
+        // the stage of chunk k goes back once this warp's output has left it
+        auto release = [&]() {
+          __syncwarp();
+          if (lane == 0) {
+            if (OUT) bulk_wait_read<0>();
+            mbar_arrive(bars + PB_EMPTY0 + (q & 1));
+          }
+        };
+        if (!more) release();
         if (more) {
           // ---- scalars of chunk k+1 into shared memory (every warp is past its P(k): Yd(k) was complete) -------------
           if (half == 0) {
@@ -980,6 +983,7 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
           {
             const __half2 wt2 = __float2half2_rn(ANTI ? w_exp(cum_nxt) : w_exp(last_nxt - cum_nxt) * dt_nxt);
             const unsigned char* src = sV + ch * W_TILE_V + r * 128;
+            unsigned char* dst = sVs + ch * W_TILE_V + r * 128;
 #pragma unroll
             for (int q4 = 0; q4 < 4; ++q4) {
               const int off = ((half * 4 + q4) ^ (r & 7)) << 4;
@@ -987,10 +991,11 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
               __half2* h2 = reinterpret_cast<__half2*>(&v);
 #pragma unroll
               for (int e = 0; e < 4; ++e) h2[e] = __hmul2(h2[e], wt2);
-              *reinterpret_cast<uint4*>(stg + r * 128 + off) = v;
+              *reinterpret_cast<uint4*>(dst + off) = v;
             }
           }
           warp_arrive(bars + PB_VSREADY, lane);
+          if (k >= 0) release();
           // ---- P = G o F of chunk k+1, both heads, in place of the scores -------------------------------------------
           if (!walk_wait(bars + PB_SCAL, parn, g.status, abort)) { alive = false; break; }
           if (!walk_wait(bars + PB_GFULL, parn, g.status, abort)) { alive = false; break; }
@@ -1011,33 +1016,50 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
               const int jb0 = wg * 32 + blk * 16;
               const float2 ref0 = *reinterpret_cast<const float2*>(s_ref + (jb0 >> 3)), ref1 = *reinterpret_cast<const float2*>(s_ref + 16 + (jb0 >> 3));
               tmem_ld_wait();
+              const float cum0 = ch == 0 ? cum_nxt : oth_nxt, cum1 = ch == 0 ? oth_nxt : cum_nxt;
+              const float rarg[4] = {ANTI ? ref0.x - cum0 : cum0 - ref0.x, ANTI ? ref0.y - cum0 : cum0 - ref0.y,   // <= 0 off the diagonal
+                                     ANTI ? ref1.x - cum1 : cum1 - ref1.x, ANTI ? ref1.y - cum1 : cum1 - ref1.y};
+              const float rmax = fmaxf(fmaxf(rarg[0], rarg[1]), fmaxf(rarg[2], rarg[3]));
+              if (!__any_sync(0xffffffffu, rmax > 80.f)) {
 #pragma unroll
-              for (int hs = 0; hs < 4; ++hs) {   // head of the pair, 8 steps
-                const int hh = hs >> 1, sp = hs & 1, jb = jb0 + sp * 8;
-                const float cum_r = hh == ch ? cum_nxt : oth_nxt;
-                const float cr = hh == 0 ? (sp == 0 ? ref0.x : ref0.y) : (sp == 0 ? ref1.x : ref1.y);
-                const float rarg = ANTI ? cr - cum_r : cum_r - cr;   // <= 0 off the diagonal
-                const bool direct = rarg > 80.f;
-                const float rowf = w_exp(direct ? 0.f : rarg);
-                const float4 c0 = *reinterpret_cast<const float4*>(s_colf + hh * WQ + jb);
-                const float4 c1 = *reinterpret_cast<const float4*>(s_colf + hh * WQ + jb + 4);
-                float f[8] = {c0.x * rowf, c0.y * rowf, c0.z * rowf, c0.w * rowf, c1.x * rowf, c1.y * rowf, c1.z * rowf, c1.w * rowf};
-                if (direct) {   // rare: the step factors from global memory
-                  const size_t o0 = (hh == ch ? step0 : other0) - r + static_cast<size_t>(ANTI ? c_first - k - 1 : c_first + k + 1) * WQ + jb;
+                for (int hs = 0; hs < 4; ++hs) {   // head of the pair, 8 steps; no branch in here: the loads and exponentials of all four overlap
+                  const int hh = hs >> 1, sp = hs & 1;
+                  const float rowf = w_exp(rarg[hs]);
+                  const float4 c0 = *reinterpret_cast<const float4*>(s_colf + hh * WQ + jb0 + sp * 8);
+                  const float4 c1 = *reinterpret_cast<const float4*>(s_colf + hh * WQ + jb0 + sp * 8 + 4);
+                  const float f[8] = {c0.x * rowf, c0.y * rowf, c0.z * rowf, c0.w * rowf, c1.x * rowf, c1.y * rowf, c1.z * rowf, c1.w * rowf};
 #pragma unroll
-                  for (int e = 0; e < 8; ++e)
-                    f[e] = ANTI ? w_exp(fminf(g.cum[o0 + e] - cum_r, 0.f)) : w_exp(fminf(cum_r - g.cum[o0 + e], 0.f)) * g.dtt[o0 + e];
+                  for (int e = 0; e < 4; ++e) {
+                    const __half2 hv = __floats2half2_rn(__uint_as_float(v[sp * 8 + 2 * e]) * f[2 * e], __uint_as_float(v[sp * 8 + 2 * e + 1]) * f[2 * e + 1]);
+                    po[hs * 4 + e] = *reinterpret_cast<const uint32_t*>(&hv);
+                  }
                 }
-                if (diag) {
-                  const int l0 = blk * 16 + sp * 8;
+              } else {   // a row factor that does not fit: the step factors from global memory
 #pragma unroll
-                  for (int e = 0; e < 8; ++e)
-                    if (ANTI ? (l0 + e < lane) : (l0 + e > lane)) f[e] = 0.f;
+                for (int hh = 0; hh < 2; ++hh) {
+                  const float cum_r = hh == 0 ? cum0 : cum1;
+                  const size_t o0 = (hh == ch ? step0 : other0) - r + static_cast<size_t>(ANTI ? c_first - k - 1 : c_first + k + 1) * WQ + jb0;
+#pragma unroll
+                  for (int e = 0; e < 8; ++e) {
+                    float f[2];
+#pragma unroll
+                    for (int t = 0; t < 2; ++t)
+                      f[t] = ANTI ? w_exp(fminf(g.cum[o0 + 2 * e + t] - cum_r, 0.f)) : w_exp(fminf(cum_r - g.cum[o0 + 2 * e + t], 0.f)) * g.dtt[o0 + 2 * e + t];
+                    const __half2 hv = __floats2half2_rn(__uint_as_float(v[2 * e]) * f[0], __uint_as_float(v[2 * e + 1]) * f[1]);
+                    po[hh * 8 + e] = *reinterpret_cast<const uint32_t*>(&hv);
+                    asm volatile("" ::: "memory");   // one element's loads at a time: this path is rare and must not cost registers
+                  }
                 }
+              }
+              if (diag) {   // word e of a head holds steps 2e and 2e + 1 of the block
+                int lr = lane - blk * 16;
+                asm volatile("" : "+r"(lr));   // the masks are made here: hoisted out of the walk's loop they take sixteen registers
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  const __half2 hv = __floats2half2_rn(__uint_as_float(v[sp * 8 + 2 * e]) * f[2 * e], __uint_as_float(v[sp * 8 + 2 * e + 1]) * f[2 * e + 1]);
-                  po[hs * 4 + e] = *reinterpret_cast<const uint32_t*>(&hv);
+                for (int e = 0; e < 8; ++e) {
+                  const uint32_t keep = ANTI ? (2 * e >= lr ? 0xffffffffu : (2 * e + 1 >= lr ? 0xffff0000u : 0u))
+                                             : (2 * e + 1 <= lr ? 0xffffffffu : (2 * e <= lr ? 0xffffu : 0u));
+                  po[e] &= keep;
+                  po[8 + e] &= keep;
                 }
               }
               tmem_st_32x16(gcol + blk * 16, po);
@@ -1049,6 +1071,7 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
       }
       qb += n;
     }
+    if (OUT && lane == 0) bulk_wait_all<0>();
   }
   tcgen05_fence_before_sync();
   __syncthreads();
@@ -1585,16 +1608,16 @@ CUtensorMap walk_map(const void* base, size_t rows, size_t cols) {
   return m;
 }
 
-// r16 tensor [batch, rows, cols] (row-major), box {64 columns, 128 rows, 1}, 128-byte swizzle: rows past the end of a batch
+// r16 tensor [batch, rows, cols] (row-major), box {64 columns, 128 rows, 1}, 128-byte swizzle (64-byte with 32 columns): rows past the end of a batch
 // entry read as zeros and are not written.
-CUtensorMap walk_map3(const void* base, size_t batch, size_t rows, size_t cols) {
+CUtensorMap walk_map3(const void* base, size_t batch, size_t rows, size_t cols, uint32_t box_cols = 64, uint32_t box_rows = 128) {
   CUtensorMap m;
   const cuuint64_t dims[3] = {cols, rows, batch};
   const cuuint64_t strides[2] = {cols * sizeof(__half), rows * cols * sizeof(__half)};
-  const cuuint32_t box[3] = {64, 128, 1};
+  const cuuint32_t box[3] = {box_cols, box_rows, 1};
   const cuuint32_t es[3] = {1, 1, 1};
   MP_CU_CHECK(walk_encode_tiled()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box, es,
-                                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                  CU_TENSOR_MAP_INTERLEAVE_NONE, box_cols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE));
   return m;
 }
@@ -1677,22 +1700,31 @@ void mp_ssd_walk(int anti, const __half* q, const __half* k, const __half* v, co
   const CUtensorMap mq = walk_map3(q, B, L, static_cast<size_t>(G) * WN), mk = walk_map3(k, B, L, static_cast<size_t>(G) * WN);
   const CUtensorMap mv = walk_map3(v, B, L, static_cast<size_t>(H) * WP);
   const CUtensorMap mh = hs_out != nullptr ? walk_map(hs_out, static_cast<size_t>(B) * H * g.nc * WN, WP) : mv;
-  auto launch = [&](auto kernel, int smem) {
-    MP_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    MpLaunch(grid, pairs ? WP2_THREADS : W_THREADS, smem, st)(kernel, mq, mk, mv, mh, g);
+  auto launch = [&](auto kernel, auto pair_kernel) {
+    if (pairs) {
+      const CUtensorMap mz = z != nullptr ? walk_map3(z, B, L, static_cast<size_t>(H) * WP, 32, 128) : mv;
+      const CUtensorMap mo = out != nullptr ? walk_map3(out, B, L, static_cast<size_t>(H) * WP, 32, 32) : mv;
+      MP_CUDA_CHECK(cudaFuncSetAttribute(pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WP2_SMEM_BYTES));
+      MpLaunch(grid, WP2_THREADS, WP2_SMEM_BYTES, st)(pair_kernel, mq, mk, mv, mh, mz, mo, g);
+    } else {
+      MP_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, W_SMEM_BYTES));
+      MpLaunch(grid, W_THREADS, W_SMEM_BYTES, st)(kernel, mq, mk, mv, mh, g);
+    }
   };
   const bool dot = z != nullptr && dot_out != nullptr;
   if (!dot) { g.z = nullptr; g.dot_out = nullptr; }
   if (anti && !dot) MP_FATAL("ssd walk: the anti-causal form comes with its row dots");
-#define MP_WALK_FORM(A, D)                                                                                                          \
-  do {                                                                                                                              \
-    if (pairs) { if (L % WQ != 0) launch(ssd_walk_pair_kernel<A, D, true>, WP2_SMEM_BYTES); else launch(ssd_walk_pair_kernel<A, D, false>, WP2_SMEM_BYTES); } \
-    else { if (L % WQ != 0) launch(ssd_walk_kernel<A, D, true>, W_SMEM_BYTES); else launch(ssd_walk_kernel<A, D, false>, W_SMEM_BYTES); }                   \
-  } while (0)
-  if (anti) MP_WALK_FORM(1, true);
-  else if (dot) MP_WALK_FORM(0, true);
-  else MP_WALK_FORM(0, false);
-#undef MP_WALK_FORM
+  const bool ragged = L % WQ != 0;
+  auto form = [&](auto A, auto D) {
+    constexpr int a = decltype(A)::value;
+    constexpr bool d = decltype(D)::value;
+    if (ragged) launch(ssd_walk_kernel<a, d, true>, ssd_walk_pair_kernel<a, d, true>);
+    else launch(ssd_walk_kernel<a, d, false>, ssd_walk_pair_kernel<a, d, false>);
+  };
+  using std::integral_constant;
+  if (anti) form(integral_constant<int, 1>{}, std::true_type{});
+  else if (dot) form(integral_constant<int, 0>{}, std::true_type{});
+  else form(integral_constant<int, 0>{}, std::false_type{});
   MP_LAUNCH_CHECK();
 }
 
