@@ -809,10 +809,9 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
     for (int si = 0; alive && walk_segment(cta, ncta, nseq, nc, si, sg); ++si) {
       const int n = sg.n;
       const int h = 2 * (sg.seq % hp) + ch, b = sg.seq / hp;
-      const size_t bh = static_cast<size_t>(b) * g.H + h;
-      const size_t LP = static_cast<size_t>(nc) * WQ;
+      const uint32_t bh = static_cast<uint32_t>(b) * g.H + h, LP = static_cast<uint32_t>(nc) * WQ;   // B H LP fits 31 bits: see mp_ssd_walk
       // this thread's step in the first chunk of the walk, in the arrays per step of its head and of the other one
-      const size_t step0 = bh * LP + r, other0 = (ch == 0 ? bh + 1 : bh - 1) * LP + r;
+      const uint32_t step0 = bh * LP + r, other0 = (ch == 0 ? bh + 1 : bh - 1) * LP + r;
       const uint32_t tstate = tl + TP_S + ch * 64 + half * 32;
       const int c_first = ANTI ? nc - 1 - sg.p0 : sg.p0;
       // the 32 columns of the state a chunk receives: an r16 copy for its q H, and D times it (D: the chunk's decay) for its S to add to
@@ -844,8 +843,8 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
         }
         __syncwarp();
         if (*abort != 0) { alive = false; break; }
-        const float4* src = reinterpret_cast<const float4*>(g.carry + (bh * WN + r) * WP + half * 32);
-        const float D = w_exp(g.cum[step0 - r + static_cast<size_t>(c_first) * WQ + WQ - 1]);
+        const float4* src = reinterpret_cast<const float4*>(g.carry + (static_cast<size_t>(bh) * WN + r) * WP + half * 32);
+        const float D = w_exp(g.cum[step0 - r + static_cast<uint32_t>(c_first) * WQ + WQ - 1]);
         float hv[32];
 #pragma unroll
         for (int q4 = 0; q4 < 8; ++q4) {
@@ -855,20 +854,25 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
         store_state(hv, D);   // (the tiles are free: their last readers were complete before the previous segment's last S was)
       } else {
         if (g.hs_out != nullptr) {   // the first chunk of a sequence's walk receives nothing
-          uint4* dst = reinterpret_cast<uint4*>(g.hs_out + ((bh * nc + c_first) * WN + r) * WP + half * 32);
+          uint4* dst = reinterpret_cast<uint4*>(g.hs_out + ((static_cast<size_t>(bh) * nc + c_first) * WN + r) * WP + half * 32);
 #pragma unroll
           for (int q4 = 0; q4 < 4; ++q4) dst[q4] = make_uint4(0u, 0u, 0u, 0u);
         }
       }
       // scalars of the chunk in hand (cur) and of the one after it (nxt), which are requested a whole chunk before they are used
       float cum_cur = 0.f, dt_cur = 0.f, last_cur = 0.f;
+      // the chunk's decay, which the next state needs at once, is brought into L1 two chunks before
       float cum_nxt, dt_nxt, colf_nxt, oth_nxt, last_nxt;
       auto fetch = [&](int k) {
-        const size_t i = static_cast<size_t>(ANTI ? c_first - k : c_first + k) * WQ;
+        const uint32_t i = static_cast<uint32_t>(ANTI ? c_first - k : c_first + k) * WQ;
         cum_nxt = g.cum[step0 + i]; dt_nxt = g.dtt[step0 + i]; colf_nxt = g.colf[step0 + i]; oth_nxt = g.cum[other0 + i];
         last_nxt = g.cum[step0 - r + i + WQ - 1];
       };
+      auto prefetch_last = [&](int k) {
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(g.cum + (step0 - r + static_cast<uint32_t>(ANTI ? c_first - k : c_first + k) * WQ + WQ - 1)));
+      };
       fetch(0);
+      if (n > 1) prefetch_last(1);
 
 #pragma unroll 1
       for (int k = -1; k < n; ++k) {   // finishes chunk k, prepares chunk k+1; k = -1 only prepares
@@ -880,6 +884,7 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
           const bool has_state = k > 0 || sg.cin != 0;
           cum_cur = cum_nxt; dt_cur = dt_nxt; last_cur = last_nxt;
           if (more) fetch(k + 1);
+          if (k + 2 < n) prefetch_last(k + 2);
           // ---- the state chunk k+1 receives: D H + S of chunk k, complete in S's accumulator -------------------------
           if (!walk_wait(bars + PB_SFULL, par, g.status, abort)) { alive = false; break; }
           tcgen05_fence_after_sync();
@@ -890,7 +895,7 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
             if (more) {
               store_state(hv, w_exp(last_nxt));
             } else {   // the first part of the sequences ends here: their states go to the CTA that walks the rest
-              float4* dst = reinterpret_cast<float4*>(g.carry + (bh * WN + r) * WP + half * 32);
+              float4* dst = reinterpret_cast<float4*>(g.carry + (static_cast<size_t>(bh) * WN + r) * WP + half * 32);
 #pragma unroll
               for (int q4 = 0; q4 < 8; ++q4) __stcg(dst + q4, make_float4(hv[q4 * 4], hv[q4 * 4 + 1], hv[q4 * 4 + 2], hv[q4 * 4 + 3]));
               __threadfence();
@@ -947,9 +952,9 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
               dot_state *= fo;
               dot += dot_state;
               dot_state = warp_reduce<SumOp>(dot_state);
-              if (lane == 0) g.state_dot[(bh * nc + c) * 16 + quarter * 2 + half] = dot_state;
+              if (lane == 0) g.state_dot[(static_cast<size_t>(bh) * nc + c) * 16 + quarter * 2 + half] = dot_state;
             }
-            g.dot_out[half * (static_cast<size_t>(g.B) * g.H * LP) + step0 + static_cast<size_t>(c) * WQ] = dot;
+            g.dot_out[half * (static_cast<size_t>(g.B) * g.H * LP) + step0 + static_cast<uint32_t>(c) * WQ] = dot;
           }
           if (OUT) {
             fence_proxy_async_smem();
@@ -1038,7 +1043,7 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
 #pragma unroll
                 for (int hh = 0; hh < 2; ++hh) {
                   const float cum_r = hh == 0 ? cum0 : cum1;
-                  const size_t o0 = (hh == ch ? step0 : other0) - r + static_cast<size_t>(ANTI ? c_first - k - 1 : c_first + k + 1) * WQ + jb0;
+                  const uint32_t o0 = (hh == ch ? step0 : other0) - r + static_cast<uint32_t>(ANTI ? c_first - k - 1 : c_first + k + 1) * WQ + jb0;
 #pragma unroll
                   for (int e = 0; e < 8; ++e) {
                     float f[2];
@@ -1691,10 +1696,11 @@ void mp_ssd_walk(int anti, const __half* q, const __half* k, const __half* v, co
   // One CTA per SM slot it may use, every CTA the same number of chunks; never more CTAs than sequences, so that a CTA's
   // range is at least one sequence long (see walk_segment).  MP_SSD_WALK_PER_SEQUENCE: one CTA per sequence, no hand-off.
   // Two heads at a time where their group has an even number of heads and there are enough sequences: a chunk of a pair takes about
-  // 1.4 times as long as a chunk of one head, which pays unless CTAs are left without a sequence.
+  // 1.2 times as long as a chunk of one head, which pays unless CTAs are left without a sequence.
   const bool bounded = max_ctas > 0 && getenv("MP_SSD_WALK_PER_SEQUENCE") == nullptr;
   auto load = [&](int seqs) { return bounded && seqs > max_ctas ? static_cast<double>(seqs) / max_ctas : 1.0; };   // sequences per CTA
-  const bool pairs = (H / G) % 2 == 0 && 1.4 * load(B * H / 2) < load(B * H) && getenv("MP_SSD_WALK_NO_PAIRS") == nullptr;
+  const bool pairs = (H / G) % 2 == 0 && static_cast<size_t>(B) * H * g.nc * WQ < (size_t{1} << 31) && 1.2 * load(B * H / 2) < load(B * H) &&
+                     getenv("MP_SSD_WALK_NO_PAIRS") == nullptr;
   int grid = pairs ? B * H / 2 : B * H;
   if (bounded && max_ctas < grid) grid = max_ctas;
   const CUtensorMap mq = walk_map3(q, B, L, static_cast<size_t>(G) * WN), mk = walk_map3(k, B, L, static_cast<size_t>(G) * WN);
