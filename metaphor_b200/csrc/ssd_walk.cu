@@ -424,37 +424,48 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_con
           // diagonal sub-piece) the exponent is taken per element.
           const bool diag = pc == quarter;
           tmem_ld_wait();
+          float rarg[4];   // <= 0 off the diagonal
 #pragma unroll
           for (int sp = 0; sp < 4; ++sp) {
-            const int jb = j0 + sp * 8;
-            const float cref = s_cum[ANTI ? jb : jb + 7];
-            const float rarg = ANTI ? cref - cum_nxt : cum_nxt - cref;   // <= 0 off the diagonal
-            const bool direct = rarg > 80.f;
-            const float rowf = w_exp(direct ? 0.f : rarg);
-            const float4 c0 = *reinterpret_cast<const float4*>(s_colf + jb);
-            const float4 c1 = *reinterpret_cast<const float4*>(s_colf + jb + 4);
-            float f[8] = {c0.x * rowf, c0.y * rowf, c0.z * rowf, c0.w * rowf, c1.x * rowf, c1.y * rowf, c1.z * rowf, c1.w * rowf};
-            if (direct) {
+            const float cref = s_cum[j0 + sp * 8 + (ANTI ? 0 : 7)];
+            rarg[sp] = ANTI ? cref - cum_nxt : cum_nxt - cref;
+          }
+          uint32_t po[16];
+          if (!__any_sync(0xffffffffu, fmaxf(fmaxf(rarg[0], rarg[1]), fmaxf(rarg[2], rarg[3])) > 80.f)) {
 #pragma unroll
-              for (int e = 0; e < 8; ++e) {
-                const float cj = s_cum[jb + e];
-                f[e] = ANTI ? w_exp(fminf(cj - cum_nxt, 0.f)) : w_exp(fminf(cum_nxt - cj, 0.f)) * s_dt[jb + e];
+            for (int sp = 0; sp < 4; ++sp) {   // no branch in here: the exponentials and loads of all four overlap
+              const float rowf = w_exp(rarg[sp]);
+              const float4 c0 = *reinterpret_cast<const float4*>(s_colf + j0 + sp * 8);
+              const float4 c1 = *reinterpret_cast<const float4*>(s_colf + j0 + sp * 8 + 4);
+              const float f[8] = {c0.x * rowf, c0.y * rowf, c0.z * rowf, c0.w * rowf, c1.x * rowf, c1.y * rowf, c1.z * rowf, c1.w * rowf};
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const __half2 hv = __floats2half2_rn(__uint_as_float(v[sp * 8 + 2 * e]) * f[2 * e], __uint_as_float(v[sp * 8 + 2 * e + 1]) * f[2 * e + 1]);
+                po[sp * 4 + e] = *reinterpret_cast<const uint32_t*>(&hv);
               }
             }
-            if (diag) {
+          } else {
 #pragma unroll
-              for (int e = 0; e < 8; ++e)
-                if (ANTI ? (sp * 8 + e < lane) : (sp * 8 + e > lane)) f[e] = 0.f;
-            }
-            uint4 o;
-            uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
+            for (int e = 0; e < 16; ++e) {
+              float f[2];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const __half2 hv = __floats2half2_rn(__uint_as_float(v[sp * 8 + 2 * e]) * f[2 * e], __uint_as_float(v[sp * 8 + 2 * e + 1]) * f[2 * e + 1]);
-              ow[e] = *reinterpret_cast<const uint32_t*>(&hv);
+              for (int t = 0; t < 2; ++t) {
+                const float cj = s_cum[j0 + 2 * e + t];
+                f[t] = ANTI ? w_exp(fminf(cj - cum_nxt, 0.f)) : w_exp(fminf(cum_nxt - cj, 0.f)) * s_dt[j0 + 2 * e + t];
+              }
+              const __half2 hv = __floats2half2_rn(__uint_as_float(v[2 * e]) * f[0], __uint_as_float(v[2 * e + 1]) * f[1]);
+              po[e] = *reinterpret_cast<const uint32_t*>(&hv);
             }
-            *reinterpret_cast<uint4*>(prow + (((pp * 4 + sp) ^ (r & 7)) << 4)) = o;
           }
+          if (diag) {   // word e holds steps 2e and 2e + 1 of the piece
+#pragma unroll
+            for (int e = 0; e < 16; ++e)
+              po[e] &= ANTI ? (2 * e >= lane ? 0xffffffffu : (2 * e + 1 >= lane ? 0xffff0000u : 0u))
+                            : (2 * e + 1 <= lane ? 0xffffffffu : (2 * e <= lane ? 0xffffu : 0u));
+          }
+#pragma unroll
+          for (int q4 = 0; q4 < 4; ++q4)
+            *reinterpret_cast<uint4*>(prow + (((pp * 4 + q4) ^ (r & 7)) << 4)) = make_uint4(po[q4 * 4], po[q4 * 4 + 1], po[q4 * 4 + 2], po[q4 * 4 + 3]);
         }
         warp_arrive(bars + B_PREADY, lane);
       }
@@ -1289,22 +1300,27 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_group_grads_kernel(const __g
         tmem_ld_32x32(tl + GT_SC + s * 128 + j0, v);
         const bool diag = pc == quarter;
         tmem_ld_wait();
+        // Factors relative to the last column of each 8-column sub-piece (see the walk kernel); without a branch per sub-piece the
+        // exponentials and shared-memory loads of all four overlap.
+        const int last_col = diag ? lane : 31;
+        float rarg[4];
 #pragma unroll
-        for (int sp = 0; sp < 4; ++sp) {      // factors relative to the last column of each 8-column sub-piece (see the walk kernel)
-          const int jb = j0 + sp * 8;
-          const float rarg = cum_r - cumb[jb + 7];
-          const bool direct = rarg > 80.f;
-          const float rowf = w_exp(direct ? 0.f : rarg);
-          const float4 c0 = *reinterpret_cast<const float4*>(colfb + jb);
-          const float4 c1 = *reinterpret_cast<const float4*>(colfb + jb + 4);
-          float f[8] = {c0.x * rowf, c0.y * rowf, c0.z * rowf, c0.w * rowf, c1.x * rowf, c1.y * rowf, c1.z * rowf, c1.w * rowf};
-          if (direct) {
+        for (int sp = 0; sp < 4; ++sp) rarg[sp] = cum_r - cumb[j0 + sp * 8 + 7];
+        if (!__any_sync(0xffffffffu, fmaxf(fmaxf(rarg[0], rarg[1]), fmaxf(rarg[2], rarg[3])) > 80.f)) {
 #pragma unroll
-            for (int e = 0; e < 8; ++e) f[e] = w_exp(fminf(cum_r - cumb[jb + e], 0.f)) * dtb[jb + e];
+          for (int sp = 0; sp < 4; ++sp) {
+            const float rowf = w_exp(rarg[sp]);
+            const float4 c0 = *reinterpret_cast<const float4*>(colfb + j0 + sp * 8);
+            const float4 c1 = *reinterpret_cast<const float4*>(colfb + j0 + sp * 8 + 4);
+            const float f[8] = {c0.x * rowf, c0.y * rowf, c0.z * rowf, c0.w * rowf, c1.x * rowf, c1.y * rowf, c1.z * rowf, c1.w * rowf};
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              if (sp * 8 + e <= last_col) acc[pp * 32 + sp * 8 + e] += __uint_as_float(v[sp * 8 + e]) * f[e];
           }
+        } else {
 #pragma unroll
-          for (int e = 0; e < 8; ++e)
-            if (!diag || sp * 8 + e <= lane) acc[pp * 32 + sp * 8 + e] += __uint_as_float(v[sp * 8 + e]) * f[e];
+          for (int e = 0; e < 32; ++e)
+            if (e <= last_col) acc[pp * 32 + e] += __uint_as_float(v[e]) * (w_exp(fminf(cum_r - cumb[j0 + e], 0.f)) * dtb[j0 + e]);
         }
       }
       // ---- row factors into the operand tiles, in place (the score MMA has read them) ----
