@@ -212,3 +212,30 @@ def test_ssd_on_ragged_lengths(mp, stream, orc, dims):
         got = host(got)
         assert np.isnan(got[want.size:]).all(), f"{name} written past its end {dims}"
         assert_close(got[:want.size].reshape(want.shape), want.astype(got.dtype), TOL, f"{name} {dims}")
+
+
+@pytest.mark.parametrize("dims,shift", [
+    # (batch, seqlen, heads, headdim, dstate, groups, chunk), shift of the raw step sizes.  The walk takes two heads of a group at a time
+    # where there are enough sequences: uncut in the forward and cut in the reverse, cut in both (two groups), an odd number of
+    # heads per group beside it (one head at a time), and steps that decay by more than e^-80 in eight, whose mask is made step by step
+    ((12, 300, 16, 64, 128, 1, 128), 0.0), ((20, 256, 32, 64, 128, 2, 128), 0.0), ((20, 200, 15, 64, 128, 1, 128), 0.0),
+    ((12, 200, 16, 64, 128, 1, 128), 7.0), ((20, 160, 15, 64, 128, 1, 128), 7.0)])
+def test_ssd_heads_in_pairs(mp, stream, orc, dims, shift):
+    import torch
+    nb, L, H, P, N, G, Q = dims
+    x, dt, A, Bm, Cm, gy = make_inputs(12, nb, L, H, P, N, G)
+    if shift:
+        dt = (dt + shift * np.random.default_rng(13).uniform(size=dt.shape)).astype(np.float32)
+    f64 = lambda a: np.ascontiguousarray(a.astype(np.float64))
+    args = [dev(a) for a in (x, dt, A, Bm, Cm)]
+    y, gx, gdt, gA, gB, gC = (dev(np.full(a.shape, np.nan, a.dtype)) for a in (x, x, dt, A, Bm, Cm))
+    n = max(mp.lib().mpSsdScanScratchBytes(*dims, 0), mp.lib().mpSsdScanScratchBytes(*dims, 1))
+    scratch = torch.full((n,), 255, dtype=torch.uint8, device="cuda")
+    torch.cuda.current_stream().synchronize()
+    mp.launch("ssd_scan", torch.float16, *args, y, scratch, *dims, stream)
+    mp.launch("ssd_scan_reverse", torch.float16, *args, dev(gy), gx, gdt, gA, gB, gC, scratch, *dims, stream)
+    stream.sync()
+    assert stream.status() == 0
+    ref = (orc.ssd_forward(f64(x), f64(dt), f64(A), f64(Bm), f64(Cm)),) + tuple(orc.ssd_reverse(f64(x), f64(dt), f64(A), f64(Bm), f64(Cm), f64(gy)))
+    for got, want, name in zip((y, gx, gdt, gA, gB, gC), ref, ("y", "gx", "gdt", "gA", "gB", "gC")):
+        assert_close(host(got), want.astype(host(got).dtype), TOL, f"{name} {dims} {shift}")
