@@ -147,8 +147,8 @@ MP_DECL3(linear_ij_jk_ik_ik, const void* a, const void* b, const void* r, double
  * scratch: mpSsdScanScratchBytes(..., reverse) bytes owned by the caller (the reverse holds four
  * independent sets of intermediates, its operator instances run side by side on helper streams that
  * the library forks from and joins back into the caller's stream).
- * Two implementations: a tensor-core path (r16 with dstate = 128, headdim 64 or 128, chunk 128 or 256,
- * seqlen a multiple of chunk) and a sequential-recurrence path for every other shape of r16 and for r32 /
+ * Two implementations: a tensor-core path (r16 with dstate = 128; headdim 64 with any seqlen from 32 on, or headdim 128 with
+ * chunk 128 or 256 and seqlen a multiple of chunk) and a sequential-recurrence path for every other shape of r16 and for r32 /
  * r64 storage (dt, A, gdt, gA then have the storage type; `chunk` is ignored).  Scratch: r16 ->
  * mpSsdScanScratchBytes (either path), r32 / r64 -> mpSsdScanGenericScratchBytes(dtype_key, ...); the
  * forward of the sequential path needs none. */
