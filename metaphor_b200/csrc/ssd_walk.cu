@@ -1463,15 +1463,35 @@ __global__ void __launch_bounds__(WS_THREADS) ssd_walk_cumsum_kernel(const float
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
     d[e] = s_dt[lane * 4 + e][w];
-    v[e] = d[e] * a + (e > 0 ? v[e - 1] : 0.f);
+    v[e] = __fmul_rn(d[e], a);
   }
-  float incl = v[3];
+  // Inclusive sums of 32 steps (eight lanes) by doubling offsets, then the totals of the 32-step groups before: the order in which one
+  // thread per step would add them.
+  const int l8 = lane & 7;
+  {
+    const float p3 = __shfl_up_sync(0xffffffffu, v[3], 1);
+    const float w0 = l8 >= 1 ? v[0] + p3 : v[0], w1 = v[1] + v[0], w2 = v[2] + v[1], w3 = v[3] + v[2];
+    v[0] = w0; v[1] = w1; v[2] = w2; v[3] = w3;
+  }
+  {
+    const float p2 = __shfl_up_sync(0xffffffffu, v[2], 1), p3 = __shfl_up_sync(0xffffffffu, v[3], 1);
+    const float w2 = v[2] + v[0], w3 = v[3] + v[1];
+    if (l8 >= 1) { v[0] += p2; v[1] += p3; }
+    v[2] = w2; v[3] = w3;
+  }
 #pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    const float up = __shfl_up_sync(0xffffffffu, incl, off);
-    if (lane >= off) incl += up;
+  for (int off = 1; off < 8; off <<= 1)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float up = __shfl_up_sync(0xffffffffu, v[e], off);
+      if (l8 >= off) v[e] += up;
+    }
+  float base = 0.f;
+#pragma unroll
+  for (int g = 0; g < 3; ++g) {
+    const float tot = __shfl_sync(0xffffffffu, v[3], g * 8 + 7);
+    if (g < (lane >> 3)) base += tot;
   }
-  const float base = incl - v[3];
 #pragma unroll
   for (int e = 0; e < 4; ++e) v[e] += base;
   const float c_hi = __shfl_sync(0xffffffffu, v[3], lane | 1), c_lo = __shfl_sync(0xffffffffu, v[0], lane & ~1);
