@@ -152,6 +152,13 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
 
 // 32 lanes x 32 consecutive 32-bit columns -> 32 registers per thread (thread i
 // of the warp reads lane i of the warp's TMEM quarter).
+__device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t* v) {   // 8 columns
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+      : "r"(taddr)
+      : "memory");
+}
 __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t* v) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "

@@ -640,7 +640,7 @@ constexpr int WP2_OFF_H = WP2_OFF_V + 2 * W_TILE_V;
 constexpr int WP2_OFF_VS = WP2_OFF_H + 2 * W_TILE_V;
 constexpr int WP2_OFF_TAIL = WP2_OFF_VS + 2 * W_TILE_V;   // 229376
 constexpr int WP2_SMEM_BYTES = WP2_OFF_TAIL + 2048 + 1024;
-constexpr uint32_t TP_G = 0, TP_S = 128, TP_YD = 256, TP_YO = 384;   // TMEM columns; head h of a pair at + 64 h
+constexpr uint32_t TP_G = 0, TP_S = 128, TP_YD = 128, TP_H = 256, TP_YO = 384;   // TMEM columns; head h of a pair at + 64 h
 constexpr int WP2_THREADS = 32 * 20;   // warps 0-1 control (2-3 idle), warps 4-19 workers: 640 threads are launched with 96 registers each,
                                        // of which the control warpgroup keeps 64 and the workers take 104 (128 * 64 + 512 * 104 = 640 * 96)
 enum { PB_FULL0 = 0, PB_FULL1, PB_EMPTY0, PB_EMPTY1, PB_VFULL, PB_GFULL, PB_PREADY, PB_VSREADY, PB_YFULL, PB_SFULL, PB_SCAL, PB_ZFULL, PB_COUNT };
@@ -780,7 +780,7 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
           for (int ks = 0; ks < 8; ++ks) umma<false>(tmem + TP_YO, dq + kslice(ks), dh + ks * ROWS_U, id_yo, ks != 0 ? 1u : 0u);
         }
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) umma<false>(tmem + TP_S, dkt + ks * ROWS_U, dvs + ks * ROWS_U, id_s, (has_state || ks != 0) ? 1u : 0u);
+        for (int ks = 0; ks < 8; ++ks) umma<false>(tmem + TP_S, dkt + ks * ROWS_U, dvs + ks * ROWS_U, id_s, ks != 0 ? 1u : 0u);
         // the workers rewrite the state tiles once S(k) is complete: the stores must have read them by then
         if (g.hs_out != nullptr && has_state) bulk_wait_read<0>();
         umma_commit(bars + PB_SFULL);
@@ -832,14 +832,12 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
       const uint32_t bh = static_cast<uint32_t>(b) * g.H + h, LP = static_cast<uint32_t>(nc) * WQ;   // B H LP fits 31 bits: see mp_ssd_walk
       // this thread's step in the first chunk of the walk, in the arrays per step of its head and of the other one
       const uint32_t step0 = bh * LP + r, other0 = (ch == 0 ? bh + 1 : bh - 1) * LP + r;
-      const uint32_t tstate = tl + TP_S + ch * 64 + half * 32;
+      const uint32_t tstate = tl + TP_H + ch * 64 + half * 32;
       const int c_first = ANTI ? nc - 1 - sg.p0 : sg.p0;
-      // the 32 columns of the state a chunk receives: an r16 copy for its q H, and D times it (D: the chunk's decay) for its S to add to
-      auto store_state = [&](float* hv, float D) {
+      // the 32 columns of the state a chunk receives: fp32 in TMEM, and an r16 copy for its q H
+      auto store_state = [&](const float* hv) {
 #pragma unroll
         for (int q4 = 0; q4 < 4; ++q4) *reinterpret_cast<uint4*>(hrow + (((half * 4 + q4) ^ (r & 7)) << 4)) = walk_pack8(hv + q4 * 8);
-#pragma unroll
-        for (int e = 0; e < 32; ++e) hv[e] *= D;
         tmem_st_32x32(tstate, reinterpret_cast<const uint32_t*>(hv));
         tmem_st_wait();
       };
@@ -864,14 +862,13 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
         __syncwarp();
         if (*abort != 0) { alive = false; break; }
         const float4* src = reinterpret_cast<const float4*>(g.carry + (static_cast<size_t>(bh) * WN + r) * WP + half * 32);
-        const float D = w_exp(g.cum[step0 - r + static_cast<uint32_t>(c_first) * WQ + WQ - 1]);
         float hv[32];
 #pragma unroll
         for (int q4 = 0; q4 < 8; ++q4) {
           const float4 v4 = __ldcg(src + q4);
           hv[q4 * 4] = v4.x; hv[q4 * 4 + 1] = v4.y; hv[q4 * 4 + 2] = v4.z; hv[q4 * 4 + 3] = v4.w;
         }
-        store_state(hv, D);   // (the tiles are free: their last readers were complete before the previous segment's last S was)
+        store_state(hv);   // (the tiles are free: their last readers were complete before the previous segment's last S was)
       } else {
         if (g.hs_out != nullptr) {   // the first chunk of a sequence's walk receives nothing
           uint4* dst = reinterpret_cast<uint4*>(g.hs_out + ((static_cast<size_t>(bh) * nc + c_first) * WN + r) * WP + half * 32);
@@ -888,11 +885,7 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
         cum_nxt = g.cum[step0 + i]; dt_nxt = g.dtt[step0 + i]; colf_nxt = g.colf[step0 + i]; oth_nxt = g.cum[other0 + i];
         last_nxt = g.cum[step0 - r + i + WQ - 1];
       };
-      auto prefetch_last = [&](int k) {
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(g.cum + (step0 - r + static_cast<uint32_t>(ANTI ? c_first - k : c_first + k) * WQ + WQ - 1)));
-      };
       fetch(0);
-      if (n > 1) prefetch_last(1);
 
 #pragma unroll 1
       for (int k = -1; k < n; ++k) {   // finishes chunk k, prepares chunk k+1; k = -1 only prepares
@@ -904,25 +897,6 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
           const bool has_state = k > 0 || sg.cin != 0;
           cum_cur = cum_nxt; dt_cur = dt_nxt; last_cur = last_nxt;
           if (more) fetch(k + 1);
-          if (k + 2 < n) prefetch_last(k + 2);
-          // ---- the state chunk k+1 receives: D H + S of chunk k, complete in S's accumulator -------------------------
-          if (!walk_wait(bars + PB_SFULL, par, g.status, abort)) { alive = false; break; }
-          tcgen05_fence_after_sync();
-          if (more || sg.cout) {
-            float hv[32];
-            tmem_ld_32x32(tstate, reinterpret_cast<uint32_t*>(hv));
-            tmem_ld_wait();
-            if (more) {
-              store_state(hv, w_exp(last_nxt));
-            } else {   // the first part of the sequences ends here: their states go to the CTA that walks the rest
-              float4* dst = reinterpret_cast<float4*>(g.carry + (static_cast<size_t>(bh) * WN + r) * WP + half * 32);
-#pragma unroll
-              for (int q4 = 0; q4 < 8; ++q4) __stcg(dst + q4, make_float4(hv[q4 * 4], hv[q4 * 4 + 1], hv[q4 * 4 + 2], hv[q4 * 4 + 3]));
-              __threadfence();
-              __syncwarp();
-              if (lane == 0) atomicAdd(g.carry_flag + sg.seq, 1);
-            }
-          }
           // ---- out = r o (Yd + f o Yo) of chunk k -------------------------------------------
           if (!walk_wait(bars + PB_YFULL, par, g.status, abort)) { alive = false; break; }
           tcgen05_fence_after_sync();
@@ -1091,6 +1065,36 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
             }
           }
           tmem_st_wait();
+          // ---- the state chunk k+2 receives: H' = D H + S of chunk k+1; Yd(k+1) goes where S was -------------------------------
+          if (!walk_wait(bars + PB_SFULL, parn, g.status, abort)) { alive = false; break; }
+          tcgen05_fence_after_sync();
+          if (k + 2 < n || sg.cout) {
+            float hv[32];
+            tmem_ld_32x32(tl + TP_S + ch * 64 + half * 32, reinterpret_cast<uint32_t*>(hv));
+            if (k >= 0 || sg.cin) {
+              const float D = w_exp(last_nxt);
+#pragma unroll
+              for (int p = 0; p < 4; ++p) {
+                uint32_t h8[8];
+                tmem_ld_32x8(tstate + p * 8, h8);
+                tmem_ld_wait();
+#pragma unroll
+                for (int e = 0; e < 8; ++e) hv[p * 8 + e] = fmaf(D, __uint_as_float(h8[e]), hv[p * 8 + e]);
+              }
+            } else {
+              tmem_ld_wait();
+            }
+            if (k + 2 < n) {
+              store_state(hv);
+            } else {   // the first part of the sequences ends here: their states go to the CTA that walks the rest
+              float4* dst = reinterpret_cast<float4*>(g.carry + (static_cast<size_t>(bh) * WN + r) * WP + half * 32);
+#pragma unroll
+              for (int q4 = 0; q4 < 8; ++q4) __stcg(dst + q4, make_float4(hv[q4 * 4], hv[q4 * 4 + 1], hv[q4 * 4 + 2], hv[q4 * 4 + 3]));
+              __threadfence();
+              __syncwarp();
+              if (lane == 0) atomicAdd(g.carry_flag + sg.seq, 1);
+            }
+          }
           warp_arrive(bars + PB_PREADY, lane);
         }
       }
