@@ -924,11 +924,11 @@ void mp_ssd_walk_cumsum(const float* dt, const float* A, float* cum, float* dtt,
 void mp_ssd_walk_cumsum_raw(const __half* raw, size_t raw_pitch, const float* bias, const float* A_log, float* dt_out, float* A_out, float* cum,
                             float* dtt, float* colf_c, int B, int L, int H, int* carry_flags, int n_flags, cudaStream_t st);
 void mp_ssd_walk(int anti, const __half* q, const __half* k, const __half* v, const float* cum, const float* dtt, const float* colf, __half* out,
-                 const __half* z, float* dot_out, float* state_dot, __half* hs_out, float* carry, int* carry_flag, int max_ctas, int B, int L, int H, int G,
+                 const __half* z, float* dot_out, __half* hs_out, float* carry, int* carry_flag, int max_ctas, int B, int L, int H, int G,
                  uint32_t* status, cudaStream_t st);
 
 void mp_ssd_group_grads(const __half* gy, const __half* x, const __half* Bm, const __half* Cm, const __half* hs_causal, const __half* hs_anti,
-                        const float* cum, const float* dtt, const float* colf_c, float* state_dot, __half* gB, __half* gC, int B, int L,
+                        const float* cum, const float* dtt, const float* colf_c, __half* gB, __half* gC, int B, int L,
                         int H, int G, uint32_t* status, cudaStream_t st);
 void mp_ssd_walk_scalars(const float* u, const float* v, const float* dtt, const float* A, const float* pin, float* gdt, float* gA, float* ga_part,
                          float* gb_part, const __half* raw, size_t raw_pitch, const float* bias, __half* graw, size_t graw_pitch, float* gbias,
@@ -955,7 +955,7 @@ WalkScratch walk_carve(void* base, const SsdDims& d, bool reverse, size_t off0) 
   const size_t st = static_cast<size_t>(d.B) * d.H * nc * 128 * 64 * 2;
   w.hs_causal = static_cast<__half*>(take(reverse ? st : 0));
   w.hs_anti = static_cast<__half*>(take(reverse ? st : 0));
-  w.pin = static_cast<float*>(take(reverse ? static_cast<size_t>(d.B) * d.H * nc * 16 * 4 : 0));   // sixteen parts each
+  w.pin = static_cast<float*>(take(reverse ? static_cast<size_t>(d.B) * d.H * nc * 4 : 0));
   w.u = static_cast<float*>(take(reverse ? 2 * bhl * 4 : 0));     // one array per half of the columns
   w.v = static_cast<float*>(take(reverse ? 2 * bhl * 4 : 0));
   w.ga_part = static_cast<float*>(take(reverse ? static_cast<size_t>(d.B) * d.H * nc * 4 : 0));
@@ -1005,7 +1005,7 @@ extern "C" void launch_ssd_scan_r16(const void* x, const void* dt, const void* A
     mp_ssd_walk_cumsum(static_cast<const float*>(dt), static_cast<const float*>(A), w.cum, w.dtt, w.colf_c, nullptr, d.B, d.L, d.H, w.flags,
                        2 * d.B * d.H, st);
     mp_ssd_walk(0, static_cast<const __half*>(Cm), static_cast<const __half*>(Bm), static_cast<const __half*>(x), w.cum, w.dtt, w.colf_c,
-                static_cast<__half*>(y), nullptr, nullptr, nullptr, nullptr, w.carry_c, w.flags, state->sm_count, d.B, d.L, d.H, d.G, state->status_dev,
+                static_cast<__half*>(y), nullptr, nullptr, nullptr, w.carry_c, w.flags, state->sm_count, d.B, d.L, d.H, d.G, state->status_dev,
                 st);
     return;
   }
@@ -1053,7 +1053,7 @@ extern "C" void launch_ssd_scan_raw_r16(const void* x, const void* dt_raw, len_t
     mp_ssd_walk_cumsum_raw(static_cast<const __half*>(dt_raw), dt_pitch, static_cast<const float*>(dt_bias), static_cast<const float*>(A_log),
                            static_cast<float*>(dt_out), static_cast<float*>(A_out), w.cum, w.dtt, w.colf_c, d.B, d.L, d.H, w.flags, 2 * d.B * d.H, st);
     mp_ssd_walk(0, static_cast<const __half*>(Cm), static_cast<const __half*>(Bm), static_cast<const __half*>(x), w.cum, w.dtt, w.colf_c,
-                static_cast<__half*>(y), nullptr, nullptr, nullptr, nullptr, w.carry_c, w.flags, state->sm_count, d.B, d.L, d.H, d.G, state->status_dev,
+                static_cast<__half*>(y), nullptr, nullptr, nullptr, w.carry_c, w.flags, state->sm_count, d.B, d.L, d.H, d.G, state->status_dev,
                 st);
     return;
   }
@@ -1128,21 +1128,31 @@ static bool ssd_scan_reverse_r16_impl(const void* x, const void* dt, const void*
       MP_CUDA_CHECK(cudaEventRecord(state->aux_fork, st));
       MP_CUDA_CHECK(cudaStreamWaitEvent(lane1, state->aux_fork, 0));
     }
-    mp_ssd_walk(1, bh, ch, gyh, w.cum, w.dtt, w.colf_a, static_cast<__half*>(gx), xh, w.v, nullptr, w.hs_anti, w.carry_a, w.flags + d.B * d.H, walk_ctas,
+    mp_ssd_walk(1, bh, ch, gyh, w.cum, w.dtt, w.colf_a, static_cast<__half*>(gx), xh, w.v, w.hs_anti, w.carry_a, w.flags + d.B * d.H, walk_ctas,
                 d.B, d.L, d.H, d.G, state->status_dev, st);
-    mp_ssd_walk(0, ch, bh, xh, w.cum, w.dtt, w.colf_c, nullptr, gyh, w.u, w.pin, w.hs_causal, w.carry_c, w.flags, walk_ctas, d.B, d.L, d.H, d.G,
+    mp_ssd_walk(0, ch, bh, xh, w.cum, w.dtt, w.colf_c, nullptr, gyh, w.u, w.hs_causal, w.carry_c, w.flags, walk_ctas, d.B, d.L, d.H, d.G,
                 state->status_dev, lane1);
     if (side) {
       MP_CUDA_CHECK(cudaEventRecord(state->aux_join[0], lane1));
       MP_CUDA_CHECK(cudaStreamWaitEvent(st, state->aux_join[0], 0));
+      // gdt / gA need both walks (u, v, states) but not gB / gC: they run beside the group-gradient kernel
+      MP_CUDA_CHECK(cudaEventRecord(state->aux_sub_fork[0], st));
+      MP_CUDA_CHECK(cudaStreamWaitEvent(lane1, state->aux_sub_fork[0], 0));
     }
-    mp_ssd_group_grads(gyh, xh, bh, ch, w.hs_causal, w.hs_anti, w.cum, w.dtt, w.colf_c, w.pin, static_cast<__half*>(gB), static_cast<__half*>(gC),
+    mp_ssd_group_grads(gyh, xh, bh, ch, w.hs_causal, w.hs_anti, w.cum, w.dtt, w.colf_c, static_cast<__half*>(gB), static_cast<__half*>(gC),
                        d.B, d.L, d.H, d.G, state->status_dev, st);
+    const int wnc = (d.L + 127) / 128;
+    MpLaunch(d.B * d.H * wnc, 256, 0, lane1)(ssd_boundary_dot_kernel, w.hs_anti, w.hs_causal, w.pin, wnc, d.N * d.P);
+    MP_LAUNCH_CHECK();
     const RawSide none{nullptr, 0, nullptr, nullptr, 0, nullptr, nullptr};
     const RawSide& side_out = rs != nullptr ? *rs : none;
     mp_ssd_walk_scalars(w.u, w.v, w.dtt, static_cast<const float*>(A), w.pin, static_cast<float*>(gdt), static_cast<float*>(gA), w.ga_part, w.gb_part,
                         side_out.raw, side_out.raw_pitch, side_out.bias, side_out.graw, side_out.graw_pitch, side_out.gbias, side_out.gA_log, d.B, d.L,
-                        d.H, st);
+                        d.H, lane1);
+    if (side) {
+      MP_CUDA_CHECK(cudaEventRecord(state->aux_join[1], lane1));
+      MP_CUDA_CHECK(cudaStreamWaitEvent(st, state->aux_join[1], 0));
+    }
     return true;
   }
   const SsdScratch sc = ssd_carve(scratch, d, true);

@@ -60,7 +60,6 @@ struct WalkArgs {
   __half* out;             // [B*L, H*64] or null
   const __half* z;         // dot partner, same indexing as out, or null
   float* dot_out;          // [2][B, H, LP] row dots <z, out> from the fp32 accumulators, one array per half of the columns, or null
-  float* state_dot;        // [B, H, nc][16], first eight: sums over a chunk's rows of <z, the received state's share of out>, one per worker warp (causal form with dot_out)
   __half* hs_out;          // [B, H, nc][128][64]: state every chunk receives, or null
   float* carry;            // [B * H][128][64] fp32: state handed from the CTA that walked the first part of a sequence to the next
   int* carry_flag;         // [B * H]: number of worker warps (of 8) that have written their part of `carry`; zero before the launch
@@ -540,7 +539,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_con
 #pragma unroll
         for (int e = 0; e < 32; ++e) o[e] = ro * (__uint_as_float(yd[e]) + fo * __uint_as_float(yo[e]));
         if (DOT) {   // this thread's row of z comes back from the staging positions before the output overwrites them
-          float dot = 0.f, dot_state = 0.f;
+          float dot = 0.f;
 #pragma unroll
           for (int q4 = 0; q4 < 4; ++q4) {
             const uint4 zq = *reinterpret_cast<const uint4*>(stg + r * 128 + (((ch * 4 + q4) ^ (r & 7)) << 4));
@@ -550,14 +549,9 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_con
               const float2 zf = __half22float2(z2[e]);
               const int k0 = q4 * 8 + 2 * e;
               dot += zf.x * o[k0] + zf.y * o[k0 + 1];
-              if (!ANTI) dot_state += zf.x * __uint_as_float(yo[k0]) + zf.y * __uint_as_float(yo[k0 + 1]);
             }
           }
           g.dot_out[static_cast<size_t>(ch) * g.B * g.H * (static_cast<size_t>(g.nc) * WQ) + step0 + c * WQ] = dot;
-          if (!ANTI) {   // the received state's share of the row dots, summed over the rows
-            dot_state = warp_reduce<SumOp>(dot_state * fo);
-            if (lane == 0) g.state_dot[(bh * g.nc + c) * 16 + (warp - 2)] = dot_state;
-          }
           __syncwarp();
         }
         if (g.out != nullptr) {
@@ -904,7 +898,7 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
           const float ro = ANTI ? dt_cur : 1.f;
           unsigned char* stage = smem + (q & 1) * WP2_QK;   // q and k of chunk k, read by now: the output goes where q was, z is where k was
           if (DOT && !walk_wait(bars + PB_ZFULL, par, g.status, abort)) { alive = false; break; }
-          float dot = 0.f, dot_state = 0.f;
+          float dot = 0.f;
 #pragma unroll
           for (int p = 0; p < 2; ++p) {
             uint32_t yd[16], yo[16];
@@ -918,10 +912,8 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
 #pragma unroll
             for (int q4 = 0; q4 < 2; ++q4) {
               float o[8];
-              if (OUT) {
 #pragma unroll
-                for (int e = 0; e < 8; ++e) o[e] = ro * (__uint_as_float(yd[q4 * 8 + e]) + fo * __uint_as_float(yo[q4 * 8 + e]));
-              }
+              for (int e = 0; e < 8; ++e) o[e] = ro * (__uint_as_float(yd[q4 * 8 + e]) + fo * __uint_as_float(yo[q4 * 8 + e]));
               const uint32_t slot = half_row + ((((p * 2 + q4) ^ half_sw)) << 4);
               if (DOT) {
                 const uint4 zq = *reinterpret_cast<const uint4*>(stage + W_TILE_QK + slot);
@@ -929,25 +921,13 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                   const float2 zf = __half22float2(z2[e]);
-                  const int k0 = q4 * 8 + 2 * e;
-                  if (OUT) {
-                    dot += zf.x * o[2 * e] + zf.y * o[2 * e + 1];
-                  } else {
-                    dot += zf.x * __uint_as_float(yd[k0]) + zf.y * __uint_as_float(yd[k0 + 1]);
-                    dot_state += zf.x * __uint_as_float(yo[k0]) + zf.y * __uint_as_float(yo[k0 + 1]);
-                  }
+                  dot += zf.x * o[2 * e] + zf.y * o[2 * e + 1];
                 }
               }
               if (OUT) *reinterpret_cast<uint4*>(stage + slot) = walk_pack8(o);
             }
           }
           if (DOT) {
-            if (!OUT) {   // the received state's share of the row dots, summed over the rows
-              dot_state *= fo;
-              dot += dot_state;
-              dot_state = warp_reduce<SumOp>(dot_state);
-              if (lane == 0) g.state_dot[(static_cast<size_t>(bh) * nc + c) * 16 + quarter * 2 + half] = dot_state;
-            }
             g.dot_out[half * (static_cast<size_t>(g.B) * g.H * LP) + step0 + static_cast<uint32_t>(c) * WQ] = dot;
           }
           if (OUT) {
@@ -1130,7 +1110,6 @@ enum { GB_FULL0 = 0, GB_FULL1, GB_EMPTY0, GB_EMPTY1, GB_SC0, GB_SC1, GB_SCALED, 
 struct GroupArgs {
   int B, L, H, G, nc;
   const float* cum; const float* dtt; const float* colf;   // [B, H, nc * 128], causal column factors
-  float* state_dot;                                        // [B, H, nc][16], last eight: exp(cum_last) <Hc, Ha>, one part per worker warp
   uint32_t* status;
 };
 
@@ -1342,20 +1321,9 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_group_grads_kernel(const __g
         const __half2 w2 = __float2half2_rn(w_exp(cum_last - cum_r) * dt_r);
         unsigned char* gyrow = smem + s * GG_STAGE + r * 128;
         unsigned char* xrow = gyrow + GG_TILE;
-        float hdot = 0.f;
 #pragma unroll
         for (int q4 = 0; q4 < 4; ++q4) {
           const int off = ((ch * 4 + q4) ^ (r & 7)) << 4;
-          {   // <Hc, Ha> of the chunk: see ssd_walk_scalars_kernel
-            const uint4 c4 = *reinterpret_cast<const uint4*>(gyrow + 2 * GG_TILE + off), a4 = *reinterpret_cast<const uint4*>(gyrow + 3 * GG_TILE + off);
-            const __half2* hc = reinterpret_cast<const __half2*>(&c4);
-            const __half2* ha2 = reinterpret_cast<const __half2*>(&a4);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float2 p = __half22float2(hc[e]), q = __half22float2(ha2[e]);
-              hdot += p.x * q.x + p.y * q.y;
-            }
-          }
           uint4 a = *reinterpret_cast<const uint4*>(gyrow + off);
           uint4 x4 = *reinterpret_cast<const uint4*>(xrow + off);
           __half2* ha = reinterpret_cast<__half2*>(&a);
@@ -1365,8 +1333,6 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_group_grads_kernel(const __g
           *reinterpret_cast<uint4*>(gyrow + off) = a;
           *reinterpret_cast<uint4*>(xrow + off) = x4;
         }
-        hdot = warp_reduce<SumOp>(hdot * w_exp(cum_last));
-        if (lane == 0) g.state_dot[((static_cast<size_t>(b) * g.H + grp * hpg + hi) * g.nc + c) * 16 + 8 + (warp - 2)] = hdot;
       }
       warp_arrive(bars + GB_SCALED, lane);
     }
@@ -1512,12 +1478,9 @@ __global__ void __launch_bounds__(WS_THREADS) ssd_walk_cumsum_kernel(const float
 // u_t - v_t cancels and carries the rounding noise of two different operator instances, so a suffix sum over the whole
 // sequence random-walks (measured: gA off by 5 % at 8192 steps).  The sum is therefore pinned at every chunk boundary to a value
 // without such noise, summed only inside a chunk, and the residual between a chunk's two pins is spread linearly over its steps.
-//   pin(c) = g_a at the first step of chunk c = < what chunk c-1 receives from its successors, Hc = what chunk c receives from its
-//            predecessors >  and, the first factor being exp(cum_last) Ha + sum_i e_i C_i gy_i^T over the steps i of chunk c,
-//          = exp(cum_last) <Hc, Ha>  [the group-gradient kernel, which has both tiles in shared memory]
-//            + sum_i (the received state's share of u_i)  [the causal walk]
-// (state_dot, eight parts of each), so the states are not read again for it: a kernel of its own spent 89 us on that for
-// [8, 8192, 32, 64] and 70 us for [8, 2048, 24, 64].
+//   pin(c) = g_a just behind chunk c = < what chunk c receives from its successors, what chunk c+1 receives from its predecessors >
+// (ssd_boundary_dot_kernel, beside the group-gradient kernel).  Collecting it from the two kernels that hold the states was 60 us
+// faster at [8, 8192, 32, 64] but takes the product at another place, and the last bits of gdt with it.
 // Every chunk is then on its own: one CTA per (b, chunk, eight heads), one warp per head, four neighbouring steps per lane, and
 // gdt (and graw) leave as rows of eight heads.
 // With `raw` (the projection's raw step sizes, r16, pitched) the reverse of dt = softplus(raw + bias[h]) is applied on the
@@ -1533,7 +1496,7 @@ struct ScalarArgs {
   const float* u; const float* v;   // [2][B, H, nc * 128]: one array per half of the columns
   const float* dtt;                 // [B, H, nc * 128]
   const float* A;
-  const float* pin;                 // [B, H, nc][16]
+  const float* pin;                 // [B, H, nc]: g_a just behind the chunk
   float* gdt;                       // [B, L, H]
   float* ga_part; float* gb_part;   // [B * nc][H]
   const __half* raw; size_t raw_pitch; const float* bias; __half* graw; size_t graw_pitch;
@@ -1551,30 +1514,46 @@ __global__ void __launch_bounds__(WS_THREADS) ssd_walk_scalars_kernel(const Scal
     const float4 u0 = *reinterpret_cast<const float4*>(g.u + o), u1 = *reinterpret_cast<const float4*>(g.u + half + o);
     const float4 v0 = *reinterpret_cast<const float4*>(g.v + o), v1 = *reinterpret_cast<const float4*>(g.v + half + o);
     const float4 d4 = *reinterpret_cast<const float4*>(g.dtt + o);
-    // lanes 0-15: the parts of this chunk's pin, lanes 16-31: those of the next chunk's (zero behind the last chunk)
-    float part = 0.f;
-    if (lane < 16 || c + 1 < g.nc) part = g.pin[(bh * g.nc + c) * 16 + lane];
-#pragma unroll
-    for (int off = 8; off > 0; off >>= 1) part += __shfl_xor_sync(0xffffffffu, part, off);
-    const float left = __shfl_sync(0xffffffffu, part, 0), right = __shfl_sync(0xffffffffu, part, 16);
+    const float right = g.pin[bh * g.nc + c], left = c > 0 ? g.pin[bh * g.nc + c - 1] : 0.f;   // g_a behind the chunk and at its first step
     const float vt[4] = {v0.x + v1.x, v0.y + v1.y, v0.z + v1.z, v0.w + v1.w}, dt[4] = {d4.x, d4.y, d4.z, d4.w};
-    float within[4] = {u0.x + u1.x - vt[0], u0.y + u1.y - vt[1], u0.z + u1.z - vt[2], u0.w + u1.w - vt[3]};   // suffix sums of u - v
-#pragma unroll
-    for (int e = 2; e >= 0; --e) within[e] += within[e + 1];
-    float incl = within[0];
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const float dn = __shfl_down_sync(0xffffffffu, incl, off);
-      if (lane + off < 32) incl += dn;
+    // suffix sums of u - v: 32 steps (eight lanes) by doubling offsets, then the totals of the 32-step groups behind them
+    float x[4] = {u0.x + u1.x - vt[0], u0.y + u1.y - vt[1], u0.z + u1.z - vt[2], u0.w + u1.w - vt[3]};
+    const int l8 = 7 - (lane & 7);
+    {
+      const float n0 = __shfl_down_sync(0xffffffffu, x[0], 1);
+      const float w3 = l8 >= 1 ? x[3] + n0 : x[3], w2 = x[2] + x[3], w1 = x[1] + x[2], w0 = x[0] + x[1];
+      x[0] = w0; x[1] = w1; x[2] = w2; x[3] = w3;
     }
-    const float total = __shfl_sync(0xffffffffu, incl, 0), behind = incl - within[0];
+    {
+      const float n0 = __shfl_down_sync(0xffffffffu, x[0], 1), n1 = __shfl_down_sync(0xffffffffu, x[1], 1);
+      const float w1 = x[1] + x[3], w0 = x[0] + x[2];
+      if (l8 >= 1) { x[3] += n1; x[2] += n0; }
+      x[0] = w0; x[1] = w1;
+    }
+#pragma unroll
+    for (int off = 1; off < 8; off <<= 1)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float dn = __shfl_down_sync(0xffffffffu, x[e], off);
+        if (l8 >= off) x[e] += dn;
+      }
+    float behind = 0.f;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const float tot = __shfl_sync(0xffffffffu, x[0], 24 - 8 * q);
+      if (q < ((31 - lane) >> 3)) behind += tot;
+    }
+    float within[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) within[e] = x[e] + behind;
+    const float total = __shfl_sync(0xffffffffu, within[0], 0);
     const float resid = c > 0 ? left - (right + total) : 0.f;   // what the sum misses of the pin at the chunk's first step
     const float a_h = g.A[h];
     float ga_acc = 0.f;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const int t = lane * 4 + e;
-      const float ga = right + within[e] + behind + resid * (static_cast<float>(WQ - t) / static_cast<float>(WQ));
+      const float ga = right + within[e] + resid * (static_cast<float>(WQ - t) / static_cast<float>(WQ));
       if (c * WQ + t < g.L) ga_acc += dt[e] * ga;
       s_gd[t][w] = vt[e] / dt[e] + a_h * ga;
     }
@@ -1736,11 +1715,11 @@ void mp_ssd_walk_scalars(const float* u, const float* v, const float* dtt, const
 // One walk.  q, k: [B*L, G*128]; v, z, out: [B*L, H*64]; cum, dtt, colf (of the walk's direction): [B, H, nc * 128] from mp_ssd_walk_cumsum.
 void mp_ssd_walk(int anti, const __half* q, const __half* k, const __half* v, const float* cum, const float* dtt, const float* colf, __half* out,
                  const __half* z,
-                 float* dot_out, float* state_dot, __half* hs_out, float* carry, int* carry_flag, int max_ctas, int B, int L, int H, int G, uint32_t* status,
+                 float* dot_out, __half* hs_out, float* carry, int* carry_flag, int max_ctas, int B, int L, int H, int G, uint32_t* status,
                  cudaStream_t st) {
   WalkArgs g;
   g.B = B; g.L = L; g.H = H; g.G = G; g.nc = (L + WQ - 1) / WQ;
-  g.cum = cum; g.dtt = dtt; g.colf = colf; g.out = out; g.z = z; g.dot_out = dot_out; g.state_dot = state_dot; g.hs_out = hs_out; g.status = status;
+  g.cum = cum; g.dtt = dtt; g.colf = colf; g.out = out; g.z = z; g.dot_out = dot_out; g.hs_out = hs_out; g.status = status;
   g.carry = carry; g.carry_flag = carry_flag;
   // One CTA per SM slot it may use, every CTA the same number of chunks; never more CTAs than sequences, so that a CTA's
   // range is at least one sequence long (see walk_segment).  MP_SSD_WALK_PER_SEQUENCE: one CTA per sequence, no hand-off.
@@ -1788,11 +1767,11 @@ void mp_ssd_walk(int anti, const __half* q, const __half* k, const __half* v, co
 // gB, gC [B*L, G*128] from gy, x [B*L, H*64], Bm, Cm [B*L, G*128] and the states left by the two walks
 // (hs_causal, hs_anti: [B, H, nc][128][64]).
 void mp_ssd_group_grads(const __half* gy, const __half* x, const __half* Bm, const __half* Cm, const __half* hs_causal, const __half* hs_anti,
-                        const float* cum, const float* dtt, const float* colf_c, float* state_dot, __half* gB, __half* gC, int B, int L,
+                        const float* cum, const float* dtt, const float* colf_c, __half* gB, __half* gC, int B, int L,
                         int H, int G, uint32_t* status, cudaStream_t st) {
   GroupArgs g;
   g.B = B; g.L = L; g.H = H; g.G = G; g.nc = (L + WQ - 1) / WQ;
-  g.cum = cum; g.dtt = dtt; g.colf = colf_c; g.state_dot = state_dot; g.status = status;
+  g.cum = cum; g.dtt = dtt; g.colf = colf_c; g.status = status;
   const size_t srows = static_cast<size_t>(B) * H * g.nc * WN;
   const CUtensorMap mgy = walk_map3(gy, B, L, static_cast<size_t>(H) * WP), mx = walk_map3(x, B, L, static_cast<size_t>(H) * WP);
   const CUtensorMap mhc = walk_map(hs_causal, srows, WP), mha = walk_map(hs_anti, srows, WP);
