@@ -611,21 +611,22 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_con
 // them once and its scores are computed once; Yo and S of both are single MMAs with 128 columns.  What this buys is the chain: with
 // one head a chunk is a sequence of hand-offs between the tensor core and the worker warps that leaves both idle most of the time,
 // with two the workers have twice the work per hand-off.
-// Order of a chunk k for the workers: fold S(k) into the states, epilogue of Y(k), scale the values of chunk k+1, write P(k+1);
-// for the MMA warp: [P(k) written] Yd(k), G(k+1), [values and states of k+1 written] Yo(k+1), S(k+1).  Every MMA then runs while
-// the workers are in the step before the one that needs it.
+// Order of a chunk k for the workers: epilogue of Y(k-1), scale the values of chunk k, write P(k), fold S(k) into the states; for the
+// MMA warp: [values and states of k written] Yo(k), S(k), [P(k) written, S(k) read] Yd(k), G(k+1).
 // Shared memory has room for one v tile of each head only: v(k+1) is requested when Yd(k) has read v(k).  P lies in TMEM, in the columns
 // of the scores it is made from (16 score columns become 8 + 8 columns of packed r16 pairs, one block per head): Yd reads its
-// A operand there.  The states lie in TMEM as well: the workers leave D H (fp32) in S's accumulator, S adds to it.
+// A operand there.  The fp32 states lie in TMEM as well, S and Yd share columns.  (Letting S add to D H inside its accumulator
+// leaves Yd columns of its own and is 10 % faster, but rounds differently from the fused multiply-add of the one-head kernel: every
+// result here is bit for bit that kernel's.)
 // q and k of a chunk are read once S(k) is complete, so that their tiles take the dot partner's rows (TMA load) and the output's
 // (TMA store, 32 columns a warp) before the stage goes back to the ring.
-// Bound: the latency of the workers' steps, about 7000 cycles a chunk pair (state 1000, epilogue 1500, scaled values 1000, P 1900,
-// the rest hand-offs) beside 2100 cycles of MMAs; four worker warps a scheduler hide part of it.  What counts there is registers
+// Bound: the latency of the workers' steps, about 8000 cycles a chunk pair (state 1000, epilogue 1500, scaled values 1000, P 1900,
+// Yd 900, the rest hand-offs) beside 2100 cycles of MMAs; four worker warps a scheduler hide part of it.  What counts there is registers
 // (shared memory leaves L1 next to nothing, so a spill is an L2 access; hence the split below) and straight-line code in P, whose
 // exponentials and shared-memory loads then overlap (one exponent-per-element path for a block as a whole, not one per 8 steps).
-// 8 x 8192 steps x 32 heads, one head -> two heads at a time: forward 346 -> 252 us, reverse 1168 -> 836 us; 8 x 2048 x 24: 80 -> 75 us
-// and 249 -> 191 us.  On the way: eight worker warps with the states in registers 396 us forward; the output and the dot partner by
-// loads and stores of 64-byte row pieces 294 us and 900 us (1500 cycles a chunk in the load/store unit).
+// 8 x 8192 steps x 32 heads, one head -> two heads at a time: forward 346 -> 281 us, reverse 1168 -> 923 us; 8 x 2048 x 24 reverse 249 ->
+// 203 us.  On the way: eight worker warps with the states in registers 396 us forward; the output and the dot partner by loads and
+// stores of 64-byte row pieces 44 us more forward and reverse (1500 cycles a chunk in the load/store unit).
 // ---------------------------------------------------------------------------
 constexpr int WP2_QK = 2 * W_TILE_QK;              // q and k of a chunk, 64 KB; two stages
 constexpr int WP2_HALF = W_TILE_V / 2;             // 32 columns of one head
@@ -1723,13 +1724,13 @@ void mp_ssd_walk(int anti, const __half* q, const __half* k, const __half* v, co
   g.carry = carry; g.carry_flag = carry_flag;
   // One CTA per SM slot it may use, every CTA the same number of chunks; never more CTAs than sequences, so that a CTA's
   // range is at least one sequence long (see walk_segment).  MP_SSD_WALK_PER_SEQUENCE: one CTA per sequence, no hand-off.
-  // Two heads at a time where their group has an even number of heads and there are enough sequences: a chunk of a pair takes 1.25
-  // times as long as a chunk of one head (3.8 against 3.05 us in the forward, 4.75 against 3.9 us in the reverse), which pays unless
-  // CTAs are left without a sequence; 192 sequences on 148 CTAs, a ratio of 1.297, are past the line (80 -> 75 us).  The pair
-  // kernel counts steps in 32 bits.  MP_SSD_WALK_NO_PAIRS: one head at a time, for an A/B.
+  // Two heads at a time where their group has an even number of heads and there are enough sequences: a chunk of a pair takes 1.4
+  // times as long as a chunk of one head (4.3 against 3.05 us in the forward), which pays unless CTAs are left without a sequence; at
+  // 192 sequences on 148 CTAs, a ratio of 1.297, both take 80 us.  The pair kernel counts steps in 32 bits.
+  // MP_SSD_WALK_NO_PAIRS: one head at a time, for an A/B.
   const bool bounded = max_ctas > 0 && getenv("MP_SSD_WALK_PER_SEQUENCE") == nullptr;
   auto load = [&](int seqs) { return bounded && seqs > max_ctas ? static_cast<double>(seqs) / max_ctas : 1.0; };   // sequences per CTA
-  const bool pairs = (H / G) % 2 == 0 && static_cast<size_t>(B) * H * g.nc * WQ < (size_t{1} << 31) && 1.25 * load(B * H / 2) < load(B * H) &&
+  const bool pairs = (H / G) % 2 == 0 && static_cast<size_t>(B) * H * g.nc * WQ < (size_t{1} << 31) && 1.4 * load(B * H / 2) < load(B * H) &&
                      getenv("MP_SSD_WALK_NO_PAIRS") == nullptr;
   int grid = pairs ? B * H / 2 : B * H;
   if (bounded && max_ctas < grid) grid = max_ctas;

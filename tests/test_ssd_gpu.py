@@ -218,8 +218,8 @@ def test_ssd_on_ragged_lengths(mp, stream, orc, dims):
     # (batch, seqlen, heads, headdim, dstate, groups, chunk), shift of the raw step sizes.  The walk takes two heads of a group at a time
     # where there are enough sequences: uncut in the forward and cut in the reverse, cut in both (two groups), an odd number of
     # heads per group beside it (one head at a time), and steps that decay by more than e^-80 in eight, whose mask is made step by step
-    ((12, 300, 16, 64, 128, 1, 128), 0.0), ((20, 256, 32, 64, 128, 2, 128), 0.0), ((20, 200, 15, 64, 128, 1, 128), 0.0),
-    ((12, 200, 16, 64, 128, 1, 128), 7.0), ((20, 160, 15, 64, 128, 1, 128), 7.0)])
+    ((14, 300, 16, 64, 128, 1, 128), 0.0), ((20, 256, 32, 64, 128, 2, 128), 0.0), ((20, 200, 15, 64, 128, 1, 128), 0.0),
+    ((14, 200, 16, 64, 128, 1, 128), 7.0), ((20, 160, 15, 64, 128, 1, 128), 7.0)])
 def test_ssd_heads_in_pairs(mp, stream, orc, dims, shift):
     import torch
     nb, L, H, P, N, G, Q = dims
