@@ -147,10 +147,12 @@ MP_DECL3(linear_ij_jk_ik_ik, const void* a, const void* b, const void* r, double
  * scratch: mpSsdScanScratchBytes(..., reverse) bytes owned by the caller (the reverse holds four
  * independent sets of intermediates, its operator instances run side by side on helper streams that
  * the library forks from and joins back into the caller's stream).
- * Two implementations: a tensor-core path (r16 with dstate = 128; headdim 64 with any seqlen from 32 on, or headdim 128 with
- * chunk 128 or 256 and seqlen a multiple of chunk) and a sequential-recurrence path for every other shape of r16 and for r32 /
- * r64 storage (dt, A, gdt, gA then have the storage type; `chunk` is ignored).  Scratch: r16 ->
- * mpSsdScanScratchBytes (either path), r32 / r64 -> mpSsdScanGenericScratchBytes(dtype_key, ...); the
+ * r16 has a tensor-core path (dstate = 128, headdim 64 or 128, chunk 128 or 256, seqlen a multiple of chunk; r16 score and state
+ * tiles, and under decay so strong that next to nothing is carried from step to step gA and gdt keep few digits: they are
+ * made of differences of row dots; the r16 pointers are 16-byte aligned) and an fp32 path (dstate = 128, headdim 64, any other chunk or
+ * seqlen from 32 on).  Every other shape of r16, r32 / r64 storage (dt, A, gdt, gA then have the storage type; `chunk` is ignored)
+ * and an r16 forward of the fp32 path's shapes without scratch take a sequential recurrence.  Scratch: r16 -> mpSsdScanScratchBytes
+ * (whatever the path), r32 / r64 -> mpSsdScanGenericScratchBytes(dtype_key, ...); the
  * forward of the sequential path needs none. */
 MP_DECL3(ssd_scan, const void* x, const void* dt, const void* A, const void* B, const void* C, void* y, void* scratch, len_t batch, len_t seqlen, len_t heads, len_t headdim, len_t dstate, len_t ngroups, len_t chunk, StreamContext stream)
 /* Reverse of the scan: given gy (shape of y) writes (overwrites) gx, gdt (r32),

@@ -30,6 +30,13 @@
 #include <mutex>
 
 bool mp_ssd_walk_supported(int L, int H, int P, int N, int G);   // ssd_walk.cu
+// ssd_segments.cu
+bool mp_ssd_segments_supported(int L, int H, int P, int N, int G);
+size_t mp_ssd_segments_scratch(int B, int L, int H, int G, bool reverse);
+void mp_ssd_segments_forward(const void* x, const void* dt, const void* A, const void* Bm, const void* Cm, void* y, void* scratch, int B, int L,
+                             int H, int G, cudaStream_t st);
+void mp_ssd_segments_reverse(const void* x, const void* dt, const void* A, const void* Bm, const void* Cm, const void* gy, void* gx, void* gdt,
+                             void* gA, void* gB, void* gC, void* scratch, int B, int L, int H, int G, cudaStream_t st);
 
 namespace {
 
@@ -892,12 +899,16 @@ bool ssd_whole_chunks(const SsdDims& d) {
   return d.N == 128 && (d.P == 64 || d.P == 128) && (d.Q == 128 || d.Q == 256) && d.L % d.Q == 0;
 }
 
-// Shapes the tensor-core paths cover; everything else takes the sequential-recurrence kernels of ssd_generic.cu.  The
-// chunk walk takes any sequence length, whatever the `chunk` argument (its chunks are 128 steps, the last one padded): on
-// [2, 1000, 24, 64] forward + reverse the recurrence needs 43.7 ms, one step after the other on 48 SMs.
+// Shapes the tensor-core paths cover.  Others of head size 64 and state 128 take the fp32 segments of ssd_segments.cu (the chunk walk could
+// evaluate any length with a padded last chunk, but its r16 score and state tiles lose what these lengths had: at [2, 1000, 24] gdt
+// went from 2e-7 to 4e-4 of its norm, and under strong decay nothing was left of gA); everything else takes the sequential
+// recurrence of ssd_generic.cu.
 bool ssd_tensor_path(const SsdDims& d) {
   if (d.G <= 0 || d.H % d.G != 0) MP_FATAL("ssd_scan: heads %d not divisible by groups %d", d.H, d.G);
-  return (mp_ssd_walk_supported(d.L, d.H, d.P, d.N, d.G) || ssd_whole_chunks(d)) && getenv("MP_SSD_FORCE_GENERIC") == nullptr;
+  return ssd_whole_chunks(d) && getenv("MP_SSD_FORCE_GENERIC") == nullptr;
+}
+bool ssd_segment_path(const SsdDims& d) {
+  return !ssd_tensor_path(d) && mp_ssd_segments_supported(d.L, d.H, d.P, d.N, d.G) && getenv("MP_SSD_FORCE_GENERIC") == nullptr;
 }
 
 SsdDims ssd_dims(len_t batch, len_t seqlen, len_t heads, len_t headdim, len_t dstate, len_t ngroups, len_t chunk) {
@@ -938,16 +949,16 @@ namespace {
 // Scratch of the walk path: prefix sums and dt in [B,H,L] order; for the reverse also the states every 128-step
 // chunk receives from its predecessors and from its successors (r16 [B,H,L/128][128][64]).
 struct WalkScratch { float* cum; float* dtt; float* colf_c; float* colf_a; __half* hs_causal; __half* hs_anti; float* pin; float* u; float* v; float* ga_part; float* gb_part; float* carry_c; float* carry_a; int* flags; size_t total; };
-// The forward takes the chunk walk where it applies; MP_SSD_LEGACY_FORWARD selects the three-phase path on the shapes that it has too.
+// The forward takes the chunk walk where it applies; MP_SSD_LEGACY_FORWARD selects the three-phase path.
 bool ssd_forward_walks(const SsdDims& d) {
-  return mp_ssd_walk_supported(d.L, d.H, d.P, d.N, d.G) && (getenv("MP_SSD_LEGACY_FORWARD") == nullptr || !ssd_whole_chunks(d));
+  return mp_ssd_walk_supported(d.L, d.H, d.P, d.N, d.G) && getenv("MP_SSD_LEGACY_FORWARD") == nullptr;
 }
 WalkScratch walk_carve(void* base, const SsdDims& d, bool reverse, size_t off0) {
   WalkScratch w;
   size_t off = off0;
   auto take = [&](size_t bytes) { void* p = base ? static_cast<unsigned char*>(base) + off : nullptr; off += (bytes + 255) & ~size_t(255); return p; };
-  const size_t nc = (static_cast<size_t>(d.L) + 127) / 128;
-  const size_t bhl = static_cast<size_t>(d.B) * d.H * nc * 128;
+  const size_t nc = static_cast<size_t>(d.L) / 128;
+  const size_t bhl = static_cast<size_t>(d.B) * d.H * d.L;
   w.cum = static_cast<float*>(take(bhl * 4));
   w.dtt = static_cast<float*>(take(bhl * 4));
   w.colf_c = static_cast<float*>(take(bhl * 4));
@@ -975,6 +986,7 @@ extern "C" len_t mpSsdScanScratchBytes(len_t batch, len_t seqlen, len_t heads, l
                                        len_t chunk, uint32_t reverse) {
   const SsdDims d = ssd_dims(batch, seqlen, heads, headdim, dstate, ngroups, chunk);
   if (batch == 0 || seqlen == 0 || heads == 0) return 256;
+  if (ssd_segment_path(d)) return mp_ssd_segments_scratch(d.B, d.L, d.H, d.G, reverse != 0);
   if (!ssd_tensor_path(d)) return mpSsdScanGenericScratchBytes(0, batch, seqlen, heads, headdim, dstate, ngroups, reverse);
   if (mp_ssd_walk_supported(d.L, d.H, d.P, d.N, d.G)) {
     if (reverse != 0) return walk_carve(nullptr, d, true, 0).total;
@@ -991,7 +1003,11 @@ extern "C" void launch_ssd_scan_r16(const void* x, const void* dt, const void* A
                                     len_t ngroups, len_t chunk, StreamContext ctx) {
   if (batch == 0 || seqlen == 0 || heads == 0) return;
   const SsdDims d = ssd_dims(batch, seqlen, heads, headdim, dstate, ngroups, chunk);
-  if (!ssd_tensor_path(d) || (scratch == nullptr && !ssd_whole_chunks(d))) {   // the recurrence's forward needs no scratch
+  if (scratch != nullptr && ssd_segment_path(d)) {
+    mp_ssd_segments_forward(x, dt, A, Bm, Cm, y, scratch, d.B, d.L, d.H, d.G, mp_stream(ctx));
+    return;
+  }
+  if (!ssd_tensor_path(d)) {   // the recurrence's forward needs no scratch
     mp_ssd_generic_forward_r16(x, dt, A, Bm, Cm, y, batch, seqlen, heads, headdim, dstate, ngroups, ctx);
     return;
   }
@@ -1045,7 +1061,7 @@ extern "C" void launch_ssd_scan_raw_r16(const void* x, const void* dt_raw, len_t
                                         len_t headdim, len_t dstate, len_t ngroups, len_t chunk, StreamContext ctx) {
   if (batch == 0 || seqlen == 0 || heads == 0) return;
   const SsdDims d = ssd_dims(batch, seqlen, heads, headdim, dstate, ngroups, chunk);
-  if (ssd_tensor_path(d) && ssd_forward_walks(d) && (scratch != nullptr || ssd_whole_chunks(d))) {
+  if (ssd_tensor_path(d) && ssd_forward_walks(d)) {
     if (scratch == nullptr) MP_FATAL("ssd_scan_raw: scratch must not be NULL");
     MpStreamState* state = mp_state(ctx);
     cudaStream_t st = mp_stream(ctx);
@@ -1101,6 +1117,10 @@ static bool ssd_scan_reverse_r16_impl(const void* x, const void* dt, const void*
                                       len_t headdim, len_t dstate, len_t ngroups, len_t chunk, StreamContext ctx, const RawSide* rs) {
   if (batch == 0 || seqlen == 0 || heads == 0) return true;
   const SsdDims d = ssd_dims(batch, seqlen, heads, headdim, dstate, ngroups, chunk);
+  if (scratch != nullptr && ssd_segment_path(d)) {
+    mp_ssd_segments_reverse(x, dt, A, Bm, Cm, gy, gx, gdt, gA, gB, gC, scratch, d.B, d.L, d.H, d.G, mp_stream(ctx));
+    return false;
+  }
   if (!ssd_tensor_path(d)) {
     mp_ssd_generic_reverse_r16(x, dt, A, Bm, Cm, gy, gx, gdt, gA, gB, gC, scratch, batch, seqlen, heads, headdim, dstate, ngroups, ctx);
     return false;
@@ -1141,7 +1161,7 @@ static bool ssd_scan_reverse_r16_impl(const void* x, const void* dt, const void*
     }
     mp_ssd_group_grads(gyh, xh, bh, ch, w.hs_causal, w.hs_anti, w.cum, w.dtt, w.colf_c, static_cast<__half*>(gB), static_cast<__half*>(gC),
                        d.B, d.L, d.H, d.G, state->status_dev, st);
-    const int wnc = (d.L + 127) / 128;
+    const int wnc = d.L / 128;
     MpLaunch(d.B * d.H * wnc, 256, 0, lane1)(ssd_boundary_dot_kernel, w.hs_anti, w.hs_causal, w.pin, wnc, d.N * d.P);
     MP_LAUNCH_CHECK();
     const RawSide none{nullptr, 0, nullptr, nullptr, 0, nullptr, nullptr};

@@ -49,17 +49,14 @@ constexpr uint32_t TC_G = 0, TC_S = 128, TC_Y = 192, TC_COLS = 512;   // Yd / Yo
 
 enum { B_FULL0 = 0, B_FULL1, B_EMPTY0, B_EMPTY1, B_GFULL, B_PREADY, B_VSREADY, B_HREADY, B_YFULL, B_SFULL, B_SCAL, B_COUNT };
 
-// Sequence lengths need not be a multiple of the chunk: the tensor maps are [batch, step, column], so the rows of the last
-// chunk beyond the sequence are read as zeros (and not written), and their dt is zero, which makes them steps that neither
-// decay nor feed the state.  Arrays per step of the scratch are padded to LP = nc * 128 steps.
 struct WalkArgs {
   int B, L, H, G, nc;
-  const float* cum;        // [B, H, LP] inclusive prefix sums of dt*A inside each 128-step chunk
-  const float* dtt;        // [B, H, LP] dt
-  const float* colf;       // [B, H, LP] column factor of every step relative to the far end of its 8-step piece
+  const float* cum;        // [B, H, L] inclusive prefix sums of dt*A inside each 128-step chunk
+  const float* dtt;        // [B, H, L] dt
+  const float* colf;       // [B, H, L] column factor of every step relative to the far end of its 8-step piece
   __half* out;             // [B*L, H*64] or null
   const __half* z;         // dot partner, same indexing as out, or null
-  float* dot_out;          // [2][B, H, LP] row dots <z, out> from the fp32 accumulators, one array per half of the columns, or null
+  float* dot_out;          // [2][B, H, L] row dots <z, out> from the fp32 accumulators, one array per half of the columns, or null
   __half* hs_out;          // [B, H, nc][128][64]: state every chunk receives, or null
   float* carry;            // [B * H][128][64] fp32: state handed from the CTA that walked the first part of a sequence to the next
   int* carry_flag;         // [B * H]: number of worker warps (of 8) that have written their part of `carry`; zero before the launch
@@ -128,9 +125,9 @@ __device__ __forceinline__ bool walk_wait(uint64_t* bar, uint32_t parity, uint32
   return mbar_wait_abortable(bar, parity, status, abort);
 }
 
-// RAGGED: L is no multiple of the chunk (rows of z and out beyond it must not be touched).  DOT: the row dots <z, out> are wanted (the reverse pass); a template parameter, so that the forward pass does not
-// carry the registers of the dot partner's rows.
-template <int ANTI, bool DOT, bool RAGGED>
+// DOT: the row dots <z, out> are wanted (the reverse pass); a template parameter, so that the forward pass does not carry the
+// registers of the dot partner's rows.
+template <int ANTI, bool DOT>
 __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_constant__ CUtensorMap map_q,
                                                                const __grid_constant__ CUtensorMap map_k,
                                                                const __grid_constant__ CUtensorMap map_v,
@@ -472,9 +469,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_con
         if (DOT) {    // the dot partner's rows of chunk k, whole 64-byte row pieces per load
 #pragma unroll
           for (int it = 0; it < 4; ++it) {
-            int zt = c * WQ + quarter * 32 + it * 8 + (lane >> 2);
-            if (RAGGED) zt = min(zt, g.L - 1);   // the output rows beyond the sequence are zero: any row serves as their partner
-            const size_t zrow = static_cast<size_t>(b) * g.L + zt;
+            const size_t zrow = static_cast<size_t>(b) * g.L + c * WQ + quarter * 32 + it * 8 + (lane >> 2);
             zc[it] = *reinterpret_cast<const uint4*>(g.z + zrow * pitch + h * WP + ch * 32 + (lane & 3) * 8);
           }
         }
@@ -573,7 +568,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_con
             const int lr = quarter * 32 + it * 8 + (lane >> 2), cc = ch * 4 + (lane & 3);
             const uint4 val = *reinterpret_cast<const uint4*>(stg + lr * 128 + ((cc ^ (lr & 7)) << 4));
             const size_t orow = static_cast<size_t>(b) * g.L + c * WQ + lr;
-            if (!RAGGED || c * WQ + lr < g.L) *reinterpret_cast<uint4*>(g.out + orow * pitch + h * WP + cc * 8) = val;
+            *reinterpret_cast<uint4*>(g.out + orow * pitch + h * WP + cc * 8) = val;
           }
           __syncwarp();
         }
@@ -640,7 +635,7 @@ constexpr int WP2_THREADS = 32 * 20;   // warps 0-1 control (2-3 idle), warps 4-
                                        // of which the control warpgroup keeps 64 and the workers take 104 (128 * 64 + 512 * 104 = 640 * 96)
 enum { PB_FULL0 = 0, PB_FULL1, PB_EMPTY0, PB_EMPTY1, PB_VFULL, PB_GFULL, PB_PREADY, PB_VSREADY, PB_YFULL, PB_SFULL, PB_SCAL, PB_ZFULL, PB_COUNT };
 
-template <int ANTI, bool DOT, bool RAGGED>
+template <int ANTI, bool DOT>
 __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __grid_constant__ CUtensorMap map_q,
                                                                     const __grid_constant__ CUtensorMap map_k,
                                                                     const __grid_constant__ CUtensorMap map_v,
@@ -934,9 +929,8 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
           if (OUT) {
             fence_proxy_async_smem();
             __syncwarp();
-            const int row0 = c * WQ + quarter * 32;
-            if (lane == 0 && (!RAGGED || row0 < g.L)) {   // rows beyond the sequence are not written
-              tma_store_3d(&map_out, stage + (ch * 2 + half) * WP2_HALF + quarter * 32 * 64, h * WP + half * 32, row0, b);
+            if (lane == 0) {
+              tma_store_3d(&map_out, stage + (ch * 2 + half) * WP2_HALF + quarter * 32 * 64, h * WP + half * 32, c * WQ + quarter * 32, b);
               bulk_commit();
             }
           }
@@ -1110,7 +1104,7 @@ enum { GB_FULL0 = 0, GB_FULL1, GB_EMPTY0, GB_EMPTY1, GB_SC0, GB_SC1, GB_SCALED, 
 
 struct GroupArgs {
   int B, L, H, G, nc;
-  const float* cum; const float* dtt; const float* colf;   // [B, H, nc * 128], causal column factors
+  const float* cum; const float* dtt; const float* colf;   // [B, H, L], causal column factors
   uint32_t* status;
 };
 
@@ -1386,7 +1380,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_group_grads_kernel(const __g
 }
 
 // dt*A prefix sums inside every 128-step chunk, dt, and the column factors of both walk directions, all in
-// [B, H, nc * 128] order (steps beyond the sequence: dt = 0).  One CTA per (b, chunk, eight heads), one warp per head, four
+// [B, H, L] order.  One CTA per (b, chunk, eight heads), one warp per head, four
 // neighbouring steps per lane; dt comes in as rows of eight heads (one sector each) through shared memory, where one head per CTA
 // read a sector for every value.
 // Column factor of step t relative to the far end of its 8-step piece: causal exp(cum[t | 7] - cum[t]) dt[t], anti-causal
@@ -1407,13 +1401,13 @@ __global__ void __launch_bounds__(WS_THREADS) ssd_walk_cumsum_kernel(const float
   __shared__ float s_dt[WQ][WS_HEADS + 1];
   if (blockIdx.x == 0)   // the walks that follow in stream order hand states from CTA to CTA through these counters
     for (int i = threadIdx.x; i < n_flags; i += WS_THREADS) carry_flags[i] = 0;
-  const int nc = (L + WQ - 1) / WQ;
+  const int nc = L / WQ;
   const int h0 = static_cast<int>(blockIdx.x % hblocks) * WS_HEADS, bc = blockIdx.x / hblocks, c = bc % nc, b = bc / nc;
 #pragma unroll
   for (int k = 0; k < WQ * WS_HEADS / WS_THREADS; ++k) {
     const int idx = k * WS_THREADS + threadIdx.x, t = idx / WS_HEADS, h = h0 + idx % WS_HEADS;
     float d = 0.f;
-    if (c * WQ + t < L && h < H) {
+    if (h < H) {
       const size_t row = static_cast<size_t>(b) * L + c * WQ + t;
       if (RAW) {
         const float pre = __half2float(raw[row * raw_pitch + h]) + bias[h];
@@ -1494,8 +1488,8 @@ __device__ __forceinline__ float walk_sigmoid(float x) {
   return r;
 }
 struct ScalarArgs {
-  const float* u; const float* v;   // [2][B, H, nc * 128]: one array per half of the columns
-  const float* dtt;                 // [B, H, nc * 128]
+  const float* u; const float* v;   // [2][B, H, L]: one array per half of the columns
+  const float* dtt;                 // [B, H, L]
   const float* A;
   const float* pin;                 // [B, H, nc]: g_a just behind the chunk
   float* gdt;                       // [B, L, H]
@@ -1555,7 +1549,7 @@ __global__ void __launch_bounds__(WS_THREADS) ssd_walk_scalars_kernel(const Scal
     for (int e = 0; e < 4; ++e) {
       const int t = lane * 4 + e;
       const float ga = right + within[e] + resid * (static_cast<float>(WQ - t) / static_cast<float>(WQ));
-      if (c * WQ + t < g.L) ga_acc += dt[e] * ga;
+      ga_acc += dt[e] * ga;
       s_gd[t][w] = vt[e] / dt[e] + a_h * ga;
     }
     ga_acc = warp_reduce<SumOp>(ga_acc);
@@ -1566,7 +1560,7 @@ __global__ void __launch_bounds__(WS_THREADS) ssd_walk_scalars_kernel(const Scal
 #pragma unroll
   for (int k = 0; k < WQ * WS_HEADS / WS_THREADS; ++k) {
     const int idx = k * WS_THREADS + threadIdx.x, t = idx / WS_HEADS, hh = h0 + idx % WS_HEADS;
-    if (c * WQ + t < g.L && hh < g.H) {
+    if (hh < g.H) {
       const size_t row = static_cast<size_t>(b) * g.L + c * WQ + t;
       const float gd = s_gd[t][idx % WS_HEADS];
       g.gdt[row * g.H + hh] = gd;
@@ -1672,10 +1666,8 @@ extern "C" int mpSsdWalkPartition(int cta, int ncta, int nseq, int nc, int idx, 
 // ---------------------------------------------------------------------------
 // Interface to the launchers in ssd.cu.
 // ---------------------------------------------------------------------------
-// Sequences of less than 32 steps stay with the recurrence: A's gradient there is a difference of nearly equal row dots, of
-// which the walk's r16 score tile leaves too little.
 bool mp_ssd_walk_supported(int L, int H, int P, int N, int G) {
-  return P == WP && N == WN && L >= 32 && G > 0 && H % G == 0 && getenv("MP_SSD_NO_WALK") == nullptr;
+  return P == WP && N == WN && L % WQ == 0 && L > 0 && G > 0 && H % G == 0 && getenv("MP_SSD_NO_WALK") == nullptr;
 }
 
 static int walk_head_blocks(int H) { return (H + WS_HEADS - 1) / WS_HEADS; }
@@ -1683,7 +1675,7 @@ static int walk_head_blocks(int H) { return (H + WS_HEADS - 1) / WS_HEADS; }
 void mp_ssd_walk_cumsum(const float* dt, const float* A, float* cum, float* dtt, float* colf_c, float* colf_a, int B, int L, int H,
                         int* carry_flags, int n_flags, cudaStream_t st) {
   const int hb = walk_head_blocks(H);
-  MpLaunch(B * ((L + WQ - 1) / WQ) * hb, WS_THREADS, 0, st)(ssd_walk_cumsum_kernel<false>, dt, A, cum, dtt, colf_c, colf_a, L, H, hb, carry_flags, n_flags,
+  MpLaunch(B * (L / WQ) * hb, WS_THREADS, 0, st)(ssd_walk_cumsum_kernel<false>, dt, A, cum, dtt, colf_c, colf_a, L, H, hb, carry_flags, n_flags,
                                                             nullptr, 0, nullptr, nullptr, nullptr);
   MP_LAUNCH_CHECK();
 }
@@ -1692,7 +1684,7 @@ void mp_ssd_walk_cumsum(const float* dt, const float* A, float* cum, float* dtt,
 void mp_ssd_walk_cumsum_raw(const __half* raw, size_t raw_pitch, const float* bias, const float* A_log, float* dt_out, float* A_out, float* cum,
                             float* dtt, float* colf_c, int B, int L, int H, int* carry_flags, int n_flags, cudaStream_t st) {
   const int hb = walk_head_blocks(H);
-  MpLaunch(B * ((L + WQ - 1) / WQ) * hb, WS_THREADS, 0, st)(ssd_walk_cumsum_kernel<true>, nullptr, A_log, cum, dtt, colf_c, nullptr, L, H, hb, carry_flags,
+  MpLaunch(B * (L / WQ) * hb, WS_THREADS, 0, st)(ssd_walk_cumsum_kernel<true>, nullptr, A_log, cum, dtt, colf_c, nullptr, L, H, hb, carry_flags,
                                                             n_flags, raw, raw_pitch, bias, dt_out, A_out);
   MP_LAUNCH_CHECK();
 }
@@ -1704,7 +1696,7 @@ void mp_ssd_walk_scalars(const float* u, const float* v, const float* dtt, const
   ScalarArgs g;
   g.u = u; g.v = v; g.dtt = dtt; g.A = A; g.pin = pin; g.gdt = gdt; g.ga_part = ga_part; g.gb_part = gb_part;
   g.raw = raw; g.raw_pitch = raw_pitch; g.bias = bias; g.graw = graw; g.graw_pitch = graw_pitch;
-  g.B = B; g.L = L; g.H = H; g.nc = (L + WQ - 1) / WQ; g.hblocks = walk_head_blocks(H);
+  g.B = B; g.L = L; g.H = H; g.nc = L / WQ; g.hblocks = walk_head_blocks(H);
   const int grid = B * g.nc * g.hblocks;
   if (raw != nullptr) MpLaunch(grid, WS_THREADS, 0, st)(ssd_walk_scalars_kernel<true>, g);
   else MpLaunch(grid, WS_THREADS, 0, st)(ssd_walk_scalars_kernel<false>, g);
@@ -1713,13 +1705,13 @@ void mp_ssd_walk_scalars(const float* u, const float* v, const float* dtt, const
   MP_LAUNCH_CHECK();
 }
 
-// One walk.  q, k: [B*L, G*128]; v, z, out: [B*L, H*64]; cum, dtt, colf (of the walk's direction): [B, H, nc * 128] from mp_ssd_walk_cumsum.
+// One walk.  q, k: [B*L, G*128]; v, z, out: [B*L, H*64]; cum, dtt, colf (of the walk's direction): [B, H, L] from mp_ssd_walk_cumsum.
 void mp_ssd_walk(int anti, const __half* q, const __half* k, const __half* v, const float* cum, const float* dtt, const float* colf, __half* out,
                  const __half* z,
                  float* dot_out, __half* hs_out, float* carry, int* carry_flag, int max_ctas, int B, int L, int H, int G, uint32_t* status,
                  cudaStream_t st) {
   WalkArgs g;
-  g.B = B; g.L = L; g.H = H; g.G = G; g.nc = (L + WQ - 1) / WQ;
+  g.B = B; g.L = L; g.H = H; g.G = G; g.nc = L / WQ;
   g.cum = cum; g.dtt = dtt; g.colf = colf; g.out = out; g.z = z; g.dot_out = dot_out; g.hs_out = hs_out; g.status = status;
   g.carry = carry; g.carry_flag = carry_flag;
   // One CTA per SM slot it may use, every CTA the same number of chunks; never more CTAs than sequences, so that a CTA's
@@ -1751,12 +1743,10 @@ void mp_ssd_walk(int anti, const __half* q, const __half* k, const __half* v, co
   const bool dot = z != nullptr && dot_out != nullptr;
   if (!dot) { g.z = nullptr; g.dot_out = nullptr; }
   if (anti && !dot) MP_FATAL("ssd walk: the anti-causal form comes with its row dots");
-  const bool ragged = L % WQ != 0;
   auto form = [&](auto A, auto D) {
     constexpr int a = decltype(A)::value;
     constexpr bool d = decltype(D)::value;
-    if (ragged) launch(ssd_walk_kernel<a, d, true>, ssd_walk_pair_kernel<a, d, true>);
-    else launch(ssd_walk_kernel<a, d, false>, ssd_walk_pair_kernel<a, d, false>);
+    launch(ssd_walk_kernel<a, d>, ssd_walk_pair_kernel<a, d>);
   };
   using std::integral_constant;
   if (anti) form(integral_constant<int, 1>{}, std::true_type{});
@@ -1771,7 +1761,7 @@ void mp_ssd_group_grads(const __half* gy, const __half* x, const __half* Bm, con
                         const float* cum, const float* dtt, const float* colf_c, __half* gB, __half* gC, int B, int L,
                         int H, int G, uint32_t* status, cudaStream_t st) {
   GroupArgs g;
-  g.B = B; g.L = L; g.H = H; g.G = G; g.nc = (L + WQ - 1) / WQ;
+  g.B = B; g.L = L; g.H = H; g.G = G; g.nc = L / WQ;
   g.cum = cum; g.dtt = dtt; g.colf = colf_c; g.status = status;
   const size_t srows = static_cast<size_t>(B) * H * g.nc * WN;
   const CUtensorMap mgy = walk_map3(gy, B, L, static_cast<size_t>(H) * WP), mx = walk_map3(x, B, L, static_cast<size_t>(H) * WP);
