@@ -27,6 +27,7 @@
 #include "mp_tcgen05.cuh"
 
 #include <cuda.h>
+#include <initializer_list>
 #include <mutex>
 
 bool mp_ssd_walk_supported(int L, int H, int P, int N, int G);   // ssd_walk.cu
@@ -907,6 +908,12 @@ bool ssd_tensor_path(const SsdDims& d) {
   if (d.G <= 0 || d.H % d.G != 0) MP_FATAL("ssd_scan: heads %d not divisible by groups %d", d.H, d.G);
   return ssd_whole_chunks(d) && getenv("MP_SSD_FORCE_GENERIC") == nullptr;
 }
+// Their kernels move r16 tensors by TMA and in 16-byte pieces.  Checked before anything is launched: the walk of one head at a time stores
+// its output, and loads the partner of the row dots, without a tensor map whose encoding would refuse the pointer.
+void ssd_require_aligned(std::initializer_list<const void*> ptrs) {
+  for (const void* p : ptrs)
+    if (!mp_aligned16(p)) MP_FATAL("ssd_scan: whole chunks need 16-byte aligned r16 tensors");
+}
 bool ssd_segment_path(const SsdDims& d) {
   return !ssd_tensor_path(d) && mp_ssd_segments_supported(d.L, d.H, d.P, d.N, d.G) && getenv("MP_SSD_FORCE_GENERIC") == nullptr;
 }
@@ -1012,6 +1019,7 @@ extern "C" void launch_ssd_scan_r16(const void* x, const void* dt, const void* A
     return;
   }
   if (scratch == nullptr) MP_FATAL("ssd_scan: scratch must not be NULL");
+  ssd_require_aligned({x, Bm, Cm, y});
   MpStreamState* state = mp_state(ctx);
   cudaStream_t st = mp_stream(ctx);
   // The chunk walk (no chunk state in global memory) where it applies; MP_SSD_LEGACY_FORWARD selects the three-phase
@@ -1063,6 +1071,7 @@ extern "C" void launch_ssd_scan_raw_r16(const void* x, const void* dt_raw, len_t
   const SsdDims d = ssd_dims(batch, seqlen, heads, headdim, dstate, ngroups, chunk);
   if (ssd_tensor_path(d) && ssd_forward_walks(d)) {
     if (scratch == nullptr) MP_FATAL("ssd_scan_raw: scratch must not be NULL");
+    ssd_require_aligned({x, Bm, Cm, y});
     MpStreamState* state = mp_state(ctx);
     cudaStream_t st = mp_stream(ctx);
     const WalkScratch w = walk_carve(scratch, d, false, 0);
@@ -1126,6 +1135,7 @@ static bool ssd_scan_reverse_r16_impl(const void* x, const void* dt, const void*
     return false;
   }
   if (scratch == nullptr) MP_FATAL("ssd_scan_reverse: scratch must not be NULL");
+  ssd_require_aligned({x, Bm, Cm, gy, gx, gB, gC});
   MpStreamState* state = mp_state(ctx);
   cudaStream_t st = mp_stream(ctx);
   const __half* xh = static_cast<const __half*>(x);
