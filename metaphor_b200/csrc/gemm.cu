@@ -1002,6 +1002,10 @@ void gemm_dispatch(const void* a_, const void* b_, const void* bias, double alph
     const bool pad_a = !mp_aligned16(a) || a_pitch % 16 != 0, pad_b = !mp_aligned16(b) || b_pitch % 16 != 0;
     // a problem of one or two tiles is over on the FP pipe before the copy's launch has paid
     if (pad_a || pad_b) tensor_path = tensor_path && static_cast<double>(M) * N * K * batch > 1.0e6;
+    // r32 with a short K: the FP pipe's sum has seen few roundings, the split's own losses are larger.  2-norm of the error at [301, K, 307],
+    // FP pipe / split: normal operands K = 33 1.04e-7 / 1.32e-7, 53 1.32e-7 / 1.29e-7, 129 2.0e-7 / 1.4e-7; operands of one sign 65 1.23e-7 /
+    // 1.38e-7, 129 1.58e-7 / 1.35e-7.  (Up to there the FP pipe takes 13 us where the output is small; [4097, 63, 4099] 121 against 64 us.)
+    if (sizeof(T) == 4 && (pad_a || pad_b)) tensor_path = tensor_path && K >= 96;
     if (tensor_path) {
       GemmArgs args;
       args.bias = bias;

@@ -5,6 +5,14 @@
 // 1.5e-5 at K = 1001, growing with K).  The accumulator is therefore handed over every CHUNK_KB k-blocks (24 MMAs) to the
 // epilogue warps, which add it up in registers with rounding; two TMEM accumulators take turns.
 //
+// EXACT: problems that were summed on the FP pipe before (padded operands) keep its exactness.  What the form above loses there is
+// the product lo_a lo_b and lo's own last bits, both of which have the sign of a b when hi is x cut off (up to 2^-20 and 2^-21 of a
+// product), and the truncated additions.  So hi is x rounded to the nearest instead (lo takes both signs, the losses average out),
+// the small products of a k-block come before the large ones (only whose four additions then truncate at full size), and
+// every k-block is handed over.  2-norm of the error at [301, K, 307], normal operands, K = 65 / 1001 / 16385: FP pipe 1.5e-7 / 5.7e-7 /
+// 2.3e-6, this 1.3e-7 / 1.5e-7 / 1.9e-7, the form above 9.2e-7 throughout.  It costs the write of B's hi tile and twice the
+// hand-overs: 4096^3 719 instead of 659 us, [2000, 999, 1501] with its copies 73 instead of 68.
+//
 // What bounds the kernel is shared memory bandwidth: three MMAs on operands there read every tile three times, which at 128
 // columns takes as long as the MMAs themselves (126 of 128 bytes a cycle), and the split comes on top.  A is therefore kept in TMEM:
 // the split warps read its tile once and write the raw words (hi: the MMA ignores the low bits) and lo there with tcgen05.st, so
@@ -26,7 +34,7 @@ constexpr int R_UMMA_K = 8;
 constexpr int R_SPLIT_WARPS = 6, R_SPLIT_B_FIRST = 6, R_SPLIT_B_THREADS = 64, R_EPI_FIRST = 8, R_EPI_WARPS = 8;
 constexpr int R_SLOTS = 4, R_MAX_STAGES = 8;      // slots: split k-blocks (A in TMEM, lo tile of B in shared memory)
 constexpr int R_BOX_BYTES = 32 * 32 * 4;
-constexpr int CHUNK_KB = 2;           // k-blocks per TMEM accumulation
+template <bool EXACT> constexpr int CHUNK_KB = EXACT ? 1 : 2;   // k-blocks per TMEM accumulation
 
 template <int BN> struct R32Cfg {
   static constexpr int A_BYTES = BM * SWIZZLE_BYTES, B_BYTES = BN * SWIZZLE_BYTES;
@@ -55,7 +63,7 @@ __device__ __forceinline__ R32Unit r32_unit(const GemmArgs& g, int unit, int til
   return u;
 }
 
-template <int BN>
+template <int BN, bool EXACT>
 __global__ void __launch_bounds__(R_THREADS, 1) gemm_r32_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                                                                 const __grid_constant__ CUtensorMap tmap_c, const GemmArgs g) {
   using Cfg = R32Cfg<BN>;
@@ -142,12 +150,12 @@ __global__ void __launch_bounds__(R_THREADS, 1) gemm_r32_kernel(const __grid_con
     bool ok = true;
     for (int unit = worker; unit < num_units && ok; unit += workers) {
       const R32Unit u = r32_unit<BN>(g, unit, tiles_m, num_tiles, num_kb, kb_per);
-      for (int kb = u.kb0; kb < u.kb1 && ok; kb += CHUNK_KB, ++chunk) {
+      for (int kb = u.kb0; kb < u.kb1 && ok; kb += CHUNK_KB<EXACT>, ++chunk) {
         const uint32_t buf = chunk & 1u;
         ok = mbar_wait_abortable(acc_empty + buf, ((chunk >> 1) & 1u) ^ 1u, g.status, abort);
         ok = __all_sync(0xffffffffu, ok);
         const uint32_t acc = tmem_base + buf * BN;
-        const int kend = min(kb + CHUNK_KB, u.kb1);
+        const int kend = min(kb + CHUNK_KB<EXACT>, u.kb1);
         for (int k = kb; ok && k < kend; ++k, ++it) {
           const uint32_t l = it % R_SLOTS;
           ok = mbar_wait_abortable(ready + l, (it / R_SLOTS) & 1u, g.status, abort);
@@ -158,12 +166,22 @@ __global__ void __launch_bounds__(R_THREADS, 1) gemm_r32_kernel(const __grid_con
           const uint32_t ta = tmem_base + Cfg::TM_A + l * 64;
           const uint32_t first = k != kb ? 1u : 0u;
           if (elect_one()) {
+            if constexpr (EXACT) {   // one k-block per accumulation
 #pragma unroll
-            for (int ks = 0; ks < R_BK / R_UMMA_K; ++ks) {
-              umma_tf32_ta(acc, ta + ks * R_UMMA_K, bd + ks * kunits, idesc, ks != 0 ? 1u : first);
-              if (split) {
-                umma_tf32_ta(acc, ta + 32 + ks * R_UMMA_K, bd + ks * kunits, idesc, 1u);   // lo * hi
-                umma_tf32_ta(acc, ta + ks * R_UMMA_K, ld + ks * kunits, idesc, 1u);        // hi * lo
+              for (int ks = 0; ks < R_BK / R_UMMA_K; ++ks) {
+                umma_tf32_ta(acc, ta + 32 + ks * R_UMMA_K, bd + ks * kunits, idesc, ks != 0 ? 1u : 0u);   // lo * hi
+                umma_tf32_ta(acc, ta + ks * R_UMMA_K, ld + ks * kunits, idesc, 1u);                       // hi * lo
+              }
+#pragma unroll
+              for (int ks = 0; ks < R_BK / R_UMMA_K; ++ks) umma_tf32_ta(acc, ta + ks * R_UMMA_K, bd + ks * kunits, idesc, 1u);
+            } else {
+#pragma unroll
+              for (int ks = 0; ks < R_BK / R_UMMA_K; ++ks) {
+                umma_tf32_ta(acc, ta + ks * R_UMMA_K, bd + ks * kunits, idesc, ks != 0 ? 1u : first);
+                if (split) {
+                  umma_tf32_ta(acc, ta + 32 + ks * R_UMMA_K, bd + ks * kunits, idesc, 1u);   // lo * hi
+                  umma_tf32_ta(acc, ta + ks * R_UMMA_K, ld + ks * kunits, idesc, 1u);        // hi * lo
+                }
               }
             }
             umma_commit(raw_empty + s);
@@ -181,7 +199,9 @@ __global__ void __launch_bounds__(R_THREADS, 1) gemm_r32_kernel(const __grid_con
     const bool does_b = warp >= R_SPLIT_B_FIRST;
     const int tb = threadIdx.x - 32 * R_SPLIT_B_FIRST;
     const int quarter = warp & 3, arow = quarter * 32 + lane;
-    auto low = [](uint32_t v) { return __float_as_uint(__uint_as_float(v) - __uint_as_float(v & 0xFFFFE000u)); };
+    // hi in its 19 high bits.  A NaN may lose its own (rounding can carry out of the exponent), lo = NaN - hi remains one.
+    auto high = [](uint32_t v) { return (EXACT ? v + 0x1000u : v) & 0xFFFFE000u; };
+    auto low = [&](uint32_t v) { return __float_as_uint(__uint_as_float(v) - __uint_as_float(high(v))); };
     // k-blocks that this CTA splits, over all of its units (they run through the rings without a break)
     uint32_t total = 0;
     for (int unit = worker; unit < num_units; unit += workers) {
@@ -203,7 +223,7 @@ __global__ void __launch_bounds__(R_THREADS, 1) gemm_r32_kernel(const __grid_con
     if (does_b) {
       for (uint32_t it = 0; it < total; ++it, advance()) {
         if (!blocking(it)) break;
-        const unsigned char* src = smem + s * RAW + A_BYTES;
+        unsigned char* src = smem + s * RAW + A_BYTES;
         unsigned char* dst = lo_ring + (it % R_SLOTS) * B_BYTES;
         constexpr int STEP = R_SPLIT_B_THREADS * 16, BATCH = 8;
 #pragma unroll
@@ -212,10 +232,12 @@ __global__ void __launch_bounds__(R_THREADS, 1) gemm_r32_kernel(const __grid_con
 #pragma unroll
           for (int e = 0; e < BATCH; ++e) v[e] = *reinterpret_cast<const uint4*>(src + base + e * STEP + tb * 16);
 #pragma unroll
-          for (int e = 0; e < BATCH; ++e)
+          for (int e = 0; e < BATCH; ++e) {
             *reinterpret_cast<uint4*>(dst + base + e * STEP + tb * 16) = make_uint4(low(v[e].x), low(v[e].y), low(v[e].z), low(v[e].w));
+            if (EXACT) *reinterpret_cast<uint4*>(src + base + e * STEP + tb * 16) = make_uint4(high(v[e].x), high(v[e].y), high(v[e].z), high(v[e].w));
+          }
         }
-        fence_proxy_async_smem();   // the tensor core reads the lo tile through the async proxy
+        fence_proxy_async_smem();   // the tensor core reads the tiles through the async proxy
         arrive(it);
       }
     } else if (total > 0) {
@@ -242,7 +264,13 @@ __global__ void __launch_bounds__(R_THREADS, 1) gemm_r32_kernel(const __grid_con
       for (uint32_t it = 0; ok && it < total; ++it) {
         tcgen05_fence_after_sync();
         const uint32_t ta = tmem_base + Cfg::TM_A + (it % R_SLOTS) * 64 + (static_cast<uint32_t>(quarter * 32) << 16);
-        tmem_st_32x32(ta, v);
+        if constexpr (EXACT) {
+#pragma unroll
+          for (int k = 0; k < 32; ++k) w[k] = high(v[k]);
+          tmem_st_32x32(ta, w);
+        } else {
+          tmem_st_32x32(ta, v);   // the MMA ignores the low bits
+        }
 #pragma unroll
         for (int k = 0; k < 32; ++k) v[k] = low(v[k]);
         tmem_st_32x32(ta + 32, v);
@@ -279,7 +307,7 @@ __global__ void __launch_bounds__(R_THREADS, 1) gemm_r32_kernel(const __grid_con
       for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
         for (int j = 0; j < 32; ++j) acc[nb][j] = 0.f;
-      for (int kb = u.kb0; kb < u.kb1; kb += CHUNK_KB, ++chunk) {
+      for (int kb = u.kb0; kb < u.kb1; kb += CHUNK_KB<EXACT>, ++chunk) {
         const uint32_t buf = chunk & 1u;
         ok = mbar_wait_abortable(acc_full + buf, (chunk >> 1) & 1u, g.status, abort);
         ok = __all_sync(0xffffffffu, ok);   // tcgen05.ld is warp-collective
@@ -364,7 +392,7 @@ __global__ void __launch_bounds__(R_THREADS, 1) gemm_r32_kernel(const __grid_con
   if (warp == 1) tmem_dealloc(tmem_base, Cfg::TM_COLS);
 }
 
-template <int BN>
+template <int BN, bool EXACT>
 void launch_r32(Operand<float> a, Operand<float> b, const GemmArgs& g, int sms, cudaStream_t st) {
   using Cfg = R32Cfg<BN>;
   const size_t nb = static_cast<size_t>(g.batch);
@@ -372,9 +400,9 @@ void launch_r32(Operand<float> a, Operand<float> b, const GemmArgs& g, int sms, 
   const CUtensorMap tb = g.b_mn ? make_map<float>(b.p, g.K, g.N, b.ld, R_BK, R_BK, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B, nb) : make_map<float>(b.p, g.N, g.K, b.ld, R_BK, BN, CU_TENSOR_MAP_SWIZZLE_128B, nb);
   CUtensorMap tc = ta;
   if ((g.ldc * sizeof(float)) % 16 == 0 && mp_aligned16(g.c)) tc = make_store_map<float>(g.c, g.M, g.N, g.ldc, false, nb);
-  MP_CUDA_CHECK(cudaFuncSetAttribute(gemm_r32_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM));
+  MP_CUDA_CHECK(cudaFuncSetAttribute(gemm_r32_kernel<BN, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM));
   const long units = static_cast<long>((g.N + BN - 1) / BN) * ((g.M + BM - 1) / BM) * g.ksplit * g.batch;
-  MpLaunch(static_cast<unsigned>(units < sms ? units : sms), R_THREADS, Cfg::SMEM, st)(gemm_r32_kernel<BN>, ta, tb, tc, g);
+  MpLaunch(static_cast<unsigned>(units < sms ? units : sms), R_THREADS, Cfg::SMEM, st)(gemm_r32_kernel<BN, EXACT>, ta, tb, tc, g);
   MP_LAUNCH_CHECK();
   if (g.ksplit > 1) launch_fold<float>(g, st);
 }
@@ -398,12 +426,16 @@ void gemm_run_r32(Operand<float> a, Operand<float> b, GemmArgs args, int sms, vo
     const long n_tiles = static_cast<long>((args.M + BM - 1) / BM) * ((args.N + width - 1) / width) * args.batch;
     for (int ks = 1; ks <= (may_split ? 32 : 1); ++ks) {
       const long per = (num_kb + ks - 1) / ks;
-      if (ks > 1 && (per < CHUNK_KB || (ks - 1) * per >= num_kb || ks * mn_bytes > static_cast<double>(workspace_bytes))) continue;
+      if (ks > 1 && (per < 2 || (ks - 1) * per >= num_kb || ks * mn_bytes > static_cast<double>(workspace_bytes))) continue;
       double cost = static_cast<double>((n_tiles * ks + sms - 1) / sms) * (per * cycles + 3000.0);
       if (ks > 1) cost += 5000.0 + 2.0 * ks * mn_bytes / 3500.0;   // the fold's launch; partials out and in at 3.5 KB a cycle
       if (cost < best) { best = cost; bn = width; args.ksplit = ks; }
     }
   }
-  if (bn == 128) launch_r32<128>(a, b, args, sms, st);
-  else launch_r32<64>(a, b, args, sms, st);
+  const bool exact = args.exact != 0 && args.split != 0;
+  if (bn == 128) {
+    if (exact) launch_r32<128, true>(a, b, args, sms, st); else launch_r32<128, false>(a, b, args, sms, st);
+  } else {
+    if (exact) launch_r32<64, true>(a, b, args, sms, st); else launch_r32<64, false>(a, b, args, sms, st);
+  }
 }

@@ -16,7 +16,7 @@ struct GemmArgs {
   int M, N, K;
   int a_mn, b_mn;     // operand major-ness: 0 = K contiguous, 1 = M resp. N contiguous
   int stages;
-  int exact = 0;      // r16: sum with rounding between chunks of K where the single-CTA kernel runs
+  int exact = 0;      // sum as exactly as the FP pipe does (the EXACT forms of the kernels)
   int epi_boxes = 2;  // pair kernel: 64-column staging boxes per epilogue warp
   int split;          // r32 only: 1 = error-compensated hi/lo split (3 MMAs per k-slice), 0 = one tf32 MMA (for timing)
   int ksplit;         // > 1: the K range of every tile is cut into ksplit work units whose raw fp32

@@ -194,3 +194,26 @@ def test_unaligned_operands(mp, stream, sfx, shape, variant):
         run(mp, stream, "linear_ij_jk_ik_ik", sfx, a, b, c0, 1.0, c, 0.0, *dims)
         assert float((c.double()[0] - ref - c0.double()[0]).abs().max() / ref.abs().max()) <= TOL_RED[sfx]
     assert stream.status() == 0
+
+
+# Contractions of unaligned r32 operands are as exact as sums of K fused multiply-adds.  The bound is that of such a sum of random
+# signs, 2^-24 sqrt(K / 2) of the result's norm at most (its roundings are half an ulp at most, and grow with the partial sums), but at
+# least 2.2e-7: two roundings of the operands' splits and the four truncated additions of a k-block.  K: below and at the line to the
+# tensor cores, one k-block and one value more, chunks of one block with a remainder, a split of K.
+@pytest.mark.parametrize("shape", [(301, 33, 307), (301, 95, 307), (301, 97, 307), (301, 129, 307), (2001, 999, 1501), (131, 4097, 127), (129, 16385, 67)])
+@pytest.mark.parametrize("variant", ["ij_jk_ik", "ij_kj_ik", "ji_jk_ik"])
+@pytest.mark.parametrize("positive", [False, True])
+def test_unaligned_r32_keeps_fp32_sums(mp, stream, shape, variant, positive):
+    import torch
+    m, n, k = shape
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    a = torch.randn(*((n, m) if variant[0] == "j" else (m, n)), generator=g, device="cuda")
+    b = torch.randn(*((k, n) if variant[3:5] == "kj" else (n, k)), generator=g, device="cuda")
+    if positive:
+        a, b = a.abs(), b.abs()
+    c = torch.empty(m, k, device="cuda")
+    run(mp, stream, "inner_product_" + variant, "r32", a, b, 1.0, c, 0.0, m, n, k)
+    ref = (a.double().t() if variant[0] == "j" else a.double()) @ (b.double().t() if variant[3:5] == "kj" else b.double())
+    err = float((c.double() - ref).norm() / ref.norm())
+    assert err <= max(2.2e-7, 2.0 ** -24 * (n / 2) ** 0.5), err
+    assert stream.status() == 0
