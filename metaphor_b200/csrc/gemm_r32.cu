@@ -347,6 +347,23 @@ __global__ void __launch_bounds__(R_THREADS, 1) gemm_r32_kernel(const __grid_con
             }
           } else {
             const bool by_rows = !use_tma && !(vec_ok && col0 + 32 <= g.N);
+            if constexpr (EXACT) {
+              bool nan = false;
+#pragma unroll
+              for (int j = 0; j < 32; ++j) nan = nan || r[j] != r[j];
+              if (__any_sync(0xffffffffu, nan)) {   // rare; the block goes through the staging, so that its elements can be walked by index
+                if (lane == 0) bulk_wait_read<0>();
+                __syncwarp();
+#pragma unroll
+                for (int j = 0; j < 32; ++j) stage[j * 32 + lane] = r[j];
+#pragma unroll 1
+                for (int j = 0; j < 32; ++j)
+                  if (row < g.M && col0 + j < g.N && stage[j * 32 + lane] != stage[j * 32 + lane]) stage[j * 32 + lane] = dot_again(g, u.bz, row, col0 + j);
+#pragma unroll
+                for (int j = 0; j < 32; ++j) r[j] = stage[j * 32 + lane];
+                __syncwarp();
+              }
+            }
 #pragma unroll
             for (int j = 0; j < 32; ++j) r[j] *= g.alpha;
             if (bias != nullptr && (g.bias_pitch == 0 || (row < g.M && !by_rows))) {
@@ -433,6 +450,7 @@ void gemm_run_r32(Operand<float> a, Operand<float> b, GemmArgs args, int sms, vo
     }
   }
   const bool exact = args.exact != 0 && args.split != 0;
+  if (exact) { args.a_raw = a.p; args.a_ld = a.ld; args.b_raw = b.p; args.b_ld = b.ld; }
   if (bn == 128) {
     if (exact) launch_r32<128, true>(a, b, args, sms, st); else launch_r32<128, false>(a, b, args, sms, st);
   } else {

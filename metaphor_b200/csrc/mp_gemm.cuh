@@ -17,6 +17,9 @@ struct GemmArgs {
   int a_mn, b_mn;     // operand major-ness: 0 = K contiguous, 1 = M resp. N contiguous
   int stages;
   int exact = 0;      // sum as exactly as the FP pipe does (the EXACT forms of the kernels)
+  const float* a_raw = nullptr;   // EXACT r32: the operands, for results that come out as NaN (see dot_again); row pitches
+  const float* b_raw = nullptr;
+  size_t a_ld, b_ld;
   int epi_boxes = 2;  // pair kernel: 64-column staging boxes per epilogue warp
   int split;          // r32 only: 1 = error-compensated hi/lo split (3 MMAs per k-slice), 0 = one tf32 MMA (for timing)
   int ksplit;         // > 1: the K range of every tile is cut into ksplit work units whose raw fp32
@@ -56,11 +59,32 @@ __device__ __forceinline__ void store_block_rows(float* stage, const float* r, i
   __syncwarp();
 }
 
+// An operand split into hi + lo makes a NaN of every infinite value (lo = inf - inf) and of values that round up to infinity, and with it
+// of every result they enter.  A result that comes out as NaN is therefore summed once more from the operands themselves, by fused
+// multiply-adds in the order of K: infinities and overflows come out as the FP pipe has them, and what is NaN there remains one.
+__device__ __noinline__ float dot_again(const float* a, size_t a_step, const float* b, size_t b_step, int k) {
+  float s = 0.f;
+#pragma unroll 4
+  for (; k > 0; --k) {
+    s = fmaf(*a, *b, s);
+    if (s != s) break;
+    a += a_step;
+    b += b_step;
+  }
+  return s;
+}
+__device__ __forceinline__ float dot_again(const GemmArgs& g, int bz, int row, int col) {
+  const float* a = g.a_raw + static_cast<size_t>(bz) * (g.a_mn ? g.K : g.M) * g.a_ld + (g.a_mn ? row : row * g.a_ld);
+  const float* b = g.b_raw + static_cast<size_t>(bz) * (g.b_mn ? g.K : g.N) * g.b_ld + (g.b_mn ? col : col * g.b_ld);
+  return dot_again(a, g.a_mn ? g.a_ld : 1, b, g.b_mn ? g.b_ld : 1, g.K);
+}
+
 // C = alpha * sum_s partial[s] + bias + beta * C  (finishes a split-K contraction).  A thread folds four neighbouring columns
 // of a row; partial rows have a pitch of whole fours whatever N is.
 template <typename T>
 __global__ void __launch_bounds__(256) gemm_fold_kernel(const float* __restrict__ partial, int ksplit, int M, int N, int ld, float alpha,
-                                                        const T* __restrict__ bias, float beta, T* c, size_t ldc, size_t bias_pitch) {
+                                                        const T* __restrict__ bias, float beta, T* c, size_t ldc, size_t bias_pitch,
+                                                        const GemmArgs g) {
   mp_grid_dependency();
   const size_t mn = static_cast<size_t>(M) * ld;
   const size_t i0 = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) * 4;
@@ -80,6 +104,7 @@ __global__ void __launch_bounds__(256) gemm_fold_kernel(const float* __restrict_
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
     if (col + e < N) {
+      if (sizeof(T) == 4 && g.a_raw != nullptr && acc[e] != acc[e]) acc[e] = dot_again(g, 0, static_cast<int>(row), col + e);
       float o = alpha * acc[e];
       if (br != nullptr) o += mp_up(br[e]);
       if (beta != 0.0f) o += beta * mp_up(cr[e]);
@@ -159,7 +184,7 @@ void launch_fold(const GemmArgs& args, cudaStream_t st) {
   const size_t units = static_cast<size_t>(args.M) * args.partial_ld / 4;
   MpLaunch(static_cast<unsigned>((units + 255) / 256), 256, 0, st)(gemm_fold_kernel<T>, args.partial, args.ksplit, args.M, args.N, args.partial_ld,
                                                                                 args.alpha, static_cast<const T*>(args.bias), args.beta,
-                                                                                static_cast<T*>(args.c), args.ldc, args.bias_pitch);
+                                                                                static_cast<T*>(args.c), args.ldc, args.bias_pitch, args);
   MP_LAUNCH_CHECK();
 }
 

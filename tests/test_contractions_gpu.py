@@ -217,3 +217,52 @@ def test_unaligned_r32_keeps_fp32_sums(mp, stream, shape, variant, positive):
     err = float((c.double() - ref).norm() / ref.norm())
     assert err <= max(2.2e-7, 2.0 ** -24 * (n / 2) ** 0.5), err
     assert stream.status() == 0
+
+
+# Infinite and overflowing r32 operands off the 16-byte boundary: one infinity in each operand (meeting zeros, values that the split's high
+# part holds whole, and each other), a NaN, the largest float (which rounds up to infinity in 11 bits) and results beyond it.
+# One k-block, several, a split of K, a batch; bias, matrix term and the old C on top.
+@pytest.mark.parametrize("shape", [(1, 131, 97, 133), (1, 301, 999, 307), (1, 67, 16385, 67), (3, 131, 101, 99)])
+@pytest.mark.parametrize("variant", ["ij_jk_ik", "ij_kj_ik", "ji_jk_ik"])
+def test_unaligned_r32_not_finite(mp, stream, shape, variant):
+    import torch
+    nb, m, n, k = shape
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    a, b = torch.randn(nb, m, n, generator=g, device="cuda"), torch.randn(nb, n, k, generator=g, device="cuda")
+    inf, big = float("inf"), torch.finfo(torch.float32).max
+    a[0, 3, 5], b[0, 5, 7], b[0, 5, 9], b[0, 5, 10] = inf, 0.0, 1.0, -0.5
+    b[-1, n - 1, 20] = -inf
+    a[-1, 40, n - 1], a[-1, 41, n - 1] = 0.0, 2.0
+    a[0, 66, 11] = float("nan")
+    a[0, 50], a[0, 50, 2], b[0, 2, 30], b[0, 2, 31] = 0.0, big, 0.5, 4.0
+    ta, tb = variant[0] == "j", variant[3:5] == "kj"
+    da, db = (a.transpose(1, 2) if ta else a).contiguous(), (b.transpose(1, 2) if tb else b).contiguous()
+    name = "inner_product_" + ("_".join("b" + p for p in variant.split("_")) if nb > 1 else variant)
+    dims = (nb, m, n, k) if nb > 1 else (m, n, k)
+    # products and sums in r64, and what of it is beyond r32; no sum here comes near the limit without being far beyond it
+    ref = (a.double() @ b.double()).float()
+    scale = torch.where(torch.isfinite(ref), ref, torch.zeros_like(ref))
+    scale[0, 50] = 0
+
+    def check(c, want, what):
+        assert torch.equal(torch.isnan(c), torch.isnan(want)), what
+        sel = torch.isinf(want) | torch.isinf(c)
+        assert torch.equal(c[sel], want[sel]), what
+        fin = torch.isfinite(want)
+        assert float((c - want)[fin].abs().max() / want[fin].abs().max()) <= 1e-5, what
+        fin[0, 50] = False      # (the row with the largest float: the others are small against it)
+        assert float((c - want)[fin].abs().max() / scale.abs().max()) <= 1e-5, what
+
+    c = torch.full((nb, m, k), 3.0, device="cuda")
+    run(mp, stream, name, "r32", da, db, 1.0, c, 0.0, *dims)
+    check(c, ref, "plain")
+    c = torch.full((nb, m, k), 3.0, device="cuda")
+    run(mp, stream, name, "r32", da, db, 0.5, c, 1.0, *dims)
+    check(c, 0.5 * ref + 3.0, "beta")
+    if nb == 1 and variant == "ij_jk_ik":
+        bias, mat = torch.randn(k, device="cuda"), torch.randn(m, k, device="cuda")
+        run(mp, stream, "linear_ij_jk_ik", "r32", da, db, bias, 1.0, c, 0.0, *dims)
+        check(c, ref + bias, "bias")
+        run(mp, stream, "linear_ij_jk_ik_ik", "r32", da, db, mat, 1.0, c, 0.0, *dims)
+        check(c, ref + mat, "matrix")
+    assert stream.status() == 0
