@@ -119,8 +119,10 @@ template <int BN> constexpr int stage_bytes() { return BM * SWIZZLE_BYTES + BN *
 //               32x32 blocks go registers -> shared staging -> TMA store (coalesced, edge-clipped)
 //
 // EXACT: the tensor core's fp32 accumulation truncates, which drifts by up to 2^-24 of the sum per MMA.  Problems that were
-// summed on the FP pipe before (padded operands) keep its exactness where they are small enough for the single-CTA kernel: the
-// accumulator is handed over every CHUNK_KB k-blocks (8 MMAs) and added up in the epilogue warps' registers with rounding.
+// summed on the FP pipe before (padded operands) keep its exactness: the accumulator is handed over every CHUNK_KB k-blocks
+// (8 MMAs) and added up in the epilogue warps' registers with rounding.  That leaves the pair kernel out.  Results that are not the r16
+// nearest to the exact sum, operands of one sign, [5001, 4097, 5001]: 0.1 % on the FP pipe, 0.07 % here, 3.4 % with the pair kernel; times
+// 9 733, 431 and 317 us.
 constexpr int CHUNK_KB = 2;
 template <int BN, bool EXACT>
 __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
@@ -826,7 +828,7 @@ void pick_split_k(GemmArgs& args, int sms, size_t workspace_bytes, int* bn_io) {
   const int bns[2] = {128, 256};
   for (int bi = 0; bi < 2; ++bi) {
     const int bn = bns[bi];
-    if (bn == 256 && args.N <= 128) continue;
+    if (bn == 256 && (args.N <= 128 || args.exact)) continue;
     for (int ks = 2; ks <= 16; ++ks) {
       if (static_cast<double>(ks) * mn_bytes > static_cast<double>(workspace_bytes)) break;
       if (num_kb / ks < 8) break;
@@ -843,6 +845,7 @@ void pick_split_k(GemmArgs& args, int sms, size_t workspace_bytes, int* bn_io) {
 void gemm_run_r16(Operand<__half> a, Operand<__half> b, GemmArgs args, int sms, void* workspace, size_t workspace_bytes, cudaStream_t st) {
   args.partial_ld = (args.N + 3) & ~3;
   int bn = pick_bn(args.M, args.N, sms, args.batch);
+  if (args.exact && bn == 256) bn = 128;   // the widest tile whose sums the epilogue warps can hold
   args.ksplit = 1;
   args.partial = static_cast<float*>(workspace);
   if (args.batch == 1 && !env_flag("MP_GEMM_NO_SPLITK")) pick_split_k(args, sms, workspace_bytes, &bn);
@@ -853,9 +856,9 @@ void gemm_run_r16(Operand<__half> a, Operand<__half> b, GemmArgs args, int sms, 
     if (s > MAX_STAGES) s = MAX_STAGES;
     return s < 2 ? 2 : s;
   };
-  // CTA pairs for wide problems with enough 256 x 256 tiles to fill the pairs
+  // CTA pairs for wide problems with enough 256 x 256 tiles to fill the pairs (their accumulators are handed over once per tile: not EXACT)
   const long pair_tiles = static_cast<long>((args.M + 255) / 256) * ((args.N + 255) / 256);
-  if (args.batch == 1 && !env_flag("MP_GEMM_NO_PAIRS") && args.M >= 256 && args.N >= 256) {
+  if (args.batch == 1 && !args.exact && !env_flag("MP_GEMM_NO_PAIRS") && args.M >= 256 && args.N >= 256) {
     if (args.ksplit == 1 && bn == 256 && pair_tiles >= sms / 2) {
       launch_pair(a, b, args, sms, st);
       return;
@@ -879,7 +882,6 @@ void gemm_run_r16(Operand<__half> a, Operand<__half> b, GemmArgs args, int sms, 
       }
     }
   }
-  if (bn == 256 && args.exact) bn = 128;
   if (bn == 256) {
     args.stages = stages_for(stage_bytes<256>());
     launch_tc<256, false>(a, b, args, sms, st);

@@ -266,3 +266,20 @@ def test_unaligned_r32_not_finite(mp, stream, shape, variant):
         run(mp, stream, "linear_ij_jk_ik_ik", "r32", da, db, mat, 1.0, c, 0.0, *dims)
         check(c, ref + mat, "matrix")
     assert stream.status() == 0
+
+
+# r16 operands off the 16-byte boundary, of one sign, so that truncated additions do not cancel: enough 256 x 256 tiles for CTA pairs, a
+# long K in few tiles, and one tile.  A sum that is off by at most 8 x 2^-24 of itself (the additions of one hand-over) comes to lie beyond
+# the middle between two r16 values, which are 2^-11 to 2^-10 apart, in at most 8 x 2^-13 = 1e-3 of all cases; the fp32 additions of the
+# hand-overs may add as much.
+@pytest.mark.parametrize("shape", [(2571, 2049, 1993), (301, 4097, 307), (101, 513, 99)])
+def test_unaligned_r16_keeps_fp32_sums(mp, stream, shape):
+    import torch
+    m, n, k = shape
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    a, b = (torch.randn(*s, generator=g, device="cuda").abs().half() for s in ((m, n), (n, k)))
+    c = torch.empty(m, k, device="cuda", dtype=torch.float16)
+    run(mp, stream, "inner_product_ij_jk_ik", "r16", a, b, 2.0 ** -6, c, 0.0, m, n, k)
+    ref = (a.double() @ b.double()) * 2.0 ** -6
+    assert float((c != ref.half()).double().mean()) <= 2e-3
+    assert stream.status() == 0
