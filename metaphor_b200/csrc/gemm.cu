@@ -18,7 +18,7 @@
 // operand's major-ness.  r32 has a kernel of its own (gemm_r32.cu: three tf32 MMAs per
 // product on an error-compensated split).  Operands TMA cannot address
 // (row pitch not a multiple of 16 bytes) are copied into aligned rows first; r64 and
-// the smallest of those problems use an FP-pipe tile kernel.
+// those of them with a short K use an FP-pipe tile kernel.
 #include "mp_gemm.cuh"
 
 namespace {
@@ -1002,12 +1002,17 @@ void gemm_dispatch(const void* a_, const void* b_, const void* bias, double alph
     // TMA needs 16-byte aligned bases, row pitches and batch pitches
     const size_t a_pitch = (a_mn ? M : K) * sizeof(T), b_pitch = (b_mn ? N : K) * sizeof(T);
     const bool pad_a = !mp_aligned16(a) || a_pitch % 16 != 0, pad_b = !mp_aligned16(b) || b_pitch % 16 != 0;
-    // a problem of one or two tiles is over on the FP pipe before the copy's launch has paid
-    if (pad_a || pad_b) tensor_path = tensor_path && static_cast<double>(M) * N * K * batch > 1.0e6;
-    // r32 with a short K: the FP pipe's sum has seen few roundings, the split's own losses are larger.  2-norm of the error at [301, K, 307],
-    // FP pipe / split: normal operands K = 33 1.04e-7 / 1.32e-7, 53 1.32e-7 / 1.29e-7, 129 2.0e-7 / 1.4e-7; operands of one sign 65 1.23e-7 /
-    // 1.38e-7, 129 1.58e-7 / 1.35e-7.  (Up to there the FP pipe takes 13 us where the output is small; [4097, 63, 4099] 121 against 64 us.)
-    if (sizeof(T) == 4 && (pad_a || pad_b)) tensor_path = tensor_path && K >= 96;
+    if (pad_a || pad_b) {
+      // r16: the copies, the launch and a tile's way through TMEM take 8 - 12 us whatever the size.  The FP pipe takes 2.4 us and 0.11 us per step of
+      // K where the output is small, and 16 TFLOP/s where it is not; with few steps of K it is bound by the output.  FP pipe / tensor cores in
+      // us: [9, 301, 9] 35 / 9.5, [65, 65, 65] 10.9 / 9.2, [257, 17, 257] 5.8 / 11.4, [1001, 33, 1003] 10.4 / 12.3, [1501, 33, 1503] 15.6 / 13.3,
+      // [2001, 17, 2003] 18 / 20, [3001, 9, 3003] 25 / 32.
+      // r32: with a short K the FP pipe's sum has seen few roundings, the split's own losses are larger.  2-norm of the error at [301, K, 307],
+      // FP pipe / split: normal operands K = 33 1.04e-7 / 1.32e-7, 53 1.32e-7 / 1.29e-7, 129 2.0e-7 / 1.4e-7; operands of one sign 65 1.23e-7 /
+      // 1.38e-7, 129 1.58e-7 / 1.35e-7.  (Up to there the FP pipe takes 13 us where the output is small; [4097, 63, 4099] 121 against 64 us.)
+      const double volume = static_cast<double>(M) * N * K * batch;
+      tensor_path = tensor_path && (sizeof(T) == 4 ? K >= 96 : K >= 64 || (K >= 16 && volume > 6.0e7));
+    }
     if (tensor_path) {
       GemmArgs args;
       args.bias = bias;

@@ -155,7 +155,10 @@ def test_large_shape_against_float64_matmul(mp, stream, sfx):
 # (partial rows padded to four columns), odd batch entries, and copies beyond the workspace (worked off in slabs of rows, of
 # columns, of batch entries).
 ODD_SHAPES = [(1, 101, 103, 107), (1, 257, 65, 515), (1, 2571, 77, 1993), (1, 255, 4099, 130), (1, 130, 4098, 131), (7, 101, 99, 63),
-              (1, 16411, 1101, 67), (1, 67, 1101, 16411), (90, 513, 301, 515)]
+              (1, 16411, 1101, 67), (1, 67, 1101, 16411), (90, 513, 301, 515),
+              # a single result, rows and columns of one, both sides of the lines to the tensor cores (K of 16, 64 and 96, volume of 6e7)
+              (1, 1, 97, 1), (1, 2, 131, 1), (5, 3, 99, 2), (1, 1, 4099, 1), (1, 33, 63, 35), (1, 33, 65, 35), (1, 2001, 15, 2003), (1, 2001, 17, 2003),
+              (1, 1001, 95, 33)]
 
 
 @pytest.mark.parametrize("sfx", ["r16", "r32"])
