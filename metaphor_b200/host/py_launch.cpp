@@ -162,16 +162,35 @@ PyObject* py_launch(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject
   return PyObject_Vectorcall(g_fallback, args, nargs, kwnames);
 }
 
-bool to_pointers(PyObject* seq, std::vector<void*>& out) {
+// An operand of a chain: something with a `data_ptr` method (an AttributeError is raised for anything else), or None where there may be
+// no tensor.  The kernels write through these pointers, so nothing else stands for an address here.
+bool chain_pointer(PyObject* o, bool optional, void** out) {
+  if (o == Py_None && optional) { *out = nullptr; return true; }
+  const bool tensor = Py_TYPE(o) == g_tensor || PyType_IsSubtype(Py_TYPE(o), g_tensor);
+  PyObject* v = tensor ? PyObject_CallOneArg(g_data_ptr, o) : PyObject_CallMethod(o, "data_ptr", nullptr);
+  if (v == nullptr) return false;
+  *out = PyLong_AsVoidPtr(v);
+  Py_DECREF(v);
+  return PyErr_Occurred() == nullptr;
+}
+
+bool chain_pointers(PyObject* seq, bool optional, std::vector<void*>& out) {
   PyObject* fast = PySequence_Fast(seq, "a list of tensors is expected");
   if (fast == nullptr) return false;
   const Py_ssize_t n = PySequence_Fast_GET_SIZE(fast);
   out.resize(static_cast<size_t>(n));
   bool ok = true;
-  for (Py_ssize_t i = 0; ok && i < n; ++i) ok = to_pointer(PySequence_Fast_GET_ITEM(fast, i), &out[static_cast<size_t>(i)]);
+  for (Py_ssize_t i = 0; ok && i < n; ++i) ok = chain_pointer(PySequence_Fast_GET_ITEM(fast, i), optional, &out[static_cast<size_t>(i)]);
   Py_DECREF(fast);
-  if (!ok) PyErr_SetString(PyExc_TypeError, "tensors or None expected");
   return ok;
+}
+
+// The scalar arguments: handle of the compiled chain, element count, stream context.
+bool chain_scalars(PyObject* handle, PyObject* count, PyObject* stream, void** h, len_t* n, StreamContext* ctx) {
+  if (handle == Py_None) { PyErr_SetString(PyExc_ValueError, "the chain is closed"); return false; }
+  if (to_pointer(handle, h) && Convert<len_t>::get(count, n) && Convert<StreamContext>::get(stream, ctx)) return true;
+  PyErr_SetString(PyExc_TypeError, "(handle, ..., element count, StreamContext) expected");
+  return false;
 }
 
 // chain_forward(handle, leaves, out, n, stream)
@@ -180,11 +199,9 @@ PyObject* py_chain_forward(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   std::vector<void*> leaves;
   len_t n;
   StreamContext ctx;
-  if (nargs != 5 || !to_pointers(args[1], leaves)) { if (!PyErr_Occurred()) PyErr_SetString(PyExc_TypeError, "chain_forward: 5 arguments"); return nullptr; }
-  if (!to_pointer(args[0], &handle) || !to_pointer(args[2], &out) || !Convert<len_t>::get(args[3], &n) || !Convert<StreamContext>::get(args[4], &ctx)) {
-    PyErr_SetString(PyExc_TypeError, "chain_forward: (handle, leaves, out, n, stream)");
+  if (nargs != 5) { PyErr_SetString(PyExc_TypeError, "chain_forward: 5 arguments"); return nullptr; }
+  if (!chain_scalars(args[0], args[3], args[4], &handle, &n, &ctx) || !chain_pointers(args[1], false, leaves) || !chain_pointer(args[2], false, &out))
     return nullptr;
-  }
   Py_BEGIN_ALLOW_THREADS
   mpJitForward(handle, leaves.data(), out, n, ctx);
   Py_END_ALLOW_THREADS
@@ -198,15 +215,11 @@ PyObject* py_chain_reverse(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   double alpha;
   len_t n;
   StreamContext ctx;
-  if (nargs != 7 || !to_pointers(args[1], leaves) || !to_pointers(args[3], grads)) {
-    if (!PyErr_Occurred()) PyErr_SetString(PyExc_TypeError, "chain_reverse: 7 arguments");
+  if (nargs != 7) { PyErr_SetString(PyExc_TypeError, "chain_reverse: 7 arguments"); return nullptr; }
+  if (!chain_scalars(args[0], args[5], args[6], &handle, &n, &ctx) || !chain_pointers(args[1], true, leaves) || !chain_pointer(args[2], true, &gout) ||
+      !chain_pointers(args[3], true, grads))
     return nullptr;
-  }
-  if (!to_pointer(args[0], &handle) || !to_pointer(args[2], &gout) || !Convert<double>::get(args[4], &alpha) || !Convert<len_t>::get(args[5], &n) ||
-      !Convert<StreamContext>::get(args[6], &ctx)) {
-    PyErr_SetString(PyExc_TypeError, "chain_reverse: (handle, leaves, g_out, g_leaves, alpha, n, stream)");
-    return nullptr;
-  }
+  if (!Convert<double>::get(args[4], &alpha)) { PyErr_SetString(PyExc_TypeError, "chain_reverse: alpha is a float"); return nullptr; }
   Py_BEGIN_ALLOW_THREADS
   mpJitReverse(handle, leaves.data(), gout, grads.data(), alpha, n, ctx);
   Py_END_ALLOW_THREADS

@@ -118,11 +118,11 @@ class FusedChain:
 
     def forward(self, leaves, out, n, stream):
         assert len(leaves) == len(self.leaves)
-        _native.chain_forward(self.handle, leaves, out, n, stream)
+        _native.chain_forward(self.handle, leaves, out, n, stream.ctx)
 
     def reverse(self, leaves, g_out, g_leaves, alpha, n, stream):
         assert len(leaves) == len(self.leaves) == len(g_leaves)
-        _native.chain_reverse(self.handle, leaves, g_out, g_leaves, float(alpha), n, stream)
+        _native.chain_reverse(self.handle, leaves, g_out, g_leaves, float(alpha), n, stream.ctx)
 
     def close(self):
         if self.handle:
