@@ -1604,7 +1604,7 @@ __global__ void __launch_bounds__(128) ssd_walk_sum_parts_kernel(const float* __
   if (threadIdx.x == 0) {
     gA[h] = sa;
     if (gA_log != nullptr) gA_log[h] += sa * A[h];
-    if (gbias != nullptr) gbias[h] += sb;
+    if (gbias != nullptr) atomicAdd(gbias + h, sb);   // scans on two streams may share a bias
   }
 }
 

@@ -185,6 +185,42 @@ def test_reverse_with_the_raw_side_gradients_is_the_three_launches_in_one(mp, st
         assert_close(b, a.astype(np.float64), 1e-5, name)
 
 
+def test_scans_on_several_streams_share_a_bias_gradient(mp):
+    """Every scan adds its step sizes' bias gradient: 4 streams x 16 scans of the same inputs into one vector."""
+    import torch
+    dims = nb, L, H, P, N, G, Q = 1, 128, 8, 64, 128, 1, 128
+    x, _, _, Bm, Cm, gy = make_inputs(30, *dims[:-1])
+    ins = [dev(a) for a in (x, np.full((nb, L, H), 0.5, np.float32), -np.ones(H, np.float32), Bm, Cm)]
+    zero, draw, dbias, dgy = dev(np.zeros(H, np.float32)), dev(np.zeros((nb * L, H), np.float16)), dev(np.zeros(H, np.float32)), dev(gy)
+    shared = torch.zeros_like(zero)
+
+    class Lane:
+        def __init__(self):
+            self.stream = mp.Stream()
+            self.out = [torch.empty_like(t) for t in (ins[0], ins[1], ins[2], draw, ins[3], ins[4])]
+            self.scratch = scratch_for(mp, dims, True)
+
+        def scan(self, gbias):
+            gx, gdt, gA, graw, gB, gC = self.out
+            mp.launch("ssd_scan_reverse_raw", torch.float16, *ins, dgy, draw, H, dbias, gx, gdt, gA, graw, H, gbias, None, gB, gC, self.scratch, *dims,
+                      self.stream)
+
+    lanes = [Lane() for _ in range(4)]
+    one = torch.zeros_like(zero)
+    torch.cuda.synchronize()
+    lanes[0].scan(one)
+    lanes[0].stream.sync()
+    for _ in range(16):
+        for lane in lanes:
+            lane.scan(shared)
+    for lane in lanes:
+        lane.stream.sync()
+        assert lane.stream.status() == 0
+        lane.stream.close()
+    # 64 additions of one value: each rounds the sum, by 2^-24 of it at most
+    np.testing.assert_allclose(host(shared), 64 * host(one).astype(np.float64), rtol=64 * 2.0 ** -24)
+
+
 @pytest.mark.parametrize("dims", [
     # (batch, seqlen, heads, headdim, dstate, groups, chunk): the chunk walk on lengths that are no multiple of its 128-step
     # chunk - the shortest, less than one chunk, one step past a chunk, one step short of one, and sequences cut between CTAs
