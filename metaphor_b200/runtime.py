@@ -80,13 +80,15 @@ def _launch_ctypes(name: str, dtype, *args):
     fn(*conv, ctx)
 
 
-def _load_native():
-    """The native call path (host/py_launch.cpp), None while the library is not built."""
+@functools.lru_cache(maxsize=None)
+def _native():
+    """The native call path (host/py_launch.cpp); raises ImportError while it, or the library behind it, is not built."""
     import importlib.machinery
     import importlib.util
+    lib()
     path = abi.LIB_PATH.parent / "mp_launch.so"
     if not path.exists():
-        return None
+        raise ImportError(f"{path} is missing: run `python -m metaphor_b200.build` (needs nvcc)")
     import torch
     loader = importlib.machinery.ExtensionFileLoader("mp_launch", str(path))
     mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("mp_launch", loader))
@@ -95,12 +97,12 @@ def _load_native():
     return mod
 
 
-_native = _load_native()
-if _native is not None:
-    launch = _native.launch
-else:
+try:
+    launch = _native().launch
+except ImportError:      # not built yet, or built from other sources: this package also holds the build
     def launch(name: str, dtype, *args):
-        raise ImportError(f"{abi.LIB_PATH.parent / 'mp_launch.so'} is missing: run `python -m metaphor_b200.build` (needs nvcc)")
+        """``launch_<name>_<suffix>(*args)`` as soon as the library is built."""
+        return _native().launch(name, dtype, *args)
 
 
 class FusedChain:
@@ -108,6 +110,7 @@ class FusedChain:
 
     def __init__(self, expr: str, dtype):
         self._lib = lib()
+        _native()
         self.dtype = dtype
         key = {"r16": 0, "r32": 1, "r64": 2}[suffix_of(dtype)]
         self.handle = self._lib.mpJitCompile(expr.encode(), key)
@@ -118,11 +121,11 @@ class FusedChain:
 
     def forward(self, leaves, out, n, stream):
         assert len(leaves) == len(self.leaves)
-        _native.chain_forward(self.handle, leaves, out, n, stream.ctx)
+        _native().chain_forward(self.handle, leaves, out, n, stream.ctx)
 
     def reverse(self, leaves, g_out, g_leaves, alpha, n, stream):
         assert len(leaves) == len(self.leaves) == len(g_leaves)
-        _native.chain_reverse(self.handle, leaves, g_out, g_leaves, float(alpha), n, stream.ctx)
+        _native().chain_reverse(self.handle, leaves, g_out, g_leaves, float(alpha), n, stream.ctx)
 
     def close(self):
         if self.handle:

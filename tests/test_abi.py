@@ -71,3 +71,27 @@ def test_reference_artefact_names_exist(mp):
     # build.zig:125-146 links src/lib/mp_kernels.a and libdev_utils.so
     libdir = Path(mp.LIB_PATH).parent
     assert (libdir / "mp_kernels.a").exists() and (libdir / "libdev_utils.so").exists()
+
+
+def test_package_imports_while_half_built(tmp_path):
+    """The build lives in the package: it must import without the library, with the library alone, and with the native call path left over
+    from an earlier build, and say what is missing when something is launched or compiled; once both are there, launches go through."""
+    import shutil
+    import sys
+    pkg = tmp_path / "metaphor_b200"
+    shutil.copytree(ROOT / "metaphor_b200", pkg, ignore=shutil.ignore_patterns("lib", "__pycache__", "csrc"))
+    (pkg / "lib").mkdir()
+    lib = ROOT / "metaphor_b200" / "lib"
+    code = ("import shutil, torch, metaphor_b200 as mp, metaphor_b200.build\n"
+            "for call in (lambda: mp.launch('fill', torch.float32, 16, 1.0, 0, mp.StreamContext()), lambda: mp.FusedChain('a+b', torch.float32)):\n"
+            "    try:\n        call()\n    except ImportError as e:\n        print('ImportError', 'metaphor_b200.build' in str(e))\n")
+    both = ("import os\n"
+            f"for f in ('libmp_kernels.so', 'mp_launch.so'):\n    os.path.exists(r'{pkg}/lib/' + f) or shutil.copy(r'{lib}/' + f, r'{pkg}/lib/' + f)\n"
+            "mp.launch('fill', torch.float32, 16, 1.0, 0, mp.StreamContext())\nprint('launched')\n")
+    for present in (("mp_launch.so",), ("libmp_kernels.so",)):
+        for f in present:
+            shutil.copy(lib / f, pkg / "lib" / f)
+        res = subprocess.run([sys.executable, "-c", code + both], capture_output=True, text=True, cwd=tmp_path, timeout=300)
+        assert res.stdout.split() == ["ImportError", "True", "ImportError", "True", "launched"], res.stdout + res.stderr
+        for f in ("libmp_kernels.so", "mp_launch.so"):
+            (pkg / "lib" / f).unlink()
