@@ -1097,9 +1097,9 @@ __global__ void __launch_bounds__(RowCfg<GROUP>::THREADS) rmsnorm_rev_shift(cons
 }
 
 // --------------------- fallback (any n, any alignment) ---------------------
-// One CTA per row, scalar coalesced accesses, the row is re-read from L2 for
-// each pass.  Used when n is not a multiple of the pack width, a pointer is
-// not 16-byte aligned, or the row does not fit the register-resident kernels.
+// One CTA per row, scalar coalesced accesses, the row is re-read from L2 for each pass.  Used when the row does not fit the
+// register-resident kernels, the tensors of a call lie at different offsets from a 16-byte boundary, or (RMSNorm) the gain is not
+// 16-byte aligned beside rows that are not.
 constexpr int GEN_THREADS = 256;
 
 template <typename T>
@@ -1367,21 +1367,25 @@ RowPlan shift_plan(size_t n, std::initializer_list<const void*> ptrs, int* off0)
   return p;
 }
 
-#define MP_SHIFT_DISPATCH_G(PLAN, CALL, G)                                    \
-  do {                                                                        \
-    if ((PLAN).ppt == 1) { CALL(G, 1); }                                      \
-    else if ((PLAN).ppt == 2) { CALL(G, 2); }                                 \
-    else if ((PLAN).ppt == 3) { CALL(G, 3); }                                 \
-    else if ((PLAN).ppt == 4) { CALL(G, 4); }                                 \
-    else { CALL(G, 5); }                                                      \
-  } while (0)
+// The pairs that shift_plan gives: a group beyond the first holds more packs than five per thread of the group before it.
 #define MP_SHIFT_DISPATCH(PLAN, CALL)                                         \
   do {                                                                        \
-    if ((PLAN).group == 32) MP_SHIFT_DISPATCH_G(PLAN, CALL, 32);              \
-    else if ((PLAN).group == 128) MP_SHIFT_DISPATCH_G(PLAN, CALL, 128);       \
-    else if ((PLAN).group == 256) MP_SHIFT_DISPATCH_G(PLAN, CALL, 256);       \
-    else if ((PLAN).group == 512) MP_SHIFT_DISPATCH_G(PLAN, CALL, 512);       \
-    else MP_SHIFT_DISPATCH_G(PLAN, CALL, 1024);                               \
+    if ((PLAN).group == 32) {                                                 \
+      if ((PLAN).ppt == 1) { CALL(32, 1); }                                   \
+      else if ((PLAN).ppt == 2) { CALL(32, 2); }                              \
+      else MP_SHIFT_DISPATCH_345(PLAN, CALL, 32);                             \
+    } else if ((PLAN).group == 128) {                                         \
+      if ((PLAN).ppt == 2) { CALL(128, 2); }                                  \
+      else MP_SHIFT_DISPATCH_345(PLAN, CALL, 128);                            \
+    } else if ((PLAN).group == 256) MP_SHIFT_DISPATCH_345(PLAN, CALL, 256);   \
+    else if ((PLAN).group == 512) MP_SHIFT_DISPATCH_345(PLAN, CALL, 512);     \
+    else MP_SHIFT_DISPATCH_345(PLAN, CALL, 1024);                             \
+  } while (0)
+#define MP_SHIFT_DISPATCH_345(PLAN, CALL, G)                                  \
+  do {                                                                        \
+    if ((PLAN).ppt == 3) { CALL(G, 3); }                                      \
+    else if ((PLAN).ppt == 4) { CALL(G, 4); }                                 \
+    else { CALL(G, 5); }                                                      \
   } while (0)
 // Softmax: one CTA per row group, or one wave of eight per SM (a multiple of every pack length) where that is at most four rows
 // each (the launches then overlap, see MP_OVERLAP_CTAS).
