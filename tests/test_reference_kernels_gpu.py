@@ -14,7 +14,9 @@ pytestmark = pytest.mark.gpu
 
 @pytest.fixture(scope="module")
 def ref(stream):
-    from refkernels import RefLib
+    from refkernels import REF_SO, RefLib
+    if not REF_SO.exists():   # built by oracle/build_ref.py where the reference's sources are mounted
+        pytest.skip(f"{REF_SO.name} is not built: no reference sources here")
     r = RefLib()
     yield r
     r.close()
