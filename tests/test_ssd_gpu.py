@@ -287,6 +287,32 @@ def test_ssd_heads_in_pairs(mp, stream, orc, dims, shift):
             assert_close(got, want.astype(got.dtype), TOL, f"{name} {dims} {shift}")
 
 
+@pytest.mark.parametrize("dims,shift", [((14, 384, 16, 64, 128, 1, 128), 0.0), ((20, 256, 32, 64, 128, 2, 256), 0.0), ((8, 512, 24, 64, 128, 1, 256), 0.0),
+                                        ((14, 256, 16, 64, 128, 1, 128), 7.0)])
+def test_ssd_heads_in_pairs_have_the_bits_of_single_heads(mp, stream, monkeypatch, dims, shift):
+    """Whether the walk takes two heads of a group at a time depends on the batch size; its results must not."""
+    import torch
+    x, dt, A, Bm, Cm, gy = make_inputs(23, *dims[:-1])
+    if shift:
+        dt = (dt + shift * np.random.default_rng(24).uniform(size=dt.shape)).astype(np.float32)
+    args = [dev(a) for a in (x, dt, A, Bm, Cm)]
+    dgy = dev(gy)
+    outs = []
+    for single in (False, True):
+        if single:
+            monkeypatch.setenv("MP_SSD_WALK_NO_PAIRS", "1")      # read at every launch
+        y, gx, gdt, gA, gB, gC = (dev(np.full(a.shape, np.nan, a.dtype)) for a in (x, x, dt, A, Bm, Cm))
+        scratch = scratch_for(mp, dims, True)
+        torch.cuda.current_stream().synchronize()
+        mp.launch("ssd_scan", torch.float16, *args, y, scratch, *dims, stream)
+        mp.launch("ssd_scan_reverse", torch.float16, *args, dgy, gx, gdt, gA, gB, gC, scratch, *dims, stream)
+        stream.sync()
+        assert stream.status() == 0
+        outs.append((y, gx, gdt, gA, gB, gC))
+    for a, b, name in zip(*outs, ("y", "gx", "gdt", "gA", "gB", "gC")):
+        assert torch.equal(a, b), name
+
+
 @pytest.mark.parametrize("dims,shift,off", [
     # (batch, seqlen, heads, headdim, dstate, groups, chunk), shift of the raw step sizes, elements between a 16-byte boundary and the
     # r16 bases.  fp32 segments of 64 steps: one segment and its edges, several, one step past a segment and one short of it, whole
