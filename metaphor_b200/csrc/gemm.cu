@@ -767,7 +767,7 @@ void launch_tc(Operand<__half> a, Operand<__half> b, const GemmArgs& args, int s
   const int grid = tiles < sm_count ? static_cast<int>(tiles) : sm_count;   // persistent: one CTA per SM
   MpLaunch(grid, GEMM_THREADS, smem, st)(gemm_tcgen05_kernel<BN, EXACT>, ta, tb, tc, args);
   MP_LAUNCH_CHECK();
-  if (args.ksplit > 1) launch_fold<T>(args, st);
+  if (args.ksplit > 1) launch_fold<T>(args, NoAgain{}, st);
 }
 
 void launch_pair(Operand<__half> a, Operand<__half> b, GemmArgs args, int sm_count, cudaStream_t st) {
@@ -792,7 +792,7 @@ void launch_pair(Operand<__half> a, Operand<__half> b, GemmArgs args, int sm_cou
   const int pairs = tiles < sm_count / 2 ? tiles : sm_count / 2;
   MpLaunch(2 * pairs, GEMM_THREADS, smem, st)(gemm_tcgen05_pair_kernel, ta, tb, tc, args);
   MP_LAUNCH_CHECK();
-  if (args.ksplit > 1) launch_fold<T>(args, st);
+  if (args.ksplit > 1) launch_fold<T>(args, NoAgain{}, st);
 }
 
 // Output-tile width: wide tiles for wide problems, narrower ones when they are

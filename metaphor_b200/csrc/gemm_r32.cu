@@ -65,7 +65,7 @@ __device__ __forceinline__ R32Unit r32_unit(const GemmArgs& g, int unit, int til
 
 template <int BN, bool EXACT>
 __global__ void __launch_bounds__(R_THREADS, 1) gemm_r32_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                                                                const __grid_constant__ CUtensorMap tmap_c, const GemmArgs g) {
+                                                                const __grid_constant__ CUtensorMap tmap_c, const GemmArgs g, const Again again) {
   using Cfg = R32Cfg<BN>;
   constexpr int A_BYTES = Cfg::A_BYTES, B_BYTES = Cfg::B_BYTES, RAW = Cfg::RAW, STAGES = Cfg::STAGES;
   extern __shared__ unsigned char gemm_smem_raw[];
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(R_THREADS, 1) gemm_r32_kernel(const __grid_con
                 for (int j = 0; j < 32; ++j) stage[j * 32 + lane] = r[j];
 #pragma unroll 1
                 for (int j = 0; j < 32; ++j)
-                  if (row < g.M && col0 + j < g.N && stage[j * 32 + lane] != stage[j * 32 + lane]) stage[j * 32 + lane] = dot_again(g, u.bz, row, col0 + j);
+                  if (row < g.M && col0 + j < g.N && stage[j * 32 + lane] != stage[j * 32 + lane]) stage[j * 32 + lane] = again(g, u.bz, row, col0 + j);
 #pragma unroll
                 for (int j = 0; j < 32; ++j) r[j] = stage[j * 32 + lane];
                 __syncwarp();
@@ -419,9 +419,13 @@ void launch_r32(Operand<float> a, Operand<float> b, const GemmArgs& g, int sms, 
   if ((g.ldc * sizeof(float)) % 16 == 0 && mp_aligned16(g.c)) tc = make_store_map<float>(g.c, g.M, g.N, g.ldc, false, nb);
   MP_CUDA_CHECK(cudaFuncSetAttribute(gemm_r32_kernel<BN, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM));
   const long units = static_cast<long>((g.N + BN - 1) / BN) * ((g.M + BM - 1) / BM) * g.ksplit * g.batch;
-  MpLaunch(static_cast<unsigned>(units < sms ? units : sms), R_THREADS, Cfg::SMEM, st)(gemm_r32_kernel<BN, EXACT>, ta, tb, tc, g);
+  const Again again{a.p, b.p, a.ld, b.ld};
+  MpLaunch(static_cast<unsigned>(units < sms ? units : sms), R_THREADS, Cfg::SMEM, st)(gemm_r32_kernel<BN, EXACT>, ta, tb, tc, g, again);
   MP_LAUNCH_CHECK();
-  if (g.ksplit > 1) launch_fold<float>(g, st);
+  if (g.ksplit > 1) {
+    if (EXACT) launch_fold<float>(g, AgainFold{again, g.a_mn, g.b_mn, g.K}, st);
+    else launch_fold<float>(g, NoAgain{}, st);
+  }
 }
 
 }  // namespace
@@ -450,7 +454,6 @@ void gemm_run_r32(Operand<float> a, Operand<float> b, GemmArgs args, int sms, vo
     }
   }
   const bool exact = args.exact != 0 && args.split != 0;
-  if (exact) { args.a_raw = a.p; args.a_ld = a.ld; args.b_raw = b.p; args.b_ld = b.ld; }
   if (bn == 128) {
     if (exact) launch_r32<128, true>(a, b, args, sms, st); else launch_r32<128, false>(a, b, args, sms, st);
   } else {

@@ -17,9 +17,6 @@ struct GemmArgs {
   int a_mn, b_mn;     // operand major-ness: 0 = K contiguous, 1 = M resp. N contiguous
   int stages;
   int exact = 0;      // sum as exactly as the FP pipe does (the EXACT forms of the kernels)
-  const float* a_raw = nullptr;   // EXACT r32: the operands, for results that come out as NaN (see dot_again); row pitches
-  const float* b_raw = nullptr;
-  size_t a_ld, b_ld;
   int epi_boxes = 2;  // pair kernel: 64-column staging boxes per epilogue warp
   int split;          // r32 only: 1 = error-compensated hi/lo split (3 MMAs per k-slice), 0 = one tf32 MMA (for timing)
   int ksplit;         // > 1: the K range of every tile is cut into ksplit work units whose raw fp32
@@ -73,18 +70,26 @@ __device__ __noinline__ float dot_again(const float* a, size_t a_step, const flo
   }
   return s;
 }
-__device__ __forceinline__ float dot_again(const GemmArgs& g, int bz, int row, int col) {
-  const float* a = g.a_raw + static_cast<size_t>(bz) * (g.a_mn ? g.K : g.M) * g.a_ld + (g.a_mn ? row : row * g.a_ld);
-  const float* b = g.b_raw + static_cast<size_t>(bz) * (g.b_mn ? g.K : g.N) * g.b_ld + (g.b_mn ? col : col * g.b_ld);
-  return dot_again(a, g.a_mn ? g.a_ld : 1, b, g.b_mn ? g.b_ld : 1, g.K);
-}
+// The operands of an EXACT r32 contraction, for that.
+struct Again {
+  const float* a;
+  const float* b;
+  size_t a_ld, b_ld;
+  __device__ __forceinline__ float operator()(const GemmArgs& g, int bz, int row, int col) const { return at(g.a_mn, g.b_mn, g.M, g.N, g.K, bz, row, col); }
+  __device__ __forceinline__ float at(int a_mn, int b_mn, int M, int N, int K, int bz, int row, int col) const {
+    return dot_again(a + static_cast<size_t>(bz) * (a_mn ? K : M) * a_ld + (a_mn ? row : row * a_ld), a_mn ? a_ld : 1,
+                     b + static_cast<size_t>(bz) * (b_mn ? K : N) * b_ld + (b_mn ? col : col * b_ld), b_mn ? b_ld : 1, K);
+  }
+};
+struct AgainFold { Again again; int a_mn, b_mn, K; };   // one problem, K cut into parts
+struct NoAgain {};
 
 // C = alpha * sum_s partial[s] + bias + beta * C  (finishes a split-K contraction).  A thread folds four neighbouring columns
 // of a row; partial rows have a pitch of whole fours whatever N is.
-template <typename T>
+template <typename T, typename R>
 __global__ void __launch_bounds__(256) gemm_fold_kernel(const float* __restrict__ partial, int ksplit, int M, int N, int ld, float alpha,
                                                         const T* __restrict__ bias, float beta, T* c, size_t ldc, size_t bias_pitch,
-                                                        const GemmArgs g) {
+                                                        const R r) {
   mp_grid_dependency();
   const size_t mn = static_cast<size_t>(M) * ld;
   const size_t i0 = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) * 4;
@@ -104,7 +109,9 @@ __global__ void __launch_bounds__(256) gemm_fold_kernel(const float* __restrict_
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
     if (col + e < N) {
-      if (sizeof(T) == 4 && g.a_raw != nullptr && acc[e] != acc[e]) acc[e] = dot_again(g, 0, static_cast<int>(row), col + e);
+      if constexpr (std::is_same<R, AgainFold>::value) {
+        if (acc[e] != acc[e]) acc[e] = r.again.at(r.a_mn, r.b_mn, M, N, r.K, 0, static_cast<int>(row), col + e);
+      }
       float o = alpha * acc[e];
       if (br != nullptr) o += mp_up(br[e]);
       if (beta != 0.0f) o += beta * mp_up(cr[e]);
@@ -179,12 +186,12 @@ CUtensorMap make_store_map(void* base, size_t rows, size_t cols, size_t ld, bool
   return map;
 }
 
-template <typename T>
-void launch_fold(const GemmArgs& args, cudaStream_t st) {
+template <typename T, typename R>
+void launch_fold(const GemmArgs& args, const R& again, cudaStream_t st) {
   const size_t units = static_cast<size_t>(args.M) * args.partial_ld / 4;
-  MpLaunch(static_cast<unsigned>((units + 255) / 256), 256, 0, st)(gemm_fold_kernel<T>, args.partial, args.ksplit, args.M, args.N, args.partial_ld,
+  MpLaunch(static_cast<unsigned>((units + 255) / 256), 256, 0, st)(gemm_fold_kernel<T, R>, args.partial, args.ksplit, args.M, args.N, args.partial_ld,
                                                                                 args.alpha, static_cast<const T*>(args.bias), args.beta,
-                                                                                static_cast<T*>(args.c), args.ldc, args.bias_pitch, args);
+                                                                                static_cast<T*>(args.c), args.ldc, args.bias_pitch, again);
   MP_LAUNCH_CHECK();
 }
 
