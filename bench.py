@@ -49,10 +49,9 @@ UNIT = "GB/s"
 # DRAM bytes per launch from ncu (dram__bytes_read.sum + dram__bytes_write.sum)
 # for the kernels of this step; filled from profiles/ (None = not captured).
 NCU_TRAFFIC_BYTES = {
-    # profiles/rmsnorm_reverse_m32768_n4096.md, captured at 32768 rows and scaled x2 (traffic is linear in rows)
+    # captured at 32768 rows and scaled x2 (traffic is linear in rows)
     "rmsnorm_rev_r32": 2 * (1_073_854_000 + 510_001_152),
     "rmsnorm_rev_r16": 2 * (537_149_952 + 252_880_128),
-    # profiles/softmax_m32768_n4096.md
     "softmax_rev_r32": 2 * (1_073_749_000 + 495_847_168),
     "softmax_fwd_r16": 2 * (268_444_928 + 213_376_768),
 }
@@ -477,14 +476,14 @@ def lm_workload_text(n_layer, batch):
 
 # launcher -> DRAM bytes of one call from ncu (dram__bytes_read.sum + dram__bytes_write.sum over the launcher's tensor-core
 # kernels: both chunk walks and the group-gradient kernel; the prefix-sum and scalar-gradient kernels were not captured),
-# taken at batch 4 x seqlen 4096 x 32 heads (profiles/ssd_walk_and_group_gradients_b4_l4096_h32.md).  Every CTA walks one
-# (batch, head) sequence, so traffic grows in proportion to batch x seqlen x heads and is scaled to the step's shape.
-# A launcher that is not listed reports traffic null.
+# taken at batch 4 x seqlen 4096 x 32 heads: forward one head at a time, reverse two heads of a group at a time, the forms that the
+# step's 192 sequences take as well.  Every chunk of every sequence is read once per walk, so traffic grows in proportion to
+# batch x seqlen x heads and is scaled to the step's shape.  A launcher that is not listed reports traffic null.
 LM_NCU_TRAFFIC = {
-    "ssd_scan_raw_r16": {"bytes": 81.9e6 + 29.9e6, "units": 4 * 4096 * 32},
-    "ssd_scan_reverse_r16": {"bytes": 247.2e6 + 194.5e6 + 286.7e6, "units": 4 * 4096 * 32},
-    "ssd_scan_reverse_raw_r16": {"bytes": 247.2e6 + 194.5e6 + 286.7e6, "units": 4 * 4096 * 32},   # the same three kernels
-    "ssd_scan_r16": {"bytes": 81.9e6 + 29.9e6, "units": 4 * 4096 * 32},
+    "ssd_scan_raw_r16": {"bytes": 82.0e6 + 30.9e6, "units": 4 * 4096 * 32},
+    "ssd_scan_reverse_r16": {"bytes": 247.3e6 + 193.0e6 + 283.6e6, "units": 4 * 4096 * 32},
+    "ssd_scan_reverse_raw_r16": {"bytes": 247.3e6 + 193.0e6 + 283.6e6, "units": 4 * 4096 * 32},   # the same three kernels
+    "ssd_scan_r16": {"bytes": 82.0e6 + 30.9e6, "units": 4 * 4096 * 32},
 }
 
 

@@ -700,7 +700,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 // Operands that TMA cannot address (a row pitch or a base that is no multiple of 16 bytes: odd widths) are copied into rows of
 // a 16-byte pitch in the stream's workspace and multiplied from there.  The copy moves each element twice against the tensor
 // pipe's M or N uses of it; the FP-pipe kernel that served these shapes before reached 16 TFLOP/s ([2000, 999] x [999, 1501] and
-// the two contractions of its reverse in r32: 1150 us there, 190 us from copies, 15 us of them the copies).  One thread makes one
+// the two contractions of its reverse in r32: 1148 us there, 196 us from copies, 15 us of them the copies).  Every contraction copies the
+// operands it reads: a training step of a dense block copies x, its weights and the upstream gradient twice each.  One thread makes one
 // 16-byte chunk of a destination row from 2- or 4-byte loads (neighbouring threads share the sectors); the bytes of the last
 // chunk past the row's end are zeros that the tensor map does not read.
 // ---------------------------------------------------------------------------

@@ -17,7 +17,8 @@
 // Launches: states made inside every segment, both directions (segment_states); carried from segment to segment, element by element
 // (segment_carry); outputs (segment_forward / segment_reverse); for the reverse two folds.
 //
-// What bounds it is the FP pipe with its shared-memory operands: 1.8 M (forward) and 4.1 M (reverse) multiply-adds per head and segment.
+// What bounds it is the FP pipe with its shared-memory operands: 1.5 M (forward) and 3.7 M (reverse) multiply-adds per head and segment,
+// states included; at a third of the pipe's peak, since the reverse's tiles leave room for one CTA of eight warps per SM.
 // Forward / reverse in us, the recurrence -> segments (the chunk walk on padded chunks, with its r16 losses):
 //   [2, 1000, 24] 1 806 / 41 544 -> 97 / 259 (29 / 82),   [8, 8191, 32] 41 650 / 800 600 -> 3 945 / 8 951 (279 / 923),
 //   [2, 32, 24] 62 / 1 260 -> 9.5 / 24 (11 / 60),   [1, 100, 2] 182 / 3 957 -> 22 / 38 (11 / 33).

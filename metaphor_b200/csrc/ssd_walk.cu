@@ -868,7 +868,6 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
       }
       // scalars of the chunk in hand (cur) and of the one after it (nxt), which are requested a whole chunk before they are used
       float cum_cur = 0.f, dt_cur = 0.f, last_cur = 0.f;
-      // the chunk's decay, which the next state needs at once, is brought into L1 two chunks before
       float cum_nxt, dt_nxt, colf_nxt, oth_nxt, last_nxt;
       auto fetch = [&](int k) {
         const uint32_t i = static_cast<uint32_t>(ANTI ? c_first - k : c_first + k) * WQ;
@@ -1689,7 +1688,7 @@ void mp_ssd_walk_cumsum_raw(const __half* raw, size_t raw_pitch, const float* bi
   MP_LAUNCH_CHECK();
 }
 
-// gdt, gA (and graw, gbias, gA_log, with raw) from the row dots and the pins' parts; ga_part, gb_part: [B * nc][H].
+// gdt, gA (and graw, gbias, gA_log, with raw) from the row dots and the pins; ga_part, gb_part: [B * nc][H].
 void mp_ssd_walk_scalars(const float* u, const float* v, const float* dtt, const float* A, const float* pin, float* gdt, float* gA, float* ga_part,
                          float* gb_part, const __half* raw, size_t raw_pitch, const float* bias, __half* graw, size_t graw_pitch, float* gbias,
                          float* gA_log, int B, int L, int H, cudaStream_t st) {
