@@ -1012,7 +1012,8 @@ void gemm_dispatch(const void* a_, const void* b_, const void* bias, double alph
       // FP pipe / split: normal operands K = 33 1.04e-7 / 1.32e-7, 53 1.32e-7 / 1.29e-7, 129 2.0e-7 / 1.4e-7; operands of one sign 65 1.23e-7 /
       // 1.38e-7, 129 1.58e-7 / 1.35e-7.  (Up to there the FP pipe takes 13 us where the output is small; [4097, 63, 4099] 121 against 64 us.)
       const double volume = static_cast<double>(M) * N * K * batch;
-      tensor_path = tensor_path && (sizeof(T) == 4 ? K >= 96 : K >= 64 || (K >= 16 && volume > 6.0e7));
+      const bool too_tall = (M + 63) / 64 > 65535;   // for the FP-pipe kernel's grid
+      tensor_path = tensor_path && (too_tall || (sizeof(T) == 4 ? K >= 96 : K >= 64 || (K >= 16 && volume > 6.0e7)));
     }
     if (tensor_path) {
       GemmArgs args;

@@ -158,7 +158,9 @@ ODD_SHAPES = [(1, 101, 103, 107), (1, 257, 65, 515), (1, 2571, 77, 1993), (1, 25
               (1, 16411, 1101, 67), (1, 67, 1101, 16411), (90, 513, 301, 515),
               # a single result, rows and columns of one, both sides of the lines to the tensor cores (K of 16, 64 and 96, volume of 6e7)
               (1, 1, 97, 1), (1, 2, 131, 1), (5, 3, 99, 2), (1, 1, 4099, 1), (1, 33, 63, 35), (1, 33, 65, 35), (1, 2001, 15, 2003), (1, 2001, 17, 2003),
-              (1, 1001, 95, 33)]
+              (1, 1001, 95, 33),
+              # more rows than the FP-pipe kernel's grid holds
+              (1, 4194401, 9, 3)]
 
 
 @pytest.mark.parametrize("sfx", ["r16", "r32"])
