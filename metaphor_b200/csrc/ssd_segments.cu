@@ -1,7 +1,7 @@
-// Mamba-2 SSD scan of r16 tensors with fp32 arithmetic throughout, over segments of 64 steps that run side by side (head size 64,
+// Mamba-2 SSD scan of r16 tensors to the accuracy of fp32 arithmetic, over segments of 64 steps that run side by side (head size 64,
 // state 128, any number of steps).  It serves the calls that whole tensor-core chunks do not cover: lengths that are no multiple of
 // the chunk, and other chunk lengths; pointers need no more than the alignment of their elements.  Its results are those of the
-// recurrence (ssd_generic.cu) to the accuracy of fp32 sums: weights, scores and states are never rounded to r16, and A's gradient is a sum of the
+// recurrence (ssd_generic.cu) to the accuracy of fp32 sums: weights, scores and states keep their 24 bits, and A's gradient is a sum of the
 // products that make it up, not a difference of row dots, so that it keeps its digits where almost nothing is carried from step to
 // step ([2, 200, 16] with step sizes around 2: the r16 chunk walk is off by 0.6 of gA and 0.03 of gdt, this by 1.4e-7 and 1.3e-7).
 //
@@ -14,43 +14,50 @@
 //   s_j  = sum_i M G X + e_j <B_j, Y x_j>
 //   ga_t = sum_{i >= t > j} M G X dt_j + sum_{i >= t} exp(cum_i) <C_i, H gy_i> + sum_{j < t} dt_j e_j <B_j, Y x_j> + exp(E) <Y, H>
 //   gdt_t = s_t + A ga_t,   gA = sum_t dt_t ga_t
-// Launches: states made inside every segment, both directions (segment_states); carried from segment to segment, element by element
+// Launches: states made inside every segment, both directions (segment_states); carried from segment to segment, block by block
 // (segment_carry); outputs (segment_forward / segment_reverse); for the reverse two folds.
 //
-// What bounds it is the FP pipe with its shared-memory operands: 1.5 M (forward) and 3.7 M (reverse) multiply-adds per head and segment,
-// states included; at a third of the pipe's peak, since the reverse's tiles leave room for one CTA of eight warps per SM.
-// Forward / reverse in us, the recurrence -> segments (the chunk walk on padded chunks, with its r16 losses):
-//   [2, 1000, 24] 1 806 / 41 544 -> 97 / 259 (29 / 82),   [8, 8191, 32] 41 650 / 800 600 -> 3 945 / 8 951 (279 / 923),
-//   [2, 32, 24] 62 / 1 260 -> 9.5 / 24 (11 / 60),   [1, 100, 2] 182 / 3 957 -> 22 / 38 (11 / 33).
+// Every product has one operand that is r16 in memory (x, B, C, gy).  The other, in fp32 (weights times scores, scaled values, states), is
+// split into two r16 terms under a power of two that brings the largest value of its row (states: of its 16 x 16 block) below 2^15: 23 bits,
+// and 40 binary orders below the largest value.  A product is then two tensor-core MMAs with the r16 operand unsplit, and the scores
+// are one.  mma.sync and not tcgen05, because the sums stay in registers: a warp turns its scores into the next product's operand without
+// a trip through TMEM or shared memory, and sums that reach gdt and gA are taken out of the accumulator, which truncates, after every
+// 16 products and added up rounded.
+// A CTA with an infinity or a NaN among its results does its share again on the FP pipe (*_plain below): where an r16 tile holds one, the
+// lower term of a value that needs none would meet it with a zero, and so would a step that the mask leaves out.
+//
+// Forward / reverse in us, recurrence -> fp32 on the FP pipe (24 TFLOP/s of its 72) -> here:
+//   [2, 1000, 24] 1 806 / 41 544 -> 96 / 261 -> 44 / 93,   [8, 8191, 32] 41 650 / 800 600 -> 3 947 / 8 996 -> 1 255 / 3 242,
+//   [1, 8191, 2] 57 / 107 -> 52 / 84 (FP pipe -> here),    [1, 100, 2] 182 / 3 957 -> 21 / 38 -> 12 / 20.
+// The 2-norm of the errors against r64: y, gx, gB, gC are r16 roundings on all three; gdt 1.2e-7 - 1.6e-7 here, 1.3e-7 - 2.4e-7 on the FP pipe
+// (mma.sync: 555 TFLOP/s in r16, so that two terms leave 280).  What bounds the reverse is the latency of its sixteen warps: tensor pipe a
+// quarter busy; the states and the carry move 128 KB of global memory a head and segment.
 // Below 32 steps the recurrence stays (60 / 1 214 us at [2, 31, 24]): its forward needs no scratch, and callers may rely on that.
-#include "mp_common.cuh"
+#include "mp_async.cuh"
 
 namespace {
 
 constexpr int SG_Q = 64;              // steps per segment
 constexpr int SG_N = 128, SG_P = 64;  // state size, head size
-constexpr int SG_THREADS = 256;
-constexpr int SG_NPITCH = SG_N + 4, SG_PPITCH = SG_P + 4;   // floats per row of a shared tile: rows 16 bytes apart in the banks
-constexpr int SG_STATE = SG_N * SG_P;
+constexpr int SG_STATE_BYTES = SG_N * SG_P * 4;   // a state as r16 pairs
+constexpr int SG_BLOCKS = SG_N / 16 * (SG_P / 16);   // 16 x 16 blocks of a state, each with a scale
 
 struct SegArgs {
   const __half* x; const float* dt; const float* A; const __half* Bm; const __half* Cm; const __half* gy;
   __half* y;                 // forward
   __half* gx; float* gdt;    // reverse
-  float* states;             // [B H][nseg][128][64]: causal states; the adjoint ones follow in the reverse
+  unsigned char* states;     // [B H][nseg] states received (see state_load); the adjoint ones follow in the reverse
   float* decay;              // [B H][nseg]: exp(E)
+  float* scales;             // [B H][nseg][4 of p][8 of n]: what a block's pairs are multiplied by; adjoint ones likewise
   float* ga_part;            // [B H][nseg]
   float* gb_part;            // [splits][B L G][128] sums over the heads of a split, gB then gC
   int B, L, H, G, nseg, splits;
   bool vec;                  // every r16 pointer is 16-byte aligned
 };
 
-// Scalars of a segment, by one warp: cum[64] (r64) and dt[64]; steps past the sequence do not decay and have dt = 0.
-__device__ __forceinline__ void segment_scalars(const SegArgs& g, int b, int h, int t0, double* cum, float* dt, int lane) {
-  const double a = static_cast<double>(g.A[h]);
-  const int t = t0 + 2 * lane;
-  const float* src = g.dt + (static_cast<size_t>(b) * g.L + t) * g.H + h;
-  const float d0 = t < g.L ? src[0] : 0.f, d1 = t + 1 < g.L ? src[g.H] : 0.f;
+// Scalars of a segment, by one warp: a lane's two inclusive sums of dt A and the last one; steps past the sequence do not decay (dt = 0).
+struct SegScan { double c0, c1, last; };
+__device__ __forceinline__ SegScan segment_scan(double a, float d0, float d1, int lane) {
   const double v0 = d0 * a, v1 = d1 * a;
   double s = v0 + v1;
 #pragma unroll
@@ -58,37 +65,550 @@ __device__ __forceinline__ void segment_scalars(const SegArgs& g, int b, int h, 
     const double up = __shfl_up_sync(0xffffffffu, s, o);
     if (lane >= o) s += up;
   }
-  cum[2 * lane] = s - v1;
-  cum[2 * lane + 1] = s;
+  return {s - v1, s, __shfl_sync(0xffffffffu, s, 31)};
+}
+__device__ __forceinline__ void segment_scalars(const SegArgs& g, int b, int h, int t0, double* cum, float* dt, int lane) {
+  const int t = t0 + 2 * lane;
+  const float* src = g.dt + (static_cast<size_t>(b) * g.L + t) * g.H + h;
+  const float d0 = t < g.L ? src[0] : 0.f, d1 = t + 1 < g.L ? src[g.H] : 0.f;
+  const SegScan s = segment_scan(static_cast<double>(g.A[h]), d0, d1, lane);
+  cum[2 * lane] = s.c0;
+  cum[2 * lane + 1] = s.c1;
   dt[2 * lane] = d0;
   dt[2 * lane + 1] = d1;
 }
 __device__ __forceinline__ float segment_exp(double v) { return expf(static_cast<float>(v)); }
 
-// [64 steps][COLS] of r16 -> fp32 tile; `scale`: a factor per step or null.  Steps past the sequence become zeros.
-template <int COLS, int PITCH>
-__device__ __forceinline__ void segment_tile(float* dst, const __half* src, size_t pitch, int rows, bool vec, const float* scale) {
+// ---------------------------------------------------------------------------
+// r16 tiles in shared memory: rows of PITCH bytes, their 16-byte chunks exchanged by the row, so that the eight rows of an ldmatrix
+// lie in different banks.
+// ---------------------------------------------------------------------------
+template <int PITCH>
+__device__ __forceinline__ uint32_t tile_at(uint32_t base, int r, int c) {
+  return base + r * PITCH + ((c ^ (PITCH == 64 ? (r >> 1) & 3 : r & 7)) << 4);
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void st_shared16(uint32_t dst, uint4 v) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ uint4 ld_shared16(uint32_t src) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(src) : "memory");
+  return v;
+}
+
+// 64 steps of CHUNKS 16-byte chunks; steps past the sequence become zeros.
+template <int CHUNKS, int THREADS>
+__device__ __forceinline__ void tile_load(uint32_t dst, const __half* src, size_t pitch, int rows, bool vec) {
 #pragma unroll
-  for (int k = 0; k < SG_Q * COLS / 8 / SG_THREADS; ++k) {
-    const int idx = k * SG_THREADS + threadIdx.x, r = idx / (COLS / 8), c = idx % (COLS / 8) * 8;
-    float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (r < rows) {
-      const __half* p = src + r * pitch + c;
-      if (vec) {
-        unpack<__half>(ld_pack(p, 0), f);
-      } else {
+  for (int k = 0; k < SG_Q * CHUNKS / THREADS; ++k) {
+    const int idx = k * THREADS + threadIdx.x, r = idx / CHUNKS, c = idx % CHUNKS;
+    const uint32_t at = tile_at<CHUNKS * 16>(dst, r, c);
+    const __half* p = src + r * pitch + c * 8;
+    if (r >= rows) {
+      st_shared16(at, make_uint4(0, 0, 0, 0));
+    } else if (vec) {
+      cp_async16(at, p);
+    } else {
+      const unsigned short* u = reinterpret_cast<const unsigned short*>(p);
+      uint32_t w[4];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) f[e] = __half2float(p[e]);
+      for (int e = 0; e < 4; ++e) w[e] = u[2 * e] | static_cast<uint32_t>(u[2 * e + 1]) << 16;
+      st_shared16(at, make_uint4(w[0], w[1], w[2], w[3]));
+    }
+  }
+}
+__device__ __forceinline__ uint32_t r16_finite(uint32_t v) {   // infinities and NaN replaced by zero
+  if ((v & 0x7c00u) == 0x7c00u) v &= 0xffff0000u;
+  if ((v & 0x7c000000u) == 0x7c000000u) v &= 0x0000ffffu;
+  return v;
+}
+
+// A state in global memory: blocks of 16 x 16 (p, n), a block's sixteen rows p after another, a row as four chunks: the upper terms of its
+// values, then the lower ones.  In shared memory rows p of 512 bytes, the blocks' chunks after another; the scales lie behind.
+template <int THREADS>
+__device__ __forceinline__ void state_load(uint32_t dst, const unsigned char* src, const float* scales) {
+#pragma unroll
+  for (int k = 0; k < SG_STATE_BYTES / 16 / THREADS; ++k) {
+    const int idx = k * THREADS + threadIdx.x;
+    cp_async16(tile_at<512>(dst, (idx >> 9) * 16 + ((idx >> 2) & 15), ((idx >> 6) & 7) * 4 + (idx & 3)), src + idx * 16);
+  }
+  if (threadIdx.x < SG_BLOCKS / 4) cp_async16(dst + SG_STATE_BYTES + threadIdx.x * 16, scales + threadIdx.x * 4);
+}
+
+// ---------------------------------------------------------------------------
+// Fragments.  A lane holds rows g and g + 8 of a 16-row operand or result, columns 2 q, 2 q + 1 of every eight (g = lane / 4, q = lane % 4).
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void ldsm(uint32_t (&r)[4], uint32_t at) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at) : "memory");
+}
+__device__ __forceinline__ void ldsm_t(uint32_t (&r)[4], uint32_t at) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at) : "memory");
+}
+__device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma0(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {   // nothing accumulated before
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+               : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+// Operand of 16 rows from r0 on, 16 columns from chunk c0 on (two chunks), of a tile [rows][columns]; _t: of a tile [columns][rows], rows
+// of chunks r0, r0 + 1, columns from c0 on.
+template <int PITCH>
+__device__ __forceinline__ void load_a(uint32_t (&a)[4], uint32_t tile, int r0, int c0, int lane) { ldsm(a, tile_at<PITCH>(tile, r0 + (lane & 15), c0 + (lane >> 4))); }
+template <int PITCH>
+__device__ __forceinline__ void load_a_t(uint32_t (&a)[4], uint32_t tile, int c0, int r0, int lane) {
+  ldsm_t(a, tile_at<PITCH>(tile, c0 + (lane & 7) + ((lane >> 4) << 3), r0 + ((lane >> 3) & 1)));
+}
+// Two neighbouring column operands (eight columns each): columns are rows n0 .. n0 + 15 of the tile, the sum runs over chunks c0, c0 + 1.
+template <int PITCH>
+__device__ __forceinline__ void load_b(uint32_t (&b)[4], uint32_t tile, int n0, int c0, int lane) {
+  ldsm(b, tile_at<PITCH>(tile, n0 + (lane & 7) + ((lane >> 4) << 3), c0 + ((lane >> 3) & 1)));
+}
+// The same where the sum runs over rows k0 .. k0 + 15 of the tile and the columns are those of chunks c0, c0 + 1.
+template <int PITCH>
+__device__ __forceinline__ void load_b_t(uint32_t (&b)[4], uint32_t tile, int k0, int c0, int lane) { ldsm_t(b, tile_at<PITCH>(tile, k0 + (lane & 15), c0 + (lane >> 4))); }
+
+// The power of two that brings a value with these bits (a magnitude, finite) below 2^15, and its reciprocal.
+__device__ __forceinline__ float split_scale(uint32_t bits, float* inverse) {
+  int e = 268 - static_cast<int>(bits >> 23);
+  e = e < 253 ? e : 253;
+  *inverse = __uint_as_float(static_cast<uint32_t>(254 - e) << 23);
+  return __uint_as_float(static_cast<uint32_t>(e) << 23);
+}
+__device__ __forceinline__ uint32_t magnitude(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+__device__ __forceinline__ uint32_t finite_bits(float v) { return magnitude(v) < 0x7f800000u ? magnitude(v) : 0u; }
+constexpr uint32_t SG_INFINITE = 0x7f800000u;
+// Two scaled values as pairs of r16 terms.  KEEP: an infinity stays one (its lower term must not be inf - inf; any finite value does, lower
+// terms stay below 2^4).
+template <bool KEEP>
+__device__ __forceinline__ void split(float v0, float v1, uint32_t& hi, uint32_t& lo) {
+  const __half2 h = __floats2half2_rn(v0, v1);
+  const float2 f = __half22float2(h);
+  const float l0 = v0 - f.x, l1 = v1 - f.y;
+  const __half2 l = KEEP ? __floats2half2_rn(fmaxf(l0, -64.f), fmaxf(l1, -64.f)) : __floats2half2_rn(l0, l1);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
+// ---------------------------------------------------------------------------
+// What a segment adds to the state behind it (blockIdx.y = 0) and to the adjoint state before it (1): fp32, in blocks of 16 x 16 (p, n), a block
+// as the fragments of its two 8-column tiles: eight values a lane.  A warp has 16 of the 64 rows p.
+// ---------------------------------------------------------------------------
+constexpr int SS_THREADS = 128;
+constexpr size_t SS_SMEM = SG_Q * SG_P * 2 + SG_Q * SG_N * 2 + SG_Q * sizeof(float);
+
+__global__ void __launch_bounds__(SS_THREADS) segment_states_kernel(const SegArgs g) {
+  mp_grid_dependency();
+  extern __shared__ __align__(128) unsigned char seg_smem[];
+  const bool anti = blockIdx.y != 0;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane & 3;
+  const int seq = blockIdx.x / g.nseg, seg = blockIdx.x % g.nseg, b = seq / g.H, h = seq % g.H, grp = h / (g.H / g.G);
+  const int t0 = seg * SG_Q, rows = min(SG_Q, g.L - t0);
+  const uint32_t sv = mp_smem_u32(seg_smem), sk = sv + SG_Q * SG_P * 2;
+  float* wt = reinterpret_cast<float*>(seg_smem + SG_Q * SG_P * 2 + SG_Q * SG_N * 2);
+  const bool needed = anti ? seg > 0 : seg < g.nseg - 1;   // something lies beyond
+  if (needed) {
+    const size_t row = static_cast<size_t>(b) * g.L + t0;
+    tile_load<SG_P / 8, SS_THREADS>(sv, (anti ? g.gy : g.x) + (row * g.H + h) * SG_P, static_cast<size_t>(g.H) * SG_P, rows, g.vec);
+    tile_load<SG_N / 8, SS_THREADS>(sk, (anti ? g.Cm : g.Bm) + (row * g.G + grp) * SG_N, static_cast<size_t>(g.G) * SG_N, rows, g.vec);
+    cp_async_commit();
+  }
+  if (warp == 0) {
+    const int t = t0 + 2 * lane;
+    const float* src = g.dt + (static_cast<size_t>(b) * g.L + t) * g.H + h;
+    const float d0 = t < g.L ? src[0] : 0.f, d1 = t + 1 < g.L ? src[g.H] : 0.f;
+    const SegScan sc = segment_scan(static_cast<double>(g.A[h]), d0, d1, lane);
+    wt[2 * lane] = anti ? segment_exp(sc.c0) : d0 * segment_exp(sc.last - sc.c0);
+    wt[2 * lane + 1] = anti ? segment_exp(sc.c1) : d1 * segment_exp(sc.last - sc.c1);
+    if (lane == 0 && !anti) g.decay[blockIdx.x] = segment_exp(sc.last);
+  }
+  if (!needed) return;
+  cp_async_wait<0>();
+  __syncthreads();
+  // rows p of the scaled values, over the 64 steps
+  float v[4][8];
+  uint32_t m0 = 0, m1 = 0;
+#pragma unroll
+  for (int kt = 0; kt < 4; ++kt) {
+    uint32_t r[4];
+    load_a_t<SG_P * 2>(r, sv, kt * 16, warp * 2, lane);
+    const float2 wa = *reinterpret_cast<const float2*>(wt + kt * 16 + 2 * q), wb = *reinterpret_cast<const float2*>(wt + kt * 16 + 8 + 2 * q);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&r[e]));
+      v[kt][2 * e] = f.x * (e < 2 ? wa.x : wb.x);
+      v[kt][2 * e + 1] = f.y * (e < 2 ? wa.y : wb.y);
+      uint32_t& m = e & 1 ? m1 : m0;
+      m = max(m, max(magnitude(v[kt][2 * e]), magnitude(v[kt][2 * e + 1])));
+    }
+  }
+  if (__any_sync(0xffffffffu, max(m0, m1) >= SG_INFINITE)) {   // the finite values set the scale
+    m0 = m1 = 0;
+#pragma unroll
+    for (int kt = 0; kt < 4; ++kt)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        uint32_t& m = (e >> 1) & 1 ? m1 : m0;
+        m = max(m, finite_bits(v[kt][e]));
       }
-      if (scale != nullptr) {
-        const float s = scale[r];
+  }
 #pragma unroll
-        for (int e = 0; e < 8; ++e) f[e] *= s;
+  for (int o = 1; o < 4; o <<= 1) {
+    m0 = max(m0, __shfl_xor_sync(0xffffffffu, m0, o));
+    m1 = max(m1, __shfl_xor_sync(0xffffffffu, m1, o));
+  }
+  float i0, i1;
+  const float f0 = split_scale(m0, &i0), f1 = split_scale(m1, &i1);
+  uint32_t hi[4][4], lo[4][4];
+#pragma unroll
+  for (int kt = 0; kt < 4; ++kt)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) split<true>(v[kt][2 * e] * (e & 1 ? f1 : f0), v[kt][2 * e + 1] * (e & 1 ? f1 : f0), hi[kt][e], lo[kt][e]);
+  float* out = reinterpret_cast<float*>(g.states + (static_cast<size_t>(anti) * g.B * g.H * g.nseg + blockIdx.x) * SG_STATE_BYTES) + warp * 2048 + lane * 8;
+#pragma unroll 2
+  for (int nb = 0; nb < SG_N / 16; ++nb) {
+    // `finite`: the r16 operand of the lower terms, whose zeros must not meet an infinity
+    auto sums = [&](float (&s)[2][4], bool finite) {
+#pragma unroll
+      for (int kt = 0; kt < 4; ++kt) {
+        uint32_t bb[4];
+        load_b_t<SG_N * 2>(bb, sk, kt * 16, nb * 2, lane);
+        float c0[4], c1[4];
+        if (finite) {
+          mma0(c0, lo[kt], r16_finite(bb[0]), r16_finite(bb[1]));
+          mma0(c1, lo[kt], r16_finite(bb[2]), r16_finite(bb[3]));
+        } else {
+          mma0(c0, lo[kt], bb[0], bb[1]);
+          mma0(c1, lo[kt], bb[2], bb[3]);
+        }
+        mma(c0, hi[kt], bb[0], bb[1]);
+        mma(c1, hi[kt], bb[2], bb[3]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          s[0][e] = kt == 0 ? c0[e] : s[0][e] + c0[e];
+          s[1][e] = kt == 0 ? c1[e] : s[1][e] + c1[e];
+        }
+      }
+    };
+    float s[2][4];
+    sums(s, false);
+    float check = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) check = fmaf(s[0][e], 0.f, fmaf(s[1][e], 0.f, check));
+    if (__any_sync(0xffffffffu, check != 0.f)) sums(s, true);
+    *reinterpret_cast<float4*>(out + nb * 256) = make_float4(s[0][0] * i0, s[0][1] * i0, s[0][2] * i1, s[0][3] * i1);
+    *reinterpret_cast<float4*>(out + nb * 256 + 4) = make_float4(s[1][0] * i0, s[1][1] * i0, s[1][2] * i1, s[1][3] * i1);
+  }
+}
+
+// In place: what every segment adds becomes what every segment receives, in two terms.  One warp per block of a sequence's state; it reads
+// four segments ahead, and what it overwrites (the segment behind the one whose sum it has) it has read before.
+constexpr int SC_THREADS = 128;
+__global__ void __launch_bounds__(SC_THREADS) segment_carry_kernel(const SegArgs g) {
+  mp_grid_dependency();
+  constexpr int PER = SG_BLOCKS / (SC_THREADS / 32);   // CTAs per sequence
+  const bool anti = blockIdx.y != 0;
+  const int lane = threadIdx.x & 31, q = lane & 3;
+  const int seq = blockIdx.x / PER, blk = (blockIdx.x % PER) * (SC_THREADS / 32) + (threadIdx.x >> 5);
+  const size_t first = (static_cast<size_t>(anti) * g.B * g.H + seq) * g.nseg;
+  unsigned char* base = g.states + first * SG_STATE_BYTES + blk * 1024;
+  float* scales = g.scales + first * SG_BLOCKS + blk;
+  const float* decay = g.decay + static_cast<size_t>(seq) * g.nseg;
+  const int steps = g.nseg - 1;
+  auto segment = [&](int k) { return anti ? g.nseg - 1 - k : k; };
+  float4 next[4][2];
+  float dnext[4];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int k = min(k0 + u, steps - 1);
+      const float4* p = reinterpret_cast<const float4*>(base + static_cast<size_t>(segment(k)) * SG_STATE_BYTES) + lane * 2;
+      next[u][0] = p[0];
+      next[u][1] = p[1];
+      dnext[u] = decay[segment(k)];
+    }
+  };
+  fetch(0);
+  float c[2][4] = {};
+#pragma unroll 1
+  for (int k0 = 0; k0 < steps; k0 += 4) {
+    float4 add[4][2];
+    float d[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) { add[u][0] = next[u][0]; add[u][1] = next[u][1]; d[u] = dnext[u]; }
+    if (k0 + 4 < steps) fetch(k0 + 4);
+    __syncwarp();   // every lane has read segment k0 + 4 before the state that takes its place is written
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (k0 + u >= steps) break;
+      const float a[2][4] = {{add[u][0].x, add[u][0].y, add[u][0].z, add[u][0].w}, {add[u][1].x, add[u][1].y, add[u][1].z, add[u][1].w}};
+      uint32_t m = 0;
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          c[t][e] = fmaf(d[u], c[t][e], a[t][e]);
+          m = max(m, magnitude(c[t][e]));
+        }
+      m = __reduce_max_sync(0xffffffffu, m);
+      if (m >= SG_INFINITE) {   // the finite values set the scale
+        m = 0;
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) m = max(m, finite_bits(c[t][e]));
+        m = __reduce_max_sync(0xffffffffu, m);
+      }
+      float inv;
+      const float f = split_scale(m, &inv);
+      const int to = segment(k0 + u) + (anti ? -1 : 1);
+      if (lane == 0) scales[static_cast<size_t>(to) * SG_BLOCKS] = inv;
+      unsigned char* out = base + static_cast<size_t>(to) * SG_STATE_BYTES + (lane >> 2) * 64 + q * 16;
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {   // rows g, g + 8: four chunks of the row over the four lanes of a quad, exchanged for one chunk a lane
+        uint32_t t[4];
+        split<true>(c[0][2 * r] * f, c[0][2 * r + 1] * f, t[0], t[2]);
+        split<true>(c[1][2 * r] * f, c[1][2 * r + 1] * f, t[1], t[3]);
+        uint32_t x0 = q & 1 ? t[1] : t[0], x1 = q & 1 ? t[0] : t[1], x2 = q & 1 ? t[3] : t[2], x3 = q & 1 ? t[2] : t[3];
+        x1 = __shfl_xor_sync(0xffffffffu, x1, 1);
+        x3 = __shfl_xor_sync(0xffffffffu, x3, 1);
+        t[0] = q & 1 ? x1 : x0; t[1] = q & 1 ? x0 : x1; t[2] = q & 1 ? x3 : x2; t[3] = q & 1 ? x2 : x3;
+        x0 = q & 2 ? t[2] : t[0]; x2 = q & 2 ? t[0] : t[2]; x1 = q & 2 ? t[3] : t[1]; x3 = q & 2 ? t[1] : t[3];
+        x2 = __shfl_xor_sync(0xffffffffu, x2, 2);
+        x3 = __shfl_xor_sync(0xffffffffu, x3, 2);
+        *reinterpret_cast<uint4*>(out + r * 512) = q & 2 ? make_uint4(x2, x3, x0, x1) : make_uint4(x0, x1, x2, x3);
       }
     }
-    float4* o = reinterpret_cast<float4*>(dst + r * PITCH + c);
-    o[0] = make_float4(f[0], f[1], f[2], f[3]);
-    o[1] = make_float4(f[4], f[5], f[6], f[7]);
+  }
+}
+
+constexpr int SG_THREADS = 256;
+
+// A CTA's share: one segment of one batch entry, one group, some of the group's heads.
+struct SegShare { int b, seg, grp, split, h_first, h_end; };
+__device__ __forceinline__ SegShare segment_share(const SegArgs& g) {
+  SegShare s;
+  const int hpg = g.H / g.G;
+  s.split = blockIdx.x % g.splits;
+  int rest = blockIdx.x / g.splits;
+  s.grp = rest % g.G;
+  rest /= g.G;
+  s.seg = rest % g.nseg;
+  s.b = rest / g.nseg;
+  s.h_first = s.grp * hpg + static_cast<int>(static_cast<long long>(hpg) * s.split / g.splits);
+  s.h_end = s.grp * hpg + static_cast<int>(static_cast<long long>(hpg) * (s.split + 1) / g.splits);
+  return s;
+}
+
+// What the kernels need of one head's steps in the segment.
+struct SegSteps { double cum[SG_Q]; float dt[SG_Q], grow[SG_Q], left[SG_Q]; };   // grow = exp(cum), left = exp(E - cum)
+__device__ __forceinline__ void segment_steps(const SegArgs& g, int b, int h, int t0, SegSteps& s, int lane) {
+  segment_scalars(g, b, h, t0, s.cum, s.dt, lane);
+  __syncwarp();
+  const double last = s.cum[SG_Q - 1];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const double c = s.cum[2 * lane + e];
+    s.grow[2 * lane + e] = segment_exp(c);
+    s.left[2 * lane + e] = segment_exp(last - c);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Scores.  The ten 16 x 16 blocks on and below the diagonal of a 64 x 64 matrix are dealt out to the warps; a block's scores of C and B stay
+// with its warp over the heads.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ bool block_of(int k, int& ib, int& jb) {
+  ib = k < 1 ? 0 : k < 3 ? 1 : k < 6 ? 2 : 3;
+  jb = k - ib * (ib + 1) / 2;
+  return k < 10;
+}
+// Rows 16 ib of tile a times rows 16 jb of tile b, over K; 16 products at a time are taken out of the accumulator.
+template <int K>
+__device__ __forceinline__ void block_scores(float (&s)[2][4], uint32_t a, uint32_t b, int ib, int jb, int lane) {
+#pragma unroll
+  for (int e = 0; e < 4; ++e) s[0][e] = s[1][e] = 0.f;
+#pragma unroll
+  for (int k = 0; k < K / 16; ++k) {
+    uint32_t av[4], bv[4];
+    load_a<K * 2>(av, a, ib * 16, 2 * k, lane);
+    load_b<K * 2>(bv, b, jb * 16, 2 * k, lane);
+    float c0[4], c1[4];
+    mma0(c0, av, bv[0], bv[1]);
+    mma0(c1, av, bv[2], bv[3]);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) { s[0][e] += c0[e]; s[1][e] += c1[e]; }
+  }
+}
+// M of a block: exp(cum_i - cum_j), zero above the diagonal.
+__device__ __forceinline__ void block_decays(float (&m)[2][4], const double* cum, int ib, int jb, int g, int q) {
+  const double c0 = cum[ib * 16 + g], c1 = cum[ib * 16 + g + 8];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int j = u * 8 + 2 * q;   // in the block
+    const double2 cj = *reinterpret_cast<const double2*>(cum + jb * 16 + j);
+    m[u][0] = segment_exp(c0 - cj.x);
+    m[u][1] = segment_exp(c0 - cj.y);
+    m[u][2] = segment_exp(c1 - cj.x);
+    m[u][3] = segment_exp(c1 - cj.y);
+    if (ib == jb) {
+      if (j > g) m[u][0] = 0.f;
+      if (j + 1 > g) m[u][1] = 0.f;
+      if (j > g + 8) m[u][2] = 0.f;
+      if (j + 1 > g + 8) m[u][3] = 0.f;
+    }
+  }
+}
+// A block as pairs of r16 terms in two tiles [64][64]; its scale's reciprocal goes to inv[4 ib + jb].
+__device__ __forceinline__ void block_split(const float (&v)[2][4], uint32_t hi, uint32_t lo, float* inv, int ib, int jb, int lane) {
+  float m = 0.f;
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) m = fmaxf(m, fabsf(v[u][e]));
+  float back;
+  const float f = split_scale(min(__reduce_max_sync(0xffffffffu, __float_as_uint(m)), SG_INFINITE - 1), &back);
+  if (lane == 0) inv[4 * ib + jb] = back;
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      uint32_t h, l;
+      split<false>(v[u][2 * r] * f, v[u][2 * r + 1] * f, h, l);
+      const uint32_t at = tile_at<SG_Q * 2>(0, ib * 16 + (lane >> 2) + 8 * r, jb * 2 + u) + 4 * (lane & 3);
+      asm volatile("st.shared.b32 [%0], %1;" ::"r"(hi + at), "r"(h) : "memory");
+      asm volatile("st.shared.b32 [%0], %1;" ::"r"(lo + at), "r"(l) : "memory");
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Products.  A warp has a few columns of the result and all 64 rows (NR = 4 blocks of 16), or two of the four blocks (NR = 2: `part` 0 has the
+// first and the last, 1 the others, which is as many blocks of scores), so that what it reads of a state, and of the tiles that the scores are
+// multiplied by, serves all of them.
+// ---------------------------------------------------------------------------
+template <int NR>
+__device__ __forceinline__ int row_block(int i, int part) { return NR == 4 ? i : part ? 1 + i : 3 * i; }
+
+// Rows of a tile [64][128] (over n) times a state: columns p = 8 c .. 8 c + 7.
+template <int NR>
+__device__ __forceinline__ void times_state_p(float (&o)[NR][4], uint32_t rows, uint32_t state, const float* scales, int c, int part, int lane) {
+#pragma unroll
+  for (int i = 0; i < NR; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[i][e] = 0.f;
+#pragma unroll 2
+  for (int k = 0; k < 8; ++k) {
+    uint32_t b[4];
+    ldsm(b, tile_at<512>(state, c * 8 + (lane & 7), k * 4 + (lane >> 3)));
+    const float f = scales[(c >> 1) * 8 + k];
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+      uint32_t a[4];
+      load_a<SG_N * 2>(a, rows, row_block<NR>(i, part) * 16, 2 * k, lane);
+      float s[4];
+      mma0(s, a, b[2], b[3]);
+      mma(s, a, b[0], b[1]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[i][e] = fmaf(s[e], f, o[i][e]);
+    }
+  }
+}
+// Rows of a tile [64][64] (over p) times a state: columns n = 16 nb .. 16 nb + 15.
+template <int NR>
+__device__ __forceinline__ void times_state_n(float (&o)[NR][2][4], uint32_t rows, uint32_t state, const float* scales, int nb, int part, int lane) {
+#pragma unroll
+  for (int i = 0; i < NR; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[i][0][e] = o[i][1][e] = 0.f;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    uint32_t b[2][4];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) ldsm_t(b[u], tile_at<512>(state, k * 16 + (lane & 15), nb * 4 + u + ((lane >> 4) << 1)));
+    const float f = scales[k * 8 + nb];
+#pragma unroll
+    for (int i = 0; i < NR; ++i) {
+      uint32_t a[4];
+      load_a<SG_P * 2>(a, rows, row_block<NR>(i, part) * 16, 2 * k, lane);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        float s[4];
+        mma0(s, a, b[u][2], b[u][3]);
+        mma(s, a, b[u][0], b[u][1]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[i][u][e] = fmaf(s[e], f, o[i][u][e]);
+      }
+    }
+  }
+}
+// The operand for eight columns (chunk c) and all 64 steps of a tile [64][64].
+__device__ __forceinline__ void load_steps(uint32_t (&b)[4][2], uint32_t tile, int c, int lane) {
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    uint32_t v[4];
+    ldsm_t(v, tile_at<SG_P * 2>(tile, k * 32 + lane, c));
+    b[2 * k][0] = v[0]; b[2 * k][1] = v[1]; b[2 * k + 1][0] = v[2]; b[2 * k + 1][1] = v[3];
+  }
+}
+// o += scores (LOWER: rows i, over j up to the row's block; otherwise rows j, over i from the row's block on) times COLS tiles of eight columns.
+template <int NR, bool LOWER, int COLS>
+__device__ __forceinline__ void times_scores(float (&o)[NR][COLS][4], uint32_t hi, uint32_t lo, const float* inv, const uint32_t (&b)[4][2 * COLS], int part,
+                                             int lane) {
+#pragma unroll
+  for (int i = 0; i < NR; ++i)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int rb = row_block<NR>(i, part);
+      if (LOWER ? k > rb : k < rb) continue;
+      uint32_t h[4], l[4];
+      if (LOWER) {
+        load_a<SG_Q * 2>(h, hi, rb * 16, 2 * k, lane);
+        load_a<SG_Q * 2>(l, lo, rb * 16, 2 * k, lane);
+      } else {
+        load_a_t<SG_Q * 2>(h, hi, k * 16, 2 * rb, lane);
+        load_a_t<SG_Q * 2>(l, lo, k * 16, 2 * rb, lane);
+      }
+      const float f = LOWER ? inv[4 * rb + k] : inv[4 * k + rb];
+#pragma unroll
+      for (int u = 0; u < COLS; ++u) {
+        float s[4];
+        mma0(s, l, b[k][2 * u], b[k][2 * u + 1]);
+        mma(s, h, b[k][2 * u], b[k][2 * u + 1]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[i][u][e] = fmaf(s[e], f, o[i][u][e]);
+      }
+    }
+}
+// Two neighbouring r16 results.
+__device__ __forceinline__ void store_pair(__half* dst, float v0, float v1, bool vec) {
+  const __half2 h = __floats2half2_rn(v0, v1);
+  if (vec) {
+    *reinterpret_cast<__half2*>(dst) = h;
+  } else {
+    dst[0] = __low2half(h);
+    dst[1] = __high2half(h);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The same outputs on the FP pipe, for a CTA that met an infinity or a NaN: fp32 tiles, and steps that the mask leaves out are not read.
+// ---------------------------------------------------------------------------
+constexpr int SG_NPITCH = SG_N + 4, SG_PPITCH = SG_P + 4;   // floats per row of a shared tile: rows 16 bytes apart in the banks
+
+// [64 steps][COLS] of r16 -> fp32 tile.  Steps past the sequence become zeros.
+template <int COLS, int PITCH, int THREADS>
+__device__ __forceinline__ void plain_tile(float* dst, const __half* src, size_t pitch, int rows) {
+#pragma unroll 1
+  for (int idx = threadIdx.x; idx < SG_Q * COLS; idx += THREADS) {
+    const int r = idx / COLS, c = idx % COLS;
+    dst[r * PITCH + c] = r < rows ? __half2float(src[r * pitch + c]) : 0.f;
   }
 }
 
@@ -113,87 +633,18 @@ __device__ __forceinline__ void segment_store(__half* dst, const float* v, bool 
   }
 }
 
-// What a segment adds to the state behind it (blockIdx.y = 0) and to the adjoint state before it (1).
-// Threads: eight state rows x four head columns each.
-__global__ void __launch_bounds__(SG_THREADS) segment_states_kernel(const SegArgs g) {
-  mp_grid_dependency();
-  extern __shared__ __align__(16) float seg_smem[];
-  float* sK = seg_smem;                         // [64][132] B or C
-  float* sV = sK + SG_Q * SG_NPITCH;            // [64][68] x or gy, scaled
-  double* cum = reinterpret_cast<double*>(sV + SG_Q * SG_PPITCH);
-  float* dt = reinterpret_cast<float*>(cum + SG_Q);
-  float* w = dt + SG_Q;
-  const bool anti = blockIdx.y != 0;
-  const int seq = blockIdx.x / g.nseg, seg = blockIdx.x % g.nseg, b = seq / g.H, h = seq % g.H, grp = h / (g.H / g.G);
-  const int t0 = seg * SG_Q, rows = min(SG_Q, g.L - t0);
-  if (threadIdx.x < 32) {
-    segment_scalars(g, b, h, t0, cum, dt, threadIdx.x);
-    __syncwarp();
-    const double last = cum[SG_Q - 1];
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int t = 2 * threadIdx.x + e;
-      w[t] = anti ? segment_exp(cum[t]) : dt[t] * segment_exp(last - cum[t]);
-    }
-    if (threadIdx.x == 0 && !anti) g.decay[blockIdx.x] = segment_exp(last);
-  }
-  if (anti ? seg == 0 : seg == g.nseg - 1) return;   // nothing lies beyond
-  __syncthreads();
-  const size_t row = static_cast<size_t>(b) * g.L + t0;
-  segment_tile<SG_N, SG_NPITCH>(sK, (anti ? g.Cm : g.Bm) + (row * g.G + grp) * SG_N, static_cast<size_t>(g.G) * SG_N, rows, g.vec, nullptr);
-  segment_tile<SG_P, SG_PPITCH>(sV, (anti ? g.gy : g.x) + (row * g.H + h) * SG_P, static_cast<size_t>(g.H) * SG_P, rows, g.vec, w);
-  __syncthreads();
-  const int n0 = threadIdx.x / 16 * 8, p0 = threadIdx.x % 16 * 4;
-  float acc[8][4] = {};
-#pragma unroll 4
-  for (int k = 0; k < SG_Q; ++k) {
-    const float4 a0 = ld4(sK + k * SG_NPITCH + n0), a1 = ld4(sK + k * SG_NPITCH + n0 + 4), v = ld4(sV + k * SG_PPITCH + p0);
-#pragma unroll
-    for (int r = 0; r < 8; ++r)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(r < 4 ? at(a0, r) : at(a1, r - 4), at(v, c), acc[r][c]);
-  }
-  float* out = g.states + (static_cast<size_t>(anti) * g.B * g.H * g.nseg + blockIdx.x) * SG_STATE;
-#pragma unroll
-  for (int r = 0; r < 8; ++r) *reinterpret_cast<float4*>(out + (n0 + r) * SG_P + p0) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+// The value (n, p) of a state in global memory.
+__device__ __forceinline__ float state_value(const unsigned char* state, const float* scales, int n, int p) {
+  const int blk = (p >> 4) * 8 + (n >> 4);
+  const __half* v = reinterpret_cast<const __half*>(state + blk * 1024 + (p & 15) * 64) + (n & 15);
+  return (__half2float(v[0]) + __half2float(v[16])) * scales[blk];
 }
-
-// In place: what every segment adds becomes what every segment receives.  One thread per four elements of a sequence's state.
-__global__ void __launch_bounds__(SG_THREADS) segment_carry_kernel(const SegArgs g) {
-  mp_grid_dependency();
-  const bool anti = blockIdx.y != 0;
-  constexpr int PER = SG_STATE / 4 / SG_THREADS;   // CTAs per sequence
-  const int seq = blockIdx.x / PER, e = (blockIdx.x % PER) * SG_THREADS + threadIdx.x;
-  float4* st = reinterpret_cast<float4*>(g.states + (static_cast<size_t>(anti) * g.B * g.H + seq) * g.nseg * SG_STATE) + e;
-  const float* decay = g.decay + static_cast<size_t>(seq) * g.nseg;
-  constexpr size_t STEP = SG_STATE / 4;
-  float4 carry = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int s0 = 0; s0 < g.nseg; s0 += 4) {
-    float4 add[4];
-    float d[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {      // (the last segment in walk order has nothing to add)
-      const int s = anti ? g.nseg - 1 - s0 - u : s0 + u;
-      const bool live = s0 + u < g.nseg - 1;
-      add[u] = live ? st[s * STEP] : make_float4(0.f, 0.f, 0.f, 0.f);
-      d[u] = live ? decay[s] : 0.f;
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      if (s0 + u >= g.nseg) break;
-      const int s = anti ? g.nseg - 1 - s0 - u : s0 + u;
-      st[s * STEP] = carry;
-      carry = make_float4(fmaf(d[u], carry.x, add[u].x), fmaf(d[u], carry.y, add[u].y), fmaf(d[u], carry.z, add[u].z), fmaf(d[u], carry.w, add[u].w));
-    }
-  }
-}
-
-// State of a segment from global to shared memory (see state_at).
-__device__ __forceinline__ void segment_load_state(float* dst, const float* src) {
-#pragma unroll
-  for (int k = 0; k < SG_STATE / 4 / SG_THREADS; ++k) {
-    const int idx = k * SG_THREADS + threadIdx.x, n = idx / (SG_P / 4), p4 = idx % (SG_P / 4);
-    *reinterpret_cast<float4*>(dst + state_at(n, p4)) = *reinterpret_cast<const float4*>(src + idx * 4);
+template <int THREADS>
+__device__ __forceinline__ void plain_state(float* dst, const unsigned char* state, const float* scales) {
+#pragma unroll 1
+  for (int idx = threadIdx.x; idx < SG_N * SG_P; idx += THREADS) {
+    const int p = idx / SG_N, n = idx % SG_N;
+    dst[state_at(n, p >> 2) + (p & 3)] = state_value(state, scales, n, p);
   }
 }
 
@@ -204,7 +655,7 @@ __device__ __forceinline__ void segment_scores(const float* a, const float* b, i
   for (int u = 0; u < 4; ++u)
 #pragma unroll
     for (int v = 0; v < 4; ++v) acc[u][v] = 0.f;
-  // sixteen products at a time: the sums of the long chain would carry most of gdt's error (2.5e-7 of its norm with one chain)
+  // sixteen products at a time, as the tensor cores have them
 #pragma unroll 1
   for (int k0 = 0; k0 < K; k0 += 16) {
     float part[4][4] = {};
@@ -227,97 +678,390 @@ __device__ __forceinline__ void segment_scores(const float* a, const float* b, i
   }
 }
 
-// y of one (sequence, segment).  Thread (ty, tx): four rows 16 apart or next to each other, four columns.
-__global__ void __launch_bounds__(SG_THREADS, 2) segment_forward_kernel(const SegArgs g) {
-  mp_grid_dependency();
-  extern __shared__ __align__(16) float seg_smem[];
-  float* sC = seg_smem;                          // [64][132]
+// y of heads h_first .. h_end - 1 in one segment.  Thread (ty, tx): four rows 16 apart, four columns.
+__device__ __noinline__ void segment_forward_plain(const SegArgs& g, float* smem, int b, int seg, int grp, int h_first, int h_end) {
+  float* sC = smem;                              // [64][132]
   float* sB = sC + SG_Q * SG_NPITCH;             // [64][132], then the state [128][64]
   float* sX = sB + SG_Q * SG_NPITCH;             // [64][68]
   float* sW = sX + SG_Q * SG_PPITCH;             // [64][68]
   double* cum = reinterpret_cast<double*>(sW + SG_Q * SG_PPITCH);
   float* dt = reinterpret_cast<float*>(cum + SG_Q);
-  const int seq = blockIdx.x / g.nseg, seg = blockIdx.x % g.nseg, b = seq / g.H, h = seq % g.H, grp = h / (g.H / g.G);
   const int t0 = seg * SG_Q, rows = min(SG_Q, g.L - t0);
   const size_t row = static_cast<size_t>(b) * g.L + t0;
-  if (threadIdx.x < 32) segment_scalars(g, b, h, t0, cum, dt, threadIdx.x);
-  segment_tile<SG_N, SG_NPITCH>(sC, g.Cm + (row * g.G + grp) * SG_N, static_cast<size_t>(g.G) * SG_N, rows, g.vec, nullptr);
-  segment_tile<SG_N, SG_NPITCH>(sB, g.Bm + (row * g.G + grp) * SG_N, static_cast<size_t>(g.G) * SG_N, rows, g.vec, nullptr);
-  segment_tile<SG_P, SG_PPITCH>(sX, g.x + (row * g.H + h) * SG_P, static_cast<size_t>(g.H) * SG_P, rows, g.vec, nullptr);
-  __syncthreads();
-  const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
-  {
-    float s[4][4];
-    segment_scores<SG_N, SG_NPITCH>(sC, sB, ty, tx, s);
+#pragma unroll 1
+  for (int h = h_first; h < h_end; ++h) {
+    __syncthreads();
+    if (threadIdx.x < 32) segment_scalars(g, b, h, t0, cum, dt, threadIdx.x);
+    plain_tile<SG_N, SG_NPITCH, SG_THREADS>(sC, g.Cm + (row * g.G + grp) * SG_N, static_cast<size_t>(g.G) * SG_N, rows);
+    plain_tile<SG_N, SG_NPITCH, SG_THREADS>(sB, g.Bm + (row * g.G + grp) * SG_N, static_cast<size_t>(g.G) * SG_N, rows);
+    plain_tile<SG_P, SG_PPITCH, SG_THREADS>(sX, g.x + (row * g.H + h) * SG_P, static_cast<size_t>(g.H) * SG_P, rows);
+    __syncthreads();
+    const int ty = threadIdx.x / 16, tx = threadIdx.x % 16, p0 = tx * 4;
+    {
+      float s[4][4];
+      segment_scores<SG_N, SG_NPITCH>(sC, sB, ty, tx, s);
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
+      for (int u = 0; u < 4; ++u)
 #pragma unroll
-      for (int v = 0; v <= u; ++v) {
-        const int i = ty + 16 * u, j = tx + 16 * v;
-        sW[i * SG_PPITCH + j] = s[u][v] * segment_exp(cum[i] - cum[j]) * dt[j];   // (read for j <= i)
-      }
-  }
-  __syncthreads();
-  if (seg > 0) segment_load_state(sB, g.states + static_cast<size_t>(blockIdx.x) * SG_STATE);
-  const int p0 = tx * 4;
-  float acc[4][4] = {};
+        for (int v = 0; v <= u; ++v) {
+          const int i = ty + 16 * u, j = tx + 16 * v;
+          sW[i * SG_PPITCH + j] = s[u][v] * segment_exp(cum[i] - cum[j]) * dt[j];   // (read for j <= i)
+        }
+    }
+    __syncthreads();
+    if (seg > 0) {
+      const size_t unit = (static_cast<size_t>(b) * g.H + h) * g.nseg + seg;
+      plain_state<SG_THREADS>(sB, g.states + unit * SG_STATE_BYTES, g.scales + unit * SG_BLOCKS);
+      __syncthreads();
+    }
+    {
+      float acc[4][4] = {};
 #pragma unroll
-  for (int jb = 0; jb < 4; ++jb) {
+      for (int jb = 0; jb < 4; ++jb) {
 #pragma unroll 2
-    for (int j = jb * 16; j < jb * 16 + 16; j += 4) {
-      float4 v[4];
+        for (int j = jb * 16; j < jb * 16 + 16; j += 4) {
+          float4 v[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) v[e] = ld4(sX + (j + e) * SG_PPITCH + p0);
+          for (int e = 0; e < 4; ++e) v[e] = ld4(sX + (j + e) * SG_PPITCH + p0);
 #pragma unroll
-      for (int u = jb; u < 4; ++u) {
-        const float4 w = ld4(sW + (ty + 16 * u) * SG_PPITCH + j);
+          for (int u = jb; u < 4; ++u) {
+            const float4 w = ld4(sW + (ty + 16 * u) * SG_PPITCH + j);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          if (u == jb && j + e > ty + 16 * u) continue;   // left out, not multiplied by zero: a later step may be infinite
+            for (int e = 0; e < 4; ++e) {
+              if (u == jb && j + e > ty + 16 * u) continue;   // left out, not multiplied by zero: a later step may be infinite
 #pragma unroll
-          for (int c = 0; c < 4; ++c) acc[u][c] = fmaf(at(w, e), at(v[e], c), acc[u][c]);
+              for (int c = 0; c < 4; ++c) acc[u][c] = fmaf(at(w, e), at(v[e], c), acc[u][c]);
+            }
+          }
         }
       }
-    }
-  }
-  if (seg > 0) {
-    __syncthreads();
-    float st[4][4] = {};
+      if (seg > 0) {
+        float st[4][4] = {};
 #pragma unroll 2
-    for (int n = 0; n < SG_N; n += 4) {
-      float4 v[4];
+        for (int n = 0; n < SG_N; n += 4) {
+          float4 v[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) v[e] = ld4(sB + state_at(n + e, tx));
+          for (int e = 0; e < 4; ++e) v[e] = ld4(sB + state_at(n + e, tx));
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const float4 w = ld4(sC + (ty + 16 * u) * SG_NPITCH + n);
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+#pragma unroll
+              for (int c = 0; c < 4; ++c) st[u][c] = fmaf(at(w, e), at(v[e], c), st[u][c]);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const float f = segment_exp(cum[ty + 16 * u]);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) acc[u][c] = fmaf(f, st[u][c], acc[u][c]);
+        }
+      }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const float4 w = ld4(sC + (ty + 16 * u) * SG_NPITCH + n);
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-#pragma unroll
-          for (int c = 0; c < 4; ++c) st[u][c] = fmaf(at(w, e), at(v[e], c), st[u][c]);
+        const int i = ty + 16 * u;
+        if (i < rows) segment_store(g.y + ((row + i) * g.H + h) * SG_P + p0, acc[u], g.vec);
       }
     }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const float f = segment_exp(cum[ty + 16 * u]);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) acc[u][c] = fmaf(f, st[u][c], acc[u][c]);
-    }
-  }
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int i = ty + 16 * u;
-    if (i < rows) segment_store(g.y + ((row + i) * g.H + h) * SG_P + p0, acc[u], g.vec);
   }
 }
 
-// Gradients of one (batch entry, segment, group, share of the group's heads); gB and gC of the share stay in registers.
-// Thread (ty, tx): scores as in segment_scores; everything else rows 4 ty .. 4 ty + 3, head columns 4 tx .. 4 tx + 3, state columns
-// 4 tx .. 4 tx + 3 and those 64 further.
-__global__ void __launch_bounds__(SG_THREADS, 1) segment_reverse_kernel(const SegArgs g) {
+
+// ---------------------------------------------------------------------------
+// y of one (batch entry, segment, group, share of the group's heads).  A warp has eight of the 64 columns; the next head's tiles arrive
+// while one is worked on.
+// ---------------------------------------------------------------------------
+constexpr int SF_X = SG_Q * SG_P * 2, SF_S = SG_STATE_BYTES + SG_BLOCKS * 4;
+constexpr size_t SF_TILES = SG_Q * SG_N * 2 + 2 * SF_X + SF_S + 2 * SG_Q * SG_Q * 2;   // C, x twice, state, weights in two terms
+constexpr size_t SF_SMEM = SF_TILES + 2 * sizeof(SegSteps) + 16 * sizeof(float);
+
+__global__ void __launch_bounds__(SG_THREADS, 2) segment_forward_kernel(const SegArgs g) {
   mp_grid_dependency();
-  extern __shared__ __align__(16) float seg_smem[];
-  float* sB = seg_smem;                          // [64][132]
+  extern __shared__ __align__(128) unsigned char seg_smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane & 3, r0 = lane >> 2;
+  const SegShare sh = segment_share(g);
+  const int t0 = sh.seg * SG_Q, rows = min(SG_Q, g.L - t0);
+  const size_t row = static_cast<size_t>(sh.b) * g.L + t0;
+  const bool before = sh.seg > 0;
+  const uint32_t sC = mp_smem_u32(seg_smem), sX = sC + SG_Q * SG_N * 2, sH = sX + 2 * SF_X, sPh = sH + SF_S, sPl = sPh + SG_Q * SG_Q * 2;
+  const float* hscales = reinterpret_cast<const float*>(seg_smem + (sH + SG_STATE_BYTES - sC));
+  SegSteps* steps = reinterpret_cast<SegSteps*>(seg_smem + SF_TILES);
+  float* inv = reinterpret_cast<float*>(steps + 2);
+  auto load_x = [&](int h) {
+    tile_load<SG_P / 8, SG_THREADS>(sX + ((h - sh.h_first) & 1) * SF_X, g.x + (row * g.H + h) * SG_P, static_cast<size_t>(g.H) * SG_P, rows, g.vec);
+  };
+  auto load_state = [&](int h) {
+    const size_t unit = (static_cast<size_t>(sh.b) * g.H + h) * g.nseg + sh.seg;
+    if (before) state_load<SG_THREADS>(sH, g.states + unit * SG_STATE_BYTES, g.scales + unit * SG_BLOCKS);
+  };
+  tile_load<SG_N / 8, SG_THREADS>(sC, g.Cm + (row * g.G + sh.grp) * SG_N, static_cast<size_t>(g.G) * SG_N, rows, g.vec);
+  tile_load<SG_N / 8, SG_THREADS>(sH, g.Bm + (row * g.G + sh.grp) * SG_N, static_cast<size_t>(g.G) * SG_N, rows, g.vec);   // B, for the scores
+  load_x(sh.h_first);
+  cp_async_commit();
+  if (warp == 7) segment_steps(g, sh.b, sh.h_first, t0, steps[0], lane);
+  cp_async_wait<0>();
+  __syncthreads();
+  float G[2][2][4];
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    int ib, jb;
+    if ((s == 0 || warp >> 1 == 2) && block_of(warp + 4 * s, ib, jb)) block_scores<SG_N>(G[s], sC, sH, ib, jb, lane);
+  }
+  __syncthreads();   // the state takes the place of B
+  load_state(sh.h_first);
+  cp_async_commit();
+  float check = 0.f;   // becomes NaN with the first result that is none, or infinite
+#pragma unroll 1
+  for (int h = sh.h_first; h < sh.h_end; ++h) {
+    const int par = (h - sh.h_first) & 1;
+    cp_async_wait<0>();
+    __syncthreads();   // this head's tiles are there, the last one's have been read
+    if (h + 1 < sh.h_end) {
+      load_x(h + 1);
+      if (warp == 7) segment_steps(g, sh.b, h + 1, t0, steps[par ^ 1], lane);
+    }
+    const SegSteps& st = steps[par];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      int ib, jb;
+      if (s == 1 && warp >> 1 != 2) continue;   // the last two blocks are the second ones of warps 4 and 5
+      block_of(warp + 4 * s, ib, jb);
+      float m[2][4];
+      block_decays(m, st.cum, ib, jb, r0, q);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const float2 dj = *reinterpret_cast<const float2*>(st.dt + jb * 16 + u * 8 + 2 * q);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) m[u][e] = G[s][u][e] * m[u][e] * (e & 1 ? dj.y : dj.x);
+      }
+      block_split(m, sPh, sPl, inv, ib, jb, lane);
+    }
+    float o[4][1][4];
+    if (before) {
+      float v[4][4];
+      times_state_p<4>(v, sC, sH, hscales, warp, 0, lane);
+#pragma unroll
+      for (int rb = 0; rb < 4; ++rb) {
+        const float f0 = st.grow[rb * 16 + r0], f1 = st.grow[rb * 16 + r0 + 8];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[rb][0][e] = v[rb][e] * (e < 2 ? f0 : f1);
+      }
+    } else {
+#pragma unroll
+      for (int rb = 0; rb < 4; ++rb)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[rb][0][e] = 0.f;
+    }
+    __syncthreads();   // the weights are complete, the state has been read
+    if (h + 1 < sh.h_end) load_state(h + 1);
+    cp_async_commit();
+    uint32_t b[4][2];
+    load_steps(b, sX + par * SF_X, warp, lane);
+    times_scores<4, true, 1>(o, sPh, sPl, inv, b, 0, lane);
+    __half* y = g.y + ((row + r0) * g.H + h) * SG_P + warp * 8 + 2 * q;
+#pragma unroll
+    for (int rb = 0; rb < 4; ++rb)
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const int i = rb * 16 + r * 8;
+        check = fmaf(o[rb][0][2 * r], 0.f, fmaf(o[rb][0][2 * r + 1], 0.f, check));
+        if (r0 + i < rows) store_pair(y + static_cast<size_t>(i) * g.H * SG_P, o[rb][0][2 * r], o[rb][0][2 * r + 1], g.vec);
+      }
+  }
+  if (__syncthreads_or(check != 0.f)) segment_forward_plain(g, reinterpret_cast<float*>(seg_smem), sh.b, sh.seg, sh.grp, sh.h_first, sh.h_end);
+}
+
+// ---------------------------------------------------------------------------
+// Gradients of one (batch entry, segment, group, share of the group's heads).  Of the sixteen warps two share 16 of the 128 columns of gB and
+// gC, which stay in their registers over the heads, and eight of the 64 columns of gx.
+// ---------------------------------------------------------------------------
+constexpr int SR_THREADS = 512, SR_WARPS = SR_THREADS / 32;
+constexpr int SR_X = SG_Q * SG_P * 2, SR_S = SG_STATE_BYTES + SG_BLOCKS * 4;
+constexpr int SR_STAGE = 2 * SR_X + SR_S;   // x, gy, H: two of them; Y is read first and loaded again in the middle
+struct SegScalars {   // of one head; two of them, and three SegSteps (the next head's are made while the last one's are read)
+  float s[4][SG_Q];       // [row block] sums over the block's rows of M G X
+  float ga[4][SG_Q];      // [column block] sums over the block's columns of M G X dt, for the row blocks below it
+  float tri[SG_Q];        // ga from inside the diagonal blocks
+  float su[8][SG_Q];      // [16 columns] exp(cum_i) <C_i, H gy_i>
+  float sv[8][SG_Q];      // [16 columns] e_j <B_j, Y x_j>
+  float pin[SR_WARPS];    // [warp] parts of <Y, H>
+};
+constexpr size_t SR_TILES = 2 * SG_Q * SG_N * 2 + 2 * SR_STAGE + SR_S + 4 * SG_Q * SG_Q * 2;
+constexpr size_t SR_SMEM = SR_TILES + 3 * sizeof(SegSteps) + 2 * sizeof(SegScalars) + 32 * sizeof(float);
+
+// gdt and a part of gA of one head, by one warp; a lane has two steps, eight lanes a block of 16.
+__device__ __forceinline__ void segment_gradients(const SegArgs& g, const SegScalars& w, const SegSteps& st, int h, size_t row, int rows, size_t unit, int lane) {
+  const int t = 2 * lane, blk = lane >> 3;
+  const float2 d = *reinterpret_cast<const float2*>(st.dt + t);
+  float s0 = 0.f, s1 = 0.f;               // s of these steps (columns)
+  float below0 = 0.f, below1 = 0.f;       // the same from the row blocks below the diagonal one
+  float left0 = 0.f, left1 = 0.f;         // sums of these steps' rows over the column blocks left of the diagonal one
+  float across = 0.f;                     // blocks below and left of the diagonal one, whole
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float2 c = *reinterpret_cast<const float2*>(w.s[k] + t), r = *reinterpret_cast<const float2*>(w.ga[k] + t);
+    if (k > blk) { below0 += c.x; below1 += c.y; }
+    if (k == blk) { s0 = c.x; s1 = c.y; }
+    if (k < blk) { left0 += r.x; left1 += r.y; }
+    const float all = warp_reduce_width<SumOp, 8>(k < blk ? r.x + r.y : 0.f);   // block (blk, k)
+#pragma unroll
+    for (int i = k + 2; i < 4; ++i) {
+      const float v = __shfl_sync(0xffffffffu, all, i * 8);
+      if (k < blk && blk < i) across += v;
+    }
+  }
+  s0 += below0;
+  s1 += below1;
+  float u0 = 0.f, u1 = 0.f, v0 = 0.f, v1 = 0.f;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const float2 u = *reinterpret_cast<const float2*>(w.su[k] + t), v = *reinterpret_cast<const float2*>(w.sv[k] + t);
+    u0 += u.x; u1 += u.y; v0 += v.x; v1 += v.y;
+  }
+  s0 += v0;
+  s1 += v1;
+  v0 *= d.x;
+  v1 *= d.y;
+  const float q0 = d.x * below0, q1 = d.y * below1;
+  float suf = u0 + u1, pre = v0 + v1;                       // over the segment: this lane's steps and those behind / before them
+  float suf_b = left0 + left1, pre_b = q0 + q1;             // over the block
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const float dn = __shfl_down_sync(0xffffffffu, suf, off), up = __shfl_up_sync(0xffffffffu, pre, off);
+    if (lane + off < 32) suf += dn;
+    if (lane >= off) pre += up;
+    if (off < 8) {
+      const float dn_b = __shfl_down_sync(0xffffffffu, suf_b, off, 8), up_b = __shfl_up_sync(0xffffffffu, pre_b, off, 8);
+      if ((lane & 7) + off < 8) suf_b += dn_b;
+      if ((lane & 7) >= off) pre_b += up_b;
+    }
+  }
+  float suf1 = __shfl_down_sync(0xffffffffu, suf, 1), pre0 = __shfl_up_sync(0xffffffffu, pre, 1);
+  float suf1_b = __shfl_down_sync(0xffffffffu, suf_b, 1, 8), pre0_b = __shfl_up_sync(0xffffffffu, pre_b, 1, 8);
+  if (lane == 31) suf1 = 0.f;
+  if (lane == 0) pre0 = 0.f;
+  if ((lane & 7) == 7) suf1_b = 0.f;
+  if ((lane & 7) == 0) pre0_b = 0.f;
+  float through = 0.f;
+#pragma unroll
+  for (int k = 0; k < SR_WARPS; ++k) through += w.pin[k];
+  through *= segment_exp(st.cum[SG_Q - 1]);
+  const float2 tri = *reinterpret_cast<const float2*>(w.tri + t);
+  const float ga0 = tri.x + suf_b + pre0_b + across + (suf + pre0 + through);
+  const float ga1 = tri.y + left1 + suf1_b + (pre0_b + q0) + across + (u1 + suf1 + pre0 + v0 + through);
+  const float a = g.A[h];
+  float* gdt = g.gdt + (row + t) * g.H + h;
+  if (t < rows) gdt[0] = fmaf(a, ga0, s0);
+  if (t + 1 < rows) gdt[g.H] = fmaf(a, ga1, s1);
+  const float sum = warp_reduce<SumOp>(d.x * ga0 + d.y * ga1);
+  if (lane == 0) g.ga_part[unit] = sum;
+}
+
+// The sums of M G X that s and ga are made of, from one block of it (w).
+__device__ __forceinline__ void block_sums(const float (&w)[2][4], const float* dt, SegScalars& sc, int ib, int jb, int lane) {
+  const int q = lane & 3, r = lane >> 2;
+  // over the block's rows: four columns a lane, one of them left to each half of the lanes with this q twice, then added up
+  float c[2][2], c2[2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) c[u][e] = w[u][e] + w[u][2 + e];
+  const bool b16 = lane & 16, b8 = lane & 8;
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const float other = __shfl_xor_sync(0xffffffffu, b16 ? c[0][e] : c[1][e], 16);
+    c2[e] = (b16 ? c[1][e] : c[0][e]) + other;
+  }
+  const float other = __shfl_xor_sync(0xffffffffu, b8 ? c2[0] : c2[1], 8);
+  float c1 = (b8 ? c2[1] : c2[0]) + other;
+  c1 += __shfl_xor_sync(0xffffffffu, c1, 4);
+  if ((lane & 4) == 0) sc.s[ib][jb * 16 + (b16 ? 8 : 0) + 2 * q + (b8 ? 1 : 0)] = c1;
+  float p[2][4];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const float2 dj = *reinterpret_cast<const float2*>(dt + jb * 16 + u * 8 + 2 * q);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) p[u][e] = w[u][e] * (e & 1 ? dj.y : dj.x);
+  }
+  if (ib != jb) {   // over the block's columns
+    float s0 = (p[0][0] + p[0][1]) + (p[1][0] + p[1][1]), s1 = (p[0][2] + p[0][3]) + (p[1][2] + p[1][3]);
+#pragma unroll
+    for (int off = 1; off < 4; off <<= 1) {
+      s0 += __shfl_xor_sync(0xffffffffu, s0, off);
+      s1 += __shfl_xor_sync(0xffffffffu, s1, off);
+    }
+    if (q == 0) { sc.ga[jb][ib * 16 + r] = s0; sc.ga[jb][ib * 16 + r + 8] = s1; }
+    return;
+  }
+  // the diagonal block: sum_{i >= t > j}, in a row the sum over the columns before t, then over the rows
+  float t4[2][2] = {};
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {   // row r, row r + 8
+    float base = 0.f;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const float q0 = p[u][2 * k], q1 = p[u][2 * k + 1];
+      float sum = q0 + q1;
+#pragma unroll
+      for (int off = 1; off < 4; off <<= 1) {
+        const float up = __shfl_up_sync(0xffffffffu, sum, off, 4);
+        if (q >= off) sum += up;
+      }
+      float ex = __shfl_up_sync(0xffffffffu, sum, 1, 4);
+      const float all = __shfl_sync(0xffffffffu, sum, 3, 4);
+      if (q == 0) ex = 0.f;
+      ex += base;
+      const int j = u * 8 + 2 * q, i = r + 8 * k;
+      if (j <= i) t4[u][0] += ex;
+      if (j + 1 <= i) t4[u][1] += ex + q0;
+      base += all;
+    }
+  }
+  float t2[2];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const float o = __shfl_xor_sync(0xffffffffu, b16 ? t4[0][e] : t4[1][e], 16);
+    t2[e] = (b16 ? t4[1][e] : t4[0][e]) + o;
+  }
+  const float o = __shfl_xor_sync(0xffffffffu, b8 ? t2[0] : t2[1], 8);
+  float t1 = (b8 ? t2[1] : t2[0]) + o;
+  t1 += __shfl_xor_sync(0xffffffffu, t1, 4);
+  if ((lane & 4) == 0) sc.tri[jb * 16 + (b16 ? 8 : 0) + 2 * q + (b8 ? 1 : 0)] = t1;
+}
+
+// Rows' dot products over a warp's 16 columns: those of `v` with the tile's, and v[row] *= f[row] before.
+__device__ __forceinline__ void row_dots(float (&v)[2][2][4], const float* f, uint32_t tile, int nb, float* out, int part, int lane) {
+  const int q = lane & 3, r = lane >> 2;
+#pragma unroll
+  for (int rb = 0; rb < 2; ++rb) {
+    const int i = row_block<2>(rb, part) * 16 + r;
+    const float f0 = f[i], f1 = f[i + 8];
+    float d0 = 0.f, d1 = 0.f;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      uint32_t t0, t1;
+      asm volatile("ld.shared.b32 %0, [%1];" : "=r"(t0) : "r"(tile_at<SG_N * 2>(tile, i, nb * 2 + u) + 4 * q) : "memory");
+      asm volatile("ld.shared.b32 %0, [%1];" : "=r"(t1) : "r"(tile_at<SG_N * 2>(tile, i + 8, nb * 2 + u) + 4 * q) : "memory");
+      const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&t0)), b = __half22float2(*reinterpret_cast<const __half2*>(&t1));
+      v[rb][u][0] *= f0; v[rb][u][1] *= f0; v[rb][u][2] *= f1; v[rb][u][3] *= f1;
+      d0 += a.x * v[rb][u][0] + a.y * v[rb][u][1];
+      d1 += b.x * v[rb][u][2] + b.y * v[rb][u][3];
+    }
+#pragma unroll
+    for (int off = 1; off < 4; off <<= 1) {
+      d0 += __shfl_xor_sync(0xffffffffu, d0, off);
+      d1 += __shfl_xor_sync(0xffffffffu, d1, off);
+    }
+    if (q == 0) { out[i] = d0; out[i + 8] = d1; }
+  }
+}
+
+// Gradients of heads h_first .. h_end - 1 of a group in one segment; gB and gC of the heads stay in registers.
+// The first 256 threads of the CTA; thread (ty, tx): scores as in segment_scores; everything else rows 4 ty .. 4 ty + 3, head columns 4 tx .. 4 tx + 3, state columns
+// 4 tx .. 4 tx + 3 and those 64 further.
+__device__ __noinline__ void segment_reverse_plain(const SegArgs& g, float* smem, int b, int seg, int grp, int split, int h_first, int h_end) {
+  float* sB = smem;                              // [64][132]
   float* sC = sB + SG_Q * SG_NPITCH;             // [64][132]
   float* sG = sC + SG_Q * SG_NPITCH;             // [64][68] G
   float* sMG = sG + SG_Q * SG_PPITCH;            // [64][68] M G
@@ -325,26 +1069,20 @@ __global__ void __launch_bounds__(SG_THREADS, 1) segment_reverse_kernel(const Se
   float* sX = sMX + SG_Q * SG_PPITCH;            // [64][68]
   float* sGy = sX + SG_Q * SG_PPITCH;            // [64][68]
   float* sS = sGy + SG_Q * SG_PPITCH;            // [128][64] state: Y, then H
-  double* cum = reinterpret_cast<double*>(sS + SG_STATE);
+  double* cum = reinterpret_cast<double*>(sS + SG_N * SG_P);
   float* dt = reinterpret_cast<float*>(cum + SG_Q);
   float* su = dt + SG_Q;                         // [64] exp(cum_i) <C_i, H gy_i>
   float* sv = su + SG_Q;                         // [64] e_j <B_j, Y x_j>
   float* part = sv + SG_Q;                       // [2][8 warps][64]: parts of s and ga from inside the segment
   float* red = part + 2 * 8 * SG_Q;              // [8]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ty = threadIdx.x / 16, tx = threadIdx.x % 16;
-  const int hpg = g.H / g.G;
-  const int split = blockIdx.x % g.splits;
-  int rest = blockIdx.x / g.splits;
-  const int grp = rest % g.G;
-  rest /= g.G;
-  const int seg = rest % g.nseg, b = rest / g.nseg;
   const int t0 = seg * SG_Q, rows = min(SG_Q, g.L - t0);
   const bool before = seg > 0, behind = seg < g.nseg - 1;
   const size_t row = static_cast<size_t>(b) * g.L + t0;
   const int r0 = ty * 4, c0 = tx * 4, rb = ty / 4 * 16;   // rb: first row of the 16-row block (the same for a whole warp)
-  segment_tile<SG_N, SG_NPITCH>(sB, g.Bm + (row * g.G + grp) * SG_N, static_cast<size_t>(g.G) * SG_N, rows, g.vec, nullptr);
-  segment_tile<SG_N, SG_NPITCH>(sC, g.Cm + (row * g.G + grp) * SG_N, static_cast<size_t>(g.G) * SG_N, rows, g.vec, nullptr);
-  __syncthreads();
+  plain_tile<SG_N, SG_NPITCH, SG_THREADS>(sB, g.Bm + (row * g.G + grp) * SG_N, static_cast<size_t>(g.G) * SG_N, rows);
+  plain_tile<SG_N, SG_NPITCH, SG_THREADS>(sC, g.Cm + (row * g.G + grp) * SG_N, static_cast<size_t>(g.G) * SG_N, rows);
+  named_bar_sync(1, SG_THREADS);
   {
     float s[4][4];
     segment_scores<SG_N, SG_NPITCH>(sC, sB, ty, tx, s);
@@ -354,19 +1092,18 @@ __global__ void __launch_bounds__(SG_THREADS, 1) segment_reverse_kernel(const Se
       for (int v = 0; v <= u; ++v) sG[(ty + 16 * u) * SG_PPITCH + tx + 16 * v] = s[u][v];
   }
   float gB[4][8] = {}, gC[4][8] = {};
-  const int h_first = grp * hpg + static_cast<int>(static_cast<long long>(hpg) * split / g.splits);
-  const int h_end = grp * hpg + static_cast<int>(static_cast<long long>(hpg) * (split + 1) / g.splits);
 #pragma unroll 1
   for (int h = h_first; h < h_end; ++h) {
     const size_t unit = (static_cast<size_t>(b) * g.H + h) * g.nseg + seg;
-    const float* hstate = g.states + unit * SG_STATE;
-    const float* ystate = g.states + (static_cast<size_t>(g.B) * g.H * g.nseg + unit) * SG_STATE;
-    __syncthreads();   // the previous head's tiles and scalars have been read (and sG is complete)
+    const size_t yunit = static_cast<size_t>(g.B) * g.H * g.nseg + unit;
+    const unsigned char *hstate = g.states + unit * SG_STATE_BYTES, *ystate = g.states + yunit * SG_STATE_BYTES;
+    const float *hscales = g.scales + unit * SG_BLOCKS, *yscales = g.scales + yunit * SG_BLOCKS;
+    named_bar_sync(1, SG_THREADS);   // the previous head's tiles and scalars have been read (and sG is complete)
     if (warp == 0) segment_scalars(g, b, h, t0, cum, dt, lane);
-    segment_tile<SG_P, SG_PPITCH>(sX, g.x + (row * g.H + h) * SG_P, static_cast<size_t>(g.H) * SG_P, rows, g.vec, nullptr);
-    segment_tile<SG_P, SG_PPITCH>(sGy, g.gy + (row * g.H + h) * SG_P, static_cast<size_t>(g.H) * SG_P, rows, g.vec, nullptr);
-    if (behind) segment_load_state(sS, ystate);
-    __syncthreads();
+    plain_tile<SG_P, SG_PPITCH, SG_THREADS>(sX, g.x + (row * g.H + h) * SG_P, static_cast<size_t>(g.H) * SG_P, rows);
+    plain_tile<SG_P, SG_PPITCH, SG_THREADS>(sGy, g.gy + (row * g.H + h) * SG_P, static_cast<size_t>(g.H) * SG_P, rows);
+    if (behind) plain_state<SG_THREADS>(sS, ystate, yscales);
+    named_bar_sync(1, SG_THREADS);
     {
       float s[4][4];
       segment_scores<SG_P, SG_PPITCH>(sGy, sX, ty, tx, s);
@@ -380,7 +1117,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) segment_reverse_kernel(const Se
           sMG[o] = m * sG[o];
         }
     }
-    __syncthreads();
+    named_bar_sync(1, SG_THREADS);
     const double last = cum[SG_Q - 1];
     {   // s and ga from inside the segment: a warp takes eight rows, a lane two columns
       const float d0 = dt[2 * lane], d1 = dt[2 * lane + 1];
@@ -524,23 +1261,20 @@ __global__ void __launch_bounds__(SG_THREADS, 1) segment_reverse_kernel(const Se
 #pragma unroll
         for (int c = 0; c < 8; ++c) gB[r][c] = fmaf(dr[r], o[r][c], gB[r][c]);
     }
-    __syncthreads();   // Y has been read
+    named_bar_sync(1, SG_THREADS);   // Y has been read
     float pin = 0.f;
     if (before) {
-#pragma unroll
-      for (int k = 0; k < SG_STATE / 4 / SG_THREADS; ++k) {
-        const int idx = k * SG_THREADS + threadIdx.x, n = idx / (SG_P / 4), p4 = idx % (SG_P / 4);
-        const float4 v = *reinterpret_cast<const float4*>(hstate + idx * 4);
-        if (behind) {
-          const float4 w = *reinterpret_cast<const float4*>(ystate + idx * 4);
-          pin += v.x * w.x + v.y * w.y + v.z * w.z + v.w * w.w;
-        }
-        *reinterpret_cast<float4*>(sS + state_at(n, p4)) = v;
+#pragma unroll 1
+      for (int idx = threadIdx.x; idx < SG_N * SG_P; idx += SG_THREADS) {
+        const int p = idx / SG_N, n = idx % SG_N;
+        const float v = state_value(hstate, hscales, n, p);
+        if (behind) pin += v * state_value(ystate, yscales, n, p);
+        sS[state_at(n, p >> 2) + (p & 3)] = v;
       }
       pin = warp_reduce<SumOp>(pin);
     }
     if (lane == 0) red[warp] = pin;
-    __syncthreads();
+    named_bar_sync(1, SG_THREADS);
     {   // ---- gC ----
       if (before) {
         state_rows(sGy, o);
@@ -588,7 +1322,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) segment_reverse_kernel(const Se
 #pragma unroll
         for (int c = 0; c < 8; ++c) gC[r][c] += o[r][c];
     }
-    __syncthreads();   // su, sv, red
+    named_bar_sync(1, SG_THREADS);   // su, sv, red
     if (warp == 0) {   // ---- gdt, gA ----
       const int t = 2 * lane;
       float s0 = sv[t], s1 = sv[t + 1], ga0 = 0.f, ga1 = 0.f;
@@ -636,6 +1370,211 @@ __global__ void __launch_bounds__(SG_THREADS, 1) segment_reverse_kernel(const Se
   }
 }
 
+__global__ void __launch_bounds__(SR_THREADS, 1) segment_reverse_kernel(const SegArgs g) {
+  mp_grid_dependency();
+  extern __shared__ __align__(128) unsigned char seg_smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane & 3, r0 = lane >> 2;
+  const int cols = warp & 7, part = warp >> 3;
+  const SegShare sh = segment_share(g);
+  const int t0 = sh.seg * SG_Q, rows = min(SG_Q, g.L - t0);
+  const bool before = sh.seg > 0, behind = sh.seg < g.nseg - 1;
+  const size_t row = static_cast<size_t>(sh.b) * g.L + t0;
+  const uint32_t smem = mp_smem_u32(seg_smem), sB = smem, sC = sB + SG_Q * SG_N * 2, stages = sC + SG_Q * SG_N * 2, sY = stages + 2 * SR_STAGE;
+  const uint32_t sWh = sY + SR_S, sWl = sWh + SG_Q * SG_Q * 2, sMh = sWl + SG_Q * SG_Q * 2, sMl = sMh + SG_Q * SG_Q * 2;   // M X dt, M G
+  SegSteps* steps = reinterpret_cast<SegSteps*>(seg_smem + SR_TILES);
+  SegScalars* scalars = reinterpret_cast<SegScalars*>(steps + 3);
+  float *invW = reinterpret_cast<float*>(scalars + 2), *invM = invW + 16;
+  const float* yscales = reinterpret_cast<const float*>(seg_smem + (sY + SG_STATE_BYTES - smem));
+  auto unit_of = [&](int h) { return (static_cast<size_t>(sh.b) * g.H + h) * g.nseg + sh.seg; };
+  auto load_stage = [&](int h) {
+    const uint32_t st = stages + ((h - sh.h_first) & 1) * SR_STAGE;
+    tile_load<SG_P / 8, SR_THREADS>(st, g.x + (row * g.H + h) * SG_P, static_cast<size_t>(g.H) * SG_P, rows, g.vec);
+    tile_load<SG_P / 8, SR_THREADS>(st + SR_X, g.gy + (row * g.H + h) * SG_P, static_cast<size_t>(g.H) * SG_P, rows, g.vec);
+    if (before) state_load<SR_THREADS>(st + 2 * SR_X, g.states + unit_of(h) * SG_STATE_BYTES, g.scales + unit_of(h) * SG_BLOCKS);
+  };
+  auto load_adjoint = [&](int h) {
+    const size_t unit = static_cast<size_t>(g.B) * g.H * g.nseg + unit_of(h);
+    if (behind) state_load<SR_THREADS>(sY, g.states + unit * SG_STATE_BYTES, g.scales + unit * SG_BLOCKS);
+  };
+  tile_load<SG_N / 8, SR_THREADS>(sB, g.Bm + (row * g.G + sh.grp) * SG_N, static_cast<size_t>(g.G) * SG_N, rows, g.vec);
+  tile_load<SG_N / 8, SR_THREADS>(sC, g.Cm + (row * g.G + sh.grp) * SG_N, static_cast<size_t>(g.G) * SG_N, rows, g.vec);
+  cp_async_commit();
+  load_stage(sh.h_first);
+  load_adjoint(sh.h_first);
+  cp_async_commit();
+  if (warp == 15) segment_steps(g, sh.b, sh.h_first, t0, steps[0], lane);
+  cp_async_wait<1>();
+  __syncthreads();
+  float G[2][4];   // C B^T of the warp's block
+  int ib, jb;
+  const bool scores = block_of(warp, ib, jb);
+  if (scores) block_scores<SG_N>(G, sC, sB, ib, jb, lane);
+  float gB[2][2][4] = {}, gC[2][2][4] = {};
+#pragma unroll 1
+  for (int h = sh.h_first; h < sh.h_end; ++h) {
+    const int n = h - sh.h_first;
+    const uint32_t sx = stages + (n & 1) * SR_STAGE, sgy = sx + SR_X, sH = sgy + SR_X;
+    const float* hscales = reinterpret_cast<const float*>(seg_smem + (sH + SG_STATE_BYTES - smem));
+    cp_async_wait<0>();
+    __syncthreads();   // this head's tiles are there, the other stage, the weights and the last head's scalars are complete and read
+    if (h + 1 < sh.h_end) {
+      load_stage(h + 1);
+      if (warp == 15) segment_steps(g, sh.b, h + 1, t0, steps[(n + 1) % 3], lane);
+    }
+    cp_async_commit();
+    if (warp == 14 && n > 0) segment_gradients(g, scalars[(n - 1) & 1], steps[(n - 1) % 3], h - 1, row, rows, unit_of(h - 1), lane);
+    SegScalars& sc = scalars[n & 1];
+    const SegSteps& st = steps[n % 3];
+    // ---- scores: M X dt and M G in two terms, the sums of M G X ----
+    if (scores) {
+      float x[2][4], m[2][4], w[2][4];
+      block_scores<SG_P>(x, sgy, sx, ib, jb, lane);
+      block_decays(m, st.cum, ib, jb, r0, q);
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          x[u][e] *= m[u][e];
+          w[u][e] = x[u][e] * G[u][e];
+          m[u][e] *= G[u][e];
+        }
+      if (ib == jb)   // beyond the diagonal a score may be infinite
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (u * 8 + 2 * q + (e & 1) > r0 + (e >> 1) * 8) x[u][e] = w[u][e] = m[u][e] = 0.f;
+      block_sums(w, st.dt, sc, ib, jb, lane);
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const float2 dj = *reinterpret_cast<const float2*>(st.dt + jb * 16 + u * 8 + 2 * q);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x[u][e] *= e & 1 ? dj.y : dj.x;
+      }
+      block_split(x, sWh, sWl, invW, ib, jb, lane);
+      block_split(m, sMh, sMl, invM, ib, jb, lane);
+    }
+    {   // ---- <Y, H> ----
+      float pin = 0.f;
+      if (before && behind) {
+#pragma unroll
+        for (int k = 0; k < SG_STATE_BYTES / 32 / SR_THREADS; ++k) {
+          const int idx = k * SR_THREADS + threadIdx.x, p = idx >> 4, c = ((idx & 15) >> 1) * 4 + (idx & 1);   // a chunk of upper terms
+          const uint4 yh = ld_shared16(tile_at<512>(sY, p, c)), yl = ld_shared16(tile_at<512>(sY, p, c + 2));
+          const uint4 hh = ld_shared16(tile_at<512>(sH, p, c)), hl = ld_shared16(tile_at<512>(sH, p, c + 2));
+          const uint32_t a[4] = {yh.x, yh.y, yh.z, yh.w}, al[4] = {yl.x, yl.y, yl.z, yl.w}, b[4] = {hh.x, hh.y, hh.z, hh.w}, bl[4] = {hl.x, hl.y, hl.z, hl.w};
+          float part = 0.f;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 y0 = __half22float2(*reinterpret_cast<const __half2*>(&a[e])), y1 = __half22float2(*reinterpret_cast<const __half2*>(&al[e]));
+            const float2 h0 = __half22float2(*reinterpret_cast<const __half2*>(&b[e])), h1 = __half22float2(*reinterpret_cast<const __half2*>(&bl[e]));
+            part += (y0.x + y1.x) * (h0.x + h1.x) + (y0.y + y1.y) * (h0.y + h1.y);
+          }
+          const int blk = (p >> 4) * 8 + (c >> 2);
+          pin += part * yscales[blk] * hscales[blk];
+        }
+        pin = warp_reduce<SumOp>(pin);
+      }
+      if (lane == 0) sc.pin[warp] = pin;
+    }
+    // ---- the adjoint state's part of gB and gx ----
+    float o[2][1][4];
+    if (behind) {
+      float v[2][2][4], p[2][4];
+      times_state_n<2>(v, sx, sY, yscales, cols, part, lane);
+      row_dots(v, st.left, sB, cols, sc.sv[cols], part, lane);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int r = row_block<2>(i, part) * 16 + r0;
+        const float d0 = st.dt[r], d1 = st.dt[r + 8];
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) gB[i][u][e] = fmaf(e < 2 ? d0 : d1, v[i][u][e], gB[i][u][e]);
+      }
+      times_state_p<2>(p, sB, sY, yscales, cols, part, lane);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int r = row_block<2>(i, part) * 16 + r0;
+        const float e0 = st.left[r], e1 = st.left[r + 8];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[i][0][e] = p[i][e] * (e < 2 ? e0 : e1);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[i][0][e] = 0.f;
+      if (part == 0 && lane < 16) *reinterpret_cast<float4*>(sc.sv[cols] + lane * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __syncthreads();   // the weights are complete, Y has been read
+    if (h + 1 < sh.h_end) load_adjoint(h + 1);
+    cp_async_commit();
+    // ---- gx ----
+    {
+      uint32_t b[4][2];
+      load_steps(b, sgy, cols, lane);
+      times_scores<2, false, 1>(o, sMh, sMl, invM, b, part, lane);
+      __half* gx = g.gx + (row * g.H + h) * SG_P + cols * 8 + 2 * q;
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const int j = row_block<2>(i, part) * 16 + r * 8 + r0;
+          const float d = st.dt[j];
+          if (j < rows) store_pair(gx + static_cast<size_t>(j) * g.H * SG_P, o[i][0][2 * r] * d, o[i][0][2 * r + 1] * d, g.vec);
+        }
+    }
+    // ---- gC, gB ----
+    if (before) {
+      float v[2][2][4];
+      times_state_n<2>(v, sgy, sH, hscales, cols, part, lane);
+      row_dots(v, st.grow, sC, cols, sc.su[cols], part, lane);
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) gC[i][u][e] += v[i][u][e];
+    } else if (part == 0 && lane < 16) {
+      *reinterpret_cast<float4*>(sc.su[cols] + lane * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    uint32_t b[4][4];   // these columns of B, then of C, over the steps
+#pragma unroll
+    for (int k = 0; k < 4; ++k) load_b_t<SG_N * 2>(b[k], sB, k * 16, cols * 2, lane);
+    times_scores<2, true, 2>(gC, sWh, sWl, invW, b, part, lane);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) load_b_t<SG_N * 2>(b[k], sC, k * 16, cols * 2, lane);
+    times_scores<2, false, 2>(gB, sWh, sWl, invW, b, part, lane);
+  }
+  float check = 0.f;   // becomes NaN with the first result that is none, or infinite
+  const size_t bc = static_cast<size_t>(g.B) * g.L * g.G * SG_N;
+  float* out = g.gb_part + static_cast<size_t>(sh.split) * 2 * bc + (row * g.G + sh.grp) * SG_N + cols * 16 + 2 * q;
+#pragma unroll
+  for (int rb = 0; rb < 2; ++rb)
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int i = row_block<2>(rb, part) * 16 + r * 8 + r0;
+        const float b0 = gB[rb][u][2 * r], b1 = gB[rb][u][2 * r + 1], c0 = gC[rb][u][2 * r], c1 = gC[rb][u][2 * r + 1];
+        check = fmaf(b0, 0.f, fmaf(b1, 0.f, fmaf(c0, 0.f, fmaf(c1, 0.f, check))));
+        if (i >= rows) continue;
+        float* o = out + static_cast<size_t>(i) * g.G * SG_N + u * 8;
+        *reinterpret_cast<float2*>(o) = make_float2(b0, b1);
+        *reinterpret_cast<float2*>(o + bc) = make_float2(c0, c1);
+      }
+  const bool again = __syncthreads_or(check != 0.f);
+  if (warp == 14) {
+    const int n = sh.h_end - 1 - sh.h_first;
+    segment_gradients(g, scalars[n & 1], steps[n % 3], sh.h_end - 1, row, rows, unit_of(sh.h_end - 1), lane);
+  }
+  if (again) {
+    __syncthreads();
+    if (threadIdx.x < SR_THREADS / 2) segment_reverse_plain(g, reinterpret_cast<float*>(seg_smem), sh.b, sh.seg, sh.grp, sh.split, sh.h_first, sh.h_end);
+  }
+}
+
 // gB (blockIdx.y = 0) and gC (1): the sums of the head shares, rounded; four neighbouring values per thread.
 __global__ void __launch_bounds__(SG_THREADS) segment_fold_kernel(const float* __restrict__ part, __half* gB, __half* gC, size_t bc, int splits, bool vec) {
   mp_grid_dependency();
@@ -662,33 +1601,48 @@ __global__ void __launch_bounds__(32) segment_sum_kernel(const float* __restrict
 }
 
 constexpr size_t SG_SCALARS = SG_Q * (sizeof(double) + sizeof(float));
-constexpr size_t SG_SMEM_STATES = (SG_Q * (SG_NPITCH + SG_PPITCH) + SG_Q) * sizeof(float) + SG_SCALARS;
-constexpr size_t SG_SMEM_FORWARD = SG_Q * 2 * (SG_NPITCH + SG_PPITCH) * sizeof(float) + SG_SCALARS;
-constexpr size_t SG_SMEM_REVERSE = (SG_Q * (2 * SG_NPITCH + 5 * SG_PPITCH) + SG_STATE + (2 + 16) * SG_Q + 8) * sizeof(float) + SG_SCALARS;
-static_assert(SG_STATE <= SG_Q * SG_NPITCH, "the state takes the place of B");
+constexpr size_t SG_PLAIN_FORWARD = SG_Q * 2 * (SG_NPITCH + SG_PPITCH) * sizeof(float) + SG_SCALARS;
+constexpr size_t SG_PLAIN_REVERSE = (SG_Q * (2 * SG_NPITCH + 5 * SG_PPITCH) + SG_N * SG_P + (2 + 16) * SG_Q + 8) * sizeof(float) + SG_SCALARS;
+constexpr size_t SG_SMEM_FORWARD = SF_SMEM > SG_PLAIN_FORWARD ? SF_SMEM : SG_PLAIN_FORWARD;
+constexpr size_t SG_SMEM_REVERSE = SR_SMEM > SG_PLAIN_REVERSE ? SR_SMEM : SG_PLAIN_REVERSE;
+static_assert(SG_N * SG_P <= SG_Q * SG_NPITCH, "the state takes the place of B");
+static_assert(2 * SG_SMEM_FORWARD <= 226 * 1024 && SG_SMEM_REVERSE <= 227 * 1024, "shared memory of an SM");
+static_assert(SF_S % 128 == 0 && SR_STAGE % 128 == 0, "tiles keep the phase of their chunks");
 
-// Heads of a group per CTA of the reverse: shares until there are four CTAs per SM to hand out.
-int segment_splits(int B, int L, int H, int G) {
+// Shares of a group's heads: a CTA's time is its heads' and about `setup` heads' worth of loading, scores and writing of gB and gC (which
+// are also folded over the shares: `fold` per CTA of the whole grid), `slots` CTAs run at a time.
+int segment_splits(int B, int L, int H, int G, int slots, float setup, float fold) {
   const long units = static_cast<long>(B) * ((L + SG_Q - 1) / SG_Q) * G;
-  const long want = (4 * 148 + units - 1) / units, hpg = H / G;
-  return static_cast<int>(want < 1 ? 1 : (want < hpg ? want : hpg));
+  const int hpg = H / G;
+  int best = 1;
+  float best_cost = 0.f;
+  for (int s = 1; s <= hpg; ++s) {
+    const int heads = (hpg + s - 1) / s;
+    if (s > 1 && heads == (hpg + s - 2) / (s - 1)) continue;   // no fewer heads than with one share less
+    const float cost = static_cast<float>((units * s + slots - 1) / slots) * (heads + setup) + fold * units * s;
+    if (s == 1 || cost < best_cost) { best = s; best_cost = cost; }
+  }
+  return best;
 }
+int forward_splits(int B, int L, int H, int G) { return segment_splits(B, L, H, G, 2 * 148, 0.7f, 0.f); }
+int reverse_splits(int B, int L, int H, int G) { return segment_splits(B, L, H, G, 148, 0.7f, 0.005f); }
 
-struct SegScratch { float* states; float* decay; float* ga_part; float* gb_part; size_t total; };
+struct SegScratch { unsigned char* states; float* scales; float* decay; float* ga_part; float* gb_part; size_t total; };
 SegScratch segment_carve(void* base, int B, int L, int H, int G, bool reverse) {
   SegScratch s;
   const size_t start = (256 - (reinterpret_cast<uintptr_t>(base) & 255)) & 255;   // the caller's pointer may have any alignment
   size_t off = 0;
-  auto take = [&](size_t floats) {
-    float* p = base != nullptr ? reinterpret_cast<float*>(static_cast<unsigned char*>(base) + start + off) : nullptr;
-    off += (floats * sizeof(float) + 255) & ~size_t(255);
+  auto take = [&](size_t bytes) {
+    unsigned char* p = base != nullptr ? static_cast<unsigned char*>(base) + start + off : nullptr;
+    off += (bytes + 255) & ~size_t(255);
     return p;
   };
   const size_t units = static_cast<size_t>(B) * H * ((static_cast<size_t>(L) + SG_Q - 1) / SG_Q);
-  s.states = take(units * SG_STATE * (reverse ? 2 : 1));
-  s.decay = take(units);
-  s.ga_part = take(reverse ? units : 0);
-  s.gb_part = take(reverse ? static_cast<size_t>(segment_splits(B, L, H, G)) * 2 * B * L * G * SG_N : 0);
+  s.states = take(units * SG_STATE_BYTES * (reverse ? 2 : 1));
+  s.scales = reinterpret_cast<float*>(take(units * SG_BLOCKS * sizeof(float) * (reverse ? 2 : 1)));
+  s.decay = reinterpret_cast<float*>(take(units * sizeof(float)));
+  s.ga_part = reinterpret_cast<float*>(take(reverse ? units * sizeof(float) : 0));
+  s.gb_part = reinterpret_cast<float*>(take(reverse ? static_cast<size_t>(reverse_splits(B, L, H, G)) * 2 * B * L * G * SG_N * sizeof(float) : 0));
   s.total = off + 256;
   return s;
 }
@@ -697,7 +1651,7 @@ SegArgs segment_args(const void* x, const void* dt, const void* A, const void* B
   SegArgs g{};
   g.x = static_cast<const __half*>(x); g.dt = static_cast<const float*>(dt); g.A = static_cast<const float*>(A);
   g.Bm = static_cast<const __half*>(Bm); g.Cm = static_cast<const __half*>(Cm);
-  g.states = w.states; g.decay = w.decay; g.ga_part = w.ga_part; g.gb_part = w.gb_part;
+  g.states = w.states; g.scales = w.scales; g.decay = w.decay; g.ga_part = w.ga_part; g.gb_part = w.gb_part;
   g.B = B; g.L = L; g.H = H; g.G = G; g.nseg = (L + SG_Q - 1) / SG_Q;
   g.vec = mp_aligned16(x) && mp_aligned16(Bm) && mp_aligned16(Cm);
   return g;
@@ -705,13 +1659,12 @@ SegArgs segment_args(const void* x, const void* dt, const void* A, const void* B
 
 // The states every segment receives, in one direction or both.
 void segment_state_launches(const SegArgs& g, int directions, cudaStream_t st) {
-  MP_CUDA_CHECK(cudaFuncSetAttribute(segment_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SG_SMEM_STATES)));
-  MpLaunch(dim3(g.B * g.H * g.nseg, directions), SG_THREADS, SG_SMEM_STATES, st)(segment_states_kernel, g);
+  if (g.nseg == 1) return;
+  MP_CUDA_CHECK(cudaFuncSetAttribute(segment_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SS_SMEM)));
+  MpLaunch(dim3(g.B * g.H * g.nseg, directions), SS_THREADS, SS_SMEM, st)(segment_states_kernel, g);
   MP_LAUNCH_CHECK();
-  if (g.nseg > 1) {
-    MpLaunch(dim3(g.B * g.H * (SG_STATE / 4 / SG_THREADS), directions), SG_THREADS, 0, st)(segment_carry_kernel, g);
-    MP_LAUNCH_CHECK();
-  }
+  MpLaunch(dim3(g.B * g.H * (SG_BLOCKS / (SC_THREADS / 32)), directions), SC_THREADS, 0, st)(segment_carry_kernel, g);
+  MP_LAUNCH_CHECK();
 }
 
 }  // namespace
@@ -728,9 +1681,10 @@ void mp_ssd_segments_forward(const void* x, const void* dt, const void* A, const
   SegArgs g = segment_args(x, dt, A, Bm, Cm, segment_carve(scratch, B, L, H, G, false), B, L, H, G);
   g.y = static_cast<__half*>(y);
   g.vec = g.vec && mp_aligned16(y);
-  if (g.nseg > 1) segment_state_launches(g, 1, st);
+  g.splits = forward_splits(B, L, H, G);
+  segment_state_launches(g, 1, st);
   MP_CUDA_CHECK(cudaFuncSetAttribute(segment_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SG_SMEM_FORWARD)));
-  MpLaunch(B * H * g.nseg, SG_THREADS, SG_SMEM_FORWARD, st)(segment_forward_kernel, g);
+  MpLaunch(B * g.nseg * G * g.splits, SG_THREADS, SG_SMEM_FORWARD, st)(segment_forward_kernel, g);
   MP_LAUNCH_CHECK();
 }
 
@@ -738,12 +1692,12 @@ void mp_ssd_segments_reverse(const void* x, const void* dt, const void* A, const
                              void* gA, void* gB, void* gC, void* scratch, int B, int L, int H, int G, cudaStream_t st) {
   SegArgs g = segment_args(x, dt, A, Bm, Cm, segment_carve(scratch, B, L, H, G, true), B, L, H, G);
   g.gy = static_cast<const __half*>(gy); g.gx = static_cast<__half*>(gx); g.gdt = static_cast<float*>(gdt);
-  g.splits = segment_splits(B, L, H, G);
+  g.splits = reverse_splits(B, L, H, G);
   const bool fold_vec = mp_aligned16(gB) && mp_aligned16(gC);
   g.vec = g.vec && mp_aligned16(gy) && mp_aligned16(gx);
-  if (g.nseg > 1) segment_state_launches(g, 2, st);
+  segment_state_launches(g, 2, st);
   MP_CUDA_CHECK(cudaFuncSetAttribute(segment_reverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SG_SMEM_REVERSE)));
-  MpLaunch(B * g.nseg * G * g.splits, SG_THREADS, SG_SMEM_REVERSE, st)(segment_reverse_kernel, g);
+  MpLaunch(B * g.nseg * G * g.splits, SR_THREADS, SG_SMEM_REVERSE, st)(segment_reverse_kernel, g);
   MP_LAUNCH_CHECK();
   const size_t bc = static_cast<size_t>(B) * L * G * SG_N;
   MpLaunch(dim3(static_cast<unsigned>((bc / 4 + SG_THREADS - 1) / SG_THREADS), 2), SG_THREADS, 0, st)(segment_fold_kernel, g.gb_part, static_cast<__half*>(gB),

@@ -354,3 +354,34 @@ def test_ssd_segments_keep_fp32(mp, stream, orc, dims, shift, off):
         assert torch.all(flat[:o] == 7) and torch.all(flat[o + want.size:] == 7), f"{name} written outside {dims}"
         d = host(got).astype(np.float64).reshape(want.shape) - want
         assert np.linalg.norm(d) <= tol[name] * np.linalg.norm(want), (name, np.linalg.norm(d) / np.linalg.norm(want))
+
+
+@pytest.mark.parametrize("which,value,dims", [
+    # an infinity or a NaN at two steps, in the middle of a segment and in the last one, which is partly filled: no product may carry it to a step or
+    # a column that the recurrence keeps finite, and what is finite keeps its accuracy
+    (0, np.inf, (1, 200, 4, 64, 128, 2, 128)), (3, -np.inf, (1, 200, 4, 64, 128, 2, 128)), (4, np.inf, (1, 200, 4, 64, 128, 2, 128)),
+    (5, np.inf, (1, 200, 4, 64, 128, 2, 128)), (0, np.nan, (1, 200, 4, 64, 128, 2, 128)), (3, np.inf, (2, 50, 2, 64, 128, 1, 128))])
+def test_ssd_segments_with_infinities(mp, stream, orc, which, value, dims):
+    import torch
+    nb, L, H, P, N, G, Q = dims
+    ins = list(make_inputs(31, nb, L, H, P, N, G))   # x, dt, A, B, C, gy
+    ins[which][0, 27, 0, 3] = ins[which][nb - 1, L - 5, min(1, G - 1) if which in (3, 4) else 1, 5] = value
+    x, dt, A, Bm, Cm, gy = ins
+    outs = [dev(np.full(a.shape, 7, a.dtype)) for a in (x, x, dt, A, Bm, Cm)]
+    y, gx, gdt, gA, gB, gC = outs
+    scratch = scratch_for(mp, dims, True)
+    args = [dev(a) for a in ins]
+    torch.cuda.current_stream().synchronize()
+    mp.launch("ssd_scan", torch.float16, *args[:5], y, scratch, *dims, stream)
+    mp.launch("ssd_scan_reverse", torch.float16, *args, gx, gdt, gA, gB, gC, scratch, *dims, stream)
+    stream.sync()
+    assert stream.status() == 0
+    f64 = [np.ascontiguousarray(a.astype(np.float64)) for a in ins]
+    with np.errstate(all="ignore"):
+        ref = (orc.ssd_forward(*f64[:5]),) + tuple(orc.ssd_reverse(*f64))
+    for got, want, name in zip((y, gx, gB, gC), (ref[0], ref[1], ref[4], ref[5]), ("y", "gx", "gB", "gC")):
+        got = host(got).astype(np.float64)
+        finite = np.isfinite(want)
+        assert np.array_equal(np.isfinite(got), finite), f"{name}: {np.sum(~np.isfinite(got))} not finite, {np.sum(~finite)} expected"
+        d = got[finite] - want[finite]
+        assert np.linalg.norm(d) <= 2.9e-4 * np.linalg.norm(want[finite]), name   # the rounding of an r16 result
