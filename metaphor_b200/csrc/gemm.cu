@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
   constexpr bool WIDE_STORE = BN >= 128;
   extern __shared__ unsigned char gemm_smem_raw[];
   // 1024-byte alignment: swizzle atoms are 8 rows x 128 bytes
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(gemm_smem_raw) + 1023) & ~uintptr_t(1023));
+  unsigned char* smem = mp_smem_align1024(gemm_smem_raw);
   const int stages = g.stages;
   constexpr int stage_sz = A_BYTES + B_BYTES;
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + static_cast<size_t>(stages) * stage_sz);
@@ -456,7 +456,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
   constexpr int ACC_BUFS = 2;
   constexpr int BOX_BYTES = 32 * 64 * sizeof(T);   // one [32 rows][64 columns] staging box
   extern __shared__ unsigned char gemm_smem_raw[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(gemm_smem_raw) + 1023) & ~uintptr_t(1023));
+  unsigned char* smem = mp_smem_align1024(gemm_smem_raw);
   const int stages = g.stages;
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + static_cast<size_t>(stages) * PAIR_STAGE_BYTES);
   uint64_t* empty = full + MAX_STAGES;

@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(R_THREADS, 1) gemm_r32_kernel(const __grid_con
   using Cfg = R32Cfg<BN>;
   constexpr int A_BYTES = Cfg::A_BYTES, B_BYTES = Cfg::B_BYTES, RAW = Cfg::RAW, STAGES = Cfg::STAGES;
   extern __shared__ unsigned char gemm_smem_raw[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(gemm_smem_raw) + 1023) & ~uintptr_t(1023));
+  unsigned char* smem = mp_smem_align1024(gemm_smem_raw);
   unsigned char* lo_ring = smem + STAGES * RAW;
   uint64_t* full = reinterpret_cast<uint64_t*>(lo_ring + R_SLOTS * B_BYTES);   // loads have arrived
   uint64_t* raw_empty = full + R_MAX_STAGES;

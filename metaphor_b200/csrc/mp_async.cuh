@@ -18,6 +18,11 @@ __device__ __forceinline__ uint32_t mp_smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// The first 1024-byte boundary of the dynamic shared memory (swizzle atoms are 8 rows of 128 bytes).  The pointer is moved, not made from an
+// integer: then the compiler still knows that it points to shared memory and does not turn every access behind it into a generic one, which
+// takes the way of the global ones.  Scan at 8 x 8192 x 32 heads, forward and reverse, generic / shared accesses: 1283 / 1220 us.
+__device__ __forceinline__ unsigned char* mp_smem_align1024(unsigned char* raw) { return raw + ((1024u - (mp_smem_u32(raw) & 1023u)) & 1023u); }
+
 __device__ __forceinline__ uint64_t mp_globaltimer_ns() {
   uint64_t t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));

@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(SSD_THREADS, 4) ssd_mma_kernel(const __grid_co
                                                                 const SsdArgs g) {
   mp_grid_dependency();
   extern __shared__ unsigned char ssd_smem_raw[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(ssd_smem_raw) + 1023) & ~uintptr_t(1023));
+  unsigned char* smem = mp_smem_align1024(ssd_smem_raw);
   const int STAGES = g.stages, STAGE_BYTES = g.stage_bytes;
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
   uint64_t* ready = full + SSD_MAX_STAGES;

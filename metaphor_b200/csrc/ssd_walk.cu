@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_walk_kernel(const __grid_con
                                                                const __grid_constant__ CUtensorMap map_v,
                                                                const __grid_constant__ CUtensorMap map_hs, const WalkArgs g) {
   extern __shared__ unsigned char walk_smem_raw[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(walk_smem_raw) + 1023) & ~uintptr_t(1023));
+  unsigned char* smem = mp_smem_align1024(walk_smem_raw);
   unsigned char* sP = smem + W_OFF_P;
   unsigned char* sH = smem + W_OFF_H;
   unsigned char* sVs = smem + W_OFF_VS;
@@ -643,7 +643,7 @@ __global__ void __launch_bounds__(WP2_THREADS, 1) ssd_walk_pair_kernel(const __g
                                                                     const __grid_constant__ CUtensorMap map_out, const WalkArgs g) {
   constexpr bool OUT = ANTI != 0 || !DOT;   // the causal form with row dots has no other output
   extern __shared__ unsigned char walk_smem_raw[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(walk_smem_raw) + 1023) & ~uintptr_t(1023));
+  unsigned char* smem = mp_smem_align1024(walk_smem_raw);
   unsigned char* sV = smem + WP2_OFF_V;
   unsigned char* sH = smem + WP2_OFF_H;
   unsigned char* sVs = smem + WP2_OFF_VS;
@@ -1116,7 +1116,7 @@ __global__ void __launch_bounds__(W_THREADS, 1) ssd_group_grads_kernel(const __g
                                                                       const __grid_constant__ CUtensorMap map_gb,
                                                                       const __grid_constant__ CUtensorMap map_gc, const GroupArgs g) {
   extern __shared__ unsigned char walk_smem_raw[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(walk_smem_raw) + 1023) & ~uintptr_t(1023));
+  unsigned char* smem = mp_smem_align1024(walk_smem_raw);
   unsigned char* sGG = smem + GG_OFF_ACC;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + GG_OFF_TAIL);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + GG_OFF_TAIL + 112);
