@@ -443,6 +443,22 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
 // polls: polling the ring barriers without a suspend hint (as the scan's chunk walk does) made every shape 5 - 8 % slower.
 // ---------------------------------------------------------------------------
 constexpr int PAIR_BN = 256;
+// Tiles in the order of their rows, column by column: the pairs at work share a tile of B and read all of A once per column.  Where A does not
+// stay in the L2 that long, eight row blocks at a time: A is read once, B once per group.  us, all rows / eight at a time: [16384, 3352] x
+// [3352, 768] 88 / 81, [16384, 50280] x [50280, 768] 1196 / 1058, 8192^3 891 / 818 (24 at a time: 82, 1071, 862); where A takes 25 - 50 MB
+// the two are level or all rows are ahead ([16384, 768] x [768, 3352] 84.8 / 84.6, [16384, 768] x [768, 50280] 1042 / 1074).
+constexpr int PAIR_GROUP = 8;
+constexpr double PAIR_GROUP_BYTES = 64e6;   // half of the L2
+__device__ __forceinline__ void pair_tile(const GemmArgs& g, int tile, int tiles_m, int tiles_n, int& tm, int& tn) {
+  if (g.group == 0) {
+    tm = tile % tiles_m;
+    tn = tile / tiles_m;
+    return;
+  }
+  const int per = g.group * tiles_n, first = tile / per * g.group, in = tile % per, rows = min(g.group, tiles_m - first);
+  tm = first + in % rows;
+  tn = in / rows;
+}
 constexpr int PAIR_STAGE_BYTES = BM * SWIZZLE_BYTES + (PAIR_BN / 2) * SWIZZLE_BYTES;   // 32 KB
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
@@ -502,8 +518,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
       bool ok = true;
       for (int unit = pair; unit < num_units && ok; unit += num_pairs) {
         const int tile = unit % num_tiles, sp = unit / num_tiles;
-        const int m0 = (tile % tiles_m) * 2 * BM + static_cast<int>(rank) * BM;
-        const int n0 = (tile / tiles_m) * BN + static_cast<int>(rank) * (BN / 2);
+        int tm, tn;
+        pair_tile(g, tile, tiles_m, tiles_n, tm, tn);
+        const int m0 = tm * 2 * BM + static_cast<int>(rank) * BM, n0 = tn * BN + static_cast<int>(rank) * (BN / 2);
         const int kb0 = sp * kb_per, kb1 = min(num_kb, kb0 + kb_per);
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           if (!mbar_wait_abortable(empty + s, phase ^ 1u, g.status, abort)) { ok = false; break; }
@@ -578,7 +595,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
       const int tile = unit % num_tiles, sp = unit / num_tiles;
       const int buf = local & 1;
       const uint32_t use = static_cast<uint32_t>(local >> 1);
-      const int m0 = (tile % tiles_m) * 2 * BM + static_cast<int>(rank) * BM, n0 = (tile / tiles_m) * BN;
+      int tm, tn;
+      pair_tile(g, tile, tiles_m, tiles_n, tm, tn);
+      const int m0 = tm * 2 * BM + static_cast<int>(rank) * BM, n0 = tn * BN;
       const bool acc_ready = mbar_wait_abortable(acc_full + buf, use & 1u, g.status, abort);
       __syncwarp();
       if (!acc_ready) break;
@@ -783,6 +802,7 @@ void launch_pair(Operand<__half> a, Operand<__half> b, GemmArgs args, int sm_cou
   // feeds the tensor pipe: a stage is refilled only after its MMAs have completed, so (stages - 1) x 32 KB are in flight
   // per SM against an L2 latency of 2 - 3 k cycles under load (measured: the MMA thread waited for operands 35 - 40 % of
   // every tile with five stages).
+  args.group = 2.0 * M * K > PAIR_GROUP_BYTES ? PAIR_GROUP : 0;
   args.stages = 6;
   args.epi_boxes = 1;
   if (const char* e = getenv("MP_GEMM_PAIR_STAGES")) { if (atoi(e) == 5) { args.stages = 5; args.epi_boxes = 2; } }

@@ -16,6 +16,7 @@ struct GemmArgs {
   int M, N, K;
   int a_mn, b_mn;     // operand major-ness: 0 = K contiguous, 1 = M resp. N contiguous
   int stages;
+  int group = 0;      // pair kernel: row blocks per group of tiles (see pair_tile); 0: all of them
   int exact = 0;      // sum as exactly as the FP pipe does (the EXACT forms of the kernels)
   int epi_boxes = 2;  // pair kernel: 64-column staging boxes per epilogue warp
   int split;          // r32 only: 1 = error-compensated hi/lo split (3 MMAs per k-slice), 0 = one tf32 MMA (for timing)
