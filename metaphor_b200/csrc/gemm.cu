@@ -399,6 +399,14 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
             else tma_store_2d(&tmap_c, stage, col0, m0 + quarter * 32);
             bulk_commit();
           }
+        } else if (by_rows && g.beta == 0.0f && (bias == nullptr || g.bias_pitch == 0)) {   // (nothing is aligned: all blocks come here)
+          uint32_t* words = reinterpret_cast<uint32_t*>(stage_base);
+          stage_half_words(words, r, lane, blk & 1);
+          if ((blk & 1) != 0 || blk + 1 == BLOCKS || col0 + 32 >= g.N) {
+            const int row0 = m0 + quarter * 32, colb = col0 - 32 * (blk & 1);
+            store_half_rows(words, lane, crow - static_cast<size_t>(lane) * g.ldc + colb, g.ldc, min(32, g.M - row0),
+                            min(32 * (blk & 1) + 32, g.N - colb));
+          }
         } else if (by_rows) {
           const int row0 = m0 + quarter * 32;
           store_block_rows<T>(reinterpret_cast<float*>(stage_base), r, lane, crow - static_cast<size_t>(lane) * g.ldc + col0, g.ldc,
@@ -669,6 +677,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 #pragma unroll
             for (int p = 0; p < 4; ++p)
               *reinterpret_cast<Pack<T>*>(box + lane * 128 + (((4 * hb + p) ^ (lane & 7)) << 4)) = pack<T>(r + p * PN);
+          } else if (by_rows && g.beta == 0.0f && (bias == nullptr || g.bias_pitch == 0)) {   // (nothing is aligned: all blocks come here)
+            uint32_t* words = reinterpret_cast<uint32_t*>(stage_base);
+            stage_half_words(words, r, lane, hb);
+            if (hb == 1 || colb + 32 >= g.N) {
+              const int row0 = m0 + quarter * 32;
+              store_half_rows(words, lane, crow - static_cast<size_t>(lane) * g.ldc + col0, g.ldc, min(32, g.M - row0), min(32 * hb + 32, g.N - col0));
+            }
           } else if (by_rows) {
             const int row0 = m0 + quarter * 32;
             store_block_rows<T>(reinterpret_cast<float*>(stage_base), r, lane, crow - static_cast<size_t>(lane) * g.ldc + colb, g.ldc,

@@ -38,20 +38,72 @@ constexpr int SWIZZLE_BYTES = 128;    // one operand row / k-row in shared memor
 // One 32 x 32 block of a tile (lane = row, r = its 32 columns) into a C that TMA and 16-byte stores cannot write: odd row
 // pitch or base, or the last columns under beta.  A lane's own row is 32 separate sectors per store instruction, so the block is
 // turned around through 4 KB of the warp's staging (column XOR row: no bank conflicts either way) and leaves one row per
-// instruction; the matrix term and the old C come in the same way.
+// instruction; the matrix term and the old C come in the same way.  Eight rows are read before the first of them is written: a row read
+// behind the write of the one before it took 200 cycles (r32 [2000, 999] x [999, 1501]: 20 of the 36 us of its kernel).
 template <typename T>
 __device__ __forceinline__ void store_block_rows(float* stage, const float* r, int lane, T* c, size_t ldc, int rows, bool col_in, const T* mat,
                                                  size_t mat_ld, float beta) {
 #pragma unroll
   for (int j = 0; j < 32; ++j) stage[lane * 32 + (j ^ lane)] = r[j];
   __syncwarp();
-#pragma unroll 4
-  for (int i = 0; i < rows; ++i) {
-    float v = stage[i * 32 + (lane ^ i)];
-    if (col_in) {
-      if (mat != nullptr) v += mp_up(mat[i * mat_ld + lane]);
-      if (beta != 0.0f) v += beta * mp_up(c[i * ldc + lane]);
-      c[i * ldc + lane] = mp_down<T>(v);
+  T* p = c + lane;
+  const T* q = mat != nullptr ? mat + lane : nullptr;
+#pragma unroll 1
+  for (int i0 = 0; i0 < rows; i0 += 8) {
+    float v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = stage[(i0 + u) * 32 + (lane ^ (i0 + u))];
+    const int n = col_in ? min(8, rows - i0) : 0;
+    if (q != nullptr) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (u < n) v[u] += mp_up(q[u * mat_ld]);
+      q += 8 * mat_ld;
+    }
+    if (beta != 0.0f) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (u < n) v[u] += beta * mp_up(p[u * ldc]);
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (u < n) p[u * ldc] = mp_down<T>(v[u]);
+    p += 8 * ldc;
+  }
+  __syncwarp();
+}
+
+// The same for r16 results that are neither scaled nor added to: up to 64 columns (two blocks, `second` the right one), staged as words of two
+// and written as words.  A row may begin in the middle of one: then its words are put together from neighbours, and its first and last
+// element leave alone.  (Two-byte stores take three times as long as words: [1500, 777] x [777, 1030] 18.0 us with them.)
+__device__ __forceinline__ void stage_half_words(uint32_t* stage, const float* r, int lane, int second) {
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    const __half2 h = __floats2half2_rn(r[2 * k], r[2 * k + 1]);
+    stage[lane * 32 + ((second * 16 + k) ^ lane)] = *reinterpret_cast<const uint32_t*>(&h);
+  }
+}
+__device__ __forceinline__ void store_half_rows(const uint32_t* stage, int lane, __half* c, size_t ldc, int rows, int cols) {
+  __syncwarp();
+  unsigned short* p = reinterpret_cast<unsigned short*>(c);
+  const int e = 2 * lane;   // this lane's elements: e, e + 1
+#pragma unroll 1
+  for (int i0 = 0; i0 < rows; i0 += 8) {
+    uint32_t v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = stage[(i0 + u) * 32 + (lane ^ (i0 + u))];
+#pragma unroll
+    for (int u = 0; u < 8; ++u, p += ldc) {
+      if (i0 + u >= rows) break;   // (uniform, as is the branch below)
+      if ((reinterpret_cast<uintptr_t>(p) & 2u) == 0) {
+        if (e + 1 < cols) *reinterpret_cast<uint32_t*>(p + e) = v[u];
+        else if (e < cols) p[e] = static_cast<unsigned short>(v[u]);
+      } else {
+        const uint32_t next = __shfl_down_sync(0xffffffffu, v[u], 1);
+        if (e + 2 < cols) *reinterpret_cast<uint32_t*>(p + e + 1) = __byte_perm(v[u], next, 0x5432);
+        else if (e + 1 < cols) p[e + 1] = static_cast<unsigned short>(v[u] >> 16);
+        if (lane == 0) p[0] = static_cast<unsigned short>(v[u]);
+      }
     }
   }
   __syncwarp();

@@ -288,3 +288,20 @@ def test_unaligned_r16_keeps_fp32_sums(mp, stream, shape):
     ref = (a.double() @ b.double()) * 2.0 ** -6
     assert float((c != ref.half()).double().mean()) <= 2e-3
     assert stream.status() == 0
+
+
+# r16 results in a C with rows off the 16-byte boundary: written as words of two elements, whole rows and their odd ends.
+@pytest.mark.parametrize("shape", [(33, 64, 1), (130, 64, 31), (129, 72, 33), (128, 64, 63), (300, 200, 65), (257, 64, 129), (40, 64, 258), (600, 128, 777)])
+@pytest.mark.parametrize("off", [0, 1])
+def test_r16_results_off_the_boundary(mp, stream, shape, off):
+    import torch
+    m, n, k = shape
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    a, b = torch.randn(m, n, generator=g, device="cuda").half(), torch.randn(n, k, generator=g, device="cuda").half()
+    flat = torch.full((m * k + 16,), 7.0, device="cuda", dtype=torch.float16)
+    c = flat[off:off + m * k].view(m, k)
+    run(mp, stream, "inner_product_ij_jk_ik", "r16", a, b, 1.0, c, 0.0, m, n, k)
+    ref = a.double() @ b.double()
+    assert float((c.double() - ref).norm() / ref.norm()) <= 2.9e-4      # the rounding of an r16 result
+    assert bool((flat[:off] == 7).all()) and bool((flat[off + m * k:] == 7).all())
+    assert stream.status() == 0
