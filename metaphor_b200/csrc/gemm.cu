@@ -937,6 +937,9 @@ inline void gemm_run(Operand<float> a, Operand<float> b, const GemmArgs& args, i
   gemm_run_r32(a, b, args, sms, ws, ws_bytes, st);
 }
 
+// Below this many products two launches and the pass over the operands cost more than the tf32 kernel takes ([1024, 1024, 1024]: level).
+constexpr double TERMS_MIN_VOLUME = 4e8;
+
 // The FP-pipe kernel: r64, and what does not pay on the tensor cores.
 template <typename T>
 void gemm_simt(const T* a, const T* b, const T* bias, double alpha, T* c, double beta, len_t M, len_t N, len_t K, int a_mn, int b_mn, len_t batch,
@@ -1066,6 +1069,20 @@ void gemm_dispatch(const void* a_, const void* b_, const void* bias, double alph
       args.split = (std::is_same<T, float>::value && !env_flag("MP_GEMM_TF32X1")) ? 1 : 0;
       args.status = state->status_dev;
       args.batch = static_cast<int>(batch);
+      if constexpr (sizeof(T) == 4) {
+        const char* forced = getenv("MP_GEMM_R32_TERMS");   // a test switch: 0 never, 1 wherever the terms fit
+        if (batch == 1 && args.split != 0 && (forced != nullptr || static_cast<double>(M) * N * K > TERMS_MIN_VOLUME)) {
+          int bn, ks;
+          double cycles = gemm_r32_estimate(args, state->sm_count, state->workspace_bytes, &bn, &ks);
+          if (pad_a || pad_b) cycles += 5000.0 + 8.0 * K * (pad_a ? M : 0) / 2500.0 + 8.0 * K * (pad_b ? N : 0) / 2500.0;   // the copies
+          if (forced != nullptr) cycles = forced[0] == '0' ? 0.0 : 1e300;
+          args.exact = pad_a || pad_b;
+          if (gemm_run_r32_terms(Operand<T>{a, a_mn ? M : K}, Operand<T>{b, b_mn ? N : K}, args, state->sm_count, state->workspace,
+                                 state->workspace_bytes, cycles, st))
+            return;
+          args.exact = 0;
+        }
+      }
       if (!pad_a && !pad_b) {
         gemm_run(Operand<T>{a, a_mn ? M : K}, Operand<T>{b, b_mn ? N : K}, args, state->sm_count, state->workspace, state->workspace_bytes, st);
         return;

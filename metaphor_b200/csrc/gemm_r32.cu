@@ -433,15 +433,11 @@ void launch_r32(Operand<float> a, Operand<float> b, const GemmArgs& g, int sms, 
 // The tile (128 x 128 or 128 x 64) and the number of K splits with the smallest estimate of
 //     waves over the SMs x (k-blocks per unit x cycles per k-block + cycles to fill and to drain a unit)  [+ the fold]
 // with the cycles per k-block measured at 4096^3 (1330 and 890).
-void gemm_run_r32(Operand<float> a, Operand<float> b, GemmArgs args, int sms, void* workspace, size_t workspace_bytes, cudaStream_t st) {
-  args.partial_ld = (args.N + 3) & ~3;
-  args.partial = static_cast<float*>(workspace);
+double gemm_r32_estimate(const GemmArgs& args, int sms, size_t workspace_bytes, int* bn, int* ksplit) {
   const long num_kb = (args.K + R_BK - 1) / R_BK;
-  const double mn_bytes = static_cast<double>(args.M) * args.partial_ld * 4.0;
+  const double mn_bytes = static_cast<double>(args.M) * ((args.N + 3) & ~3) * 4.0;
   const bool may_split = args.batch == 1 && !env_flag("MP_GEMM_NO_SPLITK");
   double best = 1e300;
-  int bn = 128;
-  args.ksplit = 1;
   for (int width = 128; width >= 64; width /= 2) {
     const double cycles = width == 128 ? 1330.0 : 890.0;
     const long n_tiles = static_cast<long>((args.M + BM - 1) / BM) * ((args.N + width - 1) / width) * args.batch;
@@ -450,9 +446,17 @@ void gemm_run_r32(Operand<float> a, Operand<float> b, GemmArgs args, int sms, vo
       if (ks > 1 && (per < 2 || (ks - 1) * per >= num_kb || ks * mn_bytes > static_cast<double>(workspace_bytes))) continue;
       double cost = static_cast<double>((n_tiles * ks + sms - 1) / sms) * (per * cycles + 3000.0);
       if (ks > 1) cost += 5000.0 + 2.0 * ks * mn_bytes / 3500.0;   // the fold's launch; partials out and in at 3.5 KB a cycle
-      if (cost < best) { best = cost; bn = width; args.ksplit = ks; }
+      if (cost < best) { best = cost; *bn = width; *ksplit = ks; }
     }
   }
+  return best;
+}
+
+void gemm_run_r32(Operand<float> a, Operand<float> b, GemmArgs args, int sms, void* workspace, size_t workspace_bytes, cudaStream_t st) {
+  args.partial_ld = (args.N + 3) & ~3;
+  args.partial = static_cast<float*>(workspace);
+  int bn = 128;
+  gemm_r32_estimate(args, sms, workspace_bytes, &bn, &args.ksplit);
   const bool exact = args.exact != 0 && args.split != 0;
   if (bn == 128) {
     if (exact) launch_r32<128, true>(a, b, args, sms, st); else launch_r32<128, false>(a, b, args, sms, st);

@@ -290,6 +290,38 @@ def test_unaligned_r16_keeps_fp32_sums(mp, stream, shape):
     assert stream.status() == 0
 
 
+# r32 contractions from two r16 terms per value, at the edges of tiles (256 rows, 128 or 256 columns), k-blocks (64) and 16-byte pitches, and with a
+# split of K.  Rows and columns are of sizes between 2^-40 and 2^40: the terms are scaled by rows and columns, so every result is as exact as its own
+# products: each is off by three roundings of 2^-23 at most, the sum by the truncated additions of 12 MMAs and a rounding per k-block.
+@pytest.mark.parametrize("shape", [(1, 64, 1), (255, 63, 129), (256, 64, 256), (257, 65, 257), (300, 129, 520), (513, 777, 127), (66, 4097, 300)])
+@pytest.mark.parametrize("variant", ["ij_jk_ik", "ij_kj_ik", "ji_jk_ik"])
+def test_r32_from_two_terms(mp, stream, monkeypatch, shape, variant):
+    import torch
+    monkeypatch.setenv("MP_GEMM_R32_TERMS", "1")      # read at every launch
+    m, n, k = shape
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    power = lambda c: torch.exp2(torch.randint(-40, 41, (c,), generator=g, device="cuda").float())
+    a = torch.randn(m, n, generator=g, device="cuda") * power(m)[:, None]
+    b = torch.randn(n, k, generator=g, device="cuda") * power(k)[None, :]
+    da = (a.t() if variant[0] == "j" else a).contiguous()
+    db = (b.t() if variant[3:5] == "kj" else b).contiguous()
+    ref, size = a.double() @ b.double(), a.double().abs() @ b.double().abs()
+    bound = (3 * 2.0 ** -23 + 13 * 2.0 ** -23) * size
+    c = torch.full((m + 1, k), 7.0, device="cuda")
+    run(mp, stream, "inner_product_" + variant, "r32", da, db, 1.0, c, 0.0, m, n, k)
+    assert bool(((c[:m].double() - ref).abs() <= bound).all())
+    assert bool((c[m] == 7).all())
+    old = torch.randn(m, k, generator=g, device="cuda") * power(k)[None, :]
+    c = old.clone()
+    run(mp, stream, "inner_product_" + variant, "r32", da, db, 0.5, c, 2.0, m, n, k)
+    assert bool(((c.double() - 0.5 * ref - 2 * old.double()).abs() <= bound + 2.0 ** -22 * old.double().abs()).all())
+    if variant == "ij_jk_ik":
+        bias = torch.randn(k, generator=g, device="cuda")
+        run(mp, stream, "linear_ij_jk_ik", "r32", da, db, bias, 1.0, c, 0.0, m, n, k)
+        assert bool(((c.double() - ref - bias.double()).abs() <= bound + 2.0 ** -22 * bias.double().abs()).all())
+    assert stream.status() == 0
+
+
 # r16 results in a C with rows off the 16-byte boundary: written as words of two elements, whole rows and their odd ends.
 @pytest.mark.parametrize("shape", [(33, 64, 1), (130, 64, 31), (129, 72, 33), (128, 64, 63), (300, 200, 65), (257, 64, 129), (40, 64, 258), (600, 128, 777)])
 @pytest.mark.parametrize("off", [0, 1])
