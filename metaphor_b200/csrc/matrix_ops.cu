@@ -220,7 +220,14 @@ __global__ void __launch_bounds__(256) col_sum_kernel(const T* __restrict__ src,
         for (int e = 0; e < W; ++e) acc[e] += mp_up(q.v[e]);
       }
     } else {
-      for (size_t r = rbeg + warp; r < rend; r += 8) acc[0] += mp_up(src[r * n + c]);
+      // (rows that do not come in whole packs: eight loads in flight too, added in the order of the rows)
+      for (size_t r = rbeg + warp; r < rend; r += 64) {
+        T q[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) q[u] = r + 8 * u < rend ? src[(r + 8 * u) * n + c] : mp_down<T>(A(0));
+#pragma unroll
+        for (int u = 0; u < 8; ++u) acc[0] += mp_up(q[u]);
+      }
     }
   }
 #pragma unroll
@@ -246,7 +253,13 @@ __global__ void __launch_bounds__(256) col_sum_fold_kernel(const typename Acc<T>
   const size_t col = static_cast<size_t>(blockIdx.x) * 256 + threadIdx.x;
   if (col >= n) return;
   A s = A(0);
-  for (int p = 0; p < splits; ++p) s += partial[static_cast<size_t>(p) * n + col];
+  for (int p = 0; p < splits; p += 8) {
+    A v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = p + u < splits ? partial[static_cast<size_t>(p + u) * n + col] : A(0);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) s += v[u];
+  }
   dst[col] = mp_down<T>(blend ? s + alpha * mp_up(dst[col]) : s);
 }
 
