@@ -876,6 +876,17 @@ void pick_split_k(GemmArgs& args, int sms, size_t workspace_bytes, int* bn_io) {
   if (best_ks > 1 && best < 0.85 * base) { args.ksplit = best_ks; *bn_io = best_bn; }
 }
 
+// Fewer 256 x 256 tiles than pairs: still faster where the single CTAs' tiles take more rounds.  Estimate of both in cycles: rounds x (k-blocks x
+// cycles per k-block under load + cycles to fill and to drain a tile).  us, single CTAs / pairs: [4096, 3352] x [3352, 768] 45.3 / 27.4, with a
+// residual [4096, 1536] x [1536, 768] 31.2 / 16.4, 2048^3 25.6 / 17.2, [2048, 512] x [512, 2048] 9.6 / 8.9; where a tile has few k-blocks the pairs'
+// hand-shakes cost more than a round ([8192, 256] x [256, 512] 7.1 / 7.6).
+bool pair_saves_rounds(const GemmArgs& args, int bn, long pair_tiles, int sms) {
+  const long num_kb = (args.K + GemmT::BK - 1) / GemmT::BK, tiles = static_cast<long>((args.M + BM - 1) / BM) * ((args.N + bn - 1) / bn);
+  const double one = static_cast<double>((tiles + sms - 1) / sms) * (num_kb * (bn == 256 ? 950.0 : bn == 128 ? 590.0 : 430.0) + 1500.0);
+  const double pair = static_cast<double>((pair_tiles + sms / 2 - 1) / (sms / 2)) * (num_kb * 800.0 + 4500.0);
+  return pair < 0.9 * one;
+}
+
 // One r16 contraction whose operands TMA can address.  `args` carries the problem; the tile width, the K split and the ring depth
 // are chosen here.  workspace: room for split-K partials.
 void gemm_run_r16(Operand<__half> a, Operand<__half> b, GemmArgs args, int sms, void* workspace, size_t workspace_bytes, cudaStream_t st) {
@@ -895,7 +906,7 @@ void gemm_run_r16(Operand<__half> a, Operand<__half> b, GemmArgs args, int sms, 
   // CTA pairs for wide problems with enough 256 x 256 tiles to fill the pairs (their accumulators are handed over once per tile: not EXACT)
   const long pair_tiles = static_cast<long>((args.M + 255) / 256) * ((args.N + 255) / 256);
   if (args.batch == 1 && !args.exact && !env_flag("MP_GEMM_NO_PAIRS") && args.M >= 256 && args.N >= 256) {
-    if (args.ksplit == 1 && bn == 256 && pair_tiles >= sms / 2) {
+    if (args.ksplit == 1 && ((bn == 256 && pair_tiles >= sms / 2) || pair_saves_rounds(args, bn, pair_tiles, sms))) {
       launch_pair(a, b, args, sms, st);
       return;
     }

@@ -39,7 +39,7 @@ constexpr int SWIZZLE_BYTES = 128;    // one operand row / k-row in shared memor
 // pitch or base, or the last columns under beta.  A lane's own row is 32 separate sectors per store instruction, so the block is
 // turned around through 4 KB of the warp's staging (column XOR row: no bank conflicts either way) and leaves one row per
 // instruction; the matrix term and the old C come in the same way.  Eight rows are read before the first of them is written: a row read
-// behind the write of the one before it took 200 cycles (r32 [2000, 999] x [999, 1501]: 20 of the 36 us of its kernel).
+// behind the write of the one before it took 200 cycles (r16 [1500, 777] x [777, 1030]: 12 500 of the kernel's 24 600).
 template <typename T>
 __device__ __forceinline__ void store_block_rows(float* stage, const float* r, int lane, T* c, size_t ldc, int rows, bool col_in, const T* mat,
                                                  size_t mat_ld, float beta) {
@@ -75,7 +75,7 @@ __device__ __forceinline__ void store_block_rows(float* stage, const float* r, i
 
 // The same for r16 results that are neither scaled nor added to: up to 64 columns (two blocks, `second` the right one), staged as words of two
 // and written as words.  A row may begin in the middle of one: then its words are put together from neighbours, and its first and last
-// element leave alone.  (Two-byte stores take three times as long as words: [1500, 777] x [777, 1030] 18.0 us with them.)
+// element leave alone.  (Two-byte stores take three times as long as words: [1500, 777] x [777, 1030] with its copies 18.0 us with them, 14.7 now.)
 __device__ __forceinline__ void stage_half_words(uint32_t* stage, const float* r, int lane, int second) {
 #pragma unroll
   for (int k = 0; k < 16; ++k) {

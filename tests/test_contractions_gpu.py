@@ -337,3 +337,36 @@ def test_r16_results_off_the_boundary(mp, stream, shape, off):
     assert float((c.double() - ref).norm() / ref.norm()) <= 2.9e-4      # the rounding of an r16 result
     assert bool((flat[:off] == 7).all()) and bool((flat[off + m * k:] == 7).all())
     assert stream.status() == 0
+
+
+# r16 contractions with fewer 256 x 256 tiles than CTA pairs, which take the pairs where that saves rounds of tiles: ragged last tiles of both
+# directions, one K block more than whole ones, a residual, a bias and the old C; against the single CTAs' kernel to the rounding of a result.
+@pytest.mark.parametrize("shape", [(3000, 1000, 1000), (2570, 1032, 776), (4096, 1096, 520), (2048, 2048, 2048)])
+@pytest.mark.parametrize("variant", ["ij_jk_ik", "ij_kj_ik", "ji_jk_ik"])
+def test_pairs_on_few_tiles(mp, stream, monkeypatch, shape, variant):
+    import torch
+    m, n, k = shape
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    a, b = torch.randn(m, n, generator=g, device="cuda").half(), torch.randn(n, k, generator=g, device="cuda").half()
+    term, bias = torch.randn(m, k, generator=g, device="cuda").half(), torch.randn(k, generator=g, device="cuda").half()
+    da = (a.t() if variant[0] == "j" else a).contiguous()
+    db = (b.t() if variant[3:5] == "kj" else b).contiguous()
+    ref = a.double() @ b.double()
+
+    def results():
+        out = [torch.full((m, k), 3.0, device="cuda", dtype=torch.float16) for _ in range(4)]
+        run(mp, stream, "inner_product_" + variant, "r16", da, db, 1.0, out[0], 0.0, m, n, k)
+        run(mp, stream, "inner_product_" + variant, "r16", da, db, 0.5, out[1], 2.0, m, n, k)
+        if variant == "ij_jk_ik":
+            run(mp, stream, "linear_ij_jk_ik_ik", "r16", da, db, term, 1.0, out[2], 0.0, m, n, k)
+            run(mp, stream, "linear_ij_jk_ik", "r16", da, db, bias, 1.0, out[3], 0.0, m, n, k)
+        return out
+
+    want = [ref, 0.5 * ref + 6.0, ref + term.double(), ref + bias.double()]
+    got = results()
+    monkeypatch.setenv("MP_GEMM_NO_PAIRS", "1")      # read at every launch
+    single = results()
+    for c, s, w in list(zip(got, single, want))[:4 if variant == "ij_jk_ik" else 2]:
+        assert float((c.double() - w).norm() / w.norm()) <= 2.9e-4      # the rounding of an r16 result
+        assert float((s.double() - w).norm() / w.norm()) <= 2.9e-4
+    assert stream.status() == 0
