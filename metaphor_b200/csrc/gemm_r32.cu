@@ -368,9 +368,17 @@ __global__ void __launch_bounds__(R_THREADS, 1) gemm_r32_kernel(const __grid_con
             for (int j = 0; j < 32; ++j) r[j] *= g.alpha;
             if (bias != nullptr && (g.bias_pitch == 0 || (row < g.M && !by_rows))) {
               const float* brow = bias + static_cast<size_t>(row) * g.bias_pitch;
+              if (col0 + 32 <= g.N && g.bias_pitch % 4 == 0 && mp_aligned16(bias)) {
 #pragma unroll
-              for (int j = 0; j < 32; ++j)
-                if (col0 + j < g.N) r[j] += brow[col0 + j];
+                for (int p = 0; p < 8; ++p) {
+                  const float4 add = *reinterpret_cast<const float4*>(brow + col0 + 4 * p);
+                  r[4 * p] += add.x; r[4 * p + 1] += add.y; r[4 * p + 2] += add.z; r[4 * p + 3] += add.w;
+                }
+              } else {
+#pragma unroll
+                for (int j = 0; j < 32; ++j)
+                  if (col0 + j < g.N) r[j] += brow[col0 + j];
+              }
             }
             if (use_tma) {
               if (lane == 0) bulk_wait_read<0>();   // the previous store has read the box
