@@ -322,6 +322,13 @@ def test_r32_from_two_terms(mp, stream, monkeypatch, shape, variant):
     assert stream.status() == 0
 
 
+@pytest.mark.parametrize("shape", [(1, 131, 97, 133), (1, 301, 999, 307), (1, 67, 16385, 67)])
+@pytest.mark.parametrize("variant", ["ij_jk_ik", "ij_kj_ik", "ji_jk_ik"])
+def test_r32_from_two_terms_not_finite(mp, stream, monkeypatch, shape, variant):
+    monkeypatch.setenv("MP_GEMM_R32_TERMS", "1")
+    test_unaligned_r32_not_finite(mp, stream, shape, variant)
+
+
 # r16 results in a C with rows off the 16-byte boundary: written as words of two elements, whole rows and their odd ends.
 @pytest.mark.parametrize("shape", [(33, 64, 1), (130, 64, 31), (129, 72, 33), (128, 64, 63), (300, 200, 65), (257, 64, 129), (40, 64, 258), (600, 128, 777)])
 @pytest.mark.parametrize("off", [0, 1])
