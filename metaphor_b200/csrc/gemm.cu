@@ -960,8 +960,9 @@ inline void gemm_run(Operand<float> a, Operand<float> b, const GemmArgs& args, i
   gemm_run_r32(a, b, args, sms, ws, ws_bytes, st);
 }
 
-// Below this many products two launches and the pass over the operands cost more than the tf32 kernel takes ([1024, 1024, 1024]: level).
-constexpr double TERMS_MIN_VOLUME = 4e8;
+// Up to here two launches and the pass over the operands leave no gain over the tf32 kernel (us, that / from terms: [1024, 1024, 1024] 22 / 25,
+// [777, 777, 777] 19 / 23, with A along M 21 / 23).
+constexpr double TERMS_MIN_VOLUME = 1e9;
 
 // The FP-pipe kernel: r64, and what does not pay on the tensor cores.
 template <typename T>
@@ -1097,7 +1098,8 @@ void gemm_dispatch(const void* a_, const void* b_, const void* bias, double alph
         if (batch == 1 && args.split != 0 && (forced != nullptr || static_cast<double>(M) * N * K > TERMS_MIN_VOLUME)) {
           int bn, ks;
           double cycles = gemm_r32_estimate(args, state->sm_count, state->workspace_bytes, &bn, &ks);
-          if (pad_a || pad_b) cycles += 5000.0 + 8.0 * K * (pad_a ? M : 0) / 2500.0 + 8.0 * K * (pad_b ? N : 0) / 2500.0;   // the copies
+          if (a_mn) cycles *= 1.2;   // (A goes through TMEM: [2048, 2048, 2048] 101 us, and 127 where its rows are contiguous along M)
+          if (pad_a || pad_b) cycles = 1.1 * cycles + 5000.0 + 8.0 * K * (pad_a ? M : 0) / 2500.0 + 8.0 * K * (pad_b ? N : 0) / 2500.0;   // EXACT; the copies
           if (forced != nullptr) cycles = forced[0] == '0' ? 0.0 : 1e300;
           args.exact = pad_a || pad_b;
           if (gemm_run_r32_terms(Operand<T>{a, a_mn ? M : K}, Operand<T>{b, b_mn ? N : K}, args, state->sm_count, state->workspace,

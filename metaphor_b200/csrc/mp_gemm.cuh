@@ -259,7 +259,7 @@ bool env_flag(const char* name) {
 void gemm_run_r32(Operand<float> a, Operand<float> b, GemmArgs args, int sms, void* workspace, size_t workspace_bytes, cudaStream_t st);
 // Its estimate in cycles, with the tile and the K split that give it.
 double gemm_r32_estimate(const GemmArgs& args, int sms, size_t workspace_bytes, int* bn, int* ksplit);
-// gemm_r32_terms.cu: the same from two r16 terms per value, for any operand alignment; false (and nothing done) where it would take longer than
+// gemm_r32_terms.cu: the same from three bf16 terms per value, for any operand alignment; false (and nothing done) where it would take longer than
 // `limit_cycles` or its copies do not fit.
 bool gemm_run_r32_terms(Operand<float> a, Operand<float> b, GemmArgs args, int sms, void* workspace, size_t workspace_bytes, double limit_cycles,
                         cudaStream_t st);

@@ -290,12 +290,12 @@ def test_unaligned_r16_keeps_fp32_sums(mp, stream, shape):
     assert stream.status() == 0
 
 
-# r32 contractions from two r16 terms per value, at the edges of tiles (256 rows, 128 or 256 columns), k-blocks (64) and 16-byte pitches, and with a
-# split of K.  Rows and columns are of sizes between 2^-40 and 2^40: the terms are scaled by rows and columns, so every result is as exact as its own
+# r32 contractions from three bf16 terms per value, at the edges of tiles (256 rows, 128 or 256 columns), k-blocks (64) and 16-byte pitches, and with a
+# split of K.  Rows and columns are of sizes between 2^-40 and 2^40: values have exponents of their own, so every result is as exact as its own
 # products: each is off by three roundings of 2^-23 at most, the sum by the truncated additions of 12 MMAs and a rounding per k-block.
 @pytest.mark.parametrize("shape", [(1, 64, 1), (255, 63, 129), (256, 64, 256), (257, 65, 257), (300, 129, 520), (513, 777, 127), (66, 4097, 300)])
 @pytest.mark.parametrize("variant", ["ij_jk_ik", "ij_kj_ik", "ji_jk_ik"])
-def test_r32_from_two_terms(mp, stream, monkeypatch, shape, variant):
+def test_r32_from_terms(mp, stream, monkeypatch, shape, variant):
     import torch
     monkeypatch.setenv("MP_GEMM_R32_TERMS", "1")      # read at every launch
     m, n, k = shape
@@ -324,9 +324,64 @@ def test_r32_from_two_terms(mp, stream, monkeypatch, shape, variant):
 
 @pytest.mark.parametrize("shape", [(1, 131, 97, 133), (1, 301, 999, 307), (1, 67, 16385, 67)])
 @pytest.mark.parametrize("variant", ["ij_jk_ik", "ij_kj_ik", "ji_jk_ik"])
-def test_r32_from_two_terms_not_finite(mp, stream, monkeypatch, shape, variant):
+def test_r32_from_terms_not_finite(mp, stream, monkeypatch, shape, variant):
     monkeypatch.setenv("MP_GEMM_R32_TERMS", "1")
     test_unaligned_r32_not_finite(mp, stream, shape, variant)
+
+
+# Values of one row that lie far apart along K, the large ones against zeros of the other operand: the small ones alone make the result and keep
+# their bits (the bound is that of test_r32_from_terms).  One large value in each 64 of K, at another place in each; in A, then in B.
+@pytest.mark.parametrize("shape", [(300, 129, 520), (256, 128, 256)])
+@pytest.mark.parametrize("spread", [0, 10, 17, 24, 31, 45, 90])
+@pytest.mark.parametrize("variant", ["ij_jk_ik", "ij_kj_ik", "ji_jk_ik"])
+def test_r32_terms_of_values_far_apart(mp, stream, monkeypatch, shape, spread, variant):
+    import torch
+    monkeypatch.setenv("MP_GEMM_R32_TERMS", "1")      # read at every launch
+    m, n, k = shape
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    small, other = 0.1 + 0.9 * torch.rand(max(m, k), n, generator=g, device="cuda"), torch.randn(max(m, k), n, generator=g, device="cuda")
+    at = torch.tensor([(i * 64 + (i * 23 + 5) % 64) % n for i in range((n + 63) // 64)], device="cuda")
+    small[:, at], other[:, at] = 2.0 ** spread, 0.0
+    for a, b in ((small[:m], other[:k].t()), (other[:m], small[:k].t())):
+        da = (a.t() if variant[0] == "j" else a).contiguous()
+        db = (b.t() if variant[3:5] == "kj" else b).contiguous()
+        ref, size = a.double() @ b.double(), a.double().abs() @ b.double().abs()
+        c = torch.full((m, k), 7.0, device="cuda")
+        run(mp, stream, "inner_product_" + variant, "r32", da, db, 1.0, c, 0.0, m, n, k)
+        assert bool(((c.double() - ref).abs() <= 16 * 2.0 ** -23 * size).all())
+    assert stream.status() == 0
+
+
+# The default rule: from 1e9 products on where the copies fit the workspace.  Which kernel ran shows in the bits, for the two differ in theirs.
+@pytest.mark.parametrize("shape,terms", [((2048, 2048, 2048), True), ((2000, 999, 1501), True), ((1000, 1000, 999), False), ((4096, 1400, 4096), False)])
+@pytest.mark.parametrize("variant", ["ij_jk_ik", "ij_kj_ik", "ji_jk_ik"])
+def test_r32_terms_by_default(mp, stream, monkeypatch, shape, terms, variant):
+    import torch
+    m, n, k = shape
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    a, b = torch.randn(m, n, generator=g, device="cuda"), torch.randn(n, k, generator=g, device="cuda")
+    a[:, 7::64], b[7::64] = 2.0 ** 40, 0.0
+    da = (a.t() if variant[0] == "j" else a).contiguous()
+    db = (b.t() if variant[3:5] == "kj" else b).contiguous()
+
+    def result(x, y):
+        c = torch.full((m, k), 7.0, device="cuda")
+        run(mp, stream, "inner_product_" + variant, "r32", x, y, 1.0, c, 0.0, m, n, k)
+        return c
+
+    c = result(da, db)
+    bound = lambda x, y: 16 * 2.0 ** -23 * (x.double().abs() @ y.double().abs())
+    assert bool(((c.double() - a.double() @ b.double()).abs() <= bound(a, b)).all()) or not terms
+    # results near the smallest normal number, from products of the same size; and 1e24 where only a zero meets it
+    tiny = result(torch.full_like(da, 2.0 ** -62), torch.full_like(db, 2.0 ** -61))
+    assert bool(((tiny.double() - n * 2.0 ** -123).abs() <= 16 * 2.0 ** -23 * n * 2.0 ** -123).all())
+    a, b = torch.zeros(m, n, device="cuda"), torch.zeros(n, k, device="cuda")
+    a[:, 0], b[1], a[:, 2], b[2] = 1e24, 1e24, 3.0, 5.0
+    huge = result((a.t() if variant[0] == "j" else a).contiguous(), (b.t() if variant[3:5] == "kj" else b).contiguous())
+    assert bool((huge == 15.0).all())
+    monkeypatch.setenv("MP_GEMM_R32_TERMS", "0")      # read at every launch
+    assert torch.equal(c, result(da, db)) == (not terms)
+    assert stream.status() == 0
 
 
 # r16 results in a C with rows off the 16-byte boundary: written as words of two elements, whole rows and their odd ends.
