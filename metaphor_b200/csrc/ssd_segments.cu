@@ -1,9 +1,10 @@
 // Mamba-2 SSD scan of r16 tensors to the accuracy of fp32 arithmetic, over segments of 64 steps that run side by side (head size 64,
 // state 128, any number of steps).  It serves the calls that whole tensor-core chunks do not cover: lengths that are no multiple of
 // the chunk, and other chunk lengths; pointers need no more than the alignment of their elements.  Its results are those of the
-// recurrence (ssd_generic.cu) to the accuracy of fp32 sums: weights, scores and states keep their 24 bits, and A's gradient is a sum of the
-// products that make it up, not a difference of row dots, so that it keeps its digits where almost nothing is carried from step to
-// step ([2, 200, 16] with step sizes around 2: the r16 chunk walk is off by 0.6 of gA and 0.03 of gdt, this by 1.4e-7 and 1.3e-7).
+// recurrence (ssd_generic.cu) to the accuracy of fp32 sums: weights, scores and states are fp32 values (in a product two terms, 23 bits, with
+// their own exponents), and A's gradient is a sum of the products that make it up, not a difference of row dots, so that it keeps its digits
+// where almost nothing is carried from step to step ([2, 200, 16] with step sizes around 2: the r16 chunk walk is off by 0.6 of gA and 0.03 of
+// gdt, this by 2.3e-7 and 1.2e-7).
 //
 // With cum the inclusive prefix sums of dt A inside a segment (differences of them taken in r64), E their last value, H the state a
 // segment receives from its predecessors and Y the adjoint state it receives from its successors:
@@ -17,21 +18,21 @@
 // Launches: states made inside every segment, both directions (segment_states); carried from segment to segment, block by block
 // (segment_carry); outputs (segment_forward / segment_reverse); for the reverse two folds.
 //
-// Every product has one operand that is r16 in memory (x, B, C, gy).  The other, in fp32 (weights times scores, scaled values, states), is
-// split into two r16 terms under a power of two that brings the largest value of its row (states: of its 16 x 16 block) below 2^15: 23 bits,
-// and 40 binary orders below the largest value.  A product is then two tensor-core MMAs with the r16 operand unsplit, and the scores
-// are one.  mma.sync and not tcgen05, because the sums stay in registers: a warp turns its scores into the next product's operand without
-// a trip through TMEM or shared memory, and sums that reach gdt and gA are taken out of the accumulator, which truncates, after every
-// 16 products and added up rounded.
+// Every product has one operand that is r16 in memory (x, B, C, gy), which tf32 holds whole: 11 bits and a wider exponent.  The other, in fp32
+// (weights times scores, scaled values, states), is split where it is read into two tf32 terms, 11 bits rounded and the rest, with nothing shared
+// between values.  A product is then two tensor-core MMAs; the scores, r16 by r16, are one r16 MMA.  mma.sync and not tcgen05, because the sums
+// stay in registers and are taken out of the accumulator, which truncates, after every 16 products and added up rounded.
 // A CTA with an infinity or a NaN among its results does its share again on the FP pipe (*_plain below): where an r16 tile holds one, the
 // lower term of a value that needs none would meet it with a zero, and so would a step that the mask leaves out.
 //
 // Forward / reverse in us, recurrence -> fp32 on the FP pipe (24 TFLOP/s of its 72) -> here:
-//   [2, 1000, 24] 1 806 / 41 544 -> 96 / 261 -> 44 / 93,   [8, 8191, 32] 41 650 / 800 600 -> 3 947 / 8 996 -> 1 255 / 3 242,
-//   [1, 8191, 2] 57 / 107 -> 52 / 84 (FP pipe -> here),    [1, 100, 2] 182 / 3 957 -> 21 / 38 -> 12 / 20.
-// The 2-norm of the errors against r64: y, gx, gB, gC are r16 roundings on all three; gdt 1.2e-7 - 1.6e-7 here, 1.3e-7 - 2.4e-7 on the FP pipe
-// (mma.sync: 555 TFLOP/s in r16, so that two terms leave 280).  What bounds the reverse is the latency of its sixteen warps: tensor pipe a
-// quarter busy; the states and the carry move 128 KB of global memory a head and segment.
+//   [2, 1000, 24] 1 806 / 41 544 -> 96 / 260 -> 50 / 128,   [8, 8191, 32] 41 650 / 800 600 -> 3 950 / 8 972 -> 1 853 / 4 901,
+//   [1, 8191, 2] 57 / 107 -> 40 / 89 (FP pipe -> here),     [1, 100, 2] 182 / 3 957 -> 21 / 38 -> 15 / 26.
+// The 2-norm of the errors against r64: y, gx, gB, gC are r16 roundings on all three; gdt 1.2e-7 - 1.8e-7 here, 1.3e-7 - 2.5e-7 on the FP pipe.
+// Two r16 terms under a power of two per row or 16 x 16 block are half the MMAs and nothing to widen or split when read (44 / 93 us for the first
+// shape), but values 2^33 below the largest of a block then made results wrong by up to a fifth of themselves where the large one met a zero.
+// What bounds the reverse: its sixteen warps issue in 56 % of the cycles, tensor pipe 37 %, ALU (addresses, splits) 44 %; the states and the carry
+// move 128 KB of global memory a head and segment.
 // Below 32 steps the recurrence stays (60 / 1 214 us at [2, 31, 24]): its forward needs no scratch, and callers may rely on that.
 #include "mp_async.cuh"
 
@@ -39,16 +40,14 @@ namespace {
 
 constexpr int SG_Q = 64;              // steps per segment
 constexpr int SG_N = 128, SG_P = 64;  // state size, head size
-constexpr int SG_STATE_BYTES = SG_N * SG_P * 4;   // a state as r16 pairs
-constexpr int SG_BLOCKS = SG_N / 16 * (SG_P / 16);   // 16 x 16 blocks of a state, each with a scale
+constexpr int SG_STATE_BYTES = SG_N * SG_P * 4;
 
 struct SegArgs {
   const __half* x; const float* dt; const float* A; const __half* Bm; const __half* Cm; const __half* gy;
   __half* y;                 // forward
   __half* gx; float* gdt;    // reverse
-  unsigned char* states;     // [B H][nseg] states received (see state_load); the adjoint ones follow in the reverse
+  float* states;             // [B H][nseg][64 p][128 n] states received; the adjoint ones follow in the reverse
   float* decay;              // [B H][nseg]: exp(E)
-  float* scales;             // [B H][nseg][4 of p][8 of n]: what a block's pairs are multiplied by; adjoint ones likewise
   float* ga_part;            // [B H][nseg]
   float* gb_part;            // [splits][B L G][128] sums over the heads of a split, gB then gC
   int B, L, H, G, nseg, splits;
@@ -96,11 +95,6 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 __device__ __forceinline__ void st_shared16(uint32_t dst, uint4 v) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
-__device__ __forceinline__ uint4 ld_shared16(uint32_t src) {
-  uint4 v;
-  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(src) : "memory");
-  return v;
-}
 
 // 64 steps of CHUNKS 16-byte chunks; steps past the sequence become zeros.
 template <int CHUNKS, int THREADS>
@@ -129,16 +123,34 @@ __device__ __forceinline__ uint32_t r16_finite(uint32_t v) {   // infinities and
   return v;
 }
 
-// A state in global memory: blocks of 16 x 16 (p, n), a block's sixteen rows p after another, a row as four chunks: the upper terms of its
-// values, then the lower ones.  In shared memory rows p of 512 bytes, the blocks' chunks after another; the scales lie behind.
+// fp32 tiles in shared memory: rows of PITCH bytes, their 16-byte chunks exchanged by the row, so that two chunks of four neighbouring rows, of
+// four even and of four odd ones lie in different banks.
+template <int PITCH>
+__device__ __forceinline__ uint32_t wide_at(uint32_t base, int r, int c) { return base + r * PITCH + ((c ^ (((r ^ (r >> 2)) & 3) << 1)) << 4); }
+__device__ __forceinline__ float2 ld_shared8(uint32_t src) {
+  float2 v;
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(src) : "memory");
+  return v;
+}
+__device__ __forceinline__ float ld_shared4(uint32_t src) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(src) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 ld_shared16f(uint32_t src) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(src) : "memory");
+  return v;
+}
+
+// A state: rows p of 512 bytes.
 template <int THREADS>
-__device__ __forceinline__ void state_load(uint32_t dst, const unsigned char* src, const float* scales) {
+__device__ __forceinline__ void state_load(uint32_t dst, const float* src) {
 #pragma unroll
   for (int k = 0; k < SG_STATE_BYTES / 16 / THREADS; ++k) {
     const int idx = k * THREADS + threadIdx.x;
-    cp_async16(tile_at<512>(dst, (idx >> 9) * 16 + ((idx >> 2) & 15), ((idx >> 6) & 7) * 4 + (idx & 3)), src + idx * 16);
+    cp_async16(wide_at<512>(dst, idx >> 5, idx & 31), src + idx * 4);
   }
-  if (threadIdx.x < SG_BLOCKS / 4) cp_async16(dst + SG_STATE_BYTES + threadIdx.x * 16, scales + threadIdx.x * 4);
 }
 
 // ---------------------------------------------------------------------------
@@ -150,13 +162,39 @@ __device__ __forceinline__ void ldsm(uint32_t (&r)[4], uint32_t at) {
 __device__ __forceinline__ void ldsm_t(uint32_t (&r)[4], uint32_t at) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at) : "memory");
 }
-__device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 __device__ __forceinline__ void mma0(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {   // nothing accumulated before
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
                : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+// The same in tf32 over eight columns: a lane holds columns q and q + 4, which are used for columns 2 q and 2 q + 1 of an r16 operand.
+__device__ __forceinline__ void mma8(float (&d)[4], float a0, float a1, float a2, float a3, float b0, float b1) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(__float_as_uint(a0)), "r"(__float_as_uint(a1)), "r"(__float_as_uint(a2)), "r"(__float_as_uint(a3)), "r"(__float_as_uint(b0)),
+                 "r"(__float_as_uint(b1)));
+}
+__device__ __forceinline__ void mma80(float (&d)[4], float a0, float a1, float a2, float a3, float b0, float b1) {   // nothing accumulated before
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+               : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+               : "r"(__float_as_uint(a0)), "r"(__float_as_uint(a1)), "r"(__float_as_uint(a2)), "r"(__float_as_uint(a3)), "r"(__float_as_uint(b0)),
+                 "r"(__float_as_uint(b1)), "f"(0.f));
+}
+// d += a b over 16 columns (mma160: d = a b), operands as values in the order of an r16 operand's registers.
+__device__ __forceinline__ void mma160(float (&d)[4], const float (&a)[8], const float* b) {
+  mma80(d, a[0], a[2], a[1], a[3], b[0], b[1]);
+  mma8(d, a[4], a[6], a[5], a[7], b[2], b[3]);
+}
+__device__ __forceinline__ void mma16(float (&d)[4], const float (&a)[8], const float* b) {
+  mma8(d, a[0], a[2], a[1], a[3], b[0], b[1]);
+  mma8(d, a[4], a[6], a[5], a[7], b[2], b[3]);
+}
+__device__ __forceinline__ void widen(float* v, const uint32_t* r, int n) {   // n is a constant
+#pragma unroll
+  for (int e = 0; e < n; ++e) {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(r + e));
+    v[2 * e] = f.x;
+    v[2 * e + 1] = f.y;
+  }
 }
 // Operand of 16 rows from r0 on, 16 columns from chunk c0 on (two chunks), of a tile [rows][columns]; _t: of a tile [columns][rows], rows
 // of chunks r0, r0 + 1, columns from c0 on.
@@ -175,31 +213,23 @@ __device__ __forceinline__ void load_b(uint32_t (&b)[4], uint32_t tile, int n0, 
 template <int PITCH>
 __device__ __forceinline__ void load_b_t(uint32_t (&b)[4], uint32_t tile, int k0, int c0, int lane) { ldsm_t(b, tile_at<PITCH>(tile, k0 + (lane & 15), c0 + (lane >> 4))); }
 
-// The power of two that brings a value with these bits (a magnitude, finite) below 2^15, and its reciprocal.
-__device__ __forceinline__ float split_scale(uint32_t bits, float* inverse) {
-  int e = 268 - static_cast<int>(bits >> 23);
-  e = e < 253 ? e : 253;
-  *inverse = __uint_as_float(static_cast<uint32_t>(254 - e) << 23);
-  return __uint_as_float(static_cast<uint32_t>(e) << 23);
+// A value as two terms that tf32 holds: 11 bits rounded, and the rest, of which the MMA reads 11 bits.  What is not finite, or rounds up to that,
+// makes a NaN of the result.
+__device__ __forceinline__ void split(float v, float& hi, float& lo) {
+  hi = __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xffffe000u);
+  lo = v - hi;
 }
-__device__ __forceinline__ uint32_t magnitude(float v) { return __float_as_uint(v) & 0x7fffffffu; }
-__device__ __forceinline__ uint32_t finite_bits(float v) { return magnitude(v) < 0x7f800000u ? magnitude(v) : 0u; }
-constexpr uint32_t SG_INFINITE = 0x7f800000u;
-// Two scaled values as pairs of r16 terms.  KEEP: an infinity stays one (its lower term must not be inf - inf; any finite value does, lower
-// terms stay below 2^4).
-template <bool KEEP>
-__device__ __forceinline__ void split(float v0, float v1, uint32_t& hi, uint32_t& lo) {
-  const __half2 h = __floats2half2_rn(v0, v1);
-  const float2 f = __half22float2(h);
-  const float l0 = v0 - f.x, l1 = v1 - f.y;
-  const __half2 l = KEEP ? __floats2half2_rn(fmaxf(l0, -64.f), fmaxf(l1, -64.f)) : __floats2half2_rn(l0, l1);
-  hi = *reinterpret_cast<const uint32_t*>(&h);
-  lo = *reinterpret_cast<const uint32_t*>(&l);
+// The same where an infinity has to stay one: 11 bits cut off, the rest rounded; none where there is none.
+__device__ __forceinline__ void split_keeping(float v, float& hi, float& lo) {
+  hi = __uint_as_float(__float_as_uint(v) & 0xffffe000u);
+  const float rest = v - hi;
+  uint32_t r;
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(rest));
+  lo = rest == rest ? __uint_as_float(r) : 0.f;
 }
 
 // ---------------------------------------------------------------------------
-// What a segment adds to the state behind it (blockIdx.y = 0) and to the adjoint state before it (1): fp32, in blocks of 16 x 16 (p, n), a block
-// as the fragments of its two 8-column tiles: eight values a lane.  A warp has 16 of the 64 rows p.
+// What a segment adds to the state behind it (blockIdx.y = 0) and to the adjoint state before it (1).  A warp has 16 of the 64 rows p.
 // ---------------------------------------------------------------------------
 constexpr int SS_THREADS = 128;
 constexpr size_t SS_SMEM = SG_Q * SG_P * 2 + SG_Q * SG_N * 2 + SG_Q * sizeof(float);
@@ -233,45 +263,18 @@ __global__ void __launch_bounds__(SS_THREADS) segment_states_kernel(const SegArg
   cp_async_wait<0>();
   __syncthreads();
   // rows p of the scaled values, over the 64 steps
-  float v[4][8];
-  uint32_t m0 = 0, m1 = 0;
+  float hi[4][8], lo[4][8];
 #pragma unroll
   for (int kt = 0; kt < 4; ++kt) {
     uint32_t r[4];
     load_a_t<SG_P * 2>(r, sv, kt * 16, warp * 2, lane);
+    float v[8];
+    widen(v, r, 4);
     const float2 wa = *reinterpret_cast<const float2*>(wt + kt * 16 + 2 * q), wb = *reinterpret_cast<const float2*>(wt + kt * 16 + 8 + 2 * q);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&r[e]));
-      v[kt][2 * e] = f.x * (e < 2 ? wa.x : wb.x);
-      v[kt][2 * e + 1] = f.y * (e < 2 ? wa.y : wb.y);
-      uint32_t& m = e & 1 ? m1 : m0;
-      m = max(m, max(magnitude(v[kt][2 * e]), magnitude(v[kt][2 * e + 1])));
-    }
+    for (int e = 0; e < 8; ++e) split_keeping(v[e] * (e < 4 ? (e & 1 ? wa.y : wa.x) : (e & 1 ? wb.y : wb.x)), hi[kt][e], lo[kt][e]);
   }
-  if (__any_sync(0xffffffffu, max(m0, m1) >= SG_INFINITE)) {   // the finite values set the scale
-    m0 = m1 = 0;
-#pragma unroll
-    for (int kt = 0; kt < 4; ++kt)
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        uint32_t& m = (e >> 1) & 1 ? m1 : m0;
-        m = max(m, finite_bits(v[kt][e]));
-      }
-  }
-#pragma unroll
-  for (int o = 1; o < 4; o <<= 1) {
-    m0 = max(m0, __shfl_xor_sync(0xffffffffu, m0, o));
-    m1 = max(m1, __shfl_xor_sync(0xffffffffu, m1, o));
-  }
-  float i0, i1;
-  const float f0 = split_scale(m0, &i0), f1 = split_scale(m1, &i1);
-  uint32_t hi[4][4], lo[4][4];
-#pragma unroll
-  for (int kt = 0; kt < 4; ++kt)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) split<true>(v[kt][2 * e] * (e & 1 ? f1 : f0), v[kt][2 * e + 1] * (e & 1 ? f1 : f0), hi[kt][e], lo[kt][e]);
-  float* out = reinterpret_cast<float*>(g.states + (static_cast<size_t>(anti) * g.B * g.H * g.nseg + blockIdx.x) * SG_STATE_BYTES) + warp * 2048 + lane * 8;
+  float* out = g.states + (static_cast<size_t>(anti) * g.B * g.H * g.nseg + blockIdx.x) * (SG_N * SG_P) + (warp * 16 + (lane >> 2)) * SG_N + 2 * q;
 #pragma unroll 2
   for (int nb = 0; nb < SG_N / 16; ++nb) {
     // `finite`: the r16 operand of the lower terms, whose zeros must not meet an infinity
@@ -280,20 +283,22 @@ __global__ void __launch_bounds__(SS_THREADS) segment_states_kernel(const SegArg
       for (int kt = 0; kt < 4; ++kt) {
         uint32_t bb[4];
         load_b_t<SG_N * 2>(bb, sk, kt * 16, nb * 2, lane);
-        float c0[4], c1[4];
-        if (finite) {
-          mma0(c0, lo[kt], r16_finite(bb[0]), r16_finite(bb[1]));
-          mma0(c1, lo[kt], r16_finite(bb[2]), r16_finite(bb[3]));
-        } else {
-          mma0(c0, lo[kt], bb[0], bb[1]);
-          mma0(c1, lo[kt], bb[2], bb[3]);
-        }
-        mma(c0, hi[kt], bb[0], bb[1]);
-        mma(c1, hi[kt], bb[2], bb[3]);
+        float b[8];
+        widen(b, bb, 4);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          s[0][e] = kt == 0 ? c0[e] : s[0][e] + c0[e];
-          s[1][e] = kt == 0 ? c1[e] : s[1][e] + c1[e];
+        for (int u = 0; u < 2; ++u) {
+          float c[4];
+          if (finite) {
+            const uint32_t bf[2] = {r16_finite(bb[2 * u]), r16_finite(bb[2 * u + 1])};
+            float f[4];
+            widen(f, bf, 2);
+            mma160(c, lo[kt], f);
+          } else {
+            mma160(c, lo[kt], b + 4 * u);
+          }
+          mma16(c, hi[kt], b + 4 * u);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) s[u][e] = kt == 0 ? c[e] : s[u][e] + c[e];
         }
       }
     };
@@ -303,88 +308,54 @@ __global__ void __launch_bounds__(SS_THREADS) segment_states_kernel(const SegArg
 #pragma unroll
     for (int e = 0; e < 4; ++e) check = fmaf(s[0][e], 0.f, fmaf(s[1][e], 0.f, check));
     if (__any_sync(0xffffffffu, check != 0.f)) sums(s, true);
-    *reinterpret_cast<float4*>(out + nb * 256) = make_float4(s[0][0] * i0, s[0][1] * i0, s[0][2] * i1, s[0][3] * i1);
-    *reinterpret_cast<float4*>(out + nb * 256 + 4) = make_float4(s[1][0] * i0, s[1][1] * i0, s[1][2] * i1, s[1][3] * i1);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      *reinterpret_cast<float2*>(out + nb * 16 + u * 8) = make_float2(s[u][0], s[u][1]);
+      *reinterpret_cast<float2*>(out + 8 * SG_N + nb * 16 + u * 8) = make_float2(s[u][2], s[u][3]);
+    }
   }
 }
 
-// In place: what every segment adds becomes what every segment receives, in two terms.  One warp per block of a sequence's state; it reads
-// four segments ahead, and what it overwrites (the segment behind the one whose sum it has) it has read before.
+// In place: what every segment adds becomes what every segment receives.  A thread has four values of a sequence's states; it reads four
+// segments ahead, and what it overwrites (the segment behind the one whose sum it has) it has read before.
 constexpr int SC_THREADS = 128;
 __global__ void __launch_bounds__(SC_THREADS) segment_carry_kernel(const SegArgs g) {
   mp_grid_dependency();
-  constexpr int PER = SG_BLOCKS / (SC_THREADS / 32);   // CTAs per sequence
+  constexpr int PER = SG_N * SG_P / 4 / SC_THREADS;   // CTAs per sequence
   const bool anti = blockIdx.y != 0;
-  const int lane = threadIdx.x & 31, q = lane & 3;
-  const int seq = blockIdx.x / PER, blk = (blockIdx.x % PER) * (SC_THREADS / 32) + (threadIdx.x >> 5);
-  const size_t first = (static_cast<size_t>(anti) * g.B * g.H + seq) * g.nseg;
-  unsigned char* base = g.states + first * SG_STATE_BYTES + blk * 1024;
-  float* scales = g.scales + first * SG_BLOCKS + blk;
+  const int seq = blockIdx.x / PER;
+  float4* base = reinterpret_cast<float4*>(g.states + (static_cast<size_t>(anti) * g.B * g.H + seq) * g.nseg * (SG_N * SG_P)) +
+                 (blockIdx.x % PER) * SC_THREADS + threadIdx.x;
   const float* decay = g.decay + static_cast<size_t>(seq) * g.nseg;
   const int steps = g.nseg - 1;
   auto segment = [&](int k) { return anti ? g.nseg - 1 - k : k; };
-  float4 next[4][2];
+  float4 next[4];
   float dnext[4];
   auto fetch = [&](int k0) {
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int k = min(k0 + u, steps - 1);
-      const float4* p = reinterpret_cast<const float4*>(base + static_cast<size_t>(segment(k)) * SG_STATE_BYTES) + lane * 2;
-      next[u][0] = p[0];
-      next[u][1] = p[1];
+      next[u] = base[static_cast<size_t>(segment(k)) * (SG_N * SG_P / 4)];
       dnext[u] = decay[segment(k)];
     }
   };
   fetch(0);
-  float c[2][4] = {};
+  float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 1
   for (int k0 = 0; k0 < steps; k0 += 4) {
-    float4 add[4][2];
+    float4 add[4];
     float d[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) { add[u][0] = next[u][0]; add[u][1] = next[u][1]; d[u] = dnext[u]; }
+    for (int u = 0; u < 4; ++u) { add[u] = next[u]; d[u] = dnext[u]; }
     if (k0 + 4 < steps) fetch(k0 + 4);
-    __syncwarp();   // every lane has read segment k0 + 4 before the state that takes its place is written
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       if (k0 + u >= steps) break;
-      const float a[2][4] = {{add[u][0].x, add[u][0].y, add[u][0].z, add[u][0].w}, {add[u][1].x, add[u][1].y, add[u][1].z, add[u][1].w}};
-      uint32_t m = 0;
-#pragma unroll
-      for (int t = 0; t < 2; ++t)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          c[t][e] = fmaf(d[u], c[t][e], a[t][e]);
-          m = max(m, magnitude(c[t][e]));
-        }
-      m = __reduce_max_sync(0xffffffffu, m);
-      if (m >= SG_INFINITE) {   // the finite values set the scale
-        m = 0;
-#pragma unroll
-        for (int t = 0; t < 2; ++t)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) m = max(m, finite_bits(c[t][e]));
-        m = __reduce_max_sync(0xffffffffu, m);
-      }
-      float inv;
-      const float f = split_scale(m, &inv);
-      const int to = segment(k0 + u) + (anti ? -1 : 1);
-      if (lane == 0) scales[static_cast<size_t>(to) * SG_BLOCKS] = inv;
-      unsigned char* out = base + static_cast<size_t>(to) * SG_STATE_BYTES + (lane >> 2) * 64 + q * 16;
-#pragma unroll
-      for (int r = 0; r < 2; ++r) {   // rows g, g + 8: four chunks of the row over the four lanes of a quad, exchanged for one chunk a lane
-        uint32_t t[4];
-        split<true>(c[0][2 * r] * f, c[0][2 * r + 1] * f, t[0], t[2]);
-        split<true>(c[1][2 * r] * f, c[1][2 * r + 1] * f, t[1], t[3]);
-        uint32_t x0 = q & 1 ? t[1] : t[0], x1 = q & 1 ? t[0] : t[1], x2 = q & 1 ? t[3] : t[2], x3 = q & 1 ? t[2] : t[3];
-        x1 = __shfl_xor_sync(0xffffffffu, x1, 1);
-        x3 = __shfl_xor_sync(0xffffffffu, x3, 1);
-        t[0] = q & 1 ? x1 : x0; t[1] = q & 1 ? x0 : x1; t[2] = q & 1 ? x3 : x2; t[3] = q & 1 ? x2 : x3;
-        x0 = q & 2 ? t[2] : t[0]; x2 = q & 2 ? t[0] : t[2]; x1 = q & 2 ? t[3] : t[1]; x3 = q & 2 ? t[1] : t[3];
-        x2 = __shfl_xor_sync(0xffffffffu, x2, 2);
-        x3 = __shfl_xor_sync(0xffffffffu, x3, 2);
-        *reinterpret_cast<uint4*>(out + r * 512) = q & 2 ? make_uint4(x2, x3, x0, x1) : make_uint4(x0, x1, x2, x3);
-      }
+      c.x = fmaf(d[u], c.x, add[u].x);
+      c.y = fmaf(d[u], c.y, add[u].y);
+      c.z = fmaf(d[u], c.z, add[u].z);
+      c.w = fmaf(d[u], c.w, add[u].w);
+      base[static_cast<size_t>(segment(k0 + u) + (anti ? -1 : 1)) * (SG_N * SG_P / 4)] = c;
     }
   }
 }
@@ -466,26 +437,15 @@ __device__ __forceinline__ void block_decays(float (&m)[2][4], const double* cum
     }
   }
 }
-// A block as pairs of r16 terms in two tiles [64][64]; its scale's reciprocal goes to inv[4 ib + jb].
-__device__ __forceinline__ void block_split(const float (&v)[2][4], uint32_t hi, uint32_t lo, float* inv, int ib, int jb, int lane) {
-  float m = 0.f;
+// A block of a tile [64][64] in fp32.
+__device__ __forceinline__ void block_store(const float (&v)[2][4], uint32_t tile, int ib, int jb, int lane) {
 #pragma unroll
   for (int u = 0; u < 2; ++u)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) m = fmaxf(m, fabsf(v[u][e]));
-  float back;
-  const float f = split_scale(min(__reduce_max_sync(0xffffffffu, __float_as_uint(m)), SG_INFINITE - 1), &back);
-  if (lane == 0) inv[4 * ib + jb] = back;
-#pragma unroll
-  for (int u = 0; u < 2; ++u)
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      uint32_t h, l;
-      split<false>(v[u][2 * r] * f, v[u][2 * r + 1] * f, h, l);
-      const uint32_t at = tile_at<SG_Q * 2>(0, ib * 16 + (lane >> 2) + 8 * r, jb * 2 + u) + 4 * (lane & 3);
-      asm volatile("st.shared.b32 [%0], %1;" ::"r"(hi + at), "r"(h) : "memory");
-      asm volatile("st.shared.b32 [%0], %1;" ::"r"(lo + at), "r"(l) : "memory");
-    }
+    for (int r = 0; r < 2; ++r)
+      asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(wide_at<SG_Q * 4>(tile, ib * 16 + (lane >> 2) + 8 * r, jb * 4 + u * 2 + ((lane & 3) >> 1)) +
+                                                           8 * (lane & 1)),
+                   "f"(v[u][2 * r]), "f"(v[u][2 * r + 1]) : "memory");
 }
 
 // ---------------------------------------------------------------------------
@@ -498,52 +458,63 @@ __device__ __forceinline__ int row_block(int i, int part) { return NR == 4 ? i :
 
 // Rows of a tile [64][128] (over n) times a state: columns p = 8 c .. 8 c + 7.
 template <int NR>
-__device__ __forceinline__ void times_state_p(float (&o)[NR][4], uint32_t rows, uint32_t state, const float* scales, int c, int part, int lane) {
+__device__ __forceinline__ void times_state_p(float (&o)[NR][4], uint32_t rows, uint32_t state, int c, int part, int lane) {
+  const int q = lane & 3;
 #pragma unroll
   for (int i = 0; i < NR; ++i)
 #pragma unroll
     for (int e = 0; e < 4; ++e) o[i][e] = 0.f;
 #pragma unroll 2
   for (int k = 0; k < 8; ++k) {
-    uint32_t b[4];
-    ldsm(b, tile_at<512>(state, c * 8 + (lane & 7), k * 4 + (lane >> 3)));
-    const float f = scales[(c >> 1) * 8 + k];
+    float hi[4], lo[4];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float2 v = ld_shared8(wide_at<512>(state, c * 8 + (lane >> 2), k * 4 + 2 * h + (q >> 1)) + 8 * (q & 1));
+      split(v.x, hi[2 * h], lo[2 * h]);
+      split(v.y, hi[2 * h + 1], lo[2 * h + 1]);
+    }
 #pragma unroll
     for (int i = 0; i < NR; ++i) {
-      uint32_t a[4];
-      load_a<SG_N * 2>(a, rows, row_block<NR>(i, part) * 16, 2 * k, lane);
-      float s[4];
-      mma0(s, a, b[2], b[3]);
-      mma(s, a, b[0], b[1]);
+      uint32_t r[4];
+      load_a<SG_N * 2>(r, rows, row_block<NR>(i, part) * 16, 2 * k, lane);
+      float a[8], s[4];
+      widen(a, r, 4);
+      mma160(s, a, lo);
+      mma16(s, a, hi);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) o[i][e] = fmaf(s[e], f, o[i][e]);
+      for (int e = 0; e < 4; ++e) o[i][e] += s[e];
     }
   }
 }
 // Rows of a tile [64][64] (over p) times a state: columns n = 16 nb .. 16 nb + 15.
 template <int NR>
-__device__ __forceinline__ void times_state_n(float (&o)[NR][2][4], uint32_t rows, uint32_t state, const float* scales, int nb, int part, int lane) {
+__device__ __forceinline__ void times_state_n(float (&o)[NR][2][4], uint32_t rows, uint32_t state, int nb, int part, int lane) {
+  const int q = lane & 3, n = lane >> 2;
 #pragma unroll
   for (int i = 0; i < NR; ++i)
 #pragma unroll
     for (int e = 0; e < 4; ++e) o[i][0][e] = o[i][1][e] = 0.f;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    uint32_t b[2][4];
+    float hi[2][4], lo[2][4];
 #pragma unroll
-    for (int u = 0; u < 2; ++u) ldsm_t(b[u], tile_at<512>(state, k * 16 + (lane & 15), nb * 4 + u + ((lane >> 4) << 1)));
-    const float f = scales[k * 8 + nb];
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        split(ld_shared4(wide_at<512>(state, k * 16 + 2 * q + (e & 1) + 8 * (e >> 1), nb * 4 + u * 2 + (n >> 2)) + 4 * (n & 3)), hi[u][e], lo[u][e]);
 #pragma unroll
     for (int i = 0; i < NR; ++i) {
-      uint32_t a[4];
-      load_a<SG_P * 2>(a, rows, row_block<NR>(i, part) * 16, 2 * k, lane);
+      uint32_t r[4];
+      load_a<SG_P * 2>(r, rows, row_block<NR>(i, part) * 16, 2 * k, lane);
+      float a[8];
+      widen(a, r, 4);
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         float s[4];
-        mma0(s, a, b[u][2], b[u][3]);
-        mma(s, a, b[u][0], b[u][1]);
+        mma160(s, a, lo[u]);
+        mma16(s, a, hi[u]);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) o[i][u][e] = fmaf(s[e], f, o[i][u][e]);
+        for (int e = 0; e < 4; ++e) o[i][u][e] += s[e];
       }
     }
   }
@@ -559,32 +530,39 @@ __device__ __forceinline__ void load_steps(uint32_t (&b)[4][2], uint32_t tile, i
 }
 // o += scores (LOWER: rows i, over j up to the row's block; otherwise rows j, over i from the row's block on) times COLS tiles of eight columns.
 template <int NR, bool LOWER, int COLS>
-__device__ __forceinline__ void times_scores(float (&o)[NR][COLS][4], uint32_t hi, uint32_t lo, const float* inv, const uint32_t (&b)[4][2 * COLS], int part,
-                                             int lane) {
+__device__ __forceinline__ void times_scores(float (&o)[NR][COLS][4], uint32_t scores, const uint32_t (&b)[4][2 * COLS], int part, int lane) {
+  const int q = lane & 3, r = lane >> 2;
 #pragma unroll
-  for (int i = 0; i < NR; ++i)
+  for (int k = 0; k < 4; ++k) {
+    float bv[4 * COLS];
+    widen(bv, b[k], 2 * COLS);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
+    for (int i = 0; i < NR; ++i) {
       const int rb = row_block<NR>(i, part);
       if (LOWER ? k > rb : k < rb) continue;
-      uint32_t h[4], l[4];
-      if (LOWER) {
-        load_a<SG_Q * 2>(h, hi, rb * 16, 2 * k, lane);
-        load_a<SG_Q * 2>(l, lo, rb * 16, 2 * k, lane);
-      } else {
-        load_a_t<SG_Q * 2>(h, hi, k * 16, 2 * rb, lane);
-        load_a_t<SG_Q * 2>(l, lo, k * 16, 2 * rb, lane);
+      float hi[8], lo[8];   // rows r, r + 8 of the block, steps 2 q, 2 q + 1, then those eight further
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        float2 v;
+        if (LOWER) {
+          v = ld_shared8(wide_at<SG_Q * 4>(scores, rb * 16 + r + 8 * (e & 1), k * 4 + 2 * (e >> 1) + (q >> 1)) + 8 * (q & 1));
+        } else {
+          v.x = ld_shared4(wide_at<SG_Q * 4>(scores, k * 16 + 2 * q + 8 * (e >> 1), rb * 4 + 2 * (e & 1) + (r >> 2)) + 4 * (r & 3));
+          v.y = ld_shared4(wide_at<SG_Q * 4>(scores, k * 16 + 2 * q + 1 + 8 * (e >> 1), rb * 4 + 2 * (e & 1) + (r >> 2)) + 4 * (r & 3));
+        }
+        split(v.x, hi[2 * e], lo[2 * e]);
+        split(v.y, hi[2 * e + 1], lo[2 * e + 1]);
       }
-      const float f = LOWER ? inv[4 * rb + k] : inv[4 * k + rb];
 #pragma unroll
       for (int u = 0; u < COLS; ++u) {
         float s[4];
-        mma0(s, l, b[k][2 * u], b[k][2 * u + 1]);
-        mma(s, h, b[k][2 * u], b[k][2 * u + 1]);
+        mma160(s, lo, bv + 4 * u);
+        mma16(s, hi, bv + 4 * u);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) o[i][u][e] = fmaf(s[e], f, o[i][u][e]);
+        for (int e = 0; e < 4; ++e) o[i][u][e] += s[e];
       }
     }
+  }
 }
 // Two neighbouring r16 results.
 __device__ __forceinline__ void store_pair(__half* dst, float v0, float v1, bool vec) {
@@ -633,18 +611,12 @@ __device__ __forceinline__ void segment_store(__half* dst, const float* v, bool 
   }
 }
 
-// The value (n, p) of a state in global memory.
-__device__ __forceinline__ float state_value(const unsigned char* state, const float* scales, int n, int p) {
-  const int blk = (p >> 4) * 8 + (n >> 4);
-  const __half* v = reinterpret_cast<const __half*>(state + blk * 1024 + (p & 15) * 64) + (n & 15);
-  return (__half2float(v[0]) + __half2float(v[16])) * scales[blk];
-}
 template <int THREADS>
-__device__ __forceinline__ void plain_state(float* dst, const unsigned char* state, const float* scales) {
+__device__ __forceinline__ void plain_state(float* dst, const float* state) {
 #pragma unroll 1
   for (int idx = threadIdx.x; idx < SG_N * SG_P; idx += THREADS) {
     const int p = idx / SG_N, n = idx % SG_N;
-    dst[state_at(n, p >> 2) + (p & 3)] = state_value(state, scales, n, p);
+    dst[state_at(n, p >> 2) + (p & 3)] = state[idx];
   }
 }
 
@@ -711,7 +683,7 @@ __device__ __noinline__ void segment_forward_plain(const SegArgs& g, float* smem
     __syncthreads();
     if (seg > 0) {
       const size_t unit = (static_cast<size_t>(b) * g.H + h) * g.nseg + seg;
-      plain_state<SG_THREADS>(sB, g.states + unit * SG_STATE_BYTES, g.scales + unit * SG_BLOCKS);
+      plain_state<SG_THREADS>(sB, g.states + unit * (SG_N * SG_P));
       __syncthreads();
     }
     {
@@ -772,9 +744,9 @@ __device__ __noinline__ void segment_forward_plain(const SegArgs& g, float* smem
 // y of one (batch entry, segment, group, share of the group's heads).  A warp has eight of the 64 columns; the next head's tiles arrive
 // while one is worked on.
 // ---------------------------------------------------------------------------
-constexpr int SF_X = SG_Q * SG_P * 2, SF_S = SG_STATE_BYTES + SG_BLOCKS * 4;
-constexpr size_t SF_TILES = SG_Q * SG_N * 2 + 2 * SF_X + SF_S + 2 * SG_Q * SG_Q * 2;   // C, x twice, state, weights in two terms
-constexpr size_t SF_SMEM = SF_TILES + 2 * sizeof(SegSteps) + 16 * sizeof(float);
+constexpr int SF_X = SG_Q * SG_P * 2;
+constexpr size_t SF_TILES = SG_Q * SG_N * 2 + 2 * SF_X + SG_STATE_BYTES + SG_Q * SG_Q * 4;   // C, x twice, state, weights
+constexpr size_t SF_SMEM = SF_TILES + 2 * sizeof(SegSteps);
 
 __global__ void __launch_bounds__(SG_THREADS, 2) segment_forward_kernel(const SegArgs g) {
   mp_grid_dependency();
@@ -784,16 +756,13 @@ __global__ void __launch_bounds__(SG_THREADS, 2) segment_forward_kernel(const Se
   const int t0 = sh.seg * SG_Q, rows = min(SG_Q, g.L - t0);
   const size_t row = static_cast<size_t>(sh.b) * g.L + t0;
   const bool before = sh.seg > 0;
-  const uint32_t sC = mp_smem_u32(seg_smem), sX = sC + SG_Q * SG_N * 2, sH = sX + 2 * SF_X, sPh = sH + SF_S, sPl = sPh + SG_Q * SG_Q * 2;
-  const float* hscales = reinterpret_cast<const float*>(seg_smem + (sH + SG_STATE_BYTES - sC));
+  const uint32_t sC = mp_smem_u32(seg_smem), sX = sC + SG_Q * SG_N * 2, sH = sX + 2 * SF_X, sW = sH + SG_STATE_BYTES;
   SegSteps* steps = reinterpret_cast<SegSteps*>(seg_smem + SF_TILES);
-  float* inv = reinterpret_cast<float*>(steps + 2);
   auto load_x = [&](int h) {
     tile_load<SG_P / 8, SG_THREADS>(sX + ((h - sh.h_first) & 1) * SF_X, g.x + (row * g.H + h) * SG_P, static_cast<size_t>(g.H) * SG_P, rows, g.vec);
   };
   auto load_state = [&](int h) {
-    const size_t unit = (static_cast<size_t>(sh.b) * g.H + h) * g.nseg + sh.seg;
-    if (before) state_load<SG_THREADS>(sH, g.states + unit * SG_STATE_BYTES, g.scales + unit * SG_BLOCKS);
+    if (before) state_load<SG_THREADS>(sH, g.states + ((static_cast<size_t>(sh.b) * g.H + h) * g.nseg + sh.seg) * (SG_N * SG_P));
   };
   tile_load<SG_N / 8, SG_THREADS>(sC, g.Cm + (row * g.G + sh.grp) * SG_N, static_cast<size_t>(g.G) * SG_N, rows, g.vec);
   tile_load<SG_N / 8, SG_THREADS>(sH, g.Bm + (row * g.G + sh.grp) * SG_N, static_cast<size_t>(g.G) * SG_N, rows, g.vec);   // B, for the scores
@@ -835,12 +804,12 @@ __global__ void __launch_bounds__(SG_THREADS, 2) segment_forward_kernel(const Se
 #pragma unroll
         for (int e = 0; e < 4; ++e) m[u][e] = G[s][u][e] * m[u][e] * (e & 1 ? dj.y : dj.x);
       }
-      block_split(m, sPh, sPl, inv, ib, jb, lane);
+      block_store(m, sW, ib, jb, lane);
     }
     float o[4][1][4];
     if (before) {
       float v[4][4];
-      times_state_p<4>(v, sC, sH, hscales, warp, 0, lane);
+      times_state_p<4>(v, sC, sH, warp, 0, lane);
 #pragma unroll
       for (int rb = 0; rb < 4; ++rb) {
         const float f0 = st.grow[rb * 16 + r0], f1 = st.grow[rb * 16 + r0 + 8];
@@ -858,7 +827,7 @@ __global__ void __launch_bounds__(SG_THREADS, 2) segment_forward_kernel(const Se
     cp_async_commit();
     uint32_t b[4][2];
     load_steps(b, sX + par * SF_X, warp, lane);
-    times_scores<4, true, 1>(o, sPh, sPl, inv, b, 0, lane);
+    times_scores<4, true, 1>(o, sW, b, 0, lane);
     __half* y = g.y + ((row + r0) * g.H + h) * SG_P + warp * 8 + 2 * q;
 #pragma unroll
     for (int rb = 0; rb < 4; ++rb)
@@ -877,8 +846,8 @@ __global__ void __launch_bounds__(SG_THREADS, 2) segment_forward_kernel(const Se
 // gC, which stay in their registers over the heads, and eight of the 64 columns of gx.
 // ---------------------------------------------------------------------------
 constexpr int SR_THREADS = 512, SR_WARPS = SR_THREADS / 32;
-constexpr int SR_X = SG_Q * SG_P * 2, SR_S = SG_STATE_BYTES + SG_BLOCKS * 4;
-constexpr int SR_STAGE = 2 * SR_X + SR_S;   // x, gy, H: two of them; Y is read first and loaded again in the middle
+constexpr int SR_X = SG_Q * SG_P * 2;
+constexpr int SR_STAGE = 2 * SR_X + SG_STATE_BYTES;   // x, gy, H: two of them; Y is read first and loaded again in the middle
 struct SegScalars {   // of one head; two of them, and three SegSteps (the next head's are made while the last one's are read)
   float s[4][SG_Q];       // [row block] sums over the block's rows of M G X
   float ga[4][SG_Q];      // [column block] sums over the block's columns of M G X dt, for the row blocks below it
@@ -887,8 +856,8 @@ struct SegScalars {   // of one head; two of them, and three SegSteps (the next 
   float sv[8][SG_Q];      // [16 columns] e_j <B_j, Y x_j>
   float pin[SR_WARPS];    // [warp] parts of <Y, H>
 };
-constexpr size_t SR_TILES = 2 * SG_Q * SG_N * 2 + 2 * SR_STAGE + SR_S + 4 * SG_Q * SG_Q * 2;
-constexpr size_t SR_SMEM = SR_TILES + 3 * sizeof(SegSteps) + 2 * sizeof(SegScalars) + 32 * sizeof(float);
+constexpr size_t SR_TILES = 2 * SG_Q * SG_N * 2 + 2 * SR_STAGE + SG_STATE_BYTES + 2 * SG_Q * SG_Q * 4;
+constexpr size_t SR_SMEM = SR_TILES + 3 * sizeof(SegSteps) + 2 * sizeof(SegScalars);
 
 // gdt and a part of gA of one head, by one warp; a lane has two steps, eight lanes a block of 16.
 __device__ __forceinline__ void segment_gradients(const SegArgs& g, const SegScalars& w, const SegSteps& st, int h, size_t row, int rows, size_t unit, int lane) {
@@ -1096,13 +1065,12 @@ __device__ __noinline__ void segment_reverse_plain(const SegArgs& g, float* smem
   for (int h = h_first; h < h_end; ++h) {
     const size_t unit = (static_cast<size_t>(b) * g.H + h) * g.nseg + seg;
     const size_t yunit = static_cast<size_t>(g.B) * g.H * g.nseg + unit;
-    const unsigned char *hstate = g.states + unit * SG_STATE_BYTES, *ystate = g.states + yunit * SG_STATE_BYTES;
-    const float *hscales = g.scales + unit * SG_BLOCKS, *yscales = g.scales + yunit * SG_BLOCKS;
+    const float *hstate = g.states + unit * (SG_N * SG_P), *ystate = g.states + yunit * (SG_N * SG_P);
     named_bar_sync(1, SG_THREADS);   // the previous head's tiles and scalars have been read (and sG is complete)
     if (warp == 0) segment_scalars(g, b, h, t0, cum, dt, lane);
     plain_tile<SG_P, SG_PPITCH, SG_THREADS>(sX, g.x + (row * g.H + h) * SG_P, static_cast<size_t>(g.H) * SG_P, rows);
     plain_tile<SG_P, SG_PPITCH, SG_THREADS>(sGy, g.gy + (row * g.H + h) * SG_P, static_cast<size_t>(g.H) * SG_P, rows);
-    if (behind) plain_state<SG_THREADS>(sS, ystate, yscales);
+    if (behind) plain_state<SG_THREADS>(sS, ystate);
     named_bar_sync(1, SG_THREADS);
     {
       float s[4][4];
@@ -1267,8 +1235,8 @@ __device__ __noinline__ void segment_reverse_plain(const SegArgs& g, float* smem
 #pragma unroll 1
       for (int idx = threadIdx.x; idx < SG_N * SG_P; idx += SG_THREADS) {
         const int p = idx / SG_N, n = idx % SG_N;
-        const float v = state_value(hstate, hscales, n, p);
-        if (behind) pin += v * state_value(ystate, yscales, n, p);
+        const float v = hstate[idx];
+        if (behind) pin += v * ystate[idx];
         sS[state_at(n, p >> 2) + (p & 3)] = v;
       }
       pin = warp_reduce<SumOp>(pin);
@@ -1380,21 +1348,19 @@ __global__ void __launch_bounds__(SR_THREADS, 1) segment_reverse_kernel(const Se
   const bool before = sh.seg > 0, behind = sh.seg < g.nseg - 1;
   const size_t row = static_cast<size_t>(sh.b) * g.L + t0;
   const uint32_t smem = mp_smem_u32(seg_smem), sB = smem, sC = sB + SG_Q * SG_N * 2, stages = sC + SG_Q * SG_N * 2, sY = stages + 2 * SR_STAGE;
-  const uint32_t sWh = sY + SR_S, sWl = sWh + SG_Q * SG_Q * 2, sMh = sWl + SG_Q * SG_Q * 2, sMl = sMh + SG_Q * SG_Q * 2;   // M X dt, M G
+  const uint32_t sW = sY + SG_STATE_BYTES, sM = sW + SG_Q * SG_Q * 4;   // M X dt, M G
   SegSteps* steps = reinterpret_cast<SegSteps*>(seg_smem + SR_TILES);
   SegScalars* scalars = reinterpret_cast<SegScalars*>(steps + 3);
-  float *invW = reinterpret_cast<float*>(scalars + 2), *invM = invW + 16;
-  const float* yscales = reinterpret_cast<const float*>(seg_smem + (sY + SG_STATE_BYTES - smem));
   auto unit_of = [&](int h) { return (static_cast<size_t>(sh.b) * g.H + h) * g.nseg + sh.seg; };
   auto load_stage = [&](int h) {
     const uint32_t st = stages + ((h - sh.h_first) & 1) * SR_STAGE;
     tile_load<SG_P / 8, SR_THREADS>(st, g.x + (row * g.H + h) * SG_P, static_cast<size_t>(g.H) * SG_P, rows, g.vec);
     tile_load<SG_P / 8, SR_THREADS>(st + SR_X, g.gy + (row * g.H + h) * SG_P, static_cast<size_t>(g.H) * SG_P, rows, g.vec);
-    if (before) state_load<SR_THREADS>(st + 2 * SR_X, g.states + unit_of(h) * SG_STATE_BYTES, g.scales + unit_of(h) * SG_BLOCKS);
+    if (before) state_load<SR_THREADS>(st + 2 * SR_X, g.states + unit_of(h) * (SG_N * SG_P));
   };
   auto load_adjoint = [&](int h) {
     const size_t unit = static_cast<size_t>(g.B) * g.H * g.nseg + unit_of(h);
-    if (behind) state_load<SR_THREADS>(sY, g.states + unit * SG_STATE_BYTES, g.scales + unit * SG_BLOCKS);
+    if (behind) state_load<SR_THREADS>(sY, g.states + unit * (SG_N * SG_P));
   };
   tile_load<SG_N / 8, SR_THREADS>(sB, g.Bm + (row * g.G + sh.grp) * SG_N, static_cast<size_t>(g.G) * SG_N, rows, g.vec);
   tile_load<SG_N / 8, SR_THREADS>(sC, g.Cm + (row * g.G + sh.grp) * SG_N, static_cast<size_t>(g.G) * SG_N, rows, g.vec);
@@ -1410,11 +1376,11 @@ __global__ void __launch_bounds__(SR_THREADS, 1) segment_reverse_kernel(const Se
   const bool scores = block_of(warp, ib, jb);
   if (scores) block_scores<SG_N>(G, sC, sB, ib, jb, lane);
   float gB[2][2][4] = {}, gC[2][2][4] = {};
+  float check = 0.f;   // becomes NaN with the first result that is none, or infinite
 #pragma unroll 1
   for (int h = sh.h_first; h < sh.h_end; ++h) {
     const int n = h - sh.h_first;
     const uint32_t sx = stages + (n & 1) * SR_STAGE, sgy = sx + SR_X, sH = sgy + SR_X;
-    const float* hscales = reinterpret_cast<const float*>(seg_smem + (sH + SG_STATE_BYTES - smem));
     cp_async_wait<0>();
     __syncthreads();   // this head's tiles are there, the other stage, the weights and the last head's scalars are complete and read
     if (h + 1 < sh.h_end) {
@@ -1425,7 +1391,7 @@ __global__ void __launch_bounds__(SR_THREADS, 1) segment_reverse_kernel(const Se
     if (warp == 14 && n > 0) segment_gradients(g, scalars[(n - 1) & 1], steps[(n - 1) % 3], h - 1, row, rows, unit_of(h - 1), lane);
     SegScalars& sc = scalars[n & 1];
     const SegSteps& st = steps[n % 3];
-    // ---- scores: M X dt and M G in two terms, the sums of M G X ----
+    // ---- scores: M X dt and M G, the sums of M G X ----
     if (scores) {
       float x[2][4], m[2][4], w[2][4];
       block_scores<SG_P>(x, sgy, sx, ib, jb, lane);
@@ -1451,27 +1417,17 @@ __global__ void __launch_bounds__(SR_THREADS, 1) segment_reverse_kernel(const Se
 #pragma unroll
         for (int e = 0; e < 4; ++e) x[u][e] *= e & 1 ? dj.y : dj.x;
       }
-      block_split(x, sWh, sWl, invW, ib, jb, lane);
-      block_split(m, sMh, sMl, invM, ib, jb, lane);
+      block_store(x, sW, ib, jb, lane);
+      block_store(m, sM, ib, jb, lane);
     }
     {   // ---- <Y, H> ----
       float pin = 0.f;
       if (before && behind) {
 #pragma unroll
-        for (int k = 0; k < SG_STATE_BYTES / 32 / SR_THREADS; ++k) {
-          const int idx = k * SR_THREADS + threadIdx.x, p = idx >> 4, c = ((idx & 15) >> 1) * 4 + (idx & 1);   // a chunk of upper terms
-          const uint4 yh = ld_shared16(tile_at<512>(sY, p, c)), yl = ld_shared16(tile_at<512>(sY, p, c + 2));
-          const uint4 hh = ld_shared16(tile_at<512>(sH, p, c)), hl = ld_shared16(tile_at<512>(sH, p, c + 2));
-          const uint32_t a[4] = {yh.x, yh.y, yh.z, yh.w}, al[4] = {yl.x, yl.y, yl.z, yl.w}, b[4] = {hh.x, hh.y, hh.z, hh.w}, bl[4] = {hl.x, hl.y, hl.z, hl.w};
-          float part = 0.f;
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float2 y0 = __half22float2(*reinterpret_cast<const __half2*>(&a[e])), y1 = __half22float2(*reinterpret_cast<const __half2*>(&al[e]));
-            const float2 h0 = __half22float2(*reinterpret_cast<const __half2*>(&b[e])), h1 = __half22float2(*reinterpret_cast<const __half2*>(&bl[e]));
-            part += (y0.x + y1.x) * (h0.x + h1.x) + (y0.y + y1.y) * (h0.y + h1.y);
-          }
-          const int blk = (p >> 4) * 8 + (c >> 2);
-          pin += part * yscales[blk] * hscales[blk];
+        for (int k = 0; k < SG_STATE_BYTES / 16 / SR_THREADS; ++k) {
+          const int idx = k * SR_THREADS + threadIdx.x;
+          const float4 a = ld_shared16f(wide_at<512>(sY, idx >> 5, idx & 31)), b = ld_shared16f(wide_at<512>(sH, idx >> 5, idx & 31));
+          pin += (a.x * b.x + a.y * b.y) + (a.z * b.z + a.w * b.w);
         }
         pin = warp_reduce<SumOp>(pin);
       }
@@ -1481,7 +1437,7 @@ __global__ void __launch_bounds__(SR_THREADS, 1) segment_reverse_kernel(const Se
     float o[2][1][4];
     if (behind) {
       float v[2][2][4], p[2][4];
-      times_state_n<2>(v, sx, sY, yscales, cols, part, lane);
+      times_state_n<2>(v, sx, sY, cols, part, lane);
       row_dots(v, st.left, sB, cols, sc.sv[cols], part, lane);
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
@@ -1492,7 +1448,7 @@ __global__ void __launch_bounds__(SR_THREADS, 1) segment_reverse_kernel(const Se
 #pragma unroll
           for (int e = 0; e < 4; ++e) gB[i][u][e] = fmaf(e < 2 ? d0 : d1, v[i][u][e], gB[i][u][e]);
       }
-      times_state_p<2>(p, sB, sY, yscales, cols, part, lane);
+      times_state_p<2>(p, sB, sY, cols, part, lane);
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         const int r = row_block<2>(i, part) * 16 + r0;
@@ -1514,7 +1470,7 @@ __global__ void __launch_bounds__(SR_THREADS, 1) segment_reverse_kernel(const Se
     {
       uint32_t b[4][2];
       load_steps(b, sgy, cols, lane);
-      times_scores<2, false, 1>(o, sMh, sMl, invM, b, part, lane);
+      times_scores<2, false, 1>(o, sM, b, part, lane);
       __half* gx = g.gx + (row * g.H + h) * SG_P + cols * 8 + 2 * q;
 #pragma unroll
       for (int i = 0; i < 2; ++i)
@@ -1522,13 +1478,14 @@ __global__ void __launch_bounds__(SR_THREADS, 1) segment_reverse_kernel(const Se
         for (int r = 0; r < 2; ++r) {
           const int j = row_block<2>(i, part) * 16 + r * 8 + r0;
           const float d = st.dt[j];
+          check = fmaf(o[i][0][2 * r], 0.f, fmaf(o[i][0][2 * r + 1], 0.f, check));
           if (j < rows) store_pair(gx + static_cast<size_t>(j) * g.H * SG_P, o[i][0][2 * r] * d, o[i][0][2 * r + 1] * d, g.vec);
         }
     }
     // ---- gC, gB ----
     if (before) {
       float v[2][2][4];
-      times_state_n<2>(v, sgy, sH, hscales, cols, part, lane);
+      times_state_n<2>(v, sgy, sH, cols, part, lane);
       row_dots(v, st.grow, sC, cols, sc.su[cols], part, lane);
 #pragma unroll
       for (int i = 0; i < 2; ++i)
@@ -1542,12 +1499,11 @@ __global__ void __launch_bounds__(SR_THREADS, 1) segment_reverse_kernel(const Se
     uint32_t b[4][4];   // these columns of B, then of C, over the steps
 #pragma unroll
     for (int k = 0; k < 4; ++k) load_b_t<SG_N * 2>(b[k], sB, k * 16, cols * 2, lane);
-    times_scores<2, true, 2>(gC, sWh, sWl, invW, b, part, lane);
+    times_scores<2, true, 2>(gC, sW, b, part, lane);
 #pragma unroll
     for (int k = 0; k < 4; ++k) load_b_t<SG_N * 2>(b[k], sC, k * 16, cols * 2, lane);
-    times_scores<2, false, 2>(gB, sWh, sWl, invW, b, part, lane);
+    times_scores<2, false, 2>(gB, sW, b, part, lane);
   }
-  float check = 0.f;   // becomes NaN with the first result that is none, or infinite
   const size_t bc = static_cast<size_t>(g.B) * g.L * g.G * SG_N;
   float* out = g.gb_part + static_cast<size_t>(sh.split) * 2 * bc + (row * g.G + sh.grp) * SG_N + cols * 16 + 2 * q;
 #pragma unroll
@@ -1607,7 +1563,7 @@ constexpr size_t SG_SMEM_FORWARD = SF_SMEM > SG_PLAIN_FORWARD ? SF_SMEM : SG_PLA
 constexpr size_t SG_SMEM_REVERSE = SR_SMEM > SG_PLAIN_REVERSE ? SR_SMEM : SG_PLAIN_REVERSE;
 static_assert(SG_N * SG_P <= SG_Q * SG_NPITCH, "the state takes the place of B");
 static_assert(2 * SG_SMEM_FORWARD <= 226 * 1024 && SG_SMEM_REVERSE <= 227 * 1024, "shared memory of an SM");
-static_assert(SF_S % 128 == 0 && SR_STAGE % 128 == 0, "tiles keep the phase of their chunks");
+static_assert(SF_TILES % 128 == 0 && SR_STAGE % 128 == 0, "tiles keep the phase of their chunks");
 
 // Shares of a group's heads: a CTA's time is its heads' and about `setup` heads' worth of loading, scores and writing of gB and gC (which
 // are also folded over the shares: `fold` per CTA of the whole grid), `slots` CTAs run at a time.
@@ -1627,7 +1583,7 @@ int segment_splits(int B, int L, int H, int G, int slots, float setup, float fol
 int forward_splits(int B, int L, int H, int G) { return segment_splits(B, L, H, G, 2 * 148, 0.7f, 0.f); }
 int reverse_splits(int B, int L, int H, int G) { return segment_splits(B, L, H, G, 148, 0.7f, 0.005f); }
 
-struct SegScratch { unsigned char* states; float* scales; float* decay; float* ga_part; float* gb_part; size_t total; };
+struct SegScratch { float* states; float* decay; float* ga_part; float* gb_part; size_t total; };
 SegScratch segment_carve(void* base, int B, int L, int H, int G, bool reverse) {
   SegScratch s;
   const size_t start = (256 - (reinterpret_cast<uintptr_t>(base) & 255)) & 255;   // the caller's pointer may have any alignment
@@ -1638,8 +1594,7 @@ SegScratch segment_carve(void* base, int B, int L, int H, int G, bool reverse) {
     return p;
   };
   const size_t units = static_cast<size_t>(B) * H * ((static_cast<size_t>(L) + SG_Q - 1) / SG_Q);
-  s.states = take(units * SG_STATE_BYTES * (reverse ? 2 : 1));
-  s.scales = reinterpret_cast<float*>(take(units * SG_BLOCKS * sizeof(float) * (reverse ? 2 : 1)));
+  s.states = reinterpret_cast<float*>(take(units * SG_STATE_BYTES * (reverse ? 2 : 1)));
   s.decay = reinterpret_cast<float*>(take(units * sizeof(float)));
   s.ga_part = reinterpret_cast<float*>(take(reverse ? units * sizeof(float) : 0));
   s.gb_part = reinterpret_cast<float*>(take(reverse ? static_cast<size_t>(reverse_splits(B, L, H, G)) * 2 * B * L * G * SG_N * sizeof(float) : 0));
@@ -1651,7 +1606,7 @@ SegArgs segment_args(const void* x, const void* dt, const void* A, const void* B
   SegArgs g{};
   g.x = static_cast<const __half*>(x); g.dt = static_cast<const float*>(dt); g.A = static_cast<const float*>(A);
   g.Bm = static_cast<const __half*>(Bm); g.Cm = static_cast<const __half*>(Cm);
-  g.states = w.states; g.scales = w.scales; g.decay = w.decay; g.ga_part = w.ga_part; g.gb_part = w.gb_part;
+  g.states = w.states; g.decay = w.decay; g.ga_part = w.ga_part; g.gb_part = w.gb_part;
   g.B = B; g.L = L; g.H = H; g.G = G; g.nseg = (L + SG_Q - 1) / SG_Q;
   g.vec = mp_aligned16(x) && mp_aligned16(Bm) && mp_aligned16(Cm);
   return g;
@@ -1663,7 +1618,7 @@ void segment_state_launches(const SegArgs& g, int directions, cudaStream_t st) {
   MP_CUDA_CHECK(cudaFuncSetAttribute(segment_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SS_SMEM)));
   MpLaunch(dim3(g.B * g.H * g.nseg, directions), SS_THREADS, SS_SMEM, st)(segment_states_kernel, g);
   MP_LAUNCH_CHECK();
-  MpLaunch(dim3(g.B * g.H * (SG_BLOCKS / (SC_THREADS / 32)), directions), SC_THREADS, 0, st)(segment_carry_kernel, g);
+  MpLaunch(dim3(g.B * g.H * (SG_N * SG_P / 4 / SC_THREADS), directions), SC_THREADS, 0, st)(segment_carry_kernel, g);
   MP_LAUNCH_CHECK();
 }
 

@@ -356,6 +356,56 @@ def test_ssd_segments_keep_fp32(mp, stream, orc, dims, shift, off):
         assert np.linalg.norm(d) <= tol[name] * np.linalg.norm(want), (name, np.linalg.norm(d) / np.linalg.norm(want))
 
 
+@pytest.mark.parametrize("which", ["x", "gy", "dt", "C"])
+def test_ssd_segments_of_values_far_apart(mp, stream, orc, which):
+    """Values of one 16 x 16 block up to 2^33 apart, the large ones against zeros of the other operand: the small ones alone make the results and
+    keep their bits.  A channel of x (of gy) at the end of r16's range where gy (x) has none, next to channels of 1e-5; step sizes of 1e-10
+    next to 1 where x is zero; rows of C at the end of the range where gy is zero, next to some of 1e-5."""
+    import torch
+    dims = (1, 200, 4, 64, 128, 2, 128)
+    nb, L, H, P, N, G, Q = dims
+    x, dt, A, Bm, Cm, gy = (a.astype(np.float64) for a in make_inputs(41, nb, L, H, P, N, G))
+    late = np.arange(L) % 16 >= 8
+    if which in ("x", "gy"):
+        large, other = (x, gy) if which == "x" else (gy, x)
+        Bm, Cm = 0.05 * Bm, 0.05 * Cm
+        large *= 1e-5
+        large[..., 3], other[..., 3] = 3e4, 0.0
+        other *= 1e3
+    elif which == "dt":
+        A *= 0.02
+        Bm, Cm = 30 * Bm, 30 * Cm
+        dt[:] = np.where(late, 1.0, 1e-10)[None, :, None]
+        x *= np.where(late, 0.0, 1000.0)[None, :, None, None]
+        gy *= 1e-2
+    else:
+        Bm, gy = 0.05 * Bm, 1e3 * gy
+        Cm *= np.where(late, 1e4, 1e-5)[None, :, None, None]
+        gy[:, late] = 0
+    x, Bm, Cm, gy = (a.astype(np.float16) for a in (x, Bm, Cm, gy))
+    dt, A = dt.astype(np.float32), A.astype(np.float32)
+    args = [dev(a) for a in (x, dt, A, Bm, Cm)]
+    y, gx, gdt, gA, gB, gC = (dev(np.full(a.shape, np.nan, a.dtype)) for a in (x, x, dt, A, Bm, Cm))
+    scratch = scratch_for(mp, dims, True)
+    torch.cuda.current_stream().synchronize()
+    mp.launch("ssd_scan", torch.float16, *args, y, scratch, *dims, stream)
+    mp.launch("ssd_scan_reverse", torch.float16, *args, dev(gy), gx, gdt, gA, gB, gC, scratch, *dims, stream)
+    stream.sync()
+    assert stream.status() == 0
+    f64 = lambda a: np.ascontiguousarray(a.astype(np.float64))
+    ref = (orc.ssd_forward(f64(x), f64(dt), f64(A), f64(Bm), f64(Cm)),) + tuple(orc.ssd_reverse(f64(x), f64(dt), f64(A), f64(Bm), f64(Cm), f64(gy)))
+    for got, want, name in zip((y, gx, gB, gC), (ref[0], ref[1], ref[4], ref[5]), ("y", "gx", "gB", "gC")):
+        # every row by itself, up to the rounding of its r16 values: 2^-11 / sqrt(3) of its norm, and half of 2^-24 each where that is more
+        d = np.linalg.norm(host(got).astype(np.float64) - want, axis=-1)
+        bound = 4e-4 * np.linalg.norm(want, axis=-1) + 2.0 ** -25 * np.sqrt(want.shape[-1])
+        if name == {"x": "y", "gy": "gx"}.get(which):     # (the large channel alone would be seen)
+            d = np.linalg.norm(np.delete(host(got).astype(np.float64) - want, 3, -1), axis=-1)
+            bound = 4e-4 * np.linalg.norm(np.delete(want, 3, -1), axis=-1) + 2.0 ** -25 * np.sqrt(want.shape[-1])
+        assert np.all(d <= bound), (name, (d / bound).max())
+    d = host(gdt).astype(np.float64) - ref[2]
+    assert np.linalg.norm(d) <= 2e-6 * np.linalg.norm(ref[2]), ("gdt", np.linalg.norm(d) / np.linalg.norm(ref[2]))
+
+
 @pytest.mark.parametrize("which,value,dims", [
     # an infinity or a NaN at two steps, in the middle of a segment and in the last one, which is partly filled: no product may carry it to a step or
     # a column that the recurrence keeps finite, and what is finite keeps its accuracy
