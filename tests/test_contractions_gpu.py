@@ -401,11 +401,25 @@ def test_r16_results_off_the_boundary(mp, stream, shape, off):
     assert stream.status() == 0
 
 
+def kernels(call):
+    """The kernels a call launches, by name."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        call()
+        torch.cuda.synchronize()
+    names = [e.name for e in p.events() if "gemm" in e.name]
+    assert names, "no kernel was recorded"
+    return names
+
+
 # r16 contractions with fewer 256 x 256 tiles than CTA pairs, which take the pairs where that saves rounds of tiles: ragged last tiles of both
-# directions, one K block more than whole ones, a residual, a bias and the old C; against the single CTAs' kernel to the rounding of a result.
-@pytest.mark.parametrize("shape", [(3000, 1000, 1000), (2570, 1032, 776), (4096, 1096, 520), (2048, 2048, 2048)])
+# directions, one K block more than whole ones, a residual, a bias and the old C.  Bit for bit as the single CTAs' kernel has them, and that to the
+# rounding of a result.
+@pytest.mark.parametrize("shape,pairs", [((3000, 1000, 1000), True), ((2824, 1032, 776), True), ((4096, 1096, 520), True), ((2048, 2048, 2048), True),
+                                         ((2570, 1032, 776), False)])      # (one round of single CTAs' tiles)
 @pytest.mark.parametrize("variant", ["ij_jk_ik", "ij_kj_ik", "ji_jk_ik"])
-def test_pairs_on_few_tiles(mp, stream, monkeypatch, shape, variant):
+def test_pairs_on_few_tiles(mp, stream, monkeypatch, shape, pairs, variant):
     import torch
     m, n, k = shape
     g = torch.Generator(device="cuda").manual_seed(sum(shape))
@@ -426,9 +440,59 @@ def test_pairs_on_few_tiles(mp, stream, monkeypatch, shape, variant):
 
     want = [ref, 0.5 * ref + 6.0, ref + term.double(), ref + bias.double()]
     got = results()
+    assert all(("pair" in name) == pairs for name in kernels(results))
     monkeypatch.setenv("MP_GEMM_NO_PAIRS", "1")      # read at every launch
     single = results()
+    assert not any("pair" in name for name in kernels(results))
     for c, s, w in list(zip(got, single, want))[:4 if variant == "ij_jk_ik" else 2]:
-        assert float((c.double() - w).norm() / w.norm()) <= 2.9e-4      # the rounding of an r16 result
-        assert float((s.double() - w).norm() / w.norm()) <= 2.9e-4
+        assert torch.equal(c, s)
+        assert float((s.double() - w).norm() / w.norm()) <= 2.9e-4      # the rounding of an r16 result
+    assert stream.status() == 0
+
+
+# CTA pairs on an A of more than 64 MB, where tiles come in groups of eight row blocks: 34 row blocks, so that the last group has two.
+@pytest.mark.parametrize("variant", ["ij_jk_ik", "ji_jk_ik"])
+def test_pairs_in_groups_of_row_blocks(mp, stream, monkeypatch, variant):
+    import torch
+    m, n, k = 8488, 4096, 1288
+    g = torch.Generator(device="cuda").manual_seed(m)
+    a, b = torch.randn(m, n, generator=g, device="cuda").half(), torch.randn(n, k, generator=g, device="cuda").half()
+    da = (a.t() if variant[0] == "j" else a).contiguous()
+
+    def result():
+        c = torch.full((m, k), 3.0, device="cuda", dtype=torch.float16)
+        run(mp, stream, "inner_product_" + variant, "r16", da, b, 1.0, c, 0.0, m, n, k)
+        return c
+
+    c = result()
+    assert all("pair" in name for name in kernels(result))
+    ref = a.double() @ b.double()
+    assert bool(((c.double() - ref).norm(dim=1) <= 2.9e-4 * ref.norm(dim=1)).all())      # the rounding of an r16 result, every row
+    monkeypatch.setenv("MP_GEMM_NO_PAIRS", "1")      # read at every launch
+    assert torch.equal(c, result())
+    assert stream.status() == 0
+
+
+# CTA pairs into a C with rows off the 16-byte boundary, from aligned operands: whole words, odd ends, a last block of one column.
+@pytest.mark.parametrize("shape", [(6000, 512, 1001), (5001, 128, 2049), (4870, 256, 1059)])
+@pytest.mark.parametrize("off", [0, 1])
+def test_pairs_into_rows_off_the_boundary(mp, stream, monkeypatch, shape, off):
+    import torch
+    m, n, k = shape
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    a, b = torch.randn(m, n, generator=g, device="cuda").half(), torch.randn(k, n, generator=g, device="cuda").half()
+
+    def result():
+        flat = torch.full((m * k + 16,), 7.0, device="cuda", dtype=torch.float16)
+        run(mp, stream, "inner_product_ij_kj_ik", "r16", a, b, 1.0, flat[off:off + m * k].view(m, k), 0.0, m, n, k)
+        return flat
+
+    flat = result()
+    assert all("pair" in name for name in kernels(result))
+    ref = a.double() @ b.double().t()
+    c = flat[off:off + m * k].view(m, k).double()
+    assert bool(((c - ref).norm(dim=1) <= 2.9e-4 * ref.norm(dim=1)).all())      # the rounding of an r16 result, every row
+    assert bool((flat[:off] == 7).all()) and bool((flat[off + m * k:] == 7).all())
+    monkeypatch.setenv("MP_GEMM_NO_PAIRS", "1")      # read at every launch
+    assert torch.equal(flat, result())
     assert stream.status() == 0

@@ -429,9 +429,10 @@ def test_ssd_segments_with_infinities(mp, stream, orc, which, value, dims):
     f64 = [np.ascontiguousarray(a.astype(np.float64)) for a in ins]
     with np.errstate(all="ignore"):
         ref = (orc.ssd_forward(*f64[:5]),) + tuple(orc.ssd_reverse(*f64))
-    for got, want, name in zip((y, gx, gB, gC), (ref[0], ref[1], ref[4], ref[5]), ("y", "gx", "gB", "gC")):
+    # (tolerances of test_ssd_segments_keep_fp32)
+    for got, want, name, tol in zip((y, gx, gdt, gA, gB, gC), ref, ("y", "gx", "gdt", "gA", "gB", "gC"), (2.9e-4, 2.9e-4, 2e-6, 2e-5, 2.9e-4, 2.9e-4)):
         got = host(got).astype(np.float64)
         finite = np.isfinite(want)
         assert np.array_equal(np.isfinite(got), finite), f"{name}: {np.sum(~np.isfinite(got))} not finite, {np.sum(~finite)} expected"
         d = got[finite] - want[finite]
-        assert np.linalg.norm(d) <= 2.9e-4 * np.linalg.norm(want[finite]), name   # the rounding of an r16 result
+        assert np.linalg.norm(d) <= tol * np.linalg.norm(want[finite]), name
