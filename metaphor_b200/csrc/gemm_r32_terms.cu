@@ -1,7 +1,7 @@
 // r32 contractions of some size: the operands are first written as three bf16 terms each, and the products are bf16 MMAs on CTA pairs.
 //
 // A value becomes h0 + h1 + h2, each the rest of the one before rounded to bf16: 24 bits, all there are, and as bf16 has the exponents of fp32 every
-// value keeps its own (terms below 2^-133 are rounded to multiples of it).  Of the nine products the three of the smallest terms are left out:
+// value keeps its own (the last terms of values below 2^-110 are rounded to multiples of 2^-133; gemm_r32.cu cuts them off at 2^-136).  Of the nine products the three of the smallest terms are left out:
 //     a b ~ a0 b0 + (a0 b1 + a1 b0) + (a0 b2 + a2 b0 + a1 b1),    2^-26 of a product at most.
 // The tensor core's accumulator truncates, so that it is handed over to the epilogue warps every 32 of K, which add it up in registers with
 // rounding; the small products come before the large ones, so that only two additions truncate at full size.  2-norm of the error at
